@@ -1,0 +1,91 @@
+"""Prompts of any length in one pass: the logits and the state a decode continues from, against the FP32 model."""
+import pytest
+import torch
+
+from warpstate_ai_b200 import WarpStateConfig, WarpStateLM
+from warpstate_ai_b200.ops import reference as R
+from warpstate_ai_b200.ops.gemm import check_device_errors
+from warpstate_ai_b200.serve.engine import DecodeEngine
+
+pytestmark = pytest.mark.gpu
+
+
+def model_of(heads, ffn, depth=3):
+    torch.manual_seed(heads)
+    cfg = WarpStateConfig(vocab_size=512, d_model=64 * heads, n_heads=heads, n_cores=2, logical_depth=depth, ffn_hidden=ffn,
+                          chunk_size=128, gradient_checkpointing=False, parallel_memory=True)
+    with torch.device("cuda"):
+        model = WarpStateLM(cfg).eval().requires_grad_(False)
+        for core in model.cores:
+            core.fast_decay_logit.normal_(1.0, 0.5)
+            core.memory_mix_logit.normal_(0.0, 0.5)
+    return model
+
+
+def expected_state(model, ids):
+    """(logits at the last position, fast, slow, roped K, V, U of the open chunk) of layer 0 and of the last, FP32."""
+    batch, length = ids.shape
+    complete, rest = divmod(length, 128)
+    padded = torch.nn.functional.pad(ids, (0, -length % 128))
+    x, kept = model.embed(padded), []
+    for depth, core in model._depths():
+        x = x * (1.0 + model.depth_scale[depth]) + model.depth_bias[depth]
+        packed = core.in_proj(core.norm1(x))
+        _, k, v, _, u = R.split_heads(packed, core.h, 128)
+        k = R.apply_rope(k, core.rope_cos, core.rope_sin)
+        if complete:
+            _, memories = R.attention_memory(packed[:, :complete * 128], *core._memory_arguments(), return_state=True)
+        else:
+            memories = (torch.zeros(batch, core.h, 64, 64, device="cuda"),) * 2
+        caches = [torch.zeros(batch, core.h, 128, 64, device="cuda") for _ in range(3)]
+        for cache, t in zip(caches, (k, v, u)):
+            cache[:, :, :rest] = t[:, complete, :, :rest] if rest else 0.0
+        kept.append((*memories, *caches))
+        x = core(x)
+    return model.logits_from_hidden(model.final_norm(x))[:, length - 1], kept[0], kept[-1]
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-9))
+
+
+@pytest.mark.parametrize("batch,heads,ffn,use_kernels", [(1, 4, 512, True), (3, 2, 192, True), (70, 2, 192, True), (2, 4, 512, False)])
+@pytest.mark.parametrize("length", [1, 31, 127, 128, 129, 300, 1153])
+def test_prompt_of_any_length_in_one_pass(batch, heads, ffn, use_kernels, length):
+    # BF16 inputs to every product and three layers: 2^-8 per rounding, about ten of them on the way to a logit or a
+    # state of the last layer, adding as a random walk -> 2 % at most; layer 0's K, V, U see three roundings
+    model = model_of(heads, ffn)
+    ids = torch.randint(0, 512, (batch, length + 3), device="cuda")
+    engine = DecodeEngine(model, dtype=torch.bfloat16, use_kernels=use_kernels)
+    engine.prefill(ids[:, :1])                                       # leaves values of another prompt in the state
+    engine.step(ids[:, 1])
+    logits = engine.prefill(ids[:, :length]).clone()
+    check_device_errors()
+    want, first, last = expected_state(model, ids[:, :length])
+    assert engine.pos == length % 128
+    assert rel(logits, want) < 0.02
+    for state, expected, bound in ((engine.states[0], first, 0.01), (engine.states[-1], last, 0.02)):
+        for name, value in zip(("fast", "slow", "k", "v", "u"), expected):
+            assert rel(getattr(state, name), value) < bound, (name, bound)
+            if name in ("k", "v", "u"):
+                assert torch.count_nonzero(getattr(state, name)[:, :, length % 128:]) == 0, name
+    for position in range(length, length + 3):                        # a decode continues from it
+        stepped = engine.step(ids[:, position])
+    check_device_errors()
+    assert rel(stepped, expected_state(model, ids[:, :length + 3])[0]) < 0.02
+
+
+def test_a_prefilled_state_equals_a_stepped_one():
+    """The same prompt through the step kernels: what the two leave behind differs by BF16 roundings only."""
+    model = model_of(4, 512)
+    ids = torch.randint(0, 512, (3, 200), device="cuda")
+    whole, stepped = DecodeEngine(model), DecodeEngine(model)
+    logits = whole.prefill(ids)
+    for position in range(200):
+        last = stepped.step(ids[:, position])
+    assert rel(logits, last) < 0.02 and whole.pos == stepped.pos
+    for a, b in zip(whole.states, stepped.states):
+        for name in ("fast", "slow", "mixed"):
+            assert rel(getattr(a, name), getattr(b, name)) < 0.02, name
+        for name in ("k", "v", "u"):
+            assert rel(getattr(a, name)[:, :, :72], getattr(b, name)[:, :, :72]) < 0.02, name

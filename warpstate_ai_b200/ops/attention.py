@@ -65,6 +65,15 @@ def forward_only(qkvgu: torch.Tensor, core, batch: int, seq: int, want_final: bo
     return y, writes, states, (ff, fs)
 
 
+def prefill(qkvgu: torch.Tensor, core, batch: int, seq: int, state) -> torch.Tensor:
+    """y [M,d] for prompts of any length; ``state`` (fast, slow, mixed, k, v, u of a decode layer) is overwritten with
+    what a decode continues from: the memories after the complete chunks, and the open chunk's K, V and U."""
+    _ext.require()
+    return torch.ops.ws_b200.attn_prefill(qkvgu, rope_table(qkvgu.device, pair_major=True), *_logits(core), batch, seq,
+                                          core.h, state.fast, state.slow, state.mixed, state.k, state.v, state.u,
+                                          error_flag(qkvgu.device))
+
+
 def forward(qkvgu: torch.Tensor, core, batch: int, seq: int):
     y, writes, states, _ = forward_only(qkvgu, core, batch, seq)
     return y, (writes, states)

@@ -82,4 +82,22 @@ inline int make_tile_map(CUtensorMap* map, const void* base, uint64_t cols, uint
   return make_map_bf16(map, base, cols, rows, ld, box_cols, box_rows);
 }
 
+// Host: 3-D map (column, position, sequence) over a token-major BF16 matrix [sequences * length, cols], for swizzled
+// tiles of one sequence: a box that reaches past the sequence's last position is filled with zeros on a load and
+// clipped on a store, instead of running into the next sequence.
+inline int make_sequence_map(CUtensorMap* map, const void* base, uint64_t cols, uint64_t length, uint64_t sequences,
+                             uint32_t box_cols, uint32_t box_rows) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return -10;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (cols * 2) % 16 != 0) return -11;
+  cuuint64_t dims[3] = {cols, length, sequences};
+  cuuint64_t strides[2] = {cols * 2, length * cols * 2};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -12;
+}
+
 }  // namespace ws

@@ -39,10 +39,10 @@ chunk_writes_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int n_chunks = T / CHUNK;
+  const int n_chunks = (T + CHUNK - 1) / CHUNK;
   const int tile = blockIdx.x;
   const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-  const int row0 = b * T + n * CHUNK;
+  const int row0 = n * CHUNK;
 
   if (tid == 0) {
     mbar_init(&bars[0], 1);
@@ -63,8 +63,8 @@ chunk_writes_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_c
 
   if (tid == 0) {
     mbar_expect_tx(&bars[0], 2 * TILE_BYTES);
-    tma_load_2d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0);
-    tma_load_2d(sU, &tm_qkvgu, &bars[0], 4 * d + h * HD, row0);
+    tma_load_3d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0, b);
+    tma_load_3d(sU, &tm_qkvgu, &bars[0], 4 * d + h * HD, row0, b);
   }
   bool ok = mbar_wait(&bars[0], 0, abort_flag);
   if (ok) {
@@ -158,7 +158,7 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_chunks = T / CHUNK;
+  const int n_chunks = (T + CHUNK - 1) / CHUNK;
 
   if (tid == 0) {
     for (int s = 0; s < WS_STAGES; ++s) {
@@ -193,10 +193,10 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
         const int s = i % WS_STAGES;
         if (!mbar_wait(&empty[s], ((i / WS_STAGES) & 1) ^ 1, abort_flag)) break;
         const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-        const int row0 = b * T + n * CHUNK;
+        const int row0 = n * CHUNK;
         mbar_expect_tx(&full[s], 2 * TILE_BYTES);
-        tma_load_2d(ring + s * 2 * TILE_BYTES, &tm_qkvgu, &full[s], 1 * d + h * HD, row0);
-        tma_load_2d(ring + s * 2 * TILE_BYTES + TILE_BYTES, &tm_qkvgu, &full[s], 4 * d + h * HD, row0);
+        tma_load_3d(ring + s * 2 * TILE_BYTES, &tm_qkvgu, &full[s], 1 * d + h * HD, row0, b);
+        tma_load_3d(ring + s * 2 * TILE_BYTES + TILE_BYTES, &tm_qkvgu, &full[s], 4 * d + h * HD, row0, b);
       }
     }
   } else if (warp < 16) {
@@ -312,7 +312,8 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
 
 // =============================================================================== scan
 // writes [B,N,H,4096] FP32 -> states [B,N,H,4096] BF16 (mixed state read by chunk n), and
-// optionally the fast / slow states after the last chunk [B,H,4096] FP32 (prefill).
+// optionally the fast / slow states [B,H,4096] FP32 after the first `complete` chunks, with their BF16 mix
+// (prefill: a prompt that ends inside a chunk leaves the state of the chunks before it).
 // One thread owns four consecutive state elements (16-byte loads, 8-byte stores) and requests the writes of
 // SCAN_AHEAD chunks before it runs their recurrence, so a thread keeps 128 bytes in flight instead of 4.
 constexpr int SCAN_AHEAD = 8;
@@ -321,8 +322,9 @@ __global__ void __launch_bounds__(128)
 memory_scan_kernel(const float* __restrict__ writes, const float* __restrict__ fast_logit,
                    const float* __restrict__ slow_logit, const float* __restrict__ mix_logit,
                    __nv_bfloat16* __restrict__ states, float* __restrict__ final_fast,
-                   float* __restrict__ final_slow, const float* __restrict__ init_fast,
-                   const float* __restrict__ init_slow, int B, int N, int H) {
+                   float* __restrict__ final_slow, __nv_bfloat16* __restrict__ final_mixed,
+                   const float* __restrict__ init_fast, const float* __restrict__ init_slow, int B, int N, int complete,
+                   int H) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t quad = blockIdx.x * static_cast<size_t>(128) + threadIdx.x;  // over B*H*1024 groups of four
@@ -339,6 +341,17 @@ memory_scan_kernel(const float* __restrict__ writes, const float* __restrict__ f
   float4 s = init_slow != nullptr ? *reinterpret_cast<const float4*>(init_slow + flat) : make_float4(0.f, 0.f, 0.f, 0.f);
   const size_t chunk_stride = static_cast<size_t>(H) * 4096;
   const size_t base = (static_cast<size_t>(b) * N * H + h) * 4096 + e;
+  auto mixed = [&]() {
+    uint2 o;
+    o.x = pack_bf16x2(mix * f.x + (1.f - mix) * s.x, mix * f.y + (1.f - mix) * s.y);
+    o.y = pack_bf16x2(mix * f.z + (1.f - mix) * s.z, mix * f.w + (1.f - mix) * s.w);
+    return o;
+  };
+  auto leave = [&]() {
+    *reinterpret_cast<float4*>(final_fast + flat) = f;
+    *reinterpret_cast<float4*>(final_slow + flat) = s;
+    if (final_mixed != nullptr) *reinterpret_cast<uint2*>(final_mixed + flat) = mixed();
+  };
   for (int n0 = 0; n0 < N; n0 += SCAN_AHEAD) {
     float4 w[SCAN_AHEAD];
 #pragma unroll
@@ -347,21 +360,48 @@ memory_scan_kernel(const float* __restrict__ writes, const float* __restrict__ f
 #pragma unroll
     for (int j = 0; j < SCAN_AHEAD; ++j) {
       if (n0 + j >= N) break;
-      if (states != nullptr) {
-        uint2 o;
-        o.x = pack_bf16x2(mix * f.x + (1.f - mix) * s.x, mix * f.y + (1.f - mix) * s.y);
-        o.y = pack_bf16x2(mix * f.z + (1.f - mix) * s.z, mix * f.w + (1.f - mix) * s.w);
-        *reinterpret_cast<uint2*>(states + base + (n0 + j) * chunk_stride) = o;
-      }
+      if (states != nullptr) *reinterpret_cast<uint2*>(states + base + (n0 + j) * chunk_stride) = mixed();
+      if (n0 + j == complete && final_fast != nullptr) leave();
       f.x = df * f.x + (1.f - df) * w[j].x; f.y = df * f.y + (1.f - df) * w[j].y;
       f.z = df * f.z + (1.f - df) * w[j].z; f.w = df * f.w + (1.f - df) * w[j].w;
       s.x = ds * s.x + (1.f - ds) * w[j].x; s.y = ds * s.y + (1.f - ds) * w[j].y;
       s.z = ds * s.z + (1.f - ds) * w[j].z; s.w = ds * s.w + (1.f - ds) * w[j].w;
     }
   }
-  if (final_fast != nullptr) {
-    *reinterpret_cast<float4*>(final_fast + flat) = f;
-    *reinterpret_cast<float4*>(final_slow + flat) = s;
+  if (complete == N && final_fast != nullptr) leave();
+}
+
+// =============================================================================== open chunk of a prompt
+// What a decode needs of the chunk a prompt ends in: roped K, V and U of its `rest` positions, as the step kernel
+// appends them, and zeros behind them (rest = 0 clears the caches).  One CTA per (sequence, head); 16-byte pieces.
+__global__ void __launch_bounds__(256)
+open_chunk_kernel(const __nv_bfloat16* __restrict__ qkvgu, const float2* __restrict__ rope, int T, int rest, int H, int d,
+                  __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x % H, b = blockIdx.x / H;
+  const size_t cache = static_cast<size_t>(blockIdx.x) * CHUNK * HD;
+  const __nv_bfloat16* base = qkvgu + (static_cast<size_t>(b) * T + (T - rest)) * 5 * d + h * HD;
+  for (int i = threadIdx.x; i < CHUNK * 8; i += 256) {
+    const int r = i >> 3, j = i & 7;
+    uint4 k = make_uint4(0u, 0u, 0u, 0u), v = k, u = k;
+    if (r < rest) {
+      const __nv_bfloat16* row = base + static_cast<size_t>(r) * 5 * d + j * 8;
+      k = *reinterpret_cast<const uint4*>(row + d);
+      v = *reinterpret_cast<const uint4*>(row + 2 * d);
+      u = *reinterpret_cast<const uint4*>(row + 4 * d);
+      uint32_t* w = reinterpret_cast<uint32_t*>(&k);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 x = rope_rotate(__bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t])),
+                                     rope[(j * 4 + t) * CHUNK + r]);
+        w[t] = pack_bf16x2(x.x, x.y);
+      }
+    }
+    const size_t at = cache + static_cast<size_t>(r) * HD + j * 8;
+    *reinterpret_cast<uint4*>(kc + at) = k;
+    *reinterpret_cast<uint4*>(vc + at) = v;
+    *reinterpret_cast<uint4*>(uc + at) = u;
   }
 }
 
@@ -392,10 +432,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int n_chunks = T / CHUNK;
+  const int n_chunks = (T + CHUNK - 1) / CHUNK;
   const int tile = blockIdx.x;
   const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-  const int row0 = b * T + n * CHUNK;
+  const int row0 = n * CHUNK;
 
   if (tid == 0) {
     mbar_init(&bars[0], 1);
@@ -419,10 +459,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 
   if (tid == 0) {
     mbar_expect_tx(&bars[0], 4 * TILE_BYTES + 8192);
-    tma_load_2d(sQ, &tm_qkvgu, &bars[0], 0 * d + h * HD, row0);
-    tma_load_2d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0);
-    tma_load_2d(sV, &tm_qkvgu, &bars[0], 2 * d + h * HD, row0);
-    tma_load_2d(sG, &tm_qkvgu, &bars[0], 3 * d + h * HD, row0);
+    tma_load_3d(sQ, &tm_qkvgu, &bars[0], 0 * d + h * HD, row0, b);
+    tma_load_3d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0, b);
+    tma_load_3d(sV, &tm_qkvgu, &bars[0], 2 * d + h * HD, row0, b);
+    tma_load_3d(sG, &tm_qkvgu, &bars[0], 3 * d + h * HD, row0, b);
     tma_load_2d(sSt, &tm_state, &bars[0], 0, tile * HD);
   }
   bool ok = mbar_wait(&bars[0], 0, abort_flag);
@@ -527,8 +567,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   fence_proxy_async_smem();
   __syncwarp();
   if ((tid & 31) == 0) {
-    if (ok) {
-      tma_store_2d(&tm_y, sQ + warp * 4096, h * HD, row0 + warp * 32);
+    if (ok && row0 + warp * 32 < T) {
+      tma_store_3d(&tm_y, sQ + warp * 4096, h * HD, row0 + warp * 32, b);
       tma_store_commit();
     }
     tma_store_wait_read0();
@@ -579,7 +619,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(setfree + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_chunks = T / CHUNK;
+  const int n_chunks = (T + CHUNK - 1) / CHUNK;
 
   if (tid == 0) {
     for (int s = 0; s < AS_STAGES; ++s) {
@@ -618,13 +658,13 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         const int s = i % AS_STAGES;
         if (!mbar_wait(&empty[s], ((i / AS_STAGES) & 1) ^ 1, abort_flag)) break;
         const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-        const int row0 = b * T + n * CHUNK;
+        const int row0 = n * CHUNK;
         uint8_t* st = stage_ptr(s);
         mbar_expect_tx(&full[s], AS_STAGE_BYTES);
-        tma_load_2d(st, &tm_qkvgu, &full[s], 0 * d + h * HD, row0);
-        tma_load_2d(st + TILE_BYTES, &tm_qkvgu, &full[s], 1 * d + h * HD, row0);
-        tma_load_2d(st + 2 * TILE_BYTES, &tm_qkvgu, &full[s], 3 * d + h * HD, row0);
-        tma_load_2d(st + 3 * TILE_BYTES, &tm_qkvgu, &full[s], 2 * d + h * HD, row0);
+        tma_load_3d(st, &tm_qkvgu, &full[s], 0 * d + h * HD, row0, b);
+        tma_load_3d(st + TILE_BYTES, &tm_qkvgu, &full[s], 1 * d + h * HD, row0, b);
+        tma_load_3d(st + 2 * TILE_BYTES, &tm_qkvgu, &full[s], 3 * d + h * HD, row0, b);
+        tma_load_3d(st + 3 * TILE_BYTES, &tm_qkvgu, &full[s], 2 * d + h * HD, row0, b);
         tma_load_2d(st + 4 * TILE_BYTES, &tm_state, &full[s], 0, tile * HD);
       }
     }
@@ -710,7 +750,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       uint8_t* sG = sQ + 2 * TILE_BYTES;
       uint8_t* sV = sQ + 3 * TILE_BYTES;
       const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-      const int row0 = b * T + n * CHUNK;
+      const int row0 = n * CHUNK;
       uint32_t landed = 0;
       if (lane == 0) landed = mbar_wait(&sfull[g], k2 & 1, abort_flag) ? 1u : 0u;
       bool ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
@@ -809,8 +849,8 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       __syncwarp();
       if (lane == 0) {
         mbar_arrive(&setfree[g]);   // this warp's lanes of S / O / Mem have been read
-        if (ok) {
-          tma_store_2d(&tm_y, sQ + wq * 4096, h * HD, row0 + wq * 32);
+        if (ok && row0 + wq * 32 < T) {
+          tma_store_3d(&tm_y, sQ + wq * 4096, h * HD, row0 + wq * 32, b);
           tma_store_commit();
         }
         tma_store_wait_read0();
@@ -847,11 +887,14 @@ extern "C" int ws_attn_stream_form(void) {
   return from_env ? 1 : 0;
 }
 
-extern "C" int ws_chunk_writes(const void* qkvgu, const float* rope, float* writes, int B, int T, int H, int d,
-                               int* error_flag, cudaStream_t stream) {
-  if (T % CHUNK != 0 || d != H * HD) return -1;
+// The tile kernels address tokens as (position, sequence): a chunk that reaches past the end of its sequence reads
+// zeros there (the tensor map's fill) and its stores are clipped.  Behind the causal mask those positions change
+// nothing of the others, and tanh(0) adds nothing to a write.
+static int chunk_writes(const void* qkvgu, const float* rope, float* writes, int B, int T, int H, int d, int* error_flag,
+                        cudaStream_t stream) {
+  if (T <= 0 || d != H * HD) return -1;
   CUtensorMap tm;
-  int rc = make_tile_map(&tm, qkvgu, 5 * (uint64_t)d, (uint64_t)B * T, 5 * (uint64_t)d, HD, CHUNK);
+  int rc = make_sequence_map(&tm, qkvgu, 5 * (uint64_t)d, T, B, HD, CHUNK);
   if (rc) return rc;
   static bool configured = false;
   if (!configured) {
@@ -859,7 +902,7 @@ extern "C" int ws_chunk_writes(const void* qkvgu, const float* rope, float* writ
       return -20;
     configured = true;
   }
-  const int tiles = B * (T / CHUNK) * H;
+  const int tiles = B * ((T + CHUNK - 1) / CHUNK) * H;
   CUtensorMap to;
   rc = make_map_f32(&to, writes, HD, (uint64_t)tiles * HD, HD, 32, 32);
   if (rc) return rc;
@@ -882,27 +925,40 @@ extern "C" int ws_chunk_writes(const void* qkvgu, const float* rope, float* writ
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-extern "C" int ws_memory_scan(const float* writes, const float* fast_logit, const float* slow_logit,
-                              const float* mix_logit, void* states, float* final_fast, float* final_slow,
-                              const float* init_fast, const float* init_slow, int B, int N, int H,
-                              cudaStream_t stream) {
+extern "C" int ws_chunk_writes(const void* qkvgu, const float* rope, float* writes, int B, int T, int H, int d,
+                               int* error_flag, cudaStream_t stream) {
+  return T % CHUNK != 0 ? -1 : chunk_writes(qkvgu, rope, writes, B, T, H, d, error_flag, stream);
+}
+
+static int memory_scan(const float* writes, const float* fast_logit, const float* slow_logit, const float* mix_logit,
+                       void* states, float* final_fast, float* final_slow, void* final_mixed, const float* init_fast,
+                       const float* init_slow, int B, int N, int complete, int H, cudaStream_t stream) {
   const size_t total = (size_t)B * H * 4096;
-  launch_dependent(memory_scan_kernel, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, stream, writes, fast_logit, slow_logit, mix_logit, (__nv_bfloat16*)states, final_fast, final_slow, init_fast,
-      init_slow, B, N, H);
+  launch_dependent(memory_scan_kernel, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, stream, writes, fast_logit,
+                   slow_logit, mix_logit, (__nv_bfloat16*)states, final_fast, final_slow, (__nv_bfloat16*)final_mixed,
+                   init_fast, init_slow, B, N, complete, H);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-extern "C" int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H,
-                           int d, int* error_flag, cudaStream_t stream) {
-  if (T % CHUNK != 0 || d != H * HD) return -1;
-  const int tiles = B * (T / CHUNK) * H;
+extern "C" int ws_memory_scan(const float* writes, const float* fast_logit, const float* slow_logit,
+                              const float* mix_logit, void* states, float* final_fast, float* final_slow,
+                              const float* init_fast, const float* init_slow, int B, int N, int H,
+                              cudaStream_t stream) {
+  return memory_scan(writes, fast_logit, slow_logit, mix_logit, states, final_fast, final_slow, nullptr, init_fast,
+                     init_slow, B, N, N, H, stream);
+}
+
+static int attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H, int d,
+                    int* error_flag, cudaStream_t stream) {
+  if (T <= 0 || d != H * HD) return -1;
+  const int tiles = B * ((T + CHUNK - 1) / CHUNK) * H;
   CUtensorMap tm, ts, ty;
-  int rc = make_tile_map(&tm, qkvgu, 5 * (uint64_t)d, (uint64_t)B * T, 5 * (uint64_t)d, HD, CHUNK);
+  int rc = make_sequence_map(&tm, qkvgu, 5 * (uint64_t)d, T, B, HD, CHUNK);
   if (rc) return rc;
   rc = make_tile_map(&ts, states, HD, (uint64_t)tiles * HD, HD, HD, HD);
   if (rc) return rc;
-  rc = make_tile_map(&ty, y, (uint64_t)d, (uint64_t)B * T, (uint64_t)d, HD, 32);
+  rc = make_sequence_map(&ty, y, (uint64_t)d, T, B, HD, 32);
   if (rc) return rc;
   static bool configured = false;
   if (!configured) {
@@ -924,6 +980,29 @@ extern "C" int ws_attn_fwd(const void* qkvgu, const void* states, const float* r
   else
     launch_dependent(attn_fwd_kernel, dim3(tiles), dim3(128), AF_SMEM, stream, tm, ts, ty, reinterpret_cast<const float2*>(rope), T, H, d,
                      error_flag);
+  ws_count_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+extern "C" int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H,
+                           int d, int* error_flag, cudaStream_t stream) {
+  return T % CHUNK != 0 ? -1 : attn_fwd(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
+}
+
+extern "C" int ws_attn_prefill(const void* qkvgu, const float* rope, const float* fast_logit, const float* slow_logit,
+                               const float* mix_logit, float* writes, void* states, void* y, float* fast, float* slow,
+                               void* mixed, void* kc, void* vc, void* uc, int B, int T, int H, int d, int* error_flag,
+                               cudaStream_t stream) {
+  const int complete = T / CHUNK, rest = T % CHUNK;
+  int rc = chunk_writes(qkvgu, rope, writes, B, T, H, d, error_flag, stream);
+  if (!rc)
+    rc = memory_scan(writes, fast_logit, slow_logit, mix_logit, states, fast, slow, mixed, nullptr, nullptr, B,
+                     complete + (rest > 0), complete, H, stream);
+  if (!rc) rc = attn_fwd(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
+  if (rc) return rc;
+  launch_dependent(open_chunk_kernel, dim3(B * H), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkvgu),
+                   reinterpret_cast<const float2*>(rope), T, rest, H, d, static_cast<__nv_bfloat16*>(kc),
+                   static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc));
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

@@ -34,9 +34,14 @@ int64_t opt_ld(const c10::optional<at::Tensor>& t) {
 // Generic GEMM entry.  `a`/`b` are 2-D BF16 tensors whose last dimension is contiguous; the
 // caller states how they are to be read (a_mn/b_mn) and the problem size.
 void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_t epilogue,
-          int64_t m, int64_t n, int64_t k, at::Tensor out, c10::optional<at::Tensor> out2,
+          int64_t m, int64_t n, int64_t k, c10::optional<at::Tensor> out_, c10::optional<at::Tensor> out2,
           c10::optional<at::Tensor> aux, c10::optional<at::Tensor> row_scale, double alpha,
           double beta, c10::optional<at::Tensor> error_flag) {
+  // the packed (up | gate) matrix of the SwiGLU epilogue is optional: only a backward pass reads it
+  const bool has_out = out_.has_value() && out_->defined();
+  TORCH_CHECK(has_out || (out2.has_value() && out2->defined()), "gemm: an output is required");
+  TORCH_CHECK(has_out || epilogue == WS_EPI_SWIGLU, "gemm: out required");
+  const at::Tensor& out = has_out ? *out_ : *out2;
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && out.is_cuda(), "gemm: CUDA tensors required");
   TORCH_CHECK(a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16,
               "gemm: BF16 operands required");
@@ -54,7 +59,7 @@ void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_
   else { TORCH_CHECK(b.size(0) == k && b.size(1) == b_rows, "gemm: B must be [k,n]"); }
   const bool f32_out = epilogue == WS_EPI_RESID_F32 || epilogue == WS_EPI_ACC_F32 || epilogue == WS_EPI_F32;
   TORCH_CHECK(out.scalar_type() == (f32_out ? at::kFloat : at::kBFloat16), "gemm: wrong out dtype");
-  const int64_t out_cols = (epilogue == WS_EPI_SWIGLU || epilogue == WS_EPI_SWIGLU_BWD) ? 2 * n : n;
+  const int64_t out_cols = has_out && (epilogue == WS_EPI_SWIGLU || epilogue == WS_EPI_SWIGLU_BWD) ? 2 * n : n;
   TORCH_CHECK(out.size(0) == m && out.size(1) == out_cols, "gemm: wrong out shape");
   if (row_scale.has_value() && row_scale->defined()) {
     TORCH_CHECK(row_scale->scalar_type() == at::kFloat && row_scale->numel() == m && row_scale->is_contiguous(),
@@ -83,7 +88,7 @@ void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_
   g.m = (int)m; g.n = (int)n; g.k = (int)k;
   g.lda = (int)a.stride(0); g.ldb = (int)b.stride(0);
   g.a_mn = a_mn; g.b_mn = b_mn; g.epilogue = (int)epilogue;
-  g.out = out.data_ptr(); g.ldo = (int)out.stride(0);
+  g.out = has_out ? out.data_ptr() : nullptr; g.ldo = has_out ? (int)out.stride(0) : 0;
   g.out2 = const_cast<void*>(opt_ptr(out2)); g.ldo2 = (int)opt_ld(out2);
   g.aux = opt_ptr(aux); g.ldaux = (int)opt_ld(aux);
   g.row_scale = reinterpret_cast<const float*>(opt_ptr(row_scale));
@@ -310,6 +315,39 @@ at::Tensor attn_fwd(const at::Tensor& qkvgu, const at::Tensor& states, const at:
   check_rc(ws_attn_fwd(qkvgu.data_ptr(), states.data_ptr(), rope.data_ptr<float>(), y.data_ptr(), (int)B, (int)T,
                        (int)H, (int)(H * 64), reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag))),
                        cur_stream()), "attn_fwd");
+  return y;
+}
+
+// Prompts of any length: y [B*T, d]; the decode state of the layer is written in place.
+at::Tensor attn_prefill(const at::Tensor& qkvgu, const at::Tensor& rope, const at::Tensor& fast_logit,
+                        const at::Tensor& slow_logit, const at::Tensor& mix_logit, int64_t B, int64_t T, int64_t H,
+                        at::Tensor fast, at::Tensor slow, at::Tensor mixed, at::Tensor kc, at::Tensor vc, at::Tensor uc,
+                        const c10::optional<at::Tensor>& error_flag) {
+  TORCH_CHECK(qkvgu.is_cuda() && qkvgu.scalar_type() == at::kBFloat16 && qkvgu.is_contiguous() && qkvgu.dim() == 2 &&
+              B >= 1 && T >= 1 && qkvgu.size(0) == B * T && qkvgu.size(1) == 5 * H * 64,
+              "attn_prefill: qkvgu must be contiguous BF16 [B*T, 5*H*64]");
+  TORCH_CHECK(rope.scalar_type() == at::kFloat && rope.is_contiguous() && rope.numel() == 128 * 64, "attn_prefill: rope table");
+  for (const at::Tensor* t : {&fast_logit, &slow_logit, &mix_logit})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == H, "attn_prefill: logits");
+  for (const at::Tensor* t : {&fast, &slow})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == B * H * 4096,
+                "attn_prefill: fast and slow must be contiguous FP32 [B, H, 64, 64]");
+  TORCH_CHECK(mixed.is_cuda() && mixed.scalar_type() == at::kBFloat16 && mixed.is_contiguous() && mixed.numel() == B * H * 4096,
+              "attn_prefill: mixed must be contiguous BF16 [B, H, 64, 64]");
+  for (const at::Tensor* t : {&kc, &vc, &uc})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->numel() == B * H * 128 * 64,
+                "attn_prefill: caches must be contiguous BF16 [B, H, 128, 64]");
+  c10::cuda::CUDAGuard guard(qkvgu.device());
+  const int64_t chunks = (T + 127) / 128;
+  at::Tensor writes = at::empty({B, chunks, H, 64, 64}, qkvgu.options().dtype(at::kFloat));
+  at::Tensor states = at::empty({B, chunks, H, 64, 64}, qkvgu.options());
+  at::Tensor y = at::empty({B * T, H * 64}, qkvgu.options());
+  check_rc(ws_attn_prefill(qkvgu.data_ptr(), rope.data_ptr<float>(), fast_logit.data_ptr<float>(),
+                           slow_logit.data_ptr<float>(), mix_logit.data_ptr<float>(), writes.data_ptr<float>(),
+                           states.data_ptr(), y.data_ptr(), fast.data_ptr<float>(), slow.data_ptr<float>(),
+                           mixed.data_ptr(), kc.data_ptr(), vc.data_ptr(), uc.data_ptr(), (int)B, (int)T, (int)H,
+                           (int)(H * 64), reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag))), cur_stream()),
+           "attn_prefill");
   return y;
 }
 
@@ -858,6 +896,9 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("memory_scan(Tensor writes, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, bool want_states, "
         "bool want_final, Tensor? init_fast, Tensor? init_slow) -> (Tensor, Tensor, Tensor)");
   m.def("attn_fwd(Tensor qkvgu, Tensor states, Tensor rope, int B, int T, int H, Tensor(a!)? error_flag) -> Tensor");
+  m.def("attn_prefill(Tensor qkvgu, Tensor rope, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, int B, int T, "
+        "int H, Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, "
+        "Tensor(g!)? error_flag) -> Tensor");
   m.def("grad_norm_clip(Tensor g, float max_norm, Tensor? extra_sumsq, Tensor? status=None) -> Tensor");
   m.def("clip_from_partials(Tensor partial, float max_norm, Tensor? extra_sumsq=None, Tensor? status=None) -> Tensor");
   m.def("grad_reduce_segments(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int[] starts, "
@@ -872,7 +913,7 @@ TORCH_LIBRARY(ws_b200, m) {
         "float beta2, float eps, float wd, int step, Tensor? grad_scale, float grad_scale_const, "
         "Tensor? skip=None) -> ()");
   m.def("gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, int epilogue, int m, int n, int k, "
-        "Tensor(a!) out, Tensor(b!)? out2, Tensor? aux, Tensor? row_scale, float alpha, float beta, "
+        "Tensor(a!)? out, Tensor(b!)? out2, Tensor? aux, Tensor? row_scale, float alpha, float beta, "
         "Tensor(c!)? error_flag) -> ()");
   m.def("grad_weight_group(Tensor[] dys, Tensor[] xs, Tensor(a!)[] grads, float[] betas, Tensor(b!)? error_flag) -> ()");
 }
@@ -908,6 +949,7 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("chunk_writes", &chunk_writes);
   m.impl("memory_scan", &memory_scan);
   m.impl("attn_fwd", &attn_fwd);
+  m.impl("attn_prefill", &attn_prefill);
   m.impl("adamw_step", &adamw_step);
   m.impl("lm_head_fwd", &lm_head_fwd);
   m.impl("lm_head_dlogits", &lm_head_dlogits);

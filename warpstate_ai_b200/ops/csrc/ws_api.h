@@ -146,6 +146,14 @@ int ws_memory_scan(const float* writes, const float* fast_logit, const float* sl
                    const float* mix_logit, void* states, float* final_fast, float* final_slow,
                    const float* init_fast, const float* init_slow, int B, int N, int H,
                    cudaStream_t stream);
+// Forward of the block over prompts of any length T >= 1 (four launches), leaving what a decode continues from:
+// fast / slow (FP32) and mixed (BF16) [B, H, 64, 64] after the T / 128 complete chunks; kc / vc / uc (BF16
+// [B, H, 128, 64]) hold roped K, V and U of the open chunk's T % 128 positions and zeros behind them.
+// Scratch: writes FP32 and states BF16, [B, ceil(T / 128), H, 64, 64].  y: BF16 [B*T, d].  rope: pair-major.
+int ws_attn_prefill(const void* qkvgu, const float* rope, const float* fast_logit, const float* slow_logit,
+                    const float* mix_logit, float* writes, void* states, void* y, float* fast, float* slow,
+                    void* mixed, void* kc, void* vc, void* uc, int B, int T, int H, int d, int* error_flag,
+                    cudaStream_t stream);
 // y: BF16 [B*T, d] token-major.
 int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H,
                 int d, int* error_flag, cudaStream_t stream);

@@ -477,24 +477,39 @@ def lm_head_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tenso
 @torch.no_grad()
 def core_prefill(core, x: torch.Tensor, depth_scale, depth_bias):
     """Forward of one core over whole chunks that also returns the fast / slow memory states
-    after the last chunk (FP32 ``[B,H,64,64]``): the chunked prefill of the decode engine."""
-    from . import attention
-    ops = _ops()
+    after the last chunk (FP32 ``[B,H,64,64]``), for cores whose geometry the attention kernels do not take."""
     batch, seq, d = x.shape
-    x_in = x.reshape(batch * seq, d).contiguous()
-    scale = depth_scale.detach().float().contiguous()
-    bias = depth_bias.detach().float().contiguous()
-    z1, _, xmod = ops.rmsnorm_fwd(x_in, scale, bias, core.norm1.weight.detach().float(), core.cfg.rms_eps, True)
+    z1, xmod = _prefill_norm(core, x.reshape(batch * seq, d), depth_scale, depth_bias)
     qkvgu = G.linear(z1, bf16_weight(core.in_proj.weight))
-    if attention.geometry_ok(core):
-        y, _, _, (fast, slow) = attention.forward_only(qkvgu, core, batch, seq, want_final=True)
-    else:
-        y, (fast, slow) = R.attention_memory(qkvgu.view(batch, seq, -1), core.fast_decay_logit, core.slow_decay_logit,
-                                             core.memory_mix_logit, core.h, core.chunk, core.cfg.parallel_memory,
-                                             core.rope_cos, core.rope_sin, return_state=True)
-        y = y.reshape(batch * seq, -1).contiguous()
+    y, (fast, slow) = R.attention_memory(qkvgu.view(batch, seq, -1), core.fast_decay_logit, core.slow_decay_logit,
+                                         core.memory_mix_logit, core.h, core.chunk, core.cfg.parallel_memory,
+                                         core.rope_cos, core.rope_sin, return_state=True)
+    return _prefill_finish(core, y.reshape(batch * seq, -1).contiguous(), xmod).view(batch, seq, d), fast, slow
+
+
+@torch.no_grad()
+def core_prefill_state(core, x: torch.Tensor, depth_scale, depth_bias, batch: int, seq: int, state, last: bool):
+    """Forward of one core over prompts of any length ``x [B*T, d]``; ``state`` receives what a decode continues from.
+    Returns the rows ``[B*T, d]``, or with ``last`` (nothing reads the other positions of the last block) the block's
+    residual input and its attention output at the final position of every sequence, ``[B, d]`` each."""
+    from . import attention
+    z1, xmod = _prefill_norm(core, x, depth_scale, depth_bias)
+    y = attention.prefill(G.linear(z1, bf16_weight(core.in_proj.weight)), core, batch, seq, state)
+    if last:
+        return tuple(t.view(batch, seq, -1)[:, -1].contiguous() for t in (xmod, y))
+    return _prefill_finish(core, y, xmod)
+
+
+def _prefill_norm(core, x, depth_scale, depth_bias):
+    z1, _, xmod = _ops().rmsnorm_fwd(x.contiguous(), depth_scale.detach().float().contiguous(),
+                                     depth_bias.detach().float().contiguous(), core.norm1.weight.detach().float(),
+                                     core.cfg.rms_eps, True)
+    return z1, xmod
+
+
+def _prefill_finish(core, y, xmod):
+    """The block after its attention, on rows ``[M, d]``; no backward pass follows, so (up | gate) is not written."""
     x2 = G.linear_residual(y, bf16_weight(core.out_proj.weight), xmod)
-    z2, _, _ = ops.rmsnorm_fwd(x2, None, None, core.norm2.weight.detach().float(), core.cfg.rms_eps, False)
-    _, act = G.linear_swiglu(z2, bf16_weight(core.ffn.up_gate.weight))
-    x3 = G.linear_residual(act, bf16_weight(core.ffn.down.weight), x2)
-    return x3.view(batch, seq, d), fast, slow
+    z2, _, _ = _ops().rmsnorm_fwd(x2, None, None, core.norm2.weight.detach().float(), core.cfg.rms_eps, False)
+    _, act = G.linear_swiglu(z2, bf16_weight(core.ffn.up_gate.weight), want_packed=False)
+    return G.linear_residual(act, bf16_weight(core.ffn.down.weight), x2)

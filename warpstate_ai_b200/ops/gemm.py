@@ -118,11 +118,12 @@ def linear_swiglu(x: torch.Tensor, w_up_gate: torch.Tensor, row_scale: torch.Ten
     """Up/gate projection with the SwiGLU epilogue.
 
     ``w_up_gate`` is ``[2h, K]`` with the first ``h`` rows = up, last ``h`` rows = gate (the
-    reference layout, warpstate/model.py:58-60).  Returns ``(packed [M,2h], act [M,h])``.
+    reference layout, warpstate/model.py:58-60).  Returns ``(packed [M,2h], act [M,h])``; ``packed`` is None with
+    ``want_packed=False`` (only a backward pass reads it).
     """
     m, k = x.shape
     h = w_up_gate.shape[0] // 2
-    packed = torch.empty((m, 2 * h), dtype=torch.bfloat16, device=x.device)
+    packed = torch.empty((m, 2 * h), dtype=torch.bfloat16, device=x.device) if want_packed else None
     act = torch.empty((m, h), dtype=torch.bfloat16, device=x.device)
     _gemm(x, w_up_gate, False, False, EPI_SWIGLU, m, h, k, packed, out2=act, row_scale=row_scale)
     return packed, act

@@ -9,9 +9,11 @@ of fast/slow is applied before the read and a chunk's write is formed as ONE pro
 
 What is new relative to the reference (whose CLIs prefill token by token at batch 1):
 
-* `prefill` pushes all complete chunks of the prompt through the training forward path (the fused
-  sm_100a kernels on CUDA) and reads the memory states after the last complete chunk from the
-  O(N) scan kernel; only the tokens of a trailing partial chunk are stepped one by one;
+* `prefill` pushes the whole prompt, whatever its length, through the training forward path in one pass (the
+  fused sm_100a kernels on CUDA): the O(N) scan kernel leaves the memory states after the last complete
+  chunk, a small kernel the keys, values and memory-values of the chunk the prompt ends in, and the last
+  block is finished for the final position only.  Where those kernels do not apply, the complete chunks
+  take one pass and the tokens of a trailing partial chunk are stepped one by one;
 * `step` handles a whole batch in lock-step; on CUDA the step for a fixed batch size is captured
   once in a CUDA graph and replayed per token (the in-chunk position is a device scalar, the
   attention over the chunk cache is masked instead of sliced, so one graph serves all positions);
@@ -88,18 +90,23 @@ class DecodeEngine:
 
     # ------------------------------------------------------------------ state
     def new_state(self, batch: int) -> None:
+        if self._reuse_state(batch):
+            # same shapes: clear in place so that the captured graph and its buffers stay valid
+            for st in self.states:
+                for t in (st.fast, st.slow, st.mixed, st.k, st.v, st.u):
+                    t.zero_()
+
+    def _reuse_state(self, batch: int) -> bool:
+        """Position 0 of ``batch`` sequences.  True: the buffers of the previous sequences stay, with their contents;
+        False: new ones were made (zeros)."""
         # Buffers made under ``torch.inference_mode()`` (as the chat entry points run) cannot be written from outside
         # it; a caller that then uses the engine directly gets fresh ones (and a fresh graph) instead of an error.
         stranded = (self.states is not None and self.states[0].fast.is_inference()
                     and not torch.is_inference_mode_enabled())
         if self.states is not None and batch == self.batch and not stranded:
-            # same shapes: clear in place so that the captured graph and its buffers stay valid
-            for st in self.states:
-                for t in (st.fast, st.slow, st.mixed, st.k, st.v, st.u):
-                    t.zero_()
             self.pos = 0
             self.pos_dev.zero_()
-            return
+            return True
         z = lambda *shape, dtype: torch.zeros(shape, device=self.device, dtype=dtype)
         self.states = [DepthState(z(batch, self.h, self.hd, self.hd, dtype=torch.float32),
                                   z(batch, self.h, self.hd, self.hd, dtype=torch.float32),
@@ -120,6 +127,7 @@ class DecodeEngine:
         # greedy run-ahead decode: chosen tokens land in `history[:, cursor[0]]`; cursor[1] is kernel scratch
         self.history = torch.zeros(batch, self.GREEDY_CAPACITY, dtype=torch.long, device=self.device)
         self.cursor = torch.zeros(2, dtype=torch.long, device=self.device)
+        return False
 
     # ------------------------------------------------------------------ kernel path
     def _kernels_usable(self, batch: int) -> bool:
@@ -384,24 +392,65 @@ class DecodeEngine:
         last token ``[B, V]``."""
         ids = ids.to(self.device)
         b, t = ids.shape
+        fused_path = self._fused_prefill()
+        if fused_path and t > 0 and self._whole_prompt_kernels():
+            return self._prefill_whole(ids)
         self.new_state(b)
         full = (t // self.chunk) * self.chunk
         logits = None
         if full:
-            hidden = self._prefill_chunks(ids[:, :full])
+            hidden = self._prefill_chunks(ids[:, :full], fused_path)
             if full == t:
                 logits = F.linear(self._norm(hidden[:, -1], self.final_norm), self.head).float()
         for i in range(full, t):
             logits = self.step(ids[:, i])
         return logits
 
-    def _prefill_chunks(self, ids: torch.Tensor) -> torch.Tensor:
+    def _fused_prefill(self) -> bool:
+        if self.device.type != "cuda" or self.dtype != torch.bfloat16:
+            return False
+        from ..ops import fused
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return fused.active(self.embed)
+
+    def _whole_prompt_kernels(self) -> bool:
+        from ..ops import attention
+        return all(attention.geometry_ok(core) for core in self.model.cores)
+
+    def _prefill_whole(self, ids: torch.Tensor) -> torch.Tensor:
+        """The prompt in one pass: every layer's state is overwritten by its kernels, so nothing is cleared first."""
+        from ..ops import fused
+        model, (b, t) = self.model, ids.shape
+        self._reuse_state(b)
+        x = self.embed[ids].float().view(b * t, -1)
+        for depth, st in enumerate(self.states):
+            last = depth + 1 == len(self.states)
+            core = model.cores[depth % self.cfg.n_cores]
+            x = fused.core_prefill_state(core, x, model.depth_scale[depth], model.depth_bias[depth], b, t, st, last)
+        self.pos = t % self.chunk
+        return self._prefill_logits(core, *x)
+
+    def _prefill_logits(self, core, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+        """Logits from the last block's residual input ``x [B, d]`` (FP32) and attention output ``y [B, d]``: the rows
+        of one decode step, so they take its weight-streaming kernels where those apply."""
+        from ..ops import fused
+        if self._kbufs is None:
+            return F.linear(self._norm(fused._prefill_finish(core, y, x), self.final_norm), self.head).float()
+        ops, k, eps = torch.ops.ws_b200, self._kbufs, self.cfg.rms_eps
+        d, ffn = self.cfg.d_model, self.cfg.ffn_hidden
+        out, up_gate, down = (fused.bf16_weight(w) for w in (core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight))
+        ops.decode_gemm(out, y, d, 1, k["p_out"], k["flag"], False)
+        ops.decode_reduce_norm(x, k["p_out"], None, None, None, None, core.norm2.weight.detach().float(), eps, k["n"])
+        ops.decode_gemm(up_gate, k["n"], ffn, 2, k["act"], k["flag"], False)
+        ops.decode_gemm(down, k["act"], d, 1, k["p_down"], k["flag"], False)
+        ops.decode_reduce_norm(x, k["p_down"], None, None, None, None, self.final_norm, eps, k["n"])
+        logits = torch.empty(x.shape[0], self.cfg.vocab_size, device=self.device)
+        ops.decode_gemm(self.head, k["n"], self.cfg.vocab_size, 3, logits, k["flag"], False)
+        return logits
+
+    def _prefill_chunks(self, ids: torch.Tensor, use_fused: bool) -> torch.Tensor:
+        """Complete chunks where the whole-prompt kernels do not apply (CPU, FP32, other geometries)."""
         model = self.model
-        use_fused = False
-        if self.device.type == "cuda" and self.dtype == torch.bfloat16:
-            from ..ops import fused
-            with torch.autocast("cuda", dtype=torch.bfloat16):
-                use_fused = fused.active(self.embed)
         x = self.embed[ids].float()
         for depth, (w, st) in enumerate(zip(self.weights, self.states)):
             core = model.cores[depth % self.cfg.n_cores]
