@@ -1,0 +1,65 @@
+"""The LM head over the labelled rows only: selections at the edges of tiles, k-blocks and row blocks, against the FP32
+head; unlabelled rows must not reach the loss or a gradient, whatever they hold."""
+import pytest
+import torch
+
+from warpstate_ai_b200.ops import _ext, lmhead
+from warpstate_ai_b200.ops import reference as R
+from warpstate_ai_b200.ops.gemm import check_device_errors
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-9))
+
+
+def labels_with(kind, rows, vocab):
+    labels = torch.randint(0, vocab, (rows,), device="cuda")
+    keep = torch.zeros(rows, dtype=torch.bool, device="cuda")
+    if kind == "span":
+        keep[rows // 8:rows // 2 + 3] = True
+    elif kind == "random":
+        keep = torch.rand(rows, device="cuda") < 0.3
+    else:                                   # a count: that many rows, spread over the batch
+        keep[torch.randperm(rows, device="cuda")[:kind]] = True
+    labels[~keep] = -100
+    return labels, keep
+
+
+@pytest.mark.parametrize("rows,d,vocab,kind", [
+    (512, 256, 1000, 0), (512, 256, 1000, 1), (600, 256, 1000, 64), (600, 256, 1000, 65), (777, 256, 1000, 255),
+    (777, 256, 1000, 256), (777, 256, 1000, 257), (777, 256, 1000, 776), (777, 256, 1000, 777), (2048, 512, 32768, "span"),
+    (17000, 128, 520, "random"), (17000, 128, 520, 8192), (17000, 128, 520, 8193), (17000, 128, 520, 16500),
+    (17000, 128, 520, 17000)])
+def test_head_over_labelled_rows(rows, d, vocab, kind):
+    # BF16 logits and logit gradients (2^-9 each, independent per element) against FP32 ones: as in the dense test
+    _ext.require()
+    torch.manual_seed(rows + vocab)
+    hidden = torch.randn(rows, d, device="cuda").bfloat16()
+    labels, keep = labels_with(kind, rows, vocab)
+    hidden[~keep] = float("nan")
+    hidden.requires_grad_(True)
+    weight = (torch.randn(vocab, d, device="cuda") * 0.05).requires_grad_(True)
+    coef = torch.randn(rows, device="cuda")
+    assert rows >= lmhead.SELECT_FROM and lmhead.kernels_ready(hidden, weight)
+    logp = lmhead.token_logps(hidden, weight, labels)
+    (logp * coef).sum().backward()
+    check_device_errors()
+    h32 = hidden.detach()[keep].float().requires_grad_(True)
+    w32 = weight.detach().bfloat16().float().requires_grad_(True)
+    want = R.lm_head_token_logps(h32, w32, labels[keep])
+    (want * coef[keep]).sum().backward()
+    assert torch.count_nonzero(logp[~keep]) == 0 and torch.count_nonzero(hidden.grad[~keep]) == 0
+    assert torch.isfinite(hidden.grad).all() and torch.isfinite(weight.grad).all()
+    if keep.any():
+        assert rel(logp[keep], want) < 5e-3
+        assert rel(hidden.grad[keep], h32.grad) < 0.02
+        assert rel(weight.grad, w32.grad) < 0.02
+    else:
+        assert torch.count_nonzero(weight.grad) == 0
+    # a second pass accumulates into the tied gradient and changes nothing else
+    first = hidden.grad.clone()
+    hidden.grad = None
+    (lmhead.token_logps(hidden, weight, labels) * coef).sum().backward()
+    assert torch.equal(hidden.grad, first) and rel(weight.grad, 2 * w32.grad if keep.any() else weight.grad) < 0.02

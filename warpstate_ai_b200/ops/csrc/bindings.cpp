@@ -6,6 +6,7 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -83,7 +84,7 @@ void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_
   }
 
   c10::cuda::CUDAGuard guard(a.device());
-  WsGemm g;
+  WsGemm g = {};
   g.a = a.data_ptr(); g.b = b.data_ptr();
   g.m = (int)m; g.n = (int)n; g.k = (int)k;
   g.lda = (int)a.stride(0); g.ldb = (int)b.stride(0);
@@ -460,7 +461,7 @@ std::tuple<at::Tensor, at::Tensor> lm_head_fwd(const at::Tensor& hidden, const a
   const int ld = 2 * ((vocab + 255) / 256);
   at::Tensor parts = at::empty({rows, ld, 2}, hidden.options().dtype(at::kFloat));
   at::Tensor label_logit = at::zeros({rows}, hidden.options().dtype(at::kFloat));
-  WsGemm g;
+  WsGemm g = {};
   g.a = hidden.data_ptr(); g.b = weight.data_ptr();
   g.m = rows; g.n = vocab; g.k = d;
   g.lda = (int)hidden.stride(0); g.ldb = (int)weight.stride(0);
@@ -475,9 +476,135 @@ std::tuple<at::Tensor, at::Tensor> lm_head_fwd(const at::Tensor& hidden, const a
   at::Tensor logp = at::empty({rows}, hidden.options().dtype(at::kFloat));
   check_rc(ws_ce_combine(parts.data_ptr(), ld, nparts, label_logit.data_ptr<float>(),
                          reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), (long long)ignore_index, rows,
-                         lse.data_ptr<float>(), logp.data_ptr<float>(), cur_stream()), "ce_combine");
+                         nullptr, nullptr, lse.data_ptr<float>(), logp.data_ptr<float>(), cur_stream()), "ce_combine");
   return {lse, logp};
 }
+
+// The same over the labelled rows only, which are packed together on the device (see lmhead.cu).  Returns
+// (logp [rows], lse of the packed rows, index, count, hidden packed, labels packed); what backward needs of them goes
+// to lm_head_bwd_labelled.
+std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> lm_head_fwd_labelled(
+    const at::Tensor& hidden, const at::Tensor& weight, const at::Tensor& labels, int64_t ignore_index,
+    const c10::optional<at::Tensor>& error_flag) {
+  TORCH_CHECK(hidden.is_cuda() && hidden.scalar_type() == at::kBFloat16 && hidden.dim() == 2 && hidden.is_contiguous() &&
+              hidden.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(hidden.data_ptr()) % 16 == 0,
+              "lm_head_fwd_labelled: hidden must be contiguous BF16 [rows, d], d % 8 == 0");
+  TORCH_CHECK(weight.scalar_type() == at::kBFloat16 && weight.dim() == 2 && weight.is_contiguous() &&
+              weight.size(1) == hidden.size(1), "lm_head_fwd_labelled: weight must be BF16 [vocab, d]");
+  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == hidden.size(0),
+              "lm_head_fwd_labelled: labels must be int64 [rows]");
+  c10::cuda::CUDAGuard guard(hidden.device());
+  const int rows = (int)hidden.size(0), d = (int)hidden.size(1), vocab = (int)weight.size(0);
+  const int ld = 2 * ((vocab + 255) / 256);
+  const int nparts = ld - (((vocab % 256) != 0 && (vocab % 256) <= 128) ? 1 : 0);
+  const auto f32 = hidden.options().dtype(at::kFloat);
+  at::Tensor index = at::empty({rows}, hidden.options().dtype(at::kInt));
+  at::Tensor count = at::empty({1}, hidden.options().dtype(at::kInt));
+  at::Tensor labels_sel = at::empty({rows}, labels.options());
+  at::Tensor packed = at::empty_like(hidden);
+  at::Tensor logp = at::empty({rows}, f32);
+  at::Tensor parts = at::empty({rows, ld, 2}, f32);
+  at::Tensor per_row = at::zeros({2, rows}, f32);   // label logits, log-sum-exps (0 in the padding rows)
+  float* label_logit = per_row.data_ptr<float>();
+  at::Tensor lse = per_row.select(0, 1);
+  const long long* lab = reinterpret_cast<const long long*>(labels_sel.data_ptr<int64_t>());
+  check_rc(ws_select_rows(reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), (long long)ignore_index, rows,
+                          index.data_ptr<int>(), count.data_ptr<int>(),
+                          reinterpret_cast<long long*>(labels_sel.data_ptr<int64_t>()), logp.data_ptr<float>(),
+                          cur_stream()), "select_rows");
+  check_rc(ws_gather_rows(hidden.data_ptr(), d, index.data_ptr<int>(), count.data_ptr<int>(), rows, d, packed.data_ptr(),
+                          cur_stream()), "gather_rows");
+  WsGemm g = {};
+  g.a = packed.data_ptr(); g.b = weight.data_ptr();
+  g.m = rows; g.n = vocab; g.k = d;
+  g.lda = d; g.ldb = d;
+  g.epilogue = WS_EPI_CE_FWD;
+  g.out = parts.data_ptr(); g.ldo = ld;
+  g.out2 = label_logit;
+  g.aux = lab;
+  g.alpha = 1.f;
+  g.error_flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
+  g.limit = count.data_ptr<int>();
+  g.whole = hidden.data_ptr(); g.whole_rows = rows; g.ldwhole = d;
+  check_rc(ws_gemm(&g, cur_stream()), "lm_head_fwd_labelled gemm");
+  check_rc(ws_ce_combine(parts.data_ptr(), ld, nparts, label_logit, lab, (long long)ignore_index, rows,
+                         index.data_ptr<int>(), count.data_ptr<int>(), lse.data_ptr<float>(), logp.data_ptr<float>(),
+                         cur_stream()), "ce_combine");
+  return {logp, lse, index, count, packed, labels_sel};
+}
+
+// dhidden [rows, d] (every row written) and grad_weight [vocab, d] += of sum(row_weight * -logp), the rows in blocks of
+// `block`: logits recomputed into dlogits, then the two products.  row_weight is per row before the selection.
+void lm_head_bwd_labelled(const at::Tensor& hidden, const at::Tensor& packed, const at::Tensor& weight,
+                          const at::Tensor& labels, const at::Tensor& labels_sel, const at::Tensor& index,
+                          const at::Tensor& count, const at::Tensor& lse, const at::Tensor& row_weight,
+                          int64_t ignore_index, int64_t block, at::Tensor dhidden, at::Tensor grad_weight,
+                          const c10::optional<at::Tensor>& error_flag) {
+  const int rows = (int)hidden.size(0), d = (int)hidden.size(1), vocab = (int)weight.size(0);
+  TORCH_CHECK(hidden.is_cuda() && hidden.scalar_type() == at::kBFloat16 && hidden.is_contiguous() &&
+              packed.scalar_type() == at::kBFloat16 && packed.is_contiguous() && packed.sizes() == hidden.sizes() &&
+              weight.scalar_type() == at::kBFloat16 && weight.is_contiguous() && weight.size(1) == d && vocab % 8 == 0,
+              "lm_head_bwd_labelled: operands");
+  TORCH_CHECK(labels.scalar_type() == at::kLong && labels.is_contiguous() && labels.numel() == rows &&
+              labels_sel.scalar_type() == at::kLong && labels_sel.is_contiguous() && labels_sel.numel() == rows &&
+              index.scalar_type() == at::kInt && index.is_contiguous() && index.numel() == rows &&
+              count.scalar_type() == at::kInt && count.numel() == 1 && lse.scalar_type() == at::kFloat &&
+              lse.is_contiguous() && lse.numel() == rows && row_weight.scalar_type() == at::kFloat &&
+              row_weight.is_contiguous() && row_weight.numel() == rows, "lm_head_bwd_labelled: per-row vectors");
+  TORCH_CHECK(dhidden.scalar_type() == at::kBFloat16 && dhidden.is_contiguous() && dhidden.sizes() == hidden.sizes() &&
+              grad_weight.scalar_type() == at::kFloat && grad_weight.dim() == 2 && grad_weight.stride(1) == 1 &&
+              grad_weight.size(0) == vocab && grad_weight.size(1) == d && block > 0 && block % 256 == 0,
+              "lm_head_bwd_labelled: outputs");
+  c10::cuda::CUDAGuard guard(hidden.device());
+  check_rc(ws_clear_unlabelled(reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), (long long)ignore_index,
+                               rows, d, dhidden.data_ptr(), cur_stream()), "clear_unlabelled");
+  at::Tensor dlogits = at::empty({std::min<int64_t>(block, rows), vocab}, hidden.options());
+  int* flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
+  for (int start = 0; start < rows; start += (int)block) {
+    const int here = std::min((int)block, rows - start);
+    const auto from_start = [&](const at::Tensor& t) { return t.data_ptr<at::BFloat16>() + static_cast<int64_t>(start) * d; };
+    WsGemm g = {};
+    g.a = from_start(packed); g.b = weight.data_ptr();
+    g.m = here; g.n = vocab; g.k = d;
+    g.lda = d; g.ldb = d;
+    g.epilogue = WS_EPI_CE_BWD;
+    g.out = dlogits.data_ptr(); g.ldo = vocab;
+    g.aux = labels_sel.data_ptr<int64_t>() + start;
+    g.row_scale = row_weight.data_ptr<float>(); g.row_vec = lse.data_ptr<float>() + start;
+    g.row_map = index.data_ptr<int>() + start;
+    g.alpha = 1.f;
+    g.error_flag = flag;
+    g.limit = count.data_ptr<int>(); g.limit_from = start;
+    g.whole = from_start(hidden); g.whole_rows = rows; g.ldwhole = d;
+    check_rc(ws_gemm(&g, cur_stream()), "lm_head_bwd_labelled dlogits");
+    WsGemm x = {};
+    x.a = dlogits.data_ptr(); x.b = weight.data_ptr();
+    x.m = here; x.n = d; x.k = vocab;
+    x.lda = vocab; x.ldb = d;
+    x.b_mn = 1;
+    x.epilogue = WS_EPI_BF16;
+    x.out = dhidden.data_ptr(); x.ldo = d;
+    x.row_map = index.data_ptr<int>() + start;
+    x.alpha = 1.f;
+    x.error_flag = flag;
+    x.limit = count.data_ptr<int>(); x.limit_from = start;
+    check_rc(ws_gemm(&x, cur_stream()), "lm_head_bwd_labelled dhidden");
+    WsGemm w = {};
+    w.a = dlogits.data_ptr(); w.b = from_start(packed);
+    w.m = vocab; w.n = d; w.k = here;
+    w.lda = vocab; w.ldb = d;
+    w.a_mn = 1; w.b_mn = 1;
+    w.epilogue = WS_EPI_ACC_F32;
+    w.out = grad_weight.data_ptr(); w.ldo = (int)grad_weight.stride(0);
+    w.alpha = 1.f; w.beta = 1.f;
+    w.error_flag = flag;
+    w.limit = count.data_ptr<int>(); w.limit_from = start;
+    w.whole = from_start(hidden); w.whole_rows = rows; w.ldwhole = d;
+    check_rc(ws_gemm(&w, cur_stream()), "lm_head_bwd_labelled dweight");
+  }
+}
+
+bool gemm_pair_available() { return ws_gemm_pair_available() != 0; }
 
 // dlogits [rows, vocab] BF16 = (softmax(hidden @ weight.T) - onehot(labels)) * row_weight
 at::Tensor lm_head_dlogits(const at::Tensor& hidden, const at::Tensor& weight, const at::Tensor& labels,
@@ -494,7 +621,7 @@ at::Tensor lm_head_dlogits(const at::Tensor& hidden, const at::Tensor& weight, c
               "lm_head_dlogits: per-row vectors");
   c10::cuda::CUDAGuard guard(hidden.device());
   at::Tensor out = at::empty({rows, vocab}, hidden.options());
-  WsGemm g;
+  WsGemm g = {};
   g.a = hidden.data_ptr(); g.b = weight.data_ptr();
   g.m = rows; g.n = vocab; g.k = d;
   g.lda = (int)hidden.stride(0); g.ldb = (int)weight.stride(0);
@@ -882,6 +1009,12 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("embed_bwd(Tensor dx, Tensor ids, Tensor(a!) grad_table) -> ()");
   m.def("launch_count() -> int");
   m.def("lm_head_fwd(Tensor hidden, Tensor weight, Tensor labels, int ignore_index, Tensor(a!)? error_flag) -> (Tensor, Tensor)");
+  m.def("lm_head_fwd_labelled(Tensor hidden, Tensor weight, Tensor labels, int ignore_index, Tensor(a!)? error_flag) -> "
+        "(Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
+  m.def("lm_head_bwd_labelled(Tensor hidden, Tensor packed, Tensor weight, Tensor labels, Tensor labels_sel, Tensor index, "
+        "Tensor count, Tensor lse, Tensor row_weight, int ignore_index, int block, Tensor(a!) dhidden, "
+        "Tensor(b!) grad_weight, Tensor(c!)? error_flag) -> ()");
+  m.def("gemm_pair_available() -> bool");
   m.def("lm_head_dlogits(Tensor hidden, Tensor weight, Tensor labels, Tensor lse, Tensor row_weight, Tensor(a!)? error_flag) -> Tensor");
   m.def("grad_allreduce(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int start, int count, "
         "int bucket, int seq, float scale, bool push, int ctas, Tensor(a!)? sumsq_out, Tensor(b!) status, "
@@ -919,6 +1052,7 @@ TORCH_LIBRARY(ws_b200, m) {
 }
 
 TORCH_LIBRARY_IMPL(ws_b200, CompositeExplicitAutograd, m) {
+  m.impl("gemm_pair_available", &gemm_pair_available);
   m.impl("launch_count", &launch_count);
   m.impl("decode_gemm_splits", &decode_gemm_splits);
   m.impl("raise_for_status", &raise_for_status);
@@ -953,6 +1087,8 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("adamw_step", &adamw_step);
   m.impl("lm_head_fwd", &lm_head_fwd);
   m.impl("lm_head_dlogits", &lm_head_dlogits);
+  m.impl("lm_head_fwd_labelled", &lm_head_fwd_labelled);
+  m.impl("lm_head_bwd_labelled", &lm_head_bwd_labelled);
   m.impl("grad_allreduce", &grad_allreduce);
   m.impl("wait_probe", &wait_probe);
   m.impl("adamw_shard_push", &adamw_shard_push);

@@ -91,6 +91,7 @@ struct alignas(64) PairGroup {
   GemmParams p[MAX_GROUP];
   CUtensorMap epi[4];  // staged epilogue of problem 0, 32 x 32 boxes.  SwiGLU backward: aux up, aux gate,
                        // out up, out gate; SwiGLU forward: packed up, packed gate, activation
+  CUtensorMap whole;   // row selection (problem 0): the operand before its rows were selected
   int tile_start[MAX_GROUP + 1];
   int count;
 };
@@ -124,12 +125,31 @@ __device__ __forceinline__ uint8_t* tile_chunk128(uint8_t* tile, int r, int j) {
 struct PairTile {
   int prob, mb, nb, num_k;
 };
-__device__ __forceinline__ PairTile resolve_tile(const PairGroup& g, int tile, int n_tile, bool n_major = false) {
+// `rows`, `depth`: m and k of problem 0 as far as they are computed (row selection), those of the others are their own.
+struct PairExtent {
+  int rows, depth, tiles;
+  bool whole;
+};
+template <bool A_MN>
+__device__ __forceinline__ PairExtent pair_extent(const PairGroup& g, int n_tile) {
+  const GemmParams& p = g.p[0];
+  PairExtent e{p.m, p.k, g.tile_start[g.count], false};
+  if (p.limit != nullptr) {
+    const int selected = *p.limit;
+    e.whole = selected == p.whole_rows;
+    const int here = min(max(selected - p.limit_from, 0), A_MN ? p.k : p.m);
+    if (A_MN) e.depth = here; else e.rows = here;
+    e.tiles = here == 0 ? 0 : ((e.rows + 2 * pair::BM - 1) / (2 * pair::BM)) * ((p.n + n_tile - 1) / n_tile);
+  }
+  return e;
+}
+__device__ __forceinline__ PairTile resolve_tile(const PairGroup& g, const PairExtent& e, int tile, int n_tile,
+                                                 bool n_major = false) {
   PairTile t;
   t.prob = 0;
   while (t.prob + 1 < g.count && tile >= g.tile_start[t.prob + 1]) ++t.prob;
   const GemmParams& p = g.p[t.prob];
-  const int num_m = (p.m + 2 * pair::BM - 1) / (2 * pair::BM);
+  const int num_m = ((t.prob == 0 ? e.rows : p.m) + 2 * pair::BM - 1) / (2 * pair::BM);
   const int num_n = (p.n + n_tile - 1) / n_tile;
   if (n_major) {  // every M tile of one N block before the next block (weight-gather variant)
     const int local = tile - g.tile_start[t.prob];
@@ -138,7 +158,7 @@ __device__ __forceinline__ PairTile resolve_tile(const PairGroup& g, int tile, i
   } else {
     pair_tile_coords(tile - g.tile_start[t.prob], num_m, num_n, t.mb, t.nb);
   }
-  t.num_k = (p.k + pair::BK - 1) / pair::BK;
+  t.num_k = ((t.prob == 0 ? e.depth : p.k) + pair::BK - 1) / pair::BK;
   return t;
 }
 
@@ -211,7 +231,8 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
 
   constexpr bool kSwiglu = (EPI == WS_EPI_SWIGLU);
   const int n_tile = kSwiglu ? 128 : BN;
-  const int tiles = g.tile_start[g.count];
+  const PairExtent extent = pair_extent<A_MN>(g, n_tile);
+  const int tiles = extent.tiles;
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
 
@@ -222,10 +243,10 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       bool ok = true;
       [[maybe_unused]] int ready_nb = -1;
       for (int tile = pair_id; tile < tiles && ok; tile += num_pairs) {
-        const PairTile t = resolve_tile(g, tile, n_tile, GATHER);
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const GemmParams& p = g.p[t.prob];
-        const CUtensorMap* tma_a = &g.a[t.prob];
-        const CUtensorMap* tma_b = &g.b[t.prob];
+        const CUtensorMap* tma_a = !A_MN && extent.whole ? &g.whole : &g.a[t.prob];
+        const CUtensorMap* tma_b = A_MN && extent.whole ? &g.whole : &g.b[t.prob];
         const int nb = t.nb;
         const int m0 = t.mb * 2 * BM + rank * BM;  // this CTA's rows
         if constexpr (GATHER) {
@@ -301,7 +322,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         if (!mbar_wait(&tempty[buf], tph ^ 1, abort_flag)) break;
         tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + buf * BN;
-        const int num_k = resolve_tile(g, tile, n_tile, GATHER).num_k;
+        const int num_k = resolve_tile(g, extent, tile, n_tile, GATHER).num_k;
         for (int kb = 0; kb < num_k; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -340,7 +361,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       constexpr int STEPS = (128 / GROUPS) / 32;
       const GemmParams& p = g.p[0];
       for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
-        const PairTile t = resolve_tile(g, tile, n_tile, GATHER);
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const int buf_t = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
         if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
@@ -400,7 +421,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       constexpr int STEPS = (BN / GROUPS) / 32;
       const GemmParams& p = g.p[0];
       auto coords = [&](int tile, int step, int& x, int& y) {
-        const PairTile t = resolve_tile(g, tile, n_tile, GATHER);
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
         y = t.mb * 2 * BM + rank * BM + quarter * 32;
       };
@@ -471,7 +492,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       constexpr int STEPS = (BN / GROUPS) / 32;
       const GemmParams& p = g.p[0];
       auto coords = [&](int tile, int step, int& x, int& y) {
-        const PairTile t = resolve_tile(g, tile, n_tile, GATHER);
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
         y = t.mb * 2 * BM + rank * BM + quarter * 32;
       };
@@ -556,7 +577,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       if (lane == 0) tma_store_wait_all();
     } else {
       for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
-        const PairTile t = resolve_tile(g, tile, n_tile, GATHER);
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const GemmParams& p = g.p[t.prob];
         const int nb = t.nb;
         const int buf = tcount & 1;
@@ -564,10 +585,15 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         if (!mbar_wait(&tfull[buf], tph, abort_flag)) break;
         tc_fence_after_sync();
         const int row = t.mb * 2 * BM + rank * BM + quarter * 32 + lane;
-        const bool row_ok = row < p.m;
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
-        const float rs = (p.row_scale != nullptr && row_ok) ? p.row_scale[row] : 1.0f;
-        gemm_epilogue<EPI, GROUPS>(p, taddr, row, row_ok, rs, nb, egroup);
+        const bool inside = row < p.m;
+        const int place = p.row_map != nullptr && inside ? p.row_map[row] : row;  // the row before the selection
+        float rs = 1.0f;
+        if (p.row_scale != nullptr && inside) rs = place >= 0 ? p.row_scale[place] : 0.f;
+        if constexpr (EPI == WS_EPI_BF16)
+          gemm_epilogue<EPI, GROUPS>(p, taddr, place, inside && place >= 0, rs, nb, egroup);
+        else
+          gemm_epilogue<EPI, GROUPS>(p, taddr, row, inside, rs, nb, egroup);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf]), 0));
@@ -700,7 +726,16 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
   p.row_vec = g->row_vec;
   p.alpha = g->alpha; p.beta = g->beta;
   p.error_flag = g->error_flag;
+  p.limit = g->limit; p.limit_from = g->limit_from;
+  p.row_map = g->row_map;
+  p.whole_rows = g->whole != nullptr ? g->whole_rows : -1;
   p.debug = 0;
+  if (g->whole != nullptr) {  // the same boxes over the rows before their selection: A, or B of a weight gradient
+    if (i != 0) return -9;
+    rc = !g->a_mn ? make_map_bf16(&grp.whole, g->whole, g->k, g->m, g->ldwhole, pair::BK, pair::BM)
+                  : make_map_bf16(&grp.whole, g->whole, b_rows, g->k, g->ldwhole, 64, pair::BK);
+    if (rc) return rc;
+  }
   const int n_tile = swiglu ? 128 : pair::BN;
   *tiles_out = ((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + n_tile - 1) / n_tile);
   return 0;
@@ -771,6 +806,9 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     if (!rc) rc = make_map_bf16_swz(&grp.epi[3], out + g0->n, g0->n, g0->m, g0->ldo, 32, 32, sw);
     if (rc) return rc;
   }
+  if (count > 1)
+    for (int i = 0; i < count; ++i)
+      if (items[i].limit != nullptr) return -9;
   int pairs = sms / 2;
   if (pairs < 1) pairs = 1;
   if (total < pairs) pairs = total;

@@ -23,6 +23,10 @@ struct GemmParams {
   const float* row_vec;
   float alpha, beta;
   int* error_flag;
+  const int* limit;    // row selection, see WsGemm
+  int limit_from;
+  const int* row_map;
+  int whole_rows;
   int debug;  // experiment switch: 1 = no loads (MMA issue rate only), 2 = always load tile (0,0)
 };
 

@@ -301,6 +301,9 @@ static int usable_sms() {
   return sms;
 }
 
+// Whether a problem with at least 256 rows takes the CTA-pair kernel now (the row-selecting LM head needs it).
+extern "C" int ws_gemm_pair_available(void) { return pair_mode() && usable_sms() >= 2; }
+
 extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaStream_t stream);
 
 // Several problems of one kind in one persistent launch when the CTA-pair kernel can take them
@@ -329,7 +332,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   }
   using namespace ws;
   const int sms = usable_sms();
-  if (pair_mode() && g->m >= 256 && sms >= 2) return ws_gemm_pair(g, sms, stream);
+  if (g->limit != nullptr || (pair_mode() && g->m >= 256 && sms >= 2)) return ws_gemm_pair(g, sms, stream);
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   const int b_rows = swiglu ? 2 * g->n : g->n;  // output features held by B
   CUtensorMap ta, tb;
@@ -356,6 +359,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   p.row_vec = g->row_vec;
   p.alpha = g->alpha; p.beta = g->beta;
   p.error_flag = g->error_flag;
+  p.limit = nullptr; p.row_map = nullptr; p.limit_from = p.whole_rows = 0;
   p.debug = 0;
 
   const int n_tile = swiglu ? 128 : BN;

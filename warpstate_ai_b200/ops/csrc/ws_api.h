@@ -46,9 +46,17 @@ typedef struct WsGemm {
   float alpha;
   float beta;
   int* error_flag;  // device int; set non-zero if a bounded wait ran out (may be NULL)
+  // Row selection (LM head over labelled rows; CTA-pair kernel only, NULL elsewhere).  With `limit` only the first
+  // clamp(*limit - limit_from, 0, rows) rows of A are computed (a_mn: that many steps of the contraction).
+  const int* limit;
+  int limit_from;
+  const int* row_map;  // BF16: output row of row m; CE_BWD: its index into row_scale; < 0: none
+  const void* whole;   // replaces A (a_mn: B) where *limit == whole_rows: the rows before their selection
+  int whole_rows, ldwhole;
 } WsGemm;
 
 int ws_gemm(const WsGemm* g, cudaStream_t stream);
+int ws_gemm_pair_available(void);  // 1 where problems with >= 256 rows take the CTA-pair kernel
 // Number of SMs the GEMM may use on this stream's device (0 = all).  Lets a communication
 // kernel keep a few SMs for itself while persistent GEMM CTAs fill the rest.
 // `count` problems in one persistent launch where possible (same operand majors and epilogue, each
@@ -188,10 +196,23 @@ int ws_adamw(float* p, const float* g, float* m, float* v, void* p_bf16, size_t 
              float grad_scale_const, const float* skip_ptr, cudaStream_t stream);
 
 // ----------------------------------------------------------------------------- LM head
+// The rows whose label is not `ignore_index`, in order: index[r] their places, labels_sel[r] their labels, *count how
+// many.  Rows from *count up to the next multiple of 256 (at most `rows`) get index -1 and label `ignore_index`.
+// logp is set to 0 at the rows that are left out.
+int ws_select_rows(const long long* labels, long long ignore_index, int rows, int* index, int* count,
+                   long long* labels_sel, float* logp, cudaStream_t stream);
+// out[r] = in[index[r]] for r < *count, zeros up to the next multiple of 256; nothing where *count == rows.
+int ws_gather_rows(const void* in, int ld, const int* index, const int* count, int rows, int d, void* out,
+                   cudaStream_t stream);
+// Zeros in the rows of out whose label is `ignore_index`.
+int ws_clear_unlabelled(const long long* labels, long long ignore_index, int rows, int d, void* out,
+                        cudaStream_t stream);
 // parts: float2 [rows, ld] of (max, sum exp) per 128 vocabulary columns (nparts valid per row),
-// written by the WS_EPI_CE_FWD epilogue.  lse[rows], logp[rows] (0 where label == ignore_index).
+// written by the WS_EPI_CE_FWD epilogue.  lse[rows], logp[rows] (0 where label == ignore_index).  With index and
+// count (may be NULL) only rows r < *count are combined and their logp goes to logp[index[r]].
 int ws_ce_combine(const void* parts, int ld, int nparts, const float* label_logit, const long long* labels,
-                  long long ignore_index, int rows, float* lse, float* logp, cudaStream_t stream);
+                  long long ignore_index, int rows, const int* index, const int* count, float* lse, float* logp,
+                  cudaStream_t stream);
 
 // ----------------------------------------------------------------------------- communication
 // Peer tables are arrays of `world` (<= 8) device addresses valid in THIS process: its mappings

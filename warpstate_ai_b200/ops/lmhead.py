@@ -6,6 +6,10 @@ logits are never written.  Backward: the same GEMM recomputes the logits and its
 ``(softmax - onehot) * row_weight`` in BF16, which feeds the dX GEMM (gradient of the hidden
 states) and the dW GEMM (FP32 accumulation into the tied embedding's gradient).
 
+An unlabelled row (-100: prompts and padding, most of a post-training batch) adds nothing to either pass, so from
+`SELECT_FROM` rows on the labelled rows are packed together on the device and the GEMMs run over them alone; their
+number is read by the kernels, not by the host.  Where every row is labelled nothing is copied.
+
 `loss_sum` is the summed cross-entropy over labels != -100 (reference warpstate/model.py:316-334,
 ops/loss_experiment.py:14-19); `token_logps` is the per-row label log-probability used for
 per-sequence sums in DPO (reference dpo.py:150-161).
@@ -17,6 +21,9 @@ import torch
 from . import _ext
 from . import gemm as G
 
+IGNORE = -100
+# Below one tile of the CTA-pair GEMM there is nothing to leave out, and the single-CTA kernel is the faster one.
+SELECT_FROM = 512
 ROWS_PER_BLOCK = 8192  # bounds the BF16 dlogits scratch to 512 MiB at vocab 32768
 
 
@@ -36,24 +43,34 @@ class _TokenLogps(torch.autograd.Function):
         labels = labels.contiguous()
         wb = bf16_weight(weight)
         flag = G.error_flag(hidden.device)
-        lse, logp = ops.lm_head_fwd(hidden, wb, labels, -100, flag)
-        ctx.save_for_backward(hidden, labels, lse)
         ctx.weight = weight
+        ctx.selected = hidden.shape[0] >= SELECT_FROM and ops.gemm_pair_available()
+        if ctx.selected:
+            logp, *rest = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, flag)
+            ctx.save_for_backward(hidden, labels, *rest)
+            return logp
+        lse, logp = ops.lm_head_fwd(hidden, wb, labels, IGNORE, flag)
+        ctx.save_for_backward(hidden, labels, lse)
         return logp
 
     @staticmethod
     def backward(ctx, grad_logp):
         from .fused import bf16_weight
         ops = torch.ops.ws_b200
-        hidden, labels, lse = ctx.saved_tensors
+        hidden, labels, lse, *selection = ctx.saved_tensors
         weight = ctx.weight
         wb = bf16_weight(weight)
         flag = G.error_flag(hidden.device)
         # d logp / d logits = onehot - softmax  ->  dlogits = (softmax - onehot) * (-grad), masked rows 0
-        row_weight = (-grad_logp.float() * labels.ne(-100)).contiguous()
+        row_weight = (-grad_logp.float() * labels.ne(IGNORE)).contiguous()
         dh = torch.empty_like(hidden)
         main = getattr(weight, "main_grad", None)
         grad_w = main if main is not None else torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
+        if ctx.selected:
+            index, count, packed, labels_sel = selection
+            ops.lm_head_bwd_labelled(hidden, packed, wb, labels, labels_sel, index, count, lse, row_weight, IGNORE,
+                                     ROWS_PER_BLOCK, dh, grad_w, flag)
+            return dh, (None if main is not None else grad_w.to(weight.dtype)), None
         for start in range(0, hidden.shape[0], ROWS_PER_BLOCK):
             stop = min(start + ROWS_PER_BLOCK, hidden.shape[0])
             h = hidden[start:stop]
