@@ -87,6 +87,4 @@ def backward(dy, qkvgu, saved, core, batch: int, seq: int):
     fl, sl, ml = _logits(core)
     dqkvgu, partials = torch.ops.ws_b200.attn_bwd(qkvgu, dy.contiguous(), states, writes, rope_table(qkvgu.device, pair_major=True),
                                                   fl, sl, ml, batch, seq, core.h, error_flag(qkvgu.device))
-    g = partials.view(batch, core.h, 16, 3).sum(dim=(0, 2))  # [H, 3] gradients w.r.t. the sigmoids
-    df, ds, mix = torch.sigmoid(fl), torch.sigmoid(sl), torch.sigmoid(ml)
-    return (dqkvgu, g[:, 0] * df * (1 - df), g[:, 1] * ds * (1 - ds), g[:, 2] * mix * (1 - mix))
+    return (dqkvgu, *torch.ops.ws_b200.memory_logit_grads(partials, fl, sl, ml, batch).unbind(0))

@@ -418,6 +418,28 @@ memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict
   }
 }
 
+// Gradients of the decay and mix logits from the scan's partial sums: out[q][h] = sigmoid'(logit_q[h]) * sum over the
+// head's B * 16 partials.  One CTA per head, one warp per logit, fixed order.  (A launch in place of the sum, three
+// sigmoids and nine products that a framework expression of it takes: 15 launches of 2 us for 3 H numbers.)
+__global__ void __launch_bounds__(96)
+memory_logit_grads_kernel(const float* __restrict__ partials, const float* __restrict__ fast_logit,
+                          const float* __restrict__ slow_logit, const float* __restrict__ mix_logit, int B, int H,
+                          float* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int h = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float v = 0.f;
+  for (int i = lane; i < B * 16; i += 32)
+    v += partials[((static_cast<size_t>(i >> 4) * H + h) * 16 + (i & 15)) * 3 + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) {
+    const float* logit = q == 0 ? fast_logit : q == 1 ? slow_logit : mix_logit;
+    const float s = 1.f / (1.f + expf(-logit[h]));
+    out[q * H + h] = v * s * (1.f - s);
+  }
+}
+
 // =============================================================================== attention bwd
 // One CTA of 128 threads per (batch, chunk, head) tile; thread t owns row t of the chunk.
 // The kernel is a chain of four MMA phases with element-wise work between them, so a single
@@ -881,6 +903,15 @@ extern "C" int ws_attn_bwd(const void* qkvgu, const void* states, const void* dy
   }
   launch_dependent(attn_bwd_kernel, dim3(tiles), dim3(AB_THREADS), AB_SMEM, stream, tm, ts, td, tw, to, reinterpret_cast<const float2*>(rope),
                                                           T, H, d, error_flag);
+  ws_count_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
+
+extern "C" int ws_memory_logit_grads(const float* partials, const float* fast_logit, const float* slow_logit,
+                                     const float* mix_logit, int B, int H, float* out, cudaStream_t stream) {
+  if (B <= 0 || H <= 0) return -1;
+  launch_dependent(memory_logit_grads_kernel, dim3(H), dim3(96), 0, stream, partials, fast_logit, slow_logit, mix_logit, B,
+                   H, out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

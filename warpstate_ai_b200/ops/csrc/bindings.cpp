@@ -383,6 +383,22 @@ std::tuple<at::Tensor, at::Tensor> attn_bwd(const at::Tensor& qkvgu, const at::T
   return {dqkvgu, partials};
 }
 
+// partials [B*H*16, 3] of attn_bwd -> FP32 [3, H]: gradients of the fast decay, slow decay and mix logits
+at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast_logit, const at::Tensor& slow_logit,
+                              const at::Tensor& mix_logit, int64_t B) {
+  const int64_t H = fast_logit.numel();
+  TORCH_CHECK(partials.is_cuda() && partials.scalar_type() == at::kFloat && partials.is_contiguous() &&
+              partials.numel() == B * H * 48, "memory_logit_grads: partials must be contiguous FP32 [B*H*16, 3]");
+  for (const at::Tensor* t : {&fast_logit, &slow_logit, &mix_logit})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == H, "memory_logit_grads: logits");
+  c10::cuda::CUDAGuard guard(partials.device());
+  at::Tensor out = at::empty({3, H}, partials.options());
+  check_rc(ws_memory_logit_grads(partials.data_ptr<float>(), fast_logit.data_ptr<float>(), slow_logit.data_ptr<float>(),
+                                 mix_logit.data_ptr<float>(), (int)B, (int)H, out.data_ptr<float>(), cur_stream()),
+           "memory_logit_grads");
+  return out;
+}
+
 // ----------------------------------------------------------------------------- optimizer
 static const int* opt_status(const c10::optional<at::Tensor>& status) {
   if (!status.has_value() || !status->defined()) return nullptr;
@@ -1032,6 +1048,7 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("attn_prefill(Tensor qkvgu, Tensor rope, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, int B, int T, "
         "int H, Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, "
         "Tensor(g!)? error_flag) -> Tensor");
+  m.def("memory_logit_grads(Tensor partials, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, int B) -> Tensor");
   m.def("grad_norm_clip(Tensor g, float max_norm, Tensor? extra_sumsq, Tensor? status=None) -> Tensor");
   m.def("clip_from_partials(Tensor partial, float max_norm, Tensor? extra_sumsq=None, Tensor? status=None) -> Tensor");
   m.def("grad_reduce_segments(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int[] starts, "
@@ -1082,6 +1099,7 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("attn_bwd", &attn_bwd);
   m.impl("chunk_writes", &chunk_writes);
   m.impl("memory_scan", &memory_scan);
+  m.impl("memory_logit_grads", &memory_logit_grads);
   m.impl("attn_fwd", &attn_fwd);
   m.impl("attn_prefill", &attn_prefill);
   m.impl("adamw_step", &adamw_step);

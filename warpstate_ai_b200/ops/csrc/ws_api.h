@@ -173,6 +173,9 @@ int ws_attn_dstate(const void* qkvgu, const void* dy, const float* rope, float* 
 int ws_memory_scan_bwd(const float* dstate, const float* writes, const float* fast_logit,
                        const float* slow_logit, const float* mix_logit, void* dwrites, float* partials,
                        int B, int N, int H, cudaStream_t stream);
+// out FP32 [3, H]: gradients of the fast decay, slow decay and mix logits from those partials.
+int ws_memory_logit_grads(const float* partials, const float* fast_logit, const float* slow_logit,
+                          const float* mix_logit, int B, int H, float* out, cudaStream_t stream);
 // dqkvgu: BF16 [B*T, 5d], fully written.
 int ws_attn_bwd(const void* qkvgu, const void* states, const void* dy, const void* dwrites,
                 const float* rope, void* dqkvgu, int B, int T, int H, int d, int* error_flag,
