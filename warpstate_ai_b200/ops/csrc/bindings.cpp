@@ -199,6 +199,29 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz,
   return {dx, dxb, dw};
 }
 
+// The norm behind a depth modulation (FP32 stream): -> (dx, FP32 [3, d]: gradients of w, of the bias, of the scale)
+std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const at::Tensor& xmod, const at::Tensor& rstd,
+                                                   const at::Tensor& w, const at::Tensor& dres, const at::Tensor& scale,
+                                                   const at::Tensor& bias) {
+  TORCH_CHECK(dz.is_cuda() && dz.scalar_type() == at::kBFloat16 && dz.is_contiguous(), "rmsnorm_bwd_mod: dz");
+  for (const at::Tensor* t : {&xmod, &dres})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->sizes() == dz.sizes(),
+                "rmsnorm_bwd_mod: xmod and dres must be FP32 [rows, d]");
+  const int rows = (int)xmod.size(0), d = (int)xmod.size(1);
+  for (const at::Tensor* t : {&w, &scale, &bias})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == d, "rmsnorm_bwd_mod: vectors must be FP32 [d]");
+  TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.is_contiguous() && rstd.numel() == rows, "rmsnorm_bwd_mod: rstd");
+  c10::cuda::CUDAGuard guard(xmod.device());
+  at::Tensor dx = at::empty_like(xmod);
+  at::Tensor partial = at::empty({3, ws_rmsnorm_bwd_mod_parts(rows), d}, xmod.options());
+  at::Tensor grads = at::empty({3, d}, xmod.options());
+  check_rc(ws_rmsnorm_bwd_mod(dz.data_ptr(), xmod.data_ptr<float>(), rstd.data_ptr<float>(), w.data_ptr<float>(),
+                              dres.data_ptr<float>(), scale.data_ptr<float>(), bias.data_ptr<float>(), rows, d,
+                              dx.data_ptr<float>(), partial.data_ptr<float>(), grads.data_ptr<float>(), cur_stream()),
+           "rmsnorm_bwd_mod");
+  return {dx, grads};
+}
+
 // (sum_rows a / (1+inv_scale), sum_rows a*b / (1+inv_scale))
 std::tuple<at::Tensor, at::Tensor> colsum2(const at::Tensor& a, const at::Tensor& b,
                                            const c10::optional<at::Tensor>& inv_scale) {
@@ -1019,6 +1042,7 @@ TORCH_LIBRARY(ws_b200, m) {
         "int H, Tensor(d!) y) -> ()");
   m.def("rmsnorm_fwd(Tensor x, Tensor? col_scale, Tensor? col_bias, Tensor w, float eps, bool want_xmod) -> (Tensor, Tensor, Tensor)");
   m.def("rmsnorm_bwd(Tensor dz, Tensor x, Tensor rstd, Tensor w, Tensor? dres, Tensor? out_scale, bool want_bf16) -> (Tensor, Tensor, Tensor)");
+  m.def("rmsnorm_bwd_mod(Tensor dz, Tensor xmod, Tensor rstd, Tensor w, Tensor dres, Tensor scale, Tensor bias) -> (Tensor, Tensor)");
   m.def("colsum2(Tensor a, Tensor b, Tensor? inv_scale) -> (Tensor, Tensor)");
   m.def("cast_bf16(Tensor x, Tensor(a!)? out) -> Tensor");
   m.def("embed_fwd(Tensor ids, Tensor table, bool out_bf16) -> Tensor");
@@ -1086,6 +1110,7 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("grad_weight_group", &grad_weight_group);
   m.impl("rmsnorm_fwd", &rmsnorm_fwd);
   m.impl("rmsnorm_bwd", &rmsnorm_bwd);
+  m.impl("rmsnorm_bwd_mod", &rmsnorm_bwd_mod);
   m.impl("colsum2", &colsum2);
   m.impl("cast_bf16", &cast_bf16);
   m.impl("embed_fwd", &embed_fwd);

@@ -146,6 +146,11 @@ rmsnorm_fwd_rows_kernel(const T* __restrict__ x, const float* __restrict__ col_s
 // block walks over groups of RB_ROWS rows, so every operand is read from global memory exactly
 // once with 16/32-byte coalesced accesses, the per-row mean needs one block reduction per group
 // (double-buffered, one __syncthreads), and the weight-gradient column sums stay in 8 registers.
+//
+// MOD (FP32 stream, the norm behind a depth modulation xmod = x * (1 + scale) + bias): the gradients of scale and bias
+// are column sums of dxmod * x and dxmod, and dxmod is in registers here, as is xmod, which gives x * (1 + scale) =
+// xmod - bias.  Summed in the same pass they cost 16 registers; as a pass of their own (colsum2_kernel, still used for
+// the BF16 stream, whose rounded xmod does not give x back) 268 MB more per 16384 x 2048 rows.
 constexpr int RB_ROWS = 2;
 
 template <typename T>
@@ -159,13 +164,13 @@ __device__ __forceinline__ void st8(T* p, const float (&v)[8]) {
   st4(p + 4, make_float4(v[4], v[5], v[6], v[7]));
 }
 
-template <typename T>
-__global__ void __launch_bounds__(ROW_THREADS, 3)
+template <typename T, bool MOD = false>
+__global__ void __launch_bounds__(ROW_THREADS, MOD ? 2 : 3)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x,
                    const float* __restrict__ rstd_in, const float* __restrict__ w,
                    const T* __restrict__ dres, const float* __restrict__ out_scale, int rows, int d,
                    T* __restrict__ dx_out, __nv_bfloat16* __restrict__ dx_bf16,
-                   float* __restrict__ dw_partial) {
+                   float* __restrict__ dw_partial, const float* __restrict__ mod_bias) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[2][RB_ROWS][ROW_WARPS];
@@ -174,8 +179,9 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x
   const bool active = c < d;
   const float inv_d = 1.0f / static_cast<float>(d);
   float wv[8], sv[8], acc[8];
+  [[maybe_unused]] float acc_bias[8], acc_scale[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { wv[j] = 0.f; sv[j] = 1.f; acc[j] = 0.f; }
+  for (int j = 0; j < 8; ++j) { wv[j] = 0.f; sv[j] = 1.f; acc[j] = 0.f; acc_bias[j] = 0.f; acc_scale[j] = 0.f; }
   if (active) {
     ld8(w + c, wv);
     if (out_scale != nullptr) {
@@ -234,6 +240,16 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
+        if constexpr (MOD) {
+          float xm[8], bi[8];
+          ld8(x + base, xm);      // in L1 since the first pass over the row
+          ld8(mod_bias + c, bi);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            acc_bias[j] += o[j];
+            acc_scale[j] += o[j] * (xm[j] - bi[j]);
+          }
+        }
 #pragma unroll
         for (int j = 0; j < 8; ++j) o[j] *= sv[j];
         st8(dx_out + base, o);
@@ -242,6 +258,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x
     }
   }
   if (dw_partial != nullptr && active) st8(dw_partial + static_cast<size_t>(blockIdx.x) * d + c, acc);
+  if constexpr (MOD) {
+    if (active) {
+      st8(dw_partial + (static_cast<size_t>(gridDim.x) + blockIdx.x) * d + c, acc_bias);
+      st8(dw_partial + (2 * static_cast<size_t>(gridDim.x) + blockIdx.x) * d + c, acc_scale);
+    }
+  }
 }
 
 // --------------------------------------------------------------------------- column sums
@@ -270,16 +292,19 @@ colsum2_kernel(const T* __restrict__ a, const T* __restrict__ b, int rows, int d
   }
 }
 
-// out[c] = beta*out[c] + scale(c) * sum_p partial[p][c];  scale(c) = 1/(1+inv_scale[c]) if given
+// out[c] = beta*out[c] + scale(c) * sum_p partial[p][c];  scale(c) = 1/(1+inv_scale[c]) if given.  gridDim.y sums of
+// that kind lie behind one another ([gridDim.y][parts][d] -> [gridDim.y][d]); only sum `inv_plane` is scaled.
 // One block per 32 columns; warp w sums parts w, w+8, ... (independent 128-byte loads in
 // flight), then the eight warp sums are combined in a fixed order: the result is deterministic.
 constexpr int FIN_COLS = 32;
 __global__ void __launch_bounds__(ROW_THREADS)
 colsum_finalize_kernel(const float* __restrict__ partial, int parts, int d,
-                       const float* __restrict__ inv_scale, float beta, float* __restrict__ out) {
+                       const float* __restrict__ inv_scale, int inv_plane, float beta, float* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[ROW_WARPS][FIN_COLS];
+  partial += static_cast<size_t>(blockIdx.y) * parts * d;
+  out += static_cast<size_t>(blockIdx.y) * d;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * FIN_COLS + lane;
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
@@ -299,7 +324,7 @@ colsum_finalize_kernel(const float* __restrict__ partial, int parts, int d,
     float s = 0.f;
 #pragma unroll
     for (int wi = 0; wi < ROW_WARPS; ++wi) s += red[wi][lane];
-    if (inv_scale != nullptr) {
+    if (inv_scale != nullptr && static_cast<int>(blockIdx.y) == inv_plane) {
       const float den = 1.f + inv_scale[c];
       s = den != 0.f ? s / den : 0.f;
     }
@@ -435,10 +460,31 @@ extern "C" int ws_rmsnorm_bwd(const void* dz, const void* x, int x_bf16, const f
   const int grid = ws_rmsnorm_bwd_parts(rows);
   if (x_bf16)
     launch_dependent(rmsnorm_bwd_kernel<__nv_bfloat16>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)x, rstd, w, (const __nv_bfloat16*)dres, out_scale,
-        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial);
+        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial, nullptr);
   else
     launch_dependent(rmsnorm_bwd_kernel<float>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const float*)x, rstd, w, (const float*)dres, out_scale, rows, d,
-        (float*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial);
+        (float*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial, nullptr);
+  ws_count_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+}
+
+// Two resident blocks per SM: the modulation's column sums take the registers of the third.
+extern "C" int ws_rmsnorm_bwd_mod_parts(int rows) {
+  const int blocks = (rows + RB_ROWS - 1) / RB_ROWS;
+  return blocks < 148 * 2 ? (blocks > 0 ? blocks : 1) : 148 * 2;
+}
+
+extern "C" int ws_rmsnorm_bwd_mod(const void* dz, const float* xmod, const float* rstd, const float* w, const float* dres,
+                                  const float* scale, const float* bias, int rows, int d, float* dx_out,
+                                  float* partial, float* grads, cudaStream_t stream) {
+  if (d % 128 != 0 || d > ROW_THREADS * 8 || rows <= 0) return -1;
+  const int parts = ws_rmsnorm_bwd_mod_parts(rows);
+  launch_dependent(rmsnorm_bwd_kernel<float, true>, dim3(parts), dim3(ROW_THREADS), 0, stream,
+                   static_cast<const __nv_bfloat16*>(dz), xmod, rstd, w, dres, scale, rows, d, dx_out,
+                   static_cast<__nv_bfloat16*>(nullptr), partial, bias);
+  ws_count_launch();
+  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS, 3), dim3(ROW_THREADS), 0, stream, partial,
+                   parts, d, scale, 2, 0.f, grads);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -460,7 +506,7 @@ extern "C" int ws_colsum2(const void* a, const void* b, int is_bf16, int rows, i
 
 extern "C" int ws_colsum_finalize(const float* partial, int parts, int d, const float* inv_scale, float beta,
                                   float* out, cudaStream_t stream) {
-  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, partial, parts, d, inv_scale, beta, out);
+  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, partial, parts, d, inv_scale, 0, beta, out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -571,12 +617,12 @@ extern "C" int ws_rmsnorm_bwd_static(const void* dz, const void* x, int x_bf16, 
   // previous call's contents never leak into this result.
   if (x_bf16)
     launch_dependent(rmsnorm_bwd_kernel<__nv_bfloat16>, dim3(parts), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)x, rstd, w, (const __nv_bfloat16*)dres, out_scale,
-        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, scratch);
+        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, scratch, nullptr);
   else
     launch_dependent(rmsnorm_bwd_kernel<float>, dim3(parts), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const float*)x, rstd, w, (const float*)dres, out_scale, rows, d,
-        (float*)dx_out, (__nv_bfloat16*)dx_bf16, scratch);
+        (float*)dx_out, (__nv_bfloat16*)dx_bf16, scratch, nullptr);
   ws_count_launch();
-  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, scratch, parts, d, nullptr, 0.f, dw_out);
+  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, scratch, parts, d, nullptr, 0, 0.f, dw_out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : WS_STATIC_ERR_LAUNCH;
 }

@@ -248,8 +248,9 @@ class CoreFn(torch.autograd.Function):
             ctx.save_for_backward(x_in, scale if has_mod else dummy, bias if has_mod else dummy, n1w, n2w)
         else:
             ctx.attn_saved = attn_saved
-            ctx.save_for_backward(x_in if has_mod else xmod, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act,
-                                  scale if has_mod else dummy, n1w, n2w)
+            # the block's input is read again only where its modulated copy is rounded (`_modulation_sums`)
+            ctx.save_for_backward(x_in if has_mod and x_in.dtype != torch.float32 else xmod, xmod, rstd1, z1, qkvgu, y, x2,
+                                  rstd2, z2, packed, act, scale if has_mod else dummy, bias if has_mod else dummy, n1w, n2w)
         return x3.view(batch, seq, d)
 
     @staticmethod
@@ -269,7 +270,7 @@ class CoreFn(torch.autograd.Function):
                                          batch, seq, want_output=False)
             xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, attn_saved = saved
         else:
-            x_in, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, scale, n1w, n2w = ctx.saved_tensors
+            x_in, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, scale, bias, n1w, n2w = ctx.saved_tensors
             attn_saved = ctx.attn_saved
         bw_in, bw_out, bw_ug, bw_down = weights.backward_weights()
         dx3 = dx3.reshape(m, d)
@@ -289,22 +290,14 @@ class CoreFn(torch.autograd.Function):
         dqkvgu, g_fast, g_slow, g_mix = _attention_backward(dy, qkvgu, attn_saved, core, batch, seq)
         del dy
         dz1 = G.grad_input(dqkvgu, bw_in)
-        dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
-        g_scale = g_bias = None
-        side = _side_stream(dx_in.device) if ctx.has_mod else None
-        if ctx.has_mod:
-            # d bias = colsum(d x_mod), d scale = colsum(d x_mod * x_in), with d x_mod = dx_in / (1+scale).
-            # Bandwidth-bound and independent of the weight gradients: it runs on a second stream under
-            # the grouped dW launch below, whose CTAs leave room for it on every SM.
-            if side is not None:
-                main = torch.cuda.current_stream(dx_in.device)
-                side.wait_stream(main)
-                with torch.cuda.stream(side):
-                    g_bias, g_scale = ops.colsum2(dx_in, x_in, scale)
-                for t in (g_bias, g_scale, dx_in, x_in, scale):
-                    t.record_stream(side)
-            else:
-                g_bias, g_scale = ops.colsum2(dx_in, x_in, scale)
+        g_scale = g_bias = side = None
+        if ctx.has_mod and not stream_bf16:
+            dx_in, sums = ops.rmsnorm_bwd_mod(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale, bias)
+            g_n1, g_bias, g_scale = sums.unbind(0)
+        else:
+            dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
+            if ctx.has_mod:
+                g_bias, g_scale, side = _modulation_sums(dx_in, x_in, scale)
         # ---- the four weight gradients, deferred to one grouped launch (their tiles share waves)
         g_down, g_ug, g_out, g_in = _wgrad_group([(dx3b, act, w_down), (dpacked, z2, w_ug), (dx2b, y, w_out),
                                                   (dqkvgu, z1, w_in)])
@@ -318,6 +311,21 @@ class CoreFn(torch.autograd.Function):
             g_n1 = g_n2 = g_fast = g_slow = g_mix = None
         return (dx_in.view(batch, seq, d), g_scale, g_bias, g_n1, g_in, g_out, g_n2, g_ug, g_down,
                 g_fast, g_slow, g_mix, None, None, None)
+
+
+def _modulation_sums(dx_in, x_in, scale):
+    """d bias = colsum(d x_mod), d scale = colsum(d x_mod * x_in) of a BF16 stream, with d x_mod = dx_in / (1+scale).
+    Bandwidth-bound and independent of the weight gradients: it runs on a second stream under the grouped dW launch,
+    whose CTAs leave room for it on every SM; the caller waits for the stream that is returned."""
+    side = _side_stream(dx_in.device)
+    if side is None:
+        return (*_ops().colsum2(dx_in, x_in, scale), None)
+    side.wait_stream(torch.cuda.current_stream(dx_in.device))
+    with torch.cuda.stream(side):
+        g_bias, g_scale = _ops().colsum2(dx_in, x_in, scale)
+    for t in (g_bias, g_scale, dx_in, x_in, scale):
+        t.record_stream(side)
+    return g_bias, g_scale, side
 
 
 def _attach_small_grads(core, g_n1, g_n2, g_fast, g_slow, g_mix) -> None:
