@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "ws_api.h"
@@ -420,6 +421,112 @@ at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast
                                  mix_logit.data_ptr<float>(), (int)B, (int)H, out.data_ptr<float>(), cur_stream()),
            "memory_logit_grads");
   return out;
+}
+
+// ----------------------------------------------------------------------------- whole blocks
+// The kernel sequences of one block (ops/fused.py) as one call each.  A block is eight to twelve launches of 2-20 us in
+// a short sequence, and issued one by one from Python the host takes longer than the device below a few thousand rows;
+// here a launch costs its allocation, its tensor maps and the launch.  Same kernels, same order, same results.
+at::Tensor project(const at::Tensor& x, const at::Tensor& w, bool b_mn, int64_t epilogue, int64_t n, at::Tensor out,
+                   const c10::optional<at::Tensor>& out2, const c10::optional<at::Tensor>& aux,
+                   const c10::optional<at::Tensor>& flag) {
+  gemm(x, w, false, b_mn, epilogue, x.size(0), n, x.size(1), out, out2, aux, c10::nullopt, 1.0, 0.0, flag);
+  return out;
+}
+at::Tensor project_bf16(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& flag) {
+  return project(x, w, false, WS_EPI_BF16, w.size(0), at::empty({x.size(0), w.size(0)}, x.options()), c10::nullopt, c10::nullopt, flag);
+}
+at::Tensor project_residual(const at::Tensor& x, const at::Tensor& w, const at::Tensor& resid,
+                            const c10::optional<at::Tensor>& flag) {
+  return project(x, w, false, resid.scalar_type() == at::kFloat ? WS_EPI_RESID_F32 : WS_EPI_RESID_BF16, w.size(0),
+                 at::empty_like(resid), c10::nullopt, resid, flag);
+}
+at::Tensor input_grad(const at::Tensor& dy, const at::Tensor& w, const c10::optional<at::Tensor>& flag) {
+  return project(dy, w, true, WS_EPI_BF16, w.size(1), at::empty({dy.size(0), w.size(1)}, dy.options()), c10::nullopt, c10::nullopt, flag);
+}
+
+// x2 = xmod + out_proj(y), then x2 + down(swiglu(up_gate(norm2 x2))).  -> (x2, rstd2, z2, packed, act, x3); packed only
+// with `keep` (the backward pass reads it), x3 only with `want_output`.
+struct BlockTail { at::Tensor x2, rstd2, z2, packed, act, x3; };
+BlockTail block_tail(const at::Tensor& y, const at::Tensor& xmod, const at::Tensor& w_out, const at::Tensor& n2,
+                     const at::Tensor& w_ug, const at::Tensor& w_down, double eps, bool keep, bool want_output,
+                     const c10::optional<at::Tensor>& flag) {
+  BlockTail t;
+  t.x2 = project_residual(y, w_out, xmod, flag);
+  at::Tensor unchanged;
+  std::tie(t.z2, t.rstd2, unchanged) = rmsnorm_fwd(t.x2, c10::nullopt, c10::nullopt, n2, eps, false);
+  const int64_t h = w_ug.size(0) / 2;
+  if (keep) t.packed = at::empty({y.size(0), 2 * h}, y.options());
+  t.act = at::empty({y.size(0), h}, y.options());
+  project(t.z2, w_ug, false, WS_EPI_SWIGLU, h, t.packed, t.act, c10::nullopt, flag);
+  if (want_output) t.x3 = project_residual(t.act, w_down, t.x2, flag);
+  return t;
+}
+
+// -> (x3, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, writes, states); x3 and packed may be undefined.
+std::vector<at::Tensor> block_fwd(const at::Tensor& x, const c10::optional<at::Tensor>& scale,
+                                  const c10::optional<at::Tensor>& bias, const at::Tensor& n1, const at::Tensor& w_in,
+                                  const at::Tensor& w_out, const at::Tensor& n2, const at::Tensor& w_ug,
+                                  const at::Tensor& w_down, const at::Tensor& fast_logit, const at::Tensor& slow_logit,
+                                  const at::Tensor& mix_logit, const at::Tensor& rope, double eps, int64_t B, int64_t T,
+                                  int64_t H, bool keep, bool want_output, const c10::optional<at::Tensor>& flag) {
+  auto [z1, rstd1, xmod] = rmsnorm_fwd(x, scale, bias, n1, eps, true);
+  at::Tensor qkvgu = project_bf16(z1, w_in, flag);
+  at::Tensor writes = chunk_writes(qkvgu, rope, B, T, H, flag);
+  at::Tensor states = std::get<0>(memory_scan(writes, fast_logit, slow_logit, mix_logit, true, false, c10::nullopt, c10::nullopt));
+  at::Tensor y = attn_fwd(qkvgu, states, rope, B, T, H, flag);
+  BlockTail t = block_tail(y, xmod, w_out, n2, w_ug, w_down, eps, keep, want_output, flag);
+  at::Tensor none = at::empty({0}, x.options());
+  return {want_output ? t.x3 : none, xmod, rstd1, z1, qkvgu, y, t.x2, t.rstd2, t.z2, keep ? t.packed : none, t.act, writes, states};
+}
+
+// Backward up to the gradient of the block's input; the weight gradients follow as one group (grad_weight_group).
+// -> (dx, dx3 BF16, dpacked, dx2 BF16, dqkvgu, g_norm2, logit gradients [3, H], first norm's [3, d] or [1, d]): w, and
+// behind an FP32 depth modulation its bias and scale.
+std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& xmod, const at::Tensor& rstd1,
+                                  const at::Tensor& qkvgu, const at::Tensor& x2, const at::Tensor& rstd2,
+                                  const at::Tensor& packed, const at::Tensor& writes, const at::Tensor& states,
+                                  const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& bias,
+                                  const at::Tensor& n1, const at::Tensor& n2, const at::Tensor& w_in, const at::Tensor& w_out,
+                                  const at::Tensor& w_ug, const at::Tensor& w_down, const at::Tensor& fast_logit,
+                                  const at::Tensor& slow_logit, const at::Tensor& mix_logit, const at::Tensor& rope, int64_t B, int64_t T, int64_t H,
+                                  const c10::optional<at::Tensor>& flag) {
+  const bool bf16_stream = dx3.scalar_type() == at::kBFloat16;
+  at::Tensor dx3b = bf16_stream ? dx3 : cast_bf16(dx3, c10::nullopt);
+  const int64_t h = w_down.size(1);
+  at::Tensor dpacked = project(dx3b, w_down, true, WS_EPI_SWIGLU_BWD, h, at::empty({dx3b.size(0), 2 * h}, dx3b.options()),
+                               c10::nullopt, packed, flag);
+  auto [dx2, dx2b, g_n2] = rmsnorm_bwd(input_grad(dpacked, w_ug, flag), x2, rstd2, n2, dx3, c10::nullopt, !bf16_stream);
+  if (bf16_stream) dx2b = dx2;
+  auto [dqkvgu, partials] = attn_bwd(qkvgu, input_grad(dx2b, w_out, flag), states, writes, rope, fast_logit, slow_logit,
+                                   mix_logit, B, T, H, flag);
+  at::Tensor logits = memory_logit_grads(partials, fast_logit, slow_logit, mix_logit, B);
+  at::Tensor dz1 = input_grad(dqkvgu, w_in, flag);
+  if (scale.has_value() && scale->defined() && !bf16_stream) {
+    auto [dx, norm] = rmsnorm_bwd_mod(dz1, xmod, rstd1, n1, dx2, *scale, *bias);
+    return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm};
+  }
+  auto [dx, unused, g_n1] = rmsnorm_bwd(dz1, xmod, rstd1, n1, dx2, scale, false);
+  return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, g_n1.unsqueeze(0)};
+}
+
+// Forward over prompts of any length; the layer's decode state is written.  -> the block's output rows [B*T, d], or with
+// `last` (residual input, attention output) at the final position of every sequence, [B, d] each.
+std::vector<at::Tensor> block_prefill(const at::Tensor& x, const at::Tensor& scale, const at::Tensor& bias,
+                                      const at::Tensor& n1, const at::Tensor& w_in, const at::Tensor& w_out,
+                                      const at::Tensor& n2, const at::Tensor& w_ug, const at::Tensor& w_down,
+                                      const at::Tensor& fast_logit, const at::Tensor& slow_logit, const at::Tensor& mix_logit,
+                                      const at::Tensor& rope, double eps, int64_t B, int64_t T, int64_t H, at::Tensor fast,
+                                      at::Tensor slow, at::Tensor mixed, at::Tensor kc, at::Tensor vc, at::Tensor uc, bool last,
+                                      const c10::optional<at::Tensor>& flag) {
+  auto [z1, rstd1, xmod] = rmsnorm_fwd(x, scale, bias, n1, eps, true);
+  at::Tensor y = attn_prefill(project_bf16(z1, w_in, flag), rope, fast_logit, slow_logit, mix_logit, B, T, H, fast, slow,
+                              mixed, kc, vc, uc, flag);
+  if (last) {
+    const int64_t d = x.size(1);
+    return {xmod.view({B, T, d}).select(1, T - 1).contiguous(), y.view({B, T, d}).select(1, T - 1).contiguous()};
+  }
+  return {block_tail(y, xmod, w_out, n2, w_ug, w_down, eps, false, true, flag).x3};
 }
 
 // ----------------------------------------------------------------------------- optimizer
@@ -1073,6 +1180,16 @@ TORCH_LIBRARY(ws_b200, m) {
         "int H, Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, "
         "Tensor(g!)? error_flag) -> Tensor");
   m.def("memory_logit_grads(Tensor partials, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, int B) -> Tensor");
+  m.def("block_fwd(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
+        "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
+        "bool keep, bool want_output, Tensor(a!)? flag) -> Tensor[]");
+  m.def("block_bwd(Tensor dx3, Tensor xmod, Tensor rstd1, Tensor qkvgu, Tensor x2, Tensor rstd2, Tensor packed, Tensor writes, "
+        "Tensor states, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor w_in, Tensor w_out, Tensor w_ug, Tensor w_down, "
+        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, int B, int T, int H, Tensor(a!)? flag) -> Tensor[]");
+  m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
+        "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
+        "Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, bool last, "
+        "Tensor(g!)? flag) -> Tensor[]");
   m.def("grad_norm_clip(Tensor g, float max_norm, Tensor? extra_sumsq, Tensor? status=None) -> Tensor");
   m.def("clip_from_partials(Tensor partial, float max_norm, Tensor? extra_sumsq=None, Tensor? status=None) -> Tensor");
   m.def("grad_reduce_segments(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int[] starts, "
@@ -1125,6 +1242,9 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("chunk_writes", &chunk_writes);
   m.impl("memory_scan", &memory_scan);
   m.impl("memory_logit_grads", &memory_logit_grads);
+  m.impl("block_fwd", &block_fwd);
+  m.impl("block_bwd", &block_bwd);
+  m.impl("block_prefill", &block_prefill);
   m.impl("attn_fwd", &attn_fwd);
   m.impl("attn_prefill", &attn_prefill);
   m.impl("adamw_step", &adamw_step);

@@ -197,12 +197,31 @@ def _weights_of(core, params):
 
 
 # --------------------------------------------------------------------------- one core
-def _core_kernels(core, weights, x_in, scale, bias, n1w, n2w, batch, seq, want_output=True):
+def _native(core, weights) -> bool:
+    """The block runs as one native call each way: whole weights, the attention kernels' geometry, and no tuned choice of
+    GEMM kernel per problem (which is made launch by launch)."""
+    from . import attention
+    return type(weights) is LocalWeights and attention.kernels_ready(core) and not G._policy
+
+
+def _native_arguments(core, device):
+    from . import attention
+    return (*attention._logits(core), attention.rope_table(device, pair_major=True))
+
+
+def _core_kernels(core, weights, x_in, scale, bias, n1w, n2w, batch, seq, want_output=True, keep=True):
     """The forward kernel sequence of one core on ``x_in [M, d]`` (FP32 or BF16 residual stream).
     Returns every tensor the backward pass reads, and ``x3`` (None when ``want_output`` is False: the
-    recomputation inside a checkpointed backward stops before the down projection)."""
+    recomputation inside a checkpointed backward stops before the down projection).  Without ``keep`` no backward
+    follows and (up | gate) need not be written."""
     ops = _ops()
     has_mod = scale is not None
+    if _native(core, weights):
+        w_in, w_out, w_ug, w_down = weights.backward_weights()
+        x3, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, *attn_saved = ops.block_fwd(
+            x_in, scale, bias, n1w, w_in, w_out, n2w, w_ug, w_down, *_native_arguments(core, x_in.device),
+            core.cfg.rms_eps, batch, seq, core.h, keep, want_output, G.error_flag(x_in.device))
+        return (xmod if has_mod else x_in, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, attn_saved), x3
     weights.begin_forward()
     z1, rstd1, xmod = ops.rmsnorm_fwd(x_in, scale, bias, n1w, core.cfg.rms_eps, True)
     qkvgu = weights.in_proj(z1)
@@ -222,7 +241,7 @@ class CoreFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, depth_scale, depth_bias, n1w, w_in, w_out, n2w, w_ug, w_down, fast_logit,
-                slow_logit, mix_logit, core, notify=True, checkpoint=False):
+                slow_logit, mix_logit, core, notify=True, checkpoint=False, keep=True):
         batch, seq, d = x.shape
         m = batch * seq
         x_in = x.reshape(m, d)
@@ -234,7 +253,7 @@ class CoreFn(torch.autograd.Function):
         n1 = n1w.detach().float()
         n2 = n2w.detach().float()
         weights = _weights_of(core, (w_in, w_out, w_ug, w_down))
-        saved, x3 = _core_kernels(core, weights, x_in, scale, bias, n1, n2, batch, seq)
+        saved, x3 = _core_kernels(core, weights, x_in, scale, bias, n1, n2, batch, seq, keep=keep and not checkpoint)
         xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, attn_saved = saved
         ctx.core = core
         ctx.notify = notify
@@ -277,27 +296,38 @@ class CoreFn(torch.autograd.Function):
         if not dx3.is_contiguous():
             dx3 = dx3.contiguous()
         stream_bf16 = dx3.dtype == torch.bfloat16
-        # ---- FFN
-        dx3b = dx3 if stream_bf16 else ops.cast_bf16(dx3, None)
-        dpacked = G.grad_input_swiglu(dx3b, bw_down, packed)
-        dz2 = G.grad_input(dpacked, bw_ug)
-        dx2, dx2b, g_n2 = ops.rmsnorm_bwd(dz2, x2, rstd2, n2w.detach().float(), dx3, None, not stream_bf16)
-        if stream_bf16:
-            dx2b = dx2
-        del dz2
-        # ---- attention / memory
-        dy = G.grad_input(dx2b, bw_out)
-        dqkvgu, g_fast, g_slow, g_mix = _attention_backward(dy, qkvgu, attn_saved, core, batch, seq)
-        del dy
-        dz1 = G.grad_input(dqkvgu, bw_in)
         g_scale = g_bias = side = None
-        if ctx.has_mod and not stream_bf16:
-            dx_in, sums = ops.rmsnorm_bwd_mod(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale, bias)
-            g_n1, g_bias, g_scale = sums.unbind(0)
+        modulated = ctx.has_mod and not stream_bf16
+        if _native(core, weights) and attn_saved is not None:
+            dx_in, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm = ops.block_bwd(
+                dx3, xmod, rstd1, qkvgu, x2, rstd2, packed, *attn_saved, scale if ctx.has_mod else None,
+                bias if ctx.has_mod else None, n1w.detach().float(), n2w.detach().float(), bw_in, bw_out, bw_ug, bw_down,
+                *_native_arguments(core, dx3.device), batch, seq, core.h, G.error_flag(dx3.device))
+            g_fast, g_slow, g_mix = logits.unbind(0)
+            g_n1, *g_mod = norm.unbind(0)
+            if modulated:
+                g_bias, g_scale = g_mod
         else:
-            dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
-            if ctx.has_mod:
-                g_bias, g_scale, side = _modulation_sums(dx_in, x_in, scale)
+            # ---- FFN
+            dx3b = dx3 if stream_bf16 else ops.cast_bf16(dx3, None)
+            dpacked = G.grad_input_swiglu(dx3b, bw_down, packed)
+            dz2 = G.grad_input(dpacked, bw_ug)
+            dx2, dx2b, g_n2 = ops.rmsnorm_bwd(dz2, x2, rstd2, n2w.detach().float(), dx3, None, not stream_bf16)
+            if stream_bf16:
+                dx2b = dx2
+            del dz2
+            # ---- attention / memory
+            dy = G.grad_input(dx2b, bw_out)
+            dqkvgu, g_fast, g_slow, g_mix = _attention_backward(dy, qkvgu, attn_saved, core, batch, seq)
+            del dy
+            dz1 = G.grad_input(dqkvgu, bw_in)
+            if modulated:
+                dx_in, sums = ops.rmsnorm_bwd_mod(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale, bias)
+                g_n1, g_bias, g_scale = sums.unbind(0)
+            else:
+                dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
+        if ctx.has_mod and not modulated:
+            g_bias, g_scale, side = _modulation_sums(dx_in, x_in, scale)
         # ---- the four weight gradients, deferred to one grouped launch (their tiles share waves)
         g_down, g_ug, g_out, g_in = _wgrad_group([(dx3b, act, w_down), (dpacked, z2, w_ug), (dx2b, y, w_out),
                                                   (dqkvgu, z1, w_in)])
@@ -310,7 +340,7 @@ class CoreFn(torch.autograd.Function):
             _core_grad_hook(core)
             g_n1 = g_n2 = g_fast = g_slow = g_mix = None
         return (dx_in.view(batch, seq, d), g_scale, g_bias, g_n1, g_in, g_out, g_n2, g_ug, g_down,
-                g_fast, g_slow, g_mix, None, None, None)
+                g_fast, g_slow, g_mix, None, None, None, None)
 
 
 def _modulation_sums(dx_in, x_in, scale):
@@ -349,7 +379,7 @@ def core_forward(core, x: torch.Tensor, depth_scale=None, depth_bias=None, notif
     return CoreFn.apply(x, depth_scale, depth_bias, core.norm1.weight, core.in_proj.weight,
                         core.out_proj.weight, core.norm2.weight, core.ffn.up_gate.weight,
                         core.ffn.down.weight, core.fast_decay_logit, core.slow_decay_logit,
-                        core.memory_mix_logit, core, notify, checkpoint)
+                        core.memory_mix_logit, core, notify, checkpoint, torch.is_grad_enabled())
 
 
 # --------------------------------------------------------------------------- embedding / final norm
@@ -410,11 +440,12 @@ def trunk_forward(model, input_ids: torch.Tensor) -> torch.Tensor:
     cfg = model.cfg
     x = EmbedFn.apply(input_ids, model.embed.weight, bool(getattr(model, "bf16_residuals", False)))
     checkpoint = bool(cfg.gradient_checkpointing and model.training and torch.is_grad_enabled())
+    # one backward node for all depths' rows, instead of a zero-filled table and an addition per depth
+    scales, biases = model.depth_scale.unbind(0), model.depth_bias.unbind(0)
     for depth in range(cfg.logical_depth):
         core = model.cores[depth % cfg.n_cores]
         # the first forward use of a (possibly shared) core is its last use in backward
-        x = core_forward(core, x, model.depth_scale[depth], model.depth_bias[depth], notify=depth < cfg.n_cores,
-                         checkpoint=checkpoint)
+        x = core_forward(core, x, scales[depth], biases[depth], notify=depth < cfg.n_cores, checkpoint=checkpoint)
     return NormFn.apply(x, model.final_norm.weight, cfg.rms_eps)
 
 
@@ -501,6 +532,15 @@ def core_prefill_state(core, x: torch.Tensor, depth_scale, depth_bias, batch: in
     Returns the rows ``[B*T, d]``, or with ``last`` (nothing reads the other positions of the last block) the block's
     residual input and its attention output at the final position of every sequence, ``[B, d]`` each."""
     from . import attention
+    weights = LocalWeights(core.in_proj.weight, core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight)
+    if _native(core, weights):
+        w_in, w_out, w_ug, w_down = weights.backward_weights()
+        out = _ops().block_prefill(x, depth_scale.detach().float().contiguous(), depth_bias.detach().float().contiguous(),
+                                   core.norm1.weight.detach().float(), w_in, w_out, core.norm2.weight.detach().float(),
+                                   w_ug, w_down, *_native_arguments(core, x.device), core.cfg.rms_eps, batch, seq, core.h,
+                                   state.fast, state.slow, state.mixed, state.k, state.v, state.u, last,
+                                   G.error_flag(x.device))
+        return tuple(out) if last else out[0]
     z1, xmod = _prefill_norm(core, x, depth_scale, depth_bias)
     y = attention.prefill(G.linear(z1, bf16_weight(core.in_proj.weight)), core, batch, seq, state)
     if last:
