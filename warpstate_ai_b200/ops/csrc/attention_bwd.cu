@@ -441,10 +441,12 @@ memory_logit_grads_kernel(const float* __restrict__ partials, const float* __res
 }
 
 // =============================================================================== attention bwd
-// One CTA of 128 threads per (batch, chunk, head) tile; thread t owns row t of the chunk.
+// One CTA of 256 threads per (batch, chunk, head) tile; threads t and t + 128 own row t of the chunk, one half of its
+// columns each (of the 128 score columns, every other block of 32, so that the causal triangle is halved too).
 // The kernel is a chain of four MMA phases with element-wise work between them, so a single
-// tile cannot keep an SM busy; what matters is how many tiles an SM holds at once.  Shared
-// memory is therefore kept to 112 KiB and TMEM to 256 columns, so that TWO CTAs fit per SM:
+// tile cannot keep an SM busy; what matters is how many tiles an SM holds at once, and how long the element-wise
+// stretches of the chain are.  Shared memory is therefore kept to 112 KiB and TMEM to 256 columns, so that TWO CTAs fit
+// per SM, and a row is shared by two threads, which exchange its softmax statistics and its D through shared memory.
 //
 //   smem: B0 Qr | B1 Kr | B2 dy -> dlocal -> tanh(U) | B3 dmem/8 -> V -> tanh(Kr) | sP (32K: P -> dS)
 //         | sSt (8K) | sDW (8K) | barriers
@@ -453,7 +455,8 @@ memory_logit_grads_kernel(const float* __restrict__ partials, const float* __res
 //
 // V and U are fetched late (into buffers that earlier operands have left), each behind work that
 // hides most of the load latency.  P is stored normalised, so O and dV need no row scaling.
-constexpr int AB_THREADS = 128;
+constexpr int AB_THREADS = 256;
+constexpr int AB_PIECES = 4;   // 16-byte pieces of a 64-column row that a thread owns
 // No alignment slack: 2 x (114816 + 1024 reserved) = 231680 <= 233472 bytes of an SM.  The dynamic
 // segment is declared 1024-byte aligned (the 128-byte swizzle needs it); the kernel checks.
 constexpr int AB_SMEM = 4 * TILE_BYTES + 2 * TILE_BYTES + 2 * 8192 + 128;
@@ -479,7 +482,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDW + 8192);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, half = tid >> 7, quarter = warp & 3;
+  const int piece0 = half * AB_PIECES;
   const int n_chunks = T / CHUNK;
   const int tile = blockIdx.x;
   const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
@@ -503,7 +507,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   const uint32_t t_lo = tmem;          // S / O / dP / dKr+dtK
   const uint32_t t_mid = tmem + 128;   // Mem / dV / dtU
   const uint32_t t_dq = tmem + 192;    // dQr
-  const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+  const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
 
   if (tid == 0) {
     mbar_expect_tx(&bars[0], 4 * TILE_BYTES + 2 * 8192);
@@ -514,20 +518,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
     tma_load_2d(sSt, &tm_state, &bars[0], 0, tile * HD);
     tma_load_2d(sDW, &tm_dw, &bars[0], 0, tile * HD);
   }
-  // The thread's gate row, its dGate row and its dV row stay in registers (8 x 16 bytes each) until
+  // The thread's half of the gate row, of the dGate row and of the dV row stay in registers (4 x 16 bytes each) until
   // the last stage, where all five gradient tiles leave through shared memory and TMA stores.
-  uint4 gate_row[8], dgate_row[8], dv_row[8];
+  uint4 gate_row[AB_PIECES], dgate_row[AB_PIECES], dv_row[AB_PIECES];
 
   bool ok = mbar_wait(&bars[0], 0, abort_flag);
 #pragma unroll
-  for (int j = 0; j < 8; ++j) gate_row[j] = *reinterpret_cast<const uint4*>(tile_chunk(sP, tid, j));
+  for (int j = 0; j < AB_PIECES; ++j) gate_row[j] = *reinterpret_cast<const uint4*>(tile_chunk(sP, row, piece0 + j));
   if (ok) {
-    rope_tanh_row(sQ, tid, rope, true, false);
-    rope_tanh_row(sK, tid, rope, true, false);
+    rope_tanh_row(sQ, row, rope, true, false, piece0, AB_PIECES);
+    rope_tanh_row(sK, row, rope, true, false, piece0, AB_PIECES);
     // dmem/8 = dy * (1 - sigmoid(gate)) / 8  -> B3
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const uint4 dyq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, tid, j));
+    for (int j = 0; j < AB_PIECES; ++j) {
+      const uint4 dyq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, row, piece0 + j));
       const uint4 gq = gate_row[j];
       const __nv_bfloat162* dyb = reinterpret_cast<const __nv_bfloat162*>(&dyq);
       const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
@@ -539,7 +543,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
         const float2 gf = __bfloat1622float2(gb[t]);
         wo[t] = pack_bf16x2(dyv.x * (1.f - sigmoid_f(gf.x)) * 0.125f, dyv.y * (1.f - sigmoid_f(gf.y)) * 0.125f);
       }
-      *reinterpret_cast<uint4*>(tile_chunk(sB3, tid, j)) = o;
+      *reinterpret_cast<uint4*>(tile_chunk(sB3, row, piece0 + j)) = o;
     }
   }
   fence_proxy_async_smem();
@@ -570,45 +574,57 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
     tma_load_2d(sB3, &tm_qkvgu, &bars[2], 2 * d + h * HD, row0);
   }
 
-  // ---- softmax: max, sum, then normalised P (BF16) to smem
+  // ---- softmax over this thread's two blocks of columns, {half, half + 2} x 32, held in registers: one TMEM read and
+  // one exponential per score.  The two threads of a row meet once, with (max, sum) of their columns, in the State
+  // tile's space (the State has been consumed); a block behind the causal mask counts as (-inf, 0).
   const float kScale = 0.125f * 1.4426950408889634f;
-  const int last_chunk = warp;
-  float row_max = -INFINITY;
-  for (int cc = 0; cc <= last_chunk; ++cc) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
-    tmem_ld_wait();
+  float* meet = reinterpret_cast<float*>(sSt);   // [2][128] max | [2][128] sum | [2][128] D
+  float e[2][32];
+  float my_max = -INFINITY, my_sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (cc * 32 + j <= tid) row_max = fmaxf(row_max, __uint_as_float(r[j]));
-  }
-  float row_sum = 0.f;
-  for (int cc = 0; cc <= last_chunk; ++cc) {
-    uint32_t r[32];
-    tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-      if (cc * 32 + j <= tid) row_sum += exp2f((__uint_as_float(r[j]) - row_max) * kScale);
-  }
-  const float inv_l = 1.f / row_sum;
-  for (int cc = 0; cc < 4; ++cc) {
-    uint32_t pk[16];
-    if (cc <= last_chunk) {
+  for (int k = 0; k < 2; ++k) {
+    const int cc = half + 2 * k;
+    if (cc <= quarter) {
       uint32_t r[32];
       tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const float p0 = (cc * 32 + j <= tid) ? exp2f((__uint_as_float(r[j]) - row_max) * kScale) * inv_l : 0.f;
-        const float p1 = (cc * 32 + j + 1 <= tid) ? exp2f((__uint_as_float(r[j + 1]) - row_max) * kScale) * inv_l : 0.f;
-        pk[j >> 1] = pack_bf16x2(p0, p1);
+      for (int j = 0; j < 32; ++j) {
+        e[k][j] = cc * 32 + j <= row ? __uint_as_float(r[j]) : -INFINITY;
+        my_max = fmaxf(my_max, e[k][j]);
       }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (half + 2 * k <= quarter) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        e[k][j] = exp2f((e[k][j] - my_max) * kScale);
+        my_sum += e[k][j];
+      }
+    }
+  }
+  meet[half * 128 + row] = my_max;
+  meet[256 + half * 128 + row] = my_sum;
+  __syncthreads();
+  const float other_max = meet[(half ^ 1) * 128 + row];
+  const float row_max = fmaxf(my_max, other_max);
+  const float my_share = exp2f((my_max - row_max) * kScale);
+  const float row_sum = my_sum * my_share + meet[256 + (half ^ 1) * 128 + row] * exp2f((other_max - row_max) * kScale);
+  const float to_p = my_share / row_sum;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int cc = half + 2 * k;
+    uint32_t pk[16];
+    if (cc <= quarter) {
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) pk[j >> 1] = pack_bf16x2(e[k][j] * to_p, e[k][j + 1] * to_p);
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j) pk[j] = 0u;
     }
-    store_row_chunk32(sP, tid, cc * 32, pk);
+    store_row_chunk32(sP, row, cc * 32, pk);
   }
   tc_fence_before_sync();
   fence_proxy_async_smem();
@@ -632,17 +648,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   // ---- element-wise stage 1: dlocal = dy * g (in place in B2), dGate, D = sum(dlocal * local)
   float Drow = 0.f;
 #pragma unroll
-  for (int c = 0; c < HD; c += 16) {
+  for (int i = 0; i < AB_PIECES; i += 2) {
+    const int c = (piece0 + i) * 8;
     uint32_t ro[16], rm[16];
     tmem_ld_32x32b_x16(t_lo + lane_base + c, ro);
     tmem_ld_32x32b_x16(t_mid + lane_base + c, rm);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; j += 8) {
-      const int chunk = (c + j) >> 3;
-      uint4* pdl = reinterpret_cast<uint4*>(tile_chunk(sB2, tid, chunk));
+      const int mine = i + (j >> 3);
+      uint4* pdl = reinterpret_cast<uint4*>(tile_chunk(sB2, row, piece0 + mine));
       const uint4 dyq = *pdl;
-      const uint4 gq = gate_row[chunk];
+      const uint4 gq = gate_row[mine];
       const __nv_bfloat162* dyb = reinterpret_cast<const __nv_bfloat162*>(&dyq);
       const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
       uint4 o_dl, o_dg;
@@ -661,12 +678,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
         w_dg[t] = pack_bf16x2(dyv.x * (l0 - m0) * g0 * (1.f - g0), dyv.y * (l1 - m1) * g1 * (1.f - g1));
       }
       *pdl = o_dl;
-      dgate_row[chunk] = o_dg;
+      dgate_row[mine] = o_dg;
     }
   }
+  meet[512 + half * 128 + row] = Drow;
   tc_fence_before_sync();
   fence_proxy_async_smem();
   __syncthreads();
+  Drow += meet[512 + (half ^ 1) * 128 + row];
   // ---- MMA C: dP = dlocal V^T, dV = P^T dlocal
   if (tid == 0 && ok) {
     tc_fence_after_sync();
@@ -690,10 +709,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   }
 
   // ---- dS = P * (dP - D) / 8 over P; dV out; tanh(Kr) -> B3
-  for (int cc = 0; cc <= last_chunk; ++cc) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int cc = half + 2 * k;
+    if (cc > quarter) continue;
     uint32_t r[32], pk[16];
     tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
-    load_row_chunk32(sP, tid, cc * 32, pk);
+    load_row_chunk32(sP, row, cc * 32, pk);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
@@ -702,24 +724,24 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       const float s1 = pv.y * (__uint_as_float(r[2 * j + 1]) - Drow) * 0.125f;
       pk[j] = pack_bf16x2(s0, s1);
     }
-    store_row_chunk32(sP, tid, cc * 32, pk);
+    store_row_chunk32(sP, row, cc * 32, pk);
   }
 #pragma unroll
-  for (int c = 0; c < HD; c += 16) {
+  for (int i = 0; i < AB_PIECES; i += 2) {
     uint32_t rv[16];
-    tmem_ld_32x32b_x16(t_mid + lane_base + c, rv);
+    tmem_ld_32x32b_x16(t_mid + lane_base + (piece0 + i) * 8, rv);
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; j += 8) {
-      dv_row[(c + j) >> 3] = make_uint4(pack_bf16x2(__uint_as_float(rv[j]), __uint_as_float(rv[j + 1])),
+      dv_row[i + (j >> 3)] = make_uint4(pack_bf16x2(__uint_as_float(rv[j]), __uint_as_float(rv[j + 1])),
                                         pack_bf16x2(__uint_as_float(rv[j + 2]), __uint_as_float(rv[j + 3])),
                                         pack_bf16x2(__uint_as_float(rv[j + 4]), __uint_as_float(rv[j + 5])),
                                         pack_bf16x2(__uint_as_float(rv[j + 6]), __uint_as_float(rv[j + 7])));
     }
   }
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {  // tanh(Kr) -> B3 (V is no longer needed)
-    const uint4 kq = *reinterpret_cast<const uint4*>(tile_chunk(sK, tid, j));
+  for (int j = piece0; j < piece0 + AB_PIECES; ++j) {  // tanh(Kr) -> B3 (V is no longer needed)
+    const uint4 kq = *reinterpret_cast<const uint4*>(tile_chunk(sK, row, j));
     const __nv_bfloat162* kb = reinterpret_cast<const __nv_bfloat162*>(&kq);
     uint4 o;
     uint32_t* wo = reinterpret_cast<uint32_t*>(&o);
@@ -728,10 +750,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       const float2 kv = __bfloat1622float2(kb[t]);
       wo[t] = pack_bf16x2(tanh_fast(kv.x), tanh_fast(kv.y));
     }
-    *reinterpret_cast<uint4*>(tile_chunk(sB3, tid, j)) = o;
+    *reinterpret_cast<uint4*>(tile_chunk(sB3, row, j)) = o;
   }
   ok = mbar_wait(&bars[5], 0, abort_flag) && ok;  // U has landed
-  if (ok) rope_tanh_row(sB2, tid, rope, false, true);
+  if (ok) rope_tanh_row(sB2, row, rope, false, true, piece0, AB_PIECES);
   tc_fence_before_sync();
   fence_proxy_async_smem();
   __syncthreads();
@@ -764,7 +786,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 
   // ---- final: dQ, dK (RoPE transpose), dU
 #pragma unroll
-  for (int c = 0; c < HD; c += 16) {
+  for (int i = 0; i < AB_PIECES; i += 2) {
+    const int c = (piece0 + i) * 8;
     uint32_t rq[16], rk[16], rtk[16], rtu[16];
     tmem_ld_32x32b_x16(t_dq + lane_base + c, rq);
     tmem_ld_32x32b_x16(t_lo + lane_base + c, rk);
@@ -773,9 +796,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; j += 8) {
-      const int chunk = (c + j) >> 3;
-      const uint4 tkq = *reinterpret_cast<const uint4*>(tile_chunk(sB3, tid, chunk));
-      const uint4 tuq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, tid, chunk));
+      const int mine = i + (j >> 3), chunk = piece0 + mine;
+      const uint4 tkq = *reinterpret_cast<const uint4*>(tile_chunk(sB3, row, chunk));
+      const uint4 tuq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, row, chunk));
       const __nv_bfloat162* tkb = reinterpret_cast<const __nv_bfloat162*>(&tkq);
       const __nv_bfloat162* tub = reinterpret_cast<const __nv_bfloat162*>(&tuq);
       uint4 o_q, o_k, o_u;
@@ -785,7 +808,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const int e0 = j + 2 * t, e1 = e0 + 1;
-        const float2 cs = rope[((c + e0) >> 1) * CHUNK + tid];
+        const float2 cs = rope[((c + e0) >> 1) * CHUNK + row];
         const float2 tk = __bfloat1622float2(tkb[t]);
         const float2 tu = __bfloat1622float2(tub[t]);
         // y0 = x0 c - x1 s ; y1 = x1 c + x0 s   =>   dx0 = dy0 c + dy1 s ; dx1 = dy1 c - dy0 s
@@ -798,18 +821,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
                              __uint_as_float(rtu[e1]) * (1.f / CHUNK) * (1.f - tu.y * tu.y));
       }
       // every operand of the last MMA group has been consumed: Q, K, P, State and dW tiles are free
-      *reinterpret_cast<uint4*>(tile_chunk(sQ, tid, chunk)) = o_q;
-      *reinterpret_cast<uint4*>(tile_chunk(sK, tid, chunk)) = o_k;
-      *reinterpret_cast<uint4*>(tile_chunk(sP, tid, chunk)) = o_u;
-      *reinterpret_cast<uint4*>(tile_chunk(sP + TILE_BYTES, tid, chunk)) = dgate_row[chunk];
-      *reinterpret_cast<uint4*>(tile_chunk(sSt, tid, chunk)) = dv_row[chunk];
+      *reinterpret_cast<uint4*>(tile_chunk(sQ, row, chunk)) = o_q;
+      *reinterpret_cast<uint4*>(tile_chunk(sK, row, chunk)) = o_k;
+      *reinterpret_cast<uint4*>(tile_chunk(sP, row, chunk)) = o_u;
+      *reinterpret_cast<uint4*>(tile_chunk(sP + TILE_BYTES, row, chunk)) = dgate_row[mine];
+      *reinterpret_cast<uint4*>(tile_chunk(sSt, row, chunk)) = dv_row[mine];
     }
   }
   fence_proxy_async_smem();
-  __syncwarp();
-  if ((tid & 31) == 0) {  // one store per gradient tile for the warp's 32 token rows
+  // the two warps that share 32 token rows (immediate barrier numbers: a register would reserve all sixteen)
+  if (quarter == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+  else if (quarter == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+  else if (quarter == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+  else asm volatile("bar.sync 4, 64;" ::: "memory");
+  if (tid < 128 && (tid & 31) == 0) {  // one store per gradient tile for those rows
     if (ok) {
-      const int r = row0 + warp * 32, off = warp * 4096;
+      const int r = row0 + quarter * 32, off = quarter * 4096;
       tma_store_2d(&tm_dout, sQ + off, 0 * d + h * HD, r);
       tma_store_2d(&tm_dout, sK + off, 1 * d + h * HD, r);
       tma_store_2d(&tm_dout, sSt + off, 2 * d + h * HD, r);

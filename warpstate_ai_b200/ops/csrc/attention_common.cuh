@@ -35,11 +35,13 @@ __device__ __forceinline__ uint8_t* tile_chunk(uint8_t* tile, int r, int j) {
 
 // In place on row `r` of a tile: optional rotary embedding at in-chunk position r (pairs are
 // adjacent elements; rope[p*128 + r] = (cos, sin) of pair p at position r -- pair-major, so that
-// the 32 rows of a warp read 256 contiguous bytes instead of 32 cache lines), then optional tanh.
+// the 32 rows of a warp read 256 contiguous bytes instead of 32 cache lines), then optional tanh;
+// of the row's eight 16-byte pieces only `count` from `first` on.
 __device__ __forceinline__ void rope_tanh_row(uint8_t* tile, int r, const float2* __restrict__ rope,
-                                              bool do_rope, bool do_tanh) {
+                                              bool do_rope, bool do_tanh, int first = 0, int count = 8) {
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
+  for (int i = 0; i < count; ++i) {
+    const int j = first + i;
     uint4* p = reinterpret_cast<uint4*>(tile_chunk(tile, r, j));
     uint4 v = *p;
     uint32_t* w = reinterpret_cast<uint32_t*>(&v);
