@@ -260,8 +260,22 @@ decode_reduce_norm_kernel(float* __restrict__ x, const float* __restrict__ parti
                           float eps, int d, int batch, __nv_bfloat16* __restrict__ out) {
   __shared__ float red[8];
   pdl_launch_dependents();
-  pdl_wait();
   const int b = blockIdx.x;
+  // Up to HELD * 1024 columns stay in registers between the two passes; what no kernel of the step writes (norm weight,
+  // modulation) is requested before the wait for the previous kernel.
+  constexpr int HELD = 2;
+  float4 held[HELD], ww[HELD], sc[HELD], bi[HELD];
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    const int c = (threadIdx.x + i * 256) * 4;
+    if (c >= d) continue;
+    if (out != nullptr) ww[i] = *reinterpret_cast<const float4*>(w + c);
+    if (scale != nullptr) {
+      sc[i] = *reinterpret_cast<const float4*>(scale + c);
+      bi[i] = *reinterpret_cast<const float4*>(bias + c);
+    }
+  }
+  pdl_wait();
   float* xr = x + static_cast<size_t>(b) * d;
   const float* src = xr;
   if (token != nullptr) {
@@ -270,19 +284,34 @@ decode_reduce_norm_kernel(float* __restrict__ x, const float* __restrict__ parti
     if (id >= vocab) id = vocab - 1;
     src = table + static_cast<size_t>(id) * d;
   }
-  float ss = 0.f;
-  for (int c = threadIdx.x * 4; c < d; c += 256 * 4) {
+  auto updated = [&](int c, const float4& m, const float4& a) {
     float4 v = *reinterpret_cast<const float4*>(src + c);
     for (int s = 0; s < splits; ++s) {
       const float4 q = *reinterpret_cast<const float4*>(partial + (static_cast<size_t>(s) * batch + b) * d + c);
       v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
     }
     if (scale != nullptr) {
-      const float4 sc = *reinterpret_cast<const float4*>(scale + c), bi = *reinterpret_cast<const float4*>(bias + c);
-      v.x = v.x * (1.f + sc.x) + bi.x; v.y = v.y * (1.f + sc.y) + bi.y;
-      v.z = v.z * (1.f + sc.z) + bi.z; v.w = v.w * (1.f + sc.w) + bi.w;
+      v.x = v.x * (1.f + m.x) + a.x; v.y = v.y * (1.f + m.y) + a.y;
+      v.z = v.z * (1.f + m.z) + a.z; v.w = v.w * (1.f + m.w) + a.w;
     }
     *reinterpret_cast<float4*>(xr + c) = v;
+    return v;
+  };
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    const int c = (threadIdx.x + i * 256) * 4;
+    if (c >= d) continue;
+    held[i] = updated(c, sc[i], bi[i]);
+    ss += held[i].x * held[i].x + held[i].y * held[i].y + held[i].z * held[i].z + held[i].w * held[i].w;
+  }
+  for (int c = (threadIdx.x + HELD * 256) * 4; c < d; c += 256 * 4) {
+    float4 m = make_float4(0.f, 0.f, 0.f, 0.f), a = m;
+    if (scale != nullptr) {
+      m = *reinterpret_cast<const float4*>(scale + c);
+      a = *reinterpret_cast<const float4*>(bias + c);
+    }
+    const float4 v = updated(c, m, a);
     ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
   }
 #pragma unroll
@@ -294,14 +323,19 @@ decode_reduce_norm_kernel(float* __restrict__ x, const float* __restrict__ parti
   for (int i = 0; i < 8; ++i) total += red[i];
   const float rstd = rsqrtf(total / static_cast<float>(d) + eps);
   if (out == nullptr) return;
-  for (int c = threadIdx.x * 4; c < d; c += 256 * 4) {
-    const float4 v = *reinterpret_cast<const float4*>(xr + c);  // this thread's own stores
-    const float4 ww = *reinterpret_cast<const float4*>(w + c);
+  auto emit = [&](int c, const float4& v, const float4& g) {
     uint2 o;
-    o.x = pack_bf16x2(v.x * rstd * ww.x, v.y * rstd * ww.y);
-    o.y = pack_bf16x2(v.z * rstd * ww.z, v.w * rstd * ww.w);
+    o.x = pack_bf16x2(v.x * rstd * g.x, v.y * rstd * g.y);
+    o.y = pack_bf16x2(v.z * rstd * g.z, v.w * rstd * g.w);
     *reinterpret_cast<uint2*>(out + static_cast<size_t>(b) * d + c) = o;
+  };
+#pragma unroll
+  for (int i = 0; i < HELD; ++i) {
+    const int c = (threadIdx.x + i * 256) * 4;
+    if (c < d) emit(c, held[i], ww[i]);
   }
+  for (int c = (threadIdx.x + HELD * 256) * 4; c < d; c += 256 * 4)  // xr: this thread's own stores
+    emit(c, *reinterpret_cast<const float4*>(xr + c), *reinterpret_cast<const float4*>(w + c));
 }
 
 // --------------------------------------------------------------------------- attention step
@@ -320,7 +354,6 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.x % H, b = blockIdx.x / H;
   pdl_launch_dependents();
-  pdl_wait();
   int pos = static_cast<int>(*pos_ptr);
   pos = pos < 0 ? 0 : (pos >= C ? C - 1 : pos);
   const __nv_bfloat16* row = qkvgu + static_cast<size_t>(b) * 5 * d + h * HD;
@@ -328,6 +361,9 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
   // Thread (rg, jg) owns columns 8*jg .. 8*jg+7 of the rows rg, rg+16, ... of the K and V caches and of M: a warp
   // instruction reads four whole 128-byte rows.  Every load the step needs from the caches is issued here, before
   // the RoPE of the new token, so that the three dependent phases below (scores, softmax, P.V) wait for memory once.
+  // They are issued before the wait for the previous kernel, too, and run under the tail of the projection: the
+  // position, the cache rows before it and M are what the previous STEP left, and steps are separated by full
+  // dependencies (a graph replay, or the kernel that writes the position).  Only `row` is this step's.
   const int jg = tid & 7, rg = tid >> 3;
   uint4 kreg[C / 16], vreg[C / 16], mreg[HD / 16];
 #pragma unroll
@@ -336,16 +372,18 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
     if (c < pos) {
       kreg[it] = *reinterpret_cast<const uint4*>(kc + cache + static_cast<size_t>(c) * HD + jg * 8);
       vreg[it] = *reinterpret_cast<const uint4*>(vc + cache + static_cast<size_t>(c) * HD + jg * 8);
-    } else if (c == pos) {
-      vreg[it] = *reinterpret_cast<const uint4*>(row + 2 * d + jg * 8);  // the new token's own value row
     }
   }
   const __nv_bfloat16* mbase = mixed + (static_cast<size_t>(b) * H + h) * HD * HD;
 #pragma unroll
   for (int it = 0; it < HD / 16; ++it) mreg[it] = *reinterpret_cast<const uint4*>(mbase + (rg + it * 16) * HD + jg * 8);
+  const float2 cs = rope[pos * 32 + lane];
+  pdl_wait();
+#pragma unroll
+  for (int it = 0; it < C / 16; ++it)
+    if (rg + it * 16 == pos) vreg[it] = *reinterpret_cast<const uint4*>(row + 2 * d + jg * 8);  // the new token's own value row
   // RoPE (adjacent pairs) of q and k; append k, v, u at `pos`
   if (tid < 32) {
-    const float2 cs = rope[pos * 32 + tid];
     const float2 q = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + 2 * tid));
     const float2 k = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(row + d + 2 * tid));
     // round through BF16 as the cached / batched path does
