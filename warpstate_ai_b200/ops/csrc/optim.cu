@@ -14,15 +14,15 @@ extern "C" void ws_count_launch(void);
 
 constexpr int OPT_THREADS = 256;
 
-__device__ __forceinline__ float block_sum(float v, float* smem) {
+__device__ __forceinline__ double block_sum(double v, double* smem) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0) smem[warp] = v;
   __syncthreads();
-  float s = 0.f;
+  double s = 0.0;
   if (warp == 0) {
-    s = lane < (blockDim.x >> 5) ? smem[lane] : 0.f;
+    s = lane < (blockDim.x >> 5) ? smem[lane] : 0.0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   }
@@ -30,22 +30,29 @@ __device__ __forceinline__ float block_sum(float v, float* smem) {
   return s;  // valid in warp 0
 }
 
-// partial[block] = sum of squares of a fixed, contiguous slice of g (slice size is a function
-// of n and gridDim only, so the summation order is reproducible).
+// Sum of squares of a fixed, contiguous slice of g per block (slice size is a function of n and gridDim only, so the
+// summation order is reproducible).  Four squares are added in FP32 and everything above them in FP64: arenas that hold
+// the same gradients in another order (sharded, replicated) then agree on the norm to the last bit, where FP32 sums
+// left them an ulp apart, and a clip coefficient an ulp apart turns into other signs of near-zero AdamW steps.  The
+// block's sum leaves as two floats, partial[block] + partial[gridDim + block].  Still bound by the 4 bytes per element.
 __global__ void __launch_bounds__(OPT_THREADS)
 sumsq_kernel(const float* __restrict__ g, size_t n4, float* __restrict__ partial) {
-  __shared__ float red[32];
+  __shared__ double red[32];
   const size_t per_block = (n4 + gridDim.x - 1) / gridDim.x;
   const size_t begin = per_block * blockIdx.x;
   size_t end = begin + per_block;
   if (end > n4) end = n4;
-  float s = 0.f;
+  double s = 0.0;
   for (size_t i = begin + threadIdx.x; i < end; i += OPT_THREADS) {
     const float4 v = reinterpret_cast<const float4*>(g)[i];
-    s += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    s += static_cast<double>(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
   }
   s = block_sum(s, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (threadIdx.x == 0) {
+    const float high = static_cast<float>(s);
+    partial[blockIdx.x] = high;
+    partial[gridDim.x + blockIdx.x] = static_cast<float>(s - static_cast<double>(high));
+  }
 }
 
 __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
@@ -58,12 +65,13 @@ __device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x)
 // `extra_sumsq` (optional) is added first: other ranks' shares when the gradient is sharded.
 __global__ void clip_coef_kernel(const float* __restrict__ partial, int parts, const float* extra_sumsq,
                                  float max_norm, const int* __restrict__ status, float* __restrict__ stats) {
-  __shared__ float red[32];
-  float s = 0.f;
-  for (int i = threadIdx.x; i < parts; i += blockDim.x) s += partial[i];
-  s = block_sum(s, red);
+  __shared__ double red[32];
+  double sum = 0.0;
+  for (int i = threadIdx.x; i < parts; i += blockDim.x) sum += static_cast<double>(partial[i]);
+  sum = block_sum(sum, red);
   if (threadIdx.x == 0) {
-    if (extra_sumsq != nullptr) s += *extra_sumsq;
+    if (extra_sumsq != nullptr) sum += static_cast<double>(*extra_sumsq);
+    const float s = static_cast<float>(sum);   // past FP32 it is infinite, and the update is skipped
     const float norm = __fsqrt_rn(s);
     float coef = max_norm > 0.f ? __fdiv_rn(max_norm, norm + 1e-6f) : 1.0f;
     if (coef > 1.0f) coef = 1.0f;
@@ -125,14 +133,15 @@ adamw_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restri
 
 using namespace ws;
 
-extern "C" int ws_sumsq_parts(void) { return 148 * 8; }
+constexpr int SUMSQ_BLOCKS = 148 * 8;
+extern "C" int ws_sumsq_parts(void) { return 2 * SUMSQ_BLOCKS; }
 
 // stats: 4 floats on the device.  partial: ws_sumsq_parts() floats of scratch.
 extern "C" int ws_grad_norm_clip(const float* g, size_t n, float* partial, const float* extra_sumsq,
                                  float max_norm, const int* status, float* stats, cudaStream_t stream) {
   if (n % 4 != 0) return -1;
   const int parts = ws_sumsq_parts();
-  sumsq_kernel<<<parts, OPT_THREADS, 0, stream>>>(g, n / 4, partial);
+  sumsq_kernel<<<SUMSQ_BLOCKS, OPT_THREADS, 0, stream>>>(g, n / 4, partial);
   ws_count_launch();
   clip_coef_kernel<<<1, 256, 0, stream>>>(partial, parts, extra_sumsq, max_norm, status, stats);
   ws_count_launch();
