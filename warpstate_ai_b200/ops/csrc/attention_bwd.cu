@@ -327,15 +327,20 @@ constexpr int SCAN_MAX_CHUNKS = SCAN_GROUP * SCAN_MAX_GROUPS;  // 32768 tokens p
 
 // dstate [B,N,H,4096] FP32 (gradient of the mixed state read by chunk n), writes [B,N,H,4096] FP32
 // -> dwrites [B,N,H,4096] BF16 and partial sums [B*H*16][3] of d(fast decay), d(slow decay), d(mix).
-__global__ void __launch_bounds__(256)
+// A thread owns two neighbouring state elements (8-byte loads of the writes and of the state gradients, 4-byte stores):
+// half the memory instructions of the one-element form, and 256 bytes in flight per thread.
+constexpr int SCAN_THREADS = 128;
+constexpr int SCAN_VEC = 2;
+
+__global__ void __launch_bounds__(SCAN_THREADS, 3)
 memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict__ writes,
                        const float* __restrict__ fast_logit, const float* __restrict__ slow_logit,
                        const float* __restrict__ mix_logit, __nv_bfloat16* __restrict__ dwrites,
                        float* __restrict__ partials, int B, int N, int H) {
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float red[3][8];
-  const size_t idx = blockIdx.x * static_cast<size_t>(256) + threadIdx.x;  // over B*H*4096 (exact multiple)
+  __shared__ float red[3][SCAN_THREADS / 32];
+  const size_t idx = (blockIdx.x * static_cast<size_t>(SCAN_THREADS) + threadIdx.x) * SCAN_VEC;  // over B*H*4096 (exact multiple)
   const int e = idx % 4096;
   const int h = (idx / 4096) % H;
   const int b = idx / (4096 * static_cast<size_t>(H));
@@ -343,59 +348,65 @@ memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict
   const float ds = 1.f / (1.f + expf(-slow_logit[h]));
   const float mix = 1.f / (1.f + expf(-mix_logit[h]));
   const size_t chunk_stride = static_cast<size_t>(H) * 4096;
-  const size_t base = (static_cast<size_t>(b) * N * H + h) * 4096 + e;  // chunk 0 of this element
+  const size_t base = (static_cast<size_t>(b) * N * H + h) * 4096 + e;  // chunk 0 of these elements
   const int groups = (N + SCAN_GROUP - 1) / SCAN_GROUP;
-  float start_f[SCAN_MAX_GROUPS], start_s[SCAN_MAX_GROUPS];
+  float2 start_f[SCAN_MAX_GROUPS], start_s[SCAN_MAX_GROUPS];
+  auto advance = [&](float2& f, float2& s, const float2& w) {
+    f.x = df * f.x + (1.f - df) * w.x;
+    f.y = df * f.y + (1.f - df) * w.y;
+    s.x = ds * s.x + (1.f - ds) * w.x;
+    s.y = ds * s.y + (1.f - ds) * w.y;
+  };
   {
-    float f = 0.f, s = 0.f;
+    float2 f = make_float2(0.f, 0.f), s = f;
 #pragma unroll 1
     for (int g = 0; g < groups; ++g) {
       start_f[g] = f;
       start_s[g] = s;
       if (g + 1 < groups) {
 #pragma unroll
-        for (int i = 0; i < SCAN_GROUP; ++i) {
-          const float w = writes[base + (g * SCAN_GROUP + i) * chunk_stride];
-          f = df * f + (1.f - df) * w;
-          s = ds * s + (1.f - ds) * w;
-        }
+        for (int i = 0; i < SCAN_GROUP; ++i)
+          advance(f, s, *reinterpret_cast<const float2*>(writes + base + (g * SCAN_GROUP + i) * chunk_stride));
       }
     }
   }
   // a, bb: gradients of the fast and slow state AFTER the chunk being visited (F_{n+1}, S_{n+1})
-  float a = 0.f, bb = 0.f, g_df = 0.f, g_ds = 0.f, g_mix = 0.f;
+  float2 a = make_float2(0.f, 0.f), bb = a;
+  float g_df = 0.f, g_ds = 0.f, g_mix = 0.f;
 #pragma unroll 1
   for (int g = groups - 1; g >= 0; --g) {
     const int n0 = g * SCAN_GROUP;
     const int count = min(SCAN_GROUP, N - n0);
     // every load of the group is requested before its recurrences run: 2 x SCAN_GROUP independent loads in flight
-    float F[SCAN_GROUP], S[SCAN_GROUP], W[SCAN_GROUP], G[SCAN_GROUP];
+    float2 F[SCAN_GROUP], S[SCAN_GROUP], W[SCAN_GROUP], G[SCAN_GROUP];
 #pragma unroll
     for (int i = 0; i < SCAN_GROUP; ++i) {
       if (i < count) {
-        W[i] = writes[base + (n0 + i) * chunk_stride];
-        G[i] = dstate[base + (n0 + i) * chunk_stride];
+        W[i] = *reinterpret_cast<const float2*>(writes + base + (n0 + i) * chunk_stride);
+        G[i] = *reinterpret_cast<const float2*>(dstate + base + (n0 + i) * chunk_stride);
       }
     }
-    float f = start_f[g], s = start_s[g];
+    float2 f = start_f[g], s = start_s[g];
 #pragma unroll
     for (int i = 0; i < SCAN_GROUP; ++i) {  // forward: state seen by chunk n0 + i
       if (i < count) {
         F[i] = f;
         S[i] = s;
-        f = df * f + (1.f - df) * W[i];
-        s = ds * s + (1.f - ds) * W[i];
+        advance(f, s, W[i]);
       }
     }
 #pragma unroll
     for (int i = SCAN_GROUP - 1; i >= 0; --i) {
       if (i < count) {
-        dwrites[base + (n0 + i) * chunk_stride] = __float2bfloat16_rn((1.f - df) * a + (1.f - ds) * bb);
-        g_df += a * (F[i] - W[i]);    // F_{n+1} = df F_n + (1 - df) w_n
-        g_ds += bb * (S[i] - W[i]);
-        g_mix += G[i] * (F[i] - S[i]);
-        a = mix * G[i] + df * a;      // gradient of F_n
-        bb = (1.f - mix) * G[i] + ds * bb;
+        *reinterpret_cast<uint32_t*>(dwrites + base + (n0 + i) * chunk_stride) =
+            pack_bf16x2((1.f - df) * a.x + (1.f - ds) * bb.x, (1.f - df) * a.y + (1.f - ds) * bb.y);
+        g_df += a.x * (F[i].x - W[i].x) + a.y * (F[i].y - W[i].y);    // F_{n+1} = df F_n + (1 - df) w_n
+        g_ds += bb.x * (S[i].x - W[i].x) + bb.y * (S[i].y - W[i].y);
+        g_mix += G[i].x * (F[i].x - S[i].x) + G[i].y * (F[i].y - S[i].y);
+        a.x = mix * G[i].x + df * a.x;      // gradient of F_n
+        a.y = mix * G[i].y + df * a.y;
+        bb.x = (1.f - mix) * G[i].x + ds * bb.x;
+        bb.y = (1.f - mix) * G[i].y + ds * bb.y;
       }
     }
   }
@@ -413,7 +424,7 @@ memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict
   if (threadIdx.x < 3) {
     float v = 0.f;
 #pragma unroll
-    for (int wi = 0; wi < 8; ++wi) v += red[threadIdx.x][wi];
+    for (int wi = 0; wi < SCAN_THREADS / 32; ++wi) v += red[threadIdx.x][wi];
     partials[static_cast<size_t>(blockIdx.x) * 3 + threadIdx.x] = v;
   }
 }
@@ -899,7 +910,7 @@ extern "C" int ws_memory_scan_bwd(const float* dstate, const float* writes, cons
                                   int B, int N, int H, cudaStream_t stream) {
   if (N > SCAN_MAX_CHUNKS) return -1;
   const size_t total = (size_t)B * H * 4096;
-  launch_dependent(memory_scan_bwd_kernel, dim3((unsigned)(total / 256)), dim3(256), 0, stream, dstate, writes, fast_logit, slow_logit,
+  launch_dependent(memory_scan_bwd_kernel, dim3((unsigned)(total / (SCAN_THREADS * SCAN_VEC))), dim3(SCAN_THREADS), 0, stream, dstate, writes, fast_logit, slow_logit,
                                                                       mix_logit, (__nv_bfloat16*)dwrites, partials,
                                                                       B, N, H);
   ws_count_launch();
