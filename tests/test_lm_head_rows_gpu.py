@@ -63,3 +63,36 @@ def test_head_over_labelled_rows(rows, d, vocab, kind):
     hidden.grad = None
     (lmhead.token_logps(hidden, weight, labels) * coef).sum().backward()
     assert torch.equal(hidden.grad, first) and rel(weight.grad, 2 * w32.grad if keep.any() else weight.grad) < 0.02
+
+
+@pytest.mark.parametrize("rows,kept,kind", [(777, 777, 777), (777, 777, 300), (777, 256, 777), (777, 512, 257), (9000, 256, "random"),
+                                            (9000, 0, "random")])
+def test_kept_logits_give_the_bits_of_recomputed_ones(monkeypatch, rows, kept, kind):
+    """Logit gradients from kept logits, from recomputed ones, and from both in one pass; a second backward over the same
+    graph recomputes what the first consumed."""
+    _ext.require()
+    torch.manual_seed(rows + kept)
+    d, vocab = 256, 1000
+    hidden = torch.randn(rows, d, device="cuda").bfloat16()
+    labels, keep = labels_with(kind, rows, vocab)
+    weight = torch.randn(vocab, d, device="cuda") * 0.05
+    coef = torch.randn(rows, device="cuda")
+
+    def gradients(keep_bytes, passes=1):
+        monkeypatch.setattr(lmhead, "KEEP_BYTES", keep_bytes)
+        h, w = hidden.clone().requires_grad_(True), weight.clone().requires_grad_(True)
+        value = (lmhead.token_logps(h, w, labels) * coef).sum()
+        for index in range(passes):
+            h.grad = w.grad = None
+            value.backward(retain_graph=index + 1 < passes)
+        check_device_errors()
+        return h.grad, w.grad
+
+    assert lmhead.kept_rows(rows, vocab) == rows
+    recomputed = gradients(0)
+    monkeypatch.setattr(lmhead, "KEEP_BYTES", 2 * vocab * kept)
+    assert lmhead.kept_rows(rows, vocab) == kept
+    mine, twice = gradients(2 * vocab * kept), gradients(2 * vocab * kept, passes=2)
+    assert torch.equal(mine[0], recomputed[0]) and torch.equal(twice[0], recomputed[0])
+    # the weight gradient is added up over blocks of rows, which end elsewhere: FP32 additions in another order
+    assert rel(mine[1], recomputed[1]) < 1e-5 and rel(twice[1], recomputed[1]) < 1e-5

@@ -627,11 +627,13 @@ std::tuple<at::Tensor, at::Tensor> lm_head_fwd(const at::Tensor& hidden, const a
 }
 
 // The same over the labelled rows only, which are packed together on the device (see lmhead.cu).  Returns
-// (logp [rows], lse of the packed rows, index, count, hidden packed, labels packed); what backward needs of them goes
-// to lm_head_bwd_labelled.
-std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> lm_head_fwd_labelled(
-    const at::Tensor& hidden, const at::Tensor& weight, const at::Tensor& labels, int64_t ignore_index,
-    const c10::optional<at::Tensor>& error_flag) {
+// (logp [rows], lse of the packed rows, index, count, hidden packed, labels packed, BF16 logits of the first keep_rows
+// packed rows); what backward needs of them goes to lm_head_bwd_labelled.
+std::vector<at::Tensor> lm_head_fwd_labelled(const at::Tensor& hidden, const at::Tensor& weight, const at::Tensor& labels,
+                                             int64_t ignore_index, int64_t keep_rows,
+                                             const c10::optional<at::Tensor>& error_flag) {
+  TORCH_CHECK(keep_rows >= 0 && keep_rows <= hidden.size(0) && (keep_rows == 0 || weight.size(0) % 8 == 0),
+              "lm_head_fwd_labelled: keep_rows");
   TORCH_CHECK(hidden.is_cuda() && hidden.scalar_type() == at::kBFloat16 && hidden.dim() == 2 && hidden.is_contiguous() &&
               hidden.size(1) % 8 == 0 && reinterpret_cast<uintptr_t>(hidden.data_ptr()) % 16 == 0,
               "lm_head_fwd_labelled: hidden must be contiguous BF16 [rows, d], d % 8 == 0");
@@ -672,20 +674,23 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tenso
   g.error_flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
   g.limit = count.data_ptr<int>();
   g.whole = hidden.data_ptr(); g.whole_rows = rows; g.ldwhole = d;
+  at::Tensor logits = at::empty({keep_rows, vocab}, hidden.options());
+  if (keep_rows > 0) { g.keep = logits.data_ptr(); g.keep_rows = (int)keep_rows; }
   check_rc(ws_gemm(&g, cur_stream()), "lm_head_fwd_labelled gemm");
   check_rc(ws_ce_combine(parts.data_ptr(), ld, nparts, label_logit, lab, (long long)ignore_index, rows,
                          index.data_ptr<int>(), count.data_ptr<int>(), lse.data_ptr<float>(), logp.data_ptr<float>(),
                          cur_stream()), "ce_combine");
-  return {logp, lse, index, count, packed, labels_sel};
+  return {logp, lse, index, count, packed, labels_sel, logits};
 }
 
 // dhidden [rows, d] (every row written) and grad_weight [vocab, d] += of sum(row_weight * -logp), the rows in blocks of
-// `block`: logits recomputed into dlogits, then the two products.  row_weight is per row before the selection.
+// `block`: the logit gradients, from the kept logits in place (`logits` is consumed) or past its rows from logits that
+// are computed again, then the two products.  row_weight is per row before the selection.
 void lm_head_bwd_labelled(const at::Tensor& hidden, const at::Tensor& packed, const at::Tensor& weight,
                           const at::Tensor& labels, const at::Tensor& labels_sel, const at::Tensor& index,
                           const at::Tensor& count, const at::Tensor& lse, const at::Tensor& row_weight,
-                          int64_t ignore_index, int64_t block, at::Tensor dhidden, at::Tensor grad_weight,
-                          const c10::optional<at::Tensor>& error_flag) {
+                          int64_t ignore_index, int64_t block, at::Tensor logits, at::Tensor dhidden,
+                          at::Tensor grad_weight, const c10::optional<at::Tensor>& error_flag) {
   const int rows = (int)hidden.size(0), d = (int)hidden.size(1), vocab = (int)weight.size(0);
   TORCH_CHECK(hidden.is_cuda() && hidden.scalar_type() == at::kBFloat16 && hidden.is_contiguous() &&
               packed.scalar_type() == at::kBFloat16 && packed.is_contiguous() && packed.sizes() == hidden.sizes() &&
@@ -704,27 +709,42 @@ void lm_head_bwd_labelled(const at::Tensor& hidden, const at::Tensor& packed, co
   c10::cuda::CUDAGuard guard(hidden.device());
   check_rc(ws_clear_unlabelled(reinterpret_cast<const long long*>(labels.data_ptr<int64_t>()), (long long)ignore_index,
                                rows, d, dhidden.data_ptr(), cur_stream()), "clear_unlabelled");
-  at::Tensor dlogits = at::empty({std::min<int64_t>(block, rows), vocab}, hidden.options());
+  const int64_t kept = logits.numel() / vocab;
+  TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && logits.is_contiguous() && logits.numel() == kept * vocab &&
+              (kept == rows || (kept < rows && kept % 256 == 0)),
+              "lm_head_bwd_labelled: logits must be contiguous BF16 [kept rows, vocab]");
+  at::Tensor scratch;
   int* flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
-  for (int start = 0; start < rows; start += (int)block) {
-    const int here = std::min((int)block, rows - start);
+  for (int start = 0, here = 0; start < rows; start += here) {
+    const bool have = start < kept;   // the kept rows are one block: the weight gradient is read and written once for them
+    here = have ? (int)kept : std::min((int)block, rows - start);
     const auto from_start = [&](const at::Tensor& t) { return t.data_ptr<at::BFloat16>() + static_cast<int64_t>(start) * d; };
-    WsGemm g = {};
-    g.a = from_start(packed); g.b = weight.data_ptr();
-    g.m = here; g.n = vocab; g.k = d;
-    g.lda = d; g.ldb = d;
-    g.epilogue = WS_EPI_CE_BWD;
-    g.out = dlogits.data_ptr(); g.ldo = vocab;
-    g.aux = labels_sel.data_ptr<int64_t>() + start;
-    g.row_scale = row_weight.data_ptr<float>(); g.row_vec = lse.data_ptr<float>() + start;
-    g.row_map = index.data_ptr<int>() + start;
-    g.alpha = 1.f;
-    g.error_flag = flag;
-    g.limit = count.data_ptr<int>(); g.limit_from = start;
-    g.whole = from_start(hidden); g.whole_rows = rows; g.ldwhole = d;
-    check_rc(ws_gemm(&g, cur_stream()), "lm_head_bwd_labelled dlogits");
+    void* dlogits;
+    if (have) {
+      dlogits = logits.data_ptr<at::BFloat16>() + static_cast<int64_t>(start) * vocab;
+      check_rc(ws_ce_dlogits(dlogits, vocab, reinterpret_cast<const long long*>(labels_sel.data_ptr<int64_t>()) + start,
+                             index.data_ptr<int>() + start, lse.data_ptr<float>() + start, row_weight.data_ptr<float>(),
+                             count.data_ptr<int>(), start, here, cur_stream()), "ce_dlogits");
+    } else {
+      if (!scratch.defined()) scratch = at::empty({std::min<int64_t>(block, rows), vocab}, hidden.options());
+      dlogits = scratch.data_ptr();
+      WsGemm g = {};
+      g.a = from_start(packed); g.b = weight.data_ptr();
+      g.m = here; g.n = vocab; g.k = d;
+      g.lda = d; g.ldb = d;
+      g.epilogue = WS_EPI_CE_BWD;
+      g.out = dlogits; g.ldo = vocab;
+      g.aux = labels_sel.data_ptr<int64_t>() + start;
+      g.row_scale = row_weight.data_ptr<float>(); g.row_vec = lse.data_ptr<float>() + start;
+      g.row_map = index.data_ptr<int>() + start;
+      g.alpha = 1.f;
+      g.error_flag = flag;
+      g.limit = count.data_ptr<int>(); g.limit_from = start;
+      g.whole = from_start(hidden); g.whole_rows = rows; g.ldwhole = d;
+      check_rc(ws_gemm(&g, cur_stream()), "lm_head_bwd_labelled dlogits");
+    }
     WsGemm x = {};
-    x.a = dlogits.data_ptr(); x.b = weight.data_ptr();
+    x.a = dlogits; x.b = weight.data_ptr();
     x.m = here; x.n = d; x.k = vocab;
     x.lda = vocab; x.ldb = d;
     x.b_mn = 1;
@@ -736,7 +756,7 @@ void lm_head_bwd_labelled(const at::Tensor& hidden, const at::Tensor& packed, co
     x.limit = count.data_ptr<int>(); x.limit_from = start;
     check_rc(ws_gemm(&x, cur_stream()), "lm_head_bwd_labelled dhidden");
     WsGemm w = {};
-    w.a = dlogits.data_ptr(); w.b = from_start(packed);
+    w.a = dlogits; w.b = from_start(packed);
     w.m = vocab; w.n = d; w.k = here;
     w.lda = vocab; w.ldb = d;
     w.a_mn = 1; w.b_mn = 1;
@@ -1156,11 +1176,11 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("embed_bwd(Tensor dx, Tensor ids, Tensor(a!) grad_table) -> ()");
   m.def("launch_count() -> int");
   m.def("lm_head_fwd(Tensor hidden, Tensor weight, Tensor labels, int ignore_index, Tensor(a!)? error_flag) -> (Tensor, Tensor)");
-  m.def("lm_head_fwd_labelled(Tensor hidden, Tensor weight, Tensor labels, int ignore_index, Tensor(a!)? error_flag) -> "
-        "(Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
+  m.def("lm_head_fwd_labelled(Tensor hidden, Tensor weight, Tensor labels, int ignore_index, int keep_rows, "
+        "Tensor(a!)? error_flag) -> Tensor[]");
   m.def("lm_head_bwd_labelled(Tensor hidden, Tensor packed, Tensor weight, Tensor labels, Tensor labels_sel, Tensor index, "
-        "Tensor count, Tensor lse, Tensor row_weight, int ignore_index, int block, Tensor(a!) dhidden, "
-        "Tensor(b!) grad_weight, Tensor(c!)? error_flag) -> ()");
+        "Tensor count, Tensor lse, Tensor row_weight, int ignore_index, int block, Tensor(a!) logits, "
+        "Tensor(b!) dhidden, Tensor(c!) grad_weight, Tensor(d!)? error_flag) -> ()");
   m.def("gemm_pair_available() -> bool");
   m.def("lm_head_dlogits(Tensor hidden, Tensor weight, Tensor labels, Tensor lse, Tensor row_weight, Tensor(a!)? error_flag) -> Tensor");
   m.def("grad_allreduce(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int start, int count, "

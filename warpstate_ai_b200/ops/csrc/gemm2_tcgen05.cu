@@ -728,6 +728,7 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
   p.error_flag = g->error_flag;
   p.limit = g->limit; p.limit_from = g->limit_from;
   p.row_map = g->row_map;
+  p.keep = g->keep; p.keep_rows = g->keep_rows < g->m ? g->keep_rows : g->m;
   p.whole_rows = g->whole != nullptr ? g->whole_rows : -1;
   p.debug = 0;
   if (g->whole != nullptr) {  // the same boxes over the rows before their selection: A, or B of a weight gradient

@@ -27,6 +27,8 @@ struct GemmParams {
   int limit_from;
   const int* row_map;
   int whole_rows;
+  void* keep;          // CE_FWD: see WsGemm
+  int keep_rows;
   int debug;  // experiment switch: 1 = no loads (MMA issue rate only), 2 = always load tile (0,0)
 };
 
@@ -259,6 +261,17 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, uint32_t tadd
         r[j] = __float_as_uint(v);
         cm = fmaxf(cm, v);
         if (n0 + c + j == lab) reinterpret_cast<float*>(p.out2)[row] = v;
+      }
+      if (p.keep != nullptr && row < p.keep_rows) {
+        __nv_bfloat16* kept = reinterpret_cast<__nv_bfloat16*>(p.keep) + static_cast<size_t>(row) * p.n + n0 + c;
+#pragma unroll
+        for (int j = 0; j < 32; j += 8)
+          if (n0 + c + j < p.n)
+            *reinterpret_cast<uint4*>(kept + j) =
+                make_uint4(pack_bf16x2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])),
+                           pack_bf16x2(__uint_as_float(r[j + 2]), __uint_as_float(r[j + 3])),
+                           pack_bf16x2(__uint_as_float(r[j + 4]), __uint_as_float(r[j + 5])),
+                           pack_bf16x2(__uint_as_float(r[j + 6]), __uint_as_float(r[j + 7])));
       }
       const float nm = fmaxf(mx, cm);
       float cs = 0.f;

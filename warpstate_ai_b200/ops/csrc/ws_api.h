@@ -51,6 +51,8 @@ typedef struct WsGemm {
   const int* limit;
   int limit_from;
   const int* row_map;  // BF16: output row of row m; CE_BWD: its index into row_scale; < 0: none
+  void* keep;          // CE_FWD: BF16 logits of the first keep_rows rows, [keep_rows, n] (may be NULL)
+  int keep_rows;
   const void* whole;   // replaces A (a_mn: B) where *limit == whole_rows: the rows before their selection
   int whole_rows, ldwhole;
 } WsGemm;
@@ -213,6 +215,11 @@ int ws_select_rows(const long long* labels, long long ignore_index, int rows, in
 // out[r] = in[index[r]] for r < *count, zeros up to the next multiple of 256; nothing where *count == rows.
 int ws_gather_rows(const void* in, int ld, const int* index, const int* count, int rows, int d, void* out,
                    cudaStream_t stream);
+// In place on `rows` rows of kept BF16 logits [rows, vocab], the selected rows from `start` on: dlogits =
+// (exp(logit - lse[r]) - onehot(labels_sel[r])) * row_weight[index[r]] for start + r < *count, zeros up to the next
+// multiple of 64; the others are left alone.  labels_sel, index and lse are those of the rows from `start` on.
+int ws_ce_dlogits(void* logits, int vocab, const long long* labels_sel, const int* index, const float* lse,
+                  const float* row_weight, const int* count, int start, int rows, cudaStream_t stream);
 // Zeros in the rows of out whose label is `ignore_index`.
 int ws_clear_unlabelled(const long long* labels, long long ignore_index, int rows, int d, void* out,
                         cudaStream_t stream);

@@ -8,7 +8,9 @@ states) and the dW GEMM (FP32 accumulation into the tied embedding's gradient).
 
 An unlabelled row (-100: prompts and padding, most of a post-training batch) adds nothing to either pass, so from
 `SELECT_FROM` rows on the labelled rows are packed together on the device and the GEMMs run over them alone; their
-number is read by the kernels, not by the host.  Where every row is labelled nothing is copied.
+number is read by the kernels, not by the host.  Where every row is labelled nothing is copied.  When a backward pass
+will follow, the forward pass leaves the BF16 logits of up to `KEEP_BYTES` worth of rows behind, from which the logit
+gradients are formed in place; the rows past them are recomputed, block by block.
 
 `loss_sum` is the summed cross-entropy over labels != -100 (reference warpstate/model.py:316-334,
 ops/loss_experiment.py:14-19); `token_logps` is the per-row label log-probability used for
@@ -25,6 +27,15 @@ IGNORE = -100
 # Below one tile of the CTA-pair GEMM there is nothing to leave out, and the single-CTA kernel is the faster one.
 SELECT_FROM = 512
 ROWS_PER_BLOCK = 8192  # bounds the BF16 dlogits scratch to 512 MiB at vocab 32768
+# Logits kept between the passes: 16384 rows at vocab 32768, the micro-batch of the production run.  They live from the
+# head's forward to its backward, which follows at once, and there they are the logit gradients' buffer.
+KEEP_BYTES = 1 << 30
+
+
+def kept_rows(rows: int, vocab: int) -> int:
+    """Rows whose logits are kept: all of them, or as many whole tiles of 256 as `KEEP_BYTES` hold."""
+    most = KEEP_BYTES // (2 * vocab)
+    return rows if rows <= most else most // 256 * 256
 
 
 def kernels_ready(hidden: torch.Tensor, weight: torch.Tensor) -> bool:
@@ -36,7 +47,7 @@ class _TokenLogps(torch.autograd.Function):
     """per-row log p(label) (0 where the label is -100); differentiable w.r.t. hidden and weight."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, labels):
+    def forward(ctx, hidden, weight, labels, keep):
         from .fused import bf16_weight
         ops = torch.ops.ws_b200
         hidden = hidden.contiguous()
@@ -46,7 +57,8 @@ class _TokenLogps(torch.autograd.Function):
         ctx.weight = weight
         ctx.selected = hidden.shape[0] >= SELECT_FROM and ops.gemm_pair_available()
         if ctx.selected:
-            logp, *rest = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, flag)
+            keep = kept_rows(hidden.shape[0], wb.shape[0]) if keep else 0
+            logp, *rest, ctx.logits = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, keep, flag)
             ctx.save_for_backward(hidden, labels, *rest)
             return logp
         lse, logp = ops.lm_head_fwd(hidden, wb, labels, IGNORE, flag)
@@ -68,20 +80,23 @@ class _TokenLogps(torch.autograd.Function):
         grad_w = main if main is not None else torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
         if ctx.selected:
             index, count, packed, labels_sel = selection
+            # the logits become their own gradients: another backward over the same graph computes them again
+            logits, ctx.logits = ctx.logits, ctx.logits.new_empty(0)
             ops.lm_head_bwd_labelled(hidden, packed, wb, labels, labels_sel, index, count, lse, row_weight, IGNORE,
-                                     ROWS_PER_BLOCK, dh, grad_w, flag)
-            return dh, (None if main is not None else grad_w.to(weight.dtype)), None
+                                     ROWS_PER_BLOCK, logits, dh, grad_w, flag)
+            return dh, (None if main is not None else grad_w.to(weight.dtype)), None, None
         for start in range(0, hidden.shape[0], ROWS_PER_BLOCK):
             stop = min(start + ROWS_PER_BLOCK, hidden.shape[0])
             h = hidden[start:stop]
             dlogits = ops.lm_head_dlogits(h, wb, labels[start:stop], lse[start:stop], row_weight[start:stop], flag)
             G.grad_input(dlogits, wb, out=dh[start:stop])
             G.grad_weight_accumulate(dlogits, h, grad_w, accumulate=True)
-        return dh, (None if main is not None else grad_w.to(weight.dtype)), None
+        return dh, (None if main is not None else grad_w.to(weight.dtype)), None, None
 
 
 def token_logps(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
-    return _TokenLogps.apply(hidden, weight, labels)
+    keep = torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)
+    return _TokenLogps.apply(hidden, weight, labels, keep)
 
 
 def loss_sum(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
