@@ -1125,6 +1125,24 @@ void decode_layer_tail(const at::Tensor& w_out, const at::Tensor& w_ug, const at
                                 reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag))), stamps, cur_stream()), "decode_layer_tail");
 }
 
+void decode_chunk_end(const at::Tensor& kc, const at::Tensor& uc, at::Tensor fast, at::Tensor slow, at::Tensor mixed,
+                      const at::Tensor& fast_keep, const at::Tensor& slow_keep, const at::Tensor& mix) {
+  TORCH_CHECK(kc.is_cuda() && kc.dim() == 4 && kc.size(2) == 128 && kc.size(3) == 64, "decode_chunk_end: caches must be [batch, H, 128, 64]");
+  const int64_t batch = kc.size(0), H = kc.size(1);
+  for (const at::Tensor* t : {&kc, &uc})
+    TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->is_contiguous() && t->numel() == batch * H * 8192, "decode_chunk_end: BF16 caches");
+  for (const at::Tensor* t : {&fast, &slow})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == batch * H * 4096, "decode_chunk_end: FP32 memories");
+  TORCH_CHECK(mixed.scalar_type() == at::kBFloat16 && mixed.is_contiguous() && mixed.numel() == batch * H * 4096,
+              "decode_chunk_end: mixed must be BF16 [batch, H, 64, 64]");
+  for (const at::Tensor* t : {&fast_keep, &slow_keep, &mix})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == H, "decode_chunk_end: per-head FP32 values");
+  c10::cuda::CUDAGuard guard(kc.device());
+  check_rc(ws_decode_chunk_end(kc.data_ptr(), uc.data_ptr(), fast.data_ptr<float>(), slow.data_ptr<float>(), mixed.data_ptr(),
+                               fast_keep.data_ptr<float>(), slow_keep.data_ptr<float>(), mix.data_ptr<float>(), (int)batch,
+                               (int)H, cur_stream()), "decode_chunk_end");
+}
+
 void decode_pick(const at::Tensor& logits, at::Tensor token, const c10::optional<at::Tensor>& history, at::Tensor cursor,
                  at::Tensor pos) {
   TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == at::kFloat && logits.dim() == 2 && logits.is_contiguous() &&
@@ -1164,6 +1182,8 @@ TORCH_LIBRARY(ws_b200, m) {
         "Tensor(b!) part_out, Tensor(c!) part_down, Tensor(d!) n, Tensor(e!) act, Tensor(f!) qkvgu, Tensor w_norm2, "
         "Tensor? next_scale, Tensor? next_bias, Tensor w_norm_next, float eps, Tensor(g!) barrier, Tensor(h!)? error_flag, "
         "Tensor(i!)? trace=None) -> ()");
+  m.def("decode_chunk_end(Tensor kc, Tensor uc, Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor fast_keep, "
+        "Tensor slow_keep, Tensor mix) -> ()");
   m.def("decode_pick(Tensor logits, Tensor(a!) token, Tensor(b!)? history, Tensor(c!) cursor, Tensor(d!) pos) -> ()");
   m.def("decode_attn(Tensor qkvgu, Tensor(a!) kc, Tensor(b!) vc, Tensor(c!) uc, Tensor mixed, Tensor rope, Tensor pos, "
         "int H, Tensor(d!) y) -> ()");
@@ -1242,6 +1262,7 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("gather_cast_linear", &gather_cast_linear);
   m.impl("decode_reduce_norm", &decode_reduce_norm);
   m.impl("decode_attn", &decode_attn);
+  m.impl("decode_chunk_end", &decode_chunk_end);
   m.impl("decode_pick", &decode_pick);
   m.impl("decode_layer_tail", &decode_layer_tail);
   m.impl("grad_weight_group", &grad_weight_group);

@@ -639,6 +639,76 @@ decode_attn_rows_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* 
   }
 }
 
+// --------------------------------------------------------------------------- end of a chunk
+// The 128 positions of a finished chunk enter the memories: write = tanh(K)^T tanh(U) / 128, then
+// fast <- df fast + (1 - df) write, slow alike, mixed <- BF16(mix fast + (1 - mix) slow).  One CTA per (sequence, head),
+// a thread owns 4 x 4 of the 64 x 64 elements; K and U go through shared memory as FP32 tanh, everything is read and
+// written once (217 MB per layer at 64 sequences x 32 heads, about as long as the 2.1 GFLOP take on the CUDA cores).
+constexpr int CHUNK_END_SMEM = 2 * 128 * 64 * 4;
+
+__global__ void __launch_bounds__(256)
+decode_chunk_end_kernel(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ uc,
+                        float* __restrict__ fast, float* __restrict__ slow, __nv_bfloat16* __restrict__ mixed,
+                        const float* __restrict__ fast_keep, const float* __restrict__ slow_keep,
+                        const float* __restrict__ mix_of, int H) {
+  constexpr int HD = 64, C = 128;
+  extern __shared__ float chunk_smem[];
+  float* sK = chunk_smem;
+  float* sU = chunk_smem + C * HD;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int tid = threadIdx.x, h = blockIdx.x % H;
+  const size_t cache = static_cast<size_t>(blockIdx.x) * C * HD, state = static_cast<size_t>(blockIdx.x) * HD * HD;
+#pragma unroll
+  for (int i = 0; i < C * HD / 8 / 256; ++i) {
+    const int at = (tid + i * 256) * 8;
+    const uint4 kv = *reinterpret_cast<const uint4*>(kc + cache + at), uv = *reinterpret_cast<const uint4*>(uc + cache + at);
+    const __nv_bfloat162* kb = reinterpret_cast<const __nv_bfloat162*>(&kv);
+    const __nv_bfloat162* ub = reinterpret_cast<const __nv_bfloat162*>(&uv);
+#pragma unroll
+    for (int t = 0; t < 4; t += 2) {
+      const float2 k0 = __bfloat1622float2(kb[t]), k1 = __bfloat1622float2(kb[t + 1]);
+      const float2 u0 = __bfloat1622float2(ub[t]), u1 = __bfloat1622float2(ub[t + 1]);
+      *reinterpret_cast<float4*>(sK + at + 2 * t) = make_float4(tanh_fast(k0.x), tanh_fast(k0.y), tanh_fast(k1.x), tanh_fast(k1.y));
+      *reinterpret_cast<float4*>(sU + at + 2 * t) = make_float4(tanh_fast(u0.x), tanh_fast(u0.y), tanh_fast(u1.x), tanh_fast(u1.y));
+    }
+  }
+  __syncthreads();
+  const int x0 = (tid >> 4) * 4, y0 = (tid & 15) * 4;
+  float acc[4][4] = {};
+#pragma unroll 4
+  for (int c = 0; c < C; ++c) {
+    const float4 a = *reinterpret_cast<const float4*>(sK + c * HD + x0), b = *reinterpret_cast<const float4*>(sU + c * HD + y0);
+    const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      acc[i][0] += av[i] * b.x;
+      acc[i][1] += av[i] * b.y;
+      acc[i][2] += av[i] * b.z;
+      acc[i][3] += av[i] * b.w;
+    }
+  }
+  const float df = fast_keep[h], ds = slow_keep[h], mix = mix_of[h];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const size_t at = state + static_cast<size_t>(x0 + i) * HD + y0;
+    float4 f = *reinterpret_cast<const float4*>(fast + at), s = *reinterpret_cast<const float4*>(slow + at);
+    float* fv = reinterpret_cast<float*>(&f);
+    float* sv = reinterpret_cast<float*>(&s);
+    float m[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float w = acc[i][j] * (1.f / C);
+      fv[j] = df * fv[j] + (1.f - df) * w;
+      sv[j] = ds * sv[j] + (1.f - ds) * w;
+      m[j] = mix * fv[j] + (1.f - mix) * sv[j];
+    }
+    *reinterpret_cast<float4*>(fast + at) = f;
+    *reinterpret_cast<float4*>(slow + at) = s;
+    *reinterpret_cast<uint2*>(mixed + at) = make_uint2(pack_bf16x2(m[0], m[1]), pack_bf16x2(m[2], m[3]));
+  }
+}
+
 // --------------------------------------------------------------------------- greedy pick
 // One CTA per sequence: token[b] = argmax of logits[b, :] (the lowest index among equal maxima, as torch.argmax
 // picks), written where the next step's embedding gather reads it and into column `*cursor` of the history
@@ -863,6 +933,23 @@ extern "C" int ws_decode_pick(const float* logits, int batch, int vocab, long lo
   if (batch <= 0 || vocab <= 0 || vocab % 4 != 0) return -1;
   const cudaError_t err = launch_chained(decode_pick_kernel, dim3(batch), dim3(256), 0, stream, logits, vocab, token, history,
                                          capacity, cursor, pos);
+  ws_count_launch();
+  return err == cudaSuccess ? 0 : -21;
+}
+
+extern "C" int ws_decode_chunk_end(const void* kc, const void* uc, float* fast, float* slow, void* mixed,
+                                   const float* fast_keep, const float* slow_keep, const float* mix, int batch, int H,
+                                   cudaStream_t stream) {
+  if (batch <= 0 || H <= 0) return -1;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(decode_chunk_end_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CHUNK_END_SMEM) != cudaSuccess)
+      return -20;
+    configured = true;
+  }
+  const cudaError_t err = launch_chained(decode_chunk_end_kernel, dim3(batch * H), dim3(256), CHUNK_END_SMEM, stream,
+                                         static_cast<const __nv_bfloat16*>(kc), static_cast<const __nv_bfloat16*>(uc), fast,
+                                         slow, static_cast<__nv_bfloat16*>(mixed), fast_keep, slow_keep, mix, H);
   ws_count_launch();
   return err == cudaSuccess ? 0 : -21;
 }

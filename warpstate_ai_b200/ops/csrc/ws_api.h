@@ -88,6 +88,10 @@ int ws_decode_reduce_norm(float* x, const float* partial, int splits, const long
 int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, const void* mixed, const float* rope,
                    const long long* pos, int batch, int H, int d, void* y, cudaStream_t stream);
 
+// A finished chunk enters the memories of every (sequence, head), in place: kc, uc BF16 [batch, H, 128, 64]; fast, slow
+// FP32 and mixed BF16 [batch, H, 64, 64]; the decays and the mix [H] are the sigmoids of their logits.
+int ws_decode_chunk_end(const void* kc, const void* uc, float* fast, float* slow, void* mixed, const float* fast_keep,
+                        const float* slow_keep, const float* mix, int batch, int H, cudaStream_t stream);
 // The part of a decode layer after its attention as ONE persistent cooperative launch (ops/csrc/decode_layer.cu):
 // out_proj, residual + norm, up/gate + SwiGLU, down, residual + next layer's modulation + norm, next layer's in_proj.
 // Weights row-major BF16: w_out [d, d], w_ug [2 ffn, d], w_down [d, ffn], w_in_next [5 d, d] or NULL after the last

@@ -278,6 +278,10 @@ class DecodeEngine:
         return F.linear(self._norm(x, self.final_norm), self.head).float()
 
     def _end_of_chunk(self) -> None:
+        if self._kbufs is not None:
+            for w, st in zip(self.weights, self.states):
+                torch.ops.ws_b200.decode_chunk_end(st.k, st.u, st.fast, st.slow, st.mixed, w["df"], w["ds"], w["mix"])
+            return
         for w, st in zip(self.weights, self.states):
             write = torch.matmul(torch.tanh(st.k).transpose(-2, -1), torch.tanh(st.u)).float() / self.chunk
             st.fast.mul_(w["df"]).add_(write * (1.0 - w["df"]))
