@@ -97,7 +97,14 @@ void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_
   g.row_vec = nullptr;
   g.alpha = (float)alpha; g.beta = (float)beta;
   g.error_flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
-  const int rc = ws_gemm(&g, cur_stream());
+  const int splits = ws_gemm_splits(&g);
+  int rc;
+  if (splits > 1) {
+    at::Tensor part = at::empty({splits, m, n}, out.options().dtype(at::kFloat));
+    rc = ws_gemm_split(&g, splits, part.data_ptr<float>(), cur_stream());
+  } else {
+    rc = ws_gemm(&g, cur_stream());
+  }
   if (rc != 0) {  // name the problem: a bare code is of little use for a tensor-map or shape refusal
     char what[256];
     snprintf(what, sizeof(what), "gemm (m=%lld n=%lld k=%lld a_mn=%d b_mn=%d epilogue=%lld lda=%d ldb=%d ldo=%d)",

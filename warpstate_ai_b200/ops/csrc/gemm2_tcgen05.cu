@@ -90,7 +90,8 @@ struct alignas(64) PairGroup {
   CUtensorMap b[MAX_GROUP];
   GemmParams p[MAX_GROUP];
   CUtensorMap epi[4];  // staged epilogue of problem 0, 32 x 32 boxes.  SwiGLU backward: aux up, aux gate,
-                       // out up, out gate; SwiGLU forward: packed up, packed gate, activation
+                       // out up, out gate; SwiGLU forward: packed up, packed gate, activation; residual: aux, out;
+                       // FP32: the output of problem i
   CUtensorMap whole;   // row selection (problem 0): the operand before its rows were selected
   int tile_start[MAX_GROUP + 1];
   int count;
@@ -102,8 +103,9 @@ struct alignas(64) PairGroup {
 // global memory never goes through L1 and each thread touches only swizzled shared memory.
 template <int EPI>
 constexpr bool staged_epilogue() {
-  return EPI == WS_EPI_SWIGLU_BWD || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_RESID_F32;
+  return EPI == WS_EPI_SWIGLU_BWD || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_RESID_F32 || EPI == WS_EPI_F32;
 }
+static_assert(MAX_GROUP == 4, "one output map per problem of an FP32 group");
 template <int EPI>
 constexpr int pair_stages() {
   return staged_epilogue<EPI>() ? pair::STAGES - 1 : pair::STAGES;
@@ -207,7 +209,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
     }
     if (STAGED) {
       for (int i = 0; i < 16; ++i) mbar_init(&ebar[i], 1);
-      for (int i = 0; i < (EPI == WS_EPI_SWIGLU ? 3 : EPI == WS_EPI_RESID_F32 ? 2 : 4); ++i) tma_prefetch_desc(&g.epi[i]);
+      for (int i = 0; i < (EPI == WS_EPI_SWIGLU ? 3 : EPI == WS_EPI_RESID_F32 ? 2 : EPI == WS_EPI_F32 ? g.count : 4); ++i) tma_prefetch_desc(&g.epi[i]);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -405,6 +407,44 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
               }
               tma_store_2d(&g.epi[2], ebuf + 4096, x, y);
             }
+            tma_store_commit();
+          }
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
+      }
+      if (lane == 0) tma_store_wait_all();
+    } else if constexpr (EPI == WS_EPI_F32) {
+      // FP32 through shared memory: per warp 32 rows, per step 32 columns, two tiles in flight.
+      uint8_t* ebuf = eStage + (warp - 2) * 8192;
+      constexpr int STEPS = (BN / GROUPS) / 32;
+      int q = 0;
+      for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
+        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
+        const GemmParams& p = g.p[t.prob];
+        const int buf_t = tcount & 1;
+        const uint32_t tph = (tcount >> 1) & 1;
+        if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
+        tc_fence_after_sync();
+        const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+#pragma unroll 1
+        for (int step = 0; step < STEPS; ++step, ++q) {
+          const int x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+          uint8_t* tr = ebuf + (q & 1) * 4096;
+          uint32_t r[32];
+          tmem_ld_32x32b_x32(taddr + step * 32, r);
+          if (lane == 0) tma_store_wait_read1();  // the store issued from this tile two steps ago has read it
+          __syncwarp();
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(tile_chunk128(tr, lane, j)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (x < p.n && y < p.m) tma_store_2d(&g.epi[t.prob], tr, x, y);
             tma_store_commit();
           }
         }
@@ -761,7 +801,114 @@ static int fill_swiglu_maps(const WsGemm* g0, PairGroup& grp) {
   return 0;
 }
 
+// --------------------------------------------------------------------------- split contraction
+// Few rows against a long contraction (down, and the input gradients of up/gate and in_proj, below a few thousand rows)
+// give fewer tiles than CTA pairs: 300 x 2048 outputs are 16 tiles, and each walks all 112 k-blocks of the FFN width
+// alone.  Such a product is cut along k into up to four problems of one grouped launch with FP32 results, which this
+// kernel adds in order, with the epilogue of the whole: one thread per four columns.
+template <int EPI>
+__global__ void __launch_bounds__(256)
+split_finish_kernel(const float* __restrict__ part, int splits, int m, int n, const void* __restrict__ aux, int ldaux,
+                    const float* __restrict__ row_scale, void* __restrict__ out, int ldo) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int per_row = n / 4;
+  const size_t total = static_cast<size_t>(m) * per_row, plane = static_cast<size_t>(m) * n;
+  for (size_t i = blockIdx.x * static_cast<size_t>(256) + threadIdx.x; i < total; i += static_cast<size_t>(gridDim.x) * 256) {
+    const int row = static_cast<int>(i / per_row), c = static_cast<int>(i % per_row) * 4;
+    const float* src = part + static_cast<size_t>(row) * n + c;
+    float4 p[MAX_GROUP];
+#pragma unroll
+    for (int s = 0; s < MAX_GROUP; ++s)
+      if (s < splits) p[s] = *reinterpret_cast<const float4*>(src + s * plane);
+    float4 v = p[0];
+#pragma unroll
+    for (int s = 1; s < MAX_GROUP; ++s)
+      if (s < splits) { v.x += p[s].x; v.y += p[s].y; v.z += p[s].z; v.w += p[s].w; }
+    if constexpr (EPI == WS_EPI_RESID_F32) {
+      const float4 r = *reinterpret_cast<const float4*>(static_cast<const float*>(aux) + static_cast<size_t>(row) * ldaux + c);
+      *reinterpret_cast<float4*>(static_cast<float*>(out) + static_cast<size_t>(row) * ldo + c) =
+          make_float4(r.x + v.x, r.y + v.y, r.z + v.z, r.w + v.w);
+    } else {
+      uint2 o;
+      if constexpr (EPI == WS_EPI_RESID_BF16) {
+        const uint2 q = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(aux) + static_cast<size_t>(row) * ldaux + c);
+        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+        const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+        o = make_uint2(pack_bf16x2(a.x + bf16_round(v.x), a.y + bf16_round(v.y)),
+                       pack_bf16x2(b.x + bf16_round(v.z), b.y + bf16_round(v.w)));
+      } else {
+        const float rs = row_scale != nullptr ? row_scale[row] : 1.f;
+        o = make_uint2(pack_bf16x2(v.x * rs, v.y * rs), pack_bf16x2(v.z * rs, v.w * rs));
+      }
+      *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(out) + static_cast<size_t>(row) * ldo + c) = o;
+    }
+  }
+}
+
 }  // namespace ws
+
+// Into how many pieces a product that the CTA-pair kernel would take is best cut along k (1: not at all), on `sms` SMs.
+// A tile costs 0.28 us per k-block (256 x 256 x 64 on two SMs); cutting costs the second launch and the FP32 pieces,
+// which are written and read once through L2.  All pieces together have to fit one round over the CTA pairs: a second
+// round repeats what a tile costs beyond its k-blocks, and measured slower (2048 x 1280 outputs of a 4480-long
+// contraction, 40 tiles in three pieces: 39.0 us against 37.1 uncut).  At 300 x 2048 outputs, k 7168: 48.0 -> 27.6 us.
+extern "C" int ws_gemm_pair_splits(const WsGemm* g, int sms) {
+  using namespace ws;
+  if (g->a_mn || g->limit != nullptr || g->row_map != nullptr || g->n % 4 != 0 ||
+      (g->epilogue != WS_EPI_BF16 && g->epilogue != WS_EPI_RESID_F32 && g->epilogue != WS_EPI_RESID_BF16))
+    return 1;
+  const long long tiles = (long long)((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + pair::BN - 1) / pair::BN);
+  const int pairs = sms / 2, blocks = (g->k + pair::BK - 1) / pair::BK;
+  if (pairs < 2 || tiles >= pairs) return 1;
+  const float tile_us = 0.28f, cut_us = 3.0f, piece_us = 8.0f * g->m * (float)g->n / 6.0e6f;
+  int best = 1;
+  float least = blocks * tile_us;
+  for (int s = 2; s <= MAX_GROUP && tiles * s <= pairs; ++s) {
+    const float us = ((blocks + s - 1) / s) * tile_us + cut_us + s * piece_us;
+    if (us < least) {
+      least = us;
+      best = s;
+    }
+  }
+  return best;
+}
+
+extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaStream_t stream);
+
+// The product in `splits` (2..4) pieces; part: FP32 [splits, m, n].
+extern "C" int ws_gemm_pair_split(const WsGemm* g, int splits, float* part, int sms, cudaStream_t stream) {
+  using namespace ws;
+  if (splits < 2 || splits > MAX_GROUP || part == nullptr) return -9;
+  const int blocks = (g->k + pair::BK - 1) / pair::BK, per = (blocks + splits - 1) / splits;
+  WsGemm items[MAX_GROUP];
+  int count = 0;
+  for (int s = 0; s < splits; ++s) {
+    const int k0 = s * per * pair::BK;
+    if (k0 >= g->k) break;
+    WsGemm& q = items[count];
+    q = *g;
+    q.k = g->k - k0 < per * pair::BK ? g->k - k0 : per * pair::BK;
+    q.a = static_cast<const __nv_bfloat16*>(g->a) + k0;
+    q.b = static_cast<const __nv_bfloat16*>(g->b) + (g->b_mn ? static_cast<size_t>(k0) * g->ldb : static_cast<size_t>(k0));
+    q.epilogue = WS_EPI_F32;
+    q.out = part + static_cast<size_t>(count) * g->m * g->n;
+    q.ldo = g->n;
+    q.out2 = nullptr; q.aux = nullptr; q.row_scale = nullptr;
+    ++count;
+  }
+  int rc = ws_gemm_pair_group(items, count, sms, stream);
+  if (rc) return rc;
+  const size_t quads = static_cast<size_t>(g->m) * (g->n / 4);
+  const unsigned grid = static_cast<unsigned>(quads < 256 * 1184 ? (quads + 255) / 256 : 1184);
+  auto finish = g->epilogue == WS_EPI_RESID_F32    ? split_finish_kernel<WS_EPI_RESID_F32>
+                : g->epilogue == WS_EPI_RESID_BF16 ? split_finish_kernel<WS_EPI_RESID_BF16>
+                                                   : split_finish_kernel<WS_EPI_BF16>;
+  launch_dependent(finish, dim3(grid), dim3(256), 0, stream, static_cast<const float*>(part), count, g->m, g->n, g->aux, g->ldaux,
+                   g->row_scale, g->out, g->ldo);
+  ws_count_launch();
+  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+}
 
 // `count` problems (1..4) of one kind (same operand majors and epilogue) in one launch.  The
 // argument checks of ws_gemm have already run on every item; `sms` bounds the SMs used.
@@ -783,6 +930,12 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     total += tiles;
   }
   for (int i = count; i <= MAX_GROUP; ++i) grp.tile_start[i] = total;
+  if (items[0].epilogue == WS_EPI_F32) {
+    for (int i = 0; i < count; ++i) {
+      const int rc = make_map_f32(&grp.epi[i], items[i].out, items[i].n, items[i].m, items[i].ldo, 32, 32);
+      if (rc) return rc;
+    }
+  }
   if (items[0].epilogue == WS_EPI_RESID_F32) {
     if (count != 1) return -9;
     const WsGemm* g0 = &items[0];
@@ -822,6 +975,7 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     case (0 | (WS_EPI_RESID_BF16 << 2)): return launch_pair<false, false, WS_EPI_RESID_BF16>(grp, pairs, stream);
     case (0 | (WS_EPI_SWIGLU << 2)): return launch_pair<false, false, WS_EPI_SWIGLU>(grp, pairs, stream);
     case (0 | (WS_EPI_F32 << 2)): return launch_pair<false, false, WS_EPI_F32>(grp, pairs, stream);
+    case (2 | (WS_EPI_F32 << 2)): return launch_pair<false, true, WS_EPI_F32>(grp, pairs, stream);
     case (3 | (WS_EPI_ACC_F32 << 2)): return launch_pair<true, true, WS_EPI_ACC_F32>(grp, pairs, stream);
     case (3 | (WS_EPI_BF16 << 2)): return launch_pair<true, true, WS_EPI_BF16>(grp, pairs, stream);
     case (2 | (WS_EPI_SWIGLU_BWD << 2)): return launch_pair<false, true, WS_EPI_SWIGLU_BWD>(grp, pairs, stream);

@@ -325,6 +325,25 @@ extern "C" int ws_gemm_group(const WsGemm* items, int count, cudaStream_t stream
   return 0;
 }
 
+extern "C" int ws_gemm_pair_splits(const WsGemm* g, int sms);
+extern "C" int ws_gemm_pair_split(const WsGemm* g, int splits, float* part, int sms, cudaStream_t stream);
+
+// The CTA-pair kernel from 96 rows on: below its 256-row tile part of the tensor work is padding, but a product of so
+// few rows is bound by the bytes an SM takes in per k-block, 32 KiB in a pair against 48 KiB in the single-CTA kernel.
+static bool takes_pair(const WsGemm* g) {
+  return g->limit != nullptr || (pair_mode() && g->m >= (g->a_mn ? 256 : 96) && usable_sms() >= 2);
+}
+
+extern "C" int ws_gemm_splits(const WsGemm* g) {
+  return validate_gemm(g) == 0 && takes_pair(g) ? ws_gemm_pair_splits(g, usable_sms()) : 1;
+}
+
+extern "C" int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream) {
+  const int rc = validate_gemm(g);
+  if (rc) return rc;
+  return splits < 2 ? ws_gemm(g, stream) : ws_gemm_pair_split(g, splits, part, usable_sms(), stream);
+}
+
 extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   {
     const int vrc = validate_gemm(g);
@@ -332,7 +351,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   }
   using namespace ws;
   const int sms = usable_sms();
-  if (g->limit != nullptr || (pair_mode() && g->m >= 256 && sms >= 2)) return ws_gemm_pair(g, sms, stream);
+  if (takes_pair(g)) return ws_gemm_pair(g, sms, stream);
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   const int b_rows = swiglu ? 2 * g->n : g->n;  // output features held by B
   CUtensorMap ta, tb;

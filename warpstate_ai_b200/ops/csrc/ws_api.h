@@ -59,6 +59,10 @@ typedef struct WsGemm {
 
 int ws_gemm(const WsGemm* g, cudaStream_t stream);
 int ws_gemm_pair_available(void);  // 1 where problems with >= 256 rows take the CTA-pair kernel
+// A product whose tiles would leave most of the chip idle may be cut along k: ws_gemm_splits says into how many pieces
+// (1: not), and ws_gemm_split computes it so, with FP32 scratch `part` of splits * m * n floats.
+int ws_gemm_splits(const WsGemm* g);
+int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream);
 // Number of SMs the GEMM may use on this stream's device (0 = all).  Lets a communication
 // kernel keep a few SMs for itself while persistent GEMM CTAs fill the rest.
 // `count` problems in one persistent launch where possible (same operand majors and epilogue, each
