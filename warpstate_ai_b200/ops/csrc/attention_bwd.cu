@@ -328,7 +328,8 @@ constexpr int SCAN_MAX_CHUNKS = SCAN_GROUP * SCAN_MAX_GROUPS;  // 32768 tokens p
 // dstate [B,N,H,4096] FP32 (gradient of the mixed state read by chunk n), writes [B,N,H,4096] FP32
 // -> dwrites [B,N,H,4096] BF16 and partial sums [B*H*16][3] of d(fast decay), d(slow decay), d(mix).
 // A thread owns two neighbouring state elements (8-byte loads of the writes and of the state gradients, 4-byte stores):
-// half the memory instructions of the one-element form, and 256 bytes in flight per thread.
+// half the memory instructions of the one-element form, and 256 bytes in flight per thread, three blocks per SM.  At
+// 4 x 16 chunks x 32 heads it takes 29.3 us (84 MB); the whole block's forward + backward went from 273 to 267 us.
 constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_VEC = 2;
 
@@ -458,6 +459,8 @@ memory_logit_grads_kernel(const float* __restrict__ partials, const float* __res
 // tile cannot keep an SM busy; what matters is how many tiles an SM holds at once, and how long the element-wise
 // stretches of the chain are.  Shared memory is therefore kept to 112 KiB and TMEM to 256 columns, so that TWO CTAs fit
 // per SM, and a row is shared by two threads, which exchange its softmax statistics and its D through shared memory.
+// 2048 tiles (4 x 2048 tokens, 32 heads): 169.6 us with one thread per row, 131.8 with two (128 registers, no spills);
+// DRAM 33 % busy, 24 % of the warps: what is left is the latency of the chain.
 //
 //   smem: B0 Qr | B1 Kr | B2 dy -> dlocal -> tanh(U) | B3 dmem/8 -> V -> tanh(Kr) | sP (32K: P -> dS)
 //         | sSt (8K) | sDW (8K) | barriers

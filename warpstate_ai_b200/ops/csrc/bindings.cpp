@@ -434,6 +434,7 @@ at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast
 // The kernel sequences of one block (ops/fused.py) as one call each.  A block is eight to twelve launches of 2-20 us in
 // a short sequence, and issued one by one from Python the host takes longer than the device below a few thousand rows;
 // here a launch costs its allocation, its tensor maps and the launch.  Same kernels, same order, same results.
+// Smoke model (d 256, 4 depths, 2 x 512 tokens), forward + backward: 2.53 -> 2.03 ms.
 at::Tensor project(const at::Tensor& x, const at::Tensor& w, bool b_mn, int64_t epilogue, int64_t n, at::Tensor out,
                    const c10::optional<at::Tensor>& out2, const c10::optional<at::Tensor>& aux,
                    const c10::optional<at::Tensor>& flag) {

@@ -363,7 +363,8 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
   // the RoPE of the new token, so that the three dependent phases below (scores, softmax, P.V) wait for memory once.
   // They are issued before the wait for the previous kernel, too, and run under the tail of the projection: the
   // position, the cache rows before it and M are what the previous STEP left, and steps are separated by full
-  // dependencies (a graph replay, or the kernel that writes the position).  Only `row` is this step's.
+  // dependencies (a graph replay, or the kernel that writes the position).  Only `row` is this step's.  With the same in
+  // the residual + norm kernel: 48 steps of 28 layers at batch 1 72.3 -> 64.9 ms, 40 of 8 layers at batch 64 32.7 -> 29.7.
   const int jg = tid & 7, rg = tid >> 3;
   uint4 kreg[C / 16], vreg[C / 16], mreg[HD / 16];
 #pragma unroll
@@ -644,6 +645,7 @@ decode_attn_rows_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* 
 // fast <- df fast + (1 - df) write, slow alike, mixed <- BF16(mix fast + (1 - mix) slow).  One CTA per (sequence, head),
 // a thread owns 4 x 4 of the 64 x 64 elements; K and U go through shared memory as FP32 tanh, everything is read and
 // written once (217 MB per layer at 64 sequences x 32 heads, about as long as the 2.1 GFLOP take on the CUDA cores).
+// 48 steps of 28 layers at batch 1 with one end of a chunk: 64.9 ms with a dozen framework operations per layer, 63.1 so.
 constexpr int CHUNK_END_SMEM = 2 * 128 * 64 * 4;
 
 __global__ void __launch_bounds__(256)

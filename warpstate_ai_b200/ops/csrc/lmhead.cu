@@ -52,6 +52,8 @@ ce_combine_kernel(const float2* __restrict__ parts, int ld, int nparts, const fl
 //
 // One CTA: a thread has SELECT_ITEMS labels in flight, a rank is the count of labelled rows before it (warp ballots,
 // then a scan over the warps of the block).  It is one round trip to memory per 16384 rows, whatever the labels are.
+// Head forward + backward at 4 x 2048 rows of which 2302 are labelled, d 2048, vocabulary 32768: 3.44 -> 1.20 ms; with
+// all of 16384 rows labelled the three small kernels are within the noise of 7.2 ms (nothing is copied).
 constexpr int SELECT_THREADS = 1024;
 constexpr int SELECT_ITEMS = 16;
 constexpr int SELECT_PAD = 256;   // rows of a tile of the CTA-pair GEMM
@@ -155,7 +157,7 @@ clear_unlabelled_kernel(const long long* __restrict__ labels, long long ignore_i
 
 // Logit gradients from logits that the forward pass kept: one CTA per row, 16-byte pieces, read and written once.  At
 // 8192 x 32768 that is 1 GiB of traffic (0.16 ms at the copy rate) in place of the product that makes the logits again
-// (1.1 TFLOP, 0.7 ms).  Same arithmetic as the WS_EPI_CE_BWD epilogue on the same BF16 logits: the same bits.
+// (1.1 TFLOP, 0.7 ms).  Head forward + backward at 16384 labelled rows: 7.32 -> 5.83 ms, at 2302: 1.22 -> 1.00 ms.  Same arithmetic as the WS_EPI_CE_BWD epilogue on the same BF16 logits: the same bits.
 constexpr int DLOGITS_PAD = 64;   // rows per k-block of the weight gradient
 
 __global__ void __launch_bounds__(256)

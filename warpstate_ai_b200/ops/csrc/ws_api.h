@@ -115,7 +115,7 @@ int ws_decode_layer_tail(const void* w_out, const void* w_ug, const void* w_down
 int ws_decode_pick(const float* logits, int batch, int vocab, long long* token, long long* history, int capacity,
                    long long* cursor, long long* pos, cudaStream_t stream);
 
-// Kernel choice for problems with >= 256 rows: 1 = CTA-pair (cta_group::2) kernel, 0 = single-CTA
+// Kernel choice for problems with >= 96 rows (weight gradients: 256): 1 = CTA-pair (cta_group::2) kernel, 0 = single-CTA
 // kernel, -1 = the process default (pair unless WS_GEMM_PAIR=0 is in the environment).
 void ws_gemm_set_pair_mode(int mode);
 
