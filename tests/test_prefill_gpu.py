@@ -89,3 +89,41 @@ def test_a_prefilled_state_equals_a_stepped_one():
             assert rel(getattr(a, name), getattr(b, name)) < 0.02, name
         for name in ("k", "v", "u"):
             assert rel(getattr(a, name)[:, :, :72], getattr(b, name)[:, :, :72]) < 0.02, name
+
+
+@pytest.mark.parametrize("stream_form", [0, 1])
+@pytest.mark.parametrize("batch,heads,length", [(1, 2, 100), (2, 3, 255), (16, 4, 128 * 3 + 44)])
+def test_open_chunk_keeps_its_softmax_weights(batch, heads, length, stream_form):
+    """A decode step weighs the values in FP32, so the positions of the chunk a prompt ends in do, too: next to the BF16
+    rounding of the output itself nothing is lost.  (Weights rounded to BF16 would be of its size, 1.4 times in all.)"""
+    from warpstate_ai_b200.ops import _ext, attention
+    _ext.require()
+    torch.manual_seed(length)
+    d, rest = 64 * heads, length % 128
+    packed = torch.randn(batch, length, 5, heads, 64, device="cuda").bfloat16()
+    packed[:, :, 3] = 40.0                                            # the gate: local attention alone
+    logits = [torch.zeros(heads, device="cuda") for _ in range(3)]
+    fast, slow = (torch.empty(batch, heads, 64, 64, device="cuda") for _ in range(2))
+    mixed = torch.empty(batch, heads, 64, 64, device="cuda", dtype=torch.bfloat16)
+    caches = [torch.empty(batch, heads, 128, 64, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    lib = _ext.cdll()
+    try:
+        lib.ws_attn_set_stream_mode(stream_form)
+        y = torch.ops.ws_b200.attn_prefill(packed.view(batch * length, 5 * d), attention.rope_table(packed.device, pair_major=True),
+                                           *logits, batch, length, heads, fast, slow, mixed, *caches,
+                                           attention.error_flag(packed.device))
+    finally:
+        lib.ws_attn_set_stream_mode(-1)
+    check_device_errors()
+    cos, sin = attention.rope_table(packed.device).double()[:rest].unsqueeze(1).unbind(-1)
+
+    def turned(x):                                                    # rounded to BF16, as a decode step caches it
+        even, odd = x.double()[..., 0::2], x.double()[..., 1::2]
+        return torch.stack((even * cos - odd * sin, odd * cos + even * sin), dim=-1).flatten(-2).bfloat16().double()
+
+    q, k, v = packed[:, length - rest:, :3].unbind(2)
+    scores = torch.einsum("brhi,bchi->bhrc", turned(q), turned(k)) / 8.0
+    future = torch.ones(rest, rest, dtype=torch.bool, device="cuda").triu(1)
+    want = torch.einsum("bhrc,bchi->brhi", torch.softmax(scores.masked_fill(future, float("-inf")), dim=-1), v.double())
+    got = y.view(batch, length, heads, 64)[:, length - rest:]
+    assert rel(got, want) < 1.1 * rel(want.bfloat16(), want)

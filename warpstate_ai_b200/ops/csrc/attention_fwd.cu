@@ -414,8 +414,14 @@ open_chunk_kernel(const __nv_bfloat16* __restrict__ qkvgu, const float2* __restr
 // is complete.  TMEM: 128 columns; S occupies all of them, and after the softmax has read S, O takes
 // columns 0-63 and Mem = Q State columns 64-127, so three CTAs fit the 512 columns of an SM too.
 // The kernel is bound by the latency of its dependent chain, so tiles in flight are what counts.
+//
+// PROMPT: the chunk that a prompt ends in.  A decode step computes such positions with FP32 softmax weights, so here, too,
+// no weight is rounded to BF16: it is split into two BF16 terms (2^-17 of it is left out), and O = P_hi V + P_lo V.  The
+// low terms wait in registers (64 of them) until the high ones have been consumed, then take their place in shared memory;
+// the tiles of complete chunks skip all of it.
 constexpr int AF_SMEM = 4 * TILE_BYTES + 8192 + 1024 + 128;
 
+template <bool PROMPT>
 __global__ void __launch_bounds__(128, 3)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                 const __grid_constant__ CUtensorMap tm_y, const float2* __restrict__ rope, int T, int H, int d,
@@ -436,11 +442,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   const int tile = blockIdx.x;
   const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
   const int row0 = n * CHUNK;
+  const bool open = PROMPT && row0 + CHUNK > T;
 
   if (tid == 0) {
     mbar_init(&bars[0], 1);
     mbar_init(&bars[1], 1);
     mbar_init(&bars[2], 1);
+    if (PROMPT) mbar_init(&bars[3], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -499,6 +507,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       if (cc * 32 + j <= tid) row_max = fmaxf(row_max, __uint_as_float(r[j]));
   }
   float row_sum = 0.f;
+  [[maybe_unused]] uint32_t low[PROMPT ? 4 : 1][16];
+#pragma unroll(PROMPT ? 4 : 1)
   for (int cc = 0; cc < 4; ++cc) {
     uint32_t pk[16];
     if (cc <= last_chunk) {
@@ -513,10 +523,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
         const float2 back = __bfloat1622float2(v);
         row_sum += back.x + back.y;  // normalise by what the MMA will actually sum
         pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&v);
+        if constexpr (PROMPT) {
+          const __nv_bfloat162 l = __floats2bfloat162_rn(p0 - back.x, p1 - back.y);
+          const float2 rest = __bfloat1622float2(l);
+          if (open) row_sum += rest.x + rest.y;
+          low[cc][j >> 1] = *reinterpret_cast<const uint32_t*>(&l);
+        }
       }
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) pk[j] = 0u;
+      for (int j = 0; j < 16; ++j) {
+        pk[j] = 0u;
+        if constexpr (PROMPT) low[cc][j] = 0u;
+      }
     }
     store_row_chunk32(sP, tid, cc * 32, pk);
   }
@@ -538,6 +557,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   }
   ok = ok && mbar_wait(&bars[2], 0, abort_flag);
   tc_fence_after_sync();
+  if constexpr (PROMPT) {
+    if (open) {  // O += P_lo V
+#pragma unroll
+      for (int cc = 0; cc < 4; ++cc) store_row_chunk32(sP, tid, cc * 32, low[cc]);
+      fence_proxy_async_smem();
+      __syncthreads();
+      if (tid == 0 && ok) {
+        constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
+#pragma unroll
+        for (int k = 0; k < CHUNK / 16; ++k)
+          umma_bf16(t_o, make_smem_desc_sw128(smem_u32(sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
+                    make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, 1u);
+        umma_commit(&bars[3]);
+      }
+      ok = ok && mbar_wait(&bars[3], 0, abort_flag);
+      tc_fence_after_sync();
+    }
+  }
 
   // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
   const float inv_l = 1.f / row_sum;
@@ -598,12 +635,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 //
 // Two tiles are in their softmax / blend phase at any time while a third is being rotated and a fourth loaded;
 // attn_fwd_kernel gets its overlap from three independent CTAs per SM, each walking the whole chain alone.
-// TMEM: set g = columns [192 g, 192 g + 192): S 128 (O reuses its first 64), Mem 64.  Bit-identical results.
+// TMEM: set g = columns [192 g, 192 g + 192): S 128, Mem 64; O of group g = columns [384 + 64 g, 448 + 64 g).  Bit-identical
+// results.  PROMPT as in attn_fwd_kernel; the low terms of P are formed from S again, which is still in TMEM, once O has
+// the high ones.
 constexpr int AS_STAGES = 3;
 constexpr int AS_THREADS = 17 * 32;
 constexpr int AS_STAGE_BYTES = 4 * TILE_BYTES + 8192;
 constexpr int AS_SMEM = AS_STAGES * AS_STAGE_BYTES + 1024 + 256;
 
+template <bool PROMPT>
 __global__ void __launch_bounds__(AS_THREADS, 1)
 attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                        const __grid_constant__ CUtensorMap tm_y, const float2* __restrict__ rope, int T, int H, int d,
@@ -616,7 +656,8 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
   uint64_t* sfull = bars + 2 * AS_STAGES;    // [2] S and Mem complete
   uint64_t* ofull = sfull + 2;               // [2] O complete
   uint64_t* setfree = ofull + 2;             // [2] TMEM set read out (4 warps)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(setfree + 2);
+  uint64_t* lowfull = setfree + 2;           // [2] O has the low terms too (PROMPT)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(lowfull + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_chunks = (T + CHUNK - 1) / CHUNK;
@@ -630,6 +671,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       mbar_init(&sfull[g], 1);
       mbar_init(&ofull[g], 1);
       mbar_init(&setfree[g], 4);
+      mbar_init(&lowfull[g], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -738,10 +780,22 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
     const int g = (warp - 8) >> 2;
     const int gt = tid - (256 + g * 128);       // row of the tile = TMEM lane
     const int wq = gt >> 5;                     // lane quarter of this warp
-    const uint32_t t_s = tmem + g * 192, t_o = t_s, t_m = t_s + 128;
+    const uint32_t t_s = tmem + g * 192, t_o = tmem + 384 + g * 64, t_m = t_s + 128;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float kScale = 0.125f * 1.4426950408889634f;  // fold log2(e)
     const int last_chunk = wq;  // columns beyond 32*wq+31 are masked for the whole warp
+    // whether any of the group's threads is not ok; a barrier of its 128 threads
+    auto any_bad = [&](bool ok) {
+      uint32_t bad;
+      if (g == 0)
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 3, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(bad) : "r"(ok ? 0u : 1u) : "memory");
+      else
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 4, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(bad) : "r"(ok ? 0u : 1u) : "memory");
+      return bad != 0u;
+    };
+    [[maybe_unused]] uint32_t opens = 0;   // open chunks this group has met
     int i = g;
     for (int tile = first + g * step; tile < tiles; tile += 2 * step, i += 2) {
       const int s = i % AS_STAGES, k2 = i >> 1;
@@ -751,13 +805,31 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       uint8_t* sV = sQ + 3 * TILE_BYTES;
       const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
       const int row0 = n * CHUNK;
+      const bool open = PROMPT && row0 + CHUNK > T;
+      // columns 0..63 of P go to the K tile's space, columns 64..127 to the Q tile's
+      auto store_p = [&](int cc, const uint32_t(&pk)[16]) {
+        uint8_t* half = (cc < 2) ? sK : sQ;
+        const int j0 = (cc & 1) * 4;
+#pragma unroll
+        for (int w4 = 0; w4 < 4; ++w4)
+          *reinterpret_cast<uint4*>(tile_chunk(half, gt, j0 + w4)) =
+              make_uint4(pk[4 * w4], pk[4 * w4 + 1], pk[4 * w4 + 2], pk[4 * w4 + 3]);
+      };
+      auto issue_o = [&](uint32_t accumulate, uint64_t* done) {
+        tc_fence_after_sync();
+        constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
+#pragma unroll
+        for (int k = 0; k < CHUNK / 16; ++k)
+          umma_bf16(t_o, make_smem_desc_sw128(smem_u32((k >> 2) ? sQ : sK) + (k & 3) * 32, 0, 1024),
+                    make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, k > 0 ? 1u : accumulate);
+        umma_commit(done);
+      };
       uint32_t landed = 0;
       if (lane == 0) landed = mbar_wait(&sfull[g], k2 & 1, abort_flag) ? 1u : 0u;
       bool ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
       tc_fence_after_sync();
-      float row_sum = 0.f;
+      float row_sum = 0.f, row_max = -INFINITY;
       if (ok) {
-        float row_max = -INFINITY;
         for (int cc = 0; cc <= last_chunk; ++cc) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
@@ -780,43 +852,60 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
               const float2 back = __bfloat1622float2(pv);
               row_sum += back.x + back.y;  // normalise by what the MMA will actually sum
               pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&pv);
+              if (PROMPT && open) {
+                const float2 rest = __bfloat1622float2(__floats2bfloat162_rn(p0 - back.x, p1 - back.y));
+                row_sum += rest.x + rest.y;
+              }
             }
           } else {
 #pragma unroll
             for (int j = 0; j < 16; ++j) pk[j] = 0u;
           }
-          // columns 0..63 of P go to the K tile's space, columns 64..127 to the Q tile's
-          uint8_t* half = (cc < 2) ? sK : sQ;
-          const int j0 = (cc & 1) * 4;
-#pragma unroll
-          for (int w4 = 0; w4 < 4; ++w4)
-            *reinterpret_cast<uint4*>(tile_chunk(half, gt, j0 + w4)) =
-                make_uint4(pk[4 * w4], pk[4 * w4 + 1], pk[4 * w4 + 2], pk[4 * w4 + 3]);
+          store_p(cc, pk);
         }
       }
-      tc_fence_before_sync();  // every thread's reads of S precede the MMA that overwrites its first columns
+      tc_fence_before_sync();
       fence_proxy_async_smem();
-      uint32_t any_bad;
-      if (g == 0)
-        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 3, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(any_bad) : "r"(ok ? 0u : 1u) : "memory");
-      else
-        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 4, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
-                     : "=r"(any_bad) : "r"(ok ? 0u : 1u) : "memory");
-      if (any_bad) break;
-      if (gt == 0) {
-        tc_fence_after_sync();
-        constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
-#pragma unroll
-        for (int k = 0; k < CHUNK / 16; ++k)
-          umma_bf16(t_o, make_smem_desc_sw128(smem_u32((k >> 2) ? sQ : sK) + (k & 3) * 32, 0, 1024),
-                    make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, k > 0);
-        umma_commit(&ofull[g]);
-      }
+      if (any_bad(ok)) break;
+      if (gt == 0) issue_o(0u, &ofull[g]);
       landed = 0;
       if (lane == 0) landed = mbar_wait(&ofull[g], k2 & 1, abort_flag) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
       tc_fence_after_sync();
+      if constexpr (PROMPT) {
+        if (open) {  // O += P_lo V
+          if (ok) {
+            for (int cc = 0; cc < 4; ++cc) {
+              uint32_t pk[16];
+              if (cc <= last_chunk) {
+                uint32_t v[32];
+                tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                  const float p0 = (cc * 32 + j <= gt) ? softmax_term(__uint_as_float(v[j]), row_max, kScale) : 0.f;
+                  const float p1 = (cc * 32 + j + 1 <= gt) ? softmax_term(__uint_as_float(v[j + 1]), row_max, kScale) : 0.f;
+                  const float2 back = __bfloat1622float2(__floats2bfloat162_rn(p0, p1));
+                  pk[j >> 1] = pack_bf16x2(p0 - back.x, p1 - back.y);
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) pk[j] = 0u;
+              }
+              store_p(cc, pk);
+            }
+          }
+          tc_fence_before_sync();
+          fence_proxy_async_smem();
+          if (any_bad(ok)) break;
+          if (gt == 0) issue_o(1u, &lowfull[g]);
+          landed = 0;
+          if (lane == 0) landed = mbar_wait(&lowfull[g], opens & 1, abort_flag) ? 1u : 0u;
+          ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
+          tc_fence_after_sync();
+          ++opens;
+        }
+      }
       if (ok) {
         // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
         const float inv_l = 1.f / row_sum;
@@ -950,6 +1039,7 @@ extern "C" int ws_memory_scan(const float* writes, const float* fast_logit, cons
                      init_slow, B, N, N, H, stream);
 }
 
+template <bool PROMPT>
 static int attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H, int d,
                     int* error_flag, cudaStream_t stream) {
   if (T <= 0 || d != H * HD) return -1;
@@ -963,7 +1053,7 @@ static int attn_fwd(const void* qkvgu, const void* states, const float* rope, vo
   if (rc) return rc;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AF_SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(attn_fwd_kernel<PROMPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AF_SMEM) != cudaSuccess)
       return -20;
     configured = true;
   }
@@ -972,22 +1062,22 @@ static int attn_fwd(const void* qkvgu, const void* states, const float* rope, vo
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(attn_fwd_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AS_SMEM) != cudaSuccess)
+        cudaFuncSetAttribute(attn_fwd_stream_kernel<PROMPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, AS_SMEM) != cudaSuccess)
       return -20;
   }
   if (ws_attn_stream_form() != 0)
-    launch_dependent(attn_fwd_stream_kernel, dim3(tiles < sms ? tiles : sms), dim3(AS_THREADS), AS_SMEM, stream, tm, ts, ty,
+    launch_dependent(attn_fwd_stream_kernel<PROMPT>, dim3(tiles < sms ? tiles : sms), dim3(AS_THREADS), AS_SMEM, stream, tm, ts, ty,
                      reinterpret_cast<const float2*>(rope), T, H, d, tiles, error_flag);
   else
-    launch_dependent(attn_fwd_kernel, dim3(tiles), dim3(128), AF_SMEM, stream, tm, ts, ty, reinterpret_cast<const float2*>(rope), T, H, d,
-                     error_flag);
+    launch_dependent(attn_fwd_kernel<PROMPT>, dim3(tiles), dim3(128), AF_SMEM, stream, tm, ts, ty,
+                     reinterpret_cast<const float2*>(rope), T, H, d, error_flag);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
 extern "C" int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H,
                            int d, int* error_flag, cudaStream_t stream) {
-  return T % CHUNK != 0 ? -1 : attn_fwd(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
+  return T % CHUNK != 0 ? -1 : attn_fwd<false>(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
 }
 
 extern "C" int ws_attn_prefill(const void* qkvgu, const float* rope, const float* fast_logit, const float* slow_logit,
@@ -999,7 +1089,7 @@ extern "C" int ws_attn_prefill(const void* qkvgu, const float* rope, const float
   if (!rc)
     rc = memory_scan(writes, fast_logit, slow_logit, mix_logit, states, fast, slow, mixed, nullptr, nullptr, B,
                      complete + (rest > 0), complete, H, stream);
-  if (!rc) rc = attn_fwd(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
+  if (!rc) rc = attn_fwd<true>(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
   if (rc) return rc;
   launch_dependent(open_chunk_kernel, dim3(B * H), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkvgu),
                    reinterpret_cast<const float2*>(rope), T, rest, H, d, static_cast<__nv_bfloat16*>(kc),
