@@ -38,7 +38,7 @@ int64_t opt_ld(const c10::optional<at::Tensor>& t) {
 void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_t epilogue,
           int64_t m, int64_t n, int64_t k, c10::optional<at::Tensor> out_, c10::optional<at::Tensor> out2,
           c10::optional<at::Tensor> aux, c10::optional<at::Tensor> row_scale, double alpha,
-          double beta, c10::optional<at::Tensor> error_flag) {
+          double beta, c10::optional<at::Tensor> error_flag, bool wide) {
   // the packed (up | gate) matrix of the SwiGLU epilogue is optional: only a backward pass reads it
   const bool has_out = out_.has_value() && out_->defined();
   TORCH_CHECK(has_out || (out2.has_value() && out2->defined()), "gemm: an output is required");
@@ -97,6 +97,7 @@ void gemm(const at::Tensor& a, const at::Tensor& b, bool a_mn, bool b_mn, int64_
   g.row_vec = nullptr;
   g.alpha = (float)alpha; g.beta = (float)beta;
   g.error_flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag)));
+  g.wide = wide;
   const int splits = ws_gemm_splits(&g);
   int rc;
   if (splits > 1) {
@@ -437,8 +438,8 @@ at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast
 // Smoke model (d 256, 4 depths, 2 x 512 tokens), forward + backward: 2.53 -> 2.03 ms.
 at::Tensor project(const at::Tensor& x, const at::Tensor& w, bool b_mn, int64_t epilogue, int64_t n, at::Tensor out,
                    const c10::optional<at::Tensor>& out2, const c10::optional<at::Tensor>& aux,
-                   const c10::optional<at::Tensor>& flag) {
-  gemm(x, w, false, b_mn, epilogue, x.size(0), n, x.size(1), out, out2, aux, c10::nullopt, 1.0, 0.0, flag);
+                   const c10::optional<at::Tensor>& flag, bool wide = false) {
+  gemm(x, w, false, b_mn, epilogue, x.size(0), n, x.size(1), out, out2, aux, c10::nullopt, 1.0, 0.0, flag, wide);
   return out;
 }
 at::Tensor project_bf16(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& flag) {
@@ -454,11 +455,11 @@ at::Tensor input_grad(const at::Tensor& dy, const at::Tensor& w, const c10::opti
 }
 
 // x2 = xmod + out_proj(y), then x2 + down(swiglu(up_gate(norm2 x2))).  -> (x2, rstd2, z2, packed, act, x3); packed only
-// with `keep` (the backward pass reads it), x3 only with `want_output`.
+// with `keep` (the backward pass reads it), x3 only with `want_output`.  `wide` (serving): (up, gate) are not rounded.
 struct BlockTail { at::Tensor x2, rstd2, z2, packed, act, x3; };
 BlockTail block_tail(const at::Tensor& y, const at::Tensor& xmod, const at::Tensor& w_out, const at::Tensor& n2,
                      const at::Tensor& w_ug, const at::Tensor& w_down, double eps, bool keep, bool want_output,
-                     const c10::optional<at::Tensor>& flag) {
+                     const c10::optional<at::Tensor>& flag, bool wide = false) {
   BlockTail t;
   t.x2 = project_residual(y, w_out, xmod, flag);
   at::Tensor unchanged;
@@ -466,7 +467,7 @@ BlockTail block_tail(const at::Tensor& y, const at::Tensor& xmod, const at::Tens
   const int64_t h = w_ug.size(0) / 2;
   if (keep) t.packed = at::empty({y.size(0), 2 * h}, y.options());
   t.act = at::empty({y.size(0), h}, y.options());
-  project(t.z2, w_ug, false, WS_EPI_SWIGLU, h, t.packed, t.act, c10::nullopt, flag);
+  project(t.z2, w_ug, false, WS_EPI_SWIGLU, h, t.packed, t.act, c10::nullopt, flag, wide);
   if (want_output) t.x3 = project_residual(t.act, w_down, t.x2, flag);
   return t;
 }
@@ -534,7 +535,7 @@ std::vector<at::Tensor> block_prefill(const at::Tensor& x, const at::Tensor& sca
     const int64_t d = x.size(1);
     return {xmod.view({B, T, d}).select(1, T - 1).contiguous(), y.view({B, T, d}).select(1, T - 1).contiguous()};
   }
-  return {block_tail(y, xmod, w_out, n2, w_ug, w_down, eps, false, true, flag).x3};
+  return {block_tail(y, xmod, w_out, n2, w_ug, w_down, eps, false, true, flag, true).x3};
 }
 
 // ----------------------------------------------------------------------------- optimizer
@@ -1253,7 +1254,7 @@ TORCH_LIBRARY(ws_b200, m) {
         "Tensor? skip=None) -> ()");
   m.def("gemm(Tensor a, Tensor b, bool a_mn, bool b_mn, int epilogue, int m, int n, int k, "
         "Tensor(a!)? out, Tensor(b!)? out2, Tensor? aux, Tensor? row_scale, float alpha, float beta, "
-        "Tensor(c!)? error_flag) -> ()");
+        "Tensor(c!)? error_flag, bool wide=False) -> ()");
   m.def("grad_weight_group(Tensor[] dys, Tensor[] xs, Tensor(a!)[] grads, float[] betas, Tensor(b!)? error_flag) -> ()");
 }
 

@@ -383,8 +383,8 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           uint32_t wu[16], wg[16], wa[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
-            const float u0 = bf16_round(__uint_as_float(ru[2 * i]) * rs), u1 = bf16_round(__uint_as_float(ru[2 * i + 1]) * rs);
-            const float g0 = bf16_round(__uint_as_float(rg[2 * i]) * rs), g1 = bf16_round(__uint_as_float(rg[2 * i + 1]) * rs);
+            const float u0 = swiglu_input(__uint_as_float(ru[2 * i]) * rs, p.wide), u1 = swiglu_input(__uint_as_float(ru[2 * i + 1]) * rs, p.wide);
+            const float g0 = swiglu_input(__uint_as_float(rg[2 * i]) * rs, p.wide), g1 = swiglu_input(__uint_as_float(rg[2 * i + 1]) * rs, p.wide);
             wu[i] = pack_bf16x2(u0, u1);
             wg[i] = pack_bf16x2(g0, g1);
             wa[i] = pack_bf16x2(g0 * sigmoidf_(g0) * u0, g1 * sigmoidf_(g1) * u1);
@@ -770,6 +770,7 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
   p.row_map = g->row_map;
   p.keep = g->keep; p.keep_rows = g->keep_rows < g->m ? g->keep_rows : g->m;
   p.whole_rows = g->whole != nullptr ? g->whole_rows : -1;
+  p.wide = g->wide;
   p.debug = 0;
   if (g->whole != nullptr) {  // the same boxes over the rows before their selection: A, or B of a weight gradient
     if (i != 0) return -9;

@@ -29,10 +29,12 @@ struct GemmParams {
   int whole_rows;
   void* keep;          // CE_FWD: see WsGemm
   int keep_rows;
+  int wide;            // SWIGLU: see WsGemm
   int debug;  // experiment switch: 1 = no loads (MMA issue rate only), 2 = always load tile (0,0)
 };
 
 __device__ __forceinline__ float sigmoidf_(float x) { return sigmoid_fast(x); }
+__device__ __forceinline__ float swiglu_input(float x, int wide) { return wide ? x : bf16_round(x); }
 
 // taddr: TMEM address of (this warp's first lane, first column of the accumulator buffer).
 // row: global output row of this thread; nb: N-tile index; egroup: which half of the columns.
@@ -139,7 +141,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, uint32_t tadd
   } else if constexpr (EPI == WS_EPI_SWIGLU) {
     // Accumulator columns 0..127 are `up`, 128..255 are `gate` of the same 128 features.
     // Both halves are rounded to BF16 first (what a BF16 GEMM would have returned); the
-    // activation is computed in FP32 from the rounded values and rounded once.
+    // activation is computed in FP32 from the rounded values (`wide`: from the accumulated ones) and rounded once.
     __nv_bfloat16* packed = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(row) * p.ldo;
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<size_t>(row) * p.ldo2;
     const int n0 = nb * 128;
@@ -161,10 +163,10 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, uint32_t tadd
             uint32_t* wa = reinterpret_cast<uint32_t*>(&va);
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-              const float u0 = bf16_round(__uint_as_float(ru[j + 2 * t]) * rs);
-              const float u1 = bf16_round(__uint_as_float(ru[j + 2 * t + 1]) * rs);
-              const float g0 = bf16_round(__uint_as_float(rg[j + 2 * t]) * rs);
-              const float g1 = bf16_round(__uint_as_float(rg[j + 2 * t + 1]) * rs);
+              const float u0 = swiglu_input(__uint_as_float(ru[j + 2 * t]) * rs, p.wide);
+              const float u1 = swiglu_input(__uint_as_float(ru[j + 2 * t + 1]) * rs, p.wide);
+              const float g0 = swiglu_input(__uint_as_float(rg[j + 2 * t]) * rs, p.wide);
+              const float g1 = swiglu_input(__uint_as_float(rg[j + 2 * t + 1]) * rs, p.wide);
               wu[t] = pack_bf16x2(u0, u1);
               wg[t] = pack_bf16x2(g0, g1);
               wa[t] = pack_bf16x2(g0 * sigmoidf_(g0) * u0, g1 * sigmoidf_(g1) * u1);

@@ -380,6 +380,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   p.alpha = g->alpha; p.beta = g->beta;
   p.error_flag = g->error_flag;
   p.limit = nullptr; p.row_map = nullptr; p.limit_from = p.whole_rows = p.keep_rows = 0; p.keep = nullptr;
+  p.wide = g->wide;
   p.debug = 0;
 
   const int n_tile = swiglu ? 128 : BN;

@@ -55,6 +55,7 @@ typedef struct WsGemm {
   int keep_rows;
   const void* whole;   // replaces A (a_mn: B) where *limit == whole_rows: the rows before their selection
   int whole_rows, ldwhole;
+  int wide;            // SWIGLU: the activation is formed from (up, gate) as accumulated, not from their BF16 values
 } WsGemm;
 
 int ws_gemm(const WsGemm* g, cudaStream_t stream);

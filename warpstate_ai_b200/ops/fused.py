@@ -556,8 +556,9 @@ def _prefill_norm(core, x, depth_scale, depth_bias):
 
 
 def _prefill_finish(core, y, xmod):
-    """The block after its attention, on rows ``[M, d]``; no backward pass follows, so (up | gate) is not written."""
+    """The block after its attention, on rows ``[M, d]``; no backward pass follows, so (up | gate) is not written, nor
+    rounded: the decode step keeps it in FP32, and a prompt's positions count as much as the tokens after it."""
     x2 = G.linear_residual(y, bf16_weight(core.out_proj.weight), xmod)
     z2, _, _ = _ops().rmsnorm_fwd(x2, None, None, core.norm2.weight.detach().float(), core.cfg.rms_eps, False)
-    _, act = G.linear_swiglu(z2, bf16_weight(core.ffn.up_gate.weight), want_packed=False)
+    _, act = G.linear_swiglu(z2, bf16_weight(core.ffn.up_gate.weight), want_packed=False, wide=True)
     return G.linear_residual(act, bf16_weight(core.ffn.down.weight), x2)

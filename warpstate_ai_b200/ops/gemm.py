@@ -74,14 +74,14 @@ def _policy_key(a_mn, b_mn, m, n, k) -> str:
     return f"fwd:{m}x{n}x{k}"
 
 
-def _gemm(a, b, a_mn, b_mn, epi, m, n, k, out, out2=None, aux=None, row_scale=None, alpha=1.0, beta=0.0):
+def _gemm(a, b, a_mn, b_mn, epi, m, n, k, out, out2=None, aux=None, row_scale=None, alpha=1.0, beta=0.0, wide=False):
     _ext.require()
     if _policy:
         choice = _policy.get(_policy_key(a_mn, b_mn, m, n, k))
         lib = _ext.cdll()
         lib.ws_gemm_set_pair_mode(-1 if choice is None else (1 if choice["kernel"] == "pair" else 0))
     torch.ops.ws_b200.gemm(a, b, a_mn, b_mn, epi, m, n, k, out, out2, aux, row_scale,
-                           float(alpha), float(beta), error_flag(a.device))
+                           float(alpha), float(beta), error_flag(a.device), wide)
     return out
 
 
@@ -114,18 +114,19 @@ def linear_residual(x: torch.Tensor, w: torch.Tensor, resid: torch.Tensor,
 
 
 def linear_swiglu(x: torch.Tensor, w_up_gate: torch.Tensor, row_scale: torch.Tensor | None = None,
-                  want_packed: bool = True):
+                  want_packed: bool = True, wide: bool = False):
     """Up/gate projection with the SwiGLU epilogue.
 
     ``w_up_gate`` is ``[2h, K]`` with the first ``h`` rows = up, last ``h`` rows = gate (the
     reference layout, warpstate/model.py:58-60).  Returns ``(packed [M,2h], act [M,h])``; ``packed`` is None with
-    ``want_packed=False`` (only a backward pass reads it).
+    ``want_packed=False`` (only a backward pass reads it).  The activation is formed from the BF16 values of up and gate,
+    as a backward pass will see them, or with ``wide`` from the FP32 ones.
     """
     m, k = x.shape
     h = w_up_gate.shape[0] // 2
     packed = torch.empty((m, 2 * h), dtype=torch.bfloat16, device=x.device) if want_packed else None
     act = torch.empty((m, h), dtype=torch.bfloat16, device=x.device)
-    _gemm(x, w_up_gate, False, False, EPI_SWIGLU, m, h, k, packed, out2=act, row_scale=row_scale)
+    _gemm(x, w_up_gate, False, False, EPI_SWIGLU, m, h, k, packed, out2=act, row_scale=row_scale, wide=wide)
     return packed, act
 
 
