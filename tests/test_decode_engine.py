@@ -353,3 +353,39 @@ def test_an_engine_first_used_in_inference_mode_can_be_used_outside_it():
     with torch.inference_mode():
         again = engine.prefill(ids)
         assert torch.equal(again, inside) and torch.equal(engine.step(torch.tensor([3, 4])), following)
+
+
+def test_only_a_captured_step_reads_ahead_of_its_turn(monkeypatch):
+    """The attention step may read the position before its predecessors are done only where a graph replay is what starts
+    it: a step launched kernel by kernel follows the kernel that writes the position at no such boundary."""
+    from collections import defaultdict
+    early = []
+
+    class Recorder:
+        def __getattr__(self, name):
+            return lambda *args: early.append(args[9] if len(args) > 9 else False) if name == "decode_attn" else None
+
+    engine = DecodeEngine(tiny(chunk=128), dtype=torch.float32, use_cuda_graph=False)
+    engine.new_state(2)
+    for w in engine.weights:
+        w.update(p_in=None, p_out=None, p_ug=None, p_down=None)
+    engine.head_packed, engine._kbufs = None, defaultdict(lambda: None)
+    monkeypatch.setattr(torch.ops, "ws_b200", Recorder(), raising=False)
+    engine.step(torch.zeros(2, dtype=torch.long))
+    assert early == [False] * 4
+    early.clear()
+    engine._step_fn(torch.zeros(2, dtype=torch.long), engine.pos_dev, replayed=True)
+    assert early == [True] * 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch", [1, 3])
+def test_steps_with_and_without_a_graph_agree_bit_for_bit(batch):
+    torch.manual_seed(batch)
+    cfg = WarpStateConfig(vocab_size=512, d_model=128, n_heads=2, n_cores=2, logical_depth=3, ffn_hidden=192,
+                          chunk_size=128, gradient_checkpointing=False, parallel_memory=True)
+    model = WarpStateLM(cfg).cuda().eval()
+    ids = torch.randint(0, 512, (batch, 140), device="cuda")          # over the end of a chunk
+    graph, single = DecodeEngine(model), DecodeEngine(model, use_cuda_graph=False)
+    for t in range(ids.shape[1]):
+        assert torch.equal(graph.step(ids[:, t]), single.step(ids[:, t])), t

@@ -76,7 +76,7 @@ def parts(batch: int, position: int = 0, only=None) -> None:
             if "in_proj" in chosen:
                 ops.decode_gemm(w["w_in"], k["n"], 5 * d, 0, k["qkvgu"], k["flag"], False)
             if "attention" in chosen:
-                ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, engine.h, k["y"])
+                ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, engine.h, k["y"], True)
             if "out_proj" in chosen:
                 ops.decode_gemm(w["w_out"], k["y"], d, 1, k["p_out"], k["flag"], False)
             if "norm" in chosen:

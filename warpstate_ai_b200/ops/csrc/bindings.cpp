@@ -1058,7 +1058,7 @@ void decode_reduce_norm(at::Tensor x, const c10::optional<at::Tensor>& partial, 
 }
 
 void decode_attn(const at::Tensor& qkvgu, at::Tensor kc, at::Tensor vc, at::Tensor uc, const at::Tensor& mixed,
-                 const at::Tensor& rope, const at::Tensor& pos, int64_t H, at::Tensor y) {
+                 const at::Tensor& rope, const at::Tensor& pos, int64_t H, at::Tensor y, bool early) {
   TORCH_CHECK(qkvgu.is_cuda() && qkvgu.scalar_type() == at::kBFloat16 && qkvgu.dim() == 2 && qkvgu.is_contiguous(),
               "decode_attn: qkvgu must be contiguous BF16 [batch, 5d]");
   const int64_t batch = qkvgu.size(0), d = qkvgu.size(1) / 5;
@@ -1075,7 +1075,7 @@ void decode_attn(const at::Tensor& qkvgu, at::Tensor kc, at::Tensor vc, at::Tens
   c10::cuda::CUDAGuard guard(qkvgu.device());
   check_rc(ws_decode_attn(qkvgu.data_ptr(), kc.data_ptr(), vc.data_ptr(), uc.data_ptr(), mixed.data_ptr(),
                           rope.data_ptr<float>(), reinterpret_cast<const long long*>(pos.data_ptr<int64_t>()), (int)batch,
-                          (int)H, (int)d, y.data_ptr(), cur_stream()), "decode_attn");
+                          (int)H, (int)d, y.data_ptr(), early, cur_stream()), "decode_attn");
 }
 
 void decode_layer_tail(const at::Tensor& w_out, const at::Tensor& w_ug, const at::Tensor& w_down,
@@ -1195,7 +1195,7 @@ TORCH_LIBRARY(ws_b200, m) {
         "Tensor slow_keep, Tensor mix) -> ()");
   m.def("decode_pick(Tensor logits, Tensor(a!) token, Tensor(b!)? history, Tensor(c!) cursor, Tensor(d!) pos) -> ()");
   m.def("decode_attn(Tensor qkvgu, Tensor(a!) kc, Tensor(b!) vc, Tensor(c!) uc, Tensor mixed, Tensor rope, Tensor pos, "
-        "int H, Tensor(d!) y) -> ()");
+        "int H, Tensor(d!) y, bool early=False) -> ()");
   m.def("rmsnorm_fwd(Tensor x, Tensor? col_scale, Tensor? col_bias, Tensor w, float eps, bool want_xmod) -> (Tensor, Tensor, Tensor)");
   m.def("rmsnorm_bwd(Tensor dz, Tensor x, Tensor rstd, Tensor w, Tensor? dres, Tensor? out_scale, bool want_bf16) -> (Tensor, Tensor, Tensor)");
   m.def("rmsnorm_bwd_mod(Tensor dz, Tensor xmod, Tensor rstd, Tensor w, Tensor dres, Tensor scale, Tensor bias) -> (Tensor, Tensor)");

@@ -348,12 +348,13 @@ __global__ void __launch_bounds__(128)
 decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __restrict__ kc,
                    __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc,
                    const __nv_bfloat16* __restrict__ mixed, const float2* __restrict__ rope,
-                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y) {
+                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool early) {
   constexpr int HD = 64, C = 128;
   __shared__ float sq[HD], sk[HD], sp[C], sl[16][HD + 1], sm[16][HD + 1], sred[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int h = blockIdx.x % H, b = blockIdx.x / H;
   pdl_launch_dependents();
+  if (!early) pdl_wait();
   int pos = static_cast<int>(*pos_ptr);
   pos = pos < 0 ? 0 : (pos >= C ? C - 1 : pos);
   const __nv_bfloat16* row = qkvgu + static_cast<size_t>(b) * 5 * d + h * HD;
@@ -361,10 +362,12 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
   // Thread (rg, jg) owns columns 8*jg .. 8*jg+7 of the rows rg, rg+16, ... of the K and V caches and of M: a warp
   // instruction reads four whole 128-byte rows.  Every load the step needs from the caches is issued here, before
   // the RoPE of the new token, so that the three dependent phases below (scores, softmax, P.V) wait for memory once.
-  // They are issued before the wait for the previous kernel, too, and run under the tail of the projection: the
-  // position, the cache rows before it and M are what the previous STEP left, and steps are separated by full
-  // dependencies (a graph replay, or the kernel that writes the position).  Only `row` is this step's.  With the same in
-  // the residual + norm kernel: 48 steps of 28 layers at batch 1 72.3 -> 64.9 ms, 40 of 8 layers at batch 64 32.7 -> 29.7.
+  // `early`: they are issued before the wait for the previous kernel, too, and run under the tail of the projection.  Only
+  // `row` is this step's; the position, the cache rows before it and M are what was there before the step, and a replay of
+  // the graph that captured the step starts after everything before it.  A step launched kernel by kernel has no such
+  // start: its first kernels may be resident while the kernel that writes the position still runs, and only the wait
+  // makes that visible.  With the same in the residual + norm kernel, 48 steps of 28 layers at batch 1: 72.3 -> 64.9 ms,
+  // 40 of 8 layers at batch 64: 32.7 -> 29.7.
   const int jg = tid & 7, rg = tid >> 3;
   uint4 kreg[C / 16], vreg[C / 16], mreg[HD / 16];
 #pragma unroll
@@ -379,7 +382,7 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
 #pragma unroll
   for (int it = 0; it < HD / 16; ++it) mreg[it] = *reinterpret_cast<const uint4*>(mbase + (rg + it * 16) * HD + jg * 8);
   const float2 cs = rope[pos * 32 + lane];
-  pdl_wait();
+  if (early) pdl_wait();
 #pragma unroll
   for (int it = 0; it < C / 16; ++it)
     if (rg + it * 16 == pos) vreg[it] = *reinterpret_cast<const uint4*>(row + 2 * d + jg * 8);  // the new token's own value row
@@ -511,7 +514,7 @@ __global__ void __launch_bounds__(128)
 decode_attn_rows_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __restrict__ kc,
                    __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc,
                    const __nv_bfloat16* __restrict__ mixed, const float2* __restrict__ rope,
-                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y) {
+                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool) {
   constexpr int HD = 64, C = 128;
   __shared__ float sq[HD], sk[HD], sp[C], sl[16][HD + 1], sm[16][HD + 1], sred[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -911,7 +914,7 @@ extern "C" int ws_decode_reduce_norm(float* x, const float* partial, int splits,
 }
 
 extern "C" int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, const void* mixed, const float* rope,
-                              const long long* pos, int batch, int H, int d, void* y, cudaStream_t stream) {
+                              const long long* pos, int batch, int H, int d, void* y, int early, cudaStream_t stream) {
   if (d != H * 64 || batch <= 0) return -1;
   // WS_DECODE_ATTN=rows selects the row-per-thread form of the kernel
   static const bool rows_form = [] {
@@ -923,7 +926,7 @@ extern "C" int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, c
       static_cast<const __nv_bfloat16*>(qkvgu),
       static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc),
       static_cast<const __nv_bfloat16*>(mixed), reinterpret_cast<const float2*>(rope), pos, H, d,
-      static_cast<__nv_bfloat16*>(y));
+      static_cast<__nv_bfloat16*>(y), early != 0);
   ws_count_launch();
   return err == cudaSuccess ? 0 : -21;
 }

@@ -85,13 +85,16 @@ int ws_decode_gemm_splits(int n, int k);
 int ws_decode_gemm(const void* w, const void* x, int n, int k, int batch, int epilogue, void* out, int ldo,
                    int* error_flag, int packed, cudaStream_t stream);
 // x (FP32 [batch, d], in place) = table[token] if token else x + sum of split partials; optional
-// depth modulation x*(1+scale)+bias; out (BF16 [batch, d], may be NULL) = RMSNorm(x) * w.
+// depth modulation x*(1+scale)+bias; out (BF16 [batch, d], may be NULL) = RMSNorm(x) * w.  scale, bias and w are read ahead
+// of the launches in front of this one, as the weights of ws_decode_gemm are: none of those may write them.
 int ws_decode_reduce_norm(float* x, const float* partial, int splits, const long long* token, const float* table,
                           int vocab, const float* scale, const float* bias, const float* w, float eps, int d,
                           int batch, void* out, cudaStream_t stream);
-// One decode step of the attention block for every (sequence, head); see decode_attn_kernel.
+// One decode step of the attention block for every (sequence, head); see decode_attn_kernel.  `early` reads pos, the cache
+// rows before it and mixed ahead of the launches in front of this one: only in a captured step, whose replay starts
+// after everything that wrote them.
 int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, const void* mixed, const float* rope,
-                   const long long* pos, int batch, int H, int d, void* y, cudaStream_t stream);
+                   const long long* pos, int batch, int H, int d, void* y, int early, cudaStream_t stream);
 
 // A finished chunk enters the memories of every (sequence, head), in place: kc, uc BF16 [batch, H, 128, 64]; fast, slow
 // FP32 and mixed BF16 [batch, H, 64, 64]; the decays and the mix [H] are the sigmoids of their logits.

@@ -197,7 +197,7 @@ class DecodeEngine:
                     (5 * d + 127) // 128, self.batch)
         return items <= torch.cuda.get_device_properties(self.device).multi_processor_count
 
-    def _step_kernels_tail(self, token: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+    def _step_kernels_tail(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool) -> torch.Tensor:
         """The step with one persistent launch per layer for everything after the attention (and the next layer's
         in_proj): 2 launches per layer instead of 7.  Bit-identical to `_step_kernels`."""
         ops = torch.ops.ws_b200
@@ -207,7 +207,7 @@ class DecodeEngine:
         ops.decode_reduce_norm(k["x"], None, token, self.embed, first["scale"], first["bias"], first["n1"], eps, k["n"])
         ops.decode_gemm(first["w_in"], k["n"], 5 * d, 0, k["qkvgu"], k["flag"], False)
         for index, (w, st) in enumerate(zip(self.weights, self.states)):
-            ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, self.h, k["y"])
+            ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, self.h, k["y"], replayed)
             nxt = self.weights[index + 1] if index + 1 < len(self.weights) else None
             ops.decode_layer_tail(w["w_out"], w["w_ug"], w["w_down"], nxt["w_in"] if nxt else None, k["y"], k["x"],
                                   k["p_out"], k["p_down"], k["n"], k["act"], k["qkvgu"], w["n2"],
@@ -216,9 +216,9 @@ class DecodeEngine:
         ops.decode_gemm(self.head, k["n"], self.cfg.vocab_size, 3, k["logits"], k["flag"], False)
         return k["logits"]
 
-    def _step_kernels(self, token: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+    def _step_kernels(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool) -> torch.Tensor:
         if self._layer_tail:
-            return self._step_kernels_tail(token, pos)
+            return self._step_kernels_tail(token, pos, replayed)
         ops = torch.ops.ws_b200
         k = self._kbufs
         d, ffn, eps = self.cfg.d_model, self.cfg.ffn_hidden, self.cfg.rms_eps
@@ -226,7 +226,7 @@ class DecodeEngine:
         ops.decode_reduce_norm(k["x"], None, token, self.embed, first["scale"], first["bias"], first["n1"], eps, k["n"])
         for index, (w, st) in enumerate(zip(self.weights, self.states)):
             ops.decode_gemm(w["p_in"], k["n"], 5 * d, 0, k["qkvgu"], k["flag"], self.pack_weights)
-            ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, self.h, k["y"])
+            ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, self.h, k["y"], replayed)
             ops.decode_gemm(w["p_out"], k["y"], d, 1, k["p_out"], k["flag"], self.pack_weights)
             ops.decode_reduce_norm(k["x"], k["p_out"], None, None, None, None, w["n2"], eps, k["n"])
             ops.decode_gemm(w["p_ug"], k["n"], ffn, 2, k["act"], k["flag"], self.pack_weights)
@@ -239,9 +239,11 @@ class DecodeEngine:
         ops.decode_gemm(self.head_packed, k["n"], self.cfg.vocab_size, 3, k["logits"], k["flag"], self.pack_weights)
         return k["logits"]
 
-    def _step_fn(self, token: torch.Tensor, pos: torch.Tensor) -> torch.Tensor:
+    def _step_fn(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool = False) -> torch.Tensor:
+        """``replayed``: the launches are being captured.  A replay starts after everything before it, which lets the
+        attention kernels read the position and the caches ahead of their turn; launched one by one they must not."""
         if self._kbufs is not None:
-            return self._step_kernels(token, pos)
+            return self._step_kernels(token, pos, replayed)
         return self._step_math(token, pos)
 
     def _norm(self, x, w):
@@ -366,7 +368,7 @@ class DecodeEngine:
         self._greedy_graph = torch.cuda.CUDAGraph()
         launched = _ext.launch_count()
         with torch.cuda.graph(self._greedy_graph):
-            logits = self._step_fn(self.token_buf, self.pos_dev)
+            logits = self._step_fn(self.token_buf, self.pos_dev, replayed=True)
             torch.ops.ws_b200.decode_pick(logits, self.token_buf, self.history, self.cursor, self.pos_dev)
         self.graph_counters.capture_calls += 1
         self.graph_counters.kernels_per_replay = _ext.launch_count() - launched
@@ -385,7 +387,7 @@ class DecodeEngine:
         self._graph = torch.cuda.CUDAGraph()
         launched = _ext.launch_count()
         with torch.cuda.graph(self._graph):
-            self.logits_buf = self._step_fn(self.token_buf, self.pos_dev)
+            self.logits_buf = self._step_fn(self.token_buf, self.pos_dev, replayed=True)
         self.graph_counters.capture_calls += 1
         self.graph_counters.kernels_per_replay = _ext.launch_count() - launched
 
