@@ -109,3 +109,20 @@ def test_comments_stand_on_their_own():
         for word in documents + other:
             assert word not in text, (p, word)
         assert not rounds.search(text), (p, rounds.search(text).group(0))
+
+
+def test_kernels_that_wait_for_their_predecessor_promise_no_read_only_inputs():
+    """``const T* __restrict__`` says that nobody writes the data while the kernel runs, so the compiler may move its loads
+    above ``griddepcontrol.wait``: a kernel that overlaps the one before it then reads what that one has not written yet."""
+    promise = re.compile(r"const\s+[A-Za-z_0-9 ]+\*\s*__restrict__")
+    waiting = 0
+    for p in NATIVE:
+        if p.suffix != ".cu":
+            continue
+        for kernel in p.read_text().split("__global__")[1:]:
+            head, body = kernel.split("{", 1)
+            if "pdl_wait()" not in body.split("\n}\n")[0]:
+                continue
+            waiting += 1
+            assert not promise.search(head), (p.name, head)
+    assert waiting > 20

@@ -29,7 +29,7 @@ constexpr int DS_SMEM = 3 * TILE_BYTES + 1024 + 128;
 
 __global__ void __launch_bounds__(128, 4)
 dstate_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_dy,
-              const __grid_constant__ CUtensorMap tm_out, const float2* __restrict__ rope, int T, int H, int d,
+              const __grid_constant__ CUtensorMap tm_out, const float2* rope, int T, int H, int d,
               int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -146,7 +146,7 @@ constexpr int DSS_SMEM = DSS_STAGES * 3 * TILE_BYTES + 2 * 16384 + 1024 + 256;
 
 __global__ void __launch_bounds__(DSS_THREADS, 1)
 dstate_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_dy,
-                     const __grid_constant__ CUtensorMap tm_out, const float2* __restrict__ rope, int T, int H, int d,
+                     const __grid_constant__ CUtensorMap tm_out, const float2* rope, int T, int H, int d,
                      int tiles, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -334,9 +334,9 @@ constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_VEC = 2;
 
 __global__ void __launch_bounds__(SCAN_THREADS, 3)
-memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict__ writes,
-                       const float* __restrict__ fast_logit, const float* __restrict__ slow_logit,
-                       const float* __restrict__ mix_logit, __nv_bfloat16* __restrict__ dwrites,
+memory_scan_bwd_kernel(const float* dstate, const float* writes,
+                       const float* fast_logit, const float* slow_logit,
+                       const float* mix_logit, __nv_bfloat16* __restrict__ dwrites,
                        float* __restrict__ partials, int B, int N, int H) {
   pdl_launch_dependents();
   pdl_wait();
@@ -434,8 +434,8 @@ memory_scan_bwd_kernel(const float* __restrict__ dstate, const float* __restrict
 // head's B * 16 partials.  One CTA per head, one warp per logit, fixed order.  (A launch in place of the sum, three
 // sigmoids and nine products that a framework expression of it takes: 15 launches of 2 us for 3 H numbers.)
 __global__ void __launch_bounds__(96)
-memory_logit_grads_kernel(const float* __restrict__ partials, const float* __restrict__ fast_logit,
-                          const float* __restrict__ slow_logit, const float* __restrict__ mix_logit, int B, int H,
+memory_logit_grads_kernel(const float* partials, const float* fast_logit,
+                          const float* slow_logit, const float* mix_logit, int B, int H,
                           float* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -478,7 +478,7 @@ constexpr int AB_SMEM = 4 * TILE_BYTES + 2 * TILE_BYTES + 2 * 8192 + 128;
 __global__ void __launch_bounds__(AB_THREADS, 2)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                 const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_dw,
-                const __grid_constant__ CUtensorMap tm_dout, const float2* __restrict__ rope, int T, int H, int d,
+                const __grid_constant__ CUtensorMap tm_dout, const float2* rope, int T, int H, int d,
                 int* error_flag) {
   extern __shared__ __align__(1024) uint8_t smem_ab[];
   uint8_t* smem = smem_ab;

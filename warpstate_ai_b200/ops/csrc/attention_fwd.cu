@@ -30,7 +30,7 @@ constexpr int WR_SMEM = 2 * TILE_BYTES + 1024 + 128;
 
 __global__ void __launch_bounds__(128, 6)
 chunk_writes_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_out,
-                    const float2* __restrict__ rope, int T, int H, int d, int* error_flag) {
+                    const float2* rope, int T, int H, int d, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* sK = smem;
@@ -145,7 +145,7 @@ constexpr int WS_SMEM = WS_STAGES * 2 * TILE_BYTES + 2 * 16384 + 1024 + 256;
 
 __global__ void __launch_bounds__(WS_THREADS, 1)
 chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_out,
-                           const float2* __restrict__ rope, int T, int H, int d, int tiles, int* error_flag) {
+                           const float2* rope, int T, int H, int d, int tiles, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* ring = smem;                                   // stage s: K at s * 32 KiB, U 16 KiB behind it
@@ -319,11 +319,11 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
 constexpr int SCAN_AHEAD = 8;
 
 __global__ void __launch_bounds__(128)
-memory_scan_kernel(const float* __restrict__ writes, const float* __restrict__ fast_logit,
-                   const float* __restrict__ slow_logit, const float* __restrict__ mix_logit,
+memory_scan_kernel(const float* writes, const float* fast_logit,
+                   const float* slow_logit, const float* mix_logit,
                    __nv_bfloat16* __restrict__ states, float* __restrict__ final_fast,
                    float* __restrict__ final_slow, __nv_bfloat16* __restrict__ final_mixed,
-                   const float* __restrict__ init_fast, const float* __restrict__ init_slow, int B, int N, int complete,
+                   const float* init_fast, const float* init_slow, int B, int N, int complete,
                    int H) {
   pdl_launch_dependents();
   pdl_wait();
@@ -375,7 +375,7 @@ memory_scan_kernel(const float* __restrict__ writes, const float* __restrict__ f
 // What a decode needs of the chunk a prompt ends in: roped K, V and U of its `rest` positions, as the step kernel
 // appends them, and zeros behind them (rest = 0 clears the caches).  One CTA per (sequence, head); 16-byte pieces.
 __global__ void __launch_bounds__(256)
-open_chunk_kernel(const __nv_bfloat16* __restrict__ qkvgu, const float2* __restrict__ rope, int T, int rest, int H, int d,
+open_chunk_kernel(const __nv_bfloat16* qkvgu, const float2* rope, int T, int rest, int H, int d,
                   __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc) {
   pdl_launch_dependents();
   pdl_wait();
@@ -424,7 +424,7 @@ constexpr int AF_SMEM = 4 * TILE_BYTES + 8192 + 1024 + 128;
 template <bool PROMPT>
 __global__ void __launch_bounds__(128, 3)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
-                const __grid_constant__ CUtensorMap tm_y, const float2* __restrict__ rope, int T, int H, int d,
+                const __grid_constant__ CUtensorMap tm_y, const float2* rope, int T, int H, int d,
                 int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -646,7 +646,7 @@ constexpr int AS_SMEM = AS_STAGES * AS_STAGE_BYTES + 1024 + 256;
 template <bool PROMPT>
 __global__ void __launch_bounds__(AS_THREADS, 1)
 attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
-                       const __grid_constant__ CUtensorMap tm_y, const float2* __restrict__ rope, int T, int H, int d,
+                       const __grid_constant__ CUtensorMap tm_y, const float2* rope, int T, int H, int d,
                        int tiles, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);

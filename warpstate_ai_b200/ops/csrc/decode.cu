@@ -254,9 +254,9 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 //   scale != null : x = x * (1 + scale) + bias    (depth modulation of the layer that follows)
 // then out = BF16(x * rsqrt(mean(x^2) + eps) * w).
 __global__ void __launch_bounds__(256)
-decode_reduce_norm_kernel(float* __restrict__ x, const float* __restrict__ partial, int splits,
-                          const long long* __restrict__ token, const float* __restrict__ table, int vocab,
-                          const float* __restrict__ scale, const float* __restrict__ bias, const float* __restrict__ w,
+decode_reduce_norm_kernel(float* x, const float* partial, int splits,
+                          const long long* token, const float* table, int vocab,
+                          const float* scale, const float* bias, const float* w,
                           float eps, int d, int batch, __nv_bfloat16* __restrict__ out) {
   __shared__ float red[8];
   pdl_launch_dependents();
@@ -345,10 +345,10 @@ decode_reduce_norm_kernel(float* __restrict__ x, const float* __restrict__ parti
 // y: [batch, d] BF16.  `pos_ptr` is the in-chunk position (device scalar, so that one captured
 // graph serves every position).
 __global__ void __launch_bounds__(128)
-decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __restrict__ kc,
-                   __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc,
-                   const __nv_bfloat16* __restrict__ mixed, const float2* __restrict__ rope,
-                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool early) {
+decode_attn_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bfloat16* vc,
+                   __nv_bfloat16* uc,
+                   const __nv_bfloat16* mixed, const float2* rope,
+                   const long long* pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool early) {
   constexpr int HD = 64, C = 128;
   __shared__ float sq[HD], sk[HD], sp[C], sl[16][HD + 1], sm[16][HD + 1], sred[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -511,10 +511,10 @@ decode_attn_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __res
 // y: [batch, d] BF16.  `pos_ptr` is the in-chunk position (device scalar, so that one captured
 // graph serves every position).
 __global__ void __launch_bounds__(128)
-decode_attn_rows_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* __restrict__ kc,
-                   __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc,
-                   const __nv_bfloat16* __restrict__ mixed, const float2* __restrict__ rope,
-                   const long long* __restrict__ pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool) {
+decode_attn_rows_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bfloat16* vc,
+                   __nv_bfloat16* uc,
+                   const __nv_bfloat16* mixed, const float2* rope,
+                   const long long* pos_ptr, int H, int d, __nv_bfloat16* __restrict__ y, bool) {
   constexpr int HD = 64, C = 128;
   __shared__ float sq[HD], sk[HD], sp[C], sl[16][HD + 1], sm[16][HD + 1], sred[4];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -652,10 +652,10 @@ decode_attn_rows_kernel(const __nv_bfloat16* __restrict__ qkvgu, __nv_bfloat16* 
 constexpr int CHUNK_END_SMEM = 2 * 128 * 64 * 4;
 
 __global__ void __launch_bounds__(256)
-decode_chunk_end_kernel(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat16* __restrict__ uc,
-                        float* __restrict__ fast, float* __restrict__ slow, __nv_bfloat16* __restrict__ mixed,
-                        const float* __restrict__ fast_keep, const float* __restrict__ slow_keep,
-                        const float* __restrict__ mix_of, int H) {
+decode_chunk_end_kernel(const __nv_bfloat16* kc, const __nv_bfloat16* uc,
+                        float* fast, float* slow, __nv_bfloat16* __restrict__ mixed,
+                        const float* fast_keep, const float* slow_keep,
+                        const float* mix_of, int H) {
   constexpr int HD = 64, C = 128;
   extern __shared__ float chunk_smem[];
   float* sK = chunk_smem;
@@ -720,9 +720,8 @@ decode_chunk_end_kernel(const __nv_bfloat16* __restrict__ kc, const __nv_bfloat1
 // [batch, capacity]; CTA 0 then advances the in-chunk position and the cursor.  With this kernel as the last node of
 // the step graph a greedy decode needs nothing from the host between steps.
 __global__ void __launch_bounds__(256)
-decode_pick_kernel(const float* __restrict__ logits, int vocab, long long* __restrict__ token,
-                   long long* __restrict__ history, int capacity, long long* __restrict__ cursor,
-                   long long* __restrict__ pos) {
+decode_pick_kernel(const float* logits, int vocab, long long* __restrict__ token,
+                   long long* __restrict__ history, int capacity, long long* cursor, long long* pos) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float best_v[8];

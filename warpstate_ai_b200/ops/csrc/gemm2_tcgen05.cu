@@ -809,8 +809,8 @@ static int fill_swiglu_maps(const WsGemm* g0, PairGroup& grp) {
 // kernel adds in order, with the epilogue of the whole: one thread per four columns.
 template <int EPI>
 __global__ void __launch_bounds__(256)
-split_finish_kernel(const float* __restrict__ part, int splits, int m, int n, const void* __restrict__ aux, int ldaux,
-                    const float* __restrict__ row_scale, void* __restrict__ out, int ldo) {
+split_finish_kernel(const float* part, int splits, int m, int n, const void* aux, int ldaux,
+                    const float* row_scale, void* __restrict__ out, int ldo) {
   pdl_launch_dependents();
   pdl_wait();
   const int per_row = n / 4;

@@ -17,9 +17,9 @@ extern "C" void ws_count_launch(void);
 // One warp per row.  parts: float2 [rows, ld] with `nparts` valid entries per row.
 // lse[row] = log sum_j exp(logit_j);  logp[row] = label_logit - lse (0 where label == ignore).
 __global__ void __launch_bounds__(256)
-ce_combine_kernel(const float2* __restrict__ parts, int ld, int nparts, const float* __restrict__ label_logit,
-                  const long long* __restrict__ labels, long long ignore_index, int rows, const int* __restrict__ index,
-                  const int* __restrict__ count, float* __restrict__ lse_out, float* __restrict__ logp_out) {
+ce_combine_kernel(const float2* parts, int ld, int nparts, const float* label_logit,
+                  const long long* labels, long long ignore_index, int rows, const int* index,
+                  const int* count, float* __restrict__ lse_out, float* __restrict__ logp_out) {
   pdl_launch_dependents();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -59,7 +59,7 @@ constexpr int SELECT_ITEMS = 16;
 constexpr int SELECT_PAD = 256;   // rows of a tile of the CTA-pair GEMM
 
 __global__ void __launch_bounds__(SELECT_THREADS)
-select_rows_kernel(const long long* __restrict__ labels, long long ignore_index, int rows, int* __restrict__ index,
+select_rows_kernel(const long long* labels, long long ignore_index, int rows, int* __restrict__ index,
                    int* __restrict__ count, long long* __restrict__ labels_sel, float* __restrict__ logp) {
   __shared__ int counts[SELECT_ITEMS * 32];   // labelled rows per (item, warp), then those before it
   __shared__ int total;
@@ -128,8 +128,8 @@ select_rows_kernel(const long long* __restrict__ labels, long long ignore_index,
 
 // One warp per row of 16-byte pieces (d % 8 == 0).
 __global__ void __launch_bounds__(256)
-gather_rows_kernel(const __nv_bfloat16* __restrict__ in, int ld, const int* __restrict__ index,
-                   const int* __restrict__ count, int rows, int d, __nv_bfloat16* __restrict__ out) {
+gather_rows_kernel(const __nv_bfloat16* in, int ld, const int* index,
+                   const int* count, int rows, int d, __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
   const int n = *count, row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -145,7 +145,7 @@ gather_rows_kernel(const __nv_bfloat16* __restrict__ in, int ld, const int* __re
 }
 
 __global__ void __launch_bounds__(256)
-clear_unlabelled_kernel(const long long* __restrict__ labels, long long ignore_index, int rows, int d,
+clear_unlabelled_kernel(const long long* labels, long long ignore_index, int rows, int d,
                         __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -161,9 +161,9 @@ clear_unlabelled_kernel(const long long* __restrict__ labels, long long ignore_i
 constexpr int DLOGITS_PAD = 64;   // rows per k-block of the weight gradient
 
 __global__ void __launch_bounds__(256)
-ce_dlogits_kernel(__nv_bfloat16* __restrict__ logits, int vocab, const long long* __restrict__ labels_sel,
-                  const int* __restrict__ index, const float* __restrict__ lse_in, const float* __restrict__ row_weight,
-                  const int* __restrict__ count, int start, int rows) {
+ce_dlogits_kernel(__nv_bfloat16* logits, int vocab, const long long* labels_sel,
+                  const int* index, const float* lse_in, const float* row_weight,
+                  const int* count, int start, int rows) {
   pdl_launch_dependents();
   pdl_wait();
   const int row = blockIdx.x;

@@ -43,8 +43,8 @@ __device__ __forceinline__ void st4(__nv_bfloat16* p, float4 v) {
 // x_mod = x * (1 + col_scale) + col_bias (when given); z = bf16(x_mod * rstd * w).
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
-rmsnorm_fwd_kernel(const T* __restrict__ x, const float* __restrict__ col_scale,
-                   const float* __restrict__ col_bias, const float* __restrict__ w, float eps, int rows,
+rmsnorm_fwd_kernel(const T* x, const float* col_scale,
+                   const float* col_bias, const float* w, float eps, int rows,
                    int d, T* __restrict__ xmod_out, __nv_bfloat16* __restrict__ z,
                    float* __restrict__ rstd_out) {
   pdl_launch_dependents();
@@ -92,8 +92,8 @@ rmsnorm_fwd_kernel(const T* __restrict__ x, const float* __restrict__ col_scale,
 // x is read from memory once, and all CHUNKS loads of a lane are in flight together.
 template <typename T, int CHUNKS>
 __global__ void __launch_bounds__(ROW_THREADS)
-rmsnorm_fwd_rows_kernel(const T* __restrict__ x, const float* __restrict__ col_scale,
-                        const float* __restrict__ col_bias, const float* __restrict__ w, float eps, int rows,
+rmsnorm_fwd_rows_kernel(const T* x, const float* col_scale,
+                        const float* col_bias, const float* w, float eps, int rows,
                         T* __restrict__ xmod_out, __nv_bfloat16* __restrict__ z, float* __restrict__ rstd_out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -167,11 +167,11 @@ __device__ __forceinline__ void st8(T* p, const float (&v)[8]) {
 
 template <typename T, bool MOD = false>
 __global__ void __launch_bounds__(ROW_THREADS, MOD ? 2 : 3)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x,
-                   const float* __restrict__ rstd_in, const float* __restrict__ w,
-                   const T* __restrict__ dres, const float* __restrict__ out_scale, int rows, int d,
+rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
+                   const float* rstd_in, const float* w,
+                   const T* dres, const float* out_scale, int rows, int d,
                    T* __restrict__ dx_out, __nv_bfloat16* __restrict__ dx_bf16,
-                   float* __restrict__ dw_partial, const float* __restrict__ mod_bias) {
+                   float* __restrict__ dw_partial, const float* mod_bias) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[2][RB_ROWS][ROW_WARPS];
@@ -271,7 +271,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dz, const T* __restrict__ x
 // partial_a[block] = sum_rows a ; partial_ab[block] = sum_rows a*b  (a, b: [rows, d])
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
-colsum2_kernel(const T* __restrict__ a, const T* __restrict__ b, int rows, int d,
+colsum2_kernel(const T* a, const T* b, int rows, int d,
                float* __restrict__ partial_a, float* __restrict__ partial_ab) {
   pdl_launch_dependents();
   pdl_wait();
@@ -299,8 +299,8 @@ colsum2_kernel(const T* __restrict__ a, const T* __restrict__ b, int rows, int d
 // flight), then the eight warp sums are combined in a fixed order: the result is deterministic.
 constexpr int FIN_COLS = 32;
 __global__ void __launch_bounds__(ROW_THREADS)
-colsum_finalize_kernel(const float* __restrict__ partial, int parts, int d,
-                       const float* __restrict__ inv_scale, int inv_plane, float beta, float* __restrict__ out) {
+colsum_finalize_kernel(const float* partial, int parts, int d,
+                       const float* inv_scale, int inv_plane, float beta, float* out) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[ROW_WARPS][FIN_COLS];
@@ -334,7 +334,7 @@ colsum_finalize_kernel(const float* __restrict__ partial, int parts, int d,
 }
 
 // --------------------------------------------------------------------------- casts
-__global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void cast_f32_bf16_kernel(const float* in, __nv_bfloat16* __restrict__ out,
                                      size_t n4) {
   pdl_launch_dependents();
   pdl_wait();

@@ -105,6 +105,10 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
 // Programmatic dependent launch: `pdl_wait` returns once every grid this one depends on has completed
 // and its writes are visible (a no-op for a normally launched grid); `pdl_launch_dependents` lets the
 // next grid of the stream start its prologue once every CTA of this grid has issued it or exited.
+// What a kernel reads after it waits is not `__restrict__`, constant or not.  The promise says that nothing else writes
+// that memory while the kernel runs, the asm statement here included, so a load may be moved above the wait.  (In the
+// attention step of a decode the load of the new token's V row was: captured steps from position 16 on used the row that
+// an earlier launch had left there.)  Pure outputs keep it, which is enough for loads to pass stores.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
