@@ -389,3 +389,53 @@ def test_steps_with_and_without_a_graph_agree_bit_for_bit(batch):
     graph, single = DecodeEngine(model), DecodeEngine(model, use_cuda_graph=False)
     for t in range(ids.shape[1]):
         assert torch.equal(graph.step(ids[:, t]), single.step(ids[:, t])), t
+
+
+def test_prefill_casts_what_its_last_kernels_read_ahead_before_its_first_kernel(monkeypatch):
+    """The weight-streaming kernels at the end of a prefill request their weights before the launches in front of them are
+    done.  Nothing but a launch that starts after everything before it, the embedding gather, orders them behind a cast."""
+    from collections import defaultdict
+    from types import SimpleNamespace
+    from warpstate_ai_b200.ops import fused
+    engine = DecodeEngine(tiny(chunk=128), dtype=torch.float32, use_cuda_graph=False)
+    engine.new_state(1)
+    engine._kbufs = defaultdict(lambda: None)
+    happened, last = [], engine.model.cores[(engine.cfg.logical_depth - 1) % engine.cfg.n_cores]
+    watched = {id(p): name for name, p in dict(out=last.out_proj.weight, up=last.ffn.up_gate.weight, down=last.ffn.down.weight).items()}
+
+    class Table:
+        def __getitem__(self, ids):
+            happened.append("gather")
+            return torch.zeros(*ids.shape, engine.cfg.d_model)
+
+    monkeypatch.setattr(fused, "bf16_weight", lambda p: happened.append(watched.get(id(p), "other")) or p)
+    monkeypatch.setattr(fused, "core_prefill_state",
+                        lambda core, x, scale, bias, b, t, state, last: happened.append("block") or ((x[:b], x[:b]) if last else x))
+    monkeypatch.setattr(torch.ops, "ws_b200", SimpleNamespace(decode_gemm=lambda *a: happened.append("gemm"),
+                                                              decode_reduce_norm=lambda *a: None), raising=False)
+    engine.embed = Table()
+    engine._prefill_whole(torch.zeros(1, 5, dtype=torch.long))
+    start = happened.index("gather")
+    assert {"out", "up", "down"} <= set(happened[:start]) and not {"out", "up", "down", "other"} & set(happened[start:])
+    assert happened.count("gemm") == 4 and happened.count("block") == 4
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [5, 128, 200])
+def test_prefill_with_a_gemm_policy_equals_the_native_one(monkeypatch, length):
+    """A policy takes the block launch by launch from Python, with its casts between the launches: the same kernels on the
+    same numbers, right after construction and after an update of the weights."""
+    from warpstate_ai_b200.ops import gemm
+    torch.manual_seed(length)
+    cfg = WarpStateConfig(vocab_size=512, d_model=128, n_heads=2, n_cores=2, logical_depth=3, ffn_hidden=192,
+                          chunk_size=128, gradient_checkpointing=False, parallel_memory=True)
+    model = WarpStateLM(cfg).cuda().eval().requires_grad_(False)
+    ids = torch.randint(0, 512, (2, length), device="cuda")
+    for _ in range(3):
+        monkeypatch.setattr(gemm, "_policy", {"fwd:0x0x0": {"kernel": "pair", "sm_limit": 0}})
+        by_policy = DecodeEngine(model).prefill(ids).clone()
+        monkeypatch.setattr(gemm, "_policy", {})
+        assert torch.equal(by_policy, DecodeEngine(model).prefill(ids))
+        for p in model.parameters():
+            p.mul_(1.25)
+    gemm.check_device_errors()

@@ -428,15 +428,24 @@ class DecodeEngine:
         from ..ops import fused
         model, (b, t) = self.model, ids.shape
         self._reuse_state(b)
+        # The kernels that finish the last block request their weights ahead of the launches in front of them, so these are
+        # cast before the gather of the embeddings, which starts after all that came before and which all that follows waits for.
+        finish = self._finish_weights(model.cores[(len(self.states) - 1) % self.cfg.n_cores])
         x = self.embed[ids].float().view(b * t, -1)
         for depth, st in enumerate(self.states):
             last = depth + 1 == len(self.states)
             core = model.cores[depth % self.cfg.n_cores]
             x = fused.core_prefill_state(core, x, model.depth_scale[depth], model.depth_bias[depth], b, t, st, last)
         self.pos = t % self.chunk
-        return self._prefill_logits(core, *x)
+        return self._prefill_logits(core, *x, *finish)
 
-    def _prefill_logits(self, core, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
+    @staticmethod
+    def _finish_weights(core):
+        from ..ops import fused
+        return (fused.bf16_weight(core.out_proj.weight), core.norm2.weight.detach().float(),
+                fused.bf16_weight(core.ffn.up_gate.weight), fused.bf16_weight(core.ffn.down.weight))
+
+    def _prefill_logits(self, core, x: torch.Tensor, y: torch.Tensor, out, norm2, up_gate, down) -> torch.Tensor:
         """Logits from the last block's residual input ``x [B, d]`` (FP32) and attention output ``y [B, d]``: the rows
         of one decode step, so they take its weight-streaming kernels where those apply."""
         from ..ops import fused
@@ -444,9 +453,8 @@ class DecodeEngine:
             return F.linear(self._norm(fused._prefill_finish(core, y, x), self.final_norm), self.head).float()
         ops, k, eps = torch.ops.ws_b200, self._kbufs, self.cfg.rms_eps
         d, ffn = self.cfg.d_model, self.cfg.ffn_hidden
-        out, up_gate, down = (fused.bf16_weight(w) for w in (core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight))
         ops.decode_gemm(out, y, d, 1, k["p_out"], k["flag"], False)
-        ops.decode_reduce_norm(x, k["p_out"], None, None, None, None, core.norm2.weight.detach().float(), eps, k["n"])
+        ops.decode_reduce_norm(x, k["p_out"], None, None, None, None, norm2, eps, k["n"])
         ops.decode_gemm(up_gate, k["n"], ffn, 2, k["act"], k["flag"], False)
         ops.decode_gemm(down, k["act"], d, 1, k["p_down"], k["flag"], False)
         ops.decode_reduce_norm(x, k["p_down"], None, None, None, None, self.final_norm, eps, k["n"])
