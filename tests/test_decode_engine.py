@@ -439,3 +439,28 @@ def test_prefill_with_a_gemm_policy_equals_the_native_one(monkeypatch, length):
         for p in model.parameters():
             p.mul_(1.25)
     gemm.check_device_errors()
+
+
+def test_ids_of_an_open_chunk_are_taken_as_a_step_takes_them():
+    """The step kernel clamps an id to the vocabulary; a prompt's open chunk, which used to be stepped, reads no further."""
+    engine = DecodeEngine(tiny(chunk=8), dtype=torch.float32, use_cuda_graph=False)
+    ids = torch.tensor([[1, 2, 3, 4, 5, 6, 7, 96, -5, 97, 96, 2 ** 40]])
+    kept = ids.clone()
+    assert engine._gathered_ids(ids)[0].tolist() == [1, 2, 3, 4, 5, 6, 7, 96, 0, 96, 96, 96]
+    assert torch.equal(ids, kept)
+    assert engine._gathered_ids(torch.tensor([[3, 200]], dtype=torch.uint8)).tolist() == [[3, 96]]
+    whole = torch.tensor([[1, 2, 3, 4, 5, 6, 7, 97]])                 # a complete chunk is refused by the gather, as before
+    assert engine._gathered_ids(whole).tolist() == whole.tolist()
+
+
+@pytest.mark.gpu
+def test_a_prompt_with_ids_outside_the_vocabulary_in_its_open_chunk():
+    torch.manual_seed(0)
+    cfg = WarpStateConfig(vocab_size=512, d_model=128, n_heads=2, n_cores=2, logical_depth=3, ffn_hidden=192,
+                          chunk_size=128, gradient_checkpointing=False, parallel_memory=True)
+    engine = DecodeEngine(WarpStateLM(cfg).cuda().eval())
+    ids = torch.randint(0, 512, (2, 140), device="cuda")
+    ids[0, 130], ids[1, 139] = -3, 4000
+    logits = engine.prefill(ids).clone()
+    assert torch.equal(logits, engine.prefill(torch.cat((ids[:, :128], ids[:, 128:].clamp(0, 511)), dim=1)))
+    assert torch.isfinite(logits).all()

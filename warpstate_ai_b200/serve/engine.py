@@ -431,13 +431,20 @@ class DecodeEngine:
         # The kernels that finish the last block request their weights ahead of the launches in front of them, so these are
         # cast before the gather of the embeddings, which starts after all that came before and which all that follows waits for.
         finish = self._finish_weights(model.cores[(len(self.states) - 1) % self.cfg.n_cores])
-        x = self.embed[ids].float().view(b * t, -1)
+        x = self.embed[self._gathered_ids(ids)].float().view(b * t, -1)
         for depth, st in enumerate(self.states):
             last = depth + 1 == len(self.states)
             core = model.cores[depth % self.cfg.n_cores]
             x = fused.core_prefill_state(core, x, model.depth_scale[depth], model.depth_bias[depth], b, t, st, last)
         self.pos = t % self.chunk
         return self._prefill_logits(core, *x, *finish)
+
+    def _gathered_ids(self, ids: torch.Tensor) -> torch.Tensor:
+        """``ids`` as indexes of the embedding table.  In the chunk a prompt ends in they are taken as `step` takes them: any
+        integer type, and an id outside the vocabulary is the nearest one in it."""
+        ids = ids.to(torch.long, copy=True)
+        ids[:, ids.shape[1] // self.chunk * self.chunk:].clamp_(0, self.cfg.vocab_size - 1)
+        return ids
 
     @staticmethod
     def _finish_weights(core):
