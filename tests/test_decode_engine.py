@@ -464,3 +464,13 @@ def test_a_prompt_with_ids_outside_the_vocabulary_in_its_open_chunk():
     logits = engine.prefill(ids).clone()
     assert torch.equal(logits, engine.prefill(torch.cat((ids[:, :128], ids[:, 128:].clamp(0, 511)), dim=1)))
     assert torch.isfinite(logits).all()
+
+
+@pytest.mark.parametrize("heads,ffn,dtype,takes", [(2, 192, torch.float32, True), (2, 192, torch.bfloat16, True),
+                                                   (3, 192, torch.float32, False), (2, 100, torch.float32, False),
+                                                   (2, 192, torch.float16, False)])
+def test_which_models_prefill_in_one_pass(heads, ffn, dtype, takes):
+    cfg = WarpStateConfig(vocab_size=64, d_model=64 * heads, n_heads=heads, n_cores=1, logical_depth=1, ffn_hidden=ffn,
+                          chunk_size=128, gradient_checkpointing=False, parallel_memory=True)
+    engine = DecodeEngine(WarpStateLM(cfg).eval().to(dtype), dtype=torch.float32, use_cuda_graph=False)
+    assert engine._whole_prompt_kernels() is takes

@@ -147,3 +147,17 @@ def test_activation_of_a_prompt_is_rounded_once(rows, d, ffn):
     u, g = packed.double().chunk(2, dim=-1)
     want = u * g * torch.sigmoid(g)
     assert rel(rounded, want) < 1.1 * rel(want.bfloat16(), want)
+
+
+@pytest.mark.parametrize("heads,ffn,dtype,use_kernels", [(3, 192, torch.float32, True), (1, 64, torch.float32, True),
+                                                         (2, 100, torch.float32, False), (2, 192, torch.float16, False)])
+def test_short_prompts_of_models_outside_the_tile_kernels(heads, ffn, dtype, use_kernels):
+    """Widths that are no multiple of 128, an FFN that is none of 8, half-precision weights: stepped, as ever."""
+    model = model_of(heads, ffn).to(dtype)
+    ids = torch.randint(0, 512, (2, 21), device="cuda")
+    engine = DecodeEngine(model, use_kernels=use_kernels)
+    logits = engine.prefill(ids[:, :20]).clone()
+    after = engine.step(ids[:, 20])
+    check_device_errors()
+    wide = model.float()
+    assert rel(logits, expected_state(wide, ids[:, :20])[0]) < 0.02 and rel(after, expected_state(wide, ids)[0]) < 0.02

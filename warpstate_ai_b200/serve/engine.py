@@ -420,8 +420,12 @@ class DecodeEngine:
             return fused.active(self.embed)
 
     def _whole_prompt_kernels(self) -> bool:
+        """Widths and weights that the row and tile kernels take.  The step kernels take more of them: a prompt of a model
+        with an odd number of heads, or with half-precision weights, is stepped past its complete chunks."""
         from ..ops import attention
-        return all(attention.geometry_ok(core) for core in self.model.cores)
+        return (self.cfg.d_model % 128 == 0 and self.cfg.ffn_hidden % 8 == 0
+                and all(attention.geometry_ok(core) and core.in_proj.weight.dtype in (torch.float32, torch.bfloat16)
+                        for core in self.model.cores))
 
     def _prefill_whole(self, ids: torch.Tensor) -> torch.Tensor:
         """The prompt in one pass: every layer's state is overwritten by its kernels, so nothing is cleared first."""
