@@ -119,3 +119,32 @@ def test_streaming_tile_kernels_equal_the_one_tile_per_cta_kernels(batch, seq, h
     check_device_errors()
     for mine, theirs in zip(results[1], results[0]):
         assert torch.equal(mine, theirs)
+
+
+@pytest.mark.parametrize("block", [0, 1, 2])
+def test_backward_where_a_block_of_scores_overflows(block):
+    """Scores of 32 columns that are -inf (a product of Q and K beyond FP32) have no weight; where they are all that one
+    of a row's two threads sees, the other one decides the row."""
+    from warpstate_ai_b200.ops import attention, reference as R
+    from warpstate_ai_b200.ops.gemm import check_device_errors
+    torch.manual_seed(block)
+    core = make_core(1)
+    packed = torch.randn(128, 5, 64, device="cuda")
+    packed[:, :2, 62:] = 0.0                       # the slowest rotary pair: all but constant within a chunk
+    packed[32:, 0, 62] = 1e20
+    packed[32 * block:32 * block + 32, 1, 62] = -1e20
+    qkvgu = packed.view(128, 320).bfloat16()
+    if block == 0:                                 # rows 32..63 still see columns 32..63; those of the first block see theirs
+        assert float(qkvgu[:32, 62].abs().max()) == 0.0
+    dy = torch.randn(128, 64, device="cuda").bfloat16()
+    y, saved = attention.forward(qkvgu, core, 1, 128)
+    dq, *_ = attention.backward(dy, qkvgu, saved, core, 1, 128)
+    check_device_errors()
+    leaf = qkvgu.double().view(1, 128, 320).requires_grad_(True)
+    ref = R.attention_memory(leaf, core.fast_decay_logit.double(), core.slow_decay_logit.double(),
+                             core.memory_mix_logit.double(), 1, 128, True, core.rope_cos.double(), core.rope_sin.double())
+    (want,) = torch.autograd.grad(ref, leaf, dy.double().view(1, 128, 64))
+    assert torch.isfinite(y).all() and torch.isfinite(dq).all()
+    got, want = (t.view(128, 5, 64)[..., :62] for t in (dq, want))
+    for index, name in enumerate(("dQ", "dK", "dV", "dGate", "dU")):
+        assert rel_l2(got[:, index], want[:, index]) < 0.02, name      # as without an overflow

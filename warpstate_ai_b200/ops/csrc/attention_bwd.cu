@@ -590,7 +590,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 
   // ---- softmax over this thread's two blocks of columns, {half, half + 2} x 32, held in registers: one TMEM read and
   // one exponential per score.  The two threads of a row meet once, with (max, sum) of their columns, in the State
-  // tile's space (the State has been consumed); a block behind the causal mask counts as (-inf, 0).
+  // tile's space (the State has been consumed); a block behind the causal mask counts as (-inf, 0), and so does a half
+  // whose visible scores are all -inf (a product that overflowed): the other half decides the row.
   const float kScale = 0.125f * 1.4426950408889634f;
   float* meet = reinterpret_cast<float*>(sSt);   // [2][128] max | [2][128] sum | [2][128] D
   float e[2][32];
@@ -609,12 +610,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       }
     }
   }
+  const float from = my_max == -INFINITY ? 0.f : my_max;
 #pragma unroll
   for (int k = 0; k < 2; ++k) {
     if (half + 2 * k <= quarter) {
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
-        e[k][j] = exp2f((e[k][j] - my_max) * kScale);
+        e[k][j] = exp2f((e[k][j] - from) * kScale);
         my_sum += e[k][j];
       }
     }
