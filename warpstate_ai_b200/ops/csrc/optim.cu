@@ -30,11 +30,15 @@ __device__ __forceinline__ double block_sum(double v, double* smem) {
   return s;  // valid in warp 0
 }
 
+__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+
 // Sum of squares of a fixed, contiguous slice of g per block (slice size is a function of n and gridDim only, so the
-// summation order is reproducible).  Four squares are added in FP32 and everything above them in FP64: arenas that hold
-// the same gradients in another order (sharded, replicated) then agree on the norm to the last bit, where FP32 sums
-// left them an ulp apart, and a clip coefficient an ulp apart turns into other signs of near-zero AdamW steps.  The
-// block's sum leaves as two floats, partial[block] + partial[gridDim + block].  Still bound by the 4 bytes per element.
+// summation order is reproducible).  Four squares are added in FP32 and everything above them in FP64: what arenas that
+// hold the same gradients in another order (sharded, replicated) differ by is then far below an ulp of the FP32 norm, and
+// as a rule they round to the same one; FP32 sums left them an ulp apart, and a clip coefficient an ulp apart turns into
+// other signs of near-zero AdamW steps.  (Sums of the fused reduction over several GPUs, `sumsq_out`, are FP32.)  The
+// block's sum leaves as two floats, partial[block] + partial[gridDim + block]; one past FP32 is infinite and has no rest.
+// Still bound by the 4 bytes per element.
 __global__ void __launch_bounds__(OPT_THREADS)
 sumsq_kernel(const float* __restrict__ g, size_t n4, float* __restrict__ partial) {
   __shared__ double red[32];
@@ -51,11 +55,9 @@ sumsq_kernel(const float* __restrict__ g, size_t n4, float* __restrict__ partial
   if (threadIdx.x == 0) {
     const float high = static_cast<float>(s);
     partial[blockIdx.x] = high;
-    partial[gridDim.x + blockIdx.x] = static_cast<float>(s - static_cast<double>(high));
+    partial[gridDim.x + blockIdx.x] = not_finite(high) ? 0.f : static_cast<float>(s - static_cast<double>(high));
   }
 }
-
-__device__ __forceinline__ bool not_finite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
 
 // stats[0] = ||g||, stats[1] = clip coefficient min(1, max_norm/(||g||+1e-6)), stats[2] = ||g||^2,
 // stats[3] = skip flag: 1 when the norm is not finite or `status` (optional device word of a
