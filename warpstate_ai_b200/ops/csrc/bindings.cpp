@@ -208,23 +208,29 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz,
   return {dx, dxb, dw};
 }
 
-// The norm behind a depth modulation (FP32 stream): -> (dx, FP32 [3, d]: gradients of w, of the bias, of the scale)
-std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const at::Tensor& xmod, const at::Tensor& rstd,
-                                                   const at::Tensor& w, const at::Tensor& dres, const at::Tensor& scale,
-                                                   const at::Tensor& bias) {
+// The norm behind a depth modulation (FP32 stream): -> (dx, FP32 [3, d]: gradients of w, of the bias, of the scale).  From
+// the modulation's input x; a caller that has only its output xmod gets x back as (xmod - bias) / (1 + scale), 0 where
+// scale is -1, with an error of an ulp of xmod over 1 + scale.
+std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const c10::optional<at::Tensor>& xmod,
+                                                   const at::Tensor& rstd, const at::Tensor& w, const at::Tensor& dres,
+                                                   const at::Tensor& scale, const at::Tensor& bias,
+                                                   const c10::optional<at::Tensor>& x_) {
+  const bool given = x_.has_value() && x_->defined();
+  TORCH_CHECK(given || (xmod.has_value() && xmod->defined()), "rmsnorm_bwd_mod: x or xmod");
   TORCH_CHECK(dz.is_cuda() && dz.scalar_type() == at::kBFloat16 && dz.is_contiguous(), "rmsnorm_bwd_mod: dz");
-  for (const at::Tensor* t : {&xmod, &dres})
+  const at::Tensor x = given ? *x_ : ((*xmod - bias) / (1.0 + scale)).masked_fill_(scale == -1.0, 0.0);
+  for (const at::Tensor* t : {&x, &dres})
     TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->sizes() == dz.sizes(),
-                "rmsnorm_bwd_mod: xmod and dres must be FP32 [rows, d]");
-  const int rows = (int)xmod.size(0), d = (int)xmod.size(1);
+                "rmsnorm_bwd_mod: x and dres must be FP32 [rows, d]");
+  const int rows = (int)x.size(0), d = (int)x.size(1);
   for (const at::Tensor* t : {&w, &scale, &bias})
     TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == d, "rmsnorm_bwd_mod: vectors must be FP32 [d]");
   TORCH_CHECK(rstd.scalar_type() == at::kFloat && rstd.is_contiguous() && rstd.numel() == rows, "rmsnorm_bwd_mod: rstd");
-  c10::cuda::CUDAGuard guard(xmod.device());
-  at::Tensor dx = at::empty_like(xmod);
-  at::Tensor partial = at::empty({3, ws_rmsnorm_bwd_mod_parts(rows), d}, xmod.options());
-  at::Tensor grads = at::empty({3, d}, xmod.options());
-  check_rc(ws_rmsnorm_bwd_mod(dz.data_ptr(), xmod.data_ptr<float>(), rstd.data_ptr<float>(), w.data_ptr<float>(),
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor dx = at::empty_like(x);
+  at::Tensor partial = at::empty({3, ws_rmsnorm_bwd_mod_parts(rows), d}, x.options());
+  at::Tensor grads = at::empty({3, d}, x.options());
+  check_rc(ws_rmsnorm_bwd_mod(dz.data_ptr(), x.data_ptr<float>(), rstd.data_ptr<float>(), w.data_ptr<float>(),
                               dres.data_ptr<float>(), scale.data_ptr<float>(), bias.data_ptr<float>(), rows, d,
                               dx.data_ptr<float>(), partial.data_ptr<float>(), grads.data_ptr<float>(), cur_stream()),
            "rmsnorm_bwd_mod");
@@ -491,8 +497,8 @@ std::vector<at::Tensor> block_fwd(const at::Tensor& x, const c10::optional<at::T
 
 // Backward up to the gradient of the block's input; the weight gradients follow as one group (grad_weight_group).
 // -> (dx, dx3 BF16, dpacked, dx2 BF16, dqkvgu, g_norm2, logit gradients [3, H], first norm's [3, d] or [1, d]): w, and
-// behind an FP32 depth modulation its bias and scale.
-std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& xmod, const at::Tensor& rstd1,
+// behind an FP32 depth modulation its bias and scale.  x: the norm's input, or behind an FP32 modulation that one's.
+std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& x, const at::Tensor& rstd1,
                                   const at::Tensor& qkvgu, const at::Tensor& x2, const at::Tensor& rstd2,
                                   const at::Tensor& packed, const at::Tensor& writes, const at::Tensor& states,
                                   const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& bias,
@@ -512,10 +518,10 @@ std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& xmod,
   at::Tensor logits = memory_logit_grads(partials, fast_logit, slow_logit, mix_logit, B);
   at::Tensor dz1 = input_grad(dqkvgu, w_in, flag);
   if (scale.has_value() && scale->defined() && !bf16_stream) {
-    auto [dx, norm] = rmsnorm_bwd_mod(dz1, xmod, rstd1, n1, dx2, *scale, *bias);
+    auto [dx, norm] = rmsnorm_bwd_mod(dz1, c10::nullopt, rstd1, n1, dx2, *scale, *bias, x);
     return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm};
   }
-  auto [dx, unused, g_n1] = rmsnorm_bwd(dz1, xmod, rstd1, n1, dx2, scale, false);
+  auto [dx, unused, g_n1] = rmsnorm_bwd(dz1, x, rstd1, n1, dx2, scale, false);
   return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, g_n1.unsqueeze(0)};
 }
 
@@ -1198,7 +1204,8 @@ TORCH_LIBRARY(ws_b200, m) {
         "int H, Tensor(d!) y, bool early=False) -> ()");
   m.def("rmsnorm_fwd(Tensor x, Tensor? col_scale, Tensor? col_bias, Tensor w, float eps, bool want_xmod) -> (Tensor, Tensor, Tensor)");
   m.def("rmsnorm_bwd(Tensor dz, Tensor x, Tensor rstd, Tensor w, Tensor? dres, Tensor? out_scale, bool want_bf16) -> (Tensor, Tensor, Tensor)");
-  m.def("rmsnorm_bwd_mod(Tensor dz, Tensor xmod, Tensor rstd, Tensor w, Tensor dres, Tensor scale, Tensor bias) -> (Tensor, Tensor)");
+  m.def("rmsnorm_bwd_mod(Tensor dz, Tensor? xmod, Tensor rstd, Tensor w, Tensor dres, Tensor scale, Tensor bias, "
+        "Tensor? x=None) -> (Tensor, Tensor)");
   m.def("colsum2(Tensor a, Tensor b, Tensor? inv_scale) -> (Tensor, Tensor)");
   m.def("cast_bf16(Tensor x, Tensor(a!)? out) -> Tensor");
   m.def("embed_fwd(Tensor ids, Tensor table, bool out_bf16) -> Tensor");
@@ -1232,7 +1239,7 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("block_fwd(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
         "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
         "bool keep, bool want_output, Tensor(a!)? flag) -> Tensor[]");
-  m.def("block_bwd(Tensor dx3, Tensor xmod, Tensor rstd1, Tensor qkvgu, Tensor x2, Tensor rstd2, Tensor packed, Tensor writes, "
+  m.def("block_bwd(Tensor dx3, Tensor x, Tensor rstd1, Tensor qkvgu, Tensor x2, Tensor rstd2, Tensor packed, Tensor writes, "
         "Tensor states, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor w_in, Tensor w_out, Tensor w_ug, Tensor w_down, "
         "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, int B, int T, int H, Tensor(a!)? flag) -> Tensor[]");
   m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "

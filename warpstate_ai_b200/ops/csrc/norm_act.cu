@@ -147,11 +147,12 @@ rmsnorm_fwd_rows_kernel(const T* x, const float* col_scale,
 // once with 16/32-byte coalesced accesses, the per-row mean needs one block reduction per group
 // (double-buffered, one __syncthreads), and the weight-gradient column sums stay in 8 registers.
 //
-// MOD (FP32 stream, the norm behind a depth modulation xmod = x * (1 + scale) + bias): the gradients of scale and bias
-// are column sums of dxmod * x and dxmod, and dxmod is in registers here, as is xmod, which gives x * (1 + scale) =
-// xmod - bias.  Summed in the same pass they cost 16 registers; as a pass of their own (colsum2_kernel, still used for
-// the BF16 stream, whose rounded xmod does not give x back) 268 MB more per 16384 x 2048 rows.  A block's forward +
-// backward there: 6.55 -> 6.39 ms; at 1792 x 1280, where the launches count, 691 -> 604 us.
+// MOD (FP32 stream, the norm behind a depth modulation xmod = x * (1 + scale) + bias): `x` is the modulation's input and
+// xmod is formed again from it.  The gradients of scale and bias are column sums of dxmod * x and dxmod, and dxmod is in
+// registers here; x is what it was, so nothing is lost where the bias is much larger than x * (1 + scale).  Summed in the
+// same pass they cost 16 registers; as a pass of their own (colsum2_kernel, still used for the BF16 stream, whose xmod is
+// rounded) 268 MB more per 16384 x 2048 rows.  A block's forward + backward at 1792 x 1280, where the launches count:
+// 691 -> 604 us; at 16384 x 2048 within the noise of 6.5 ms.
 constexpr int RB_ROWS = 2;
 
 template <typename T>
@@ -180,11 +181,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
   const bool active = c < d;
   const float inv_d = 1.0f / static_cast<float>(d);
   float wv[8], sv[8], acc[8];
-  [[maybe_unused]] float acc_bias[8], acc_scale[8];
+  [[maybe_unused]] float bi[8], acc_bias[8], acc_scale[8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) { wv[j] = 0.f; sv[j] = 1.f; acc[j] = 0.f; acc_bias[j] = 0.f; acc_scale[j] = 0.f; }
+  for (int j = 0; j < 8; ++j) { wv[j] = 0.f; sv[j] = 1.f; bi[j] = 0.f; acc[j] = 0.f; acc_bias[j] = 0.f; acc_scale[j] = 0.f; }
   if (active) {
     ld8(w + c, wv);
+    if constexpr (MOD) ld8(mod_bias + c, bi);
     if (out_scale != nullptr) {
       ld8(out_scale + c, sv);
 #pragma unroll
@@ -213,6 +215,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
     for (int r = 0; r < RB_ROWS; ++r) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
+        if constexpr (MOD) xh[r][j] = xh[r][j] * sv[j] + bi[j];
         xh[r][j] *= rs[r];
         part[r] += g[r][j] * wv[j] * xh[r][j];
       }
@@ -242,13 +245,12 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
           for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
         if constexpr (MOD) {
-          float xm[8], bi[8];
-          ld8(x + base, xm);      // in L1 since the first pass over the row
-          ld8(mod_bias + c, bi);
+          float xv[8];
+          ld8(x + base, xv);      // in L1 since the first pass over the row
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             acc_bias[j] += o[j];
-            acc_scale[j] += o[j] * (xm[j] - bi[j]);
+            acc_scale[j] += o[j] * xv[j];
           }
         }
 #pragma unroll
@@ -294,13 +296,13 @@ colsum2_kernel(const T* a, const T* b, int rows, int d,
 }
 
 // out[c] = beta*out[c] + scale(c) * sum_p partial[p][c];  scale(c) = 1/(1+inv_scale[c]) if given.  gridDim.y sums of
-// that kind lie behind one another ([gridDim.y][parts][d] -> [gridDim.y][d]); only sum `inv_plane` is scaled.
+// that kind lie behind one another ([gridDim.y][parts][d] -> [gridDim.y][d]).
 // One block per 32 columns; warp w sums parts w, w+8, ... (independent 128-byte loads in
 // flight), then the eight warp sums are combined in a fixed order: the result is deterministic.
 constexpr int FIN_COLS = 32;
 __global__ void __launch_bounds__(ROW_THREADS)
 colsum_finalize_kernel(const float* partial, int parts, int d,
-                       const float* inv_scale, int inv_plane, float beta, float* out) {
+                       const float* inv_scale, float beta, float* out) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red[ROW_WARPS][FIN_COLS];
@@ -325,7 +327,7 @@ colsum_finalize_kernel(const float* partial, int parts, int d,
     float s = 0.f;
 #pragma unroll
     for (int wi = 0; wi < ROW_WARPS; ++wi) s += red[wi][lane];
-    if (inv_scale != nullptr && static_cast<int>(blockIdx.y) == inv_plane) {
+    if (inv_scale != nullptr) {
       const float den = 1.f + inv_scale[c];
       s = den != 0.f ? s / den : 0.f;
     }
@@ -475,17 +477,17 @@ extern "C" int ws_rmsnorm_bwd_mod_parts(int rows) {
   return blocks < 148 * 2 ? (blocks > 0 ? blocks : 1) : 148 * 2;
 }
 
-extern "C" int ws_rmsnorm_bwd_mod(const void* dz, const float* xmod, const float* rstd, const float* w, const float* dres,
+extern "C" int ws_rmsnorm_bwd_mod(const void* dz, const float* x, const float* rstd, const float* w, const float* dres,
                                   const float* scale, const float* bias, int rows, int d, float* dx_out,
                                   float* partial, float* grads, cudaStream_t stream) {
   if (d % 128 != 0 || d > ROW_THREADS * 8 || rows <= 0) return -1;
   const int parts = ws_rmsnorm_bwd_mod_parts(rows);
   launch_dependent(rmsnorm_bwd_kernel<float, true>, dim3(parts), dim3(ROW_THREADS), 0, stream,
-                   static_cast<const __nv_bfloat16*>(dz), xmod, rstd, w, dres, scale, rows, d, dx_out,
+                   static_cast<const __nv_bfloat16*>(dz), x, rstd, w, dres, scale, rows, d, dx_out,
                    static_cast<__nv_bfloat16*>(nullptr), partial, bias);
   ws_count_launch();
   launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS, 3), dim3(ROW_THREADS), 0, stream, partial,
-                   parts, d, scale, 2, 0.f, grads);
+                   parts, d, nullptr, 0.f, grads);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -507,7 +509,7 @@ extern "C" int ws_colsum2(const void* a, const void* b, int is_bf16, int rows, i
 
 extern "C" int ws_colsum_finalize(const float* partial, int parts, int d, const float* inv_scale, float beta,
                                   float* out, cudaStream_t stream) {
-  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, partial, parts, d, inv_scale, 0, beta, out);
+  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, partial, parts, d, inv_scale, beta, out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
@@ -623,7 +625,7 @@ extern "C" int ws_rmsnorm_bwd_static(const void* dz, const void* x, int x_bf16, 
     launch_dependent(rmsnorm_bwd_kernel<float>, dim3(parts), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const float*)x, rstd, w, (const float*)dres, out_scale, rows, d,
         (float*)dx_out, (__nv_bfloat16*)dx_bf16, scratch, nullptr);
   ws_count_launch();
-  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, scratch, parts, d, nullptr, 0, 0.f, dw_out);
+  launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(ROW_THREADS), 0, stream, scratch, parts, d, nullptr, 0.f, dw_out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : WS_STATIC_ERR_LAUNCH;
 }

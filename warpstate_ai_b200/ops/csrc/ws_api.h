@@ -140,10 +140,10 @@ int ws_rmsnorm_bwd_parts(int rows);
 int ws_rmsnorm_bwd(const void* dz, const void* x, int x_bf16, const float* rstd, const float* w,
                    const void* dres, const float* out_scale, int rows, int d, void* dx_out,
                    void* dx_bf16, float* dw_partial, cudaStream_t stream);
-// The same behind a depth modulation xmod = x * (1 + scale) + bias, FP32 stream: dx_out is the gradient of x, and grads
-// [3, d] those of w, bias and scale.  partial: 3 * ws_rmsnorm_bwd_mod_parts(rows) rows of d floats.
+// The same behind a depth modulation xmod = x * (1 + scale) + bias, FP32 stream, from x itself: dx_out is its gradient, and
+// grads [3, d] those of w, bias and scale.  partial: 3 * ws_rmsnorm_bwd_mod_parts(rows) rows of d floats.
 int ws_rmsnorm_bwd_mod_parts(int rows);
-int ws_rmsnorm_bwd_mod(const void* dz, const float* xmod, const float* rstd, const float* w, const float* dres,
+int ws_rmsnorm_bwd_mod(const void* dz, const float* x, const float* rstd, const float* w, const float* dres,
                        const float* scale, const float* bias, int rows, int d, float* dx_out, float* partial,
                        float* grads, cudaStream_t stream);
 // Column sums of a and a*b over rows, as ws_colsum_parts(rows) partial rows.

@@ -267,9 +267,9 @@ class CoreFn(torch.autograd.Function):
             ctx.save_for_backward(x_in, scale if has_mod else dummy, bias if has_mod else dummy, n1w, n2w)
         else:
             ctx.attn_saved = attn_saved
-            # the block's input is read again only where its modulated copy is rounded (`_modulation_sums`)
-            ctx.save_for_backward(x_in if has_mod and x_in.dtype != torch.float32 else xmod, xmod, rstd1, z1, qkvgu, y, x2,
-                                  rstd2, z2, packed, act, scale if has_mod else dummy, bias if has_mod else dummy, n1w, n2w)
+            # the modulated copy of the block's input is read again only where it is rounded (a BF16 stream)
+            ctx.save_for_backward(x_in, xmod if x_in.dtype != torch.float32 else x_in, rstd1, z1, qkvgu, y, x2, rstd2, z2,
+                                  packed, act, scale if has_mod else dummy, bias if has_mod else dummy, n1w, n2w)
         return x3.view(batch, seq, d)
 
     @staticmethod
@@ -298,9 +298,10 @@ class CoreFn(torch.autograd.Function):
         stream_bf16 = dx3.dtype == torch.bfloat16
         g_scale = g_bias = side = None
         modulated = ctx.has_mod and not stream_bf16
+        norm_in = x_in if modulated else xmod
         if _native(core, weights) and attn_saved is not None:
             dx_in, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm = ops.block_bwd(
-                dx3, xmod, rstd1, qkvgu, x2, rstd2, packed, *attn_saved, scale if ctx.has_mod else None,
+                dx3, norm_in, rstd1, qkvgu, x2, rstd2, packed, *attn_saved, scale if ctx.has_mod else None,
                 bias if ctx.has_mod else None, n1w.detach().float(), n2w.detach().float(), bw_in, bw_out, bw_ug, bw_down,
                 *_native_arguments(core, dx3.device), batch, seq, core.h, G.error_flag(dx3.device))
             g_fast, g_slow, g_mix = logits.unbind(0)
@@ -322,10 +323,10 @@ class CoreFn(torch.autograd.Function):
             del dy
             dz1 = G.grad_input(dqkvgu, bw_in)
             if modulated:
-                dx_in, sums = ops.rmsnorm_bwd_mod(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale, bias)
+                dx_in, sums = ops.rmsnorm_bwd_mod(dz1, None, rstd1, n1w.detach().float(), dx2, scale, bias, norm_in)
                 g_n1, g_bias, g_scale = sums.unbind(0)
             else:
-                dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, xmod, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
+                dx_in, _, g_n1 = ops.rmsnorm_bwd(dz1, norm_in, rstd1, n1w.detach().float(), dx2, scale if ctx.has_mod else None, False)
         if ctx.has_mod and not modulated:
             g_bias, g_scale, side = _modulation_sums(dx_in, x_in, scale)
         # ---- the four weight gradients, deferred to one grouped launch (their tiles share waves)
