@@ -96,3 +96,26 @@ def test_kept_logits_give_the_bits_of_recomputed_ones(monkeypatch, rows, kept, k
     assert torch.equal(mine[0], recomputed[0]) and torch.equal(twice[0], recomputed[0])
     # the weight gradient is added up over blocks of rows, which end elsewhere: FP32 additions in another order
     assert rel(mine[1], recomputed[1]) < 1e-5 and rel(twice[1], recomputed[1]) < 1e-5
+
+
+def test_scratch_of_the_recomputed_rows_has_their_number(monkeypatch):
+    """A few rows past the kept ones take a few rows of logits beside them, not a whole block."""
+    _ext.require()
+    torch.manual_seed(0)
+    rows, kept, d, vocab = 4096 + 40, 4096, 64, 8192
+    monkeypatch.setattr(lmhead, "KEEP_BYTES", 2 * vocab * kept)
+    hidden = torch.randn(rows, d, device="cuda").bfloat16().requires_grad_(True)
+    weight = (torch.randn(vocab, d, device="cuda") * 0.05).requires_grad_(True)
+    labels = torch.randint(0, vocab, (rows,), device="cuda")
+    peak = None
+    for _ in range(2):                                       # once to have casts, flags and cached gradients in place
+        hidden.grad = weight.grad = None
+        value = lmhead.token_logps(hidden, weight, labels).sum()
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        value.backward()
+        peak = torch.cuda.max_memory_allocated() - before
+    check_device_errors()
+    small = rows * d * 2 + 2 * vocab * d * 4 + rows * 16     # dhidden, the FP32 weight gradient (once more as autograd's), vectors
+    assert peak < small + 40 * vocab * 2 + (1 << 20), peak

@@ -741,7 +741,7 @@ void lm_head_bwd_labelled(const at::Tensor& hidden, const at::Tensor& packed, co
                              index.data_ptr<int>() + start, lse.data_ptr<float>() + start, row_weight.data_ptr<float>(),
                              count.data_ptr<int>(), start, here, cur_stream()), "ce_dlogits");
     } else {
-      if (!scratch.defined()) scratch = at::empty({std::min<int64_t>(block, rows), vocab}, hidden.options());
+      if (!scratch.defined()) scratch = at::empty({here, vocab}, hidden.options());   // the first block is the largest
       dlogits = scratch.data_ptr();
       WsGemm g = {};
       g.a = from_start(packed); g.b = weight.data_ptr();
