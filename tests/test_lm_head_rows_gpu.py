@@ -119,3 +119,48 @@ def test_scratch_of_the_recomputed_rows_has_their_number(monkeypatch):
     check_device_errors()
     small = rows * d * 2 + 2 * vocab * d * 4 + rows * 16     # dhidden, the FP32 weight gradient (once more as autograd's), vectors
     assert peak < small + 40 * vocab * 2 + (1 << 20), peak
+
+
+def head_problem(rows=777, d=256, vocab=1000):
+    torch.manual_seed(rows)
+    hidden = torch.randn(rows, d, device="cuda").bfloat16()
+    labels, _ = labels_with("random", rows, vocab)
+    return hidden, torch.randn(vocab, d, device="cuda") * 0.05, labels, torch.randn(rows, device="cuda")
+
+
+def test_kept_logits_are_saved_tensors():
+    """Hooks on saved tensors (offload, checkpointing) see all that the head holds between its passes, and what they
+    give back is what the backward pass uses."""
+    _ext.require()
+    hidden, weight, labels, coef = head_problem()
+    plain_h, plain_w = hidden.clone().requires_grad_(True), weight.clone().requires_grad_(True)
+    (lmhead.token_logps(plain_h, plain_w, labels) * coef).sum().backward()
+    packed_shapes = []
+
+    def pack(t):
+        packed_shapes.append((t.dtype, tuple(t.shape)))
+        return t.cpu()
+
+    h, w = hidden.clone().requires_grad_(True), weight.clone().requires_grad_(True)
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+        value = (lmhead.token_logps(h, w, labels) * coef).sum()
+    assert (torch.bfloat16, (777, 1000)) in packed_shapes
+    for index in range(2):                                   # the second time the hooks give fresh logits back
+        h.grad = w.grad = None
+        value.backward(retain_graph=index == 0)
+        assert torch.equal(h.grad, plain_h.grad) and torch.equal(w.grad, plain_w.grad)
+
+
+def test_checkpointing_the_head_holds_no_logits():
+    _ext.require()
+    from torch.utils.checkpoint import checkpoint
+    hidden, weight, labels, coef = head_problem(rows=2048, d=64, vocab=8192)
+    plain_h, plain_w = hidden.clone().requires_grad_(True), weight.clone().requires_grad_(True)
+    (lmhead.token_logps(plain_h, plain_w, labels) * coef).sum().backward()
+    h, w = hidden.clone().requires_grad_(True), weight.clone().requires_grad_(True)
+    before = torch.cuda.memory_allocated()
+    value = (checkpoint(lmhead.token_logps, h, w, labels, use_reentrant=False) * coef).sum()
+    assert torch.cuda.memory_allocated() - before < 2 * 2048 * 8192 // 4     # the logits are 32 MiB
+    value.backward()
+    check_device_errors()
+    assert torch.equal(h.grad, plain_h.grad) and rel(w.grad, plain_w.grad) < 1e-6

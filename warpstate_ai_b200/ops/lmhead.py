@@ -58,8 +58,9 @@ class _TokenLogps(torch.autograd.Function):
         ctx.selected = hidden.shape[0] >= SELECT_FROM and ops.gemm_pair_available()
         if ctx.selected:
             keep = kept_rows(hidden.shape[0], wb.shape[0]) if keep else 0
-            logp, *rest, ctx.logits = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, keep, flag)
+            logp, *rest = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, keep, flag)
             ctx.save_for_backward(hidden, labels, *rest)
+            ctx.spent = False
             return logp
         lse, logp = ops.lm_head_fwd(hidden, wb, labels, IGNORE, flag)
         ctx.save_for_backward(hidden, labels, lse)
@@ -79,9 +80,11 @@ class _TokenLogps(torch.autograd.Function):
         main = getattr(weight, "main_grad", None)
         grad_w = main if main is not None else torch.zeros(weight.shape, dtype=torch.float32, device=weight.device)
         if ctx.selected:
-            index, count, packed, labels_sel = selection
+            index, count, packed, labels_sel, logits = selection
             # the logits become their own gradients: another backward over the same graph computes them again
-            logits, ctx.logits = ctx.logits, ctx.logits.new_empty(0)
+            if ctx.spent:
+                logits = logits.new_empty(0)
+            ctx.spent = True
             ops.lm_head_bwd_labelled(hidden, packed, wb, labels, labels_sel, index, count, lse, row_weight, IGNORE,
                                      ROWS_PER_BLOCK, logits, dh, grad_w, flag)
             return dh, (None if main is not None else grad_w.to(weight.dtype)), None, None
