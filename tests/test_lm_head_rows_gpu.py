@@ -164,3 +164,23 @@ def test_checkpointing_the_head_holds_no_logits():
     value.backward()
     check_device_errors()
     assert torch.equal(h.grad, plain_h.grad) and rel(w.grad, plain_w.grad) < 1e-6
+
+
+@pytest.mark.parametrize("checkpointing,holds", [(False, True), (True, False)])
+def test_a_model_that_checkpoints_its_blocks_keeps_no_logits(checkpointing, holds):
+    _ext.require()
+    from warpstate_ai_b200 import WarpStateConfig, WarpStateLM
+    cfg = WarpStateConfig(vocab_size=8192, d_model=128, n_heads=2, n_cores=1, logical_depth=1, ffn_hidden=192, chunk_size=128,
+                          gradient_checkpointing=checkpointing, parallel_memory=True)
+    with torch.device("cuda"):
+        model = WarpStateLM(cfg).train()
+    hidden = torch.randn(2, 1024, 128, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
+    targets = torch.randint(0, 8192, (2, 1024), device="cuda")
+    for _ in range(2):
+        before = torch.cuda.memory_allocated()
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            loss = model.loss_from_hidden(hidden, targets)
+        held = torch.cuda.memory_allocated() - before
+        loss.backward()
+        del loss
+    assert (held > 2048 * 8192 * 2) is holds                 # 32 MiB of logits

@@ -504,12 +504,13 @@ class LMHeadLossFn(torch.autograd.Function):
         return dh, (None if main is not None else grad_w.to(weight.dtype)), None
 
 
-def lm_head_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
+def lm_head_loss(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor,
+                 keep_bytes: int | None = None) -> torch.Tensor:
     if hidden.dtype != torch.bfloat16:
         hidden = hidden.to(torch.bfloat16)
     from . import lmhead
     if lmhead.kernels_ready(hidden, weight):
-        return lmhead.loss_sum(hidden, weight, labels)
+        return lmhead.loss_sum(hidden, weight, labels, keep_bytes)
     return LMHeadLossFn.apply(hidden, weight, labels)
 
 

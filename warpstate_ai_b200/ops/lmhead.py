@@ -27,14 +27,17 @@ IGNORE = -100
 # Below one tile of the CTA-pair GEMM there is nothing to leave out, and the single-CTA kernel is the faster one.
 SELECT_FROM = 512
 ROWS_PER_BLOCK = 8192  # bounds the BF16 dlogits scratch to 512 MiB at vocab 32768
-# Logits kept between the passes: 16384 rows at vocab 32768, the micro-batch of the production run.  They live from the
-# head's forward to its backward, which follows at once, and there they are the logit gradients' buffer.
+# Logits kept between the passes of one call, unless it says otherwise: 16384 rows at vocab 32768, the micro-batch of the
+# production run.  They live as long as the call's graph, in a training step from the head's forward to its backward, which
+# follows at once, and there they are the logit gradients' buffer.  They count every row, labelled or not (how many are
+# labelled is known on the device only).  Peak of a backward pass: the kept bytes and, for rows past them, the logits of
+# min(`ROWS_PER_BLOCK`, those rows); with 0 kept bytes the latter alone, at most 512 MiB at vocab 32768.
 KEEP_BYTES = 1 << 30
 
 
-def kept_rows(rows: int, vocab: int) -> int:
-    """Rows whose logits are kept: all of them, or as many whole tiles of 256 as `KEEP_BYTES` hold."""
-    most = KEEP_BYTES // (2 * vocab)
+def kept_rows(rows: int, vocab: int, keep_bytes: int | None = None) -> int:
+    """Rows whose logits are kept: all of them, or as many whole tiles of 256 as ``keep_bytes`` (`KEEP_BYTES`) hold."""
+    most = (KEEP_BYTES if keep_bytes is None else keep_bytes) // (2 * vocab)
     return rows if rows <= most else most // 256 * 256
 
 
@@ -47,7 +50,7 @@ class _TokenLogps(torch.autograd.Function):
     """per-row log p(label) (0 where the label is -100); differentiable w.r.t. hidden and weight."""
 
     @staticmethod
-    def forward(ctx, hidden, weight, labels, keep):
+    def forward(ctx, hidden, weight, labels, keep_bytes):
         from .fused import bf16_weight
         ops = torch.ops.ws_b200
         hidden = hidden.contiguous()
@@ -57,7 +60,7 @@ class _TokenLogps(torch.autograd.Function):
         ctx.weight = weight
         ctx.selected = hidden.shape[0] >= SELECT_FROM and ops.gemm_pair_available()
         if ctx.selected:
-            keep = kept_rows(hidden.shape[0], wb.shape[0]) if keep else 0
+            keep = kept_rows(hidden.shape[0], wb.shape[0], keep_bytes)
             logp, *rest = ops.lm_head_fwd_labelled(hidden, wb, labels, IGNORE, keep, flag)
             ctx.save_for_backward(hidden, labels, *rest)
             ctx.spent = False
@@ -97,10 +100,14 @@ class _TokenLogps(torch.autograd.Function):
         return dh, (None if main is not None else grad_w.to(weight.dtype)), None, None
 
 
-def token_logps(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
-    keep = torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)
-    return _TokenLogps.apply(hidden, weight, labels, keep)
+def token_logps(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor,
+                keep_bytes: int | None = None) -> torch.Tensor:
+    """``keep_bytes``: how much of the logits may be held for the backward pass (None: `KEEP_BYTES`; 0 where memory counts
+    more than the product that makes them again)."""
+    if not (torch.is_grad_enabled() and (hidden.requires_grad or weight.requires_grad)):
+        keep_bytes = 0
+    return _TokenLogps.apply(hidden, weight, labels, keep_bytes)
 
 
-def loss_sum(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor) -> torch.Tensor:
-    return -token_logps(hidden, weight, labels).sum()
+def loss_sum(hidden: torch.Tensor, weight: torch.Tensor, labels: torch.Tensor, keep_bytes: int | None = None) -> torch.Tensor:
+    return -token_logps(hidden, weight, labels, keep_bytes).sum()
