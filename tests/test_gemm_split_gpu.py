@@ -41,3 +41,30 @@ def test_runs_agree_bit_for_bit():
     x, w = torch.randn(300, 7168, device="cuda").bfloat16(), torch.randn(2048, 7168, device="cuda").bfloat16()
     first = G.linear(x, w)
     assert all(torch.equal(G.linear(x, w), first) for _ in range(3))
+
+
+BF16, RESID_F32, SWIGLU, ACC_F32, SWIGLU_BWD, F32, RESID_BF16, CE_FWD = range(8)
+
+
+@pytest.mark.parametrize("m,n,k,epilogue,pieces", [
+    (300, 2048, 7168, BF16, 4), (300, 2048, 7168, RESID_F32, 4), (777, 1280, 8960, BF16, 3), (1792, 1280, 8960, BF16, 2),
+    (129, 264, 4104, BF16, 4), (128, 2048, 2048, RESID_BF16, 4),       # long contractions of few tiles
+    (2048, 2048, 7168, BF16, 1), (1792, 2048, 7168, BF16, 1),          # two pieces would take a second round
+    (300, 2048, 1024, BF16, 1), (300, 2048, 7168, F32, 1)])
+def test_which_products_are_cut(m, n, k, epilogue, pieces):
+    """The plan, and that the launches follow it: a cut product is the grouped launch and the one that adds its pieces."""
+    _ext.require()
+    assert _ext.cdll().ws_gemm_plan(m, n, k, 0, epilogue, 1, 148) == pieces
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the launches below are those of 148 SMs")
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    resid = torch.randn(m, n, device="cuda")
+    before = _ext.launch_count()
+    if epilogue == BF16:
+        G.linear(x, w)
+    elif epilogue == F32:
+        G.linear_f32(x, w)
+    else:
+        G.linear_residual(x, w, resid if epilogue == RESID_F32 else resid.bfloat16())
+    assert _ext.launch_count() - before == (2 if pieces > 1 else 1)
+    G.check_device_errors()

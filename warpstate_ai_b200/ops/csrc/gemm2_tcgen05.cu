@@ -854,15 +854,16 @@ split_finish_kernel(const float* part, int splits, int m, int n, const void* aux
 // which are written and read once through L2.  All pieces together have to fit one round over the CTA pairs: a second
 // round repeats what a tile costs beyond its k-blocks, and measured slower (2048 x 1280 outputs of a 4480-long
 // contraction, 40 tiles in three pieces: 39.0 us against 37.1 uncut).  At 300 x 2048 outputs, k 7168: 48.0 -> 27.6 us.
-extern "C" int ws_gemm_pair_splits(const WsGemm* g, int sms) {
+// Against every number of pieces at 220 problems (96 to 2048 rows, n and k of the blocks' products): never slower than the
+// uncut product; where it does not cut, at most 3 us would be won.
+static int pair_splits(int m, int n, int k, int a_mn, int epilogue, int sms) {
   using namespace ws;
-  if (g->a_mn || g->limit != nullptr || g->row_map != nullptr || g->n % 4 != 0 ||
-      (g->epilogue != WS_EPI_BF16 && g->epilogue != WS_EPI_RESID_F32 && g->epilogue != WS_EPI_RESID_BF16))
+  if (a_mn || n % 4 != 0 || (epilogue != WS_EPI_BF16 && epilogue != WS_EPI_RESID_F32 && epilogue != WS_EPI_RESID_BF16))
     return 1;
-  const long long tiles = (long long)((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + pair::BN - 1) / pair::BN);
-  const int pairs = sms / 2, blocks = (g->k + pair::BK - 1) / pair::BK;
+  const long long tiles = (long long)((m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((n + pair::BN - 1) / pair::BN);
+  const int pairs = sms / 2, blocks = (k + pair::BK - 1) / pair::BK;
   if (pairs < 2 || tiles >= pairs) return 1;
-  const float tile_us = 0.28f, cut_us = 3.0f, piece_us = 8.0f * g->m * (float)g->n / 6.0e6f;
+  const float tile_us = 0.28f, cut_us = 3.0f, piece_us = 8.0f * m * (float)n / 6.0e6f;
   int best = 1;
   float least = blocks * tile_us;
   for (int s = 2; s <= MAX_GROUP && tiles * s <= pairs; ++s) {
@@ -873,6 +874,28 @@ extern "C" int ws_gemm_pair_splits(const WsGemm* g, int sms) {
     }
   }
   return best;
+}
+
+// Weight gradients from 256 rows on, everything else from 96, as far as it pays: below its 256-row tile part of the pair
+// kernel's tensor work is padding, but a product of so few rows is bound by the bytes an SM takes in per k-block, 32 KiB in
+// a pair against 48 KiB in the single-CTA kernel.  Measured from 96 to 255 rows (single-CTA -> pair, us):
+// - what is cut along k gains most: 128 x 2048 outputs of k 2048 34.8 -> 17.4, of k 14336 90.1 -> 35.8;
+// - the FP32 and SwiGLU-backward epilogues, which leave through shared memory here, gain at any k: 128 x 256 of k 256,
+//   residual, 22.7 -> 14.4;
+// - the others need k-blocks for the pair's set-up: at k 256 in_proj goes 10.2 -> 11.2-12.3, at k 1280 18.4 -> 18.5 and
+//   SwiGLU 22.5 -> 20.5, but without (up | gate) to write 18.5 -> 20.4, and only at k 2048 28.7 -> 26.7;
+// - and no more rounds over the chip than the single-CTA kernel takes: 128 x 32768 logits of k 2048 are one round there and
+//   two over the pairs, 38.9 -> 43.0; at 160 rows both take two, 47.1 -> 43.0.
+extern "C" int ws_gemm_plan(int m, int n, int k, int a_mn, int epilogue, int packed, int sms) {
+  using namespace ws;
+  if (sms < 2 || m < (a_mn ? 256 : 96)) return 0;
+  const int splits = pair_splits(m, n, k, a_mn, epilogue, sms);
+  if (m >= 256 || splits > 1 || epilogue == WS_EPI_RESID_F32 || epilogue == WS_EPI_F32 || epilogue == WS_EPI_SWIGLU_BWD)
+    return splits;
+  const int per_tile = epilogue == WS_EPI_SWIGLU ? 128 : pair::BN, across = (n + per_tile - 1) / per_tile;
+  const int single = (m + pair::BM - 1) / pair::BM * across, pairs = sms / 2;
+  if (k < (epilogue == WS_EPI_SWIGLU && !packed ? 2048 : 1024)) return 0;
+  return (across + pairs - 1) / pairs <= (single + sms - 1) / sms ? 1 : 0;
 }
 
 extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaStream_t stream);

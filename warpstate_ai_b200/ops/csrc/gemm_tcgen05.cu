@@ -257,7 +257,7 @@ extern "C" long long ws_launch_count(void) { return ws::g_launches.load(); }
 extern "C" void ws_count_launch(void) { ws::g_launches.fetch_add(1, std::memory_order_relaxed); }
 extern "C" void ws_gemm_set_sm_limit(int sms) { ws::g_sm_limit.store(sms); }
 
-// CTA-pair kernel (gemm2_tcgen05.cu): the default for problems with at least 96 rows (weight gradients: 256);
+// CTA-pair kernel (gemm2_tcgen05.cu): the default where `ws_gemm_plan` there says so;
 // WS_GEMM_PAIR=0 in the environment keeps every GEMM on the single-CTA kernel.
 extern "C" int ws_gemm_pair(const WsGemm* g, int sms, cudaStream_t stream);
 static std::atomic<int> g_pair_override{-1};
@@ -325,18 +325,17 @@ extern "C" int ws_gemm_group(const WsGemm* items, int count, cudaStream_t stream
   return 0;
 }
 
-extern "C" int ws_gemm_pair_splits(const WsGemm* g, int sms);
 extern "C" int ws_gemm_pair_split(const WsGemm* g, int splits, float* part, int sms, cudaStream_t stream);
 
-// The CTA-pair kernel from 96 rows on: below its 256-row tile part of the tensor work is padding, but a product of so
-// few rows is bound by the bytes an SM takes in per k-block, 32 KiB in a pair against 48 KiB in the single-CTA kernel.
-// 128 x 2048 outputs of k 2048: 34.8 -> 17.4 us, cut along k; a block's forward of 128 tokens 164 -> 126 us.
-static bool takes_pair(const WsGemm* g) {
-  return g->limit != nullptr || (pair_mode() && g->m >= (g->a_mn ? 256 : 96) && usable_sms() >= 2);
+// 0: the single-CTA kernel; else the CTA-pair kernel, and into how many pieces a caller with scratch may cut the product.
+static int plan_of(const WsGemm* g) {
+  if (g->limit != nullptr || g->row_map != nullptr) return 1;   // only the pair kernel selects rows
+  return pair_mode() ? ws_gemm_plan(g->m, g->n, g->k, g->a_mn, g->epilogue, g->out != nullptr, usable_sms()) : 0;
 }
 
 extern "C" int ws_gemm_splits(const WsGemm* g) {
-  return validate_gemm(g) == 0 && takes_pair(g) ? ws_gemm_pair_splits(g, usable_sms()) : 1;
+  const int plan = validate_gemm(g) == 0 ? plan_of(g) : 1;
+  return plan > 1 ? plan : 1;
 }
 
 extern "C" int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream) {
@@ -352,7 +351,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   }
   using namespace ws;
   const int sms = usable_sms();
-  if (takes_pair(g)) return ws_gemm_pair(g, sms, stream);
+  if (plan_of(g) > 0) return ws_gemm_pair(g, sms, stream);
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   const int b_rows = swiglu ? 2 * g->n : g->n;  // output features held by B
   CUtensorMap ta, tb;

@@ -63,6 +63,9 @@ int ws_gemm_pair_available(void);  // 1 where problems with >= 256 rows take the
 // A product whose tiles would leave most of the chip idle may be cut along k: ws_gemm_splits says into how many pieces
 // (1: not), and ws_gemm_split computes it so, with FP32 scratch `part` of splits * m * n floats.
 int ws_gemm_splits(const WsGemm* g);
+// Which kernel a product takes on `sms` SMs, a function of its arguments alone: 0 the single-CTA kernel, otherwise the
+// CTA-pair kernel with the product cut along k into that many pieces.  packed: a SwiGLU product writes (up | gate).
+int ws_gemm_plan(int m, int n, int k, int a_mn, int epilogue, int packed, int sms);
 int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream);
 // Number of SMs the GEMM may use on this stream's device (0 = all).  Lets a communication
 // kernel keep a few SMs for itself while persistent GEMM CTAs fill the rest.
@@ -119,8 +122,8 @@ int ws_decode_layer_tail(const void* w_out, const void* w_ug, const void* w_down
 int ws_decode_pick(const float* logits, int batch, int vocab, long long* token, long long* history, int capacity,
                    long long* cursor, long long* pos, cudaStream_t stream);
 
-// Kernel choice for problems with >= 96 rows (weight gradients: 256): 1 = CTA-pair (cta_group::2) kernel, 0 = single-CTA
-// kernel, -1 = the process default (pair unless WS_GEMM_PAIR=0 is in the environment).
+// Whether the CTA-pair (cta_group::2) kernel may be chosen: 1 = where `ws_gemm_plan` says so, 0 = the single-CTA kernel
+// throughout, -1 = the process default (pair unless WS_GEMM_PAIR=0 is in the environment).
 void ws_gemm_set_pair_mode(int mode);
 
 // Number of kernels this library has launched in this process.
