@@ -874,7 +874,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       tc_fence_after_sync();
       if constexpr (PROMPT) {
         if (open) {  // O += P_lo V
-          if (ok) {
+          if (ok && row0 + wq * 32 < T) {  // the rows of a warp past the prompt's end are not stored
             for (int cc = 0; cc < 4; ++cc) {
               uint32_t pk[16];
               if (cc <= last_chunk) {
