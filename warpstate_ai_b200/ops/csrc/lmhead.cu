@@ -140,8 +140,16 @@ gather_rows_kernel(const __nv_bfloat16* in, int ld, const int* index,
     return;
   }
   const uint4* src = reinterpret_cast<const uint4*>(in + static_cast<size_t>(index[row]) * ld);
-#pragma unroll 8
-  for (int i = lane; i < d / 8; i += 32) dst[i] = src[i];
+  constexpr int PIECES = 8;   // per lane in flight: a load does not pass the store of an earlier piece
+  for (int i0 = lane; i0 < d / 8; i0 += 32 * PIECES) {
+    uint4 piece[PIECES];
+#pragma unroll
+    for (int q = 0; q < PIECES; ++q)
+      if (i0 + 32 * q < d / 8) piece[q] = src[i0 + 32 * q];
+#pragma unroll
+    for (int q = 0; q < PIECES; ++q)
+      if (i0 + 32 * q < d / 8) dst[i0 + 32 * q] = piece[q];
+  }
 }
 
 __global__ void __launch_bounds__(256)
