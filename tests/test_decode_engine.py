@@ -71,7 +71,7 @@ def test_cuda_engine_matches_forward_in_bf16():
         if t in (300, 383):
             assert torch.allclose(logits, full[:, t], rtol=0.05, atol=0.05), t
     engine2 = DecodeEngine(model, dtype=torch.bfloat16, use_cuda_graph=False)
-    engine2.prefill(ids[:, :130])              # one chunk fused + 2 stepped tokens
+    engine2.prefill(ids[:, :130])              # a chunk and two positions of the next, in one pass
     for t in range(130, 384):
         last = engine2.step(ids[:, t])
     assert torch.allclose(last, logits, rtol=0.05, atol=0.05)

@@ -32,7 +32,8 @@ def test_modulation_gradients_of_the_norm_pass(rows, d):
     ((z * dz.double()).sum() + (wide * dres.double()).sum()).backward()
     want_dx, want_ds, want_db, want_dw = (t.grad for t in leaves)
     on = scale != -1.0
-    # sums of `rows` FP32 products of rounded factors: a few 2^-24 each, growing at most with the root of the count
+    # sums of `rows` FP32 products of rounded factors: a few 2^-24 each, growing at most with the root of the count; dx of
+    # the two kernels is the same formula with other contractions and xmod rounded once more, a few 2^-24 apart
     assert rel(dx, plain_dx.double()) < 1e-6 and rel(dx, want_dx) < 1e-5
     assert rel(grads[0], want_dw) < 1e-5 and rel(grads[1], want_db) < 1e-5
     assert rel(grads[2][on], want_ds[on]) < 1e-5

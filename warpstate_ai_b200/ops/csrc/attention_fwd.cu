@@ -1,9 +1,10 @@
 // Forward kernels of the middle of a WarpState core (everything between in_proj and out_proj;
 // reference math: warpstate/model.py:124-176), for chunk_size 128 and head_dim 64.
 //
-// The packed projection qkvgu [tokens, 5d] (Q,K,V,gate,U) is read in place with TMA: a tile of
-// one (batch, chunk, head) is the box rows [b*T + n*128, +128) x cols [sel*d + h*64, +64) -- the
-// reference's chunkify/permute/contiguous copies do not exist here.
+// The packed projection qkvgu [tokens, 5d] (Q,K,V,gate,U) is read in place with TMA, through a map
+// over (column, position, sequence): a tile of one (batch, chunk, head) is the box of columns
+// [sel*d + h*64, +64) x positions [n*128, +128) of sequence b, with zeros past the sequence's end --
+// the reference's chunkify/permute/contiguous copies do not exist here.
 //
 //   chunk_writes_kernel : W[b,n,h] = tanh(rope(K))^T tanh(U) / 128            (tcgen05, 64x64 out)
 //   memory_scan_kernel  : state seen by chunk n = mix*F_n + (1-mix)*S_n with
@@ -978,7 +979,7 @@ extern "C" int ws_attn_stream_form(void) {
 
 // The tile kernels address tokens as (position, sequence): a chunk that reaches past the end of its sequence reads
 // zeros there (the tensor map's fill) and its stores are clipped.  (A prompt of 300 tokens, 28 layers: 65.4 ms when the
-// 44 tokens past the second chunk were decode steps, 4.3 in one pass.)  Behind the causal mask those positions change
+// 44 tokens past the second chunk were decode steps, 3.6 in one pass.)  Behind the causal mask those positions change
 // nothing of the others, and tanh(0) adds nothing to a write.
 static int chunk_writes(const void* qkvgu, const float* rope, float* writes, int B, int T, int H, int d, int* error_flag,
                         cudaStream_t stream) {

@@ -243,9 +243,9 @@ __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, uint32_t tadd
       }
     }
   } else if constexpr (EPI == WS_EPI_CE_FWD) {
-    // LM head forward: the logits tile never leaves the SM.  Each thread folds its 128
-    // columns of one row into (max, sum exp) and the owner of the label column records the
-    // label's logit.  Logits are rounded to BF16 first, as a BF16 head GEMM would return them.
+    // LM head forward: each thread folds its 128 columns of one row into (max, sum exp) and the
+    // owner of the label column records the label's logit.  Logits are rounded to BF16 first, as a
+    // BF16 head GEMM would return them; they leave the SM only for the rows that `keep` asks for.
     const long long* labels = reinterpret_cast<const long long*>(p.aux);
     const long long lab = row_ok ? labels[row] : -1;
     const int n0 = nb * BN;

@@ -1,7 +1,8 @@
 // LM-head cross-entropy helpers.  The vocabulary projection itself runs in the tcgen05 GEMM with
-// the WS_EPI_CE_FWD / WS_EPI_CE_BWD epilogues (gemm_tcgen05.cu), so the [tokens, vocab] logits
-// never reach HBM in the forward pass; this file combines the per-128-column (max, sum exp)
-// partials of a row into its log-sum-exp and label log-probability.
+// the WS_EPI_CE_FWD / WS_EPI_CE_BWD epilogues (gemm2_tcgen05.cu, gemm_tcgen05.cu), so a forward pass that no
+// backward pass follows writes no logits; before one it may leave BF16 logits behind.  This file combines the
+// per-128-column (max, sum exp) partials of a row into its log-sum-exp and label log-probability, packs the
+// labelled rows, and turns kept logits into their gradients.
 //
 // Replaces the reference's chunked / full LM-head losses (warpstate/model.py:316-334,
 // ops/loss_experiment.py:14-19: BF16 head GEMM, FP32 cast of the logits, log-softmax, NLL) and
@@ -165,7 +166,8 @@ clear_unlabelled_kernel(const long long* labels, long long ignore_index, int row
 
 // Logit gradients from logits that the forward pass kept: one CTA per row, 16-byte pieces, read and written once.  At
 // 8192 x 32768 that is 1 GiB of traffic (0.16 ms at the copy rate) in place of the product that makes the logits again
-// (1.1 TFLOP, 0.7 ms).  Head forward + backward at 16384 labelled rows: 7.32 -> 5.83 ms, at 2302: 1.22 -> 1.00 ms.  Same arithmetic as the WS_EPI_CE_BWD epilogue on the same BF16 logits: the same bits.
+// (1.1 TFLOP, 0.7 ms).  Head forward + backward at 16384 labelled rows: 7.3 -> 5.8 ms, at 2302: 1.22 -> 0.99 ms.  Same
+// arithmetic as the WS_EPI_CE_BWD epilogue on the same BF16 logits: the same bits.
 constexpr int DLOGITS_PAD = 64;   // rows per k-block of the weight gradient
 
 __global__ void __launch_bounds__(256)

@@ -7,7 +7,9 @@
 // the predecessor has executed `griddepcontrol.launch_dependents` (the kernels here do so right after
 // their set-up) and an SM has room; the kernel runs its own set-up and then blocks in
 // `griddepcontrol.wait`, which returns when the predecessor has completed and its writes are visible.
-// Rule every kernel launched through this helper keeps: no global memory access before `pdl_wait()`.
+// Rule every kernel launched through this helper keeps: no global memory access before `pdl_wait()`, by the compiler's hand
+// either (see `pdl_wait` on `__restrict__`).  The decode kernels have a launch helper and rules of their own (decode.cu):
+// they request data that no launch in front of them writes before they wait.
 // WS_TRAIN_PDL=0 launches normally.
 #pragma once
 #include <cuda_runtime.h>
