@@ -27,8 +27,8 @@ inline bool train_pdl_enabled() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                                    Args... args) {
+inline cudaError_t launch_kernel(bool dependent, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                 cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -38,8 +38,14 @@ inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 bloc
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = train_pdl_enabled() ? 1 : 0;
+  cfg.numAttrs = dependent && train_pdl_enabled() ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                    Args... args) {
+  return launch_kernel(true, kern, grid, block, smem, stream, args...);
 }
 
 }  // namespace ws
