@@ -89,7 +89,7 @@ dstate_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constan
   }
   fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     constexpr uint32_t idesc = make_idesc_bf16(128, 64, true, true);
 #pragma unroll
     for (int k = 0; k < CHUNK / 16; ++k)
@@ -255,7 +255,7 @@ dstate_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_
           : "r"(ok ? 0u : 1u)
           : "memory");
       if (any_bad) break;
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         const int buf = i & 1;
         if (mbar_wait(&tempty[buf], ((i >> 1) & 1) ^ 1, abort_flag)) {
           tc_fence_after_sync();
@@ -563,7 +563,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   fence_proxy_async_smem();
   __syncthreads();
   // ---- MMA A: S = Qr Kr^T, Mem = Qr State, dQr = (dmem/8) State^T
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
     constexpr uint32_t idesc_m = make_idesc_bf16(128, 64, false, true);
     constexpr uint32_t idesc_kk64 = make_idesc_bf16(128, 64, false, false);
@@ -646,7 +646,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   fence_proxy_async_smem();
   __syncthreads();
   // ---- MMA B: O = P V
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     ok = mbar_wait(&bars[2], 0, abort_flag);  // V has landed
     if (ok) {
       tc_fence_after_sync();
@@ -703,7 +703,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   __syncthreads();
   Drow += meet[512 + (half ^ 1) * 128 + row];
   // ---- MMA C: dP = dlocal V^T, dV = P^T dlocal
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     tc_fence_after_sync();
     constexpr uint32_t idesc_kk128 = make_idesc_bf16(128, 128, false, false);
     constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);
@@ -774,7 +774,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   fence_proxy_async_smem();
   __syncthreads();
   // ---- MMA D: dQr += dS Kr, dKr = dS^T Qr, dtK = tU dW^T, dtU = tK dW
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     tc_fence_after_sync();
     constexpr uint32_t idesc_kmn64 = make_idesc_bf16(128, 64, false, true);
     constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);

@@ -74,7 +74,7 @@ chunk_writes_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_c
   }
   fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     // D[128 x 64]: rows 0..63 = tK^T tU.  A is read MN-major with a zero stride between its two
     // 64-wide atoms, so rows 64..127 repeat rows 0..63 and are ignored.
     constexpr uint32_t idesc = make_idesc_bf16(128, 64, true, true);
@@ -248,7 +248,7 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
           : "r"(ok ? 0u : 1u)
           : "memory");
       if (any_bad) break;
-      if (tid == 0) {
+      if (warp == 0 && elect_one()) {
         const int buf = i & 1;
         if (mbar_wait(&tempty[buf], ((i >> 1) & 1) ^ 1, abort_flag)) {
           tc_fence_after_sync();
@@ -484,7 +484,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   }
   fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
 #pragma unroll
     for (int k = 0; k < HD / 16; ++k)
@@ -543,7 +543,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   tc_fence_before_sync();  // every thread's reads of S precede the MMAs that overwrite its columns
   fence_proxy_async_smem();
   __syncthreads();
-  if (tid == 0 && ok) {
+  if (warp == 0 && elect_one() && ok) {
     tc_fence_after_sync();
     constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
 #pragma unroll
@@ -564,7 +564,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       for (int cc = 0; cc < 4; ++cc) store_row_chunk32(sP, tid, cc * 32, low[cc]);
       fence_proxy_async_smem();
       __syncthreads();
-      if (tid == 0 && ok) {
+      if (warp == 0 && elect_one() && ok) {
         constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
 #pragma unroll
         for (int k = 0; k < CHUNK / 16; ++k)
@@ -760,7 +760,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           : "r"(ok ? 0u : 1u)
           : "memory");
       if (any_bad) break;
-      if (tid == 0 && mbar_wait(&setfree[g], ((i >> 1) & 1) ^ 1, abort_flag)) {
+      if (warp == 0 && elect_one() && mbar_wait(&setfree[g], ((i >> 1) & 1) ^ 1, abort_flag)) {
         tc_fence_after_sync();
         const uint32_t t_s = tmem + g * 192, t_m = t_s + 128;
         constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
@@ -868,7 +868,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       tc_fence_before_sync();
       fence_proxy_async_smem();
       if (any_bad(ok)) break;
-      if (gt == 0) issue_o(0u, &ofull[g]);
+      if (wq == 0 && elect_one()) issue_o(0u, &ofull[g]);
       landed = 0;
       if (lane == 0) landed = mbar_wait(&ofull[g], k2 & 1, abort_flag) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
@@ -899,7 +899,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           tc_fence_before_sync();
           fence_proxy_async_smem();
           if (any_bad(ok)) break;
-          if (gt == 0) issue_o(1u, &lowfull[g]);
+          if (wq == 0 && elect_one()) issue_o(1u, &lowfull[g]);
           landed = 0;
           if (lane == 0) landed = mbar_wait(&lowfull[g], opens & 1, abort_flag) ? 1u : 0u;
           ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;

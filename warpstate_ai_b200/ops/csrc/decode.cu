@@ -157,23 +157,30 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    // A slab of in_proj or up/gate is 128 products of 128 x BPAD x 16, 40-49 clocks of tensor core each: what bounded this
+    // loop was their issue, 165 clocks a product (11 us a slab, longer than its bytes take).  One elected lane, descriptors
+    // as 32-bit sums and a counter instead of a remainder: 28 layers at one sequence 1195 -> 1034 us a step, 8 layers at 64
+    // 570 -> 522, 16 layers of width 1280 at one 534 -> 457.
+    if (elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(TM, BPAD, false, false);
       bool ok = true;
-      for (int kb = kb0, it = 0; kb < kb1; ++kb, ++it) {
-        const int s = it % Cfg::STAGES;
-        const uint32_t ph = (it / Cfg::STAGES) & 1;
+      int s = 0;
+      uint32_t ph = 0;
+      const uint32_t a0 = desc_low_sw128(smem_u32(sW)), b0 = desc_low_sw128(smem_u32(sX));
+      for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&full[s], ph, abort_flag)) {
           ok = false;
           break;
         }
         tc_fence_after_sync();
-        const uint32_t a = smem_u32(sW + s * W_BYTES), b = smem_u32(sX + s * Cfg::X_BYTES);
+        const uint32_t a = a0 + s * (W_BYTES / 16), b = b0 + s * (Cfg::X_BYTES / 16);
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k)
-          umma_bf16(tmem, make_smem_desc_sw128(a + k * 32, 0, 1024), make_smem_desc_sw128(b + k * 32, 0, 1024), idesc,
-                    (it | k) != 0 ? 1u : 0u);
+        for (int k = 0; k < BK / 16; ++k) umma_bf16_low(tmem, a + 2 * k, b + 2 * k, idesc, k != 0 || kb != kb0 ? 1u : 0u);
         umma_commit(&empty[s]);
+        if (++s == Cfg::STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
       }
       if (ok) umma_commit(tfull);
     }

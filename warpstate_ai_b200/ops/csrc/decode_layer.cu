@@ -372,7 +372,7 @@ decode_layer_tail_kernel(const __grid_constant__ CUtensorMap tm_wout, const __gr
       tail_produce<0>(c, &tm_win, &tm_n, w_in, 5 * p.d, 5u, pit);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t cit = 0;
       tail_mma(c, w_out, cit);
       tail_mma(c, w_ug, cit);

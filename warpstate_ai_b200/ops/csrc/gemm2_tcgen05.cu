@@ -313,7 +313,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && leader) {
+    if (leader && elect_one()) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       int it = 0;
       int tcount = 0;

@@ -200,6 +200,38 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t desc_a, uint
       "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// True in one lane of a converged warp, always the same one.  A role that issues MMAs runs behind this branch and not
+// behind `lane == 0`: the instruction takes its operands from uniform registers, and the two branches are compiled
+// differently.  Measured, clocks per tcgen05.mma of 128 x N x 16 issued back to back: N 16 57 -> 40, N 64 57 -> 49, N 128 64 -> 64,
+// N 256 127 -> 127 (there the tensor core is the bound); in a loop with a wait and addresses of its own for every four, 165 -> 95.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n"
+      ".reg .pred q;\n"
+      "elect.sync _|q, 0xffffffff;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n"
+      : "=r"(e));
+  return e != 0;
+}
+// Low half of a K-major descriptor with the 128-byte swizzle and 1024 bytes between 8-row groups (leading offset 0); the
+// other half is a constant.  A step of 32 bytes along k, or of a whole tile, is an addition.
+__device__ __forceinline__ uint32_t desc_low_sw128(uint32_t smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
+__device__ __forceinline__ void umma_bf16_low(uint32_t tmem_d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
+  constexpr uint32_t kHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      ".reg .b64 a, b;\n"
+      "mov.b64 a, {%1, %5};\n"
+      "mov.b64 b, {%2, %5};\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kHigh)
+      : "memory");
+}
 // A operand taken from TMEM (used by the attention kernels for P*V and dS*K products).
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
                                              uint32_t idesc, uint32_t accumulate) {
