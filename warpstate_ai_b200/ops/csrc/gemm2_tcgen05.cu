@@ -91,7 +91,7 @@ struct alignas(64) PairGroup {
   GemmParams p[MAX_GROUP];
   CUtensorMap epi[4];  // staged epilogue of problem 0, 32 x 32 boxes.  SwiGLU backward: aux up, aux gate,
                        // out up, out gate; SwiGLU forward: packed up, packed gate, activation; residual: aux, out;
-                       // FP32: the output of problem i
+                       // FP32 and its accumulation: the output of problem i
   CUtensorMap whole;   // row selection (problem 0): the operand before its rows were selected
   int tile_start[MAX_GROUP + 1];
   int count;
@@ -103,7 +103,7 @@ struct alignas(64) PairGroup {
 // global memory never goes through L1 and each thread touches only swizzled shared memory.
 template <int EPI>
 constexpr bool staged_epilogue() {
-  return EPI == WS_EPI_SWIGLU_BWD || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_RESID_F32 || EPI == WS_EPI_F32;
+  return EPI == WS_EPI_SWIGLU_BWD || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_RESID_F32 || EPI == WS_EPI_F32 || EPI == WS_EPI_ACC_F32;
 }
 static_assert(MAX_GROUP == 4, "one output map per problem of an FP32 group");
 template <int EPI>
@@ -209,7 +209,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
     }
     if (STAGED) {
       for (int i = 0; i < 16; ++i) mbar_init(&ebar[i], 1);
-      for (int i = 0; i < (EPI == WS_EPI_SWIGLU ? 3 : EPI == WS_EPI_RESID_F32 ? 2 : EPI == WS_EPI_F32 ? g.count : 4); ++i) tma_prefetch_desc(&g.epi[i]);
+      for (int i = 0; i < (EPI == WS_EPI_SWIGLU ? 3 : EPI == WS_EPI_RESID_F32 ? 2 : EPI == WS_EPI_F32 || EPI == WS_EPI_ACC_F32 ? g.count : 4); ++i) tma_prefetch_desc(&g.epi[i]);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -415,8 +415,11 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
       }
       if (lane == 0) tma_store_wait_all();
-    } else if constexpr (EPI == WS_EPI_F32) {
-      // FP32 through shared memory: per warp 32 rows, per step 32 columns, two tiles in flight.
+    } else if constexpr (EPI == WS_EPI_F32 || EPI == WS_EPI_ACC_F32) {
+      // FP32 through shared memory: per warp 32 rows, per step 32 columns, two tiles in flight.  A sum (beta 1) leaves as a
+      // bulk reduction: every element is added to once, in L2, so the result is that of a read, an addition and a write,
+      // but no thread waits for the old value.  Against a thread per row that reads and writes 16 bytes of 32 rows at a time:
+      // 27 M gradients of 1792 tokens 125 -> 85 us, 67 M of 2300 309 -> 237, 0.9 M of 1024 27 -> 16.
       uint8_t* ebuf = eStage + (warp - 2) * 8192;
       constexpr int STEPS = (BN / GROUPS) / 32;
       int q = 0;
@@ -429,6 +432,10 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         tc_fence_after_sync();
         const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+        const float alpha = EPI == WS_EPI_ACC_F32 ? p.alpha : 1.f;
+        if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f && p.beta != 1.f) {   // neither a store nor a sum: by row
+          gemm_epilogue<EPI, GROUPS>(p, taddr - egroup * (BN / GROUPS), y + lane, y + lane < p.m, 1.f, t.nb, egroup);
+        } else
 #pragma unroll 1
         for (int step = 0; step < STEPS; ++step, ++q) {
           const int x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
@@ -438,13 +445,20 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           if (lane == 0) tma_store_wait_read1();  // the store issued from this tile two steps ago has read it
           __syncwarp();
           tmem_ld_wait();
+          if constexpr (EPI == WS_EPI_ACC_F32) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+          }
 #pragma unroll
           for (int j = 0; j < 8; ++j)
             *reinterpret_cast<uint4*>(tile_chunk128(tr, lane, j)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
-            if (x < p.n && y < p.m) tma_store_2d(&g.epi[t.prob], tr, x, y);
+            if (x < p.n && y < p.m) {
+              if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f) tma_add_2d(&g.epi[t.prob], tr, x, y);
+              else tma_store_2d(&g.epi[t.prob], tr, x, y);
+            }
             tma_store_commit();
           }
         }
@@ -958,7 +972,7 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     total += tiles;
   }
   for (int i = count; i <= MAX_GROUP; ++i) grp.tile_start[i] = total;
-  if (items[0].epilogue == WS_EPI_F32) {
+  if (items[0].epilogue == WS_EPI_F32 || items[0].epilogue == WS_EPI_ACC_F32) {
     for (int i = 0; i < count; ++i) {
       const int rc = make_map_f32(&grp.epi[i], items[i].out, items[i].n, items[i].m, items[i].ldo, 32, 32);
       if (rc) return rc;
