@@ -1,0 +1,102 @@
+"""A block as one native autograd node against the node written in Python: the same kernels on the same numbers, so equal bit
+for bit, and the same answers to what autograd may ask of a node."""
+import pytest
+import torch
+
+from warpstate_ai_b200 import WarpStateConfig
+from warpstate_ai_b200.models.warpstate import WarpStateCore
+from warpstate_ai_b200.ops import fused
+from warpstate_ai_b200.optim import ParamArena
+
+
+def block(seed=0):
+    torch.manual_seed(seed)
+    cfg = WarpStateConfig(vocab_size=64, d_model=256, n_heads=4, n_cores=1, logical_depth=2, ffn_hidden=192, chunk_size=128,
+                          gradient_checkpointing=False, parallel_memory=True)
+    with torch.device("cuda"):
+        return WarpStateCore(cfg)
+
+
+def autocast():
+    return torch.autocast("cuda", dtype=torch.bfloat16, cache_enabled=False)
+
+
+def run(core, x, modulation, dy, passes=1, hooks=None):
+    for p in core.parameters():
+        if p.grad is not None:
+            p.grad.zero_()
+    leaves = [t.detach().clone().requires_grad_(t.requires_grad) if t is not None else None for t in (x, *modulation)]
+    with autocast(), hooks or torch.autograd.graph.saved_tensors_hooks(lambda t: t, lambda t: t):
+        y = core(*leaves)
+    for i in range(passes):
+        y.backward(dy, retain_graph=i + 1 < passes)
+    return [y.detach()] + [None if t is None or t.grad is None else t.grad.clone() for t in leaves] + \
+        [None if p.grad is None else p.grad.clone() for p in core.parameters()]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("modulated,input_grad,frozen", [(True, True, ()), (False, True, ()), (True, False, ()),
+                                                         (True, True, ("norm1.weight", "in_proj.weight", "fast_decay_logit"))])
+def test_native_node_equals_the_python_one(monkeypatch, modulated, input_grad, frozen):
+    core = block()
+    ParamArena(core)
+    for name, p in core.named_parameters():
+        p.requires_grad_(name not in frozen)
+    x = torch.randn(3, 256, 256, device="cuda").requires_grad_(input_grad)
+    modulation = [torch.randn(256, device="cuda").mul_(0.1).requires_grad_(True) if modulated else None for _ in range(2)]
+    dy = torch.randn(3, 256, 256, device="cuda")
+    seen = []
+    native = run(core, x, modulation, dy)
+    twice = run(core, x, modulation, dy, passes=2)
+    hooked = run(core, x, modulation, dy, hooks=torch.autograd.graph.saved_tensors_hooks(
+        lambda t: (seen.append(t.shape), t.cpu())[1], lambda t: t.cuda()))
+    assert seen
+    monkeypatch.setattr(fused, "_block_node", lambda *a: None)
+    python = run(core, x, modulation, dy)
+    python_twice = run(core, x, modulation, dy, passes=2)
+    for a, b, c in ((native, python, hooked), (twice, python_twice, python_twice)):
+        for p, q, r in zip(a, b, c):
+            assert (p is None) == (q is None) == (r is None)
+            assert p is None or (torch.equal(p, q) and torch.equal(p, r))
+
+
+@pytest.mark.gpu
+def test_scoring_pass_and_transposed_input(monkeypatch):
+    core = block(1)                                        # no arena: cached casts
+    x = torch.randn(256, 2, 256, device="cuda").transpose(0, 1)
+    scale, bias = torch.randn(2, 256, device="cuda").mul_(0.1).unbind(0)
+    with torch.no_grad(), autocast():
+        native = core(x, scale, bias)
+        assert not native.requires_grad
+        monkeypatch.setattr(fused, "_block_node", lambda *a: None)
+        assert torch.equal(native, core(x, scale, bias))
+    monkeypatch.undo()
+    with autocast():                                       # gradients that autograd holds: the Python node
+        assert type(core(x, scale, bias).grad_fn).__name__ != type(None).__name__
+        assert fused._block_node(core, x, scale, bias, True) is None
+
+
+@pytest.mark.gpu
+def test_transforms_that_the_node_does_not_support_are_refused():
+    core = block(2)
+    ParamArena(core)
+    x = torch.randn(1, 128, 256, device="cuda")
+    with autocast():
+        with pytest.raises(RuntimeError):
+            torch.func.grad(lambda t: core(t).sum())(x)
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(core)(x[None])
+        with pytest.raises((RuntimeError, NotImplementedError)):
+            with torch.autograd.forward_ad.dual_level():
+                core(torch.autograd.forward_ad.make_dual(x, torch.ones_like(x)))
+
+
+@pytest.mark.gpu
+def test_a_hook_on_finished_gradients_takes_the_python_node(monkeypatch):
+    core, called = block(3), []
+    ParamArena(core)
+    x = torch.randn(1, 128, 256, device="cuda", requires_grad=True)
+    monkeypatch.setattr(fused, "_core_grad_hook", called.append)
+    with autocast():
+        core(x).sum().backward()
+    assert called == [core]

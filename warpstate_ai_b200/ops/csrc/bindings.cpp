@@ -1,6 +1,7 @@
 // torch.ops.ws_b200.* registrations: argument checking and pointer extraction only; all
 // device work is in the .cu files behind the C ABI of ws_api.h.
 #include <cstdio>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/library.h>
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
@@ -523,6 +524,93 @@ std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& x, co
   }
   auto [dx, unused, g_n1] = rmsnorm_bwd(dz1, x, rstd1, n1, dx2, scale, false);
   return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, g_n1.unsqueeze(0)};
+}
+
+// One block as one autograd node whose two directions never enter Python: `ops.fused.CoreFn` for an FP32 stream and weights
+// whose gradients go straight into their FP32 buffers (or no backward pass at all).  What CoreFn finds by attribute at each
+// pass comes along here.  Calls bound by the host: scoring 128 tokens by a block of width 2048 128 -> 102 us (its kernels take 97), a training pass
+// of 2 x 896 tokens at width 1280 520 -> 460, the smoke model's micro-batch (four depths) 2060 -> 1750.
+struct BlockSpec {
+  at::Tensor bf16[4];   // in_proj, out_proj, up/gate, down
+  at::Tensor main[4];   // their FP32 gradients; undefined without a backward pass
+  at::Tensor rope;
+  c10::optional<at::Tensor> flag;
+  double eps;
+  int64_t H;
+  bool keep;
+};
+
+struct BlockFn : public torch::autograd::Function<BlockFn> {
+  static at::Tensor vector(const at::Tensor& t) { return t.defined() ? t.detach().to(at::kFloat).contiguous() : t; }
+  static c10::optional<at::Tensor> maybe(const at::Tensor& t) { return t.defined() ? c10::optional<at::Tensor>(t) : c10::nullopt; }
+
+  static at::Tensor forward(torch::autograd::AutogradContext* ctx, const at::Tensor& x, const c10::optional<at::Tensor>& scale,
+                            const c10::optional<at::Tensor>& bias, const at::Tensor& n1, const at::Tensor& n2, const at::Tensor& w_in,
+                            const at::Tensor& w_out, const at::Tensor& w_ug, const at::Tensor& w_down, const at::Tensor& fast,
+                            const at::Tensor& slow, const at::Tensor& mix, const BlockSpec* spec) {
+    const int64_t B = x.size(0), T = x.size(1), d = x.size(2);
+    const at::Tensor x_in = x.reshape({B * T, d}).contiguous(), sc = vector(scale.value_or(at::Tensor())), bi = vector(bias.value_or(at::Tensor()));
+    const at::Tensor logits[3] = {vector(fast), vector(slow), vector(mix)};
+    std::vector<at::Tensor> s = block_fwd(x_in, maybe(sc), maybe(bi), vector(n1), spec->bf16[0], spec->bf16[1], vector(n2),
+                                          spec->bf16[2], spec->bf16[3], logits[0], logits[1], logits[2], spec->rope, spec->eps,
+                                          B, T, spec->H, spec->keep, true, spec->flag);
+    if (spec->keep) {   // x3, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, writes, states
+      const at::Tensor none = s[2];
+      ctx->save_for_backward({x_in, sc.defined() ? sc : none, bi.defined() ? bi : none, n1, n2, s[2], s[3], s[4], s[5], s[6],
+                              s[7], s[8], s[9], s[10]});
+      auto& data = ctx->saved_data;
+      data["attention"] = std::vector<at::Tensor>{s[11], s[12]};
+      data["weights"] = std::vector<at::Tensor>(spec->bf16, spec->bf16 + 4);
+      data["gradients"] = std::vector<at::Tensor>(spec->main, spec->main + 4);
+      data["logits"] = std::vector<at::Tensor>(logits, logits + 3);
+      data["rope"] = spec->rope;
+      data["flag"] = spec->flag.has_value() ? *spec->flag : at::Tensor();
+      data["shape"] = std::vector<int64_t>{B, T, d, spec->H, sc.defined() ? 1 : 0};
+    }
+    return s[0].view({B, T, d});
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto t = ctx->get_saved_variables();   // x, scale, bias, n1, n2, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act
+    auto& data = ctx->saved_data;
+    const std::vector<int64_t> shape = data["shape"].toIntVector();
+    const int64_t B = shape[0], T = shape[1], d = shape[2];
+    const bool modulated = shape[4] != 0;
+    const auto attention = data["attention"].toTensorVector(), w = data["weights"].toTensorVector(),
+               main = data["gradients"].toTensorVector(), logits = data["logits"].toTensorVector();
+    const at::Tensor flag_tensor = data["flag"].toTensor();
+    const c10::optional<at::Tensor> flag = maybe(flag_tensor);
+    const at::Tensor dx3 = grads[0].reshape({B * T, d}).contiguous();
+    const auto scale = modulated ? c10::optional<at::Tensor>(t[1]) : c10::nullopt, bias = modulated ? c10::optional<at::Tensor>(t[2]) : c10::nullopt;
+    std::vector<at::Tensor> r = block_bwd(dx3, t[0], t[5], t[7], t[9], t[10], t[12], attention[0], attention[1], scale, bias,
+                                          vector(t[3]), vector(t[4]), w[0], w[1], w[2], w[3], logits[0], logits[1], logits[2],
+                                          data["rope"].toTensor(), B, T, shape[3], flag);
+    // r: dx, dx3 BF16, dpacked, dx2 BF16, dqkvgu, g_norm2, logit gradients, first norm's (and bias and scale)
+    const at::Tensor dys[4] = {r[1], r[2], r[3], r[4]}, xs[4] = {t[13], t[11], t[8], t[6]};
+    const at::Tensor into[4] = {main[3], main[2], main[1], main[0]};
+    const double betas[4] = {1.0, 1.0, 1.0, 1.0};
+    grad_weight_group(dys, xs, into, betas, flag);
+    const at::Tensor none;
+    return {r[0].view({B, T, d}), modulated ? r[7].select(0, 2) : none, modulated ? r[7].select(0, 1) : none, r[7].select(0, 0),
+            r[5], none, none, none, none, r[6].select(0, 0), r[6].select(0, 1), r[6].select(0, 2), none};
+  }
+};
+
+at::Tensor block(const at::Tensor& x, const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& bias,
+                 const at::Tensor& n1, const at::Tensor& n2, at::TensorList weights, at::TensorList bf16, at::TensorList main,
+                 const at::Tensor& fast, const at::Tensor& slow, const at::Tensor& mix, const at::Tensor& rope, double eps,
+                 int64_t H, const c10::optional<at::Tensor>& flag) {
+  TORCH_CHECK(x.dim() == 3 && x.scalar_type() == at::kFloat && weights.size() == 4 && bf16.size() == 4 &&
+              (main.size() == 4 || (main.empty() && !at::GradMode::is_enabled())) && scale.has_value() == bias.has_value(),
+              "block: FP32 x [B, T, d], four weights, their BF16 copies and FP32 gradients");
+  BlockSpec spec;
+  for (int i = 0; i < 4; ++i) {
+    spec.bf16[i] = bf16[i];
+    if (!main.empty()) spec.main[i] = main[i];
+  }
+  spec.rope = rope; spec.flag = flag; spec.eps = eps; spec.H = H; spec.keep = at::GradMode::is_enabled();
+  return BlockFn::apply(x, scale, bias, n1, n2, weights[0], weights[1], weights[2],
+                        weights[3], fast, slow, mix, static_cast<const BlockSpec*>(&spec));
 }
 
 // Forward over prompts of any length; the layer's decode state is written.  -> the block's output rows [B*T, d], or with
@@ -1242,6 +1330,8 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("block_bwd(Tensor dx3, Tensor x, Tensor rstd1, Tensor qkvgu, Tensor x2, Tensor rstd2, Tensor packed, Tensor writes, "
         "Tensor states, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor w_in, Tensor w_out, Tensor w_ug, Tensor w_down, "
         "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, int B, int T, int H, Tensor(a!)? flag) -> Tensor[]");
+  m.def("block(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor[] weights, Tensor[] bf16, Tensor[] main, "
+        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int H, Tensor? error_flag) -> Tensor");
   m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
         "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
         "Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, bool last, "
@@ -1264,6 +1354,8 @@ TORCH_LIBRARY(ws_b200, m) {
         "Tensor(c!)? error_flag, bool wide=False) -> ()");
   m.def("grad_weight_group(Tensor[] dys, Tensor[] xs, Tensor(a!)[] grads, float[] betas, Tensor(b!)? error_flag) -> ()");
 }
+
+TORCH_LIBRARY_IMPL(ws_b200, CompositeImplicitAutograd, m) { m.impl("block", &block); }
 
 TORCH_LIBRARY_IMPL(ws_b200, CompositeExplicitAutograd, m) {
   m.impl("gemm_pair_available", &gemm_pair_available);

@@ -373,10 +373,33 @@ def _attach_small_grads(core, g_n1, g_n2, g_fast, g_slow, g_mix) -> None:
         main.add_(g.to(main.dtype))
 
 
+def _block_node(core, x, depth_scale, depth_bias, notify):
+    """The block as one native autograd node (`BlockFn` of the library), or None where `CoreFn` is needed: a rounded stream,
+    weights that are sharded or whose gradients autograd is to hold, a hook on finished gradients, a tuned GEMM choice."""
+    from . import attention
+    if x.dtype != torch.float32 or (notify and _core_grad_hook is not None) or G._policy or not attention.kernels_ready(core) \
+            or getattr(core, "ws_weights", None) is not None:
+        return None
+    weights = (core.in_proj.weight, core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight)
+    main = []
+    if torch.is_grad_enabled():
+        main = [getattr(w, "main_grad", None) for w in weights]
+        if any(m is None for m in main) or any(getattr(w, "bf16_view", None) is None for w in weights):
+            return None
+    return _ops().block(x, depth_scale, depth_bias, core.norm1.weight, core.norm2.weight, weights,
+                        [bf16_weight(w) for w in weights], main, core.fast_decay_logit, core.slow_decay_logit,
+                        core.memory_mix_logit, attention.rope_table(x.device, pair_major=True), core.cfg.rms_eps, core.h,
+                        G.error_flag(x.device))
+
+
 def core_forward(core, x: torch.Tensor, depth_scale=None, depth_bias=None, notify: bool = True,
                  checkpoint: bool = False) -> torch.Tensor:
     if x.dtype not in (torch.float32, torch.bfloat16):
         x = x.float()
+    if not checkpoint:
+        y = _block_node(core, x, depth_scale, depth_bias, notify)
+        if y is not None:
+            return y
     return CoreFn.apply(x, depth_scale, depth_bias, core.norm1.weight, core.in_proj.weight,
                         core.out_proj.weight, core.norm2.weight, core.ffn.up_gate.weight,
                         core.ffn.down.weight, core.fast_decay_logit, core.slow_decay_logit,
