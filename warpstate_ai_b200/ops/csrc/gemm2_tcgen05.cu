@@ -40,7 +40,6 @@ constexpr int BN = 256;        // accumulator columns (128 B rows staged per CTA
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int STAGES = 6;          // staged-epilogue instantiations use one fewer (see pair_stages)
-constexpr int ESTAGE_BYTES = 8 * 8192;  // staged epilogue: 8 warps x 2 buffers x 2 tiles of 32 x 32 BF16
 constexpr int A_BYTES = BM * BK * 2;        // 16 KiB
 constexpr int B_BYTES = (BN / 2) * BK * 2;  // 16 KiB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
@@ -106,20 +105,26 @@ constexpr bool staged_epilogue() {
   return EPI == WS_EPI_SWIGLU_BWD || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_RESID_F32 || EPI == WS_EPI_F32 || EPI == WS_EPI_ACC_F32;
 }
 static_assert(MAX_GROUP == 4, "one output map per problem of an FP32 group");
+// BF16 results (and the logits that the LM head keeps) leave through two small tiles per warp, which the ring's sixth stage
+// has room for.
+template <int EPI>
+constexpr bool tiled_epilogue() {
+  return EPI == WS_EPI_BF16 || EPI == WS_EPI_CE_FWD;
+}
+template <int EPI>
+constexpr int epilogue_bytes() {   // 8 warps x 2 buffers x 2 tiles of 32 x 32 BF16; or one tile
+  return staged_epilogue<EPI>() ? 8 * 8192 : tiled_epilogue<EPI>() ? 8 * 4096 : 0;
+}
 template <int EPI>
 constexpr int pair_stages() {
   return staged_epilogue<EPI>() ? pair::STAGES - 1 : pair::STAGES;
 }
 template <int EPI>
 constexpr int pair_smem() {
-  return pair_stages<EPI>() * pair::STAGE_BYTES + (staged_epilogue<EPI>() ? pair::ESTAGE_BYTES : 0) + 1024 + 512;
+  return pair_stages<EPI>() * pair::STAGE_BYTES + epilogue_bytes<EPI>() + 1024 + 512;
 }
 
-// 16-byte chunk j of row r in a 32-row x 64-byte tile written by TMA with the 64-byte swizzle
-__device__ __forceinline__ uint8_t* tile_chunk64(uint8_t* tile, int r, int j) {
-  return tile + r * 64 + ((j ^ ((r >> 1) & 3)) << 4);
-}
-// the same for 128-byte rows and the 128-byte swizzle (32 x 32 FP32 tiles)
+// tile_chunk64 for 128-byte rows and the 128-byte swizzle (32 x 32 FP32 tiles)
 __device__ __forceinline__ uint8_t* tile_chunk128(uint8_t* tile, int r, int j) {
   return tile + r * 128 + ((j ^ (r & 7)) << 4);
 }
@@ -183,8 +188,8 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
                                              ~static_cast<uintptr_t>(1023));
   uint8_t* sA = smem;
   uint8_t* sB = smem + STAGES * A_BYTES;
-  uint8_t* eStage = smem + STAGES * STAGE_BYTES;  // staged epilogue buffers (STAGED only)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(eStage + (STAGED ? ESTAGE_BYTES : 0));
+  uint8_t* eStage = smem + STAGES * STAGE_BYTES;  // staged epilogue buffers
+  uint64_t* bars = reinterpret_cast<uint64_t*>(eStage + epilogue_bytes<EPI>());
   uint64_t* full = bars;                    // used in the leader CTA
   uint64_t* empty = bars + STAGES;          // per CTA
   uint64_t* tfull = bars + 2 * STAGES;      // per CTA
@@ -630,10 +635,14 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       }
       if (lane == 0) tma_store_wait_all();
     } else {
-      for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
+      [[maybe_unused]] WarpStage sender;
+      if constexpr (tiled_epilogue<EPI>()) sender.tiles = eStage + (warp - 2) * 4096;
+      // (rows that go back to their places before a selection are stored one by one)
+            for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const GemmParams& p = g.p[t.prob];
         const int nb = t.nb;
+        sender.map = &g.epi[t.prob];
         const int buf = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
         if (!mbar_wait(&tfull[buf], tph, abort_flag)) break;
@@ -642,16 +651,18 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
         const bool inside = row < p.m;
         const int place = p.row_map != nullptr && inside ? p.row_map[row] : row;  // the row before the selection
+        WarpStage* const stage = tiled_epilogue<EPI>() && p.row_map == nullptr ? &sender : nullptr;
         float rs = 1.0f;
         if (p.row_scale != nullptr && inside) rs = place >= 0 ? p.row_scale[place] : 0.f;
         if constexpr (EPI == WS_EPI_BF16)
-          gemm_epilogue<EPI, GROUPS>(p, taddr, place, inside && place >= 0, rs, nb, egroup);
+          gemm_epilogue<EPI, GROUPS>(p, taddr, place, inside && place >= 0, rs, nb, egroup, stage);
         else
-          gemm_epilogue<EPI, GROUPS>(p, taddr, row, inside, rs, nb, egroup);
+          gemm_epilogue<EPI, GROUPS>(p, taddr, row, inside, rs, nb, egroup, EPI == WS_EPI_CE_FWD ? stage : nullptr);
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf]), 0));
       }
+      if (tiled_epilogue<EPI>() && lane == 0) tma_store_wait_all();
     }
   }
 
@@ -799,6 +810,14 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
   const int n_tile = swiglu ? 128 : pair::BN;
   *tiles_out = ((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + n_tile - 1) / n_tile);
   return 0;
+}
+
+// 32 x 32 store boxes over BF16 results, or over the logits that are kept.
+static int fill_tile_map(const WsGemm* g, PairGroup& grp, int i) {
+  const CUtensorMapSwizzle sw = CU_TENSOR_MAP_SWIZZLE_64B;
+  if (g->epilogue == WS_EPI_BF16) return g->row_map != nullptr ? 0 : make_map_bf16_swz(&grp.epi[i], g->out, g->n, g->m, g->ldo, 32, 32, sw);
+  if (g->keep == nullptr) return 0;
+  return make_map_bf16_swz(&grp.epi[i], g->keep, g->n, grp.p[i].keep_rows, g->n, 32, 32, sw);
 }
 
 // Staged SwiGLU-forward epilogue: 32 x 32 store boxes over the packed (up | gate) matrix and the activation.
@@ -978,6 +997,12 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
       if (rc) return rc;
     }
   }
+  if (items[0].epilogue == WS_EPI_BF16 || items[0].epilogue == WS_EPI_CE_FWD) {
+    for (int i = 0; i < count; ++i) {
+      const int rc = fill_tile_map(&items[i], grp, i);
+      if (rc) return rc;
+    }
+  }
   if (items[0].epilogue == WS_EPI_RESID_F32) {
     if (count != 1) return -9;
     const WsGemm* g0 = &items[0];
@@ -1067,10 +1092,8 @@ extern "C" int ws_gather_gemm(const void* x, int m, int n, int k, const void* co
   int rc = fill_problem(&item, grp, 0, &tiles);
   if (rc) return rc;
   for (int i = 1; i <= MAX_GROUP; ++i) grp.tile_start[i] = tiles;
-  if (swiglu) {
-    rc = fill_swiglu_maps(&item, grp);
-    if (rc) return rc;
-  }
+  rc = swiglu ? fill_swiglu_maps(&item, grp) : fill_tile_map(&item, grp, 0);
+  if (rc) return rc;
   GatherJob job;
   memset(&job, 0, sizeof(job));
   for (int r = 0; r < world; ++r) job.shard[r] = static_cast<const float*>(shards[r]);
