@@ -327,6 +327,12 @@ extern "C" int ws_gemm_group(const WsGemm* items, int count, cudaStream_t stream
 
 extern "C" int ws_gemm_pair_split(const WsGemm* g, int splits, float* part, int sms, cudaStream_t stream);
 
+// A plain product of few tokens whose result is written as it is (gemm_rows.cu).
+static bool takes_rows(const WsGemm* g) {
+  return pair_mode() && !g->a_mn && !g->b_mn && g->limit == nullptr && g->row_map == nullptr && g->row_scale == nullptr &&
+         ws_gemm_rows_takes(g->m, g->n, g->k, g->epilogue, g->out != nullptr, usable_sms());
+}
+
 // 0: the single-CTA kernel; else the CTA-pair kernel, and into how many pieces a caller with scratch may cut the product.
 static int plan_of(const WsGemm* g) {
   if (g->limit != nullptr || g->row_map != nullptr) return 1;   // only the pair kernel selects rows
@@ -334,7 +340,7 @@ static int plan_of(const WsGemm* g) {
 }
 
 extern "C" int ws_gemm_splits(const WsGemm* g) {
-  const int plan = validate_gemm(g) == 0 ? plan_of(g) : 1;
+  const int plan = validate_gemm(g) == 0 && !takes_rows(g) ? plan_of(g) : 1;
   return plan > 1 ? plan : 1;
 }
 
@@ -351,6 +357,7 @@ extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {
   }
   using namespace ws;
   const int sms = usable_sms();
+  if (takes_rows(g)) return ws_gemm_rows(g, sms, stream);
   if (plan_of(g) > 0) return ws_gemm_pair(g, sms, stream);
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   const int b_rows = swiglu ? 2 * g->n : g->n;  // output features held by B

@@ -66,6 +66,10 @@ int ws_gemm_splits(const WsGemm* g);
 // Which kernel a product takes on `sms` SMs, a function of its arguments alone: 0 the single-CTA kernel, otherwise the
 // CTA-pair kernel with the product cut along k into that many pieces.  packed: a SwiGLU product writes (up | gate).
 int ws_gemm_plan(int m, int n, int k, int a_mn, int epilogue, int packed, int sms);
+// Before that: whether a product of few tokens (operands as they are stored, no row selection, no row factors) takes the
+// kernel that has the weights in its rows (gemm_rows.cu), also a function of its arguments alone.
+int ws_gemm_rows_takes(int m, int n, int k, int epilogue, int packed, int sms);
+int ws_gemm_rows(const WsGemm* g, int sms, cudaStream_t stream);
 int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream);
 // Number of SMs the GEMM may use on this stream's device (0 = all).  Lets a communication
 // kernel keep a few SMs for itself while persistent GEMM CTAs fill the rest.
