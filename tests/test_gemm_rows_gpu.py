@@ -12,7 +12,8 @@ BF16, RESID_F32, SWIGLU = 0, 1, 2
     (95, 10240, 2048, BF16, 1, 0), (96, 10240, 2048, BF16, 1, 1), (128, 10240, 2048, BF16, 1, 1), (224, 10240, 2048, BF16, 1, 1), (256, 10240, 2048, BF16, 1, 0),
     (257, 10240, 2048, BF16, 1, 1), (300, 10240, 2048, BF16, 1, 1), (384, 10240, 2048, BF16, 1, 1), (448, 10240, 2048, BF16, 1, 1), (512, 10240, 2048, BF16, 1, 0),
     (513, 10240, 2048, BF16, 1, 0), (300, 7168, 2048, SWIGLU, 0, 1), (300, 7168, 2048, SWIGLU, 1, 0), (300, 6400, 1280, BF16, 1, 0),
-    (128, 6400, 1280, BF16, 1, 1), (128, 4480, 1280, SWIGLU, 0, 1), (160, 4480, 1280, SWIGLU, 0, 0), (192, 7168, 2048, SWIGLU, 0, 1), (224, 7168, 2048, SWIGLU, 0, 0), (128, 10240, 1016, BF16, 1, 0), (128, 10240, 2048, RESID_F32, 1, 0)])
+    (128, 6400, 1280, BF16, 1, 1), (128, 4480, 1280, SWIGLU, 0, 1), (160, 4480, 1280, SWIGLU, 0, 0), (192, 7168, 2048, SWIGLU, 0, 1), (224, 7168, 2048, SWIGLU, 0, 0), (128, 10240, 1016, BF16, 1, 0), (128, 10240, 2048, RESID_F32, 1, 0),
+    (129, 264, 4104, BF16, 1, 0)])          # cut along k instead
 def test_which_products_take_it(m, n, k, epilogue, packed, takes):
     if not _ext.load():
         pytest.skip("the kernel library cannot be built here")

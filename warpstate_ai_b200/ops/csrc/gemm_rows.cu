@@ -256,7 +256,7 @@ static int rows_columns(int m) { return m <= 256 ? (m + 31) / 32 * 32 : (m + 63)
 
 using namespace ws;
 
-// Whether a product takes this kernel: few tokens, and the rounds over the chip times what a k-block takes, in units of 0.28 us
+// Whether a product takes this kernel: few tokens, not so few tiles that it is cut along k, and the rounds over the chip times what a k-block takes, in units of 0.28 us
 // (256 x 256 x 64 on a pair), here and on the pair kernel.  The SwiGLU epilogue costs 1-2 us more here, with half of its
 // warps waiting for the others, so it needs a wider margin, above all behind a short contraction.  Measured with cold
 // weights (pair -> here, us): in_proj of d 2048 at 128 tokens 23.6 -> 20.5, 192 23.6 -> 22.6, 256 23.6 -> 23.4, 300 33.8 -> 26.7,
@@ -264,7 +264,9 @@ using namespace ws;
 // 448 37.9 -> 36.9, 512 37.9 -> 41.0; d 1280 in_proj at 128 17.4 -> 16.4, 300 17.4 -> 18.5, up/gate at 128 18.5 -> 18.4, 192 18.4 -> 19.5.
 extern "C" int ws_gemm_rows_takes(int m, int n, int k, int epilogue, int packed, int sms) {
   const bool swiglu = epilogue == WS_EPI_SWIGLU;
-  if ((epilogue != WS_EPI_BF16 && !(swiglu && !packed)) || m < 96 || m > rowsk::MAX_TOKENS || n % 8 != 0 || k < 1024 || sms < 2) return 0;
+  if ((epilogue != WS_EPI_BF16 && !(swiglu && !packed)) || m < 96 || m > rowsk::MAX_TOKENS || n % 8 != 0 || k < 1024 || sms < 2 ||
+      ws_gemm_plan(m, n, k, 0, epilogue, packed, sms) > 1)
+    return 0;
   const int pairs = sms / 2, columns = rows_columns(m), weights = swiglu ? 2 * n : n;
   const int here = ((weights + 255) / 256 + pairs - 1) / pairs;
   const int there = ((m + 255) / 256 * ((weights + 255) / 256) + pairs - 1) / pairs;
