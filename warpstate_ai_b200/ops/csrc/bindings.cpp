@@ -441,7 +441,8 @@ at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast
 // ----------------------------------------------------------------------------- whole blocks
 // The kernel sequences of one block (ops/fused.py) as one call each.  A block is eight to twelve launches of 2-20 us in
 // a short sequence, and issued one by one from Python the host takes longer than the device below a few thousand rows;
-// here a launch costs its allocation, its tensor maps and the launch.  Same kernels, same order, same results.
+// here a launch costs its allocation, its tensor maps and the launch.  Same arithmetic in the same order; one launch fewer where
+// out_proj is cut along k.
 // Smoke model (d 256, 4 depths, 2 x 512 tokens), forward + backward: 2.53 -> 2.03 ms.
 at::Tensor project(const at::Tensor& x, const at::Tensor& w, bool b_mn, int64_t epilogue, int64_t n, at::Tensor out,
                    const c10::optional<at::Tensor>& out2, const c10::optional<at::Tensor>& aux,
@@ -461,6 +462,40 @@ at::Tensor input_grad(const at::Tensor& dy, const at::Tensor& w, const c10::opti
   return project(dy, w, true, WS_EPI_BF16, w.size(1), at::empty({dy.size(0), w.size(1)}, dy.options()), c10::nullopt, c10::nullopt, flag);
 }
 
+// (x + y W^T, its RMSNorm in BF16, the norm's factors).  Where the product is cut along k, the kernel that adds the pieces
+// does the norm as well.
+std::tuple<at::Tensor, at::Tensor, at::Tensor> project_residual_norm(const at::Tensor& y, const at::Tensor& w, const at::Tensor& resid,
+                                                                     const at::Tensor& norm, double eps,
+                                                                     const c10::optional<at::Tensor>& flag) {
+  const int64_t m = y.size(0), n = w.size(0), k = y.size(1);
+  const auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  if (resid.scalar_type() == at::kFloat && n % 128 == 0 && n <= 2048 && k % 8 == 0 && w.dim() == 2 && w.size(1) == k && y.is_contiguous() &&
+      w.is_contiguous() && resid.is_contiguous() && resid.size(0) == m && resid.size(1) == n && aligned(y) && aligned(w) && aligned(resid) &&
+      y.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && norm.scalar_type() == at::kFloat && norm.is_contiguous() &&
+      norm.numel() == n && aligned(norm)) {
+    WsGemm g = {};
+    g.a = y.data_ptr(); g.b = w.data_ptr();
+    g.m = (int)m; g.n = (int)n; g.k = (int)k; g.lda = (int)k; g.ldb = (int)k;
+    g.epilogue = WS_EPI_RESID_F32;
+    g.aux = resid.data_ptr(); g.ldaux = (int)n; g.ldo = (int)n;
+    g.alpha = 1.f;
+    g.error_flag = reinterpret_cast<int*>(const_cast<void*>(opt_ptr(flag)));
+    c10::cuda::CUDAGuard guard(y.device());
+    const int splits = ws_gemm_splits(&g);
+    if (splits > 1) {
+      at::Tensor part = at::empty({splits, m, n}, resid.options()), x2 = at::empty_like(resid), z = at::empty({m, n}, y.options());
+      at::Tensor rstd = at::empty({m}, resid.options());
+      g.out = x2.data_ptr();
+      check_rc(ws_gemm_split_norm(&g, splits, part.data_ptr<float>(), norm.data_ptr<float>(), (float)eps, z.data_ptr(),
+                                  rstd.data_ptr<float>(), cur_stream()), "gemm_split_norm");
+      return {x2, z, rstd};
+    }
+  }
+  at::Tensor x2 = project_residual(y, w, resid, flag);
+  auto [z, rstd, unchanged] = rmsnorm_fwd(x2, c10::nullopt, c10::nullopt, norm, eps, false);
+  return {x2, z, rstd};
+}
+
 // x2 = xmod + out_proj(y), then x2 + down(swiglu(up_gate(norm2 x2))).  -> (x2, rstd2, z2, packed, act, x3); packed only
 // with `keep` (the backward pass reads it), x3 only with `want_output`.  `wide` (serving): (up, gate) are not rounded.
 struct BlockTail { at::Tensor x2, rstd2, z2, packed, act, x3; };
@@ -468,9 +503,7 @@ BlockTail block_tail(const at::Tensor& y, const at::Tensor& xmod, const at::Tens
                      const at::Tensor& w_ug, const at::Tensor& w_down, double eps, bool keep, bool want_output,
                      const c10::optional<at::Tensor>& flag, bool wide = false) {
   BlockTail t;
-  t.x2 = project_residual(y, w_out, xmod, flag);
-  at::Tensor unchanged;
-  std::tie(t.z2, t.rstd2, unchanged) = rmsnorm_fwd(t.x2, c10::nullopt, c10::nullopt, n2, eps, false);
+  std::tie(t.x2, t.z2, t.rstd2) = project_residual_norm(y, w_out, xmod, n2, eps, flag);
   const int64_t h = w_ug.size(0) / 2;
   if (keep) t.packed = at::empty({y.size(0), 2 * h}, y.options());
   t.act = at::empty({y.size(0), h}, y.options());

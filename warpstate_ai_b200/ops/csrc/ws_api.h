@@ -63,6 +63,9 @@ int ws_gemm_pair_available(void);  // 1 where problems with >= 256 rows take the
 // A product whose tiles would leave most of the chip idle may be cut along k: ws_gemm_splits says into how many pieces
 // (1: not), and ws_gemm_split computes it so, with FP32 scratch `part` of splits * m * n floats.
 int ws_gemm_splits(const WsGemm* g);
+// A residual product (FP32) cut into `splits` > 1 pieces and the RMSNorm behind it: z [m, n] = BF16(out * rstd * w), rstd [m].
+// n % 128 == 0, n <= 2048.
+int ws_gemm_split_norm(const WsGemm* g, int splits, float* part, const float* w, float eps, void* z, float* rstd, cudaStream_t stream);
 // Which kernel a product takes on `sms` SMs, a function of its arguments alone: 0 the single-CTA kernel, otherwise the
 // CTA-pair kernel with the product cut along k into that many pieces.  packed: a SwiGLU product writes (up | gate).
 int ws_gemm_plan(int m, int n, int k, int a_mn, int epilogue, int packed, int sms);
