@@ -248,13 +248,10 @@ __device__ __forceinline__ void tail_norm_row(float* x, const float* partial, in
       const float4 q = __ldcg(reinterpret_cast<const float4*>(partial + (static_cast<size_t>(s) * batch + b) * d + col));
       v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
     }
-    if (scale != nullptr) {
-      const float4 sc = *reinterpret_cast<const float4*>(scale + col), bi = *reinterpret_cast<const float4*>(bias + col);
-      v.x = v.x * (1.f + sc.x) + bi.x; v.y = v.y * (1.f + sc.y) + bi.y;
-      v.z = v.z * (1.f + sc.z) + bi.z; v.w = v.w * (1.f + sc.w) + bi.w;
-    }
+    if (scale != nullptr)
+      v = modulated(v, *reinterpret_cast<const float4*>(scale + col), *reinterpret_cast<const float4*>(bias + col));
     *reinterpret_cast<float4*>(xr + col) = v;
-    ss[block & 1] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    ss[block & 1] = __fadd_rn(ss[block & 1], square_sum(v));
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

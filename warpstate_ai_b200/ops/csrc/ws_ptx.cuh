@@ -317,6 +317,15 @@ __device__ __forceinline__ float bf16_round(float x) {
   return __bfloat162float(__float2bfloat16_rn(x));
 }
 
+// What the norms of a decode step add up and form, with every rounding written out: three kernels do it and agree bit for bit.
+__device__ __forceinline__ float square_sum(const float4& v) {
+  return __fmaf_rn(v.w, v.w, __fmaf_rn(v.z, v.z, __fmaf_rn(v.y, v.y, __fmul_rn(v.x, v.x))));
+}
+__device__ __forceinline__ float4 modulated(const float4& v, const float4& scale, const float4& bias) {
+  return make_float4(__fmaf_rn(v.x, __fadd_rn(1.f, scale.x), bias.x), __fmaf_rn(v.y, __fadd_rn(1.f, scale.y), bias.y),
+                     __fmaf_rn(v.z, __fadd_rn(1.f, scale.z), bias.z), __fmaf_rn(v.w, __fadd_rn(1.f, scale.w), bias.w));
+}
+
 }  // namespace ws
 
 // ----------------------------------------------------------------------------- CTA pairs (cluster of 2)
