@@ -885,8 +885,8 @@ split_finish_kernel(const float* part, int splits, int m, int n, const void* aux
 }
 
 // The same behind a residual product that an RMSNorm follows (out_proj, then the second norm): a block per row adds the pieces
-// and the residual, writes x and z = BF16(x rsqrt(mean x^2 + eps) w).  The squares are added in the norm kernel's order (lane l
-// of a warp owns columns 128 i + 4 l), so that both forms agree.  n % 128 == 0, n <= 2048.  300 x 2048 in
+// and the residual, writes x and z = BF16(x rsqrt(mean x^2 + eps) w).  The squares are rounded and added as the norm kernels
+// do it (`square_sum`; lane l of a warp owns columns 128 i + 4 l), so that both forms agree bit for bit.  n % 128 == 0, n <= 2048.  300 x 2048 in
 // four pieces: 3.2 us and the norm's 5.0 before, 3.7 so; 128 x 2048: 2.5 and 5.1, 3.0.
 __global__ void __launch_bounds__(256)
 split_finish_norm_kernel(const float* part, int splits, int m, int n, const float* aux, int ldaux, float* __restrict__ out, int ldo,
@@ -915,7 +915,7 @@ split_finish_norm_kernel(const float* part, int splits, int m, int n, const floa
       if (s < splits) { v.x += p[s].x; v.y += p[s].y; v.z += p[s].z; v.w += p[s].w; }
     v = make_float4(r.x + v.x, r.y + v.y, r.z + v.z, r.w + v.w);
     *reinterpret_cast<float4*>(out + static_cast<size_t>(row) * ldo + c) = v;
-    squares[c >> 2] = v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+    squares[c >> 2] = square_sum(v);
     x[i] = v;
   }
   __syncthreads();

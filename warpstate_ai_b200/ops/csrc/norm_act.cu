@@ -63,12 +63,10 @@ rmsnorm_fwd_kernel(const T* x, const float* col_scale,
     for (int c = lane * 4; c < d; c += 128) {
       float4 v = ld4(xr + c);
       if (col_scale != nullptr) {
-        const float4 s = ld4(col_scale + c), b = ld4(col_bias + c);
-        v.x = v.x * (1.f + s.x) + b.x; v.y = v.y * (1.f + s.y) + b.y;
-        v.z = v.z * (1.f + s.z) + b.z; v.w = v.w * (1.f + s.w) + b.w;
+        v = modulated(v, ld4(col_scale + c), ld4(col_bias + c));
         if (sizeof(T) == 2) { v.x = bf16_round(v.x); v.y = bf16_round(v.y); v.z = bf16_round(v.z); v.w = bf16_round(v.w); }
       }
-      ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+      ss += square_sum(v);
     }
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / static_cast<float>(d) + eps);
@@ -76,9 +74,7 @@ rmsnorm_fwd_kernel(const T* x, const float* col_scale,
     for (int c = lane * 4; c < d; c += 128) {
       float4 v = ld4(xr + c);
       if (col_scale != nullptr) {
-        const float4 s = ld4(col_scale + c), b = ld4(col_bias + c);
-        v.x = v.x * (1.f + s.x) + b.x; v.y = v.y * (1.f + s.y) + b.y;
-        v.z = v.z * (1.f + s.z) + b.z; v.w = v.w * (1.f + s.w) + b.w;
+        v = modulated(v, ld4(col_scale + c), ld4(col_bias + c));
         if (sizeof(T) == 2) { v.x = bf16_round(v.x); v.y = bf16_round(v.y); v.z = bf16_round(v.z); v.w = bf16_round(v.w); }
       }
       const float4 ww = ld4(w + c);
@@ -118,14 +114,12 @@ rmsnorm_fwd_rows_kernel(const T* x, const float* col_scale,
     for (int i = 0; i < CHUNKS; ++i) {
       if (col_scale != nullptr) {
         const int c = i * 128 + lane * 4;
-        const float4 s = ld4(col_scale + c), b = ld4(col_bias + c);
-        v[i].x = v[i].x * (1.f + s.x) + b.x; v[i].y = v[i].y * (1.f + s.y) + b.y;
-        v[i].z = v[i].z * (1.f + s.z) + b.z; v[i].w = v[i].w * (1.f + s.w) + b.w;
+        v[i] = modulated(v[i], ld4(col_scale + c), ld4(col_bias + c));
         if (sizeof(T) == 2) {
           v[i].x = bf16_round(v[i].x); v[i].y = bf16_round(v[i].y); v[i].z = bf16_round(v[i].z); v[i].w = bf16_round(v[i].w);
         }
       }
-      ss += v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+      ss += square_sum(v[i]);
     }
     ss = warp_sum(ss);
     const float rstd = rsqrtf(ss / static_cast<float>(d) + eps);
@@ -167,14 +161,12 @@ rmsnorm_fwd_block_kernel(const T* x, const float* col_scale, const float* col_bi
     v[i] = ld4(x + base + c);
     ww[i] = ld4_parameter(w + c);
     if (col_scale != nullptr) {
-      const float4 s = ld4(col_scale + c), b = ld4(col_bias + c);
-      v[i].x = v[i].x * (1.f + s.x) + b.x; v[i].y = v[i].y * (1.f + s.y) + b.y;
-      v[i].z = v[i].z * (1.f + s.z) + b.z; v[i].w = v[i].w * (1.f + s.w) + b.w;
+      v[i] = modulated(v[i], ld4(col_scale + c), ld4(col_bias + c));
       if (sizeof(T) == 2) {
         v[i].x = bf16_round(v[i].x); v[i].y = bf16_round(v[i].y); v[i].z = bf16_round(v[i].z); v[i].w = bf16_round(v[i].w);
       }
     }
-    squares[c >> 2] = v[i].x * v[i].x + v[i].y * v[i].y + v[i].z * v[i].z + v[i].w * v[i].w;
+    squares[c >> 2] = square_sum(v[i]);
   }
   __syncthreads();
   if (threadIdx.x < 32) {
