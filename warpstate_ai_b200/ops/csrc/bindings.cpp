@@ -568,10 +568,19 @@ struct BlockSpec {
   at::Tensor main[4];   // their FP32 gradients; undefined without a backward pass
   at::Tensor rope;
   c10::optional<at::Tensor> flag;
+  at::Tensor hooked;    // CPU word: a hook on finished gradients is set
+  int64_t core;         // its number for the core
+  bool notify;
   double eps;
   int64_t H;
   bool keep;
 };
+// Into Python (ops/fused.py): the small gradients are added to their buffers there, and the hook is called.
+bool core_finished(int64_t core, bool notify, at::TensorList small) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("ws_b200::core_finished", "")
+                             .typed<bool(int64_t, bool, at::TensorList)>();
+  return op.call(core, notify, small);
+}
 
 struct BlockFn : public torch::autograd::Function<BlockFn> {
   static at::Tensor vector(const at::Tensor& t) { return t.defined() ? t.detach().to(at::kFloat).contiguous() : t; }
@@ -598,7 +607,8 @@ struct BlockFn : public torch::autograd::Function<BlockFn> {
       data["logits"] = std::vector<at::Tensor>(logits, logits + 3);
       data["rope"] = spec->rope;
       data["flag"] = spec->flag.has_value() ? *spec->flag : at::Tensor();
-      data["shape"] = std::vector<int64_t>{B, T, d, spec->H, sc.defined() ? 1 : 0};
+      data["hooked"] = spec->hooked;
+      data["shape"] = std::vector<int64_t>{B, T, d, spec->H, sc.defined() ? 1 : 0, spec->core, spec->notify ? 1 : 0};
     }
     return s[0].view({B, T, d});
   }
@@ -623,25 +633,30 @@ struct BlockFn : public torch::autograd::Function<BlockFn> {
     const at::Tensor into[4] = {main[3], main[2], main[1], main[0]};
     const double betas[4] = {1.0, 1.0, 1.0, 1.0};
     grad_weight_group(dys, xs, into, betas, flag);
+    // Whether the hook on finished gradients is set counts now, not when the forward pass ran.
     const at::Tensor none;
-    return {r[0].view({B, T, d}), modulated ? r[7].select(0, 2) : none, modulated ? r[7].select(0, 1) : none, r[7].select(0, 0),
-            r[5], none, none, none, none, r[6].select(0, 0), r[6].select(0, 1), r[6].select(0, 2), none};
+    std::vector<at::Tensor> small = {r[7].select(0, 0), r[5], r[6].select(0, 0), r[6].select(0, 1), r[6].select(0, 2)};
+    if (*data["hooked"].toTensor().data_ptr<int>() != 0 && core_finished(shape[5], shape[6] != 0, small)) small.assign(5, none);
+    return {r[0].view({B, T, d}), modulated ? r[7].select(0, 2) : none, modulated ? r[7].select(0, 1) : none, small[0],
+            small[1], none, none, none, none, small[2], small[3], small[4], none};
   }
 };
 
 at::Tensor block(const at::Tensor& x, const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& bias,
                  const at::Tensor& n1, const at::Tensor& n2, at::TensorList weights, at::TensorList bf16, at::TensorList main,
                  const at::Tensor& fast, const at::Tensor& slow, const at::Tensor& mix, const at::Tensor& rope, double eps,
-                 int64_t H, const c10::optional<at::Tensor>& flag) {
+                 int64_t H, const c10::optional<at::Tensor>& flag, const at::Tensor& hooked, int64_t core, bool notify) {
   TORCH_CHECK(x.dim() == 3 && x.scalar_type() == at::kFloat && weights.size() == 4 && bf16.size() == 4 &&
               (main.size() == 4 || (main.empty() && !at::GradMode::is_enabled())) && scale.has_value() == bias.has_value(),
               "block: FP32 x [B, T, d], four weights, their BF16 copies and FP32 gradients");
+  TORCH_CHECK(hooked.is_cpu() && hooked.scalar_type() == at::kInt && hooked.numel() == 1, "block: hooked must be one int32 on the CPU");
   BlockSpec spec;
   for (int i = 0; i < 4; ++i) {
     spec.bf16[i] = bf16[i];
     if (!main.empty()) spec.main[i] = main[i];
   }
   spec.rope = rope; spec.flag = flag; spec.eps = eps; spec.H = H; spec.keep = at::GradMode::is_enabled();
+  spec.hooked = hooked; spec.core = core; spec.notify = notify;
   return BlockFn::apply(x, scale, bias, n1, n2, weights[0], weights[1], weights[2],
                         weights[3], fast, slow, mix, static_cast<const BlockSpec*>(&spec));
 }
@@ -1364,7 +1379,9 @@ TORCH_LIBRARY(ws_b200, m) {
         "Tensor states, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor w_in, Tensor w_out, Tensor w_ug, Tensor w_down, "
         "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, int B, int T, int H, Tensor(a!)? flag) -> Tensor[]");
   m.def("block(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor[] weights, Tensor[] bf16, Tensor[] main, "
-        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int H, Tensor? error_flag) -> Tensor");
+        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int H, Tensor? error_flag, Tensor hooked, "
+        "int core, bool notify) -> Tensor");
+  m.def("core_finished(int core, bool notify, Tensor[] small) -> bool");
   m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
         "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
         "Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, bool last, "

@@ -27,7 +27,10 @@ gradient is returned to autograd.
 from __future__ import annotations
 
 import contextlib
+import itertools
 import os
+import threading
+import weakref
 
 import torch
 import torch.nn.functional as F
@@ -65,13 +68,16 @@ def _ops():
 
 
 _core_grad_hook = None
+with torch.inference_mode(False):       # this module may be imported by a first call in inference mode
+    _hook_word = torch.zeros(1, dtype=torch.int32, device="cpu")     # 1 while the hook is set, for native code
 
 
 def set_core_grad_hook(fn) -> None:
-    """``fn(core)`` is called when a core's weight gradients are final for this backward pass
-    (used by the gradient synchroniser to start reducing that core's bucket early)."""
+    """``fn(core)`` is called when a core's gradients are final for this backward pass (used by the gradient synchroniser
+    to start reducing that core's bucket early).  What counts is whether it is set when the backward pass gets there."""
     global _core_grad_hook
     _core_grad_hook = fn
+    _hook_word.fill_(0 if fn is None else 1)
 
 
 # --------------------------------------------------------------------------- BF16 weight views
@@ -373,6 +379,49 @@ def _attach_small_grads(core, g_n1, g_n2, g_fast, g_slow, g_mix) -> None:
         main.add_(g.to(main.dtype))
 
 
+# A native block's node asks for the hook behind its backward pass as `CoreFn` does, and goes into Python only where it is set.
+# It has a number for the core.
+_core_keys: weakref.WeakKeyDictionary = weakref.WeakKeyDictionary()
+_cores: weakref.WeakValueDictionary = weakref.WeakValueDictionary()
+_next_key = itertools.count()
+
+
+def _core_key(core) -> int:
+    key = _core_keys.get(core)
+    if key is None:
+        key = _core_keys[core] = next(_next_key)
+        _cores[key] = core
+    return key
+
+
+def _core_finished(key, notify, small) -> bool:
+    """`small`: gradients of the two norms and the three logits.  True if they are taken over, False if autograd is to add them
+    (no hook, not the depth that finishes the core, or nobody holds the core any more)."""
+    core = _cores.get(key)
+    if core is None or _core_grad_hook is None or not notify:
+        return False
+    _attach_small_grads(core, *small)
+    _core_grad_hook(core)
+    return True
+
+
+_native_lock = threading.Lock()
+_native_library = None      # the registration lasts as long as this object
+
+
+def _native_block():
+    """The operator, once its call back into Python has been registered."""
+    global _native_library
+    if _native_library is None:
+        with _native_lock:
+            if _native_library is None:
+                _ext.require()
+                library = torch.library.Library("ws_b200", "IMPL")
+                library.impl("core_finished", _core_finished, "CompositeImplicitAutograd")
+                _native_library = library
+    return _ops().block
+
+
 def _block_node(core, x, depth_scale, depth_bias, notify):
     """The block as one native autograd node (`BlockFn` of the library), or None where `CoreFn` is needed: a rounded stream,
     weights that are sharded or whose gradients autograd is to hold, a hook on finished gradients, a tuned GEMM choice."""
@@ -386,10 +435,10 @@ def _block_node(core, x, depth_scale, depth_bias, notify):
         main = [getattr(w, "main_grad", None) for w in weights]
         if any(m is None for m in main) or any(getattr(w, "bf16_view", None) is None for w in weights):
             return None
-    return _ops().block(x, depth_scale, depth_bias, core.norm1.weight, core.norm2.weight, weights,
-                        [bf16_weight(w) for w in weights], main, core.fast_decay_logit, core.slow_decay_logit,
-                        core.memory_mix_logit, attention.rope_table(x.device, pair_major=True), core.cfg.rms_eps, core.h,
-                        G.error_flag(x.device))
+    return _native_block()(x, depth_scale, depth_bias, core.norm1.weight, core.norm2.weight, weights,
+                           [bf16_weight(w) for w in weights], main, core.fast_decay_logit, core.slow_decay_logit,
+                           core.memory_mix_logit, attention.rope_table(x.device, pair_major=True), core.cfg.rms_eps, core.h,
+                           G.error_flag(x.device), _hook_word, _core_key(core), notify)
 
 
 def core_forward(core, x: torch.Tensor, depth_scale=None, depth_bias=None, notify: bool = True,
