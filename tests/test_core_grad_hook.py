@@ -1,5 +1,6 @@
 """The hook on a core's finished gradients: set for the backward pass alone or for both, it fires once per core and finds every
-gradient of the core final."""
+gradient of the core final, also where several depths share the core (their norms' and logits' gradients would otherwise be
+added after it, to a bucket that is already being reduced)."""
 import gc
 import weakref
 
@@ -72,7 +73,7 @@ class Node(torch.autograd.Function):
         return dy * 2.0, scale, bias, n1, n2, fast, slow, mix, None, None, None, None
 
 
-@pytest.mark.parametrize("cores,depth", [(1, 1), (2, 2)])
+@pytest.mark.parametrize("cores,depth", [(1, 1), (2, 4), (2, 3)])
 def test_a_native_node_leaves_nothing_behind_the_hook(monkeypatch, cores, depth):
     def block(x, scale, bias, n1, n2, weights, bf16, main, fast, slow, mix, rope, eps, heads, flag, hooked, core, notify):
         return Node.apply(x, scale, bias, n1, n2, fast, slow, mix, main, hooked, core, notify)
@@ -93,8 +94,8 @@ def test_a_native_node_leaves_nothing_behind_the_hook(monkeypatch, cores, depth)
 @pytest.mark.parametrize("hook_in_forward", [False, True])
 @pytest.mark.parametrize("native", [True, False])
 @pytest.mark.parametrize("checkpoint", [False, True])
-@pytest.mark.parametrize("cores,depth", [(2, 2)])
-def test_on_the_device(monkeypatch, cores, depth, native, checkpoint, hook_in_forward):
+@pytest.mark.parametrize("cores,depth", [(2, 2), (2, 4)])
+def test_shared_cores_on_the_device(monkeypatch, cores, depth, native, checkpoint, hook_in_forward):
     net = model("cuda", cores, depth).train()
     net.cfg.gradient_checkpointing = checkpoint
     arena = ParamArena(net)

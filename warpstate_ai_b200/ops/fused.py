@@ -342,10 +342,11 @@ class CoreFn(torch.autograd.Function):
         weights.end_backward()
         if side is not None:
             torch.cuda.current_stream(dx_in.device).wait_stream(side)
-        if ctx.notify and _core_grad_hook is not None:
+        if _core_grad_hook is not None:
             _attach_small_grads(core, g_n1, g_n2, g_fast, g_slow, g_mix)
-            _core_grad_hook(core)
             g_n1 = g_n2 = g_fast = g_slow = g_mix = None
+            if ctx.notify:
+                _core_grad_hook(core)
         return (dx_in.view(batch, seq, d), g_scale, g_bias, g_n1, g_in, g_out, g_n2, g_ug, g_down,
                 g_fast, g_slow, g_mix, None, None, None, None)
 
@@ -366,8 +367,8 @@ def _modulation_sums(dx_in, x_in, scale):
 
 
 def _attach_small_grads(core, g_n1, g_n2, g_fast, g_slow, g_mix) -> None:
-    """Add the core's small-parameter gradients to the arena now (instead of letting autograd do
-    it after this node returns) so that the whole bucket is final when the hook fires."""
+    """Add the core's small-parameter gradients to the arena now, so that the whole bucket is final when the hook fires.
+    Autograd would add them once the last depth that uses the core has returned, the earlier depths' included."""
     pairs = ((core.norm1.weight, g_n1), (core.norm2.weight, g_n2), (core.fast_decay_logit, g_fast),
              (core.slow_decay_logit, g_slow), (core.memory_mix_logit, g_mix))
     for p, g in pairs:
@@ -396,12 +397,13 @@ def _core_key(core) -> int:
 
 def _core_finished(key, notify, small) -> bool:
     """`small`: gradients of the two norms and the three logits.  True if they are taken over, False if autograd is to add them
-    (no hook, not the depth that finishes the core, or nobody holds the core any more)."""
+    (no hook, or nobody holds the core any more)."""
     core = _cores.get(key)
-    if core is None or _core_grad_hook is None or not notify:
+    if core is None or _core_grad_hook is None:
         return False
     _attach_small_grads(core, *small)
-    _core_grad_hook(core)
+    if notify:
+        _core_grad_hook(core)
     return True
 
 
