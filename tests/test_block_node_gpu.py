@@ -100,3 +100,30 @@ def test_a_hook_on_finished_gradients_takes_the_python_node(monkeypatch):
     with autocast():
         core(x).sum().backward()
     assert called == [core]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("train", [False, True])
+def test_a_bias_without_a_scale_is_no_modulation(monkeypatch, train):
+    """Every form of a block takes such a call: the modulation is its scale's to ask for."""
+    core = block(4)
+    ParamArena(core)
+    x, bias = torch.randn(2, 128, 256, device="cuda"), torch.randn(256, device="cuda")
+    with torch.set_grad_enabled(train), autocast():
+        native = core(x, None, bias)
+        assert torch.equal(native, core(x))
+        monkeypatch.setattr(fused, "_block_node", lambda *a: None)
+        assert torch.equal(native, core(x, None, bias))
+        with fused.disabled():
+            plain = core(x, None, bias)
+        assert torch.allclose(native, plain.float(), rtol=0.1, atol=0.1)
+
+
+@pytest.mark.gpu
+def test_scoring_in_inference_mode():
+    core = block(5)
+    x = torch.randn(1, 256, 256, device="cuda")
+    with autocast(), torch.no_grad():
+        want = core(x)
+    with autocast(), torch.inference_mode():
+        assert torch.equal(core(x), want) and torch.equal(core(x.clone()), want)

@@ -437,6 +437,8 @@ def _block_node(core, x, depth_scale, depth_bias, notify):
         main = [getattr(w, "main_grad", None) for w in weights]
         if any(m is None for m in main) or any(getattr(w, "bf16_view", None) is None for w in weights):
             return None
+    if depth_scale is None:      # the bias belongs to the modulation, here as in the other forms of a block
+        depth_bias = None
     return _native_block()(x, depth_scale, depth_bias, core.norm1.weight, core.norm2.weight, weights,
                            [bf16_weight(w) for w in weights], main, core.fast_decay_logit, core.slow_decay_logit,
                            core.memory_mix_logit, attention.rope_table(x.device, pair_major=True), core.cfg.rms_eps, core.h,
