@@ -127,3 +127,21 @@ def test_scoring_in_inference_mode():
         want = core(x)
     with autocast(), torch.inference_mode():
         assert torch.equal(core(x), want) and torch.equal(core(x.clone()), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arena", [True, False])
+def test_a_compiled_caller(arena):
+    """`torch.compile` around a block, or around the code that calls one, runs the block as it is."""
+    core = block(6)
+    if arena:
+        ParamArena(core)
+    x = torch.randn(2, 128, 256, device="cuda")
+    dy = torch.randn(2, 128, 256, device="cuda")
+    want = run(core, x.requires_grad_(True), (None, None), dy)
+    got = run(torch.compile(core, backend="eager"), x, (None, None), dy)
+    for a, b in zip(want, got):
+        assert (a is None) == (b is None) and (a is None or torch.equal(a, b))
+    with torch.no_grad(), autocast():
+        assert torch.equal(torch.compile(lambda t: core(t) * 2.0, backend="eager")(x), want[0] * 2.0)
+    torch._dynamo.reset()

@@ -426,9 +426,10 @@ def _native_block():
 
 def _block_node(core, x, depth_scale, depth_bias, notify):
     """The block as one native autograd node (`BlockFn` of the library), or None where `CoreFn` is needed: a rounded stream,
-    weights that are sharded or whose gradients autograd is to hold, a hook on finished gradients, a tuned GEMM choice."""
+    weights that are sharded or whose gradients autograd is to hold, a hook on finished gradients, a tuned GEMM choice, or a
+    tracer, which would run the node on tensors without data where it leaves `CoreFn` alone."""
     from . import attention
-    if x.dtype != torch.float32 or (notify and _core_grad_hook is not None) or G._policy or not attention.kernels_ready(core) \
+    if torch.compiler.is_compiling() or x.dtype != torch.float32 or (notify and _core_grad_hook is not None) or G._policy or not attention.kernels_ready(core) \
             or getattr(core, "ws_weights", None) is not None:
         return None
     weights = (core.in_proj.weight, core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight)
