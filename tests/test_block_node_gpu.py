@@ -145,3 +145,20 @@ def test_a_compiled_caller(arena):
     with torch.no_grad(), autocast():
         assert torch.equal(torch.compile(lambda t: core(t) * 2.0, backend="eager")(x), want[0] * 2.0)
     torch._dynamo.reset()
+
+
+@pytest.mark.gpu
+@pytest.mark.filterwarnings("ignore:.*autograd kernel was not registered")
+@pytest.mark.parametrize("native", [True, False])
+def test_create_graph_gives_gradients_without_a_second_derivative(monkeypatch, native):
+    core = block(7)
+    ParamArena(core)
+    if not native:
+        monkeypatch.setattr(fused, "_block_node", lambda *a: None)
+    x, dy = (torch.randn(1, 128, 256, device="cuda", requires_grad=True) for _ in range(2))
+    with autocast():
+        y = core(x)
+    plain, = torch.autograd.grad(y, [x], dy, retain_graph=True)
+    gradient, = torch.autograd.grad(y, [x], dy, create_graph=True)
+    assert gradient.requires_grad and torch.equal(gradient, plain)
+    assert torch.autograd.grad(gradient.sum(), [x, dy], allow_unused=True) == (None, None)

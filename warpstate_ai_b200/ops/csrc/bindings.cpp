@@ -582,6 +582,18 @@ bool core_finished(int64_t core, bool notify, at::TensorList small) {
   return op.call(core, notify, small);
 }
 
+std::vector<at::Tensor> differentiated_block_bwd(
+    const at::Tensor& dx3, const at::Tensor& x, const at::Tensor& rstd1, const at::Tensor& qkvgu, const at::Tensor& x2,
+    const at::Tensor& rstd2, const at::Tensor& packed, const at::Tensor& writes, const at::Tensor& states,
+    const c10::optional<at::Tensor>& scale, const c10::optional<at::Tensor>& bias, const at::Tensor& n1, const at::Tensor& n2,
+    const at::Tensor& w_in, const at::Tensor& w_out, const at::Tensor& w_ug, const at::Tensor& w_down, const at::Tensor& fast_logit,
+    const at::Tensor& slow_logit, const at::Tensor& mix_logit, const at::Tensor& rope, int64_t B, int64_t T, int64_t H,
+    const c10::optional<at::Tensor>& flag) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("ws_b200::block_bwd", "").typed<decltype(block_bwd)>();
+  return op.call(dx3, x, rstd1, qkvgu, x2, rstd2, packed, writes, states, scale, bias, n1, n2, w_in, w_out, w_ug, w_down, fast_logit,
+                 slow_logit, mix_logit, rope, B, T, H, flag);
+}
+
 struct BlockFn : public torch::autograd::Function<BlockFn> {
   static at::Tensor vector(const at::Tensor& t) { return t.defined() ? t.detach().to(at::kFloat).contiguous() : t; }
   static c10::optional<at::Tensor> maybe(const at::Tensor& t) { return t.defined() ? c10::optional<at::Tensor>(t) : c10::nullopt; }
@@ -625,9 +637,10 @@ struct BlockFn : public torch::autograd::Function<BlockFn> {
     const c10::optional<at::Tensor> flag = maybe(flag_tensor);
     const at::Tensor dx3 = grads[0].reshape({B * T, d}).contiguous();
     const auto scale = modulated ? c10::optional<at::Tensor>(t[1]) : c10::nullopt, bias = modulated ? c10::optional<at::Tensor>(t[2]) : c10::nullopt;
-    std::vector<at::Tensor> r = block_bwd(dx3, t[0], t[5], t[7], t[9], t[10], t[12], attention[0], attention[1], scale, bias,
-                                          vector(t[3]), vector(t[4]), w[0], w[1], w[2], w[3], logits[0], logits[1], logits[2],
-                                          data["rope"].toTensor(), B, T, shape[3], flag);
+    // With create_graph the call goes through the dispatcher, which marks its results as having no second derivative.
+    std::vector<at::Tensor> r = (at::GradMode::is_enabled() ? differentiated_block_bwd : block_bwd)(
+        dx3, t[0], t[5], t[7], t[9], t[10], t[12], attention[0], attention[1], scale, bias, vector(t[3]), vector(t[4]), w[0], w[1],
+        w[2], w[3], logits[0], logits[1], logits[2], data["rope"].toTensor(), B, T, shape[3], flag);
     // r: dx, dx3 BF16, dpacked, dx2 BF16, dqkvgu, g_norm2, logit gradients, first norm's (and bias and scale)
     const at::Tensor dys[4] = {r[1], r[2], r[3], r[4]}, xs[4] = {t[13], t[11], t[8], t[6]};
     const at::Tensor into[4] = {main[3], main[2], main[1], main[0]};
