@@ -47,9 +47,13 @@ def test_the_second_norm_is_that_of_the_norm_kernel(tokens, d):
     w_in, w_out, w_ug, w_down = ((torch.randn(n, k, device="cuda") * 0.03).bfloat16()
                                  for n, k in ((5 * d, d), (d, d), (2 * ffn, d), (d, ffn)))
     logits = torch.randn(3, heads, device="cuda").unbind(0)
-    x2, rstd2, z2 = torch.ops.ws_b200.block_fwd(x, scale, bias, n1, w_in, w_out, n2, w_ug, w_down, *logits,
-                                                attention.rope_table(x.device, pair_major=True), 1e-5, 1, tokens, heads, False, True,
-                                                gemm.error_flag(x.device))[6:9]
+    def block(w_out):
+        return torch.ops.ws_b200.block_fwd(x, scale, bias, n1, w_in, w_out, n2, w_ug, w_down, *logits,
+                                           attention.rope_table(x.device, pair_major=True), 1e-5, 1, tokens, heads, False, True,
+                                           gemm.error_flag(x.device))
+    x2, rstd2, z2 = block(w_out)[6:9]
     gemm.check_device_errors()
+    with pytest.raises(RuntimeError, match="CUDA"):      # refused on the host, as by the two launches
+        block(w_out.cpu())
     z, rstd, _ = torch.ops.ws_b200.rmsnorm_fwd(x2, None, None, n2, 1e-5, False)
     assert torch.equal(rstd2, rstd) and torch.equal(z2, z)

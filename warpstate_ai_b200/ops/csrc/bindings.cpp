@@ -468,8 +468,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> project_residual_norm(const at::T
                                                                      const at::Tensor& norm, double eps,
                                                                      const c10::optional<at::Tensor>& flag) {
   const int64_t m = y.size(0), n = w.size(0), k = y.size(1);
-  const auto aligned = [](const at::Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
-  if (resid.scalar_type() == at::kFloat && n % 128 == 0 && n <= 2048 && k % 8 == 0 && w.dim() == 2 && w.size(1) == k && y.is_contiguous() &&
+  const auto aligned = [&](const at::Tensor& t) { return t.device() == y.device() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; };
+  if (y.is_cuda() && resid.scalar_type() == at::kFloat && n % 128 == 0 && n <= 2048 && k % 8 == 0 && w.dim() == 2 && w.size(1) == k && y.is_contiguous() &&
       w.is_contiguous() && resid.is_contiguous() && resid.size(0) == m && resid.size(1) == n && aligned(y) && aligned(w) && aligned(resid) &&
       y.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && norm.scalar_type() == at::kFloat && norm.is_contiguous() &&
       norm.numel() == n && aligned(norm)) {
