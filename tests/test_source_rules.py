@@ -5,6 +5,7 @@
   CTA mask is the ``tcgen05.commit`` that signals both CTAs' barriers and moves no data.
 * The batched asynchronous memory-copy entry points of the CUDA runtime and driver are not used (nor named).
 * Device code neither traps nor asserts: a wait that runs out records a status and the kernel returns.
+* Whether a warp goes on to an instruction that it executes as one is not decided lane by lane.
 * Every translation unit is compiled for sm_100a with line information.
 * Comments and docstrings stand on their own: they name no planning document of this build and no path of a machine.
 """
@@ -126,3 +127,51 @@ def test_kernels_that_wait_for_their_predecessor_promise_no_read_only_inputs():
             waiting += 1
             assert not promise.search(head), (p.name, head)
     assert waiting > 20
+
+
+ONE_LANE = ("lane == 0", "elect_one()", "tid == 0", "threadIdx.x == 0", "et == 0")
+ONE_LANE_FUNCTIONS = ("tail_produce", "tail_mma")       # of decode_layer.cu, called by one lane
+
+
+def sites(text, name):
+    """``(line, inside one lane's code, statement so far)`` of every call of ``name``."""
+    text = "\n".join(line.split("//")[0] for line in text.splitlines())
+    scopes, begin, found = [], 0, []
+    for match in re.finditer(r"[;{}]|\b" + name + r"(?=[<(])", text):
+        token, statement = match.group(0), text[begin:match.start()]
+        if token == "{":
+            scopes.append(statement)
+        elif token == "}" and scopes:
+            scopes.pop()
+        if token in ";{}":
+            begin = match.end()
+            continue
+        if "__forceinline__" in statement:               # its definition
+            continue
+        context = [*scopes, statement]
+        alone = any(word in scope for scope in context for word in ONE_LANE) or any(
+            "__device__" in scope and f"{function}(" in scope for scope in scopes for function in ONE_LANE_FUNCTIONS)
+        found.append((text[:match.start()].count("\n") + 1, alone, statement))
+    return found
+
+
+def test_a_warp_decides_as_one_what_it_does_as_one():
+    """A bounded wait answers each lane for itself.  An epilogue warp of which some lanes gave up and some did not would meet
+    tcgen05.ld in part and never come back: such waits go through `mbar_wait_warp`.  The attention kernels go on whatever a
+    wait says, or vote; no jump there hangs on one lane's answer either."""
+    whole = one = 0
+    for p in NATIVE:
+        if p.suffix != ".cu":
+            continue
+        text = p.read_text()
+        for function in ONE_LANE_FUNCTIONS:
+            for line, alone, _ in sites(text, function):
+                assert alone, (p.name, line)
+        for line, alone, statement in sites(text, "mbar_wait"):
+            one += alone
+            if not alone:
+                assert p.name.startswith("attention_") and not re.search(r"\bif\s*\(", statement), (p.name, line, statement.strip())
+        for line, alone, _ in sites(text, "mbar_wait_warp"):
+            whole += 1
+            assert not alone, (p.name, line)             # a vote of all lanes, in code of one
+    assert whole >= 10 and one >= 20

@@ -187,7 +187,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   } else {
     const int quarter = warp & 3;  // TMEM lane quarter this warp may read
     const int row = quarter * 32 + lane;
-    const bool ok = kb1 > kb0 && mbar_wait(tfull, 0, abort_flag);
+    const bool ok = kb1 > kb0 && mbar_wait_warp(tfull, 0, abort_flag);
     tc_fence_after_sync();
     const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
     if (EPI == 2) {

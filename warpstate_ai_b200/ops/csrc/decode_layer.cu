@@ -175,7 +175,7 @@ __device__ __forceinline__ void tail_epilogue(const TailCta& c, const TailItem& 
   using namespace tail;
   const int quarter = warp & 3;
   const int row = quarter * 32 + lane;
-  const bool ok = w.valid && mbar_wait(c.tfull, tparity, c.abort_flag);
+  const bool ok = w.valid && mbar_wait_warp(c.tfull, tparity, c.abort_flag);
   tc_fence_after_sync();
   const uint32_t taddr = c.tmem + (static_cast<uint32_t>(quarter * 32) << 16);
   if (EPI == 2) {

@@ -371,7 +371,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const int buf_t = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
         tc_fence_after_sync();
         const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
         const int row = y + lane;
@@ -433,7 +433,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         const GemmParams& p = g.p[t.prob];
         const int buf_t = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
         tc_fence_after_sync();
         const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
@@ -498,7 +498,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       for (int tile = pair_id; tile < tiles && ok; tile += num_pairs, ++tcount) {
         const int buf_t = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
         tc_fence_after_sync();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
 #pragma unroll 1
@@ -512,7 +512,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           }
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + step * 32, r);
-          if (!mbar_wait(&mybar[buf], (q >> 1) & 1, abort_flag)) {
+          if (!mbar_wait_warp(&mybar[buf], (q >> 1) & 1, abort_flag)) {
             ok = false;
             tmem_ld_wait();
             break;
@@ -570,7 +570,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       for (int tile = pair_id; tile < tiles && ok; tile += num_pairs, ++tcount) {
         const int buf_t = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait(&tfull[buf_t], tph, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
         tc_fence_after_sync();
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
 #pragma unroll 1
@@ -585,7 +585,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           }
           uint32_t r[32];
           tmem_ld_32x32b_x32(taddr + step * 32, r);
-          if (!mbar_wait(&mybar[buf], (q >> 1) & 1, abort_flag)) {
+          if (!mbar_wait_warp(&mybar[buf], (q >> 1) & 1, abort_flag)) {
             ok = false;
             tmem_ld_wait();
             break;
@@ -637,20 +637,20 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
     } else {
       [[maybe_unused]] WarpStage sender;
       if constexpr (tiled_epilogue<EPI>()) sender.tiles = eStage + (warp - 2) * 4096;
-      // (rows that go back to their places before a selection are stored one by one)
-            for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
+      for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
         const GemmParams& p = g.p[t.prob];
         const int nb = t.nb;
         sender.map = &g.epi[t.prob];
         const int buf = tcount & 1;
         const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait(&tfull[buf], tph, abort_flag)) break;
+        if (!mbar_wait_warp(&tfull[buf], tph, abort_flag)) break;
         tc_fence_after_sync();
         const int row = t.mb * 2 * BM + rank * BM + quarter * 32 + lane;
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf * BN;
         const bool inside = row < p.m;
         const int place = p.row_map != nullptr && inside ? p.row_map[row] : row;  // the row before the selection
+        // rows that go back to their places before a selection are stored one by one
         WarpStage* const stage = tiled_epilogue<EPI>() && p.row_map == nullptr ? &sender : nullptr;
         float rs = 1.0f;
         if (p.row_scale != nullptr && inside) rs = place >= 0 ? p.row_scale[place] : 0.f;

@@ -167,8 +167,8 @@ gemm_rows_kernel(const __grid_constant__ RowsProblem p) {
     for (int tile = pair; tile < tiles; tile += pairs, ++count) {
       const int buf = p.buffers == 2 ? count & 1 : 0;
       const uint32_t use = p.buffers == 2 ? count >> 1 : count;
-      bool ok = mbar_wait(&tfull[buf], use & 1, abort_flag);
-      if constexpr (SWIGLU) {   // the group meets at barriers below: if one of its threads gave up, all leave together
+      bool ok = mbar_wait_warp(&tfull[buf], use & 1, abort_flag);
+      if constexpr (SWIGLU) {   // the group meets at barriers below: if one of its warps gave up, all leave together
         uint32_t bad;
         if (group == 0)
           asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 1, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
@@ -177,8 +177,6 @@ gemm_rows_kernel(const __grid_constant__ RowsProblem p) {
           asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 2, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
                        : "=r"(bad) : "r"(ok ? 0u : 1u) : "memory");
         ok = bad == 0u;
-      } else {
-        ok = __all_sync(0xffffffffu, ok);
       }
       if (!ok) break;
       tc_fence_after_sync();

@@ -198,7 +198,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
       tile_coords(tile, num_m, num_n, mb, nb);
       const int buf = tcount & 1;
       const uint32_t tph = (tcount >> 1) & 1;
-      if (!mbar_wait(&tfull[buf], tph, abort_flag)) break;
+      if (!mbar_wait_warp(&tfull[buf], tph, abort_flag)) break;
       tc_fence_after_sync();
       const int row = mb * BM + quarter * 32 + lane;
       const bool row_ok = row < p.m;

@@ -76,6 +76,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   }
 }
 
+// The same for all lanes of a converged warp, with one answer: true where every lane saw the barrier complete.  The lanes ask
+// one after another, so where the time runs out as the barrier completes some may see it and some not.  Whether a warp goes on
+// to what it does as one (tcgen05.ld, __syncwarp, its place in a group's barrier) is decided by this form or by a vote: met in
+// part, such an instruction does not end.  `mbar_wait` is for the roles of one lane, and where all lanes go on in any case.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
+}
+
 // ----------------------------------------------------------------------------- proxies
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
