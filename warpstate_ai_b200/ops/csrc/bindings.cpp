@@ -1391,8 +1391,8 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("block_bwd(Tensor dx3, Tensor x, Tensor rstd1, Tensor qkvgu, Tensor x2, Tensor rstd2, Tensor packed, Tensor writes, "
         "Tensor states, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor w_in, Tensor w_out, Tensor w_ug, Tensor w_down, "
         "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, int B, int T, int H, Tensor(a!)? flag) -> Tensor[]");
-  m.def("block(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor[] weights, Tensor[] bf16, Tensor[] main, "
-        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int H, Tensor? error_flag, Tensor hooked, "
+  m.def("block(Tensor x, Tensor? scale, Tensor? bias, Tensor n1, Tensor n2, Tensor[] weights, Tensor[] bf16, Tensor(a!)[] main, "
+        "Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int H, Tensor(b!)? error_flag, Tensor hooked, "
         "int core, bool notify) -> Tensor");
   m.def("core_finished(int core, bool notify, Tensor[] small) -> bool");
   m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
