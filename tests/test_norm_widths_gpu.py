@@ -1,4 +1,5 @@
-"""RMSNorm forward at the widths that keep a row in registers and beside them, and column sums of many partial rows."""
+"""RMSNorm forward by each of its kernels (a block per row up to 1184 rows, a warp that holds the row in registers past them, for
+every width up to 2048, and the general one for wider rows), which agree bit for bit, and column sums of many partial rows."""
 import pytest
 import torch
 
@@ -6,7 +7,8 @@ import torch
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("modulated", [False, True])
-@pytest.mark.parametrize("rows,d", [(1, 256), (9, 1280), (1792, 1280), (513, 256), (7, 384), (300, 2048)])
+@pytest.mark.parametrize("rows,d", [(1, 256), (9, 1280), (1792, 1280), (513, 256), (7, 384), (300, 2048), (1184, 1920), (1185, 256),
+                                    (1300, 384), (1185, 2048), (10000, 128), (3, 2176), (1300, 2176), (9600, 4096)])
 def test_forward(rows, d, modulated, dtype):
     from warpstate_ai_b200.ops import _ext
     _ext.require()
@@ -24,6 +26,24 @@ def test_forward(rows, d, modulated, dtype):
     # FP32 stream: one rounding to BF16; BF16 stream: the normalised value, the weight and their product are rounded
     roundings = 1 if dtype is torch.float32 else 3
     assert ((z.double() - want * factor * w.double()).abs() <= roundings * 2.0 ** -8 * (want * factor * w.double()).abs() + 1e-6).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("modulated", [False, True])
+@pytest.mark.parametrize("d", range(128, 2049, 128))
+def test_few_rows_and_many_give_the_same(d, modulated, dtype):
+    from warpstate_ai_b200.ops import _ext
+    _ext.require()
+    torch.manual_seed(d)
+    x = torch.randn(1185, d, device="cuda").to(dtype)
+    scale, bias, w = (torch.randn(d, device="cuda") * 0.2 for _ in range(3))
+    mod = (scale, bias) if modulated else (None, None)
+    many = torch.ops.ws_b200.rmsnorm_fwd(x, *mod, w, 1e-5, True)
+    few = torch.ops.ws_b200.rmsnorm_fwd(x[:1184], *mod, w, 1e-5, True)
+    last = torch.ops.ws_b200.rmsnorm_fwd(x[1184:], *mod, w, 1e-5, True)
+    for a, b, c in zip(many, few, last):
+        assert torch.equal(a[:1184], b) and torch.equal(a[1184:], c)
 
 
 @pytest.mark.gpu

@@ -1,14 +1,16 @@
 // Bandwidth-bound row kernels: RMSNorm forward / backward (with the depth modulation of the
 // residual stream folded in), casts, column sums and the embedding gather / scatter.
 //
-// One warp owns one row; a lane owns columns {lane*4 + 128*i}.  Row statistics are FP32
-// (the reference norm, warpstate/model.py:22-28; its Triton twin ops/activation_execution.py:96-158).
+// One warp owns one row (few rows of a forward norm: a block owns one); a lane owns columns {lane*4 + 128*i}.  Row statistics
+// are FP32 (the reference norm, warpstate/model.py:22-28; its Triton twin ops/activation_execution.py:96-158).
 // Weight-gradient column sums are accumulated per lane in registers, reduced across the warps
 // of a block in shared memory and written as one partial row per block; a second kernel adds the
 // partial rows in a fixed order, so the result does not depend on scheduling.
 #include "ws_ptx.cuh"
 #include "ws_api.h"
 #include "ws_launch.h"
+
+#include <utility>
 
 namespace ws {
 
@@ -143,7 +145,7 @@ rmsnorm_fwd_rows_kernel(const T* x, const float* col_scale,
 
 // The same for few rows, a block per row: with a warp per row, 300 rows are 38 blocks whose lanes walk 16 loads, as many pairs
 // of modulation values and 16 stores each.  A thread has two pieces of four columns; the squares are added in the order of
-// the kernels above (lane l of a warp: columns 128 i + 4 l), so that the three agree.  d <= 2048.
+// the kernels above (lane l of a warp: columns 128 i + 4 l), so that they agree bit for bit.  d <= 2048.
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS)
 rmsnorm_fwd_block_kernel(const T* x, const float* col_scale, const float* col_bias, const float* w, float eps, int d,
@@ -482,10 +484,37 @@ embed_bwd_kernel(const T* __restrict__ dx, const long long* __restrict__ sorted_
   }
 }
 
+constexpr int CHIP_BLOCKS = 148 * 8;   // blocks of ROW_THREADS that the chip holds at once
 static int row_grid(int rows) {
   int blocks = (rows + ROW_WARPS - 1) / ROW_WARPS;
-  const int cap = 148 * 8;
-  return blocks < cap ? (blocks > 0 ? blocks : 1) : cap;
+  return blocks < CHIP_BLOCKS ? (blocks > 0 ? blocks : 1) : CHIP_BLOCKS;
+}
+
+template <typename T>
+using RmsnormRows = void (*)(const T*, const float*, const float*, const float*, float, int, T*, __nv_bfloat16*, float*);
+// The kernel that holds rows of 128 * chunks columns (1..MAX_CHUNKS) in registers.
+template <typename T, int... I>
+static RmsnormRows<T> rmsnorm_rows(int chunks, std::integer_sequence<int, I...>) {
+  static constexpr RmsnormRows<T> kernels[] = {rmsnorm_fwd_rows_kernel<T, I + 1>...};
+  return kernels[chunks - 1];
+}
+
+template <typename T>
+static void launch_rmsnorm_fwd(const T* x, const float* col_scale, const float* col_bias, const float* w, float eps, int rows, int d,
+                               T* xmod_out, __nv_bfloat16* z, float* rstd, cudaStream_t stream) {
+  // One round of blocks over the chip; past it a warp per row has as many loads in flight.  Measured (modulated, FP32; the
+  // kernels below -> here, us): 2048 columns 128 rows 4.3 -> 2.5, 300 4.4 -> 2.8, 1184 6.2 -> 5.2; 1280 columns 300 rows
+  // 5.6 -> 2.6, 1184 6.7 -> 4.0; 256 columns 2.2 -> 2.0.
+  if (rows <= CHIP_BLOCKS && d <= 128 * MAX_CHUNKS)
+    launch_dependent(rmsnorm_fwd_block_kernel<T>, dim3(rows), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, d,
+                     xmod_out, z, rstd);
+  else if (d <= 128 * MAX_CHUNKS)   // the general kernel reads its rows twice: 4096 rows of 384, 1024, 1920 columns 5.1, 10.7, 19.7 us, 3.6, 6.5, 12.2 so
+    launch_dependent(rmsnorm_rows<T>(d / 128, std::make_integer_sequence<int, MAX_CHUNKS>{}), dim3(row_grid(rows)),
+                     dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, rows, xmod_out, z, rstd);
+  else
+    launch_dependent(rmsnorm_fwd_kernel<T>, dim3(row_grid(rows)), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps,
+                     rows, d, xmod_out, z, rstd);
+  ws_count_launch();
 }
 
 }  // namespace ws
@@ -496,41 +525,12 @@ extern "C" int ws_rmsnorm_fwd(const void* x, int x_bf16, const float* col_scale,
                               const float* w, float eps, int rows, int d, void* xmod_out, void* z,
                               float* rstd, cudaStream_t stream) {
   if (d % 128 != 0 || rows <= 0) return -1;
-  const int grid = row_grid(rows);
-  // One round of blocks over 148 SMs, eight of 256 threads on each; past it a warp per row has as many loads in flight.
-  // Measured (modulated, FP32; the kernels below -> here, us): 2048 columns 128 rows 4.3 -> 2.5, 300 4.4 -> 2.8, 1184 6.2 -> 5.2; 1280
-  // columns 300 rows 5.6 -> 2.6, 1184 6.7 -> 4.0; 256 columns 2.2 -> 2.0.
-  if (rows <= 1184 && d <= 2048) {
-    if (x_bf16)
-      launch_dependent(rmsnorm_fwd_block_kernel<__nv_bfloat16>, dim3(rows), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)x,
-                       col_scale, col_bias, w, eps, d, (__nv_bfloat16*)xmod_out, (__nv_bfloat16*)z, rstd);
-    else
-      launch_dependent(rmsnorm_fwd_block_kernel<float>, dim3(rows), dim3(ROW_THREADS), 0, stream, (const float*)x, col_scale,
-                       col_bias, w, eps, d, (float*)xmod_out, (__nv_bfloat16*)z, rstd);
-    ws_count_launch();
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  }
-  // The widths of the configurations this library is used with: the row stays in registers.  1792 x 1280: 9.6 us by the general
-  // kernel, 6.2 so.
-  const auto rows_form = [&](auto f32_kernel, auto bf16_kernel) {
-    if (x_bf16)
-      launch_dependent(bf16_kernel, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)x,
-                       col_scale, col_bias, w, eps, rows, (__nv_bfloat16*)xmod_out, (__nv_bfloat16*)z, rstd);
-    else
-      launch_dependent(f32_kernel, dim3(grid), dim3(ROW_THREADS), 0, stream, (const float*)x, col_scale,
-                       col_bias, w, eps, rows, (float*)xmod_out, (__nv_bfloat16*)z, rstd);
-    ws_count_launch();
-    return cudaGetLastError() == cudaSuccess ? 0 : -2;
-  };
-  if (d == 2048) return rows_form(rmsnorm_fwd_rows_kernel<float, 16>, rmsnorm_fwd_rows_kernel<__nv_bfloat16, 16>);
-  if (d == 1280) return rows_form(rmsnorm_fwd_rows_kernel<float, 10>, rmsnorm_fwd_rows_kernel<__nv_bfloat16, 10>);
-  if (d == 256) return rows_form(rmsnorm_fwd_rows_kernel<float, 2>, rmsnorm_fwd_rows_kernel<__nv_bfloat16, 2>);
   if (x_bf16)
-    launch_dependent(rmsnorm_fwd_kernel<__nv_bfloat16>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)x, col_scale, col_bias, w, eps, rows, d, (__nv_bfloat16*)xmod_out,
-        (__nv_bfloat16*)z, rstd);
+    launch_rmsnorm_fwd(static_cast<const __nv_bfloat16*>(x), col_scale, col_bias, w, eps, rows, d,
+                       static_cast<__nv_bfloat16*>(xmod_out), static_cast<__nv_bfloat16*>(z), rstd, stream);
   else
-    launch_dependent(rmsnorm_fwd_kernel<float>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const float*)x, col_scale, col_bias, w, eps, rows, d, (float*)xmod_out, (__nv_bfloat16*)z, rstd);
-  ws_count_launch();
+    launch_rmsnorm_fwd(static_cast<const float*>(x), col_scale, col_bias, w, eps, rows, d, static_cast<float*>(xmod_out),
+                       static_cast<__nv_bfloat16*>(z), rstd, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
