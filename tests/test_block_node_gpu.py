@@ -72,8 +72,10 @@ def test_scoring_pass_and_transposed_input(monkeypatch):
         assert torch.equal(native, core(x, scale, bias))
     monkeypatch.undo()
     with autocast():                                       # gradients that autograd holds: the Python node
-        assert type(core(x, scale, bias).grad_fn).__name__ != type(None).__name__
         assert fused._block_node(core, x, scale, bias, True) is None
+        assert type(core(x, scale, bias).grad_fn).__name__ == "CoreFnBackward"
+        ParamArena(core)                                   # gradients that the arena holds: the native one
+        assert "BlockFn" in core(x, scale, bias).grad_fn.name()
 
 
 @pytest.mark.gpu

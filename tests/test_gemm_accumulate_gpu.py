@@ -28,3 +28,26 @@ def test_accumulated_stored_and_scaled_gradients(tokens, betas):
         bound = tokens * 2.0 ** -24 * (dy.double().abs().T @ x.double().abs()) + 2.0 ** -22 * want.abs() + 1e-30
         assert ((w[:, :k].double() - want).abs() <= bound).all(), beta
         assert torch.equal(w[:, k:], old[:, k:])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("accumulate", [True, False])
+def test_a_bulk_reduction_is_a_read_an_addition_and_a_write(accumulate):
+    """Bit for bit the gradients of the single-CTA kernel, whose threads do that."""
+    from warpstate_ai_b200.ops import _ext, gemm
+    lib = _ext.cdll()
+    torch.manual_seed(1)
+    dy, x = torch.randn(1000, 520, device="cuda").bfloat16(), torch.randn(1000, 328, device="cuda").bfloat16()
+    before = torch.randn(520, 328, device="cuda")
+    results = []
+    try:
+        for mode in (1, 0):
+            lib.ws_gemm_set_pair_mode(mode)
+            grad = before.clone()
+            gemm.grad_weight_accumulate_group([(dy, x, grad, accumulate)])
+            gemm.grad_weight_accumulate(dy, x, grad, accumulate=True, alpha=0.3)
+            results.append(grad)
+    finally:
+        lib.ws_gemm_set_pair_mode(-1)
+    gemm.check_device_errors()
+    assert torch.equal(*results)

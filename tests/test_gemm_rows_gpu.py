@@ -63,3 +63,38 @@ def test_swiglu_without_up_and_gate(m, h, k, wide):
     slope = 1.1 * (up.abs() + 1)                       # of silu, and what an error of gate's sum does to the product
     bound = (2.0 ** -8 * (1 if wide else 3) + 2.0 ** -9) * want.abs() + slope * (2.0 ** -9 * gate.abs() * (0 if wide else 1) + 1e-5)
     assert ((act.double() - want).abs() <= bound + 2.0 ** -10 * up.abs()).all()
+
+
+@pytest.fixture
+def settings():
+    """(SM limit, CTA pairs or not) of the library, put back afterwards."""
+    lib = _ext.cdll()
+    def set_to(sms=0, pairs=-1):
+        lib.ws_gemm_set_sm_limit(sms)
+        lib.ws_gemm_set_pair_mode(pairs)
+    yield set_to
+    set_to()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k,epilogue,sms", [
+    (300, 32768, 2048, BF16, 148), (320, 19208, 1024, BF16, 148), (128, 40000, 1024, BF16, 148), (300, 9600, 2048, SWIGLU, 148),
+    (300, 4104, 1024, BF16, 20), (96, 1288, 1024, BF16, 4), (257, 1288, 1088, BF16, 2), (300, 2056, 2048, SWIGLU, 8), (128, 2056, 2048, SWIGLU, 4)])
+def test_several_tiles_to_a_pair(settings, m, n, k, epilogue, sms):
+    """One accumulator (above 256 tokens) or two are filled again, and the SwiGLU warps' exchange goes on from tile to tile.  The
+    results are those of the single-CTA kernel, which has the tokens in its rows and stores row by row, bit for bit."""
+    from warpstate_ai_b200.ops import gemm
+    lib = _ext.cdll()
+    sms = min(sms, torch.cuda.get_device_properties(0).multi_processor_count)
+    settings(sms=sms)
+    assert lib.ws_gemm_rows_takes(m, n, k, epilogue, 0, sms)
+    assert (n + (255 if epilogue == BF16 else 127)) // (256 if epilogue == BF16 else 128) > sms // 2
+    x, w, want, error = product(m, n, k, epilogue)
+    def run():
+        return gemm.linear(x, w) if epilogue == BF16 else gemm.linear_swiglu(x, w, want_packed=False, wide=True)[1]
+    got = run()
+    settings(pairs=0)
+    assert torch.equal(got, run())
+    gemm.check_device_errors()
+    if epilogue == BF16:
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + error).all()

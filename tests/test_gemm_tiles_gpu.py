@@ -49,3 +49,23 @@ def test_kept_logits_and_label_log_probabilities(rows, vocab, keep):
     want = torch.log_softmax(rounded, dim=-1).gather(1, labels[:, None])[:, 0]
     assert torch.allclose(logp.double(), want, rtol=0, atol=float(2.0 ** -8 * exact.abs().max()))
     assert torch.allclose(lse.double(), torch.logsumexp(rounded, dim=-1), rtol=0, atol=1e-3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,k", [(256, 264, 64), (300, 1000, 512), (2000, 1096, 1024)])
+def test_tiles_carry_what_rows_would(m, n, k):
+    """Bit for bit the results of the single-CTA kernel, which stores row by row; kept logits are the head's product."""
+    from warpstate_ai_b200.ops import _ext, gemm
+    lib = _ext.cdll()
+    torch.manual_seed(n)
+    x, w = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    try:
+        lib.ws_gemm_set_pair_mode(1)
+        pair = gemm.linear(x, w)
+        kept = torch.ops.ws_b200.lm_head_fwd_labelled(x, w, torch.zeros(m, dtype=torch.long, device="cuda"), -100, m,
+                                                      gemm.error_flag(x.device))[-1]
+        lib.ws_gemm_set_pair_mode(0)
+        assert torch.equal(pair, gemm.linear(x, w)) and torch.equal(kept, pair)
+    finally:
+        lib.ws_gemm_set_pair_mode(-1)
+    gemm.check_device_errors()
