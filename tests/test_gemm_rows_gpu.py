@@ -13,7 +13,10 @@ BF16, RESID_F32, SWIGLU = 0, 1, 2
     (257, 10240, 2048, BF16, 1, 1), (300, 10240, 2048, BF16, 1, 1), (384, 10240, 2048, BF16, 1, 1), (448, 10240, 2048, BF16, 1, 1), (512, 10240, 2048, BF16, 1, 0),
     (513, 10240, 2048, BF16, 1, 0), (300, 7168, 2048, SWIGLU, 0, 1), (300, 7168, 2048, SWIGLU, 1, 0), (300, 6400, 1280, BF16, 1, 0),
     (128, 6400, 1280, BF16, 1, 1), (128, 4480, 1280, SWIGLU, 0, 1), (160, 4480, 1280, SWIGLU, 0, 0), (192, 7168, 2048, SWIGLU, 0, 1), (224, 7168, 2048, SWIGLU, 0, 0), (128, 10240, 1016, BF16, 1, 0), (128, 10240, 2048, RESID_F32, 1, 0),
-    (129, 264, 4104, BF16, 1, 0)])          # cut along k instead
+    (129, 264, 4104, BF16, 1, 0),          # cut along k instead
+    # twice the rounds of the single-CTA kernel; less than that; as many
+    (128, 32768, 2048, BF16, 1, 0), (96, 20480, 4096, BF16, 1, 0), (128, 10752, 3072, SWIGLU, 0, 0), (128, 37888, 2048, BF16, 1, 0),
+    (128, 37896, 2048, BF16, 1, 1), (96, 60000, 2048, BF16, 1, 0), (160, 32768, 2048, BF16, 1, 1), (128, 18944, 2048, BF16, 1, 1), (128, 18952, 2048, BF16, 1, 0)])
 def test_which_products_take_it(m, n, k, epilogue, packed, takes):
     if not _ext.load():
         pytest.skip("the kernel library cannot be built here")
@@ -31,7 +34,7 @@ def product(m, n, k, epilogue):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k", [(96, 10240, 1024), (128, 6400, 1088), (129, 4104, 1280), (257, 9480, 2048), (300, 10240, 2048),
-                                   (320, 10008, 1032), (321, 10248, 1024), (128, 19208, 1024)])
+                                   (320, 10008, 1032), (321, 10248, 1024), (160, 19208, 1024)])
 def test_bf16_results(m, n, k):
     from warpstate_ai_b200.ops import gemm
     _ext.require()
@@ -79,7 +82,7 @@ def settings():
 @pytest.mark.gpu
 @pytest.mark.parametrize("m,n,k,epilogue,sms", [
     (300, 32768, 2048, BF16, 148), (320, 19208, 1024, BF16, 148), (128, 40000, 1024, BF16, 148), (300, 9600, 2048, SWIGLU, 148),
-    (300, 4104, 1024, BF16, 20), (96, 1288, 1024, BF16, 4), (257, 1288, 1088, BF16, 2), (300, 2056, 2048, SWIGLU, 8), (128, 2056, 2048, SWIGLU, 4)])
+    (300, 4104, 1024, BF16, 20), (160, 1288, 1024, BF16, 4), (257, 1288, 1088, BF16, 2), (300, 2056, 2048, SWIGLU, 8), (160, 2056, 2048, SWIGLU, 4)])
 def test_several_tiles_to_a_pair(settings, m, n, k, epilogue, sms):
     """One accumulator (above 256 tokens) or two are filled again, and the SwiGLU warps' exchange goes on from tile to tile.  The
     results are those of the single-CTA kernel, which has the tokens in its rows and stores row by row, bit for bit."""

@@ -254,19 +254,29 @@ static int rows_columns(int m) { return m <= 256 ? (m + 31) / 32 * 32 : (m + 63)
 
 using namespace ws;
 
-// Whether a product takes this kernel: few tokens, not so few tiles that it is cut along k, and the rounds over the chip times what a k-block takes, in units of 0.28 us
-// (256 x 256 x 64 on a pair), here and on the pair kernel.  The SwiGLU epilogue costs 1-2 us more here, with half of its
-// warps waiting for the others, so it needs a wider margin, above all behind a short contraction.  Measured with cold
-// weights (pair -> here, us): in_proj of d 2048 at 128 tokens 23.6 -> 20.5, 192 23.6 -> 22.6, 256 23.6 -> 23.4, 300 33.8 -> 26.7,
-// 384 33.8 -> 28.7, 448 33.8 -> 30.8, 512 33.8 -> 32.8; up/gate at 128 27.6 -> 24.6, 192 27.7 -> 26.7, 224 27.6 -> 28.7, 300 37.9 -> 32.8,
-// 448 37.9 -> 36.9, 512 37.9 -> 41.0; d 1280 in_proj at 128 17.4 -> 16.4, 300 17.4 -> 18.5, up/gate at 128 18.5 -> 18.4, 192 18.4 -> 19.5.
+// Whether a product takes this kernel: few tokens, not so few tiles that it is cut along k, and the rounds over the chip times
+// what a k-block takes, in units of 0.28 us (256 x 256 x 64 on a pair), here and on the pair kernel.  The SwiGLU epilogue costs
+// 1-2 us more here, with half of its warps waiting for the others, so it needs a wider margin, above all behind a short
+// contraction.  Measured with cold weights (pair -> here, us): in_proj of d 2048 at 128 tokens 23.6 -> 20.5, 192 23.6 -> 22.6,
+// 256 23.6 -> 23.4, 300 33.8 -> 26.7, 384 33.8 -> 28.7, 448 33.8 -> 30.8, 512 33.8 -> 32.8; up/gate at 128 27.6 -> 24.6, 192
+// 27.7 -> 26.7, 224 27.6 -> 28.7, 300 37.9 -> 32.8, 448 37.9 -> 36.9, 512 37.9 -> 41.0; d 1280 in_proj at 128 17.4 -> 16.4, 300
+// 17.4 -> 18.5, up/gate at 128 18.5 -> 18.4, 192 18.4 -> 19.5.
+// And where the single-CTA kernel would take the product, fewer than twice the rounds that it needs: its tiles of 128 tokens are
+// spread over all SMs one by one, so 75 to 148 of them are one round there and two here, 128 x 20480 outputs of k 4096 38.9 ->
+// 47.3 us, 128 x 32768 of k 2048 27.7 -> 27.5, SwiGLU 128 x 10752 of k 2048 21.8 -> 28.2; but three rounds for two pay, 128 x 40000 of
+// k 1024 26.4 -> 21.3, of k 2048 43.6 -> 37.5, SwiGLU 128 x 27000 of k 2048 43.8 -> 41.5.
+// In a chain of launches, over 29 sizes of W (k 1024 to 4096) at 12 token counts: what is taken takes 0.73 to 1.00 of what it did
+// as a BF16 product and 0.79 to 1.05 as SwiGLU; the slower ones are 160 to 192 tokens at few tiles, and 160 to 300 at k 3072
+// where two rounds are nearly empty.
 extern "C" int ws_gemm_rows_takes(int m, int n, int k, int epilogue, int packed, int sms) {
   const bool swiglu = epilogue == WS_EPI_SWIGLU;
-  if ((epilogue != WS_EPI_BF16 && !(swiglu && !packed)) || m < 96 || m > rowsk::MAX_TOKENS || n % 8 != 0 || k < 1024 || sms < 2 ||
-      ws_gemm_plan(m, n, k, 0, epilogue, packed, sms) > 1)
+  if ((epilogue != WS_EPI_BF16 && !(swiglu && !packed)) || m < 96 || m > rowsk::MAX_TOKENS || n % 8 != 0 || k < 1024 || sms < 2)
     return 0;
+  const int plan = ws_gemm_plan(m, n, k, 0, epilogue, packed, sms);
   const int pairs = sms / 2, columns = rows_columns(m), weights = swiglu ? 2 * n : n;
   const int here = ((weights + 255) / 256 + pairs - 1) / pairs;
+  const int single = ((m + 127) / 128 * ((weights + 255) / 256) + sms - 1) / sms;
+  if (plan > 1 || (plan == 0 && here >= 2 * single)) return 0;
   const int there = ((m + 255) / 256 * ((weights + 255) / 256) + pairs - 1) / pairs;
   const float tensor = columns / 256.f, intake = (16384.f + 64.f * columns) / 32768.f;
   const float margin = !swiglu ? 0.97f : k >= 2048 ? 0.9f : 0.8f;
