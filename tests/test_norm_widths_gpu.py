@@ -1,5 +1,5 @@
-"""RMSNorm forward by each of its kernels (a block per row up to 1184 rows, a warp that holds the row in registers past them, for
-every width up to 2048, and the general one for wider rows), which agree bit for bit, and column sums of many partial rows."""
+"""RMSNorm forward by each of its kernels (a block per row where rows are few, a warp that holds the row in registers past that,
+for every width up to 2048, and the general one for wider rows), which agree bit for bit, and column sums of many partial rows."""
 import pytest
 import torch
 
@@ -40,10 +40,10 @@ def test_few_rows_and_many_give_the_same(d, modulated, dtype):
     scale, bias, w = (torch.randn(d, device="cuda") * 0.2 for _ in range(3))
     mod = (scale, bias) if modulated else (None, None)
     many = torch.ops.ws_b200.rmsnorm_fwd(x, *mod, w, 1e-5, True)
-    few = torch.ops.ws_b200.rmsnorm_fwd(x[:1184], *mod, w, 1e-5, True)
-    last = torch.ops.ws_b200.rmsnorm_fwd(x[1184:], *mod, w, 1e-5, True)
-    for a, b, c in zip(many, few, last):
-        assert torch.equal(a[:1184], b) and torch.equal(a[1184:], c)
+    for rows in (1184, 297, 296, 1):
+        few = torch.ops.ws_b200.rmsnorm_fwd(x[-rows:], *mod, w, 1e-5, True)
+        for a, b in zip(many, few):
+            assert torch.equal(a[-rows:], b)
 
 
 @pytest.mark.gpu

@@ -499,13 +499,21 @@ static RmsnormRows<T> rmsnorm_rows(int chunks, std::integer_sequence<int, I...>)
   return kernels[chunks - 1];
 }
 
+// Up to how many rows a block for each is faster than a warp.  Wide rows: one round of blocks over the chip.  Narrow ones leave
+// most of a block idle, and past two blocks to an SM its start costs more than the warp's longer walk; the modulation's loads
+// lengthen that walk.  Measured in a chain of launches (a warp -> a block per row, FP32, us): modulated 2048 columns 64 rows 3.9 ->
+// 2.0, 300 3.9 -> 2.4, 1100 6.2 -> 4.3; 1280 columns 300 rows 3.4 -> 2.2, 1100 5.6 -> 3.4; 384 columns 592 rows 2.0 -> 1.8, 1100 2.9 ->
+// 2.2; 256 columns 64 rows 1.6 -> 1.5, 1024 2.0 -> 2.0; 128 columns 64 rows 1.2 -> 1.4.  Plain 1280 columns 1100 rows 3.5 -> 2.5; 640 columns
+// 64 rows 1.6 -> 1.4, 1100 2.3 -> 2.1; 512 columns 296 rows 1.5 -> 1.4, 400 1.5 -> 1.6; 256 columns 1000 rows 1.5 -> 2.0.
+static int rmsnorm_block_rows(int d, bool modulated) {
+  if (d > 128 * MAX_CHUNKS || d < 256) return 0;
+  return d >= (modulated ? 384 : 640) ? CHIP_BLOCKS : CHIP_BLOCKS / 4;
+}
+
 template <typename T>
 static void launch_rmsnorm_fwd(const T* x, const float* col_scale, const float* col_bias, const float* w, float eps, int rows, int d,
                                T* xmod_out, __nv_bfloat16* z, float* rstd, cudaStream_t stream) {
-  // One round of blocks over the chip; past it a warp per row has as many loads in flight.  Measured (modulated, FP32; the
-  // kernels below -> here, us): 2048 columns 128 rows 4.3 -> 2.5, 300 4.4 -> 2.8, 1184 6.2 -> 5.2; 1280 columns 300 rows
-  // 5.6 -> 2.6, 1184 6.7 -> 4.0; 256 columns 2.2 -> 2.0.
-  if (rows <= CHIP_BLOCKS && d <= 128 * MAX_CHUNKS)
+  if (rows <= rmsnorm_block_rows(d, col_scale != nullptr))
     launch_dependent(rmsnorm_fwd_block_kernel<T>, dim3(rows), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, d,
                      xmod_out, z, rstd);
   else if (d <= 128 * MAX_CHUNKS)   // the general kernel reads its rows twice: 4096 rows of 384, 1024, 1920 columns 5.1, 10.7, 19.7 us, 3.6, 6.5, 12.2 so
