@@ -2,10 +2,15 @@
 gradient of the core final, also where several depths share the core (their norms' and logits' gradients would otherwise be
 added after it, to a bucket that is already being reduced)."""
 import gc
+import os
+import subprocess
+import sys
 import weakref
+from pathlib import Path
 
 import pytest
 import torch
+import torch.distributed as dist
 
 from warpstate_ai_b200 import WarpStateConfig, WarpStateLM
 from warpstate_ai_b200.ops import attention, fused, gemm
@@ -58,7 +63,7 @@ class Node(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, scale, bias, n1, n2, fast, slow, mix, main, hooked, core, notify):
-        ctx.main, ctx.hook = main, (hooked, core, notify)
+        ctx.main, ctx.hook, ctx.factor = main, (hooked, core, notify), float(x.flatten()[0])
         ctx.shapes = [None if t is None else t.shape for t in (scale, bias, n1, n2)] + [t.shape for t in (fast, slow, mix)]
         return x * 2.0
 
@@ -66,28 +71,70 @@ class Node(torch.autograd.Function):
     def backward(ctx, dy):
         for m in ctx.main:
             m += 1.0
-        scale, bias, n1, n2, fast, slow, mix = (None if s is None else torch.full(s, float(i + 1)) for i, s in enumerate(ctx.shapes))
+        scale, bias, n1, n2, fast, slow, mix = (None if s is None else torch.full(s, ctx.factor * (i + 1)) for i, s in enumerate(ctx.shapes))
         hooked, core, notify = ctx.hook
         if int(hooked) and fused._core_finished(core, notify, [n1, n2, fast, slow, mix]):
             n1 = n2 = fast = slow = mix = None
         return dy * 2.0, scale, bias, n1, n2, fast, slow, mix, None, None, None, None
 
 
-@pytest.mark.parametrize("cores,depth", [(1, 1), (2, 4), (2, 3)])
-def test_a_native_node_leaves_nothing_behind_the_hook(monkeypatch, cores, depth):
+def stand_ins(replace):
     def block(x, scale, bias, n1, n2, weights, bf16, main, fast, slow, mix, rope, eps, heads, flag, hooked, core, notify):
         return Node.apply(x, scale, bias, n1, n2, fast, slow, mix, main, hooked, core, notify)
-    monkeypatch.setattr(fused, "_native_block", lambda: block)
-    monkeypatch.setattr(attention, "kernels_ready", lambda core: True)
-    monkeypatch.setattr(gemm, "error_flag", lambda device: None)
+    replace(fused, "_native_block", lambda: block)
+    replace(attention, "kernels_ready", lambda core: True)
+    replace(gemm, "error_flag", lambda device: None)
+
+
+def blocks_forward(net, value=1.0):
+    x = torch.full((1, 128, 256), value)
+    for depth, (scale, bias) in enumerate(zip(net.depth_scale.unbind(0), net.depth_bias.unbind(0))):
+        x = fused.core_forward(net.cores[depth % len(net.cores)], x, scale, bias, notify=depth < len(net.cores))
+    return x
+
+
+@pytest.mark.parametrize("cores,depth", [(1, 1), (2, 4), (2, 3)])
+def test_a_native_node_leaves_nothing_behind_the_hook(monkeypatch, cores, depth):
+    stand_ins(monkeypatch.setattr)
     net = model("cpu", cores, depth)
     arena = ParamArena(net, bf16_mirror=True)
-    def forward():
-        x = torch.ones(1, 128, 256)
-        for d, (scale, bias) in enumerate(zip(net.depth_scale.unbind(0), net.depth_bias.unbind(0))):
-            x = fused.core_forward(net.cores[d % cores], x, scale, bias, notify=d < cores)
-        return x
-    check(forward, lambda y: y.sum().backward(), arena, list(net.cores), False)
+    check(lambda: blocks_forward(net), lambda y: y.sum().backward(), arena, list(net.cores), False)
+
+
+def worker(rank, world, folder):
+    """Gradients reduced from the hook on, against the average of every rank's own."""
+    from warpstate_ai_b200.parallel.grad_sync import CollectiveGradSync
+    dist.init_process_group("gloo", init_method=(folder / "rendezvous").as_uri(), rank=rank, world_size=world)
+    stand_ins(setattr)
+    net = model("cpu", 2, 4)
+    arena = ParamArena(net, bf16_mirror=True)
+    sync = CollectiveGradSync(torch.device("cpu"), world, rank)
+    sync.attach(arena, net)
+    blocks_forward(net, 1.0 + rank).sum().backward()
+    want = arena.grad.clone()
+    dist.all_reduce(want)
+    arena.zero_grad()
+    sync.begin_update()
+    y = blocks_forward(net, 1.0 + rank)
+    with sync.last_micro_batch():
+        y.sum().backward()
+        assert len(sync.reduced) == 2                       # both cores' buckets, ahead of the tail
+    sync.finish_update()
+    assert arena.grad.abs().sum() > 0 and torch.equal(arena.grad, want / world)
+    dist.destroy_process_group()
+
+
+def test_two_ranks_with_shared_cores_hold_the_average(tmp_path):
+    env = dict(os.environ, PYTHONPATH=str(Path(__file__).resolve().parents[1]) + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    ranks = [subprocess.Popen([sys.executable, __file__, str(rank), "2", str(tmp_path)], env=env, stdout=subprocess.PIPE,
+                              stderr=subprocess.STDOUT, text=True) for rank in range(2)]
+    try:
+        for rank in ranks:
+            out, _ = rank.communicate(timeout=240)
+            assert rank.returncode == 0, out[-3000:]
+    finally:
+        for rank in ranks:
+            rank.kill()
 
 
 @pytest.mark.gpu
@@ -137,3 +184,7 @@ def test_a_core_that_nobody_holds_any_more():
     fused.set_core_grad_hook(called.append)
     y.sum().backward()
     assert called == [] and norm.grad.abs().sum() > 0
+
+
+if __name__ == "__main__":
+    worker(int(sys.argv[1]), int(sys.argv[2]), Path(sys.argv[3]))
