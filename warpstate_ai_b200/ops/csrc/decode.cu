@@ -260,6 +260,7 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 //   partial != null: x += sum_s partial[s][b]     (split-K partials of the previous projection)
 //   scale != null : x = x * (1 + scale) + bias    (depth modulation of the layer that follows)
 // then out = BF16(x * rsqrt(mean(x^2) + eps) * w).
+// This form takes rows of more than 2048 columns; shorter ones, those of every configuration, take the one below.
 __global__ void __launch_bounds__(256)
 decode_reduce_norm_kernel(float* x, const float* partial, int splits,
                           const long long* token, const float* table, int vocab,
@@ -268,7 +269,7 @@ decode_reduce_norm_kernel(float* x, const float* partial, int splits,
   __shared__ float red[8];
   pdl_launch_dependents();
   const int b = blockIdx.x;
-  // Up to HELD * 1024 columns stay in registers between the two passes; what no kernel of the step writes (norm weight,
+  // The first HELD * 1024 columns stay in registers between the two passes; what no kernel of the step writes (norm weight,
   // modulation) is requested before the wait for the previous kernel.
   constexpr int HELD = 2;
   float4 held[HELD], ww[HELD], sc[HELD], bi[HELD];
