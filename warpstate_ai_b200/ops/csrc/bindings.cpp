@@ -1212,6 +1212,67 @@ void decode_reduce_norm(at::Tensor x, const c10::optional<at::Tensor>& partial, 
                                  (int)batch, op, cur_stream()), "decode_reduce_norm");
 }
 
+// One sequence: decode_reduce_norm and the decode_gemm that reads its result as one launch; x_out takes the residual that the former leaves in x.
+void decode_norm_gemm(const at::Tensor& x, const c10::optional<at::Tensor>& x_out, const c10::optional<at::Tensor>& partial,
+                      const c10::optional<at::Tensor>& token, const c10::optional<at::Tensor>& table, const c10::optional<at::Tensor>& scale,
+                      const c10::optional<at::Tensor>& bias, const at::Tensor& norm, double eps, const at::Tensor& w, int64_t n,
+                      int64_t epilogue, at::Tensor out, const c10::optional<at::Tensor>& error_flag, bool packed) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 2 && x.is_contiguous(), "decode_norm_gemm: x must be contiguous FP32 [1, d]");
+  const int64_t d = x.size(1);
+  TORCH_CHECK(x.size(0) == 1 && d % 64 == 0 && d >= 64 && d <= 2048, "decode_norm_gemm: one sequence, d a multiple of 64 up to 2048");
+  const auto vector = [&](const at::Tensor& t, const char* what) {
+    TORCH_CHECK(t.device() == x.device() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel() == d &&
+                reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, what);
+    return t.data_ptr<float>();
+  };
+  const float* nw = vector(norm, "decode_norm_gemm: norm must be FP32 [d]");
+  const bool mod = scale.has_value() && scale->defined();
+  TORCH_CHECK(mod == (bias.has_value() && bias->defined()), "decode_norm_gemm: modulation needs scale and bias");
+  const float* sc = mod ? vector(*scale, "decode_norm_gemm: scale must be FP32 [d]") : nullptr;
+  const float* bi = mod ? vector(*bias, "decode_norm_gemm: bias must be FP32 [d]") : nullptr;
+  float* xo = nullptr;
+  if (x_out.has_value() && x_out->defined()) {
+    TORCH_CHECK(x_out->device() == x.device() && x_out->scalar_type() == at::kFloat && x_out->is_contiguous() && x_out->sizes() == x.sizes() &&
+                x_out->data_ptr() != x.data_ptr(), "decode_norm_gemm: x_out must be a buffer of its own like x");
+    xo = x_out->data_ptr<float>();
+  }
+  int splits = 0;
+  const float* pp = nullptr;
+  if (partial.has_value() && partial->defined()) {
+    TORCH_CHECK(partial->device() == x.device() && partial->scalar_type() == at::kFloat && partial->is_contiguous() &&
+                partial->numel() % d == 0, "decode_norm_gemm: partial must be FP32 [splits, 1, d]");
+    splits = (int)(partial->numel() / d);
+    pp = partial->data_ptr<float>();
+  }
+  const long long* tok = nullptr;
+  const float* tab = nullptr;
+  int vocab = 0;
+  if (token.has_value() && token->defined()) {
+    TORCH_CHECK(table.has_value() && token->device() == x.device() && token->scalar_type() == at::kLong && token->numel() == 1 &&
+                token->is_contiguous() && table->device() == x.device() && table->scalar_type() == at::kFloat && table->is_contiguous() &&
+                table->dim() == 2 && table->size(1) == d && splits == 0,
+                "decode_norm_gemm: token [1] int64 with an FP32 table [vocab, d], and no partials");
+    tok = reinterpret_cast<const long long*>(token->data_ptr<int64_t>());
+    tab = table->data_ptr<float>();
+    vocab = (int)table->size(0);
+  }
+  TORCH_CHECK(epilogue == 0 || epilogue == 2 || epilogue == 3, "decode_norm_gemm: epilogue 0, 2 or 3");
+  TORCH_CHECK(w.device() == x.device() && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && n > 0 &&
+              reinterpret_cast<uintptr_t>(w.data_ptr()) % 16 == 0, "decode_norm_gemm: contiguous BF16 W");
+  if (packed) {
+    TORCH_CHECK(w.dim() == 4 && w.size(0) == (epilogue == 2 ? n / 64 : (n + 127) / 128) && w.size(1) == d / 64 && w.size(2) == 128 && w.size(3) == 64,
+                "decode_norm_gemm: a packed W must be [slabs, d / 64, 128, 64]");
+  } else {
+    TORCH_CHECK(w.dim() == 2 && w.size(1) == d && w.size(0) == (epilogue == 2 ? 2 * n : n), "decode_norm_gemm: W must be [rows, d] with rows matching n");
+  }
+  TORCH_CHECK(out.device() == x.device() && out.is_contiguous() && out.scalar_type() == (epilogue == 3 ? at::kFloat : at::kBFloat16) &&
+              out.dim() == 2 && out.size(0) == 1 && out.size(1) == n, "decode_norm_gemm: out must be [1, n] of the epilogue's dtype");
+  c10::cuda::CUDAGuard guard(x.device());
+  check_rc(ws_decode_norm_gemm(x.data_ptr<float>(), xo, pp, splits, tok, tab, vocab, sc, bi, nw, (float)eps, w.data_ptr(), (int)n, (int)d,
+                               (int)epilogue, out.data_ptr(), (int)n, reinterpret_cast<int*>(const_cast<void*>(opt_ptr(error_flag))),
+                               packed ? 1 : 0, cur_stream()), "decode_norm_gemm");
+}
+
 void decode_attn(const at::Tensor& qkvgu, at::Tensor kc, at::Tensor vc, at::Tensor uc, const at::Tensor& mixed,
                  const at::Tensor& rope, const at::Tensor& pos, int64_t H, at::Tensor y, bool early) {
   TORCH_CHECK(qkvgu.is_cuda() && qkvgu.scalar_type() == at::kBFloat16 && qkvgu.dim() == 2 && qkvgu.is_contiguous(),
@@ -1342,6 +1403,8 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("decode_gemm(Tensor w, Tensor x, int n, int epilogue, Tensor(a!) out, Tensor(b!)? error_flag, bool packed=False) -> ()");
   m.def("decode_reduce_norm(Tensor(a!) x, Tensor? partial, Tensor? token, Tensor? table, Tensor? scale, Tensor? bias, "
         "Tensor w, float eps, Tensor(b!)? out) -> ()");
+  m.def("decode_norm_gemm(Tensor x, Tensor(a!)? x_out, Tensor? partial, Tensor? token, Tensor? table, Tensor? scale, Tensor? bias, "
+        "Tensor norm, float eps, Tensor w, int n, int epilogue, Tensor(b!) out, Tensor(c!)? error_flag, bool packed=False) -> ()");
   m.def("decode_layer_tail(Tensor w_out, Tensor w_ug, Tensor w_down, Tensor? w_in_next, Tensor y, Tensor(a!) x, "
         "Tensor(b!) part_out, Tensor(c!) part_down, Tensor(d!) n, Tensor(e!) act, Tensor(f!) qkvgu, Tensor w_norm2, "
         "Tensor? next_scale, Tensor? next_bias, Tensor w_norm_next, float eps, Tensor(g!) barrier, Tensor(h!)? error_flag, "
@@ -1432,6 +1495,7 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("decode_gemm", &decode_gemm);
   m.impl("gather_cast_linear", &gather_cast_linear);
   m.impl("decode_reduce_norm", &decode_reduce_norm);
+  m.impl("decode_norm_gemm", &decode_norm_gemm);
   m.impl("decode_attn", &decode_attn);
   m.impl("decode_chunk_end", &decode_chunk_end);
   m.impl("decode_pick", &decode_pick);

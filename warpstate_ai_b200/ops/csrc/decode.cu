@@ -18,7 +18,9 @@
 //                          append k/v/u to the chunk cache, causal attention over the cache rows
 //                          <= position, memory read q.M, gate blend.
 //
-// The ~200 launches of a step form one chain of programmatic dependent launches: every kernel lets
+//   decode_norm_gemm_kernel    the two together, for one sequence.
+//
+// The 140 to 200 launches of a step form one chain of programmatic dependent launches: every kernel lets
 // its successor start at once, and a GEMM fills its whole TMA ring with weight tiles (which no
 // kernel of the step writes) before it waits for its predecessor, so the weight stream of the
 // next projection runs under the small kernels and the tail of the previous GEMM.
@@ -73,6 +75,69 @@ struct DecodeCfg {
 };
 
 // EPI: 0 = BF16 out, 1 = FP32 split-K partial, 2 = SwiGLU (BF16 activation), 3 = FP32 out
+// Epilogue of one slab (128 weight rows from n0, or 64 up rows and their gate rows) by the four warps whose TMEM quarters it is.
+template <int BPAD, int EPI>
+__device__ __forceinline__ void decode_epilogue(const DecodeGemmParams& p, uint32_t tmem, int warp, int lane, int n0, float* sG, bool ok) {
+  const int quarter = warp & 3;  // TMEM lane quarter this warp may read
+  const int row = quarter * 32 + lane;
+  tc_fence_after_sync();
+  const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
+  if (EPI == 2) {
+    // rows 0..63 = up, 64..127 = gate: the gate warps hand silu-ready values over through smem
+    if (row >= 64 && ok) {
+#pragma unroll
+      for (int c0 = 0; c0 < BPAD; c0 += 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(taddr + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const float g = __uint_as_float(r[j]);
+          sG[(c0 + j) * 64 + (row - 64)] = g * sigmoid_fast(g);
+        }
+      }
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (row < 64 && ok) {
+      const int hcol = n0 + row;
+      __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
+#pragma unroll
+      for (int c0 = 0; c0 < BPAD; c0 += 16) {
+        uint32_t r[16];
+        tmem_ld_32x32b_x16(taddr + c0, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          const int b = c0 + j;
+          if (b < p.batch && hcol < p.n)
+            out[static_cast<size_t>(b) * p.ldo + hcol] = __float2bfloat16(__uint_as_float(r[j]) * sG[b * 64 + row]);
+        }
+      }
+    }
+  } else if (ok) {
+    const int n = n0 + row;
+#pragma unroll
+    for (int c0 = 0; c0 < BPAD; c0 += 16) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(taddr + c0, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const int b = c0 + j;
+        if (b >= p.batch || n >= p.n) continue;
+        const float v = __uint_as_float(r[j]);
+        if (EPI == 0) {
+          static_cast<__nv_bfloat16*>(p.out)[static_cast<size_t>(b) * p.ldo + n] = __float2bfloat16(v);
+        } else if (EPI == 3) {
+          static_cast<float*>(p.out)[static_cast<size_t>(b) * p.ldo + n] = v;
+        } else {
+          static_cast<float*>(p.out)[(static_cast<size_t>(blockIdx.y) * p.batch + b) * p.n + n] = v;
+        }
+      }
+    }
+  }
+}
+
 template <int BPAD, int EPI, int DEPTH>
 __global__ void __launch_bounds__(dec::THREADS, DecodeCfg<BPAD, DEPTH>::CTAS_PER_SM)
 decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
@@ -185,65 +250,8 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
       if (ok) umma_commit(tfull);
     }
   } else {
-    const int quarter = warp & 3;  // TMEM lane quarter this warp may read
-    const int row = quarter * 32 + lane;
     const bool ok = kb1 > kb0 && mbar_wait_warp(tfull, 0, abort_flag);
-    tc_fence_after_sync();
-    const uint32_t taddr = tmem + (static_cast<uint32_t>(quarter * 32) << 16);
-    if (EPI == 2) {
-      // rows 0..63 = up, 64..127 = gate: the gate warps hand silu-ready values over through smem
-      if (row >= 64 && ok) {
-#pragma unroll
-        for (int c0 = 0; c0 < BPAD; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(taddr + c0, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const float g = __uint_as_float(r[j]);
-            sG[(c0 + j) * 64 + (row - 64)] = g * sigmoid_fast(g);
-          }
-        }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (row < 64 && ok) {
-        const int hcol = n0 + row;
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
-#pragma unroll
-        for (int c0 = 0; c0 < BPAD; c0 += 16) {
-          uint32_t r[16];
-          tmem_ld_32x32b_x16(taddr + c0, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int b = c0 + j;
-            if (b < p.batch && hcol < p.n)
-              out[static_cast<size_t>(b) * p.ldo + hcol] = __float2bfloat16(__uint_as_float(r[j]) * sG[b * 64 + row]);
-          }
-        }
-      }
-    } else if (ok) {
-      const int n = n0 + row;
-#pragma unroll
-      for (int c0 = 0; c0 < BPAD; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld_32x32b_x16(taddr + c0, r);
-        tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int b = c0 + j;
-          if (b >= p.batch || n >= p.n) continue;
-          const float v = __uint_as_float(r[j]);
-          if (EPI == 0) {
-            static_cast<__nv_bfloat16*>(p.out)[static_cast<size_t>(b) * p.ldo + n] = __float2bfloat16(v);
-          } else if (EPI == 3) {
-            static_cast<float*>(p.out)[static_cast<size_t>(b) * p.ldo + n] = v;
-          } else {
-            static_cast<float*>(p.out)[(static_cast<size_t>(blockIdx.y) * p.batch + b) * p.n + n] = v;
-          }
-        }
-      }
-    }
+    decode_epilogue<BPAD, EPI>(p, tmem, warp, lane, n0, sG, ok);
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -404,6 +412,188 @@ decode_reduce_norm_short_kernel(float* x, const float* partial, int splits, cons
   if (mine)
     *reinterpret_cast<uint2*>(out + static_cast<size_t>(b) * d + c) =
         make_uint2(pack_bf16x2(v.x * rstd * ww.x, v.y * rstd * ww.y), pack_bf16x2(v.z * rstd * ww.z, v.w * rstd * ww.w));
+}
+
+// --------------------------------------------------------------------------- residual + norm + projection
+// One sequence: the two kernels above in front of the projection that reads their result, in its launch.  Every CTA adds the
+// partials and forms the norm itself, as its MMAs' operand, and CTA 0 leaves the residual for the next such launch (in another
+// buffer: the others may still be reading).  A boundary of the chain and a round trip through memory less, twice a layer,
+// against reading (1 + splits) rows of x per CTA from L2.  Bit for bit what the two launches give: same order of partials, squares
+// and k blocks.  d <= 2048.  A step of 28 layers of width 2048 1018 -> 940 us, of 16 of 1280 416 -> 375, of 8 of 256 122 -> 112.  With more sequences
+// those reads take longer than the boundary did: two 1023 -> 1065 and 418 -> 442, eight 1056 -> 1654.  Rings of four to six stages, with
+// which a CTA would fit beside its predecessor's: 1064-1153.
+struct DecodeNormParams {
+  const float* x;         // residual before, [d]; behind a token its embedding row instead
+  float* x_out;           // and after
+  const float* partial;   // [splits, d]
+  int splits;
+  const long long* token;
+  const float* table;
+  int vocab;
+  const float *scale, *bias, *w;
+  float eps;
+};
+constexpr int NORM_WORKERS = 512;                 // of four columns each
+constexpr int NORM_THREADS = 64 + NORM_WORKERS;   // warp 0 TMA, warp 1 MMA + TMEM, warps 2..17 the norm, 2..5 of them the epilogue
+constexpr int NORM_STAGES = 8;
+constexpr int NORM_ROUND = 12;                    // partials of a thread requested at once
+
+// The MMA's operand has 16 rows, of which the sequence is the first: eight rows of 128 bytes per k block, taken twice.
+static int norm_gemm_smem(int d) { return NORM_STAGES * dec::W_BYTES + d / dec::BK * 1024 + 1024 + 256; }
+
+template <int EPI>
+__global__ void __launch_bounds__(NORM_THREADS, 1)
+decode_norm_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const DecodeGemmParams p, const DecodeNormParams q) {
+  using namespace dec;
+  constexpr int BPAD = 16;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  __shared__ float upper[256], red[8];
+  const int total_kb = p.k / BK;
+  uint8_t* sW = smem;
+  uint8_t* sX = smem + NORM_STAGES * W_BYTES;    // [k block][8 rows][64 columns]; the columns of D that rows 1.. give are not read
+  float* sG = reinterpret_cast<float*>(sW);      // written only after the last MMA has read the ring
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sX + total_kb * 1024);
+  uint64_t* full = bars;
+  uint64_t* empty = bars + NORM_STAGES;
+  uint64_t* tfull = bars + 2 * NORM_STAGES;
+  uint64_t* ready = tfull + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ready + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NORM_STAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(tfull, 1);
+    mbar_init(ready, NORM_WORKERS / 32);
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tm_w);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 32);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+  pdl_launch_dependents();
+
+  const int slab = blockIdx.x, n0 = slab * (EPI == 2 ? 64 : TM);
+  const int rot = static_cast<int>((blockIdx.x * 5u) % static_cast<unsigned>(total_kb));   // as decode_gemm_kernel walks them
+  auto block_of = [&](int it) {
+    const int r = it + rot;
+    return r >= total_kb ? r - total_kb : r;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      // Weights only, which no kernel of the step writes: as far ahead as the ring goes, whatever the predecessor does.
+      for (int it = 0; it < total_kb; ++it) {
+        const int s = it % NORM_STAGES, kb = block_of(it);
+        if (!mbar_wait(&empty[s], ((it / NORM_STAGES) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(&full[s], W_BYTES);
+        if (p.packed) {
+          tma_load_2d(sW + s * W_BYTES, &tm_w, &full[s], 0, (slab * total_kb + kb) * TM);
+        } else {
+          tma_load_2d(sW + s * W_BYTES, &tm_w, &full[s], kb * BK, n0);
+          if (EPI == 2) tma_load_2d(sW + s * W_BYTES + 64 * 128, &tm_w, &full[s], kb * BK, p.n + n0);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (elect_one()) {
+      constexpr uint32_t idesc = make_idesc_bf16(TM, BPAD, false, false);
+      const uint32_t a0 = desc_low_sw128(smem_u32(sW)), b0 = desc_low_sw128(smem_u32(sX));
+      bool ok = mbar_wait(ready, 0, abort_flag);
+      int s = 0;
+      uint32_t ph = 0;
+      for (int it = 0; it < total_kb && ok; ++it) {
+        ok = mbar_wait(&full[s], ph, abort_flag);
+        if (!ok) break;
+        tc_fence_after_sync();
+        const uint32_t a = a0 + s * (W_BYTES / 16), b = b0 + block_of(it) * (1024 / 16);
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k) umma_bf16_low<0>(tmem, a + 2 * k, b + 2 * k, idesc, (it | k) != 0 ? 1u : 0u);
+        umma_commit(&empty[s]);
+        if (++s == NORM_STAGES) {
+          s = 0;
+          ph ^= 1;
+        }
+      }
+      if (ok) umma_commit(tfull);
+    }
+  } else {
+    const int worker = threadIdx.x - 64, c = worker * 4;
+    float4 weight = make_float4(0.f, 0.f, 0.f, 0.f), scale = weight, bias = weight;
+    if (c < p.k) {   // what no kernel of the step writes is requested before the wait
+      weight = *reinterpret_cast<const float4*>(q.w + c);
+      if (q.scale != nullptr) {
+        scale = *reinterpret_cast<const float4*>(q.scale + c);
+        bias = *reinterpret_cast<const float4*>(q.bias + c);
+      }
+    }
+    pdl_wait();
+    const bool mine = c < p.k;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (mine) {
+      const float* src = q.x;
+      if (q.token != nullptr) {
+        long long id = *q.token;
+        if (id < 0) id = 0;
+        if (id >= q.vocab) id = q.vocab - 1;
+        src = q.table + static_cast<size_t>(id) * p.k;
+      }
+      v = *reinterpret_cast<const float4*>(src + c);
+      for (int s0 = 0; s0 < q.splits; s0 += NORM_ROUND) {
+        float4 part[NORM_ROUND];
+#pragma unroll
+        for (int s = 0; s < NORM_ROUND; ++s)
+          if (s0 + s < q.splits) part[s] = *reinterpret_cast<const float4*>(q.partial + static_cast<size_t>(s0 + s) * p.k + c);
+#pragma unroll
+        for (int s = 0; s < NORM_ROUND; ++s)
+          if (s0 + s < q.splits) { v.x += part[s].x; v.y += part[s].y; v.z += part[s].z; v.w += part[s].w; }
+      }
+      if (q.scale != nullptr) v = modulated(v, scale, bias);
+      if (blockIdx.x == 0 && q.x_out != nullptr) *reinterpret_cast<float4*>(q.x_out + c) = v;
+    }
+    const float square = square_sum(v);   // added as decode_reduce_norm_short_kernel adds them
+    if (worker >= 256) upper[worker - 256] = square;
+    asm volatile("bar.sync 2, 512;" ::: "memory");
+    if (worker < 256) {
+      float ss = __fadd_rn(square, upper[worker]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      if (lane == 0) red[worker >> 5] = ss;
+    }
+    asm volatile("bar.sync 2, 512;" ::: "memory");
+    if (mine) {
+      float total = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) total += red[i];
+      const float rstd = rsqrtf(total / static_cast<float>(p.k) + q.eps);
+      *reinterpret_cast<uint2*>(sX + (c >> 6) * 1024 + (c & 63) * 2) =
+          make_uint2(pack_bf16x2(v.x * rstd * weight.x, v.y * rstd * weight.y), pack_bf16x2(v.z * rstd * weight.z, v.w * rstd * weight.w));
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(ready);
+    if (warp < 6) {
+      const bool ok = mbar_wait_warp(tfull, 0, abort_flag);
+      decode_epilogue<BPAD, EPI>(p, tmem, warp, lane, n0, sG, ok);
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && p.error_flag != nullptr) atomicExch(p.error_flag, 8);
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 32);
+  }
 }
 
 // --------------------------------------------------------------------------- attention step
@@ -892,6 +1082,19 @@ static int decode_ring_depth() {
   return depth;
 }
 
+template <int EPI>
+static int launch_norm_gemm(const CUtensorMap& tw, const DecodeGemmParams& p, const DecodeNormParams& q, int slabs, cudaStream_t stream) {
+  static bool configured = false;
+  auto kern = decode_norm_gemm_kernel<EPI>;
+  if (!configured) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, norm_gemm_smem(2048)) != cudaSuccess) return -20;
+    configured = true;
+  }
+  const cudaError_t err = launch_chained(kern, dim3(slabs), dim3(NORM_THREADS), norm_gemm_smem(p.k), stream, tw, p, q);
+  ws_count_launch();
+  return err == cudaSuccess ? 0 : -21;
+}
+
 template <int BPAD, int EPI>
 static int launch_decode_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const DecodeGemmParams& p, dim3 grid,
                               cudaStream_t stream) {
@@ -980,6 +1183,31 @@ extern "C" int ws_decode_reduce_norm(float* x, const float* partial, int splits,
                                          static_cast<__nv_bfloat16*>(out));
   ws_count_launch();
   return err == cudaSuccess ? 0 : -21;
+}
+
+extern "C" int ws_decode_norm_gemm(const float* x, float* x_out, const float* partial, int splits, const long long* token,
+                                   const float* table, int vocab, const float* scale, const float* bias, const float* norm, float eps,
+                                   const void* w, int n, int d, int epilogue, void* out, int ldo, int* error_flag, int packed,
+                                   cudaStream_t stream) {
+  if (d < dec::BK || d > 4 * NORM_WORKERS || d % dec::BK != 0 || n <= 0 || splits < 0 ||
+      (epilogue != 0 && epilogue != 2 && epilogue != 3) || (splits > 0 && partial == nullptr) || x_out == x)
+    return -1;
+  if (epilogue == 2 && n % 64 != 0) return -2;
+  const int slabs = epilogue == 2 ? n / 64 : (n + dec::TM - 1) / dec::TM;
+  CUtensorMap tw;
+  const int rc = packed ? make_map_bf16(&tw, w, dec::BK, (uint64_t)slabs * (d / dec::BK) * dec::TM, dec::BK, dec::BK, dec::TM)
+                        : make_map_bf16(&tw, w, d, epilogue == 2 ? 2 * n : n, d, dec::BK, epilogue == 2 ? 64 : dec::TM);
+  if (rc) return rc;
+  DecodeGemmParams p;
+  p.n = n; p.k = d; p.batch = 1; p.kb_per_split = d / dec::BK; p.packed = packed; p.out = out; p.ldo = ldo; p.error_flag = error_flag;
+  DecodeNormParams q;
+  q.x = x; q.x_out = x_out; q.partial = partial; q.splits = splits; q.token = token; q.table = table; q.vocab = vocab;
+  q.scale = scale; q.bias = bias; q.w = norm; q.eps = eps;
+  switch (epilogue) {
+    case 0: return launch_norm_gemm<0>(tw, p, q, slabs, stream);
+    case 2: return launch_norm_gemm<2>(tw, p, q, slabs, stream);
+    default: return launch_norm_gemm<3>(tw, p, q, slabs, stream);
+  }
 }
 
 extern "C" int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, const void* mixed, const float* rope,

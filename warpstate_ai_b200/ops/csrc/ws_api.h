@@ -100,6 +100,11 @@ int ws_decode_gemm(const void* w, const void* x, int n, int k, int batch, int ep
 int ws_decode_reduce_norm(float* x, const float* partial, int splits, const long long* token, const float* table,
                           int vocab, const float* scale, const float* bias, const float* w, float eps, int d,
                           int batch, void* out, cudaStream_t stream);
+// ws_decode_reduce_norm and the ws_decode_gemm behind it (epilogue 0, 2 or 3, k = d) as one launch, for one sequence and d <= 2048: x_out
+// (FP32 [d], not x; NULL: not kept) = (table[token] or x + partials), modulated; out = epilogue(RMSNorm(x_out) . w^T).
+int ws_decode_norm_gemm(const float* x, float* x_out, const float* partial, int splits, const long long* token, const float* table,
+                        int vocab, const float* scale, const float* bias, const float* norm, float eps, const void* w, int n, int d,
+                        int epilogue, void* out, int ldo, int* error_flag, int packed, cudaStream_t stream);
 // One decode step of the attention block for every (sequence, head); see decode_attn_kernel.  `early` reads pos, the cache
 // rows before it and mixed ahead of the launches in front of this one: only in a captured step, whose replay starts
 // after everything that wrote them.

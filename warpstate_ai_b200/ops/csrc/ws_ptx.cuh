@@ -231,20 +231,22 @@ __device__ __forceinline__ bool elect_one() {
   return e != 0;
 }
 // Low half of a K-major descriptor with the 128-byte swizzle and 1024 bytes between 8-row groups (leading offset 0); the
-// other half is a constant.  A step of 32 bytes along k, or of a whole tile, is an addition.
+// other half is a constant.  A step of 32 bytes along k, or of a whole tile, is an addition.  B_STRIDE: the bytes between B's 8-row
+// groups; with 0 its rows 8.. are rows 0..7 again (an operand of at most eight rows, whose other columns of D nobody reads).
 __device__ __forceinline__ uint32_t desc_low_sw128(uint32_t smem_addr) { return (smem_addr & 0x3FFFFu) >> 4; }
+template <uint32_t B_STRIDE = 1024>
 __device__ __forceinline__ void umma_bf16_low(uint32_t tmem_d, uint32_t a_low, uint32_t b_low, uint32_t idesc, uint32_t accumulate) {
-  constexpr uint32_t kHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+  constexpr uint32_t kRest = (1u << 14) | (2u << 29), kHigh = (1024u >> 4) | kRest, kHighB = (B_STRIDE >> 4) | kRest;
   asm volatile(
       "{\n"
       ".reg .pred p;\n"
       ".reg .b64 a, b;\n"
       "mov.b64 a, {%1, %5};\n"
-      "mov.b64 b, {%2, %5};\n"
+      "mov.b64 b, {%2, %6};\n"
       "setp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %3, p;\n"
       "}\n" ::"r"(tmem_d),
-      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kHigh)
+      "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kHigh), "n"(kHighB)
       : "memory");
 }
 // A operand taken from TMEM (used by the attention kernels for P*V and dS*K products).

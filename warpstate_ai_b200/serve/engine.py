@@ -21,7 +21,8 @@ What is new relative to the reference (whose CLIs prefill token by token at batc
 * on CUDA with the kernel library (BF16, head_dim 64, chunk 128, batch <= 64) the step is seven
   kernels per layer: weight-streaming tcgen05 GEMMs with swapped operand roles
   (`decode_gemm_kernel`), a fused residual + depth-modulation + RMSNorm kernel and one attention
-  kernel per (sequence, head) (ops/csrc/decode.cu); the PyTorch formulation below is the
+  kernel per (sequence, head) (ops/csrc/decode.cu); for one sequence five, the residual sums and norms in the
+  launches of the projections that read them; the PyTorch formulation below is the
   reference for it and the fallback elsewhere.
 """
 from __future__ import annotations
@@ -63,6 +64,7 @@ class DecodeEngine:
         self.pack_weights = pack_weights
         self._kbufs = None
         self._layer_tail = False
+        self._norm_in_gemm = False
         self.weights = []
         with torch.no_grad():
             for depth in range(self.cfg.logical_depth):
@@ -124,6 +126,7 @@ class DecodeEngine:
         self._graph = self._greedy_graph = None
         self._kbufs = self._kernel_buffers(batch) if self._kernels_usable(batch) else None
         self._layer_tail = self._kbufs is not None and self._tail_kernel_usable()
+        self._norm_in_gemm = self._kbufs is not None and self._norm_gemm_usable(batch)
         # greedy run-ahead decode: chosen tokens land in `history[:, cursor[0]]`; cursor[1] is kernel scratch
         self.history = torch.zeros(batch, self.GREEDY_CAPACITY, dtype=torch.long, device=self.device)
         self.cursor = torch.zeros(2, dtype=torch.long, device=self.device)
@@ -170,7 +173,7 @@ class DecodeEngine:
         from ..ops import attention, gemm
         self._pack_weights()
         return dict(
-            x=torch.zeros(batch, d, device=dev), n=torch.zeros(batch, d, device=dev, dtype=torch.bfloat16),
+            x=torch.zeros(batch, d, device=dev), x_other=torch.zeros(batch, d, device=dev), n=torch.zeros(batch, d, device=dev, dtype=torch.bfloat16),
             qkvgu=torch.zeros(batch, 5 * d, device=dev, dtype=torch.bfloat16),
             y=torch.zeros(batch, d, device=dev, dtype=torch.bfloat16),
             act=torch.zeros(batch, ffn, device=dev, dtype=torch.bfloat16),
@@ -197,6 +200,29 @@ class DecodeEngine:
                     (5 * d + 127) // 128, self.batch)
         return items <= torch.cuda.get_device_properties(self.device).multi_processor_count
 
+    def _norm_gemm_usable(self, batch: int) -> bool:
+        """One sequence: the residual sums and norms are formed in the launches of the projections that read them, whose CTAs hold at most
+        2048 columns; with more sequences that takes longer than the launches it saves (decode.cu)."""
+        return batch == 1 and self.cfg.d_model <= 2048
+
+    def _step_kernels_single(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool) -> torch.Tensor:
+        """The step of one sequence, five launches per layer instead of seven.  Bit-identical to `_step_kernels`."""
+        ops = torch.ops.ws_b200
+        k, packed = self._kbufs, self.pack_weights
+        d, ffn, eps = self.cfg.d_model, self.cfg.ffn_hidden, self.cfg.rms_eps
+        x, other = k["x"], k["x_other"]
+        for index, (w, st) in enumerate(zip(self.weights, self.states)):
+            partial, ids, table = (k["p_down"], None, None) if index else (None, token, self.embed)
+            ops.decode_norm_gemm(x, other, partial, ids, table, w["scale"], w["bias"], w["n1"], eps, w["p_in"], 5 * d, 0, k["qkvgu"],
+                                 k["flag"], packed)
+            ops.decode_attn(k["qkvgu"], st.k, st.v, st.u, st.mixed, k["rope"], pos, self.h, k["y"], replayed)
+            ops.decode_gemm(w["p_out"], k["y"], d, 1, k["p_out"], k["flag"], packed)
+            ops.decode_norm_gemm(other, x, k["p_out"], None, None, None, None, w["n2"], eps, w["p_ug"], ffn, 2, k["act"], k["flag"], packed)
+            ops.decode_gemm(w["p_down"], k["act"], d, 1, k["p_down"], k["flag"], packed)
+        ops.decode_norm_gemm(x, None, k["p_down"], None, None, None, None, self.final_norm, eps, self.head_packed, self.cfg.vocab_size, 3,
+                             k["logits"], k["flag"], packed)
+        return k["logits"]
+
     def _step_kernels_tail(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool) -> torch.Tensor:
         """The step with one persistent launch per layer for everything after the attention (and the next layer's
         in_proj): 2 launches per layer instead of 7.  Bit-identical to `_step_kernels`."""
@@ -219,6 +245,8 @@ class DecodeEngine:
     def _step_kernels(self, token: torch.Tensor, pos: torch.Tensor, replayed: bool) -> torch.Tensor:
         if self._layer_tail:
             return self._step_kernels_tail(token, pos, replayed)
+        if self._norm_in_gemm:
+            return self._step_kernels_single(token, pos, replayed)
         ops = torch.ops.ws_b200
         k = self._kbufs
         d, ffn, eps = self.cfg.d_model, self.cfg.ffn_hidden, self.cfg.rms_eps
