@@ -453,58 +453,91 @@ memory_logit_grads_kernel(const float* partials, const float* fast_logit,
 }
 
 // =============================================================================== attention bwd
-// One CTA of 256 threads per (batch, chunk, head) tile; threads t and t + 128 own row t of the chunk, one half of its
-// columns each (of the 128 score columns, every other block of 32, so that the causal triangle is halved too).
-// The kernel is a chain of four MMA phases with element-wise work between them, so a single
+// Two persistent CTAs of 256 threads per SM walk the (batch, chunk, head) tiles; threads t and t + 128 own row t of the chunk, one
+// half of its columns each (of the 128 score columns, every other block of 32, so that the causal triangle is halved too).
+// The kernel is a chain of MMA phases with element-wise work between them, so a single
 // tile cannot keep an SM busy; what matters is how many tiles an SM holds at once, and how long the element-wise
 // stretches of the chain are.  Shared memory is therefore kept to 112 KiB and TMEM to 256 columns, so that TWO CTAs fit
 // per SM, and a row is shared by two threads, which exchange its softmax statistics and its D through shared memory.
-// 2048 tiles (4 x 2048 tokens, 32 heads): 169.6 us with one thread per row, 131.8 with two (128 registers, no spills);
-// DRAM 33 % busy, 24 % of the warps: what is left is the latency of the chain.
 //
-//   smem: B0 Qr | B1 Kr | B2 dy -> dlocal -> tanh(U) | B3 dmem/8 -> V -> tanh(Kr) | sP (32K: P -> dS)
-//         | sSt (8K) | sDW (8K) | barriers
+// With a CTA per tile a third of its 30.7 k clocks went before and after the chain: 1.2 k of set-up, 5.4 k until the operands
+// had landed, 2.8 k until its stores had read shared memory.  A CTA that goes on to its next tile requests Q and K of that one
+// as soon as the last products have read dS, whose buffer they take, and everything else once the stores have drained, behind
+// the rotation of Q and K.  The six tile buffers trade places for that, in pairs, from tile to tile.  Element-wise work that
+// does not need a product's result runs under it: dmem under S, dlocal and dlocal (1 - g) under O, the tanhs and dV under dQ and dK.
+// 2048 tiles (4 x 2048 tokens, 32 heads): 122.9 us with a CTA per tile, 107.8 so; 280 tiles (one round) 16.7 and 16.6.  What
+// bounds it now is the load and store pipe, which tile traffic, tensor-core operands and TMA share: the gate row read by
+// each thread from global memory (16 bytes of 32 rows to an instruction) 117, registers spilled for 0.1 KB 118, four threads to a row 137.
+//
+//   smem, three pairs of 16 KiB tiles: A = Qr, Kr | B = dy -> dlocal -> tanh(U), V -> tanh(Kr) | P = gate, dmem/8 -> P -> dS -> next A
+//         | sSt (8K) | sDW (8K) | barriers.  Gradients leave from where their last operand was: dQ, dK from A, dU, dGate from B,
+//         dV from sSt and sDW.  Next tile: A <- P, B <- A, P <- B.
 //   TMEM: [0,128) S -> O (first 64) -> dP -> dKr (first 64) + dtK (last 64)
 //         [128,192) Mem -> dV -> dtU        [192,256) dQr (memory part, later += attention part)
 //
-// V and U are fetched late (into buffers that earlier operands have left), each behind work that
-// hides most of the load latency.  P is stored normalised, so O and dV need no row scaling.
+// U is fetched late (into the buffer that dlocal has left), behind the dS phase.  P is stored normalised, so O and dV need no
+// row scaling.
 constexpr int AB_THREADS = 256;
 constexpr int AB_PIECES = 4;   // 16-byte pieces of a 64-column row that a thread owns
 // No alignment slack: 2 x (114816 + 1024 reserved) = 231680 <= 233472 bytes of an SM.  The dynamic
 // segment is declared 1024-byte aligned (the 128-byte swizzle needs it); the kernel checks.
 constexpr int AB_SMEM = 4 * TILE_BYTES + 2 * TILE_BYTES + 2 * 8192 + 128;
 
+// The buffers trade places, so a thread reaches them by 32-bit shared addresses: `at` = its tile + where its four pieces of its row
+// begin, piece j of them at `at` ^ 16 j (the swizzle is an exclusive or of the bits that count the pieces).
+__device__ __forceinline__ uint4& ab_piece(uint32_t at, int j) {
+  return *static_cast<uint4*>(__cvta_shared_to_generic(at ^ (j << 4)));
+}
+// Rotary embedding of the thread's pieces of a Q and a K row, in place (as rope_tanh_row in attention_common.cuh).
+__device__ __forceinline__ void ab_rope(uint32_t q_at, uint32_t k_at, int row, int piece0, const float2* rope) {
+#pragma unroll
+  for (int j = 0; j < AB_PIECES; ++j) {
+    uint4 q = ab_piece(q_at, j), k = ab_piece(k_at, j);
+    uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
+    uint32_t* kw = reinterpret_cast<uint32_t*>(&k);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 cs = rope[((piece0 + j) * 4 + t) * CHUNK + row];
+      const float2 qr = rope_rotate(__bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&qw[t])), cs);
+      const float2 kr = rope_rotate(__bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&kw[t])), cs);
+      qw[t] = pack_bf16x2(qr.x, qr.y);
+      kw[t] = pack_bf16x2(kr.x, kr.y);
+    }
+    ab_piece(q_at, j) = q;
+    ab_piece(k_at, j) = k;
+  }
+}
+__device__ __forceinline__ uint4 tanh_piece(uint4 v) {
+  uint32_t* w = reinterpret_cast<uint32_t*>(&v);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float2 x = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t]));
+    w[t] = pack_bf16x2(tanh_fast(x.x), tanh_fast(x.y));
+  }
+  return v;
+}
+
 __global__ void __launch_bounds__(AB_THREADS, 2)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                 const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_dw,
                 const __grid_constant__ CUtensorMap tm_dout, const float2* rope, int T, int H, int d,
-                int* error_flag) {
+                int tiles, int* error_flag) {
   extern __shared__ __align__(1024) uint8_t smem_ab[];
   uint8_t* smem = smem_ab;
   if ((smem_u32(smem) & 1023u) != 0u) {  // uniform over the CTA: nothing has been set up yet
     if (threadIdx.x == 0 && error_flag != nullptr) atomicExch(error_flag, 7);
     return;
   }
-  uint8_t* sQ = smem;                    // B0
-  uint8_t* sK = sQ + TILE_BYTES;         // B1
-  uint8_t* sB2 = sK + TILE_BYTES;        // dy -> dlocal -> tanh(U)
-  uint8_t* sB3 = sB2 + TILE_BYTES;       // dmem/8 -> V -> tanh(Kr)
-  uint8_t* sP = sB3 + TILE_BYTES;
-  uint8_t* sSt = sP + 2 * TILE_BYTES;
+  uint8_t* sSt = smem + 6 * TILE_BYTES;
   uint8_t* sDW = sSt + 8192;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sDW + 8192);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);   // bars: loads 0 Q and K, 7 the other operands, 5 U; products 1 S, 2 A, 3 B, 4 C, 6 D
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, half = tid >> 7, quarter = warp & 3;
   const int piece0 = half * AB_PIECES;
-  const int n_chunks = T / CHUNK;
-  const int tile = blockIdx.x;
-  const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
-  const int row0 = b * T + n * CHUNK;
 
   if (tid == 0) {
-    for (int i = 0; i < 7; ++i) mbar_init(&bars[i], 1);
+    for (int i = 0; i < 8; ++i) mbar_init(&bars[i], 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -523,345 +556,386 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   const uint32_t t_dq = tmem + 192;    // dQr
   const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
 
+  auto load_qk = [&](int tile, uint32_t to) {
+    const int h = tile % H, row0 = tile / H * CHUNK;   // tiles of a chunk lie behind one another, chunks in token order
+    mbar_expect_tx(&bars[0], 2 * TILE_BYTES);
+    tma_load_2d(__cvta_shared_to_generic(to), &tm_qkvgu, &bars[0], h * HD, row0);
+    tma_load_2d(__cvta_shared_to_generic(to + TILE_BYTES), &tm_qkvgu, &bars[0], d + h * HD, row0);
+  };
+  auto load_rest = [&](int tile, uint32_t to, uint32_t gate_to) {
+    const int h = tile % H, row0 = tile / H * CHUNK;
+    mbar_expect_tx(&bars[7], 3 * TILE_BYTES + 2 * 8192);
+    tma_load_2d(__cvta_shared_to_generic(to), &tm_dy, &bars[7], h * HD, row0);
+    tma_load_2d(__cvta_shared_to_generic(gate_to), &tm_qkvgu, &bars[7], 3 * d + h * HD, row0);
+    tma_load_2d(sSt, &tm_state, &bars[7], 0, tile * HD);
+    tma_load_2d(__cvta_shared_to_generic(to + TILE_BYTES), &tm_qkvgu, &bars[7], 2 * d + h * HD, row0);
+    tma_load_2d(sDW, &tm_dw, &bars[7], 0, tile * HD);
+  };
+  uint32_t sA = smem_u32(smem), sB = sA + 2 * TILE_BYTES, sP = sA + 4 * TILE_BYTES;
+  const uint32_t mine_at = row * 128 + ((piece0 ^ (row & 7)) << 4), dv_at = smem_u32(sSt) + mine_at;
   if (tid == 0) {
-    mbar_expect_tx(&bars[0], 4 * TILE_BYTES + 2 * 8192);
-    tma_load_2d(sQ, &tm_qkvgu, &bars[0], 0 * d + h * HD, row0);
-    tma_load_2d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0);
-    tma_load_2d(sB2, &tm_dy, &bars[0], h * HD, row0);
-    tma_load_2d(sP, &tm_qkvgu, &bars[0], 3 * d + h * HD, row0);  // gate: kept in registers after the first stage
-    tma_load_2d(sSt, &tm_state, &bars[0], 0, tile * HD);
-    tma_load_2d(sDW, &tm_dw, &bars[0], 0, tile * HD);
+    load_qk(blockIdx.x, sA);
+    load_rest(blockIdx.x, sB, sP);
   }
-  // The thread's half of the gate row, of the dGate row and of the dV row stay in registers (4 x 16 bytes each) until
-  // the last stage, where all five gradient tiles leave through shared memory and TMA stores.
-  uint4 gate_row[AB_PIECES], dgate_row[AB_PIECES], dv_row[AB_PIECES];
-
-  bool ok = mbar_wait(&bars[0], 0, abort_flag);
+  bool ok = true;
+  uint32_t ph = 0;   // every barrier completes once per tile
+#pragma unroll 1
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ph ^= 1) {
+    const int h = tile % H, row0 = tile / H * CHUNK;
+    const uint32_t sQ = sA, sK = sA + TILE_BYTES, sB2 = sB, sB3 = sB + TILE_BYTES;
+    // The thread's half of the gate row, of the dGate row and of the dV row stay in registers (4 x 16 bytes each) until
+    // the last stage, where all five gradient tiles leave through shared memory and TMA stores.
+    uint4 gate_row[AB_PIECES], dgate_row[AB_PIECES], dv_row[AB_PIECES];
+    ok = mbar_wait(&bars[0], ph, abort_flag) && ok;
+    if (ok) ab_rope(sQ + mine_at, sK + mine_at, row, piece0, rope);
+    if (tid < 128 && (tid & 31) == 0) tma_store_wait_read0();   // the gradients of the tile before have left B, P, sSt and sDW
+    tc_fence_before_sync();
+    fence_proxy_async_smem();
+    __syncthreads();
+    // ---- MMA S = Qr Kr^T, and the other operands of this tile
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after_sync();
+      if (tile != static_cast<int>(blockIdx.x)) load_rest(tile, sB, sP);
+      constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
 #pragma unroll
-  for (int j = 0; j < AB_PIECES; ++j) gate_row[j] = *reinterpret_cast<const uint4*>(tile_chunk(sP, row, piece0 + j));
-  if (ok) {
-    rope_tanh_row(sQ, row, rope, true, false, piece0, AB_PIECES);
-    rope_tanh_row(sK, row, rope, true, false, piece0, AB_PIECES);
-    // dmem/8 = dy * (1 - sigmoid(gate)) / 8  -> B3
-#pragma unroll
-    for (int j = 0; j < AB_PIECES; ++j) {
-      const uint4 dyq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, row, piece0 + j));
-      const uint4 gq = gate_row[j];
-      const __nv_bfloat162* dyb = reinterpret_cast<const __nv_bfloat162*>(&dyq);
-      const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
-      uint4 o;
-      uint32_t* wo = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 dyv = __bfloat1622float2(dyb[t]);
-        const float2 gf = __bfloat1622float2(gb[t]);
-        wo[t] = pack_bf16x2(dyv.x * (1.f - sigmoid_f(gf.x)) * 0.125f, dyv.y * (1.f - sigmoid_f(gf.y)) * 0.125f);
-      }
-      *reinterpret_cast<uint4*>(tile_chunk(sB3, row, piece0 + j)) = o;
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16(t_lo, make_smem_desc_sw128((sQ) + k * 32, 0, 1024),
+                  make_smem_desc_sw128((sK) + k * 32, 0, 1024), idesc_s, k > 0);
+      umma_commit(&bars[1]);
     }
-  }
-  fence_proxy_async_smem();
-  __syncthreads();
-  // ---- MMA A: S = Qr Kr^T, Mem = Qr State, dQr = (dmem/8) State^T
-  if (warp == 0 && elect_one() && ok) {
-    constexpr uint32_t idesc_s = make_idesc_bf16(128, 128, false, false);
-    constexpr uint32_t idesc_m = make_idesc_bf16(128, 64, false, true);
-    constexpr uint32_t idesc_kk64 = make_idesc_bf16(128, 64, false, false);
+    ok = mbar_wait(&bars[7], ph, abort_flag) && ok;
 #pragma unroll
-    for (int k = 0; k < HD / 16; ++k)
-      umma_bf16(t_lo, make_smem_desc_sw128(smem_u32(sQ) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sK) + k * 32, 0, 1024), idesc_s, k > 0);
-#pragma unroll
-    for (int k = 0; k < HD / 16; ++k)
-      umma_bf16(t_mid, make_smem_desc_sw128(smem_u32(sQ) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sSt) + k * 2048, 0, 1024), idesc_m, k > 0);
-#pragma unroll
-    for (int k = 0; k < HD / 16; ++k)
-      umma_bf16(t_dq, make_smem_desc_sw128(smem_u32(sB3) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sSt) + k * 32, 0, 1024), idesc_kk64, k > 0);
-    umma_commit(&bars[1]);
-  }
-  ok = ok && mbar_wait(&bars[1], 0, abort_flag);
-  tc_fence_after_sync();
-  if (tid == 0 && ok) {  // B3 (dmem) has been consumed: fetch V into it behind the softmax
-    mbar_expect_tx(&bars[2], TILE_BYTES);
-    tma_load_2d(sB3, &tm_qkvgu, &bars[2], 2 * d + h * HD, row0);
-  }
-
-  // ---- softmax over this thread's two blocks of columns, {half, half + 2} x 32, held in registers: one TMEM read and
-  // one exponential per score.  The two threads of a row meet once, with (max, sum) of their columns, in the State
-  // tile's space (the State has been consumed); a block behind the causal mask counts as (-inf, 0), and so does a half
-  // whose visible scores are all -inf (a product that overflowed): the other half decides the row.
-  const float kScale = 0.125f * 1.4426950408889634f;
-  float* meet = reinterpret_cast<float*>(sSt);   // [2][128] max | [2][128] sum | [2][128] D
-  float e[2][32];
-  float my_max = -INFINITY, my_sum = 0.f;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int cc = half + 2 * k;
-    if (cc <= quarter) {
-      uint32_t r[32];
-      tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        e[k][j] = cc * 32 + j <= row ? __uint_as_float(r[j]) : -INFINITY;
-        my_max = fmaxf(my_max, e[k][j]);
-      }
-    }
-  }
-  const float from = my_max == -INFINITY ? 0.f : my_max;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    if (half + 2 * k <= quarter) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        e[k][j] = exp2f((e[k][j] - from) * kScale);
-        my_sum += e[k][j];
-      }
-    }
-  }
-  meet[half * 128 + row] = my_max;
-  meet[256 + half * 128 + row] = my_sum;
-  __syncthreads();
-  const float other_max = meet[(half ^ 1) * 128 + row];
-  const float row_max = fmaxf(my_max, other_max);
-  const float my_share = exp2f((my_max - row_max) * kScale);
-  const float row_sum = my_sum * my_share + meet[256 + (half ^ 1) * 128 + row] * exp2f((other_max - row_max) * kScale);
-  const float to_p = my_share / row_sum;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int cc = half + 2 * k;
-    uint32_t pk[16];
-    if (cc <= quarter) {
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) pk[j >> 1] = pack_bf16x2(e[k][j] * to_p, e[k][j + 1] * to_p);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) pk[j] = 0u;
-    }
-    store_row_chunk32(sP, row, cc * 32, pk);
-  }
-  tc_fence_before_sync();
-  fence_proxy_async_smem();
-  __syncthreads();
-  // ---- MMA B: O = P V
-  if (warp == 0 && elect_one() && ok) {
-    ok = mbar_wait(&bars[2], 0, abort_flag);  // V has landed
+    for (int j = 0; j < AB_PIECES; ++j) gate_row[j] = ab_piece(sP + mine_at, j);
     if (ok) {
+      // dmem/8 = dy * (1 - sigmoid(gate)) / 8  -> the second tile of P
+#pragma unroll
+      for (int j = 0; j < AB_PIECES; ++j) {
+        const uint4 dyq = ab_piece(sB2 + mine_at, j);
+        const uint4 gq = gate_row[j];
+        const __nv_bfloat162* dyb = reinterpret_cast<const __nv_bfloat162*>(&dyq);
+        const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
+        uint4 o;
+        uint32_t* wo = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const float2 dyv = __bfloat1622float2(dyb[t]);
+          const float2 gf = __bfloat1622float2(gb[t]);
+          // (1 - sigmoid(g)) / 8 = (1 - tanh(g / 2)) / 16
+          wo[t] = pack_bf16x2(dyv.x * fmaf(tanh_fast(0.5f * gf.x), -0.0625f, 0.0625f), dyv.y * fmaf(tanh_fast(0.5f * gf.y), -0.0625f, 0.0625f));
+        }
+        ab_piece(sP + TILE_BYTES + mine_at, j) = o;
+      }
+    }
+    fence_proxy_async_smem();
+    __syncthreads();
+    // ---- MMA A: Mem = Qr State, dQr = (dmem/8) State^T
+    if (warp == 0 && elect_one() && ok) {
+      constexpr uint32_t idesc_m = make_idesc_bf16(128, 64, false, true);
+      constexpr uint32_t idesc_kk64 = make_idesc_bf16(128, 64, false, false);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16(t_mid, make_smem_desc_sw128((sQ) + k * 32, 0, 1024),
+                  make_smem_desc_sw128(smem_u32(sSt) + k * 2048, 0, 1024), idesc_m, k > 0);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16(t_dq, make_smem_desc_sw128((sP + TILE_BYTES) + k * 32, 0, 1024),
+                  make_smem_desc_sw128(smem_u32(sSt) + k * 32, 0, 1024), idesc_kk64, k > 0);
+      umma_commit(&bars[2]);
+    }
+    ok = mbar_wait(&bars[1], ph, abort_flag) && ok;
+    tc_fence_after_sync();
+
+    // ---- softmax over this thread's two blocks of columns, {half, half + 2} x 32, held in registers: one TMEM read and
+    // one exponential per score.  The two threads of a row meet once, with (max, sum) of their columns, in the State
+    // tile's space (the State has been consumed); a block behind the causal mask counts as (-inf, 0), and so does a half
+    // whose visible scores are all -inf (a product that overflowed): the other half decides the row.
+    const float kScale = 0.125f * 1.4426950408889634f;
+    float* meet = reinterpret_cast<float*>(sSt);   // [2][128] max | [2][128] sum | [2][128] D
+    float e[2][32];
+    float my_max = -INFINITY, my_sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int cc = half + 2 * k;
+      if (cc <= quarter) {
+        uint32_t r[32];
+        tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          e[k][j] = cc * 32 + j <= row ? __uint_as_float(r[j]) : -INFINITY;
+          my_max = fmaxf(my_max, e[k][j]);
+        }
+      } else {   // never read; without a value here they would be kept from tile to tile
+#pragma unroll
+        for (int j = 0; j < 32; ++j) e[k][j] = 0.f;
+      }
+    }
+    const float from = my_max == -INFINITY ? 0.f : my_max;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      if (half + 2 * k <= quarter) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          e[k][j] = exp2f((e[k][j] - from) * kScale);
+          my_sum += e[k][j];
+        }
+      }
+    }
+    ok = mbar_wait(&bars[2], ph, abort_flag) && ok;   // State and dmem have been consumed
+    meet[half * 128 + row] = my_max;
+    meet[256 + half * 128 + row] = my_sum;
+    __syncthreads();
+    const float other_max = meet[(half ^ 1) * 128 + row];
+    const float row_max = fmaxf(my_max, other_max);
+    const float my_share = exp2f((my_max - row_max) * kScale);
+    const float row_sum = my_sum * my_share + meet[256 + (half ^ 1) * 128 + row] * exp2f((other_max - row_max) * kScale);
+    const float to_p = my_share / row_sum;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int cc = half + 2 * k;
+      uint32_t pk[16];
+      if (cc <= quarter) {
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) pk[j >> 1] = pack_bf16x2(e[k][j] * to_p, e[k][j + 1] * to_p);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) pk[j] = 0u;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ab_piece(sP + k * TILE_BYTES + mine_at, j) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+    }
+    tc_fence_before_sync();
+    fence_proxy_async_smem();
+    __syncthreads();
+    // ---- MMA B: O = P V
+    if (warp == 0 && elect_one() && ok) {
       tc_fence_after_sync();
       constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
 #pragma unroll
       for (int k = 0; k < CHUNK / 16; ++k)
-        umma_bf16(t_lo, make_smem_desc_sw128(smem_u32(sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
-                  make_smem_desc_sw128(smem_u32(sB3) + k * 2048, 0, 1024), idesc_o, k > 0);
+        umma_bf16(t_lo, make_smem_desc_sw128((sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
+                  make_smem_desc_sw128((sB3) + k * 2048, 0, 1024), idesc_o, k > 0);
       umma_commit(&bars[3]);
     }
-  }
-  ok = mbar_wait(&bars[3], 0, abort_flag) && ok;
-  tc_fence_after_sync();
-
-  // ---- element-wise stage 1: dlocal = dy * g (in place in B2), dGate, D = sum(dlocal * local)
-  float Drow = 0.f;
+    // ---- element-wise stage 1: under the product dlocal = dy * g (in place in B2) and dlocal * (1 - g), behind it
+    // dGate = dy (local - memory) g (1 - g) and D = sum(dlocal * local)
+    float dl[AB_PIECES * 8], dg[AB_PIECES * 8];
 #pragma unroll
-  for (int i = 0; i < AB_PIECES; i += 2) {
-    const int c = (piece0 + i) * 8;
-    uint32_t ro[16], rm[16];
-    tmem_ld_32x32b_x16(t_lo + lane_base + c, ro);
-    tmem_ld_32x32b_x16(t_mid + lane_base + c, rm);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 16; j += 8) {
-      const int mine = i + (j >> 3);
-      uint4* pdl = reinterpret_cast<uint4*>(tile_chunk(sB2, row, piece0 + mine));
-      const uint4 dyq = *pdl;
-      const uint4 gq = gate_row[mine];
-      const __nv_bfloat162* dyb = reinterpret_cast<const __nv_bfloat162*>(&dyq);
+    for (int i = 0; i < AB_PIECES; ++i) {
+      uint4 dyq = ab_piece(sB2 + mine_at, i);
+      const uint4 gq = gate_row[i];
+      uint32_t* w = reinterpret_cast<uint32_t*>(&dyq);
       const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
-      uint4 o_dl, o_dg;
-      uint32_t* w_dl = reinterpret_cast<uint32_t*>(&o_dl);
-      uint32_t* w_dg = reinterpret_cast<uint32_t*>(&o_dg);
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
-        const float2 dyv = __bfloat1622float2(dyb[t]);
+        const float2 dyv = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t]));
         const float2 gf = __bfloat1622float2(gb[t]);
         const float g0 = sigmoid_f(gf.x), g1 = sigmoid_f(gf.y);
-        const float l0 = __uint_as_float(ro[j + 2 * t]), l1 = __uint_as_float(ro[j + 2 * t + 1]);
-        const float m0 = __uint_as_float(rm[j + 2 * t]) * 0.125f, m1 = __uint_as_float(rm[j + 2 * t + 1]) * 0.125f;
-        const float dl0 = dyv.x * g0, dl1 = dyv.y * g1;
-        Drow += dl0 * l0 + dl1 * l1;
-        w_dl[t] = pack_bf16x2(dl0, dl1);
-        w_dg[t] = pack_bf16x2(dyv.x * (l0 - m0) * g0 * (1.f - g0), dyv.y * (l1 - m1) * g1 * (1.f - g1));
+        const int e0 = i * 8 + 2 * t, e1 = e0 + 1;
+        dl[e0] = dyv.x * g0;
+        dl[e1] = dyv.y * g1;
+        dg[e0] = dl[e0] * (1.f - g0);
+        dg[e1] = dl[e1] * (1.f - g1);
+        w[t] = pack_bf16x2(dl[e0], dl[e1]);
       }
-      *pdl = o_dl;
-      dgate_row[mine] = o_dg;
+      ab_piece(sB2 + mine_at, i) = dyq;
     }
-  }
-  meet[512 + half * 128 + row] = Drow;
-  tc_fence_before_sync();
-  fence_proxy_async_smem();
-  __syncthreads();
-  Drow += meet[512 + (half ^ 1) * 128 + row];
-  // ---- MMA C: dP = dlocal V^T, dV = P^T dlocal
-  if (warp == 0 && elect_one() && ok) {
+    ok = mbar_wait(&bars[3], ph, abort_flag) && ok;
     tc_fence_after_sync();
-    constexpr uint32_t idesc_kk128 = make_idesc_bf16(128, 128, false, false);
-    constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);
+    float Drow = 0.f;
 #pragma unroll
-    for (int k = 0; k < HD / 16; ++k)
-      umma_bf16(t_lo, make_smem_desc_sw128(smem_u32(sB2) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sB3) + k * 32, 0, 1024), idesc_kk128, k > 0);
+    for (int i = 0; i < AB_PIECES; i += 2) {
+      const int c = (piece0 + i) * 8;
+      uint32_t ro[16], rm[16];
+      tmem_ld_32x32b_x16(t_lo + lane_base + c, ro);
+      tmem_ld_32x32b_x16(t_mid + lane_base + c, rm);
+      tmem_ld_wait();
+      uint32_t w[8];
 #pragma unroll
-    for (int k = 0; k < CHUNK / 16; ++k)
-      umma_bf16(t_mid, make_smem_desc_sw128(smem_u32(sP) + k * 2048, TILE_BYTES, 1024),
-                make_smem_desc_sw128(smem_u32(sB2) + k * 2048, 0, 1024), idesc_mnmn64, k > 0);
-    umma_commit(&bars[4]);
-  }
-  ok = mbar_wait(&bars[4], 0, abort_flag) && ok;
-  tc_fence_after_sync();
-  if (tid == 0 && ok) {  // B2 (dlocal) has been consumed: fetch U into it behind the dS phase
-    mbar_expect_tx(&bars[5], TILE_BYTES);
-    tma_load_2d(sB2, &tm_qkvgu, &bars[5], 4 * d + h * HD, row0);
-  }
-
-  // ---- dS = P * (dP - D) / 8 over P; dV out; tanh(Kr) -> B3
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const int cc = half + 2 * k;
-    if (cc > quarter) continue;
-    uint32_t r[32], pk[16];
-    tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
-    load_row_chunk32(sP, row, cc * 32, pk);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const float2 pv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[j]));
-      const float s0 = pv.x * (__uint_as_float(r[2 * j]) - Drow) * 0.125f;
-      const float s1 = pv.y * (__uint_as_float(r[2 * j + 1]) - Drow) * 0.125f;
-      pk[j] = pack_bf16x2(s0, s1);
-    }
-    store_row_chunk32(sP, row, cc * 32, pk);
-  }
-#pragma unroll
-  for (int i = 0; i < AB_PIECES; i += 2) {
-    uint32_t rv[16];
-    tmem_ld_32x32b_x16(t_mid + lane_base + (piece0 + i) * 8, rv);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 16; j += 8) {
-      dv_row[i + (j >> 3)] = make_uint4(pack_bf16x2(__uint_as_float(rv[j]), __uint_as_float(rv[j + 1])),
-                                        pack_bf16x2(__uint_as_float(rv[j + 2]), __uint_as_float(rv[j + 3])),
-                                        pack_bf16x2(__uint_as_float(rv[j + 4]), __uint_as_float(rv[j + 5])),
-                                        pack_bf16x2(__uint_as_float(rv[j + 6]), __uint_as_float(rv[j + 7])));
-    }
-  }
-#pragma unroll
-  for (int j = piece0; j < piece0 + AB_PIECES; ++j) {  // tanh(Kr) -> B3 (V is no longer needed)
-    const uint4 kq = *reinterpret_cast<const uint4*>(tile_chunk(sK, row, j));
-    const __nv_bfloat162* kb = reinterpret_cast<const __nv_bfloat162*>(&kq);
-    uint4 o;
-    uint32_t* wo = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const float2 kv = __bfloat1622float2(kb[t]);
-      wo[t] = pack_bf16x2(tanh_fast(kv.x), tanh_fast(kv.y));
-    }
-    *reinterpret_cast<uint4*>(tile_chunk(sB3, row, j)) = o;
-  }
-  ok = mbar_wait(&bars[5], 0, abort_flag) && ok;  // U has landed
-  if (ok) rope_tanh_row(sB2, row, rope, false, true, piece0, AB_PIECES);
-  tc_fence_before_sync();
-  fence_proxy_async_smem();
-  __syncthreads();
-  // ---- MMA D: dQr += dS Kr, dKr = dS^T Qr, dtK = tU dW^T, dtU = tK dW
-  if (warp == 0 && elect_one() && ok) {
-    tc_fence_after_sync();
-    constexpr uint32_t idesc_kmn64 = make_idesc_bf16(128, 64, false, true);
-    constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);
-    constexpr uint32_t idesc_kk64 = make_idesc_bf16(128, 64, false, false);
-#pragma unroll
-    for (int k = 0; k < CHUNK / 16; ++k)
-      umma_bf16(t_dq, make_smem_desc_sw128(smem_u32(sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sK) + k * 2048, 0, 1024), idesc_kmn64, 1u);
-#pragma unroll
-    for (int k = 0; k < CHUNK / 16; ++k)
-      umma_bf16(t_lo, make_smem_desc_sw128(smem_u32(sP) + k * 2048, TILE_BYTES, 1024),
-                make_smem_desc_sw128(smem_u32(sQ) + k * 2048, 0, 1024), idesc_mnmn64, k > 0);
-#pragma unroll
-    for (int k = 0; k < HD / 16; ++k)  // dtK = tU dW^T
-      umma_bf16(t_lo + 64, make_smem_desc_sw128(smem_u32(sB2) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sDW) + k * 32, 0, 1024), idesc_kk64, k > 0);
-#pragma unroll
-    for (int k = 0; k < HD / 16; ++k)  // dtU = tK dW
-      umma_bf16(t_mid, make_smem_desc_sw128(smem_u32(sB3) + k * 32, 0, 1024),
-                make_smem_desc_sw128(smem_u32(sDW) + k * 2048, 0, 1024), idesc_kmn64, k > 0);
-    umma_commit(&bars[6]);
-  }
-  ok = mbar_wait(&bars[6], 0, abort_flag) && ok;
-  tc_fence_after_sync();
-
-  // ---- final: dQ, dK (RoPE transpose), dU
-#pragma unroll
-  for (int i = 0; i < AB_PIECES; i += 2) {
-    const int c = (piece0 + i) * 8;
-    uint32_t rq[16], rk[16], rtk[16], rtu[16];
-    tmem_ld_32x32b_x16(t_dq + lane_base + c, rq);
-    tmem_ld_32x32b_x16(t_lo + lane_base + c, rk);
-    tmem_ld_32x32b_x16(t_lo + 64 + lane_base + c, rtk);
-    tmem_ld_32x32b_x16(t_mid + lane_base + c, rtu);
-    tmem_ld_wait();
-#pragma unroll
-    for (int j = 0; j < 16; j += 8) {
-      const int mine = i + (j >> 3), chunk = piece0 + mine;
-      const uint4 tkq = *reinterpret_cast<const uint4*>(tile_chunk(sB3, row, chunk));
-      const uint4 tuq = *reinterpret_cast<const uint4*>(tile_chunk(sB2, row, chunk));
-      const __nv_bfloat162* tkb = reinterpret_cast<const __nv_bfloat162*>(&tkq);
-      const __nv_bfloat162* tub = reinterpret_cast<const __nv_bfloat162*>(&tuq);
-      uint4 o_q, o_k, o_u;
-      uint32_t* w_q = reinterpret_cast<uint32_t*>(&o_q);
-      uint32_t* w_k = reinterpret_cast<uint32_t*>(&o_k);
-      uint32_t* w_u = reinterpret_cast<uint32_t*>(&o_u);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const int e0 = j + 2 * t, e1 = e0 + 1;
-        const float2 cs = rope[((c + e0) >> 1) * CHUNK + row];
-        const float2 tk = __bfloat1622float2(tkb[t]);
-        const float2 tu = __bfloat1622float2(tub[t]);
-        // y0 = x0 c - x1 s ; y1 = x1 c + x0 s   =>   dx0 = dy0 c + dy1 s ; dx1 = dy1 c - dy0 s
-        const float q0 = __uint_as_float(rq[e0]), q1 = __uint_as_float(rq[e1]);
-        w_q[t] = pack_bf16x2(q0 * cs.x + q1 * cs.y, q1 * cs.x - q0 * cs.y);
-        const float k0 = __uint_as_float(rk[e0]) + __uint_as_float(rtk[e0]) * (1.f / CHUNK) * (1.f - tk.x * tk.x);
-        const float k1 = __uint_as_float(rk[e1]) + __uint_as_float(rtk[e1]) * (1.f / CHUNK) * (1.f - tk.y * tk.y);
-        w_k[t] = pack_bf16x2(k0 * cs.x + k1 * cs.y, k1 * cs.x - k0 * cs.y);
-        w_u[t] = pack_bf16x2(__uint_as_float(rtu[e0]) * (1.f / CHUNK) * (1.f - tu.x * tu.x),
-                             __uint_as_float(rtu[e1]) * (1.f / CHUNK) * (1.f - tu.y * tu.y));
+      for (int j = 0; j < 16; j += 2) {
+        const float l0 = __uint_as_float(ro[j]), l1 = __uint_as_float(ro[j + 1]);
+        const int e0 = i * 8 + j, e1 = e0 + 1;
+        Drow += dl[e0] * l0 + dl[e1] * l1;
+        w[j >> 1] = pack_bf16x2(dg[e0] * fmaf(__uint_as_float(rm[j]), -0.125f, l0), dg[e1] * fmaf(__uint_as_float(rm[j + 1]), -0.125f, l1));
       }
-      // every operand of the last MMA group has been consumed: Q, K, P, State and dW tiles are free
-      *reinterpret_cast<uint4*>(tile_chunk(sQ, row, chunk)) = o_q;
-      *reinterpret_cast<uint4*>(tile_chunk(sK, row, chunk)) = o_k;
-      *reinterpret_cast<uint4*>(tile_chunk(sP, row, chunk)) = o_u;
-      *reinterpret_cast<uint4*>(tile_chunk(sP + TILE_BYTES, row, chunk)) = dgate_row[mine];
-      *reinterpret_cast<uint4*>(tile_chunk(sSt, row, chunk)) = dv_row[mine];
+      dgate_row[i] = make_uint4(w[0], w[1], w[2], w[3]);
+      dgate_row[i + 1] = make_uint4(w[4], w[5], w[6], w[7]);
     }
-  }
-  fence_proxy_async_smem();
-  // the two warps that share 32 token rows (immediate barrier numbers: a register would reserve all sixteen)
-  if (quarter == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
-  else if (quarter == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
-  else if (quarter == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
-  else asm volatile("bar.sync 4, 64;" ::: "memory");
-  if (tid < 128 && (tid & 31) == 0) {  // one store per gradient tile for those rows
+    meet[512 + half * 128 + row] = Drow;
+    tc_fence_before_sync();
+    fence_proxy_async_smem();
+    __syncthreads();
+    Drow = (Drow + meet[512 + (half ^ 1) * 128 + row]) * 0.125f;
+    // ---- MMA C: dP = dlocal V^T, dV = P^T dlocal
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after_sync();
+      constexpr uint32_t idesc_kk128 = make_idesc_bf16(128, 128, false, false);
+      constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16(t_lo, make_smem_desc_sw128((sB2) + k * 32, 0, 1024),
+                  make_smem_desc_sw128((sB3) + k * 32, 0, 1024), idesc_kk128, k > 0);
+#pragma unroll
+      for (int k = 0; k < CHUNK / 16; ++k)
+        umma_bf16(t_mid, make_smem_desc_sw128((sP) + k * 2048, TILE_BYTES, 1024),
+                  make_smem_desc_sw128((sB2) + k * 2048, 0, 1024), idesc_mnmn64, k > 0);
+      umma_commit(&bars[4]);
+    }
+    ok = mbar_wait(&bars[4], ph, abort_flag) && ok;
+    tc_fence_after_sync();
+    if (tid == 0 && ok) {  // B2 (dlocal) has been consumed: fetch U into it behind the dS phase
+      mbar_expect_tx(&bars[5], TILE_BYTES);
+      tma_load_2d(__cvta_shared_to_generic(sB2), &tm_qkvgu, &bars[5], 4 * d + h * HD, row0);
+    }
+
+    // ---- dS = P * (dP - D) / 8 over P
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int cc = half + 2 * k;
+      if (cc > quarter) continue;
+      uint32_t r[32], pk[16];
+      tmem_ld_32x32b_x32(t_lo + lane_base + cc * 32, r);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(&pk[4 * j]) = ab_piece(sP + k * TILE_BYTES + mine_at, j);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float2 pv = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&pk[j]));
+        const float s0 = pv.x * fmaf(__uint_as_float(r[2 * j]), 0.125f, -Drow);   // (dP - D) / 8
+        const float s1 = pv.y * fmaf(__uint_as_float(r[2 * j + 1]), 0.125f, -Drow);
+        pk[j] = pack_bf16x2(s0, s1);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) ab_piece(sP + k * TILE_BYTES + mine_at, j) = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+    }
+    tc_fence_before_sync();
+    fence_proxy_async_smem();
+    __syncthreads();
+    // ---- MMA D, first half: dQr += dS Kr, dKr = dS^T Qr
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after_sync();
+      constexpr uint32_t idesc_kmn64 = make_idesc_bf16(128, 64, false, true);
+      constexpr uint32_t idesc_mnmn64 = make_idesc_bf16(128, 64, true, true);
+#pragma unroll
+      for (int k = 0; k < CHUNK / 16; ++k)
+        umma_bf16(t_dq, make_smem_desc_sw128((sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
+                  make_smem_desc_sw128((sK) + k * 2048, 0, 1024), idesc_kmn64, 1u);
+#pragma unroll
+      for (int k = 0; k < CHUNK / 16; ++k)
+        umma_bf16(t_lo, make_smem_desc_sw128((sP) + k * 2048, TILE_BYTES, 1024),
+                  make_smem_desc_sw128((sQ) + k * 2048, 0, 1024), idesc_mnmn64, k > 0);
+    }
+    // ---- under it: dV out; tanh(Kr) -> B3, tanh(U)
+#pragma unroll
+    for (int i = 0; i < AB_PIECES; i += 2) {
+      uint32_t rv[16];
+      tmem_ld_32x32b_x16(t_mid + lane_base + (piece0 + i) * 8, rv);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; j += 8) {
+        dv_row[i + (j >> 3)] = make_uint4(pack_bf16x2(__uint_as_float(rv[j]), __uint_as_float(rv[j + 1])),
+                                          pack_bf16x2(__uint_as_float(rv[j + 2]), __uint_as_float(rv[j + 3])),
+                                          pack_bf16x2(__uint_as_float(rv[j + 4]), __uint_as_float(rv[j + 5])),
+                                          pack_bf16x2(__uint_as_float(rv[j + 6]), __uint_as_float(rv[j + 7])));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < AB_PIECES; ++j) ab_piece(sB3 + mine_at, j) = tanh_piece(ab_piece(sK + mine_at, j));   // V is no longer needed
+    ok = mbar_wait(&bars[5], ph, abort_flag) && ok;  // U has landed
     if (ok) {
-      const int r = row0 + quarter * 32, off = quarter * 4096;
-      tma_store_2d(&tm_dout, sQ + off, 0 * d + h * HD, r);
-      tma_store_2d(&tm_dout, sK + off, 1 * d + h * HD, r);
-      tma_store_2d(&tm_dout, sSt + off, 2 * d + h * HD, r);
-      tma_store_2d(&tm_dout, sP + TILE_BYTES + off, 3 * d + h * HD, r);
-      tma_store_2d(&tm_dout, sP + off, 4 * d + h * HD, r);
-      tma_store_commit();
+#pragma unroll
+      for (int j = 0; j < AB_PIECES; ++j) ab_piece(sB2 + mine_at, j) = tanh_piece(ab_piece(sB2 + mine_at, j));
     }
-    tma_store_wait_read0();
+    tc_fence_before_sync();
+    fence_proxy_async_smem();
+    __syncthreads();
+    // ---- second half: dtK = tU dW^T, dtU = tK dW; the arrival counts for both halves
+    if (warp == 0 && elect_one() && ok) {
+      tc_fence_after_sync();
+      constexpr uint32_t idesc_kmn64 = make_idesc_bf16(128, 64, false, true);
+      constexpr uint32_t idesc_kk64 = make_idesc_bf16(128, 64, false, false);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)  // dtK = tU dW^T
+        umma_bf16(t_lo + 64, make_smem_desc_sw128((sB2) + k * 32, 0, 1024),
+                  make_smem_desc_sw128(smem_u32(sDW) + k * 32, 0, 1024), idesc_kk64, k > 0);
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)  // dtU = tK dW
+        umma_bf16(t_mid, make_smem_desc_sw128((sB3) + k * 32, 0, 1024),
+                  make_smem_desc_sw128(smem_u32(sDW) + k * 2048, 0, 1024), idesc_kmn64, k > 0);
+      umma_commit(&bars[6]);
+    }
+    ok = mbar_wait(&bars[6], ph, abort_flag) && ok;
+    tc_fence_after_sync();
+
+    if (tid == 0 && ok && tile + static_cast<int>(gridDim.x) < tiles) load_qk(tile + gridDim.x, sP);   // dS has been consumed
+
+    // ---- final: dQ, dK (RoPE transpose), dU
+#pragma unroll
+    for (int i = 0; i < AB_PIECES; i += 2) {
+      const int c = (piece0 + i) * 8;
+      uint32_t rq[16], rk[16], rtk[16], rtu[16];
+      tmem_ld_32x32b_x16(t_dq + lane_base + c, rq);
+      tmem_ld_32x32b_x16(t_lo + lane_base + c, rk);
+      tmem_ld_32x32b_x16(t_lo + 64 + lane_base + c, rtk);
+      tmem_ld_32x32b_x16(t_mid + lane_base + c, rtu);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; j += 8) {
+        const int mine = i + (j >> 3);
+        const uint4 tkq = ab_piece(sB3 + mine_at, mine);
+        const uint4 tuq = ab_piece(sB2 + mine_at, mine);
+        const __nv_bfloat162* tkb = reinterpret_cast<const __nv_bfloat162*>(&tkq);
+        const __nv_bfloat162* tub = reinterpret_cast<const __nv_bfloat162*>(&tuq);
+        uint4 o_q, o_k, o_u;
+        uint32_t* w_q = reinterpret_cast<uint32_t*>(&o_q);
+        uint32_t* w_k = reinterpret_cast<uint32_t*>(&o_k);
+        uint32_t* w_u = reinterpret_cast<uint32_t*>(&o_u);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const int e0 = j + 2 * t, e1 = e0 + 1;
+          const float2 cs = rope[((c + e0) >> 1) * CHUNK + row];
+          const float2 tk = __bfloat1622float2(tkb[t]);
+          const float2 tu = __bfloat1622float2(tub[t]);
+          // y0 = x0 c - x1 s ; y1 = x1 c + x0 s   =>   dx0 = dy0 c + dy1 s ; dx1 = dy1 c - dy0 s
+          const float q0 = __uint_as_float(rq[e0]), q1 = __uint_as_float(rq[e1]);
+          w_q[t] = pack_bf16x2(q0 * cs.x + q1 * cs.y, q1 * cs.x - q0 * cs.y);
+          const float k0 = __uint_as_float(rk[e0]) + __uint_as_float(rtk[e0]) * (1.f / CHUNK) * (1.f - tk.x * tk.x);
+          const float k1 = __uint_as_float(rk[e1]) + __uint_as_float(rtk[e1]) * (1.f / CHUNK) * (1.f - tk.y * tk.y);
+          w_k[t] = pack_bf16x2(k0 * cs.x + k1 * cs.y, k1 * cs.x - k0 * cs.y);
+          w_u[t] = pack_bf16x2(__uint_as_float(rtu[e0]) * (1.f / CHUNK) * (1.f - tu.x * tu.x),
+                               __uint_as_float(rtu[e1]) * (1.f / CHUNK) * (1.f - tu.y * tu.y));
+        }
+        // every operand of the last MMA group has been consumed, and tanh(U) and tanh(Kr) by the thread that takes their place
+        ab_piece(sQ + mine_at, mine) = o_q;
+        ab_piece(sK + mine_at, mine) = o_k;
+        ab_piece(sB2 + mine_at, mine) = o_u;
+        ab_piece(sB3 + mine_at, mine) = dgate_row[mine];
+        ab_piece(dv_at, mine) = dv_row[mine];
+      }
+    }
+    fence_proxy_async_smem();
+    // the two warps that share 32 token rows (immediate barrier numbers: a register would reserve all sixteen)
+    if (quarter == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+    else if (quarter == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+    else if (quarter == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+    else asm volatile("bar.sync 4, 64;" ::: "memory");
+    if (tid < 128 && (tid & 31) == 0) {  // one store per gradient tile for those rows
+      if (ok) {
+        const int r = row0 + quarter * 32, off = quarter * 4096;
+        tma_store_2d(&tm_dout, __cvta_shared_to_generic(sQ + off), 0 * d + h * HD, r);
+        tma_store_2d(&tm_dout, __cvta_shared_to_generic(sK + off), 1 * d + h * HD, r);
+        tma_store_2d(&tm_dout, sSt + off, 2 * d + h * HD, r);
+        tma_store_2d(&tm_dout, __cvta_shared_to_generic(sB3 + off), 3 * d + h * HD, r);
+        tma_store_2d(&tm_dout, __cvta_shared_to_generic(sB2 + off), 4 * d + h * HD, r);
+        tma_store_commit();
+      }
+    }
+    const uint32_t next = sP;
+    sP = sB;
+    sB = sA;
+    sA = next;
   }
+  if (tid < 128 && (tid & 31) == 0) tma_store_wait_read0();
   tc_fence_before_sync();
   __syncthreads();
   if (tid == 0 && *abort_flag != 0 && error_flag != nullptr) atomicExch(error_flag, 5);
@@ -944,8 +1018,13 @@ extern "C" int ws_attn_bwd(const void* qkvgu, const void* states, const void* dy
       return -20;
     configured = true;
   }
-  launch_dependent(attn_bwd_kernel, dim3(tiles), dim3(AB_THREADS), AB_SMEM, stream, tm, ts, td, tw, to, reinterpret_cast<const float2*>(rope),
-                                                          T, H, d, error_flag);
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -20;
+  }
+  launch_dependent(attn_bwd_kernel, dim3(tiles < 2 * sms ? tiles : 2 * sms), dim3(AB_THREADS), AB_SMEM, stream, tm, ts, td, tw, to,
+                   reinterpret_cast<const float2*>(rope), T, H, d, tiles, error_flag);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
