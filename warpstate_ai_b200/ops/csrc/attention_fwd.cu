@@ -20,6 +20,7 @@
 #include "attention_common.cuh"
 
 #include <cstdlib>
+#include <type_traits>
 
 namespace ws {
 
@@ -507,7 +508,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
     for (int j = 0; j < 32; ++j)
       if (cc * 32 + j <= tid) row_max = fmaxf(row_max, __uint_as_float(r[j]));
   }
-  float row_sum = 0.f;
+  float even_sum = 0.f, odd_sum = 0.f;   // over the blocks of 32 columns, as the streaming form's two threads of a row have them
   [[maybe_unused]] uint32_t low[PROMPT ? 4 : 1][16];
 #pragma unroll(PROMPT ? 4 : 1)
   for (int cc = 0; cc < 4; ++cc) {
@@ -516,6 +517,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       uint32_t r[32];
       tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, r);
       tmem_ld_wait();
+      float row_sum = cc & 1 ? odd_sum : even_sum;
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
         const float p0 = (cc * 32 + j <= tid) ? softmax_term(__uint_as_float(r[j]), row_max, kScale) : 0.f;
@@ -531,6 +533,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
           low[cc][j >> 1] = *reinterpret_cast<const uint32_t*>(&l);
         }
       }
+      if (cc & 1) odd_sum = row_sum;
+      else even_sum = row_sum;
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -578,7 +582,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   }
 
   // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
-  const float inv_l = 1.f / row_sum;
+  const float inv_l = 1.f / (even_sum + odd_sum);
 #pragma unroll
   for (int c = 0; c < HD; c += 16) {
     uint32_t ro[16], rm[16];
@@ -621,17 +625,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 }
 
 // =============================================================================== attention, streaming form
-// attn_fwd_kernel as one persistent CTA per SM with specialised warps (17 warps):
+// attn_fwd_kernel as one persistent CTA per SM with specialised warps (25 warps):
 //
-//   warp 16        producer: TMA loads of tile i (Q, K, gate, V, state: 72 KiB) into stage i % 3 of a ring
+//   warp 24        producer: TMA loads of tile i (Q, K, gate, V, state: 72 KiB) into stage i % 3 of a ring
 //   warps 0..7     RoPE workers: thread (row r, half q) rotates four of the eight 16-byte pieces of row r of Q and of
 //                  K in place (its 16 (cos, sin) pairs live in registers); worker 0 then issues S = Qr Kr^T and
 //                  Mem = Qr State into TMEM set i % 2 -- Mem does not depend on the softmax, so it rides with S
-//   warps 8..11    softmax group 0 (tiles 0, 2, 4, ...), warps 12..15 softmax group 1 (tiles 1, 3, ...): one thread per
-//                  token row, as in attn_fwd_kernel: causal softmax straight out of TMEM, unnormalised P (BF16) into
+//   warps 8..15    softmax group 0 (tiles 0, 2, 4, ...), warps 16..23 softmax group 1 (tiles 1, 3, ...): two threads per token
+//                  row, each with every other block of 32 score columns and half of the output columns; they exchange their
+//                  maxima and sums through shared memory.  With one thread per row a tile was 14.9 k clocks of its group,
+//                  8192 rows of 32 heads took 54.2 us, 48.7 so.
+//                  As in attn_fwd_kernel: causal softmax straight out of TMEM, unnormalised P (BF16) into
 //                  the tile's K and Q space (both dead once S and Mem are complete; the gate tile stays where it is),
-//                  O = P V issued by the group's first thread into the first 64 columns of S, gate blend from O, Mem
-//                  and the gate tile into the Q space, one TMA store per warp; the store's read of the tile releases
+//                  O = P V issued by the group's first warp into the first 64 columns of S, gate blend from O, Mem
+//                  and the gate tile into the Q space, one TMA store per 32 rows; the store's read of the tile releases
 //                  the ring stage, the group's last TMEM read releases the TMEM set.
 //
 // Two tiles are in their softmax / blend phase at any time while a third is being rotated and a fourth loaded;
@@ -640,9 +647,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 // results.  PROMPT as in attn_fwd_kernel; the low terms of P are formed from S again, which is still in TMEM, once O has
 // the high ones.
 constexpr int AS_STAGES = 3;
-constexpr int AS_THREADS = 17 * 32;
+constexpr int AS_THREADS = 25 * 32;
 constexpr int AS_STAGE_BYTES = 4 * TILE_BYTES + 8192;
-constexpr int AS_SMEM = AS_STAGES * AS_STAGE_BYTES + 1024 + 256;
+constexpr int AS_MEET = 2 * 4 * 128 * 4;   // per group and row: two maxima, two sums
+constexpr int AS_SMEM = AS_STAGES * AS_STAGE_BYTES + AS_MEET + 1024 + 256;
 
 template <bool PROMPT>
 __global__ void __launch_bounds__(AS_THREADS, 1)
@@ -651,12 +659,13 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
                        int tiles, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AS_STAGES * AS_STAGE_BYTES);
+  float* meetings = reinterpret_cast<float*>(smem + AS_STAGES * AS_STAGE_BYTES);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + AS_STAGES * AS_STAGE_BYTES + AS_MEET);
   uint64_t* full = bars;                     // [3] stage loaded
-  uint64_t* empty = bars + AS_STAGES;        // [3] stage released (4 warps of the owning group)
+  uint64_t* empty = bars + AS_STAGES;        // [3] stage released (4 storing warps of the owning group)
   uint64_t* sfull = bars + 2 * AS_STAGES;    // [2] S and Mem complete
   uint64_t* ofull = sfull + 2;               // [2] O complete
-  uint64_t* setfree = ofull + 2;             // [2] TMEM set read out (4 warps)
+  uint64_t* setfree = ofull + 2;             // [2] TMEM set read out (4 storing warps, for two each)
   uint64_t* lowfull = setfree + 2;           // [2] O has the low terms too (PROMPT)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(lowfull + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -694,7 +703,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
   const int first = blockIdx.x, step = gridDim.x;
   auto stage_ptr = [&](int s) { return smem + s * AS_STAGE_BYTES; };  // Q | K | gate | V | state
 
-  if (warp == 16) {
+  if (warp == 24) {
     if (lane == 0) {
       int i = 0;
       for (int tile = first; tile < tiles; tile += step, ++i) {
@@ -778,24 +787,27 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
     }
   } else {
     // ------------------------------------------------------------------ softmax groups
-    const int g = (warp - 8) >> 2;
-    const int gt = tid - (256 + g * 128);       // row of the tile = TMEM lane
-    const int wq = gt >> 5;                     // lane quarter of this warp
+    const int g = (warp - 8) >> 3;
+    const int wq = warp & 3, half = ((warp - 8) >> 2) & 1;   // lane quarter of this warp; which blocks of columns it has
+    const int gt = wq * 32 + lane;              // row of the tile = TMEM lane
     const uint32_t t_s = tmem + g * 192, t_o = tmem + 384 + g * 64, t_m = t_s + 128;
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float kScale = 0.125f * 1.4426950408889634f;  // fold log2(e)
     const int last_chunk = wq;  // columns beyond 32*wq+31 are masked for the whole warp
-    // whether any of the group's threads is not ok; a barrier of its 128 threads
+    float* meet = meetings + g * 512;           // [2][128] maxima | [2][128] sums
+    // whether any of the group's threads is not ok; a barrier of its 256 threads
     auto any_bad = [&](bool ok) {
       uint32_t bad;
       if (g == 0)
-        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 3, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 3, 256, q;\n selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(bad) : "r"(ok ? 0u : 1u) : "memory");
       else
-        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 4, 128, q;\n selp.u32 %0, 1, 0, p;\n}\n"
+        asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 4, 256, q;\n selp.u32 %0, 1, 0, p;\n}\n"
                      : "=r"(bad) : "r"(ok ? 0u : 1u) : "memory");
       return bad != 0u;
     };
+    // the two warps that share 32 rows
+    auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(5 + g * 4 + wq) : "memory"); };
     [[maybe_unused]] uint32_t opens = 0;   // open chunks this group has met
     int i = g;
     for (int tile = first + g * step; tile < tiles; tile += 2 * step, i += 2) {
@@ -831,7 +843,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       tc_fence_after_sync();
       float row_sum = 0.f, row_max = -INFINITY;
       if (ok) {
-        for (int cc = 0; cc <= last_chunk; ++cc) {
+        for (int cc = half; cc <= last_chunk; cc += 2) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
           tmem_ld_wait();
@@ -839,36 +851,49 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           for (int j = 0; j < 32; ++j)
             if (cc * 32 + j <= gt) row_max = fmaxf(row_max, __uint_as_float(v[j]));
         }
-        for (int cc = 0; cc < 4; ++cc) {
-          uint32_t pk[16];
-          if (cc <= last_chunk) {
-            uint32_t v[32];
-            tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
-            tmem_ld_wait();
-#pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              const float p0 = (cc * 32 + j <= gt) ? softmax_term(__uint_as_float(v[j]), row_max, kScale) : 0.f;
-              const float p1 = (cc * 32 + j + 1 <= gt) ? softmax_term(__uint_as_float(v[j + 1]), row_max, kScale) : 0.f;
-              const __nv_bfloat162 pv = __floats2bfloat162_rn(p0, p1);
-              const float2 back = __bfloat1622float2(pv);
-              row_sum += back.x + back.y;  // normalise by what the MMA will actually sum
-              pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&pv);
-              if (PROMPT && open) {
-                const float2 rest = __bfloat1622float2(__floats2bfloat162_rn(p0 - back.x, p1 - back.y));
-                row_sum += rest.x + rest.y;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) pk[j] = 0u;
-          }
-          store_p(cc, pk);
-        }
       }
+      meet[half * 128 + gt] = row_max;
+      pair_sync();
+      if (ok) {
+        row_max = fmaxf(row_max, meet[(half ^ 1) * 128 + gt]);
+        // REST: a prompt's open chunk, whose weights are two BF16 terms (a branch per score would cost every tile)
+        auto weights = [&](auto rest_too) {
+          constexpr bool REST = decltype(rest_too)::value;
+          for (int cc = half; cc < 4; cc += 2) {
+            uint32_t pk[16];
+            if (cc <= last_chunk) {
+              uint32_t v[32];
+              tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 32; j += 2) {
+                const float p0 = (cc * 32 + j <= gt) ? softmax_term(__uint_as_float(v[j]), row_max, kScale) : 0.f;
+                const float p1 = (cc * 32 + j + 1 <= gt) ? softmax_term(__uint_as_float(v[j + 1]), row_max, kScale) : 0.f;
+                const __nv_bfloat162 pv = __floats2bfloat162_rn(p0, p1);
+                const float2 back = __bfloat1622float2(pv);
+                row_sum += back.x + back.y;  // normalise by what the MMA will actually sum
+                pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&pv);
+                if constexpr (REST) {
+                  const float2 rest = __bfloat1622float2(__floats2bfloat162_rn(p0 - back.x, p1 - back.y));
+                  row_sum += rest.x + rest.y;
+                }
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 16; ++j) pk[j] = 0u;
+            }
+            store_p(cc, pk);
+          }
+        };
+        if (PROMPT && open) weights(std::integral_constant<bool, PROMPT>{});
+        else weights(std::false_type{});
+      }
+      meet[256 + half * 128 + gt] = row_sum;
       tc_fence_before_sync();
       fence_proxy_async_smem();
       if (any_bad(ok)) break;
-      if (wq == 0 && elect_one()) issue_o(0u, &ofull[g]);
+      row_sum = meet[256 + gt] + meet[384 + gt];
+      if (warp == 8 + 8 * g && elect_one()) issue_o(0u, &ofull[g]);
       landed = 0;
       if (lane == 0) landed = mbar_wait(&ofull[g], k2 & 1, abort_flag) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
@@ -876,7 +901,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       if constexpr (PROMPT) {
         if (open) {  // O += P_lo V
           if (ok && row0 + wq * 32 < T) {  // the rows of a warp past the prompt's end are not stored
-            for (int cc = 0; cc < 4; ++cc) {
+            for (int cc = half; cc < 4; cc += 2) {
               uint32_t pk[16];
               if (cc <= last_chunk) {
                 uint32_t v[32];
@@ -899,7 +924,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           tc_fence_before_sync();
           fence_proxy_async_smem();
           if (any_bad(ok)) break;
-          if (wq == 0 && elect_one()) issue_o(1u, &lowfull[g]);
+          if (warp == 8 + 8 * g && elect_one()) issue_o(1u, &lowfull[g]);
           landed = 0;
           if (lane == 0) landed = mbar_wait(&lowfull[g], opens & 1, abort_flag) ? 1u : 0u;
           ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
@@ -911,7 +936,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
         const float inv_l = 1.f / row_sum;
 #pragma unroll
-        for (int c = 0; c < HD; c += 16) {
+        for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 16) {
           uint32_t ro[16], rm[16];
           tmem_ld_32x32b_x16(t_o + lane_base + c, ro);
           tmem_ld_32x32b_x16(t_m + lane_base + c, rm);
@@ -936,19 +961,19 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       }
       tc_fence_before_sync();
       fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(&setfree[g]);   // this warp's lanes of S / O / Mem have been read
+      pair_sync();
+      if (half == 0 && lane == 0) {
+        mbar_arrive(&setfree[g]);   // these lanes of S / O / Mem have been read
         if (ok && row0 + wq * 32 < T) {
           tma_store_3d(&tm_y, sQ + wq * 4096, h * HD, row0 + wq * 32, b);
           tma_store_commit();
         }
         tma_store_wait_read0();
-        mbar_arrive(&empty[s]);     // this warp no longer touches the stage
+        mbar_arrive(&empty[s]);     // neither warp touches these rows of the stage any more
       }
       __syncwarp();
       // a warp that gave up does not leave alone: its next wait fails at once (the abort flag is up), and the
-      // group's vote at the next barrier takes all four warps out together
+      // group's vote at the next barrier takes all eight warps out together
     }
   }
   tc_fence_before_sync();
