@@ -65,6 +65,13 @@ def forward_only(qkvgu: torch.Tensor, core, batch: int, seq: int, want_final: bo
     return y, writes, states, (ff, fs)
 
 
+def forward_first_chunk(qkvgu: torch.Tensor, core, batch: int) -> torch.Tensor:
+    """y [M,d] of sequences of one chunk, which read empty memories and whose writes nothing reads."""
+    _ext.require()
+    return torch.ops.ws_b200.attn_fwd(qkvgu, None, rope_table(qkvgu.device, pair_major=True), batch, core.chunk, core.h,
+                                      error_flag(qkvgu.device))
+
+
 def prefill(qkvgu: torch.Tensor, core, batch: int, seq: int, state) -> torch.Tensor:
     """y [M,d] for prompts of any length; ``state`` (fast, slow, mixed, k, v, u of a decode layer) is overwritten with
     what a decode continues from: the memories after the complete chunks, and the open chunk's K, V and U."""

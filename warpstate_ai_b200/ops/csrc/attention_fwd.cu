@@ -319,17 +319,68 @@ chunk_writes_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const _
 // One thread owns four consecutive state elements (16-byte loads, 8-byte stores) and requests the writes of
 // SCAN_AHEAD chunks before it runs their recurrence, so a thread keeps 128 bytes in flight instead of 4.
 constexpr int SCAN_AHEAD = 8;
+constexpr int SCAN_THREADS_FWD = 128;
 
-__global__ void __launch_bounds__(128)
+// What a decode needs of the chunk a prompt ends in: roped K, V and U of its `rest` positions, as the step kernel
+// appends them, and zeros behind them (rest = 0 clears the caches).  OPEN_BLOCKS blocks per (sequence, head); 16-byte pieces.  They go
+// with the scan's blocks in one launch: neither fills the chip for a few sequences, and a launch of their own was 3 us a layer
+// of a 300-token prompt.
+constexpr int OPEN_BLOCKS = 4;
+struct OpenChunk {
+  const __nv_bfloat16* qkvgu;
+  const float2* rope;
+  int T, rest, H, d;
+  __nv_bfloat16 *kc, *vc, *uc;
+};
+__device__ __forceinline__ void open_chunk(const OpenChunk& o, int block) {
+  const int at_head = block / OPEN_BLOCKS, part = block - at_head * OPEN_BLOCKS;
+  const int h = at_head % o.H, b = at_head / o.H;
+  const size_t cache = static_cast<size_t>(at_head) * CHUNK * HD;
+  const __nv_bfloat16* base = o.qkvgu + (static_cast<size_t>(b) * o.T + (o.T - o.rest)) * 5 * o.d + h * HD;
+  constexpr int PIECES = CHUNK * 8 / OPEN_BLOCKS;
+#pragma unroll
+  for (int k0 = 0; k0 < PIECES; k0 += SCAN_THREADS_FWD) {
+    const int i = part * PIECES + k0 + threadIdx.x, r = i >> 3, j = i & 7;
+    uint4 k = make_uint4(0u, 0u, 0u, 0u), v = k, u = k;
+    if (r < o.rest) {
+      const __nv_bfloat16* row = base + static_cast<size_t>(r) * 5 * o.d + j * 8;
+      k = *reinterpret_cast<const uint4*>(row + o.d);
+      v = *reinterpret_cast<const uint4*>(row + 2 * o.d);
+      u = *reinterpret_cast<const uint4*>(row + 4 * o.d);
+      uint32_t* w = reinterpret_cast<uint32_t*>(&k);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 x = rope_rotate(__bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t])),
+                                     o.rope[(j * 4 + t) * CHUNK + r]);
+        w[t] = pack_bf16x2(x.x, x.y);
+      }
+    }
+    const size_t at = cache + static_cast<size_t>(r) * HD + j * 8;
+    *reinterpret_cast<uint4*>(o.kc + at) = k;
+    *reinterpret_cast<uint4*>(o.vc + at) = v;
+    *reinterpret_cast<uint4*>(o.uc + at) = u;
+  }
+}
+
+// PROMPT: the blocks past the scan's take the open chunk, and `writes` may be absent where there is no complete chunk.
+template <bool PROMPT>
+__global__ void __launch_bounds__(SCAN_THREADS_FWD)
 memory_scan_kernel(const float* writes, const float* fast_logit,
                    const float* slow_logit, const float* mix_logit,
                    __nv_bfloat16* __restrict__ states, float* __restrict__ final_fast,
                    float* __restrict__ final_slow, __nv_bfloat16* __restrict__ final_mixed,
                    const float* init_fast, const float* init_slow, int B, int N, int complete,
-                   int H) {
+                   int H, const OpenChunk tail) {
   pdl_launch_dependents();
   pdl_wait();
-  const size_t quad = blockIdx.x * static_cast<size_t>(128) + threadIdx.x;  // over B*H*1024 groups of four
+  if constexpr (PROMPT) {
+    const int scan_blocks = B * H * (1024 / SCAN_THREADS_FWD);
+    if (static_cast<int>(blockIdx.x) >= scan_blocks) {
+      open_chunk(tail, blockIdx.x - scan_blocks);
+      return;
+    }
+  }
+  const size_t quad = blockIdx.x * static_cast<size_t>(SCAN_THREADS_FWD) + threadIdx.x;  // over B*H*1024 groups of four
   const size_t total = static_cast<size_t>(B) * H * 1024;
   if (quad >= total) return;
   const int e = static_cast<int>(quad % 1024) * 4;
@@ -358,7 +409,8 @@ memory_scan_kernel(const float* writes, const float* fast_logit,
     float4 w[SCAN_AHEAD];
 #pragma unroll
     for (int j = 0; j < SCAN_AHEAD; ++j)
-      if (n0 + j < N) w[j] = *reinterpret_cast<const float4*>(writes + base + (n0 + j) * chunk_stride);
+      if (PROMPT ? n0 + j < complete : n0 + j < N) w[j] = *reinterpret_cast<const float4*>(writes + base + (n0 + j) * chunk_stride);
+      else w[j] = make_float4(0.f, 0.f, 0.f, 0.f);   // nothing reads the state behind it
 #pragma unroll
     for (int j = 0; j < SCAN_AHEAD; ++j) {
       if (n0 + j >= N) break;
@@ -371,40 +423,6 @@ memory_scan_kernel(const float* writes, const float* fast_logit,
     }
   }
   if (complete == N && final_fast != nullptr) leave();
-}
-
-// =============================================================================== open chunk of a prompt
-// What a decode needs of the chunk a prompt ends in: roped K, V and U of its `rest` positions, as the step kernel
-// appends them, and zeros behind them (rest = 0 clears the caches).  One CTA per (sequence, head); 16-byte pieces.
-__global__ void __launch_bounds__(256)
-open_chunk_kernel(const __nv_bfloat16* qkvgu, const float2* rope, int T, int rest, int H, int d,
-                  __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc, __nv_bfloat16* __restrict__ uc) {
-  pdl_launch_dependents();
-  pdl_wait();
-  const int h = blockIdx.x % H, b = blockIdx.x / H;
-  const size_t cache = static_cast<size_t>(blockIdx.x) * CHUNK * HD;
-  const __nv_bfloat16* base = qkvgu + (static_cast<size_t>(b) * T + (T - rest)) * 5 * d + h * HD;
-  for (int i = threadIdx.x; i < CHUNK * 8; i += 256) {
-    const int r = i >> 3, j = i & 7;
-    uint4 k = make_uint4(0u, 0u, 0u, 0u), v = k, u = k;
-    if (r < rest) {
-      const __nv_bfloat16* row = base + static_cast<size_t>(r) * 5 * d + j * 8;
-      k = *reinterpret_cast<const uint4*>(row + d);
-      v = *reinterpret_cast<const uint4*>(row + 2 * d);
-      u = *reinterpret_cast<const uint4*>(row + 4 * d);
-      uint32_t* w = reinterpret_cast<uint32_t*>(&k);
-#pragma unroll
-      for (int t = 0; t < 4; ++t) {
-        const float2 x = rope_rotate(__bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t])),
-                                     rope[(j * 4 + t) * CHUNK + r]);
-        w[t] = pack_bf16x2(x.x, x.y);
-      }
-    }
-    const size_t at = cache + static_cast<size_t>(r) * HD + j * 8;
-    *reinterpret_cast<uint4*>(kc + at) = k;
-    *reinterpret_cast<uint4*>(vc + at) = v;
-    *reinterpret_cast<uint4*>(uc + at) = u;
-  }
 }
 
 // =============================================================================== attention
@@ -426,7 +444,7 @@ constexpr int AF_SMEM = 4 * TILE_BYTES + 8192 + 1024 + 128;
 template <bool PROMPT>
 __global__ void __launch_bounds__(128, 3)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
-                const __grid_constant__ CUtensorMap tm_y, const float2* rope, int T, int H, int d,
+                const __grid_constant__ CUtensorMap tm_y, const float2* rope, int T, int H, int d, bool memory,
                 int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
@@ -468,12 +486,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
 
   if (tid == 0) {
-    mbar_expect_tx(&bars[0], 4 * TILE_BYTES + 8192);
+    mbar_expect_tx(&bars[0], 4 * TILE_BYTES + (memory ? 8192 : 0));
     tma_load_3d(sQ, &tm_qkvgu, &bars[0], 0 * d + h * HD, row0, b);
     tma_load_3d(sK, &tm_qkvgu, &bars[0], 1 * d + h * HD, row0, b);
     tma_load_3d(sV, &tm_qkvgu, &bars[0], 2 * d + h * HD, row0, b);
     tma_load_3d(sG, &tm_qkvgu, &bars[0], 3 * d + h * HD, row0, b);
-    tma_load_2d(sSt, &tm_state, &bars[0], 0, tile * HD);
+    if (memory) tma_load_2d(sSt, &tm_state, &bars[0], 0, tile * HD);
   }
   bool ok = mbar_wait(&bars[0], 0, abort_flag);
   uint4 gate_row[8];  // this thread's gate row: the tile's space becomes half of P
@@ -555,7 +573,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       umma_bf16(t_o, make_smem_desc_sw128(smem_u32(sP) + (k >> 2) * TILE_BYTES + (k & 3) * 32, 0, 1024),
                 make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, k > 0);
 #pragma unroll
-    for (int k = 0; k < HD / 16; ++k)  // Mem = Q State
+    for (int k = 0; memory && k < HD / 16; ++k)  // Mem = Q State
       umma_bf16(t_m, make_smem_desc_sw128(smem_u32(sQ) + k * 32, 0, 1024),
                 make_smem_desc_sw128(smem_u32(sSt) + k * 2048, 0, 1024), idesc_o, k > 0);
     umma_commit(&bars[2]);
@@ -587,7 +605,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   for (int c = 0; c < HD; c += 16) {
     uint32_t ro[16], rm[16];
     tmem_ld_32x32b_x16(t_o + lane_base + c, ro);
-    tmem_ld_32x32b_x16(t_m + lane_base + c, rm);
+    if (memory) {
+      tmem_ld_32x32b_x16(t_m + lane_base + c, rm);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) rm[j] = 0u;
+    }
     tmem_ld_wait();
 #pragma unroll
     for (int j = 0; j < 16; j += 8) {
@@ -656,7 +679,7 @@ template <bool PROMPT>
 __global__ void __launch_bounds__(AS_THREADS, 1)
 attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                        const __grid_constant__ CUtensorMap tm_y, const float2* rope, int T, int H, int d,
-                       int tiles, int* error_flag) {
+                       int tiles, bool memory, int* error_flag) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   float* meetings = reinterpret_cast<float*>(smem + AS_STAGES * AS_STAGE_BYTES);
@@ -712,12 +735,12 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         const int h = tile % H, n = (tile / H) % n_chunks, b = tile / (H * n_chunks);
         const int row0 = n * CHUNK;
         uint8_t* st = stage_ptr(s);
-        mbar_expect_tx(&full[s], AS_STAGE_BYTES);
+        mbar_expect_tx(&full[s], memory ? AS_STAGE_BYTES : 4 * TILE_BYTES);
         tma_load_3d(st, &tm_qkvgu, &full[s], 0 * d + h * HD, row0, b);
         tma_load_3d(st + TILE_BYTES, &tm_qkvgu, &full[s], 1 * d + h * HD, row0, b);
         tma_load_3d(st + 2 * TILE_BYTES, &tm_qkvgu, &full[s], 3 * d + h * HD, row0, b);
         tma_load_3d(st + 3 * TILE_BYTES, &tm_qkvgu, &full[s], 2 * d + h * HD, row0, b);
-        tma_load_2d(st + 4 * TILE_BYTES, &tm_state, &full[s], 0, tile * HD);
+        if (memory) tma_load_2d(st + 4 * TILE_BYTES, &tm_state, &full[s], 0, tile * HD);
       }
     }
   } else if (warp < 8) {
@@ -779,7 +802,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           umma_bf16(t_s, make_smem_desc_sw128(smem_u32(sQ) + k * 32, 0, 1024),
                     make_smem_desc_sw128(smem_u32(sK) + k * 32, 0, 1024), idesc_s, k > 0);
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)  // Mem = Qr State
+        for (int k = 0; memory && k < HD / 16; ++k)  // Mem = Qr State
           umma_bf16(t_m, make_smem_desc_sw128(smem_u32(sQ) + k * 32, 0, 1024),
                     make_smem_desc_sw128(smem_u32(sSt) + k * 2048, 0, 1024), idesc_m, k > 0);
         umma_commit(&sfull[g]);
@@ -939,7 +962,12 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         for (int c = half * (HD / 2); c < (half + 1) * (HD / 2); c += 16) {
           uint32_t ro[16], rm[16];
           tmem_ld_32x32b_x16(t_o + lane_base + c, ro);
-          tmem_ld_32x32b_x16(t_m + lane_base + c, rm);
+          if (memory) {
+            tmem_ld_32x32b_x16(t_m + lane_base + c, rm);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) rm[j] = 0u;
+          }
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 16; j += 8) {
@@ -1046,13 +1074,15 @@ extern "C" int ws_chunk_writes(const void* qkvgu, const float* rope, float* writ
   return T % CHUNK != 0 ? -1 : chunk_writes(qkvgu, rope, writes, B, T, H, d, error_flag, stream);
 }
 
+// `tail`: a prompt's open chunk, which goes along; NULL: none.
 static int memory_scan(const float* writes, const float* fast_logit, const float* slow_logit, const float* mix_logit,
                        void* states, float* final_fast, float* final_slow, void* final_mixed, const float* init_fast,
-                       const float* init_slow, int B, int N, int complete, int H, cudaStream_t stream) {
-  const size_t total = (size_t)B * H * 4096;
-  launch_dependent(memory_scan_kernel, dim3((unsigned)((total / 4 + 127) / 128)), dim3(128), 0, stream, writes, fast_logit,
+                       const float* init_slow, int B, int N, int complete, int H, const OpenChunk* tail, cudaStream_t stream) {
+  const int blocks = B * H * (1024 / SCAN_THREADS_FWD);
+  launch_dependent(tail != nullptr ? memory_scan_kernel<true> : memory_scan_kernel<false>,
+                   dim3(blocks + (tail != nullptr ? B * H * OPEN_BLOCKS : 0)), dim3(SCAN_THREADS_FWD), 0, stream, writes, fast_logit,
                    slow_logit, mix_logit, (__nv_bfloat16*)states, final_fast, final_slow, (__nv_bfloat16*)final_mixed,
-                   init_fast, init_slow, B, N, complete, H);
+                   init_fast, init_slow, B, N, complete, H, tail != nullptr ? *tail : OpenChunk{});
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
@@ -1062,7 +1092,7 @@ extern "C" int ws_memory_scan(const float* writes, const float* fast_logit, cons
                               const float* init_fast, const float* init_slow, int B, int N, int H,
                               cudaStream_t stream) {
   return memory_scan(writes, fast_logit, slow_logit, mix_logit, states, final_fast, final_slow, nullptr, init_fast,
-                     init_slow, B, N, N, H, stream);
+                     init_slow, B, N, N, H, nullptr, stream);
 }
 
 template <bool PROMPT>
@@ -1073,7 +1103,8 @@ static int attn_fwd(const void* qkvgu, const void* states, const float* rope, vo
   CUtensorMap tm, ts, ty;
   int rc = make_sequence_map(&tm, qkvgu, 5 * (uint64_t)d, T, B, HD, CHUNK);
   if (rc) return rc;
-  rc = make_tile_map(&ts, states, HD, (uint64_t)tiles * HD, HD, HD, HD);
+  const bool memory = states != nullptr;   // otherwise every position is in a sequence's first chunk, whose memories are empty
+  rc = make_tile_map(&ts, memory ? states : qkvgu, HD, (uint64_t)tiles * HD, HD, HD, HD);
   if (rc) return rc;
   rc = make_sequence_map(&ty, y, (uint64_t)d, T, B, HD, 32);
   if (rc) return rc;
@@ -1093,10 +1124,10 @@ static int attn_fwd(const void* qkvgu, const void* states, const float* rope, vo
   }
   if (ws_attn_stream_form() != 0)
     launch_dependent(attn_fwd_stream_kernel<PROMPT>, dim3(tiles < sms ? tiles : sms), dim3(AS_THREADS), AS_SMEM, stream, tm, ts, ty,
-                     reinterpret_cast<const float2*>(rope), T, H, d, tiles, error_flag);
+                     reinterpret_cast<const float2*>(rope), T, H, d, tiles, memory, error_flag);
   else
     launch_dependent(attn_fwd_kernel<PROMPT>, dim3(tiles), dim3(128), AF_SMEM, stream, tm, ts, ty,
-                     reinterpret_cast<const float2*>(rope), T, H, d, error_flag);
+                     reinterpret_cast<const float2*>(rope), T, H, d, memory, error_flag);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
@@ -1111,15 +1142,13 @@ extern "C" int ws_attn_prefill(const void* qkvgu, const float* rope, const float
                                void* mixed, void* kc, void* vc, void* uc, int B, int T, int H, int d, int* error_flag,
                                cudaStream_t stream) {
   const int complete = T / CHUNK, rest = T % CHUNK;
-  int rc = chunk_writes(qkvgu, rope, writes, B, T, H, d, error_flag, stream);
+  // A prompt without a complete chunk writes nothing into the memories and reads nothing from them.
+  int rc = complete > 0 ? chunk_writes(qkvgu, rope, writes, B, T, H, d, error_flag, stream) : 0;
+  const OpenChunk tail{static_cast<const __nv_bfloat16*>(qkvgu), reinterpret_cast<const float2*>(rope), T, rest, H, d,
+                       static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc)};
   if (!rc)
-    rc = memory_scan(writes, fast_logit, slow_logit, mix_logit, states, fast, slow, mixed, nullptr, nullptr, B,
-                     complete + (rest > 0), complete, H, stream);
-  if (!rc) rc = attn_fwd<true>(qkvgu, states, rope, y, B, T, H, d, error_flag, stream);
-  if (rc) return rc;
-  launch_dependent(open_chunk_kernel, dim3(B * H), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(qkvgu),
-                   reinterpret_cast<const float2*>(rope), T, rest, H, d, static_cast<__nv_bfloat16*>(kc),
-                   static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc));
-  ws_count_launch();
-  return cudaGetLastError() == cudaSuccess ? 0 : -21;
+    rc = memory_scan(writes, fast_logit, slow_logit, mix_logit, complete > 0 ? states : nullptr, fast, slow, mixed, nullptr, nullptr, B,
+                     complete + (rest > 0), complete, H, &tail, stream);
+  if (!rc) rc = attn_fwd<true>(qkvgu, complete > 0 ? states : nullptr, rope, y, B, T, H, d, error_flag, stream);
+  return rc;
 }

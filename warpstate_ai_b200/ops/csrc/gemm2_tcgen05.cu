@@ -884,13 +884,13 @@ split_finish_kernel(const float* part, int splits, int m, int n, const void* aux
   }
 }
 
-// The same behind a residual product that an RMSNorm follows (out_proj, then the second norm): a block per row adds the pieces
-// and the residual, writes x and z = BF16(x rsqrt(mean x^2 + eps) w).  The squares are rounded and added as the norm kernels
+// The same behind a residual product that an RMSNorm follows (out_proj and the second norm; down, the next block's modulation and its
+// first norm): a block per row adds the pieces and the residual, writes x and z = BF16(x rsqrt(mean x^2 + eps) w).  The squares are rounded and added as the norm kernels
 // do it (`square_sum`; lane l of a warp owns columns 128 i + 4 l), so that both forms agree bit for bit.  n % 128 == 0, n <= 2048.  300 x 2048 in
 // four pieces: 3.2 us and the norm's 5.0 before, 3.7 so; 128 x 2048: 2.5 and 5.1, 3.0.
 __global__ void __launch_bounds__(256)
 split_finish_norm_kernel(const float* part, int splits, int m, int n, const float* aux, int ldaux, float* __restrict__ out, int ldo,
-                         const float* w, float eps, __nv_bfloat16* __restrict__ z, float* __restrict__ rstd_out) {
+                         const float* scale, const float* bias, const float* w, float eps, __nv_bfloat16* __restrict__ z, float* __restrict__ rstd_out) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float squares[512];
@@ -914,6 +914,8 @@ split_finish_norm_kernel(const float* part, int splits, int m, int n, const floa
     for (int s = 1; s < MAX_GROUP; ++s)
       if (s < splits) { v.x += p[s].x; v.y += p[s].y; v.z += p[s].z; v.w += p[s].w; }
     v = make_float4(r.x + v.x, r.y + v.y, r.z + v.z, r.w + v.w);
+    if (scale != nullptr)
+      v = modulated(v, *reinterpret_cast<const float4*>(scale + c), *reinterpret_cast<const float4*>(bias + c));
     *reinterpret_cast<float4*>(out + static_cast<size_t>(row) * ldo + c) = v;
     squares[c >> 2] = square_sum(v);
     x[i] = v;
@@ -1037,15 +1039,15 @@ extern "C" int ws_gemm_pair_split(const WsGemm* g, int splits, float* part, int 
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
-extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part, const float* w, float eps, void* z, float* rstd,
-                                       int sms, cudaStream_t stream) {
+extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part, const float* scale, const float* bias, const float* w, float eps,
+                                       void* z, float* rstd, int sms, cudaStream_t stream) {
   using namespace ws;
   if (g->epilogue != WS_EPI_RESID_F32 || g->n % 128 != 0 || g->n > 2048) return -9;
   int count = 0;
   const int rc = split_pieces(g, splits, part, sms, &count, stream);
   if (rc) return rc;
   launch_dependent(split_finish_norm_kernel, dim3(g->m), dim3(256), 0, stream, static_cast<const float*>(part), count, g->m, g->n,
-                   static_cast<const float*>(g->aux), g->ldaux, static_cast<float*>(g->out), g->ldo, w, eps,
+                   static_cast<const float*>(g->aux), g->ldaux, static_cast<float*>(g->out), g->ldo, scale, bias, w, eps,
                    static_cast<__nv_bfloat16*>(z), rstd);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;

@@ -350,14 +350,14 @@ extern "C" int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStrea
   return splits < 2 ? ws_gemm(g, stream) : ws_gemm_pair_split(g, splits, part, usable_sms(), stream);
 }
 
-extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part, const float* w, float eps, void* z, float* rstd,
-                                       int sms, cudaStream_t stream);
+extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part, const float* scale, const float* bias, const float* w, float eps,
+                                       void* z, float* rstd, int sms, cudaStream_t stream);
 
-extern "C" int ws_gemm_split_norm(const WsGemm* g, int splits, float* part, const float* w, float eps, void* z, float* rstd,
-                                  cudaStream_t stream) {
+extern "C" int ws_gemm_split_norm(const WsGemm* g, int splits, float* part, const float* scale, const float* bias, const float* w, float eps,
+                                       void* z, float* rstd, cudaStream_t stream) {
   const int rc = validate_gemm(g);
   if (rc) return rc;
-  return ws_gemm_pair_split_norm(g, splits, part, w, eps, z, rstd, usable_sms(), stream);
+  return ws_gemm_pair_split_norm(g, splits, part, scale, bias, w, eps, z, rstd, usable_sms(), stream);
 }
 
 extern "C" int ws_gemm(const WsGemm* g, cudaStream_t stream) {

@@ -63,9 +63,10 @@ int ws_gemm_pair_available(void);  // 1 where problems with >= 256 rows take the
 // A product whose tiles would leave most of the chip idle may be cut along k: ws_gemm_splits says into how many pieces
 // (1: not), and ws_gemm_split computes it so, with FP32 scratch `part` of splits * m * n floats.
 int ws_gemm_splits(const WsGemm* g);
-// A residual product (FP32) cut into `splits` > 1 pieces and the RMSNorm behind it: z [m, n] = BF16(out * rstd * w), rstd [m].
-// n % 128 == 0, n <= 2048.
-int ws_gemm_split_norm(const WsGemm* g, int splits, float* part, const float* w, float eps, void* z, float* rstd, cudaStream_t stream);
+// A residual product (FP32) cut into `splits` > 1 pieces, the depth modulation of its rows (scale and bias [n], or NULL) and the
+// RMSNorm behind it: out = (aux + product) * (1 + scale) + bias, z [m, n] = BF16(out * rstd * w), rstd [m].  n % 128 == 0, n <= 2048.
+int ws_gemm_split_norm(const WsGemm* g, int splits, float* part, const float* scale, const float* bias, const float* w, float eps,
+                       void* z, float* rstd, cudaStream_t stream);
 // Which kernel a product takes on `sms` SMs, a function of its arguments alone: 0 the single-CTA kernel, otherwise the
 // CTA-pair kernel with the product cut along k into that many pieces.  packed: a SwiGLU product writes (up | gate).
 int ws_gemm_plan(int m, int n, int k, int a_mn, int epilogue, int packed, int sms);
@@ -189,7 +190,7 @@ int ws_memory_scan(const float* writes, const float* fast_logit, const float* sl
                    const float* mix_logit, void* states, float* final_fast, float* final_slow,
                    const float* init_fast, const float* init_slow, int B, int N, int H,
                    cudaStream_t stream);
-// Forward of the block over prompts of any length T >= 1 (four launches), leaving what a decode continues from:
+// Forward of the block over prompts of any length T >= 1 (three launches, two below a chunk), leaving what a decode continues from:
 // fast / slow (FP32) and mixed (BF16) [B, H, 64, 64] after the T / 128 complete chunks; kc / vc / uc (BF16
 // [B, H, 128, 64]) hold roped K, V and U of the open chunk's T % 128 positions and zeros behind them.
 // Scratch: writes FP32 and states BF16, [B, ceil(T / 128), H, 64, 64].  y: BF16 [B*T, d].  rope: pair-major.
@@ -197,7 +198,7 @@ int ws_attn_prefill(const void* qkvgu, const float* rope, const float* fast_logi
                     const float* mix_logit, float* writes, void* states, void* y, float* fast, float* slow,
                     void* mixed, void* kc, void* vc, void* uc, int B, int T, int H, int d, int* error_flag,
                     cudaStream_t stream);
-// y: BF16 [B*T, d] token-major.
+// y: BF16 [B*T, d] token-major.  states NULL: every sequence is one chunk, and its memories are empty.
 int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* y, int B, int T, int H,
                 int d, int* error_flag, cudaStream_t stream);
 

@@ -119,10 +119,12 @@ def _wgrad_group(items):
 
 
 # --------------------------------------------------------------------------- attention hook
-def _attention_forward(qkvgu: torch.Tensor, core, batch: int, seq: int):
-    """qkvgu [M,5d] BF16 -> (y [M,d] BF16, saved-for-backward)."""
+def _attention_forward(qkvgu: torch.Tensor, core, batch: int, seq: int, keep: bool = True):
+    """qkvgu [M,5d] BF16 -> (y [M,d] BF16, saved-for-backward).  Without ``keep`` no backward follows."""
     from . import attention
     if attention.kernels_ready(core):
+        if not keep and seq == core.chunk:      # one chunk, whose memories are empty
+            return attention.forward_first_chunk(qkvgu, core, batch), None
         return attention.forward(qkvgu, core, batch, seq)
     with torch.no_grad():
         y = R.attention_memory(qkvgu.view(batch, seq, -1), core.fast_decay_logit, core.slow_decay_logit,
@@ -231,7 +233,7 @@ def _core_kernels(core, weights, x_in, scale, bias, n1w, n2w, batch, seq, want_o
     weights.begin_forward()
     z1, rstd1, xmod = ops.rmsnorm_fwd(x_in, scale, bias, n1w, core.cfg.rms_eps, True)
     qkvgu = weights.in_proj(z1)
-    y, attn_saved = _attention_forward(qkvgu, core, batch, seq)
+    y, attn_saved = _attention_forward(qkvgu, core, batch, seq, keep)
     x2 = G.linear_residual(y, weights.out_w(), xmod)
     z2, rstd2, _ = ops.rmsnorm_fwd(x2, None, None, n2w, core.cfg.rms_eps, False)
     packed, act = weights.up_gate(z2)
@@ -606,6 +608,26 @@ def core_prefill(core, x: torch.Tensor, depth_scale, depth_bias):
 
 
 @torch.no_grad()
+def cores_prefill_state(cores, x: torch.Tensor, depth_scale, depth_bias, batch: int, seq: int, states):
+    """`core_prefill_state` of all blocks in one native call: the last block's residual input and attention output, or None where a
+    block does not run natively."""
+    from . import attention
+    if G._policy or not all(attention.kernels_ready(core) for core in cores):
+        return None
+    of, weights, vectors = {}, [], []
+    for core in cores:
+        own = of.get(id(core))
+        if own is None:
+            own = of[id(core)] = ([bf16_weight(p) for p in (core.in_proj.weight, core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight)],
+                                  [core.norm1.weight, core.norm2.weight, core.fast_decay_logit, core.slow_decay_logit, core.memory_mix_logit])
+        weights += own[0]
+        vectors += own[1]
+    kept = [t for st in states for t in (st.fast, st.slow, st.mixed, st.k, st.v, st.u)]
+    return _ops().blocks_prefill(x, depth_scale.detach().float().contiguous(), depth_bias.detach().float().contiguous(), weights, vectors,
+                                 kept, attention.rope_table(x.device, pair_major=True), cores[0].cfg.rms_eps, batch, seq, cores[0].h,
+                                 G.error_flag(x.device))
+
+
 def core_prefill_state(core, x: torch.Tensor, depth_scale, depth_bias, batch: int, seq: int, state, last: bool):
     """Forward of one core over prompts of any length ``x [B*T, d]``; ``state`` receives what a decode continues from.
     Returns the rows ``[B*T, d]``, or with ``last`` (nothing reads the other positions of the last block) the block's

@@ -464,10 +464,13 @@ class DecodeEngine:
         # cast before the gather of the embeddings, which starts after all that came before and which all that follows waits for.
         finish = self._finish_weights(model.cores[(len(self.states) - 1) % self.cfg.n_cores])
         x = self.embed[self._gathered_ids(ids)].float().view(b * t, -1)
-        for depth, st in enumerate(self.states):
-            last = depth + 1 == len(self.states)
-            core = model.cores[depth % self.cfg.n_cores]
-            x = fused.core_prefill_state(core, x, model.depth_scale[depth], model.depth_bias[depth], b, t, st, last)
+        cores = [model.cores[depth % self.cfg.n_cores] for depth in range(len(self.states))]
+        core, whole = cores[-1], fused.cores_prefill_state(cores, x, model.depth_scale, model.depth_bias, b, t, self.states)
+        if whole is not None:
+            x = whole
+        else:
+            for depth, (core, st) in enumerate(zip(cores, self.states)):
+                x = fused.core_prefill_state(core, x, model.depth_scale[depth], model.depth_bias[depth], b, t, st, depth + 1 == len(cores))
         self.pos = t % self.chunk
         return self._prefill_logits(core, *x, *finish)
 
