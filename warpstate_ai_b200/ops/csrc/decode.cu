@@ -1,4 +1,5 @@
-// Decode-step kernels: one new token for every sequence of a batch (batch <= 64).
+// Decode-step kernels: one new token for every sequence of a batch (batch <= 64; the projections also for the rows of a prompt of up
+// to 128 tokens).
 //
 // A decode step is bound by streaming the weights once (4.0 GB for the 2.005 B model) and the
 // current chunk's K/V cache, so the GEMMs here are weight-streaming kernels, not tile kernels:
@@ -18,7 +19,7 @@
 //                          append k/v/u to the chunk cache, causal attention over the cache rows
 //                          <= position, memory read q.M, gate blend.
 //
-//   decode_norm_gemm_kernel    the two together, for one sequence.
+//   decode_norm_gemm_kernel    the residual + norm and the projection that reads it in one launch, for one sequence.
 //
 // The 140 to 200 launches of a step form one chain of programmatic dependent launches: every kernel lets
 // its successor start at once, and a GEMM fills its whole TMA ring with weight tiles (which no
@@ -70,7 +71,7 @@ struct DecodeCfg {
   static constexpr int EXCHANGE_BYTES = 64 * BPAD * 4;
   static_assert(EXCHANGE_BYTES <= STAGES * dec::W_BYTES, "the exchange buffer overlays the weight stages");
   static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
-  static constexpr int TMEM_COLS = BPAD < 32 ? 32 : BPAD;
+  static constexpr int TMEM_COLS = BPAD <= 32 ? 32 : BPAD <= 64 ? 64 : 128;   // a power of two
   static constexpr int CTAS_PER_SM = 2 * (SMEM + 1024) <= 233472 ? 2 : 1;
 };
 
@@ -1098,10 +1099,24 @@ static int launch_norm_gemm(const CUtensorMap& tw, const DecodeGemmParams& p, co
 template <int BPAD, int EPI>
 static int launch_decode_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const DecodeGemmParams& p, dim3 grid,
                               cudaStream_t stream) {
-  switch (decode_ring_depth()) {
+  // up to 16 KiB of X go to a stage, and the ring is what fits
+  if constexpr (BPAD > 64) return launch_decode_gemm_depth<BPAD, EPI, BPAD <= 96 ? 7 : 6>(tw, tx, p, grid, stream);
+  else if constexpr (BPAD != 16 && BPAD != 64) return launch_decode_gemm_depth<BPAD, EPI, 8>(tw, tx, p, grid, stream);
+  else switch (decode_ring_depth()) {
     case 4: return launch_decode_gemm_depth<BPAD, EPI, 4>(tw, tx, p, grid, stream);
     case 9: return launch_decode_gemm_depth<BPAD, EPI, 9>(tw, tx, p, grid, stream);
     default: return launch_decode_gemm_depth<BPAD, EPI, 8>(tw, tx, p, grid, stream);
+  }
+}
+
+template <int BPAD>
+static int launch_decode_epilogue(int epilogue, const CUtensorMap& tw, const CUtensorMap& tx, const DecodeGemmParams& p, dim3 grid,
+                                  cudaStream_t stream) {
+  switch (epilogue) {
+    case 0: return launch_decode_gemm<BPAD, 0>(tw, tx, p, grid, stream);
+    case 1: return launch_decode_gemm<BPAD, 1>(tw, tx, p, grid, stream);
+    case 2: return launch_decode_gemm<BPAD, 2>(tw, tx, p, grid, stream);
+    default: return launch_decode_gemm<BPAD, 3>(tw, tx, p, grid, stream);
   }
 }
 
@@ -1130,13 +1145,13 @@ extern "C" int ws_decode_gemm_splits(int n, int k) {
 
 // epilogue: 0 BF16 out [batch, ldo]; 1 FP32 split-K partials [splits, batch, n] (splits from
 // ws_decode_gemm_splits); 2 SwiGLU, W is [2n, k] (up rows then gate rows), BF16 out [batch, ldo];
-// 3 FP32 out [batch, ldo].  batch <= 64; k % 8 == 0.
+// 3 FP32 out [batch, ldo].  batch <= 128; k % 8 == 0.
 // packed != 0: W is the tile-by-tile copy [slabs][ceil(k/64)][128][64] (zero padded; for SwiGLU a tile
 // holds 64 up rows followed by their 64 gate rows), so that every TMA load reads 16 contiguous KiB
 // instead of 128 row pieces of 128 bytes that lie a full weight row apart.
 extern "C" int ws_decode_gemm(const void* w, const void* x, int n, int k, int batch, int epilogue, void* out, int ldo,
                               int* error_flag, int packed, cudaStream_t stream) {
-  if (n <= 0 || k <= 0 || batch <= 0 || batch > 64 || k % 8 != 0 || epilogue < 0 || epilogue > 3) return -1;
+  if (n <= 0 || k <= 0 || batch <= 0 || batch > 128 || k % 8 != 0 || epilogue < 0 || epilogue > 3) return -1;
   if (epilogue == 2 && n % 64 != 0) return -2;
   CUtensorMap tw, tx;
   const int w_rows = epilogue == 2 ? 2 * n : n;
@@ -1148,7 +1163,9 @@ extern "C" int ws_decode_gemm(const void* w, const void* x, int n, int k, int ba
     rc = make_map_bf16(&tw, w, k, w_rows, k, dec::BK, epilogue == 2 ? 64 : dec::TM);
   }
   if (rc) return rc;
-  const int bpad = batch <= 16 ? 16 : 64;
+  // The rows of X are padded to what the MMA and its operand's tile take: every CTA reads all of X, so a step of 8 layers is 334 us at 16
+  // sequences and, padded to 64, 397 at 17 and 414 at 32; padded to 32 353 and 390, at 48 450 -> 434.
+  const int bpad = batch <= 16 ? 16 : batch <= 32 ? 32 : batch <= 48 ? 48 : batch <= 64 ? 64 : batch <= 96 ? 96 : 128;
   rc = make_map_bf16(&tx, x, k, batch, k, dec::BK, bpad);
   if (rc) return rc;
   DecodeGemmParams p;
@@ -1159,16 +1176,13 @@ extern "C" int ws_decode_gemm(const void* w, const void* x, int n, int k, int ba
   p.kb_per_split = (total_kb + splits - 1) / splits;
   const int slabs = epilogue == 2 ? n / 64 : (n + dec::TM - 1) / dec::TM;
   const dim3 grid(slabs, splits);
-  const int key = (bpad == 16 ? 0 : 4) + epilogue;
-  switch (key) {
-    case 0: return launch_decode_gemm<16, 0>(tw, tx, p, grid, stream);
-    case 1: return launch_decode_gemm<16, 1>(tw, tx, p, grid, stream);
-    case 2: return launch_decode_gemm<16, 2>(tw, tx, p, grid, stream);
-    case 3: return launch_decode_gemm<16, 3>(tw, tx, p, grid, stream);
-    case 4: return launch_decode_gemm<64, 0>(tw, tx, p, grid, stream);
-    case 5: return launch_decode_gemm<64, 1>(tw, tx, p, grid, stream);
-    case 6: return launch_decode_gemm<64, 2>(tw, tx, p, grid, stream);
-    default: return launch_decode_gemm<64, 3>(tw, tx, p, grid, stream);
+  switch (bpad) {
+    case 16: return launch_decode_epilogue<16>(epilogue, tw, tx, p, grid, stream);
+    case 32: return launch_decode_epilogue<32>(epilogue, tw, tx, p, grid, stream);
+    case 48: return launch_decode_epilogue<48>(epilogue, tw, tx, p, grid, stream);
+    case 64: return launch_decode_epilogue<64>(epilogue, tw, tx, p, grid, stream);
+    case 96: return launch_decode_epilogue<96>(epilogue, tw, tx, p, grid, stream);
+    default: return launch_decode_epilogue<128>(epilogue, tw, tx, p, grid, stream);
   }
 }
 
