@@ -85,3 +85,32 @@ def test_all_blocks_of_a_prompt_equal_the_blocks_one_by_one(monkeypatch, batch, 
     assert torch.equal(got, want)
     for mine, theirs in zip(want_engine_state, apart.states[2:]):
         assert all(torch.equal(a, getattr(theirs, name)) for a, name in zip(mine, ("fast", "slow", "mixed", "k", "v", "u")))
+
+
+# the widths that rows are padded to and one row past each; several sequences, whole chunks among them; ragged contractions
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,length,d,ffn", [(1, 1, 512, 704), (1, 16, 1280, 4480), (1, 17, 512, 704), (3, 11, 640, 1088), (1, 49, 512, 704),
+                                                (13, 5, 1280, 4480), (1, 96, 512, 704), (1, 97, 640, 704), (1, 128, 2048, 1024)])
+def test_a_short_prompt_streams_its_weights(monkeypatch, batch, length, d, ffn):
+    """In other kernels than longer prompts: the same BF16 products added in FP32 in another order, so both are as far from the FP32 forward
+    pass, and no further from each other than roundings to BF16 that a changed ulp flips."""
+    torch.manual_seed(length + d)
+    with torch.device("cuda"):
+        model = WarpStateLM(config(d, ffn, depth=4, cores=2))
+    with torch.no_grad():
+        model.depth_scale.normal_(0, 0.1)
+        model.depth_bias.normal_(0, 0.1)
+    model.eval().requires_grad_(False)
+    ids = torch.randint(0, 512, (batch, length), device="cuda")
+    streamed, tiled = DecodeEngine(model), DecodeEngine(model)
+    got = streamed.prefill(ids).clone()
+    monkeypatch.setattr(fused, "cores_prefill_state", lambda *a: None)
+    want = tiled.prefill(ids)
+    gemm.check_device_errors()
+    exact = model(torch.nn.functional.pad(ids, (0, -length % 128)))[:, length - 1].float()
+    assert float((got - want).norm()) < 0.01 * float(want.norm())
+    assert float((got - exact).norm()) < 1.2 * float((want - exact).norm()) + 1e-3 * float(exact.norm())
+    for mine, theirs in zip(streamed.states, tiled.states):
+        for name in ("fast", "slow", "mixed", "k", "v", "u"):
+            a, b = getattr(mine, name).float(), getattr(theirs, name).float()
+            assert float((a - b).norm()) <= 0.01 * float(b.norm()), name

@@ -176,7 +176,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_fwd(const at::Tensor& x,
   check_rc(ws_rmsnorm_fwd(x.data_ptr(), x.scalar_type() == at::kBFloat16,
                           mod ? col_scale->data_ptr<float>() : nullptr,
                           mod ? col_bias->data_ptr<float>() : nullptr, w.data_ptr<float>(), (float)eps, rows, d,
-                          xmod.defined() ? xmod.data_ptr() : nullptr, z.data_ptr(), rstd.data_ptr<float>(),
+                          xmod.defined() ? xmod.data_ptr() : nullptr, z.data_ptr(), rstd.data_ptr<float>(), 0,
                           cur_stream()), "rmsnorm_fwd");
   return {z, rstd, xmod.defined() ? xmod : x};
 }
@@ -540,6 +540,7 @@ class ForwardBlocks {
  public:
   struct Weights { const at::Tensor *in, *out, *ug, *down; };
 
+  // `wide`: prompts, whose (up, gate) stay FP32 until the activation.
   ForwardBlocks(int64_t B, int64_t T, int64_t H, int64_t h, const at::Tensor& rope, double eps, const c10::optional<at::Tensor>& flag, bool wide,
                 const at::TensorOptions& f32)
       : B_(B), T_(T), H_(H), M_(B * T), d_(H * 64), h_(h), rope_(rope.data_ptr<float>()), eps_((float)eps),
@@ -549,10 +550,10 @@ class ForwardBlocks {
     const int64_t chunks = (T + 127) / 128, memories = B * chunks * H * 4096;
     // the second half of a block lies where the first one's packed projections and memories were
     const int64_t front = aligned(10 * M_ * d_) + aligned(4 * memories) + aligned(2 * memories);
-    pieces_out_ = pieces(residual(nullptr, nullptr, nullptr, nullptr, d_), f32);
-    pieces_down_ = pieces(residual(nullptr, nullptr, nullptr, nullptr, h_), f32);
+    pieces_out_ = streamed() ? ws_decode_gemm_splits((int)d_, (int)d_) : pieces(residual(nullptr, nullptr, nullptr, nullptr, d_));
+    pieces_down_ = streamed() ? ws_decode_gemm_splits((int)d_, (int)h_) : pieces(residual(nullptr, nullptr, nullptr, nullptr, h_));
     const int64_t cut = std::max(pieces_out_, pieces_down_);
-    const int64_t back = aligned(4 * M_ * d_) + aligned(2 * M_ * h_) + (cut > 1 ? aligned(4 * cut * M_ * d_) : 0);
+    const int64_t back = aligned(4 * M_ * d_) + aligned(2 * M_ * h_) + (cut > 1 || streamed() ? aligned(4 * cut * M_ * d_) : 0);
     scratch_ = at::empty({aligned(4 * M_ * d_) * 2 + aligned(2 * M_ * d_) * 2 + aligned(4 * M_) + std::max(front, back)}, f32.dtype(at::kByte));
     uint8_t* at = scratch_.data_ptr<uint8_t>();
     const auto take = [&](int64_t bytes) { uint8_t* p = at; at += aligned(bytes); return p; };
@@ -585,16 +586,21 @@ class ForwardBlocks {
     for (int i = 0; i < 4; ++i)
       TORCH_CHECK(t[i]->device() == scratch_.device() && t[i]->scalar_type() == at::kBFloat16 && t[i]->dim() == 2 && t[i]->size(0) == rows[i] &&
                   t[i]->size(1) == cols[i] && t[i]->stride(1) == 1 && t[i]->stride(0) % 8 == 0 &&
-                  reinterpret_cast<uintptr_t>(t[i]->data_ptr()) % 16 == 0, "blocks: BF16 CUDA weights [5d, d], [d, d], [2 ffn, d], [d, ffn]");
+                  reinterpret_cast<uintptr_t>(t[i]->data_ptr()) % 16 == 0 && (!streamed() || t[i]->is_contiguous()),
+                  "blocks: BF16 CUDA weights [5d, d], [d, d], [2 ffn, d], [d, ffn]");
   }
 
-  // The first block's modulation (scale may be NULL) and norm of x [M, d].
+  // The first block's modulation (scale may be NULL) and norm of x [M, d].  For prompts it is launched behind everything before it:
+  // nothing writes weights after that, and every product of the chain reads its own ahead of the launches in front of it (28 blocks at 300
+  // tokens 2843 -> 2814 us; for one block the start costs as much as that gives).
   void begin(const float* x, const float* scale, const float* bias, const float* n1) {
-    check_rc(ws_rmsnorm_fwd(x, 0, scale, bias, n1, eps_, (int)M_, (int)d_, scale != nullptr ? xmod_ : nullptr, z_, rstd_, stream_), "rmsnorm_fwd");
+    check_rc(ws_rmsnorm_fwd(x, 0, scale, bias, n1, eps_, (int)M_, (int)d_, scale != nullptr ? xmod_ : nullptr, z_, rstd_, wide_,
+                            stream_), "rmsnorm_fwd");
     residual_ = scale != nullptr ? xmod_ : x;
   }
 
   void project_in(const Weights& w) {
+    if (streamed()) return stream(*w.in, z_, 5 * d_, d_, 0, qkvgu_, "in_proj");
     WsGemm g = product(z_, d_, *w.in, 5 * d_, WS_EPI_BF16);
     g.out = qkvgu_; g.ldo = (int)(5 * d_);
     run(g, 1, "in_proj");
@@ -616,9 +622,10 @@ class ForwardBlocks {
                              (int)B_, (int)T_, (int)H_, (int)d_, flag_, stream_), "attn_prefill");
   }
 
-  // out_proj to the output of the block: into `out`, or into this object with the next block's modulation and norm.
+  // From out_proj to the output of the block: into `out`, or into this object with the next block's modulation and norm.
   void finish(const Weights& w, const float* n2, float* out, const float* next_scale = nullptr, const float* next_bias = nullptr,
               const float* next_n1 = nullptr) {
+    if (streamed()) return finish_streamed(w, n2, next_scale, next_bias, next_n1);
     residual_norm(residual(y_, w.out, residual_, x2_, d_), pieces_out_, nullptr, nullptr, n2, "out_proj");
     WsGemm g = product(z_, d_, *w.ug, h_, WS_EPI_SWIGLU);
     g.out2 = act_; g.ldo2 = (int)h_;
@@ -635,24 +642,47 @@ class ForwardBlocks {
   const void* attention_rows() const { return y_; }
 
  private:
+  // A prompt of at most 128 tokens is the rows of a decode step as far as its projections go: their time is that of the weights, which
+  // the step's kernels stream (decode.cu), and the rounding of (up, gate) is the step's too.  28 blocks of width 2048, with the products'
+  // own kernels -> so: 5 tokens 3911 -> 1450 us, 32 3991 -> 1567, 64 4139 -> 1909, 65 3811 -> 1999, 96 2226 -> 2055, 128 2440 -> 2253; 16 of
+  // 1280 at 16, 64, 96, 128 tokens 1605 -> 691, 1756 -> 843, 1050 -> 977, 1121 -> 1096.  Narrower blocks have projections of a few k-blocks,
+  // which there is nothing to stream of.
+  // Weights are read as they lie, row behind row, and the chain starts behind everything before it, as those kernels demand.
+  bool streamed() const { return wide_ && M_ <= 128 && d_ >= 512 && h_ % 64 == 0; }
+
+  void stream(const at::Tensor& w, const void* x, int64_t n, int64_t k, int epilogue, void* out, const char* what) {
+    check_rc(ws_decode_gemm(w.data_ptr(), x, (int)n, (int)k, (int)M_, epilogue, out, (int)n, flag_, 0, stream_), what);
+  }
+  void finish_streamed(const Weights& w, const float* n2, const float* next_scale, const float* next_bias, const float* next_n1) {
+    // the residual stream is added to in place: the first block's modulated rows are this object's own
+    float* const x = const_cast<float*>(residual_);
+    stream(*w.out, y_, d_, d_, 1, part_, "out_proj");
+    check_rc(ws_decode_reduce_norm(x, part_, (int)pieces_out_, nullptr, nullptr, 0, nullptr, nullptr, n2, eps_, (int)d_, (int)M_, z_, stream_),
+             "decode_reduce_norm");
+    stream(*w.ug, z_, h_, d_, 2, act_, "up_gate");
+    stream(*w.down, act_, d_, h_, 1, part_, "down");
+    check_rc(ws_decode_reduce_norm(x, part_, (int)pieces_down_, nullptr, nullptr, 0, next_scale, next_bias, next_n1, eps_, (int)d_, (int)M_, z_,
+                                   stream_), "decode_reduce_norm");
+  }
+
   static int64_t aligned(int64_t bytes) { return (bytes + 1023) / 1024 * 1024; }
 
   WsGemm product(const void* a, int64_t k, const at::Tensor& w, int64_t n, int epilogue) const {
     WsGemm g = {};
     g.a = a; g.b = w.data_ptr(); g.m = (int)M_; g.n = (int)n; g.k = (int)k; g.lda = (int)k; g.ldb = (int)w.stride(0);
-    g.epilogue = epilogue; g.alpha = 1.f; g.error_flag = flag_; g.wide = wide_;
+    g.epilogue = epilogue; g.alpha = 1.f; g.error_flag = flag_; g.wide = wide_; g.b_ahead = wide_;
     return g;
   }
   WsGemm residual(const void* a, const at::Tensor* w, const float* aux, float* out, int64_t k) const {
     WsGemm g = {};
     g.a = a; g.b = w != nullptr ? w->data_ptr() : nullptr; g.m = (int)M_; g.n = (int)d_; g.k = (int)k;
     g.lda = (int)k; g.ldb = w != nullptr ? (int)w->stride(0) : (int)k;
-    g.epilogue = WS_EPI_RESID_F32; g.alpha = 1.f; g.error_flag = flag_;
+    g.epilogue = WS_EPI_RESID_F32; g.alpha = 1.f; g.error_flag = flag_; g.b_ahead = wide_;
     g.aux = aux; g.ldaux = (int)d_; g.out = out; g.ldo = (int)d_;
     return g;
   }
   // Into how many pieces a residual product of these sizes is cut: the plan looks at sizes, and its checks at addresses.
-  static int64_t pieces(WsGemm g, const at::TensorOptions& f32) {
+  static int64_t pieces(WsGemm g) {
     g.a = g.b = g.aux = g.out = reinterpret_cast<void*>(16);
     return ws_gemm_splits(&g);
   }
@@ -668,7 +698,8 @@ class ForwardBlocks {
     float* const to = static_cast<float*>(g.out);
     if (scale != nullptr) g.out = x_;
     run(g, cut, what);
-    check_rc(ws_rmsnorm_fwd(g.out, 0, scale, bias, norm, eps_, (int)M_, (int)d_, scale != nullptr ? to : nullptr, z_, rstd_, stream_), "rmsnorm_fwd");
+    check_rc(ws_rmsnorm_fwd(g.out, 0, scale, bias, norm, eps_, (int)M_, (int)d_, scale != nullptr ? to : nullptr, z_, rstd_, 0,
+                            stream_), "rmsnorm_fwd");
   }
 
   const int64_t B_, T_, H_, M_, d_, h_;

@@ -94,6 +94,7 @@ struct alignas(64) PairGroup {
   CUtensorMap whole;   // row selection (problem 0): the operand before its rows were selected
   int tile_start[MAX_GROUP + 1];
   int count;
+  int ahead;           // B may be read ahead of the launches in front of this one (WsGemm::b_ahead)
 };
 
 // The SwiGLU-backward epilogue reads and writes 4 bytes of global memory per accumulator element.
@@ -234,7 +235,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
   const uint32_t tmem_base = *tmem_slot;
   // set-up is done: let the next kernel of the stream be scheduled, then wait for the previous one's results
   pdl_launch_dependents();
-  pdl_wait();
+  if (warp != 0 || !g.ahead) pdl_wait();
 
   constexpr bool kSwiglu = (EPI == WS_EPI_SWIGLU);
   const int n_tile = kSwiglu ? 128 : BN;
@@ -248,6 +249,22 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
     if (lane == 0) {
       int it = 0;
       bool ok = true;
+      // Weights ahead: those of the first ring are requested under the tail of the kernel whose result is A.  (In a chain of few-row
+      // products a launch's first round trip is 2 us, and DRAM is idle until then.)
+      int requested = 0;
+      if constexpr (!A_MN && !B_MN && !GATHER) {
+        if (g.ahead) {
+          if (pair_id < tiles) {
+            const PairTile t = resolve_tile(g, extent, pair_id, n_tile);
+            const int r0 = kSwiglu ? (rank ? g.p[0].h + t.nb * 128 : t.nb * 128) : t.nb * BN + rank * 128;
+            for (; requested < min(t.num_k, STAGES); ++requested) {
+              if (leader) mbar_expect_tx(&full[requested], 2 * STAGE_BYTES);
+              tma_load_2d_pair(sB + requested * B_BYTES, &g.b[t.prob], mapa_shared(smem_u32(&full[requested]), 0), requested * BK, r0);
+            }
+          }
+          pdl_wait();
+        }
+      }
       [[maybe_unused]] int ready_nb = -1;
       for (int tile = pair_id; tile < tiles && ok; tile += num_pairs) {
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
@@ -295,7 +312,8 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           const uint32_t bar = full_leader;
           // The leader alone announces the bytes of both CTAs (a remote expect-tx arrival with
           // release semantics from the peer measured 2x slower for the whole kernel).
-          if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+          const bool b_there = it < requested;
+          if (leader && !b_there) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
           uint8_t* a_dst = sA + s * A_BYTES;
           uint8_t* b_dst = sB + s * B_BYTES;
           if (!A_MN) {
@@ -305,6 +323,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
             for (int i = 0; i < BM / 64; ++i)
               tma_load_2d_pair(a_dst + i * (BK * 128), tma_a, bar, m0 + i * 64, kb * BK);
           }
+          if (b_there) continue;
           if (!B_MN) {
             const int r0 = kSwiglu ? (rank ? p.h + nb * 128 : nb * 128) : nb * BN + rank * 128;
             tma_load_2d_pair(b_dst, tma_b, bar, kb * BK, r0);
@@ -1073,6 +1092,8 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     total += tiles;
   }
   for (int i = count; i <= MAX_GROUP; ++i) grp.tile_start[i] = total;
+  grp.ahead = !items[0].a_mn && !items[0].b_mn && items[0].limit == nullptr;
+  for (int i = 0; i < count; ++i) grp.ahead = grp.ahead && items[i].b_ahead;
   if (items[0].epilogue == WS_EPI_F32 || items[0].epilogue == WS_EPI_ACC_F32) {
     for (int i = 0; i < count; ++i) {
       const int rc = make_map_f32(&grp.epi[i], items[i].out, items[i].n, items[i].m, items[i].ldo, 32, 32);

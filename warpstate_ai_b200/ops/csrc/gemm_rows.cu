@@ -45,7 +45,7 @@ struct alignas(64) RowsProblem {
   int m, n, k;           // n: features of the output
   int blocks, width;     // accumulators per tile, columns of each
   int stages, buffers;
-  int wide;
+  int wide, ahead;         // ahead: W may be read ahead of the launches in front of this one (WsGemm::b_ahead)
   int* error_flag;
 };
 
@@ -93,7 +93,7 @@ gemm_rows_kernel(const __grid_constant__ RowsProblem p) {
   tc_fence_after_sync();
   const uint32_t tmem = tmem_address;
   pdl_launch_dependents();
-  pdl_wait();
+  if (warp != 0 || !p.ahead) pdl_wait();
 
   constexpr int FEATURES = SWIGLU ? 128 : 256;   // of a tile; a CTA has half of them
   const int tiles = (p.n + FEATURES - 1) / FEATURES, num_k = (p.k + BK - 1) / BK;
@@ -104,6 +104,21 @@ gemm_rows_kernel(const __grid_constant__ RowsProblem p) {
       int s = 0;
       uint32_t ph = 1;
       bool ok = true;
+      auto load_weights = [&](int stage, int f0, int kb) {
+        const uint32_t bar = mapa_shared(smem_u32(&full[stage]), 0);
+        if (leader) mbar_expect_tx(&full[stage], 2 * stage_bytes);
+        uint8_t* a = sA + stage * A_BYTES;
+        tma_load_2d_pair(a, &p.w, bar, kb * BK, f0);
+        if (SWIGLU) tma_load_2d_pair(a + 64 * 128, &p.w, bar, kb * BK, p.n + f0);
+      };
+      // the weights of the first ring, under the tail of the kernel whose result the tokens are
+      int requested = 0;
+      if (p.ahead) {
+        if (pair < tiles)
+          for (; requested < min(num_k, stages); ++requested)
+            load_weights(requested, pair * FEATURES + static_cast<int>(rank) * (FEATURES / 2), requested);
+        pdl_wait();
+      }
       for (int tile = pair; tile < tiles && ok; tile += pairs) {
         const int f0 = tile * FEATURES + static_cast<int>(rank) * (FEATURES / 2);
         for (int kb = 0; kb < num_k; ++kb) {
@@ -112,10 +127,7 @@ gemm_rows_kernel(const __grid_constant__ RowsProblem p) {
             break;
           }
           const uint32_t bar = mapa_shared(smem_u32(&full[s]), 0);
-          if (leader) mbar_expect_tx(&full[s], 2 * stage_bytes);
-          uint8_t* a = sA + s * A_BYTES;
-          tma_load_2d_pair(a, &p.w, bar, kb * BK, f0);
-          if (SWIGLU) tma_load_2d_pair(a + 64 * 128, &p.w, bar, kb * BK, p.n + f0);
+          if (tile != pair || kb >= requested) load_weights(s, f0, kb);
           for (int j = 0; j < p.blocks; ++j)
             tma_load_2d_pair(sB + s * b_bytes + j * half * 128, &p.x, bar, kb * BK, j * p.width + static_cast<int>(rank) * half);
           if (++s == stages) {
@@ -287,7 +299,7 @@ extern "C" int ws_gemm_rows(const WsGemm* g, int sms, cudaStream_t stream) {
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   RowsProblem p;
   memset(&p, 0, sizeof(p));
-  p.m = g->m; p.n = g->n; p.k = g->k; p.wide = g->wide; p.error_flag = g->error_flag;
+  p.m = g->m; p.n = g->n; p.k = g->k; p.wide = g->wide; p.ahead = g->b_ahead; p.error_flag = g->error_flag;
   const int columns = rows_columns(g->m);
   p.blocks = columns <= 256 ? 1 : 2;
   p.width = columns / p.blocks;

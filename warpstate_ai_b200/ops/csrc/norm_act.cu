@@ -512,15 +512,15 @@ static int rmsnorm_block_rows(int d, bool modulated) {
 
 template <typename T>
 static void launch_rmsnorm_fwd(const T* x, const float* col_scale, const float* col_bias, const float* w, float eps, int rows, int d,
-                               T* xmod_out, __nv_bfloat16* z, float* rstd, cudaStream_t stream) {
+                               T* xmod_out, __nv_bfloat16* z, float* rstd, bool dependent, cudaStream_t stream) {
   if (rows <= rmsnorm_block_rows(d, col_scale != nullptr))
-    launch_dependent(rmsnorm_fwd_block_kernel<T>, dim3(rows), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, d,
+    launch_kernel(dependent, rmsnorm_fwd_block_kernel<T>, dim3(rows), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, d,
                      xmod_out, z, rstd);
   else if (d <= 128 * MAX_CHUNKS)   // the general kernel reads its rows twice: 4096 rows of 384, 1024, 1920 columns 5.1, 10.7, 19.7 us, 3.6, 6.5, 12.2 so
-    launch_dependent(rmsnorm_rows<T>(d / 128, std::make_integer_sequence<int, MAX_CHUNKS>{}), dim3(row_grid(rows)),
+    launch_kernel(dependent, rmsnorm_rows<T>(d / 128, std::make_integer_sequence<int, MAX_CHUNKS>{}), dim3(row_grid(rows)),
                      dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps, rows, xmod_out, z, rstd);
   else
-    launch_dependent(rmsnorm_fwd_kernel<T>, dim3(row_grid(rows)), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps,
+    launch_kernel(dependent, rmsnorm_fwd_kernel<T>, dim3(row_grid(rows)), dim3(ROW_THREADS), 0, stream, x, col_scale, col_bias, w, eps,
                      rows, d, xmod_out, z, rstd);
   ws_count_launch();
 }
@@ -531,14 +531,14 @@ using namespace ws;
 
 extern "C" int ws_rmsnorm_fwd(const void* x, int x_bf16, const float* col_scale, const float* col_bias,
                               const float* w, float eps, int rows, int d, void* xmod_out, void* z,
-                              float* rstd, cudaStream_t stream) {
+                              float* rstd, int first, cudaStream_t stream) {
   if (d % 128 != 0 || rows <= 0) return -1;
   if (x_bf16)
     launch_rmsnorm_fwd(static_cast<const __nv_bfloat16*>(x), col_scale, col_bias, w, eps, rows, d,
-                       static_cast<__nv_bfloat16*>(xmod_out), static_cast<__nv_bfloat16*>(z), rstd, stream);
+                       static_cast<__nv_bfloat16*>(xmod_out), static_cast<__nv_bfloat16*>(z), rstd, first == 0, stream);
   else
     launch_rmsnorm_fwd(static_cast<const float*>(x), col_scale, col_bias, w, eps, rows, d, static_cast<float*>(xmod_out),
-                       static_cast<__nv_bfloat16*>(z), rstd, stream);
+                       static_cast<__nv_bfloat16*>(z), rstd, first == 0, stream);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

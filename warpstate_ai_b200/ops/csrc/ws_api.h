@@ -56,6 +56,8 @@ typedef struct WsGemm {
   const void* whole;   // replaces A (a_mn: B) where *limit == whole_rows: the rows before their selection
   int whole_rows, ldwhole;
   int wide;            // SWIGLU: the activation is formed from (up, gate) as accumulated, not from their BF16 values
+  int b_ahead;         // B is weights that no launch writes since one that was not a dependent launch: it may be read ahead of the
+                       // launches in front of this one (which is a hint)
 } WsGemm;
 
 int ws_gemm(const WsGemm* g, cudaStream_t stream);
@@ -88,7 +90,7 @@ void ws_gemm_set_sm_limit(int sms);
 int ws_gather_gemm(const void* x, int m, int n, int k, const void* const* shards, int world, int rows_per_shard,
                    void* wb, void* flags, int epilogue, void* out, int ldo, void* out2, int ldo2, int* error_flag,
                    float budget_seconds, int sms, cudaStream_t stream);
-// ---- decode step (ops/csrc/decode.cu); batch <= 64
+// ---- decode step (ops/csrc/decode.cu); batch <= 64, ws_decode_gemm and ws_decode_reduce_norm also the rows of a prompt of up to 128 tokens
 // out[b, n] = sum_k x[b, k] W[n, k] as a weight-streaming kernel.  epilogue: 0 BF16 [batch, ldo];
 // 1 FP32 split-K partials [ws_decode_gemm_splits(n, k), batch, n]; 2 SwiGLU with W = [2n, k]
 // (up rows, then gate rows), BF16 [batch, ldo]; 3 FP32 [batch, ldo].
@@ -146,9 +148,10 @@ void ws_count_launch(void);
 // ----------------------------------------------------------------------------- row kernels
 // RMSNorm forward over `rows` rows of width d (d % 128 == 0).  The residual stream `x` is FP32
 // (x_bf16 = 0) or BF16.  When col_scale/col_bias are given the depth modulation
-// x*(1+scale)+bias is applied first and (optionally) written to xmod_out.  z is BF16.
+// x*(1+scale)+bias is applied first and (optionally) written to xmod_out.  z is BF16.  `first`: not as a dependent launch, so that
+// all that was launched before it has finished when the launches behind it begin.
 int ws_rmsnorm_fwd(const void* x, int x_bf16, const float* col_scale, const float* col_bias,
-                   const float* w, float eps, int rows, int d, void* xmod_out, void* z, float* rstd,
+                   const float* w, float eps, int rows, int d, void* xmod_out, void* z, float* rstd, int first,
                    cudaStream_t stream);
 // RMSNorm backward: dx_out = (dres + norm_bwd(dz)) * (1 + out_scale); optional BF16 copy;
 // dw_partial holds ws_rmsnorm_bwd_parts(rows) partial rows of d floats (d <= 2048).

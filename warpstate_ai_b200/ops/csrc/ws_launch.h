@@ -9,7 +9,7 @@
 // `griddepcontrol.wait`, which returns when the predecessor has completed and its writes are visible.
 // Rule every kernel launched through this helper keeps: no global memory access before `pdl_wait()`, by the compiler's hand
 // either (see `pdl_wait` on `__restrict__`).  The decode kernels have a launch helper and rules of their own (decode.cu):
-// they request data that no launch in front of them writes before they wait.
+// they request data that no launch in front of them writes before they wait.  So do products marked WsGemm::b_ahead.
 // WS_TRAIN_PDL=0 launches normally.
 #pragma once
 #include <cuda_runtime.h>
