@@ -1,0 +1,39 @@
+"""The decode attention with a warp per (sequence, head), which many of them take, against the kernel with a CTA for each, which few take."""
+import pytest
+import torch
+
+from warpstate_ai_b200.ops import _ext, attention
+
+
+# the first row, the edges of the 32 rows that come at a time, the last row; a count that leaves warps of the last CTA idle
+@pytest.mark.gpu
+@pytest.mark.parametrize("pos", [0, 1, 31, 32, 33, 64, 95, 127])
+@pytest.mark.parametrize("batch,heads", [(40, 32), (64, 19), (61, 21)])
+def test_a_warp_per_head_gives_what_a_cta_per_head_gives(batch, heads, pos):
+    """FP32 sums in another order, then one rounding to BF16: half an ulp of the larger neighbour at most, 2 ** -8 of the value."""
+    _ext.require()
+    torch.manual_seed(pos + heads)
+    ops, d = torch.ops.ws_b200, 64 * heads
+    rope, at = attention.rope_table(torch.device("cuda", 0)), torch.tensor(pos, device="cuda")
+    qkvgu = (torch.randn(batch, 5 * d, device="cuda") * 1.5).bfloat16()
+    state = [torch.randn(batch, heads, 128, 64, device="cuda").bfloat16() for _ in range(3)]
+    mixed = torch.randn(batch, heads, 64, 64, device="cuda").bfloat16()
+    for cache in state:
+        cache[:, :, pos + 1:] = float("nan")               # nothing behind the position may be looked at
+    assert batch * heads > 1184
+
+    def step(part, caches):
+        y = torch.full((qkvgu[part].shape[0], d), float("nan"), device="cuda", dtype=torch.bfloat16)
+        ops.decode_attn(qkvgu[part].contiguous(), *caches, mixed[part].contiguous(), rope, at, heads, y, False)
+        return y
+
+    many = [t.clone() for t in state]
+    y = step(slice(None), many)
+    for first in range(0, batch, 20):                      # at most 640 heads: a CTA for each
+        part = slice(first, first + 20)
+        few = [t[part].clone() for t in state]
+        want = step(part, few)
+        assert torch.allclose(y[part].float(), want.float(), rtol=2 ** -7, atol=1e-4)
+        assert float((y[part].float() - want.float()).norm() / want.float().norm()) < 1e-3
+        for mine, theirs in zip(many, few):
+            assert torch.equal(mine[part].view(torch.int16), theirs.view(torch.int16))

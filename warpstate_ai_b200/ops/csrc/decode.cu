@@ -17,7 +17,7 @@
 //                          GEMMs of the residual stream in one pass, one CTA per sequence.
 //   decode_attn_kernel     one CTA per (sequence, head): RoPE of q/k at the in-chunk position,
 //                          append k/v/u to the chunk cache, causal attention over the cache rows
-//                          <= position, memory read q.M, gate blend.
+//                          <= position, memory read q.M, gate blend.  decode_attn_warp_kernel: a warp for each, where there are many.
 //
 //   decode_norm_gemm_kernel    the residual + norm and the projection that reads it in one launch, for one sequence.
 //
@@ -902,6 +902,163 @@ decode_attn_rows_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bflo
   }
 }
 
+// --------------------------------------------------------------------------- attention step, a warp per head
+// The same for many (sequence, head) pairs: one warp each, four to a CTA.  With a CTA of 128 threads to a pair, 64 sequences x 32 heads are
+// 3.5 rounds of CTAs that meet at six barriers each; here they are one round of warps that meet at none.  Cache rows come 32 at a time,
+// only as many as the position asks for, and the softmax is carried from one 32 to the next (running maximum and sum).  Lane (rg, jg) has
+// the 16-byte piece jg of the rows rg, rg + 4, ...: eight lanes hold a score, all of them its weight, and the sums over rows meet at the end.
+// The first 32 rows of K and V and half of M are requested ahead of the wait where that is allowed (`early`, as above).
+// us a layer with a CTA per pair -> so, at positions 20, 70 and 120: 64 sequences x 32 heads 13.5 -> 7.2, 16.4 -> 12.4, 20.3 -> 15.8; 32 sequences
+// 7.4 -> 5.4, 8.9 -> 9.7, 10.4 -> 11.9; one 2.6 -> 2.4, 2.6 -> 4.1, 2.6 -> 4.8.  So from more than two rounds of CTAs (four to an SM) on.
+constexpr int ATTN_WARPS = 4;
+constexpr int ATTN_ROUND = 148 * 4;   // CTAs of decode_attn_kernel that the chip holds at once
+
+__global__ void __launch_bounds__(32 * ATTN_WARPS, 4)
+decode_attn_warp_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bfloat16* vc, __nv_bfloat16* uc, const __nv_bfloat16* mixed,
+                        const float2* rope, const long long* pos_ptr, int H, int d, int items, __nv_bfloat16* __restrict__ y, bool early) {
+  constexpr int HD = 64, C = 128;
+  __shared__ __align__(16) float query[ATTN_WARPS][HD];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, jg = lane & 7, rg = lane >> 3;
+  const int item = blockIdx.x * ATTN_WARPS + warp;
+  pdl_launch_dependents();
+  if (!early) pdl_wait();
+  if (item >= items) return;
+  const int h = item % H, b = item / H;
+  int pos = static_cast<int>(*pos_ptr);
+  pos = pos < 0 ? 0 : (pos >= C ? C - 1 : pos);
+  const __nv_bfloat16* row = qkvgu + static_cast<size_t>(b) * 5 * d + h * HD;
+  const size_t cache = static_cast<size_t>(item) * C * HD;
+  const __nv_bfloat16* memory = mixed + static_cast<size_t>(item) * HD * HD;
+  uint4 k[8], v[8], m[8];
+  auto request = [&](uint4 (&to)[8], const __nv_bfloat16* from, int r0) {   // rows from `pos` on as zeros
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = r0 + rg + 4 * i;
+      to[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (r < pos) to[i] = *reinterpret_cast<const uint4*>(from + cache + r * HD + jg * 8);
+    }
+  };
+  auto request_memory = [&](int r0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) m[i] = *reinterpret_cast<const uint4*>(memory + (r0 + rg + 4 * i) * HD + jg * 8);
+  };
+  request(k, kc, 0);
+  request(v, vc, 0);
+  request_memory(0);
+  const float2 cs = rope[pos * 32 + lane];
+  if (early) pdl_wait();
+  // RoPE (adjacent pairs) of q and k, rounded through BF16 as the cached / batched path does; k, v, u are appended at `pos`
+  const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(row);
+  const float2 q = __bfloat1622float2(pairs[lane]), kk = __bfloat1622float2(pairs[d / 2 + lane]);
+  const __nv_bfloat162 v_new = pairs[d + lane], u_new = pairs[2 * d + lane];
+  const uint4 own = *reinterpret_cast<const uint4*>(row + 2 * d + jg * 8), gate = *reinterpret_cast<const uint4*>(row + 3 * d + jg * 8);
+  const __nv_bfloat162 qr = __floats2bfloat162_rn(q.x * cs.x - q.y * cs.y, q.y * cs.x + q.x * cs.y);
+  const __nv_bfloat162 kr = __floats2bfloat162_rn(kk.x * cs.x - kk.y * cs.y, kk.y * cs.x + kk.x * cs.y);
+  const float2 qf = __bfloat1622float2(qr), kf = __bfloat1622float2(kr);
+  query[warp][2 * lane] = qf.x;
+  query[warp][2 * lane + 1] = qf.y;
+  *reinterpret_cast<__nv_bfloat162*>(kc + cache + pos * HD + 2 * lane) = kr;
+  *reinterpret_cast<__nv_bfloat162*>(vc + cache + pos * HD + 2 * lane) = v_new;
+  *reinterpret_cast<__nv_bfloat162*>(uc + cache + pos * HD + 2 * lane) = u_new;
+  float top = qf.x * kf.x + qf.y * kf.y;   // the new token's own score, with which the softmax begins
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top += __shfl_xor_sync(0xffffffffu, top, o);
+  top *= 0.125f;
+  __syncwarp();
+  float qv[8];
+  *reinterpret_cast<float4*>(qv) = *reinterpret_cast<const float4*>(&query[warp][jg * 8]);
+  *reinterpret_cast<float4*>(qv + 4) = *reinterpret_cast<const float4*>(&query[warp][jg * 8 + 4]);
+  float sum = 1.f, local[8], mem[8];
+  const __nv_bfloat162* ob = reinterpret_cast<const __nv_bfloat162*>(&own);
+#pragma unroll
+  for (int t = 0; t < 4; ++t) {
+    const float2 f = __bfloat1622float2(ob[t]);
+    local[2 * t] = rg == 0 ? f.x : 0.f;
+    local[2 * t + 1] = rg == 0 ? f.y : 0.f;
+    mem[2 * t] = mem[2 * t + 1] = 0.f;
+  }
+  auto add_memory = [&](int r0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&m[i]);
+      const float qi = query[warp][r0 + rg + 4 * i];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 f = __bfloat1622float2(pb[t]);
+        mem[2 * t] += qi * f.x;
+        mem[2 * t + 1] += qi * f.y;
+      }
+    }
+  };
+  add_memory(0);
+  request_memory(32);
+  for (int r0 = 0; r0 < pos; r0 += 32) {
+    float s[8], most = top;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&k[i]);
+      float acc = 0.f;
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 f = __bfloat1622float2(pb[t]);
+        acc += qv[2 * t] * f.x + qv[2 * t + 1] * f.y;
+      }
+      acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+      acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+      s[i] = r0 + rg + 4 * i < pos ? acc * 0.125f : -INFINITY;
+      most = fmaxf(most, s[i]);
+    }
+    request(k, kc, r0 + 32);   // under the sum over V, as V's next rows are under the scores
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 8));
+    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, 16));
+    const float keep = __expf(top - most);
+    top = most;
+    float here = 0.f;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) local[t] *= keep;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float e = __expf(s[i] - most);
+      here += e;
+      const __nv_bfloat162* pb = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 f = __bfloat1622float2(pb[t]);
+        local[2 * t] += e * f.x;
+        local[2 * t + 1] += e * f.y;
+      }
+    }
+    request(v, vc, r0 + 32);
+    here += __shfl_xor_sync(0xffffffffu, here, 8);
+    here += __shfl_xor_sync(0xffffffffu, here, 16);
+    sum = sum * keep + here;
+  }
+  add_memory(32);
+#pragma unroll
+  for (int t = 0; t < 8; ++t) {
+#pragma unroll
+    for (int o = 8; o < 32; o <<= 1) {
+      local[t] += __shfl_xor_sync(0xffffffffu, local[t], o);
+      mem[t] += __shfl_xor_sync(0xffffffffu, mem[t], o);
+    }
+  }
+  if (rg == 0) {
+    const float inv = 1.f / sum;
+    const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gate);
+    uint4 out;
+    uint32_t* w = reinterpret_cast<uint32_t*>(&out);
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const float2 gf = __bfloat1622float2(gb[t]);
+      const float g0 = sigmoid_fast(gf.x), g1 = sigmoid_fast(gf.y);
+      w[t] = pack_bf16x2(g0 * (local[2 * t] * inv) + (1.f - g0) * (mem[2 * t] * 0.125f),
+                         g1 * (local[2 * t + 1] * inv) + (1.f - g1) * (mem[2 * t + 1] * 0.125f));
+    }
+    *reinterpret_cast<uint4*>(y + static_cast<size_t>(b) * d + h * HD + jg * 8) = out;
+  }
+}
+
 // --------------------------------------------------------------------------- end of a chunk
 // The 128 positions of a finished chunk enter the memories: write = tanh(K)^T tanh(U) / 128, then
 // fast <- df fast + (1 - df) write, slow alike, mixed <- BF16(mix fast + (1 - mix) slow).  One CTA per (sequence, head),
@@ -1232,12 +1389,20 @@ extern "C" int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, c
     const char* e = std::getenv("WS_DECODE_ATTN");
     return e != nullptr && e[0] == 'r';
   }();
-  const cudaError_t err = launch_chained(
-      rows_form ? decode_attn_rows_kernel : decode_attn_kernel, dim3(batch * H), dim3(128), 0, stream,
-      static_cast<const __nv_bfloat16*>(qkvgu),
-      static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc),
-      static_cast<const __nv_bfloat16*>(mixed), reinterpret_cast<const float2*>(rope), pos, H, d,
-      static_cast<__nv_bfloat16*>(y), early != 0);
+  const int items = batch * H;
+  cudaError_t err;
+  if (!rows_form && items > 2 * ATTN_ROUND)
+    err = launch_chained(decode_attn_warp_kernel, dim3((items + ATTN_WARPS - 1) / ATTN_WARPS), dim3(32 * ATTN_WARPS), 0, stream,
+                         static_cast<const __nv_bfloat16*>(qkvgu), static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc),
+                         static_cast<__nv_bfloat16*>(uc), static_cast<const __nv_bfloat16*>(mixed), reinterpret_cast<const float2*>(rope), pos,
+                         H, d, items, static_cast<__nv_bfloat16*>(y), early != 0);
+  else
+    err = launch_chained(
+        rows_form ? decode_attn_rows_kernel : decode_attn_kernel, dim3(items), dim3(128), 0, stream,
+        static_cast<const __nv_bfloat16*>(qkvgu),
+        static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc), static_cast<__nv_bfloat16*>(uc),
+        static_cast<const __nv_bfloat16*>(mixed), reinterpret_cast<const float2*>(rope), pos, H, d,
+        static_cast<__nv_bfloat16*>(y), early != 0);
   ws_count_launch();
   return err == cudaSuccess ? 0 : -21;
 }
