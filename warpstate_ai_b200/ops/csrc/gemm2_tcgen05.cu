@@ -94,6 +94,7 @@ struct alignas(64) PairGroup {
   CUtensorMap whole;   // row selection (problem 0): the operand before its rows were selected
   int tile_start[MAX_GROUP + 1];
   int count;
+  int fetch;           // ACC_F32: the old sums are fetched and stored again, not added to in L2 (see `sums_are_fetched`)
   int ahead;           // B may be read ahead of the launches in front of this one (WsGemm::b_ahead)
 };
 
@@ -439,129 +440,132 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
       }
       if (lane == 0) tma_store_wait_all();
-    } else if constexpr (EPI == WS_EPI_F32 || EPI == WS_EPI_ACC_F32) {
-      // FP32 through shared memory: per warp 32 rows, per step 32 columns, two tiles in flight.  A sum (beta 1) leaves as a
-      // bulk reduction: every element is added to once, in L2, so the result is that of a read, an addition and a write,
-      // but no thread waits for the old value.  Against a thread per row that reads and writes 16 bytes of 32 rows at a time:
-      // 27 M gradients of 1792 tokens 125 -> 85 us, 67 M of 2300 309 -> 237, 0.9 M of 1024 27 -> 16.
-      uint8_t* ebuf = eStage + (warp - 2) * 8192;
-      constexpr int STEPS = (BN / GROUPS) / 32;
-      int q = 0;
-      for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
-        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
-        const GemmParams& p = g.p[t.prob];
-        const int buf_t = tcount & 1;
-        const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
-        tc_fence_after_sync();
-        const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
-        const float alpha = EPI == WS_EPI_ACC_F32 ? p.alpha : 1.f;
-        if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f && p.beta != 1.f) {   // neither a store nor a sum: by row
-          gemm_epilogue<EPI, GROUPS>(p, taddr - egroup * (BN / GROUPS), y + lane, y + lane < p.m, 1.f, t.nb, egroup);
-        } else
+    } else if constexpr (EPI == WS_EPI_F32 || EPI == WS_EPI_RESID_F32 || EPI == WS_EPI_ACC_F32) {
+      if (EPI == WS_EPI_F32 || (EPI == WS_EPI_ACC_F32 && !g.fetch)) {
+        // FP32 through shared memory: per warp 32 rows, per step 32 columns, two tiles in flight.  A sum (beta 1) leaves as a
+        // bulk reduction: every element is added to once, in L2, so the result is that of a read, an addition and a write,
+        // but no thread waits for the old value.  Against a thread per row that reads and writes 16 bytes of 32 rows at a time:
+        // 27 M gradients of 1792 tokens 125 -> 85 us, 67 M of 2300 309 -> 237, 0.9 M of 1024 27 -> 16.
+        uint8_t* ebuf = eStage + (warp - 2) * 8192;
+        constexpr int STEPS = (BN / GROUPS) / 32;
+        int q = 0;
+        for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
+          const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
+          const GemmParams& p = g.p[t.prob];
+          const int buf_t = tcount & 1;
+          const uint32_t tph = (tcount >> 1) & 1;
+          if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
+          tc_fence_after_sync();
+          const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+          const float alpha = EPI == WS_EPI_ACC_F32 ? p.alpha : 1.f;
+          if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f && p.beta != 1.f) {   // neither a store nor a sum: by row
+            gemm_epilogue<EPI, GROUPS>(p, taddr - egroup * (BN / GROUPS), y + lane, y + lane < p.m, 1.f, t.nb, egroup);
+          } else
 #pragma unroll 1
-        for (int step = 0; step < STEPS; ++step, ++q) {
-          const int x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
-          uint8_t* tr = ebuf + (q & 1) * 4096;
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + step * 32, r);
-          if (lane == 0) tma_store_wait_read1();  // the store issued from this tile two steps ago has read it
-          __syncwarp();
-          tmem_ld_wait();
-          if constexpr (EPI == WS_EPI_ACC_F32) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(tile_chunk128(tr, lane, j)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) {
-            if (x < p.n && y < p.m) {
-              if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f) tma_add_2d(&g.epi[t.prob], tr, x, y);
-              else tma_store_2d(&g.epi[t.prob], tr, x, y);
-            }
-            tma_store_commit();
-          }
-        }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
-      }
-      if (lane == 0) tma_store_wait_all();
-    } else if constexpr (EPI == WS_EPI_RESID_F32) {
-      // out = residual + acc through shared memory: per warp 32 rows, per step 32 FP32 columns;
-      // the residual tile is TMA-loaded (double-buffered), updated in place and TMA-stored.
-      uint8_t* ebuf = eStage + (warp - 2) * 8192;  // two buffers of one 4 KiB tile
-      uint64_t* mybar = ebar + (warp - 2) * 2;
-      constexpr int STEPS = (BN / GROUPS) / 32;
-      const GemmParams& p = g.p[0];
-      auto coords = [&](int tile, int step, int& x, int& y) {
-        const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
-        x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
-        y = t.mb * 2 * BM + rank * BM + quarter * 32;
-      };
-      auto issue_load = [&](int tile, int step, int buf) {
-        if (lane == 0) {
-          int x, y;
-          coords(tile, step, x, y);
-          mbar_expect_tx(&mybar[buf], 4096);
-          tma_load_2d(ebuf + buf * 4096, &g.epi[0], &mybar[buf], x, y);
-        }
-      };
-      int q = 0;
-      if (pair_id < tiles) issue_load(pair_id, 0, 0);
-      bool ok = true;
-      for (int tile = pair_id; tile < tiles && ok; tile += num_pairs, ++tcount) {
-        const int buf_t = tcount & 1;
-        const uint32_t tph = (tcount >> 1) & 1;
-        if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
-        tc_fence_after_sync();
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
-#pragma unroll 1
-        for (int step = 0; step < STEPS; ++step, ++q) {
-          const int buf = q & 1;
-          if (lane == 0) tma_store_wait_read0();
-          if (step + 1 < STEPS) {
-            issue_load(tile, step + 1, buf ^ 1);
-          } else if (tile + num_pairs < tiles) {
-            issue_load(tile + num_pairs, 0, buf ^ 1);
-          }
-          uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + step * 32, r);
-          if (!mbar_wait_warp(&mybar[buf], (q >> 1) & 1, abort_flag)) {
-            ok = false;
+          for (int step = 0; step < STEPS; ++step, ++q) {
+            const int x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+            uint8_t* tr = ebuf + (q & 1) * 4096;
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + step * 32, r);
+            if (lane == 0) tma_store_wait_read1();  // the store issued from this tile two steps ago has read it
+            __syncwarp();
             tmem_ld_wait();
-            break;
-          }
-          tmem_ld_wait();
-          uint8_t* tr = ebuf + buf * 4096;
+            if constexpr (EPI == WS_EPI_ACC_F32) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float4* pv = reinterpret_cast<float4*>(tile_chunk128(tr, lane, j));
-            float4 v = *pv;
-            v.x += __uint_as_float(r[4 * j]);
-            v.y += __uint_as_float(r[4 * j + 1]);
-            v.z += __uint_as_float(r[4 * j + 2]);
-            v.w += __uint_as_float(r[4 * j + 3]);
-            *pv = v;
+              for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(tile_chunk128(tr, lane, j)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              if (x < p.n && y < p.m) {
+                if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f) tma_add_2d(&g.epi[t.prob], tr, x, y);
+                else tma_store_2d(&g.epi[t.prob], tr, x, y);
+              }
+              tma_store_commit();
+            }
           }
-          fence_proxy_async_smem();
+          tc_fence_before_sync();
           __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
+        }
+        if (lane == 0) tma_store_wait_all();
+      } else {
+        // out = residual + acc through shared memory (or sum + alpha acc, in place): per warp 32 rows, per step 32 FP32 columns;
+        // the residual tile is TMA-loaded (double-buffered), updated in place and TMA-stored.
+        uint8_t* ebuf = eStage + (warp - 2) * 8192;  // two buffers of one 4 KiB tile
+        uint64_t* mybar = ebar + (warp - 2) * 2;
+        constexpr int STEPS = (BN / GROUPS) / 32;
+        auto coords = [&](int tile, int step, int& x, int& y) {
+          const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
+          x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+          y = t.mb * 2 * BM + rank * BM + quarter * 32;
+          return t.prob;
+        };
+        auto issue_load = [&](int tile, int step, int buf) {
           if (lane == 0) {
             int x, y;
-            coords(tile, step, x, y);
-            if (x < p.n && y < p.m) tma_store_2d(&g.epi[1], tr, x, y);
-            tma_store_commit();
+            const int prob = coords(tile, step, x, y);
+            mbar_expect_tx(&mybar[buf], 4096);
+            tma_load_2d(ebuf + buf * 4096, &g.epi[EPI == WS_EPI_ACC_F32 ? prob : 0], &mybar[buf], x, y);
           }
+        };
+        int q = 0;
+        if (pair_id < tiles) issue_load(pair_id, 0, 0);
+        bool ok = true;
+        for (int tile = pair_id; tile < tiles && ok; tile += num_pairs, ++tcount) {
+          const int buf_t = tcount & 1;
+          const uint32_t tph = (tcount >> 1) & 1;
+          if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
+          tc_fence_after_sync();
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+          const float alpha = EPI == WS_EPI_ACC_F32 ? g.p[resolve_tile(g, extent, tile, n_tile, GATHER).prob].alpha : 1.f;
+#pragma unroll 1
+          for (int step = 0; step < STEPS; ++step, ++q) {
+            const int buf = q & 1;
+            if (lane == 0) tma_store_wait_read0();
+            if (step + 1 < STEPS) {
+              issue_load(tile, step + 1, buf ^ 1);
+            } else if (tile + num_pairs < tiles) {
+              issue_load(tile + num_pairs, 0, buf ^ 1);
+            }
+            uint32_t r[32];
+            tmem_ld_32x32b_x32(taddr + step * 32, r);
+            if (!mbar_wait_warp(&mybar[buf], (q >> 1) & 1, abort_flag)) {
+              ok = false;
+              tmem_ld_wait();
+              break;
+            }
+            tmem_ld_wait();
+            uint8_t* tr = ebuf + buf * 4096;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              float4* pv = reinterpret_cast<float4*>(tile_chunk128(tr, lane, j));
+              float4 v = *pv;
+              v.x = __fadd_rn(v.x, __fmul_rn(__uint_as_float(r[4 * j]), alpha));
+              v.y = __fadd_rn(v.y, __fmul_rn(__uint_as_float(r[4 * j + 1]), alpha));
+              v.z = __fadd_rn(v.z, __fmul_rn(__uint_as_float(r[4 * j + 2]), alpha));
+              v.w = __fadd_rn(v.w, __fmul_rn(__uint_as_float(r[4 * j + 3]), alpha));
+              *pv = v;
+            }
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              int x, y;
+              const int prob = coords(tile, step, x, y);
+              if (x < g.p[prob].n && y < g.p[prob].m) tma_store_2d(&g.epi[EPI == WS_EPI_ACC_F32 ? prob : 1], tr, x, y);
+              tma_store_commit();
+            }
+          }
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
         }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(mapa_shared(smem_u32(&tempty[buf_t]), 0));
+        if (lane == 0) tma_store_wait_all();
       }
-      if (lane == 0) tma_store_wait_all();
     } else if constexpr (STAGED) {
       // SwiGLU backward through shared memory.  Per warp: 32 rows; per step: 32 columns; two
       // buffers, each holding the (up, gate) tiles that become (dUp, dGate) in place.
@@ -1072,6 +1076,22 @@ extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part,
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
+// How weight gradients (beta 1) are added to.  As bulk reductions they cost no round trip, and a tile's epilogue is over once it has
+// handed them on; but L2 takes them at about 1.3 TB/s, and a tile of few k-blocks waits for that.  Fetched, added to in shared memory
+// and stored they move at the rate of copies.  Same bits.  Reduced -> fetched, us: the four gradients of a block of width 2048 at 256
+// rows 129 -> 112, 512 134 -> 119, 1024 165 -> 151, 2048 247 -> 243, 4096 424 -> 427; 1280 at 256 49 -> 52, 512 56 -> 54, 896 65 -> 60, 1280 74 ->
+// 73, 1792 91 -> 92; 256 at 1024 16 -> 17; a head of 32768 x 2048 at 512 125 -> 110, 1024 154 -> 134, 2304 249 -> 248, 8192 742 -> 765, of
+// 32768 x 1280 at 1024 111 -> 92, of 32768 x 256 26 -> 30.  So up to 24 k-blocks where the tiles are four rounds, and below eight
+// only where the sums lie outside L2.
+static bool sums_are_fetched(const WsGemm* items, int count, int tiles, int sms) {
+  long long sums = 0;
+  for (int i = 0; i < count; ++i) {
+    if (items[i].beta != 1.f || items[i].k > 1536) return false;   // with selected rows k is the most there can be
+    sums += static_cast<long long>(items[i].m) * items[i].n;
+  }
+  return tiles >= 4 * (sms / 2) && (items[0].k >= 512 || sums > (32ll << 20));
+}
+
 // `count` problems (1..4) of one kind (same operand majors and epilogue) in one launch.  The
 // argument checks of ws_gemm have already run on every item; `sms` bounds the SMs used.
 // Returns -6 for a combination this kernel does not build.
@@ -1092,6 +1112,7 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
     total += tiles;
   }
   for (int i = count; i <= MAX_GROUP; ++i) grp.tile_start[i] = total;
+  grp.fetch = items[0].epilogue == WS_EPI_ACC_F32 && sums_are_fetched(items, count, total, sms);
   grp.ahead = !items[0].a_mn && !items[0].b_mn && items[0].limit == nullptr;
   for (int i = 0; i < count; ++i) grp.ahead = grp.ahead && items[i].b_ahead;
   if (items[0].epilogue == WS_EPI_F32 || items[0].epilogue == WS_EPI_ACC_F32) {
