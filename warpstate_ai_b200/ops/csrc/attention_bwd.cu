@@ -14,6 +14,7 @@
 //
 // All ten matrix products of the tile run on tcgen05 with accumulators in TMEM; one thread owns
 // one token row in every element-wise stage.
+#include <type_traits>
 #include "ws_ptx.cuh"
 #include "ws_api.h"
 #include "ws_launch.h"
@@ -327,106 +328,175 @@ constexpr int SCAN_MAX_CHUNKS = SCAN_GROUP * SCAN_MAX_GROUPS;  // 32768 tokens p
 
 // dstate [B,N,H,4096] FP32 (gradient of the mixed state read by chunk n), writes [B,N,H,4096] FP32
 // -> dwrites [B,N,H,4096] BF16 and partial sums [B*H*16][3] of d(fast decay), d(slow decay), d(mix).
-// A thread owns two neighbouring state elements (8-byte loads of the writes and of the state gradients, 4-byte stores):
-// half the memory instructions of the one-element form, and 256 bytes in flight per thread, three blocks per SM.  At
-// 4 x 16 chunks x 32 heads it takes 29.3 us (84 MB); the whole block's forward + backward went from 273 to 267 us.
+// A thread owns two neighbouring state elements of each unit (SCAN_THREADS threads' worth), one operand of its packed
+// instructions.  Bound by DRAM: 10 bytes an element and chunk.  Persistent, three CTAs per SM: while a warp walks one group of
+// chunks, what it needs of its next group (the next unit's, after the last) is on its way into its own places in shared memory,
+// so no barrier of the block is needed.  Such a copy has to pass L1 by: with 192 KiB taken as shared memory L1 is so small that
+// copies through it (8 bytes a thread) waited for its lines, 24.7 us at 4 x 16 chunks x 32 heads.  Now 16.5 us (84 MB, 5.1 TB/s),
+// 8 x 16 x 32 29.1 (5.8 TB/s), 2 x 7 x 20 5.0; a block per unit that loaded into registers, computed and left took 27.1, 50.2
+// and 5.8.
 constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_VEC = 2;
+constexpr int SCAN_SLOT = 2 * SCAN_GROUP * SCAN_THREADS;   // pairs: the writes and the state gradients of a group
+constexpr int SCAN_SMEM = 2 * SCAN_SLOT * 8;
+
+// Two FP32 numbers in a register pair, the first in the low half; every operation rounds each of them once.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pair2(float lo, float hi) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+  return d;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 d;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+  return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
 
 __global__ void __launch_bounds__(SCAN_THREADS, 3)
 memory_scan_bwd_kernel(const float* dstate, const float* writes,
                        const float* fast_logit, const float* slow_logit,
                        const float* mix_logit, __nv_bfloat16* __restrict__ dwrites,
                        float* __restrict__ partials, int B, int N, int H) {
+  extern __shared__ __align__(16) uint8_t scan_smem[];
+  __shared__ float red[2][3][SCAN_THREADS / 32];
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float red[3][SCAN_THREADS / 32];
-  const size_t idx = (blockIdx.x * static_cast<size_t>(SCAN_THREADS) + threadIdx.x) * SCAN_VEC;  // over B*H*4096 (exact multiple)
-  const int e = idx % 4096;
-  const int h = (idx / 4096) % H;
-  const int b = idx / (4096 * static_cast<size_t>(H));
-  const float df = 1.f / (1.f + expf(-fast_logit[h]));
-  const float ds = 1.f / (1.f + expf(-slow_logit[h]));
-  const float mix = 1.f / (1.f + expf(-mix_logit[h]));
-  const size_t chunk_stride = static_cast<size_t>(H) * 4096;
-  const size_t base = (static_cast<size_t>(b) * N * H + h) * 4096 + e;  // chunk 0 of these elements
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int units = B * H * 16;
   const int groups = (N + SCAN_GROUP - 1) / SCAN_GROUP;
-  float2 start_f[SCAN_MAX_GROUPS], start_s[SCAN_MAX_GROUPS];
-  auto advance = [&](float2& f, float2& s, const float2& w) {
-    f.x = df * f.x + (1.f - df) * w.x;
-    f.y = df * f.y + (1.f - df) * w.y;
-    s.x = ds * s.x + (1.f - ds) * w.x;
-    s.y = ds * s.y + (1.f - ds) * w.y;
+  const int pieces = 2 * groups - 1;   // of a unit: the first pass over all groups but the last, then every group, the last one first
+  const size_t chunk_stride = static_cast<size_t>(H) * 4096;
+  f32x2* const mine = reinterpret_cast<f32x2*>(scan_smem) + tid;
+  auto place = [&](int unit) {   // chunk 0 of this warp's elements
+    const int head = unit >> 4;
+    return (static_cast<size_t>(head / H) * N * H + head % H) * 4096 + (unit & 15) * (SCAN_THREADS * SCAN_VEC) + warp * (32 * SCAN_VEC);
   };
-  {
-    float2 f = make_float2(0.f, 0.f), s = f;
-#pragma unroll 1
-    for (int g = 0; g < groups; ++g) {
-      start_f[g] = f;
-      start_s[g] = s;
-      if (g + 1 < groups) {
-#pragma unroll
-        for (int i = 0; i < SCAN_GROUP; ++i)
-          advance(f, s, *reinterpret_cast<const float2*>(writes + base + (g * SCAN_GROUP + i) * chunk_stride));
-      }
-    }
-  }
-  // a, bb: gradients of the fast and slow state AFTER the chunk being visited (F_{n+1}, S_{n+1})
-  float2 a = make_float2(0.f, 0.f), bb = a;
-  float g_df = 0.f, g_ds = 0.f, g_mix = 0.f;
-#pragma unroll 1
-  for (int g = groups - 1; g >= 0; --g) {
-    const int n0 = g * SCAN_GROUP;
-    const int count = min(SCAN_GROUP, N - n0);
-    // every load of the group is requested before its recurrences run: 2 x SCAN_GROUP independent loads in flight
-    float2 F[SCAN_GROUP], S[SCAN_GROUP], W[SCAN_GROUP], G[SCAN_GROUP];
+  auto group_of = [&](int piece) { return piece < groups - 1 ? piece : pieces - 1 - piece; };
+  // a warp fetches its own 64 elements of every chunk, one half of it those of the writes, the other those of the gradients
+  const int half = lane >> 4;
+  const float* const from = half == 0 ? writes : dstate;
+  const uint32_t into = smem_u32(scan_smem) + half * (SCAN_GROUP * SCAN_THREADS * 8) + warp * 256 + (lane & 15) * 16;
+  auto request = [&](int unit, int piece, int slot) {
+    const int n0 = group_of(piece) * SCAN_GROUP;
+    const int count = half == 0 || piece >= groups - 1 ? min(SCAN_GROUP, N - n0) : 0;
+    const float* at = from + place(unit) + n0 * chunk_stride + (lane & 15) * 4;
+    const uint32_t to = into + slot * (SCAN_SLOT * 8);
 #pragma unroll
     for (int i = 0; i < SCAN_GROUP; ++i) {
-      if (i < count) {
-        W[i] = *reinterpret_cast<const float2*>(writes + base + (n0 + i) * chunk_stride);
-        G[i] = *reinterpret_cast<const float2*>(dstate + base + (n0 + i) * chunk_stride);
-      }
+      if (i < count) cp_async_16(to + i * (SCAN_THREADS * 8), at);
+      at += chunk_stride;
+      asm volatile("" : "+l"(at));   // one address that moves on, not sixteen kept from unit to unit
     }
-    float2 f = start_f[g], s = start_s[g];
-#pragma unroll
-    for (int i = 0; i < SCAN_GROUP; ++i) {  // forward: state seen by chunk n0 + i
-      if (i < count) {
-        F[i] = f;
-        S[i] = s;
-        advance(f, s, W[i]);
-      }
-    }
-#pragma unroll
-    for (int i = SCAN_GROUP - 1; i >= 0; --i) {
-      if (i < count) {
-        *reinterpret_cast<uint32_t*>(dwrites + base + (n0 + i) * chunk_stride) =
-            pack_bf16x2((1.f - df) * a.x + (1.f - ds) * bb.x, (1.f - df) * a.y + (1.f - ds) * bb.y);
-        g_df += a.x * (F[i].x - W[i].x) + a.y * (F[i].y - W[i].y);    // F_{n+1} = df F_n + (1 - df) w_n
-        g_ds += bb.x * (S[i].x - W[i].x) + bb.y * (S[i].y - W[i].y);
-        g_mix += G[i].x * (F[i].x - S[i].x) + G[i].y * (F[i].y - S[i].y);
-        a.x = mix * G[i].x + df * a.x;      // gradient of F_n
-        a.y = mix * G[i].y + df * a.y;
-        bb.x = (1.f - mix) * G[i].x + ds * bb.x;
-        bb.y = (1.f - mix) * G[i].y + ds * bb.y;
-      }
-    }
+  };
+  f32x2 start_f[SCAN_MAX_GROUPS], start_s[SCAN_MAX_GROUPS];
+  float next_fast = 0.f, next_slow = 0.f, next_mix = 0.f;
+  auto request_logits = [&](int unit) {
+    const int h = (unit >> 4) % H;
+    next_fast = fast_logit[h];
+    next_slow = slow_logit[h];
+    next_mix = mix_logit[h];
+  };
+  int slot = 0, turn = 0;
+  if (blockIdx.x < units) {
+    request_logits(blockIdx.x);
+    request(blockIdx.x, 0, 0);
   }
-  // block reduction (fixed order)
-  float vals[3] = {g_df, g_ds, g_mix};
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cp_async_commit();
+  for (int unit = blockIdx.x; unit < units; unit += gridDim.x, turn ^= 1) {
+    const float df1 = 1.f / (1.f + expf(-next_fast)), ds1 = 1.f / (1.f + expf(-next_slow)), mix1 = 1.f / (1.f + expf(-next_mix));
+    const f32x2 df = pair2(df1, df1), ds = pair2(ds1, ds1), mix = pair2(mix1, mix1), minus = pair2(-1.f, -1.f);
+    const f32x2 rf = pair2(1.f - df1, 1.f - df1), rs = pair2(1.f - ds1, 1.f - ds1), rm = pair2(1.f - mix1, 1.f - mix1);
+    __nv_bfloat16* const out = dwrites + place(unit) + lane * SCAN_VEC;
+    f32x2 f = 0, s = 0;
+    // a, bb: gradients of the fast and slow state AFTER the chunk being visited (F_{n+1}, S_{n+1})
+    f32x2 a = 0, bb = 0, g_df = 0, g_ds = 0, g_mix = 0;
+#pragma unroll 1
+    for (int piece = 0; piece < pieces; ++piece, slot ^= 1) {
+      __syncwarp();   // every lane has done with the slot that is filled next
+      const int to_come = piece + 1 < pieces ? unit : unit + static_cast<int>(gridDim.x);
+      if (to_come < units) {
+        if (to_come != unit) request_logits(to_come);
+        request(to_come, to_come == unit ? piece + 1 : 0, slot ^ 1);
+      }
+      cp_async_commit();
+      cp_async_wait<1>();   // this piece is there, the next one on its way
+      __syncwarp();         // and the other lanes' part of it
+      const int g = group_of(piece), n0 = g * SCAN_GROUP;
+      const int count = min(SCAN_GROUP, N - n0);
+      const f32x2 *W = mine + slot * SCAN_SLOT, *G = W + SCAN_GROUP * SCAN_THREADS;
+      auto advance = [&](f32x2 w) {
+        f = fma2(df, f, mul2(rf, w));
+        s = fma2(ds, s, mul2(rs, w));
+      };
+      if (piece < groups - 1) {
+        start_f[g] = f;
+        start_s[g] = s;
 #pragma unroll
-  for (int q = 0; q < 3; ++q) {
-    float v = vals[q];
+        for (int i = 0; i < SCAN_GROUP; ++i) advance(W[i * SCAN_THREADS]);
+        continue;
+      }
+      if (g < groups - 1) {   // the last group goes on from the first pass
+        f = start_f[g];
+        s = start_s[g];
+      }
+      auto walk = [&](auto whole) {
+        f32x2 F[SCAN_GROUP], S[SCAN_GROUP];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[q][warp] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    float v = 0.f;
+        for (int i = 0; i < SCAN_GROUP; ++i) {  // forward: state seen by chunk n0 + i
+          if (whole.value || i < count) {
+            F[i] = f;
+            S[i] = s;
+            advance(W[i * SCAN_THREADS]);
+          }
+        }
+        __nv_bfloat16* to = out + (n0 + count - 1) * chunk_stride;
 #pragma unroll
-    for (int wi = 0; wi < SCAN_THREADS / 32; ++wi) v += red[threadIdx.x][wi];
-    partials[static_cast<size_t>(blockIdx.x) * 3 + threadIdx.x] = v;
+        for (int i = SCAN_GROUP - 1; i >= 0; --i) {
+          if (whole.value || i < count) {
+            const f32x2 w = W[i * SCAN_THREADS], gr = G[i * SCAN_THREADS];
+            const float2 dw = halves(fma2(rf, a, mul2(rs, bb)));
+            *reinterpret_cast<uint32_t*>(to) = pack_bf16x2(dw.x, dw.y);
+            to -= chunk_stride;
+            asm volatile("" : "+l"(to));   // as above
+            g_df = fma2(a, fma2(w, minus, F[i]), g_df);    // F_{n+1} = df F_n + (1 - df) w_n
+            g_ds = fma2(bb, fma2(w, minus, S[i]), g_ds);
+            g_mix = fma2(gr, fma2(S[i], minus, F[i]), g_mix);
+            a = fma2(mix, gr, mul2(df, a));                // gradient of F_n
+            bb = fma2(rm, gr, mul2(ds, bb));
+          }
+        }
+      };
+      if (count == SCAN_GROUP) walk(std::true_type());
+      else walk(std::false_type());
+    }
+    // block reduction (fixed order)
+    const float2 of_f = halves(g_df), of_s = halves(g_ds), of_mix = halves(g_mix);
+    const float vals[3] = {of_f.x + of_f.y, of_s.x + of_s.y, of_mix.x + of_mix.y};
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      float v = vals[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0) red[turn][q][warp] = v;
+    }
+    __syncthreads();   // the other half of `red` is written before the next one of these, this half only after it
+    if (tid < 3) {
+      float v = 0.f;
+#pragma unroll
+      for (int wi = 0; wi < SCAN_THREADS / 32; ++wi) v += red[turn][tid][wi];
+      partials[static_cast<size_t>(unit) * 3 + tid] = v;
+    }
   }
 }
 
@@ -988,10 +1058,17 @@ extern "C" int ws_memory_scan_bwd(const float* dstate, const float* writes, cons
                                   const float* slow_logit, const float* mix_logit, void* dwrites, float* partials,
                                   int B, int N, int H, cudaStream_t stream) {
   if (N > SCAN_MAX_CHUNKS) return -1;
-  const size_t total = (size_t)B * H * 4096;
-  launch_dependent(memory_scan_bwd_kernel, dim3((unsigned)(total / (SCAN_THREADS * SCAN_VEC))), dim3(SCAN_THREADS), 0, stream, dstate, writes, fast_logit, slow_logit,
-                                                                      mix_logit, (__nv_bfloat16*)dwrites, partials,
-                                                                      B, N, H);
+  static int sms = 0;
+  if (sms == 0) {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(memory_scan_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) != cudaSuccess)
+      return -20;
+    sms = n;
+  }
+  const int units = B * H * 16;
+  launch_dependent(memory_scan_bwd_kernel, dim3(units < 3 * sms ? units : 3 * sms), dim3(SCAN_THREADS), SCAN_SMEM, stream, dstate, writes,
+                   fast_logit, slow_logit, mix_logit, (__nv_bfloat16*)dwrites, partials, B, N, H);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

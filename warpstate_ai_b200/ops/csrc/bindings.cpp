@@ -415,7 +415,9 @@ std::tuple<at::Tensor, at::Tensor> attn_bwd(const at::Tensor& qkvgu, const at::T
                           (int)T, (int)H, (int)d, err, cur_stream()), "attn_dstate");
   at::Tensor dwrites = at::empty({B, N, H, 64, 64}, qkvgu.options());
   at::Tensor partials = at::empty({B * H * 16, 3}, qkvgu.options().dtype(at::kFloat));
-  check_rc(ws_memory_scan_bwd(dstate.data_ptr<float>(), writes.data_ptr<float>(), fast_logit.data_ptr<float>(),
+  // the scan fetches 16 bytes at a time
+  const at::Tensor aligned = reinterpret_cast<uintptr_t>(writes.data_ptr()) % 16 == 0 ? writes : writes.clone();
+  check_rc(ws_memory_scan_bwd(dstate.data_ptr<float>(), aligned.data_ptr<float>(), fast_logit.data_ptr<float>(),
                               slow_logit.data_ptr<float>(), mix_logit.data_ptr<float>(), dwrites.data_ptr(),
                               partials.data_ptr<float>(), (int)B, (int)N, (int)H, cur_stream()), "memory_scan_bwd");
   at::Tensor dqkvgu = at::empty_like(qkvgu);

@@ -208,7 +208,8 @@ int ws_attn_fwd(const void* qkvgu, const void* states, const float* rope, void* 
 // Backward of the same block.  dy: BF16 [B*T, d].  dstate: FP32 [B,N,H,64,64].
 int ws_attn_dstate(const void* qkvgu, const void* dy, const float* rope, float* dstate, int B, int T, int H,
                    int d, int* error_flag, cudaStream_t stream);
-// dwrites: BF16 [B,N,H,64,64]; partials: FP32 [B*H*16][3] (d fast decay, d slow decay, d mix); N <= 64.
+// dwrites: BF16 [B,N,H,64,64]; partials: FP32 [B*H*16][3] (d fast decay, d slow decay, d mix); N <= 256; dstate and
+// writes aligned to 16 bytes.
 int ws_memory_scan_bwd(const float* dstate, const float* writes, const float* fast_logit,
                        const float* slow_logit, const float* mix_logit, void* dwrites, float* partials,
                        int B, int N, int H, cudaStream_t stream);

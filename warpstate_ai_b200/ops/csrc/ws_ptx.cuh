@@ -89,6 +89,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Copies of 16 bytes to shared memory that hold no register and no line of L1 on their way (both addresses aligned to them).  The
+// thread that asked may read them after cp_async_wait, the other lanes of its warp after a __syncwarp behind that.
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
 // ----------------------------------------------------------------------------- TMA
 // Plain (single-CTA destination) tiled loads.  The innermost coordinate times the element
 // size must be a multiple of 16 bytes; callers guarantee that by construction.
