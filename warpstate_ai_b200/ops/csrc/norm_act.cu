@@ -204,9 +204,15 @@ rmsnorm_fwd_block_kernel(const T* x, const float* col_scale, const float* col_bi
 // dw_partial[block] = sum over the block's rows of dz * x_hat.
 //
 // Column-owner layout: thread t owns columns 8t .. 8t+7 (256 threads cover d <= 2048) and the
-// block walks over groups of RB_ROWS rows, so every operand is read from global memory exactly
-// once with 16/32-byte coalesced accesses, the per-row mean needs one block reduction per group
+// block walks over pairs of rows, so every operand is read from global memory exactly
+// once, the per-row mean needs one block reduction per step of one or two rows
 // (double-buffered, one __syncthreads), and the weight-gradient column sums stay in 8 registers.
+//
+// Bound by DRAM (14 bytes an element, 470 MB at 16384 x 2048: 72 us at the rate of a copy).  While a block has a step of rows in
+// hand, the rows of its next steps are on their way into shared memory, past L1 and without registers; requested into registers
+// in one step and used in the next, behind the barrier and the stores of the step before, they came at 4.7 TB/s.  16384 x 2048: 97 -> 82 us,
+// MOD 100 -> 76; 8192 x 1280 45 -> 29 and 45 -> 31; BF16 stream 76 -> 59 (alone, in a chain of launches).  In a block's backward pass:
+// 1792 x 1280 11.8 -> 8.8 us and 11.7 -> 9.3, 128 x 2048 4.6 -> 3.7 and 4.8 -> 4.6.
 //
 // MOD (FP32 stream, the norm behind a depth modulation xmod = x * (1 + scale) + bias): `x` is the modulation's input and
 // xmod is formed again from it.  The gradients of scale and bias are column sums of dxmod * x and dxmod, and dxmod is in
@@ -227,20 +233,91 @@ __device__ __forceinline__ void st8(T* p, const float (&v)[8]) {
   st4(p + 4, make_float4(v[4], v[5], v[6], v[7]));
 }
 
-template <typename T, bool MOD = false>
-__global__ void __launch_bounds__(ROW_THREADS, MOD ? 2 : 3)
+// DEPTH steps of STEP rows of dz, x, dres and rstd in shared memory; a warp fetches its own 256 columns of each.
+template <typename T, bool MOD, int STEP>
+struct NormBackward {
+  static constexpr int BF16_BYTES = ROW_THREADS * 16, T_BYTES = ROW_THREADS * 8 * (int)sizeof(T);
+  static constexpr int SLOT = BF16_BYTES + 2 * T_BYTES + ROW_THREADS * 4;   // a row
+  static constexpr int BLOCKS_PER_SM = STEP == 2 ? 2 : 3;
+  static constexpr int DEPTH = STEP == 2 ? 2 : 3;
+  static constexpr int SMEM = DEPTH * STEP * SLOT;
+};
+
+// Eight columns of a lane, and how its warp's 256 of them get there: 16 bytes a lane in the order of memory, so that a request covers
+// whole sectors.  FP32: two rounds, and the pieces' low bit flipped in every other eight, so that lanes that read 32 bytes each do
+// not meet in a bank.
+__device__ __forceinline__ void fetch_columns(uint32_t warp_to, int lane, const float* warp_from, int columns, bool) {
+#pragma unroll
+  for (int p = lane; p < 64; p += 32)
+    if (p * 4 < columns) cp_async_16(warp_to + ((p ^ ((p >> 3) & 1)) << 4), warp_from + p * 4);
+}
+__device__ __forceinline__ void fetch_columns(uint32_t warp_to, int lane, const __nv_bfloat16* warp_from, int columns, bool whole) {
+  if (lane * 8 >= columns) return;
+  const __nv_bfloat16* from = warp_from + lane * 8;
+  if (whole) {
+    cp_async_16(warp_to + lane * 16, from);
+  } else {   // BF16 operands may begin at any 8 bytes
+    cp_async_small<8>(warp_to + lane * 16, from);
+    cp_async_small<8>(warp_to + lane * 16 + 8, from + 4);
+  }
+}
+__device__ __forceinline__ void fetched_columns(uint32_t warp_at, int lane, float (&v)[8], float) {
+  const uint32_t at = warp_at + lane * 32, flip = ((lane >> 2) & 1) << 4;
+  float4 a, b;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w) : "r"(at ^ flip) : "memory");
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "r"((at ^ flip) ^ 16) : "memory");
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void fetched_columns(uint32_t warp_at, int lane, float (&v)[8], __nv_bfloat16) {
+  uint32_t w[4];
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(warp_at + lane * 16) : "memory");
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
+    v[2 * j] = a.x;
+    v[2 * j + 1] = a.y;
+  }
+}
+
+template <typename T, bool MOD, int STEP>
+__global__ void __launch_bounds__(ROW_THREADS, (NormBackward<T, MOD, STEP>::BLOCKS_PER_SM))
 rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
                    const float* rstd_in, const float* w,
                    const T* dres, const float* out_scale, int rows, int d,
                    T* __restrict__ dx_out, __nv_bfloat16* __restrict__ dx_bf16,
                    float* __restrict__ dw_partial, const float* mod_bias) {
+  using Cfg = NormBackward<T, MOD, STEP>;
+  extern __shared__ __align__(16) uint8_t ring[];
+  __shared__ float red[2][STEP][ROW_WARPS];
   pdl_launch_dependents();
   pdl_wait();
-  __shared__ float red[2][RB_ROWS][ROW_WARPS];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = threadIdx.x * 8;
   const bool active = c < d;
   const float inv_d = 1.0f / static_cast<float>(d);
+  const int columns = d - warp * 256;   // the warp's, at most 256 of them
+  const uint32_t at_dz = smem_u32(ring) + warp * 512, at_x = smem_u32(ring) + Cfg::BF16_BYTES + warp * (256 * (int)sizeof(T));
+  const uint32_t at_dres = at_x + Cfg::T_BYTES, at_rstd = smem_u32(ring) + Cfg::BF16_BYTES + 2 * Cfg::T_BYTES + threadIdx.x * 4;
+  const bool whole = (reinterpret_cast<uintptr_t>(dz) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dres)) % 16 == 0;
+  // this block's k-th row: pairs of neighbours, the blocks' pairs by turns
+  auto row_of = [&](int k) { return (static_cast<int>(blockIdx.x) + (k / RB_ROWS) * static_cast<int>(gridDim.x)) * RB_ROWS + k % RB_ROWS; };
+  auto request = [&](int k, int slot) {
+#pragma unroll
+    for (int r = 0; r < STEP; ++r) {
+      const int row = row_of(k + r);
+      if (row < rows && columns > 0) {
+        const size_t base = static_cast<size_t>(row) * d + warp * 256;
+        const uint32_t at = (slot * STEP + r) * Cfg::SLOT;
+        fetch_columns(at_dz + at, lane, dz + base, columns, whole);
+        fetch_columns(at_x + at, lane, x + base, columns, whole);
+        if (dres != nullptr) fetch_columns(at_dres + at, lane, dres + base, columns, whole);
+        cp_async_small<4>(at_rstd + at, rstd_in + row);
+      }
+    }
+    cp_async_commit();
+  };
+#pragma unroll
+  for (int n = 0; n < Cfg::DEPTH - 1; ++n) request(n * STEP, n);
   float wv[8], sv[8], acc[8];
   [[maybe_unused]] float bi[8], acc_bias[8], acc_scale[8];
 #pragma unroll
@@ -254,51 +331,44 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
       for (int j = 0; j < 8; ++j) sv[j] += 1.f;
     }
   }
-  int it = 0;
-  for (int row0 = blockIdx.x * RB_ROWS; row0 < rows; row0 += gridDim.x * RB_ROWS, ++it) {
-    float g[RB_ROWS][8], xh[RB_ROWS][8], rs[RB_ROWS], part[RB_ROWS];
+  int slot = 0, turn = 0;
+  for (int k = 0; row_of(k) < rows; k += STEP, turn ^= 1) {
+    __syncwarp();   // every lane has read the rows before these
+    request(k + (Cfg::DEPTH - 1) * STEP, slot == 0 ? Cfg::DEPTH - 1 : slot - 1);   // into their place
+    cp_async_wait<Cfg::DEPTH - 1>();
+    __syncwarp();
+    float g[STEP][8], xh[STEP][8], rs[STEP];
 #pragma unroll
-    for (int r = 0; r < RB_ROWS; ++r) {
-      const int row = row0 + r;
-      part[r] = 0.f;
+    for (int r = 0; r < STEP; ++r) {
+      const uint32_t at = (slot * STEP + r) * Cfg::SLOT;
+      float part = 0.f;
       rs[r] = 0.f;
-      if (row < rows && active) {
-        const size_t base = static_cast<size_t>(row) * d + c;
-        ld8(dz + base, g[r]);
-        ld8(x + base, xh[r]);
-        rs[r] = rstd_in[row];
+      if (active && row_of(k + r) < rows) {
+        fetched_columns(at_dz + at, lane, g[r], __nv_bfloat16());
+        fetched_columns(at_x + at, lane, xh[r], T());
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(rs[r]) : "r"(at_rstd + at) : "memory");
       } else {
 #pragma unroll
         for (int j = 0; j < 8; ++j) { g[r][j] = 0.f; xh[r][j] = 0.f; }
       }
-    }
-#pragma unroll
-    for (int r = 0; r < RB_ROWS; ++r) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         if constexpr (MOD) xh[r][j] = xh[r][j] * sv[j] + bi[j];
         xh[r][j] *= rs[r];
-        part[r] += g[r][j] * wv[j] * xh[r][j];
+        part += g[r][j] * wv[j] * xh[r][j];
       }
-      part[r] = warp_sum(part[r]);
-      if (lane == 0) red[it & 1][r][warp] = part[r];
+      part = warp_sum(part);
+      if (lane == 0) red[turn][r][warp] = part;
     }
     __syncthreads();
-    // MOD has the registers to request both rows' before the first store, which a load does not pass (16384 x 2048: 112.7 ->
-    // 102.2 us); at three blocks per SM they would be spilled.
-    [[maybe_unused]] float both[MOD ? RB_ROWS : 1][8];
-    if constexpr (MOD) {
 #pragma unroll
-      for (int r = 0; r < RB_ROWS; ++r)
-        if (dres != nullptr && row0 + r < rows && active) ld8(dres + static_cast<size_t>(row0 + r) * d + c, both[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < RB_ROWS; ++r) {
-      const int row = row0 + r;
+    for (int r = 0; r < STEP; ++r) {
+      const int row = row_of(k + r);
       if (row < rows && active) {
+        const uint32_t at = (slot * STEP + r) * Cfg::SLOT;
         float dot = 0.f;
 #pragma unroll
-        for (int wi = 0; wi < ROW_WARPS; ++wi) dot += red[it & 1][r][wi];
+        for (int wi = 0; wi < ROW_WARPS; ++wi) dot += red[turn][r][wi];
         dot *= inv_d;  // mean(dz * w * x_hat)
         const size_t base = static_cast<size_t>(row) * d + c;
         float o[8];
@@ -309,13 +379,13 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
         }
         if (dres != nullptr) {
           float rr[8];
-          if constexpr (!MOD) ld8(dres + base, rr);
+          fetched_columns(at_dres + at, lane, rr, T());
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += MOD ? both[MOD ? r : 0][j] : rr[j];
+          for (int j = 0; j < 8; ++j) o[j] += rr[j];
         }
         if constexpr (MOD) {
           float xv[8];
-          ld8(x + base, xv);      // in L1 since the first pass over the row
+          fetched_columns(at_x + at, lane, xv, T());
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             acc_bias[j] += o[j];
@@ -328,6 +398,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
         if (dx_bf16 != nullptr) st8(dx_bf16 + base, o);
       }
     }
+    slot = slot + 1 == Cfg::DEPTH ? 0 : slot + 1;
   }
   if (dw_partial != nullptr && active) st8(dw_partial + static_cast<size_t>(blockIdx.x) * d + c, acc);
   if constexpr (MOD) {
@@ -336,6 +407,38 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* dz, const T* x,
       st8(dw_partial + (2 * static_cast<size_t>(gridDim.x) + blockIdx.x) * d + c, acc_scale);
     }
   }
+}
+
+template <typename T, bool MOD, int STEP>
+static int launch_rmsnorm_bwd_step(const void* dz, const void* x, const float* rstd, const float* w, const void* dres,
+                                   const float* out_scale, int rows, int d, void* dx_out, void* dx_bf16, float* dw_partial,
+                                   const float* mod_bias, int grid, cudaStream_t stream) {
+  using Cfg = NormBackward<T, MOD, STEP>;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, MOD, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
+      return -20;
+    configured = true;
+  }
+  launch_dependent(rmsnorm_bwd_kernel<T, MOD, STEP>, dim3(grid), dim3(ROW_THREADS), Cfg::SMEM, stream, static_cast<const __nv_bfloat16*>(dz),
+                   static_cast<const T*>(x), rstd, w, static_cast<const T*>(dres), out_scale, rows, d, static_cast<T*>(dx_out),
+                   static_cast<__nv_bfloat16*>(dx_bf16), dw_partial, mod_bias);
+  ws_count_launch();
+  return 0;
+}
+
+// Two rows to a step where all of the blocks are resident that way, two on an SM (up to 592 rows, and always with MOD, whose registers allow
+// no third): half the barriers, and a block's only pair of rows is fetched at once (128 x 2048: 3.7 us against 4.1).  Past that three blocks on an
+// SM with one row to a step: 82 us against 89 at 16384 x 2048.  MOD with one: 79.5 against 75.6 there, within 0.5 us below 2048 rows.
+template <typename T, bool MOD>
+static int launch_rmsnorm_bwd(const void* dz, const void* x, const float* rstd, const float* w, const void* dres, const float* out_scale,
+                              int rows, int d, void* dx_out, void* dx_bf16, float* dw_partial, const float* mod_bias, int grid,
+                              cudaStream_t stream) {
+  if constexpr (!MOD) {
+    if (grid > 148 * 2)
+      return launch_rmsnorm_bwd_step<T, MOD, 1>(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, dw_partial, mod_bias, grid, stream);
+  }
+  return launch_rmsnorm_bwd_step<T, MOD, 2>(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, dw_partial, mod_bias, grid, stream);
 }
 
 // --------------------------------------------------------------------------- column sums
@@ -554,14 +657,9 @@ extern "C" int ws_rmsnorm_bwd(const void* dz, const void* x, int x_bf16, const f
                               void* dx_bf16, float* dw_partial, cudaStream_t stream) {
   if (d % 128 != 0 || d > ROW_THREADS * 8 || rows <= 0) return -1;
   const int grid = ws_rmsnorm_bwd_parts(rows);
-  if (x_bf16)
-    launch_dependent(rmsnorm_bwd_kernel<__nv_bfloat16>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)x, rstd, w, (const __nv_bfloat16*)dres, out_scale,
-        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial, nullptr);
-  else
-    launch_dependent(rmsnorm_bwd_kernel<float>, dim3(grid), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const float*)x, rstd, w, (const float*)dres, out_scale, rows, d,
-        (float*)dx_out, (__nv_bfloat16*)dx_bf16, dw_partial, nullptr);
-  ws_count_launch();
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  auto* run = x_bf16 ? &launch_rmsnorm_bwd<__nv_bfloat16, false> : &launch_rmsnorm_bwd<float, false>;
+  const int rc = run(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, dw_partial, nullptr, grid, stream);
+  return rc ? rc : cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 // Two resident blocks per SM: the modulation's column sums take the registers of the third.
@@ -575,10 +673,8 @@ extern "C" int ws_rmsnorm_bwd_mod(const void* dz, const float* x, const float* r
                                   float* partial, float* grads, cudaStream_t stream) {
   if (d % 128 != 0 || d > ROW_THREADS * 8 || rows <= 0) return -1;
   const int parts = ws_rmsnorm_bwd_mod_parts(rows);
-  launch_dependent(rmsnorm_bwd_kernel<float, true>, dim3(parts), dim3(ROW_THREADS), 0, stream,
-                   static_cast<const __nv_bfloat16*>(dz), x, rstd, w, dres, scale, rows, d, dx_out,
-                   static_cast<__nv_bfloat16*>(nullptr), partial, bias);
-  ws_count_launch();
+  const int rc = launch_rmsnorm_bwd<float, true>(dz, x, rstd, w, dres, scale, rows, d, dx_out, nullptr, partial, bias, parts, stream);
+  if (rc) return rc;
   launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS, 3), dim3(FIN_WARPS * 32), 0, stream, partial,
                    parts, d, nullptr, 0.f, grads);
   ws_count_launch();
@@ -711,13 +807,8 @@ extern "C" int ws_rmsnorm_bwd_static(const void* dz, const void* x, int x_bf16, 
   if (rc != 0) return rc;
   // Every partial row that the reduction reads below is written by the kernel first, so the
   // previous call's contents never leak into this result.
-  if (x_bf16)
-    launch_dependent(rmsnorm_bwd_kernel<__nv_bfloat16>, dim3(parts), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const __nv_bfloat16*)x, rstd, w, (const __nv_bfloat16*)dres, out_scale,
-        rows, d, (__nv_bfloat16*)dx_out, (__nv_bfloat16*)dx_bf16, scratch, nullptr);
-  else
-    launch_dependent(rmsnorm_bwd_kernel<float>, dim3(parts), dim3(ROW_THREADS), 0, stream, (const __nv_bfloat16*)dz, (const float*)x, rstd, w, (const float*)dres, out_scale, rows, d,
-        (float*)dx_out, (__nv_bfloat16*)dx_bf16, scratch, nullptr);
-  ws_count_launch();
+  auto* run = x_bf16 ? &launch_rmsnorm_bwd<__nv_bfloat16, false> : &launch_rmsnorm_bwd<float, false>;
+  if (run(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, scratch, nullptr, parts, stream) != 0) return WS_STATIC_ERR_LAUNCH;
   launch_dependent(colsum_finalize_kernel, dim3((d + FIN_COLS - 1) / FIN_COLS), dim3(FIN_WARPS * 32), 0, stream, scratch, parts, d, nullptr, 0.f, dw_out);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : WS_STATIC_ERR_LAUNCH;
