@@ -95,6 +95,7 @@ struct alignas(64) PairGroup {
   int tile_start[MAX_GROUP + 1];
   int count;
   int fetch;           // ACC_F32: the old sums are fetched and stored again, not added to in L2 (see `sums_are_fetched`)
+  int half;            // tiles of 128 columns (see `half_tiles`), which only the kernel's HALF form takes
   int ahead;           // B may be read ahead of the launches in front of this one (WsGemm::b_ahead)
 };
 
@@ -176,7 +177,7 @@ constexpr int pair_threads() {
   return 64 + 128 * epilogue_groups<EPI>();  // TMA warp, MMA warp, GROUPS x 4 epilogue warps
 }
 
-template <bool A_MN, bool B_MN, int EPI, bool GATHER = false>
+template <bool A_MN, bool B_MN, int EPI, bool GATHER = false, bool HALF = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads<EPI>() + (GATHER ? GATHER_THREADS : 0), 1)
 gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ GatherJob gj) {
   using namespace pair;
@@ -239,7 +240,9 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
   if (warp != 0 || !g.ahead) pdl_wait();
 
   constexpr bool kSwiglu = (EPI == WS_EPI_SWIGLU);
-  const int n_tile = kSwiglu ? 128 : BN;
+  constexpr int bn = HALF ? BN / 2 : BN;   // columns of the accumulator
+  constexpr int n_tile = kSwiglu ? bn / 2 : bn;
+  constexpr uint32_t stage_tx = 2 * (A_BYTES + bn / 2 * BK * 2);
   const PairExtent extent = pair_extent<A_MN>(g, n_tile);
   const int tiles = extent.tiles;
   const int pair_id = blockIdx.x >> 1;
@@ -257,9 +260,9 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         if (g.ahead) {
           if (pair_id < tiles) {
             const PairTile t = resolve_tile(g, extent, pair_id, n_tile);
-            const int r0 = kSwiglu ? (rank ? g.p[0].h + t.nb * 128 : t.nb * 128) : t.nb * BN + rank * 128;
+            const int r0 = kSwiglu ? (rank ? g.p[0].h + t.nb * n_tile : t.nb * n_tile) : t.nb * bn + rank * (bn / 2);
             for (; requested < min(t.num_k, STAGES); ++requested) {
-              if (leader) mbar_expect_tx(&full[requested], 2 * STAGE_BYTES);
+              if (leader) mbar_expect_tx(&full[requested], stage_tx);
               tma_load_2d_pair(sB + requested * B_BYTES, &g.b[t.prob], mapa_shared(smem_u32(&full[requested]), 0), requested * BK, r0);
             }
           }
@@ -314,7 +317,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           // The leader alone announces the bytes of both CTAs (a remote expect-tx arrival with
           // release semantics from the peer measured 2x slower for the whole kernel).
           const bool b_there = it < requested;
-          if (leader && !b_there) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+          if (leader && !b_there) mbar_expect_tx(&full[s], stage_tx);
           uint8_t* a_dst = sA + s * A_BYTES;
           uint8_t* b_dst = sB + s * B_BYTES;
           if (!A_MN) {
@@ -326,12 +329,12 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           }
           if (b_there) continue;
           if (!B_MN) {
-            const int r0 = kSwiglu ? (rank ? p.h + nb * 128 : nb * 128) : nb * BN + rank * 128;
+            const int r0 = kSwiglu ? (rank ? p.h + nb * n_tile : nb * n_tile) : nb * bn + rank * (bn / 2);
             tma_load_2d_pair(b_dst, tma_b, bar, kb * BK, r0);
           } else {
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-              tma_load_2d_pair(b_dst + i * (BK * 128), tma_b, bar, nb * BN + rank * 128 + i * 64, kb * BK);
+            for (int i = 0; i < bn / 128; ++i)
+              tma_load_2d_pair(b_dst + i * (BK * 128), tma_b, bar, nb * bn + rank * (bn / 2) + i * 64, kb * BK);
           }
         }
       }
@@ -339,7 +342,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
+      constexpr uint32_t idesc = make_idesc_bf16(2 * BM, bn, A_MN, B_MN);
       int it = 0;
       int tcount = 0;
       bool ok = true;
@@ -385,7 +388,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       // SwiGLU forward through shared memory: per warp 32 rows, per step 32 features; the three
       // output tiles (up, gate, activation) are written to swizzled shared memory and leave by TMA.
       uint8_t* ebuf = eStage + (warp - 2) * 8192;  // 3 tiles of 2 KiB used
-      constexpr int STEPS = (128 / GROUPS) / 32;
+      constexpr int STEPS = n_tile / GROUPS / 32;
       const GemmParams& p = g.p[0];
       for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
@@ -399,11 +402,11 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN;
 #pragma unroll 1
         for (int step = 0; step < STEPS; ++step) {
-          const int c = egroup * (128 / GROUPS) + step * 32;
-          const int x = t.nb * 128 + c;
+          const int c = egroup * (n_tile / GROUPS) + step * 32;
+          const int x = t.nb * n_tile + c;
           uint32_t ru[32], rg[32];
           tmem_ld_32x32b_x32(taddr + c, ru);
-          tmem_ld_32x32b_x32(taddr + 128 + c, rg);
+          tmem_ld_32x32b_x32(taddr + n_tile + c, rg);
           tmem_ld_wait();
           uint32_t wu[16], wg[16], wa[16];
 #pragma unroll
@@ -447,7 +450,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         // but no thread waits for the old value.  Against a thread per row that reads and writes 16 bytes of 32 rows at a time:
         // 27 M gradients of 1792 tokens 125 -> 85 us, 67 M of 2300 309 -> 237, 0.9 M of 1024 27 -> 16.
         uint8_t* ebuf = eStage + (warp - 2) * 8192;
-        constexpr int STEPS = (BN / GROUPS) / 32;
+        constexpr int STEPS = bn / GROUPS / 32;
         int q = 0;
         for (int tile = pair_id; tile < tiles; tile += num_pairs, ++tcount) {
           const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
@@ -457,14 +460,14 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
           tc_fence_after_sync();
           const int y = t.mb * 2 * BM + rank * BM + quarter * 32;
-          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (bn / GROUPS);
           const float alpha = EPI == WS_EPI_ACC_F32 ? p.alpha : 1.f;
           if (EPI == WS_EPI_ACC_F32 && p.beta != 0.f && p.beta != 1.f) {   // neither a store nor a sum: by row
-            gemm_epilogue<EPI, GROUPS>(p, taddr - egroup * (BN / GROUPS), y + lane, y + lane < p.m, 1.f, t.nb, egroup);
+            gemm_epilogue<EPI, GROUPS>(p, taddr - egroup * (bn / GROUPS), y + lane, y + lane < p.m, 1.f, t.nb, egroup);
           } else
 #pragma unroll 1
           for (int step = 0; step < STEPS; ++step, ++q) {
-            const int x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+            const int x = t.nb * bn + egroup * (bn / GROUPS) + step * 32;
             uint8_t* tr = ebuf + (q & 1) * 4096;
             uint32_t r[32];
             tmem_ld_32x32b_x32(taddr + step * 32, r);
@@ -498,10 +501,10 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         // the residual tile is TMA-loaded (double-buffered), updated in place and TMA-stored.
         uint8_t* ebuf = eStage + (warp - 2) * 8192;  // two buffers of one 4 KiB tile
         uint64_t* mybar = ebar + (warp - 2) * 2;
-        constexpr int STEPS = (BN / GROUPS) / 32;
+        constexpr int STEPS = bn / GROUPS / 32;
         auto coords = [&](int tile, int step, int& x, int& y) {
           const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
-          x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+          x = t.nb * bn + egroup * (bn / GROUPS) + step * 32;
           y = t.mb * 2 * BM + rank * BM + quarter * 32;
           return t.prob;
         };
@@ -521,7 +524,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
           const uint32_t tph = (tcount >> 1) & 1;
           if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
           tc_fence_after_sync();
-          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+          const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (bn / GROUPS);
           const float alpha = EPI == WS_EPI_ACC_F32 ? g.p[resolve_tile(g, extent, tile, n_tile, GATHER).prob].alpha : 1.f;
 #pragma unroll 1
           for (int step = 0; step < STEPS; ++step, ++q) {
@@ -571,11 +574,11 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
       // buffers, each holding the (up, gate) tiles that become (dUp, dGate) in place.
       uint8_t* ebuf = eStage + (warp - 2) * 8192;
       uint64_t* mybar = ebar + (warp - 2) * 2;
-      constexpr int STEPS = (BN / GROUPS) / 32;
+      constexpr int STEPS = bn / GROUPS / 32;
       const GemmParams& p = g.p[0];
       auto coords = [&](int tile, int step, int& x, int& y) {
         const PairTile t = resolve_tile(g, extent, tile, n_tile, GATHER);
-        x = t.nb * BN + egroup * (BN / GROUPS) + step * 32;
+        x = t.nb * bn + egroup * (bn / GROUPS) + step * 32;
         y = t.mb * 2 * BM + rank * BM + quarter * 32;
       };
       auto issue_load = [&](int tile, int step, int buf) {
@@ -595,7 +598,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         const uint32_t tph = (tcount >> 1) & 1;
         if (!mbar_wait_warp(&tfull[buf_t], tph, abort_flag)) break;
         tc_fence_after_sync();
-        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (BN / GROUPS);
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + buf_t * BN + egroup * (bn / GROUPS);
 #pragma unroll 1
         for (int step = 0; step < STEPS; ++step, ++q) {
           const int buf = q & 1;
@@ -678,7 +681,7 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
         float rs = 1.0f;
         if (p.row_scale != nullptr && inside) rs = place >= 0 ? p.row_scale[place] : 0.f;
         if constexpr (EPI == WS_EPI_BF16)
-          gemm_epilogue<EPI, GROUPS>(p, taddr, place, inside && place >= 0, rs, nb, egroup, stage);
+          gemm_epilogue<EPI, GROUPS>(p, taddr, place, inside && place >= 0, rs, nb, egroup, stage, bn);
         else
           gemm_epilogue<EPI, GROUPS>(p, taddr, row, inside, rs, nb, egroup, EPI == WS_EPI_CE_FWD ? stage : nullptr);
         tc_fence_before_sync();
@@ -763,10 +766,14 @@ gemm2_kernel(const __grid_constant__ PairGroup g, const __grid_constant__ Gather
 // 2 i + const, and pairs that share operand tiles sit side by side; placed as a draining kernel frees SMs they are scattered
 // over both dies, and these products, which re-read their operands most, run at three quarters of the rate: d 2048, 2048 rows
 // 399 -> 296 us, 512 rows 369 -> 240, 16384 rows 1752 -> 1660.  The other products differ by what their set-up takes.
-template <bool A_MN, bool B_MN, int EPI>
+template <bool A_MN, bool B_MN, int EPI, bool HALF = false>
 static int launch_pair(const PairGroup& g, int pairs, cudaStream_t stream) {
+  constexpr bool kHalved = staged_epilogue<EPI>() || (EPI == WS_EPI_BF16 && !A_MN);   // see `half_tiles`
+  if constexpr (kHalved && !HALF) {
+    if (g.half) return launch_pair<A_MN, B_MN, EPI, true>(g, pairs, stream);
+  }
   static bool configured = false;
-  auto kern = gemm2_kernel<A_MN, B_MN, EPI>;
+  auto kern = gemm2_kernel<A_MN, B_MN, EPI, false, HALF>;
   if (!configured) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem<EPI>()) != cudaSuccess)
       return -20;
@@ -791,8 +798,34 @@ static int launch_pair_gather(const PairGroup& g, const GatherJob& job, int pair
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }
 
+// Tiles of `bn` accumulator columns.
+static int pair_tiles(const WsGemm* g, int bn) {
+  const int n_tile = g->epilogue == WS_EPI_SWIGLU ? bn / 2 : bn;
+  return ((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + n_tile - 1) / n_tile);
+}
+
+// Tiles of 256 x 128 where those, too, are one round over the CTA pairs, so that twice as many SMs share the work and each has half of
+// an epilogue, which nothing hides there: it is the larger part of such a product.  Same bits.  us, 256 -> 128 columns: 1792 x 1280 of k
+// 1280 10.5 -> 8.7, with a residual 14.4 -> 10.5; 1024 x 2048 of k 2048 14.1 -> 11.0 and 18.1 -> 12.9; 128 x 2048 in four pieces, of k 2048
+// 9.5 -> 8.4, of k 7168 15.4 -> 12.7; 512 x 4480 SwiGLU backward 17.4 -> 12.7; 1024 x 688 SwiGLU of k 256 7.5 -> 6.0; the four gradients of a
+// block of width 256 12.1 -> 10.0.  A k-block of one costs three quarters of a whole one's time (shared memory feeds A as often for half of the
+// products), so past one round they lose even where they would fill the last: 1792 x 6400 of k 1280, 175 tiles or 350, 22.9 -> 27.5.
+static bool half_tiles(const WsGemm* items, int count, int pairs) {
+  int half = 0;
+  for (int i = 0; i < count; ++i) {
+    const WsGemm& g = items[i];
+    const bool scaled = g.epilogue == WS_EPI_ACC_F32 && g.beta != 0.f && g.beta != 1.f;   // whose epilogue goes by rows of 256
+    const bool built = (g.epilogue == WS_EPI_BF16 && !g.a_mn) || g.epilogue == WS_EPI_RESID_F32 || g.epilogue == WS_EPI_F32 || g.epilogue == WS_EPI_SWIGLU ||
+                       g.epilogue == WS_EPI_SWIGLU_BWD || g.epilogue == WS_EPI_ACC_F32;
+    if (!built || scaled || g.limit != nullptr || g.whole != nullptr || g.row_map != nullptr) return false;
+    half += pair_tiles(&g, pair::BN / 2);
+  }
+  return half <= pairs;
+}
+
 // Tensor maps, kernel parameters and tile count of one problem.
 static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) {
+  const int bn = grp.half ? pair::BN / 2 : pair::BN;
   if (g->m <= 0 || g->n <= 0 || g->k <= 0) return -1;
   const bool swiglu = g->epilogue == WS_EPI_SWIGLU;
   const int b_rows = swiglu ? 2 * g->n : g->n;
@@ -803,7 +836,7 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
     rc = make_map_bf16(&grp.a[i], g->a, g->m, g->k, g->lda, 64, pair::BK);
   if (rc) return rc;
   if (!g->b_mn)
-    rc = make_map_bf16(&grp.b[i], g->b, g->k, b_rows, g->ldb, pair::BK, 128);
+    rc = make_map_bf16(&grp.b[i], g->b, g->k, b_rows, g->ldb, pair::BK, bn / 2);
   else
     rc = make_map_bf16(&grp.b[i], g->b, b_rows, g->k, g->ldb, 64, pair::BK);
   if (rc) return rc;
@@ -830,8 +863,7 @@ static int fill_problem(const WsGemm* g, PairGroup& grp, int i, int* tiles_out) 
                   : make_map_bf16(&grp.whole, g->whole, b_rows, g->k, g->ldwhole, 64, pair::BK);
     if (rc) return rc;
   }
-  const int n_tile = swiglu ? 128 : pair::BN;
-  *tiles_out = ((g->m + 2 * pair::BM - 1) / (2 * pair::BM)) * ((g->n + n_tile - 1) / n_tile);
+  *tiles_out = pair_tiles(g, bn);
   return 0;
 }
 
@@ -1101,6 +1133,7 @@ extern "C" int ws_gemm_pair_group(const WsGemm* items, int count, int sms, cudaS
   PairGroup grp;
   memset(&grp, 0, sizeof(grp));
   grp.count = count;
+  grp.half = half_tiles(items, count, sms / 2 > 0 ? sms / 2 : 1);
   int total = 0;
   for (int i = 0; i < count; ++i) {
     if (items[i].a_mn != items[0].a_mn || items[i].b_mn != items[0].b_mn || items[i].epilogue != items[0].epilogue)

@@ -76,14 +76,14 @@ struct WarpStage {
 
 template <int EPI, int GROUPS = 2>
 __device__ __forceinline__ void gemm_epilogue(const GemmParams& p, uint32_t taddr, int row, bool row_ok, float rs,
-                                              int nb, int egroup, WarpStage* stage = nullptr) {
-  constexpr int BN = EPI_BN;
+                                              int nb, int egroup, WarpStage* stage = nullptr, int bn = EPI_BN) {
+  constexpr int BN = EPI_BN;   // `bn` columns, where it is less: BF16 results only
   static_assert(GROUPS == 2 || EPI == WS_EPI_SWIGLU || EPI == WS_EPI_SWIGLU_BWD, "only the SwiGLU epilogues take 4 groups");
   if constexpr (EPI == WS_EPI_BF16) {
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(row) * p.ldo;
-    const int n0 = nb * BN;
+    const int n0 = nb * bn;
 #pragma unroll 1
-    for (int c = egroup * 128; c < egroup * 128 + 128; c += 32) {
+    for (int c = egroup * (bn / 2); c < (egroup + 1) * (bn / 2); c += 32) {
       if (n0 + c >= p.n) break;
       uint32_t r[32];
       tmem_ld_32x32b_x32(taddr + c, r);
