@@ -667,8 +667,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 // Two tiles are in their softmax / blend phase at any time while a third is being rotated and a fourth loaded;
 // attn_fwd_kernel gets its overlap from three independent CTAs per SM, each walking the whole chain alone.
 // TMEM: set g = columns [192 g, 192 g + 192): S 128, Mem 64; O of group g = columns [384 + 64 g, 448 + 64 g).  Bit-identical
-// results.  PROMPT as in attn_fwd_kernel; the low terms of P are formed from S again, which is still in TMEM, once O has
-// the high ones.
+// results.  PROMPT as in attn_fwd_kernel, but the low terms of P take the place, in TMEM, of the scores that they come from; their product
+// reads them there as its first operand.  Formed again from the scores, behind the product of the high ones and into their place in shared
+// memory, they were a second pass over the open chunk: 96 tiles of a 300-token prompt (with its writes and scan) 16.8 -> 14.9 us, 4096 tiles of
+// 16 x 1000 tokens 172 -> 162.
 constexpr int AS_STAGES = 3;
 constexpr int AS_THREADS = 25 * 32;
 constexpr int AS_STAGE_BYTES = 4 * TILE_BYTES + 8192;
@@ -689,8 +691,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
   uint64_t* sfull = bars + 2 * AS_STAGES;    // [2] S and Mem complete
   uint64_t* ofull = sfull + 2;               // [2] O complete
   uint64_t* setfree = ofull + 2;             // [2] TMEM set read out (4 storing warps, for two each)
-  uint64_t* lowfull = setfree + 2;           // [2] O has the low terms too (PROMPT)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(lowfull + 2);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(setfree + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_chunks = (T + CHUNK - 1) / CHUNK;
@@ -704,7 +705,6 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       mbar_init(&sfull[g], 1);
       mbar_init(&ofull[g], 1);
       mbar_init(&setfree[g], 4);
-      mbar_init(&lowfull[g], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -831,7 +831,6 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
     };
     // the two warps that share 32 rows
     auto pair_sync = [&] { asm volatile("bar.sync %0, 64;" ::"r"(5 + g * 4 + wq) : "memory"); };
-    [[maybe_unused]] uint32_t opens = 0;   // open chunks this group has met
     int i = g;
     for (int tile = first + g * step; tile < tiles; tile += 2 * step, i += 2) {
       const int s = i % AS_STAGES, k2 = i >> 1;
@@ -851,14 +850,19 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           *reinterpret_cast<uint4*>(tile_chunk(half, gt, j0 + w4)) =
               make_uint4(pk[4 * w4], pk[4 * w4 + 1], pk[4 * w4 + 2], pk[4 * w4 + 3]);
       };
-      auto issue_o = [&](uint32_t accumulate, uint64_t* done) {
+      auto issue_o = [&] {
         tc_fence_after_sync();
         constexpr uint32_t idesc_o = make_idesc_bf16(128, 64, false, true);
 #pragma unroll
         for (int k = 0; k < CHUNK / 16; ++k)
           umma_bf16(t_o, make_smem_desc_sw128(smem_u32((k >> 2) ? sQ : sK) + (k & 3) * 32, 0, 1024),
-                    make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, k > 0 ? 1u : accumulate);
-        umma_commit(done);
+                    make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, k > 0);
+        if (open) {   // O += P_lo V
+#pragma unroll
+          for (int k = 0; k < CHUNK / 16; ++k)
+            umma_bf16_ts(t_o, t_s + (k >> 1) * 32 + (k & 1) * 8, make_smem_desc_sw128(smem_u32(sV) + k * 2048, 0, 1024), idesc_o, 1u);
+        }
+        umma_commit(&ofull[g]);
       };
       uint32_t landed = 0;
       if (lane == 0) landed = mbar_wait(&sfull[g], k2 & 1, abort_flag) ? 1u : 0u;
@@ -884,6 +888,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
           constexpr bool REST = decltype(rest_too)::value;
           for (int cc = half; cc < 4; cc += 2) {
             uint32_t pk[16];
+            [[maybe_unused]] uint32_t low[16];
             if (cc <= last_chunk) {
               uint32_t v[32];
               tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
@@ -897,16 +902,20 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
                 row_sum += back.x + back.y;  // normalise by what the MMA will actually sum
                 pk[j >> 1] = *reinterpret_cast<const uint32_t*>(&pv);
                 if constexpr (REST) {
-                  const float2 rest = __bfloat1622float2(__floats2bfloat162_rn(p0 - back.x, p1 - back.y));
+                  const __nv_bfloat162 rv = __floats2bfloat162_rn(p0 - back.x, p1 - back.y);
+                  const float2 rest = __bfloat1622float2(rv);
                   row_sum += rest.x + rest.y;
+                  low[j >> 1] = *reinterpret_cast<const uint32_t*>(&rv);
                 }
               }
             } else {
 #pragma unroll
-              for (int j = 0; j < 16; ++j) pk[j] = 0u;
+              for (int j = 0; j < 16; ++j) pk[j] = low[j] = 0u;
             }
             store_p(cc, pk);
+            if constexpr (REST) tmem_st_32x32b_x16(t_s + lane_base + cc * 32, low);   // over scores that this thread alone reads
           }
+          if constexpr (REST) tmem_st_wait();
         };
         if (PROMPT && open) weights(std::integral_constant<bool, PROMPT>{});
         else weights(std::false_type{});
@@ -916,45 +925,11 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       fence_proxy_async_smem();
       if (any_bad(ok)) break;
       row_sum = meet[256 + gt] + meet[384 + gt];
-      if (warp == 8 + 8 * g && elect_one()) issue_o(0u, &ofull[g]);
+      if (warp == 8 + 8 * g && elect_one()) issue_o();
       landed = 0;
       if (lane == 0) landed = mbar_wait(&ofull[g], k2 & 1, abort_flag) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
       tc_fence_after_sync();
-      if constexpr (PROMPT) {
-        if (open) {  // O += P_lo V
-          if (ok && row0 + wq * 32 < T) {  // the rows of a warp past the prompt's end are not stored
-            for (int cc = half; cc < 4; cc += 2) {
-              uint32_t pk[16];
-              if (cc <= last_chunk) {
-                uint32_t v[32];
-                tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
-                tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                  const float p0 = (cc * 32 + j <= gt) ? softmax_term(__uint_as_float(v[j]), row_max, kScale) : 0.f;
-                  const float p1 = (cc * 32 + j + 1 <= gt) ? softmax_term(__uint_as_float(v[j + 1]), row_max, kScale) : 0.f;
-                  const float2 back = __bfloat1622float2(__floats2bfloat162_rn(p0, p1));
-                  pk[j >> 1] = pack_bf16x2(p0 - back.x, p1 - back.y);
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) pk[j] = 0u;
-              }
-              store_p(cc, pk);
-            }
-          }
-          tc_fence_before_sync();
-          fence_proxy_async_smem();
-          if (any_bad(ok)) break;
-          if (warp == 8 + 8 * g && elect_one()) issue_o(1u, &lowfull[g]);
-          landed = 0;
-          if (lane == 0) landed = mbar_wait(&lowfull[g], opens & 1, abort_flag) ? 1u : 0u;
-          ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
-          tc_fence_after_sync();
-          ++opens;
-        }
-      }
       if (ok) {
         // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
         const float inv_l = 1.f / row_sum;

@@ -263,7 +263,7 @@ __device__ __forceinline__ void umma_bf16_low(uint32_t tmem_d, uint32_t a_low, u
       "r"(a_low), "r"(b_low), "r"(idesc), "r"(accumulate), "n"(kHigh), "n"(kHighB)
       : "memory");
 }
-// A operand taken from TMEM (used by the attention kernels for P*V and dS*K products).
+// A operand taken from TMEM: a row to a lane, two neighbouring elements of K to a column, so eight columns from `tmem_a` on.
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b,
                                              uint32_t idesc, uint32_t accumulate) {
   asm volatile(
