@@ -500,8 +500,7 @@ memory_scan_bwd_kernel(const float* dstate, const float* writes,
   }
 }
 
-// Gradients of the decay and mix logits from the scan's partial sums: out[q][h] = sigmoid'(logit_q[h]) * sum over the
-// head's B * 16 partials.  One CTA per head, one warp per logit, fixed order.  (A launch in place of the sum, three
+// Gradients of the decay and mix logits from the scan's partial sums (`logit_grad`).  (A launch in place of the sum, three
 // sigmoids and nine products that a framework expression of it takes: 15 launches of 2 us for 3 H numbers.)
 __global__ void __launch_bounds__(96)
 memory_logit_grads_kernel(const float* partials, const float* fast_logit,
@@ -509,17 +508,7 @@ memory_logit_grads_kernel(const float* partials, const float* fast_logit,
                           float* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
-  const int h = blockIdx.x, q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float v = 0.f;
-  for (int i = lane; i < B * 16; i += 32)
-    v += partials[((static_cast<size_t>(i >> 4) * H + h) * 16 + (i & 15)) * 3 + q];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (lane == 0) {
-    const float* logit = q == 0 ? fast_logit : q == 1 ? slow_logit : mix_logit;
-    const float s = 1.f / (1.f + expf(-logit[h]));
-    out[q * H + h] = v * s * (1.f - s);
-  }
+  logit_grad(partials, fast_logit, slow_logit, mix_logit, B, H, blockIdx.x, threadIdx.x >> 5, out);
 }
 
 // =============================================================================== attention bwd

@@ -102,4 +102,20 @@ inline int make_sequence_map(CUtensorMap* map, const void* base, uint64_t cols, 
   return r == CUDA_SUCCESS ? 0 : -12;
 }
 
+// out[q][h] = sigmoid'(logit_q[h]) * sum over the head's B * 16 partials of the reverse scan: one warp, fixed order.
+__device__ __forceinline__ void logit_grad(const float* partials, const float* fast_logit, const float* slow_logit, const float* mix_logit,
+                                           int B, int H, int h, int q, float* out) {
+  const int lane = threadIdx.x & 31;
+  float v = 0.f;
+  for (int i = lane; i < B * 16; i += 32)
+    v += partials[((static_cast<size_t>(i >> 4) * H + h) * 16 + (i & 15)) * 3 + q];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) {
+    const float* logit = q == 0 ? fast_logit : q == 1 ? slow_logit : mix_logit;
+    const float s = 1.f / (1.f + expf(-logit[h]));
+    out[q * H + h] = v * s * (1.f - s);
+  }
+}
+
 }  // namespace ws

@@ -182,11 +182,12 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_fwd(const at::Tensor& x,
 }
 
 // returns (dx, dx_bf16, dw) ; dw is the finished column sum [d]
-std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz, const at::Tensor& x,
-                                                           const at::Tensor& rstd, const at::Tensor& w,
-                                                           const c10::optional<at::Tensor>& dres,
-                                                           const c10::optional<at::Tensor>& out_scale,
-                                                           bool want_bf16) {
+// dx, its BF16 copy where asked for, and the partial rows of the weight's gradient
+std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd_partial(const at::Tensor& dz, const at::Tensor& x,
+                                                                   const at::Tensor& rstd, const at::Tensor& w,
+                                                                   const c10::optional<at::Tensor>& dres,
+                                                                   const c10::optional<at::Tensor>& out_scale,
+                                                                   bool want_bf16) {
   TORCH_CHECK(dz.is_cuda() && dz.scalar_type() == at::kBFloat16 && dz.is_contiguous(), "rmsnorm_bwd: dz");
   TORCH_CHECK(x.is_contiguous() && x.sizes() == dz.sizes(), "rmsnorm_bwd: x");
   c10::cuda::CUDAGuard guard(x.device());
@@ -203,6 +204,17 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz,
                           has_scale ? out_scale->data_ptr<float>() : nullptr, rows, d, dx.data_ptr(),
                           want_bf16 ? dxb.data_ptr() : nullptr, partial.data_ptr<float>(), cur_stream()),
            "rmsnorm_bwd");
+  return {dx, dxb, partial};
+}
+
+std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz, const at::Tensor& x,
+                                                           const at::Tensor& rstd, const at::Tensor& w,
+                                                           const c10::optional<at::Tensor>& dres,
+                                                           const c10::optional<at::Tensor>& out_scale,
+                                                           bool want_bf16) {
+  auto [dx, dxb, partial] = rmsnorm_bwd_partial(dz, x, rstd, w, dres, out_scale, want_bf16);
+  c10::cuda::CUDAGuard guard(x.device());
+  const int parts = (int)partial.size(0), d = (int)partial.size(1);
   at::Tensor dw = at::empty({d}, x.options().dtype(at::kFloat));
   check_rc(ws_colsum_finalize(partial.data_ptr<float>(), parts, d, nullptr, 0.f, dw.data_ptr<float>(), cur_stream()),
            "colsum_finalize");
@@ -212,10 +224,11 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz,
 // The norm behind a depth modulation (FP32 stream): -> (dx, FP32 [3, d]: gradients of w, of the bias, of the scale).  From
 // the modulation's input x; a caller that has only its output xmod gets x back as (xmod - bias) / (1 + scale), 0 where
 // scale is -1, with an error of an ulp of xmod over 1 + scale.
-std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const c10::optional<at::Tensor>& xmod,
-                                                   const at::Tensor& rstd, const at::Tensor& w, const at::Tensor& dres,
-                                                   const at::Tensor& scale, const at::Tensor& bias,
-                                                   const c10::optional<at::Tensor>& x_) {
+// The same with the gradients' sums (`summed`), or with the partial rows [3, parts, d] that they are made of.
+std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_modulated(const at::Tensor& dz, const c10::optional<at::Tensor>& xmod,
+                                                         const at::Tensor& rstd, const at::Tensor& w, const at::Tensor& dres,
+                                                         const at::Tensor& scale, const at::Tensor& bias,
+                                                         const c10::optional<at::Tensor>& x_, bool summed) {
   const bool given = x_.has_value() && x_->defined();
   TORCH_CHECK(given || (xmod.has_value() && xmod->defined()), "rmsnorm_bwd_mod: x or xmod");
   TORCH_CHECK(dz.is_cuda() && dz.scalar_type() == at::kBFloat16 && dz.is_contiguous(), "rmsnorm_bwd_mod: dz");
@@ -230,12 +243,18 @@ std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const c
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor dx = at::empty_like(x);
   at::Tensor partial = at::empty({3, ws_rmsnorm_bwd_mod_parts(rows), d}, x.options());
-  at::Tensor grads = at::empty({3, d}, x.options());
+  at::Tensor grads = summed ? at::empty({3, d}, x.options()) : at::Tensor();
   check_rc(ws_rmsnorm_bwd_mod(dz.data_ptr(), x.data_ptr<float>(), rstd.data_ptr<float>(), w.data_ptr<float>(),
                               dres.data_ptr<float>(), scale.data_ptr<float>(), bias.data_ptr<float>(), rows, d,
-                              dx.data_ptr<float>(), partial.data_ptr<float>(), grads.data_ptr<float>(), cur_stream()),
+                              dx.data_ptr<float>(), partial.data_ptr<float>(), summed ? grads.data_ptr<float>() : nullptr, cur_stream()),
            "rmsnorm_bwd_mod");
-  return {dx, grads};
+  return {dx, summed ? grads : partial};
+}
+
+std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_mod(const at::Tensor& dz, const c10::optional<at::Tensor>& xmod,
+                                                   const at::Tensor& rstd, const at::Tensor& w, const at::Tensor& dres,
+                                                   const at::Tensor& scale, const at::Tensor& bias, const c10::optional<at::Tensor>& x) {
+  return rmsnorm_bwd_modulated(dz, xmod, rstd, w, dres, scale, bias, x, true);
 }
 
 // (sum_rows a / (1+inv_scale), sum_rows a*b / (1+inv_scale))
@@ -734,18 +753,27 @@ std::vector<at::Tensor> block_bwd(const at::Tensor& dx3, const at::Tensor& x, co
   const int64_t h = w_down.size(1);
   at::Tensor dpacked = project(dx3b, w_down, true, WS_EPI_SWIGLU_BWD, h, at::empty({dx3b.size(0), 2 * h}, dx3b.options()),
                                c10::nullopt, packed, flag);
-  auto [dx2, dx2b, g_n2] = rmsnorm_bwd(input_grad(dpacked, w_ug, flag), x2, rstd2, n2, dx3, c10::nullopt, !bf16_stream);
+  auto [dx2, dx2b, second] = rmsnorm_bwd_partial(input_grad(dpacked, w_ug, flag), x2, rstd2, n2, dx3, c10::nullopt, !bf16_stream);
   if (bf16_stream) dx2b = dx2;
-  auto [dqkvgu, partials] = attn_bwd(qkvgu, input_grad(dx2b, w_out, flag), states, writes, rope, fast_logit, slow_logit,
-                                   mix_logit, B, T, H, flag);
-  at::Tensor logits = memory_logit_grads(partials, fast_logit, slow_logit, mix_logit, B);
-  at::Tensor dz1 = input_grad(dqkvgu, w_in, flag);
-  if (scale.has_value() && scale->defined() && !bf16_stream) {
-    auto [dx, norm] = rmsnorm_bwd_mod(dz1, c10::nullopt, rstd1, n1, dx2, *scale, *bias, x);
-    return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm};
-  }
-  auto [dx, unused, g_n1] = rmsnorm_bwd(dz1, x, rstd1, n1, dx2, scale, false);
-  return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, g_n1.unsqueeze(0)};
+  auto [dqkvgu, scan] = attn_bwd(qkvgu, input_grad(dx2b, w_out, flag), states, writes, rope, fast_logit, slow_logit,
+                                 mix_logit, B, T, H, flag);
+  at::Tensor dz1 = input_grad(dqkvgu, w_in, flag), dx, first;
+  const bool modulated = scale.has_value() && scale->defined() && !bf16_stream;
+  if (modulated)
+    std::tie(dx, first) = rmsnorm_bwd_modulated(dz1, c10::nullopt, rstd1, n1, dx2, *scale, *bias, x, false);
+  else
+    std::tie(dx, std::ignore, first) = rmsnorm_bwd_partial(dz1, x, rstd1, n1, dx2, scale, false);
+  c10::cuda::CUDAGuard guard(dx.device());
+  const int64_t d = x2.size(1), sums = modulated ? 3 : 1;
+  const at::TensorOptions floats = second.options();
+  at::Tensor g_n2 = at::empty({d}, floats), logits = at::empty({3, H}, floats), norm = at::empty({sums, d}, floats);
+  for (const at::Tensor* t : {&fast_logit, &slow_logit, &mix_logit})
+    TORCH_CHECK(t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == H, "block_bwd: logits");
+  check_rc(ws_block_sums(second.data_ptr<float>(), (int)second.size(0), g_n2.data_ptr<float>(), first.data_ptr<float>(),
+                         (int)first.size(modulated ? 1 : 0), (int)sums, norm.data_ptr<float>(), scan.data_ptr<float>(), fast_logit.data_ptr<float>(),
+                         slow_logit.data_ptr<float>(), mix_logit.data_ptr<float>(), (int)B, (int)H, logits.data_ptr<float>(), (int)d, cur_stream()),
+           "block_sums");
+  return {dx, dx3b, dpacked, dx2b, dqkvgu, g_n2, logits, norm};
 }
 
 // One block as one autograd node whose two directions never enter Python: `ops.fused.CoreFn` for an FP32 stream and weights

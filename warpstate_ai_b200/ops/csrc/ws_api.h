@@ -160,7 +160,8 @@ int ws_rmsnorm_bwd(const void* dz, const void* x, int x_bf16, const float* rstd,
                    const void* dres, const float* out_scale, int rows, int d, void* dx_out,
                    void* dx_bf16, float* dw_partial, cudaStream_t stream);
 // The same behind a depth modulation xmod = x * (1 + scale) + bias, FP32 stream, from x itself: dx_out is its gradient, and
-// grads [3, d] those of w, bias and scale.  partial: 3 * ws_rmsnorm_bwd_mod_parts(rows) rows of d floats.
+// grads [3, d] those of w, bias and scale.  partial: 3 * ws_rmsnorm_bwd_mod_parts(rows) rows of d floats, which are all that is left where grads
+// is NULL.
 int ws_rmsnorm_bwd_mod_parts(int rows);
 int ws_rmsnorm_bwd_mod(const void* dz, const float* x, const float* rstd, const float* w, const float* dres,
                        const float* scale, const float* bias, int rows, int d, float* dx_out, float* partial,
@@ -172,6 +173,11 @@ int ws_colsum2(const void* a, const void* b, int is_bf16, int rows, int d, float
 // out[c] = beta*out[c] + (sum_p partial[p][c]) / (1 + inv_scale[c])   (inv_scale may be NULL)
 int ws_colsum_finalize(const float* partial, int parts, int d, const float* inv_scale, float beta,
                        float* out, cudaStream_t stream);
+// What a block's backward pass leaves to add up, in one launch: the second norm's weight gradient from its partial rows, `first_sums` (1, or 3 behind a
+// modulation) of the first norm's, and the logits' gradients [3, H] from the reverse scan's partials (ws_memory_logit_grads).
+int ws_block_sums(const float* second, int second_parts, float* second_out, const float* first, int first_parts, int first_sums,
+                  float* first_out, const float* scan, const float* fast_logit, const float* slow_logit, const float* mix_logit, int B,
+                  int H, float* logits_out, int d, cudaStream_t stream);
 int ws_cast_f32_bf16(const float* in, void* out, size_t n, cudaStream_t stream);
 int ws_embed_fwd(const long long* ids, const void* table, int table_bf16, int rows, int d, int vocab,
                  void* out, int out_bf16, cudaStream_t stream);
