@@ -526,7 +526,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
     for (int j = 0; j < 32; ++j)
       if (cc * 32 + j <= tid) row_max = fmaxf(row_max, __uint_as_float(r[j]));
   }
-  float even_sum = 0.f, odd_sum = 0.f;   // over the blocks of 32 columns, as the streaming form's two threads of a row have them
+  float row_sum = 0.f;
   [[maybe_unused]] uint32_t low[PROMPT ? 4 : 1][16];
 #pragma unroll(PROMPT ? 4 : 1)
   for (int cc = 0; cc < 4; ++cc) {
@@ -535,7 +535,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       uint32_t r[32];
       tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, r);
       tmem_ld_wait();
-      float row_sum = cc & 1 ? odd_sum : even_sum;
 #pragma unroll
       for (int j = 0; j < 32; j += 2) {
         const float p0 = (cc * 32 + j <= tid) ? softmax_term(__uint_as_float(r[j]), row_max, kScale) : 0.f;
@@ -551,8 +550,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
           low[cc][j >> 1] = *reinterpret_cast<const uint32_t*>(&l);
         }
       }
-      if (cc & 1) odd_sum = row_sum;
-      else even_sum = row_sum;
     } else {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -600,7 +597,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
   }
 
   // ---- gate blend into the (now idle) Q tile, then one TMA store of the warp's 32 rows
-  const float inv_l = 1.f / (even_sum + odd_sum);
+  const float inv_l = 1.f / row_sum;
 #pragma unroll
   for (int c = 0; c < HD; c += 16) {
     uint32_t ro[16], rm[16];
@@ -655,12 +652,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 //                  K in place (its 16 (cos, sin) pairs live in registers); worker 0 then issues S = Qr Kr^T and
 //                  Mem = Qr State into TMEM set i % 2 -- Mem does not depend on the softmax, so it rides with S
 //   warps 8..15    softmax group 0 (tiles 0, 2, 4, ...), warps 16..23 softmax group 1 (tiles 1, 3, ...): two threads per token
-//                  row, each with every other block of 32 score columns and half of the output columns; they exchange their
-//                  maxima and sums through shared memory.  With one thread per row a tile was 14.9 k clocks of its group,
-//                  8192 rows of 32 heads took 54.2 us, 48.7 so.
+//                  row, the first with the front half of the visible blocks of 32 score columns, the second with the rest, each with
+//                  half of the output columns; they exchange their maxima and the sum through shared memory.  The sum goes through
+//                  the row's columns in order, as one thread has it: the second thread adds its terms to the first one's sum
+//                  from P, under the product.  (Two sums added up at the end are 3 to 4 % faster, but change an ulp of
+//                  some of a prompt's rows, which every layer behind them multiplies.)  With one thread per row a tile was 14.9 k
+//                  clocks of its group, 8192 rows of 32 heads took 50.9 us, 48.7 so; 16 prompts of 1000 tokens with their writes and scan
+//                  199 and 172.
 //                  As in attn_fwd_kernel: causal softmax straight out of TMEM, unnormalised P (BF16) into
 //                  the tile's K and Q space (both dead once S and Mem are complete; the gate tile stays where it is),
-//                  O = P V issued by the group's first warp into the first 64 columns of S, gate blend from O, Mem
+//                  O = P V issued by the group's first warp into columns of its own, gate blend from O, Mem
 //                  and the gate tile into the Q space, one TMA store per 32 rows; the store's read of the tile releases
 //                  the ring stage, the group's last TMEM read releases the TMEM set.
 //
@@ -670,11 +671,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 // results.  PROMPT as in attn_fwd_kernel, but the low terms of P take the place, in TMEM, of the scores that they come from; their product
 // reads them there as its first operand.  Formed again from the scores, behind the product of the high ones and into their place in shared
 // memory, they were a second pass over the open chunk: 96 tiles of a 300-token prompt (with its writes and scan) 16.8 -> 14.9 us, 4096 tiles of
-// 16 x 1000 tokens 172 -> 162.
+// 16 x 1000 tokens 172 -> 162 (with a row's sum in two parts).
 constexpr int AS_STAGES = 3;
 constexpr int AS_THREADS = 25 * 32;
 constexpr int AS_STAGE_BYTES = 4 * TILE_BYTES + 8192;
-constexpr int AS_MEET = 2 * 4 * 128 * 4;   // per group and row: two maxima, two sums
+constexpr int AS_MEET = 2 * 3 * 128 * 4;   // per group and row: two maxima, the sum
 constexpr int AS_SMEM = AS_STAGES * AS_STAGE_BYTES + AS_MEET + 1024 + 256;
 
 template <bool PROMPT>
@@ -817,7 +818,9 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
     const uint32_t lane_base = static_cast<uint32_t>(wq * 32) << 16;
     const float kScale = 0.125f * 1.4426950408889634f;  // fold log2(e)
     const int last_chunk = wq;  // columns beyond 32*wq+31 are masked for the whole warp
-    float* meet = meetings + g * 512;           // [2][128] maxima | [2][128] sums
+    // this warp's two blocks of 32 columns: the first thread of a row has the front of what is visible (and a block of zeros where that is one)
+    const int block0 = half == 0 ? 0 : wq < 2 ? 1 : 2, block1 = half == 0 ? (wq < 2 ? 3 : 1) : block0 + 1;
+    float* meet = meetings + g * 384;           // [2][128] maxima | [128] sums
     // whether any of the group's threads is not ok; a barrier of its 256 threads
     auto any_bad = [&](bool ok) {
       uint32_t bad;
@@ -870,7 +873,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
       tc_fence_after_sync();
       float row_sum = 0.f, row_max = -INFINITY;
       if (ok) {
-        for (int cc = half; cc <= last_chunk; cc += 2) {
+        for (int cc = block0; cc <= last_chunk; cc = cc == block0 ? block1 : CHUNK) {
           uint32_t v[32];
           tmem_ld_32x32b_x32(t_s + lane_base + cc * 32, v);
           tmem_ld_wait();
@@ -886,7 +889,7 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         // REST: a prompt's open chunk, whose weights are two BF16 terms (a branch per score would cost every tile)
         auto weights = [&](auto rest_too) {
           constexpr bool REST = decltype(rest_too)::value;
-          for (int cc = half; cc < 4; cc += 2) {
+          for (int cc = block0; cc < 4; cc = cc == block0 ? block1 : CHUNK) {
             uint32_t pk[16];
             [[maybe_unused]] uint32_t low[16];
             if (cc <= last_chunk) {
@@ -920,12 +923,42 @@ attn_fwd_stream_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __gri
         if (PROMPT && open) weights(std::integral_constant<bool, PROMPT>{});
         else weights(std::false_type{});
       }
-      meet[256 + half * 128 + gt] = row_sum;
+      if (half == 0) meet[256 + gt] = row_sum;
       tc_fence_before_sync();
       fence_proxy_async_smem();
       if (any_bad(ok)) break;
-      row_sum = meet[256 + gt] + meet[384 + gt];
       if (warp == 8 + 8 * g && elect_one()) issue_o();
+      if (wq > 0) {   // under the product: behind the first thread's terms the second one's, from P
+        if (half == 1) {
+          float sum = meet[256 + gt];
+          const auto term = [](uint32_t two) {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&two));
+            return f.x + f.y;
+          };
+          if (PROMPT && open) tc_fence_after_sync();
+#pragma unroll 1
+          for (int cc = block0; cc <= last_chunk; ++cc) {
+            uint4 p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) p[j] = *reinterpret_cast<const uint4*>(tile_chunk(cc < 2 ? sK : sQ, gt, (cc & 1) * 4 + j));
+            if (PROMPT && open) {
+              uint32_t low[16];
+              tmem_ld_32x32b_x16(t_s + lane_base + cc * 32, low);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 4; ++j)
+                sum = sum + term(p[j].x) + term(low[4 * j]) + term(p[j].y) + term(low[4 * j + 1]) + term(p[j].z) + term(low[4 * j + 2]) +
+                      term(p[j].w) + term(low[4 * j + 3]);
+            } else {
+#pragma unroll
+              for (int j = 0; j < 4; ++j) sum = sum + term(p[j].x) + term(p[j].y) + term(p[j].z) + term(p[j].w);
+            }
+          }
+          meet[256 + gt] = sum;
+        }
+        pair_sync();
+      }
+      row_sum = meet[256 + gt];
       landed = 0;
       if (lane == 0) landed = mbar_wait(&ofull[g], k2 & 1, abort_flag) ? 1u : 0u;
       ok = __shfl_sync(0xffffffffu, landed, 0) != 0u;
