@@ -334,7 +334,7 @@ constexpr int SCAN_MAX_CHUNKS = SCAN_GROUP * SCAN_MAX_GROUPS;  // 32768 tokens p
 // so no barrier of the block is needed.  Such a copy has to pass L1 by: with 192 KiB taken as shared memory L1 is so small that
 // copies through it (8 bytes a thread) waited for its lines, 24.7 us at 4 x 16 chunks x 32 heads.  Now 16.5 us (84 MB, 5.1 TB/s),
 // 8 x 16 x 32 29.1 (5.8 TB/s), 2 x 7 x 20 5.0; a block per unit that loaded into registers, computed and left took 27.1, 50.2
-// and 5.8.
+// and 5.8.  Which product of a sum is rounded on its own, and the order of the sums, are that form's, bit for bit; it costs nothing (16.6, 29.3, 5.0).
 constexpr int SCAN_THREADS = 128;
 constexpr int SCAN_VEC = 2;
 constexpr int SCAN_SLOT = 2 * SCAN_GROUP * SCAN_THREADS;   // pairs: the writes and the state gradients of a group
@@ -361,6 +361,11 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   f32x2 d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
+}
+
+// sum + (x.x y.x + x.y y.y): one chain for both elements, so that the sums, too, are those of the form without packed instructions
+__device__ __forceinline__ void add_products(float& sum, float2 x, float2 y) {
+  sum = __fadd_rn(sum, __fmaf_rn(x.x, y.x, __fmul_rn(x.y, y.y)));
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS, 3)
@@ -420,7 +425,8 @@ memory_scan_bwd_kernel(const float* dstate, const float* writes,
     __nv_bfloat16* const out = dwrites + place(unit) + lane * SCAN_VEC;
     f32x2 f = 0, s = 0;
     // a, bb: gradients of the fast and slow state AFTER the chunk being visited (F_{n+1}, S_{n+1})
-    f32x2 a = 0, bb = 0, g_df = 0, g_ds = 0, g_mix = 0;
+    f32x2 a = 0, bb = 0;
+    float g_df = 0.f, g_ds = 0.f, g_mix = 0.f;
 #pragma unroll 1
     for (int piece = 0; piece < pieces; ++piece, slot ^= 1) {
       __syncwarp();   // every lane has done with the slot that is filled next
@@ -469,11 +475,13 @@ memory_scan_bwd_kernel(const float* dstate, const float* writes,
             *reinterpret_cast<uint32_t*>(to) = pack_bf16x2(dw.x, dw.y);
             to -= chunk_stride;
             asm volatile("" : "+l"(to));   // as above
-            g_df = fma2(a, fma2(w, minus, F[i]), g_df);    // F_{n+1} = df F_n + (1 - df) w_n
-            g_ds = fma2(bb, fma2(w, minus, S[i]), g_ds);
-            g_mix = fma2(gr, fma2(S[i], minus, F[i]), g_mix);
-            a = fma2(mix, gr, mul2(df, a));                // gradient of F_n
-            bb = fma2(rm, gr, mul2(ds, bb));
+            const float2 of_f = halves(a), of_s = halves(bb), of_mix = halves(gr);
+            const float2 by_f = halves(fma2(w, minus, F[i])), by_s = halves(fma2(w, minus, S[i])), by_mix = halves(fma2(S[i], minus, F[i]));
+            add_products(g_df, of_f, by_f);     // F_{n+1} = df F_n + (1 - df) w_n
+            add_products(g_ds, of_s, by_s);
+            add_products(g_mix, of_mix, by_mix);
+            a = fma2(df, a, mul2(mix, gr));     // gradient of F_n
+            bb = fma2(ds, bb, mul2(rm, gr));
           }
         }
       };
@@ -481,8 +489,7 @@ memory_scan_bwd_kernel(const float* dstate, const float* writes,
       else walk(std::false_type());
     }
     // block reduction (fixed order)
-    const float2 of_f = halves(g_df), of_s = halves(g_ds), of_mix = halves(g_mix);
-    const float vals[3] = {of_f.x + of_f.y, of_s.x + of_s.y, of_mix.x + of_mix.y};
+    const float vals[3] = {g_df, g_ds, g_mix};
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
       float v = vals[q];
