@@ -1,11 +1,12 @@
-"""The backward pass of the memories keeps its bits from version to version: an ulp here moves every gradient of the blocks before it.
-Digests of results on inputs that are computed from a counter, recorded with the one-block-per-unit form of the scan (CUDA 12.9)."""
+"""The backward pass of the attention and of the memories keeps its bits from version to version: an ulp here moves every gradient of the
+blocks before it.  Digests of results on inputs that are computed from a counter, recorded with the one-block-per-unit form of the
+scan and the one-CTA-per-tile form of the attention (CUDA 12.9)."""
 import ctypes
 
 import pytest
 import torch
 
-from warpstate_ai_b200.ops import _ext
+from warpstate_ai_b200.ops import _ext, attention, gemm
 
 MASK = (1 << 32) - 1
 
@@ -46,3 +47,25 @@ def scan(batch, chunks, heads):
                                                      (1, 40, 8, (2012217170, 2247772373))])
 def test_reverse_scan(batch, chunks, heads, want):
     assert scan(batch, chunks, heads) == want
+
+
+def backward(batch, tokens, heads):
+    ops, flag = torch.ops.ws_b200, gemm.error_flag(torch.device("cuda", torch.cuda.current_device()))
+    rope = attention.rope_table(flag.device, pair_major=True)
+    d = heads * 64
+    qkvgu = counted(6, (batch * tokens, 5 * d), 1.6).bfloat16()
+    dy = counted(7, (batch * tokens, d), 0.02).bfloat16()
+    logits = [counted(8, (heads,), 1.0, 2.2), counted(9, (heads,), 1.0, 4.6), counted(10, (heads,), 1.0)]
+    writes = ops.chunk_writes(qkvgu, rope, batch, tokens, heads, flag)
+    states = ops.memory_scan(writes, *logits, True, False, None, None)[0]
+    dqkvgu, partials = ops.attn_bwd(qkvgu, dy, states, writes, rope, *logits, batch, tokens, heads, flag)
+    gemm.check_device_errors()
+    return digest(dqkvgu), digest(partials)
+
+
+# a tile for some of the CTAs, several tiles for each
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,tokens,heads,want", [(2, 512, 8, (1284358552, 4244229321)), (3, 1152, 20, (4009705236, 1860216500)),
+                                                     (4, 2048, 32, (3996549729, 4087909000))])
+def test_attention_backward(batch, tokens, heads, want):
+    assert backward(batch, tokens, heads) == want

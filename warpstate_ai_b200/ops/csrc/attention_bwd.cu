@@ -530,8 +530,9 @@ memory_logit_grads_kernel(const float* partials, const float* fast_logit,
 // had landed, 2.8 k until its stores had read shared memory.  A CTA that goes on to its next tile requests Q and K of that one
 // as soon as the last products have read dS, whose buffer they take, and everything else once the stores have drained, behind
 // the rotation of Q and K.  The six tile buffers trade places for that, in pairs, from tile to tile.  Element-wise work that
-// does not need a product's result runs under it: dmem under S, dlocal and dlocal (1 - g) under O, the tanhs and dV under dQ and dK.
-// 2048 tiles (4 x 2048 tokens, 32 heads): 122.9 us with a CTA per tile, 107.8 so; 280 tiles (one round) 16.7 and 16.6.  What
+// does not need a product's result runs under it: dmem under S, dlocal under O, the tanhs and dV under dQ and dK.
+// 2048 tiles (4 x 2048 tokens, 32 heads): 122.9 us with a CTA per tile, 109 so; 280 tiles (one round) 16.7 and 16.6.  (dlocal (1 - g)
+// under O, too, is a microsecond faster, but rounds dGate in another order than the form with a CTA per tile.)  What
 // bounds it now is the load and store pipe, which tile traffic, tensor-core operands and TMA share: the gate row read by
 // each thread from global memory (16 bytes of 32 rows to an instruction) 117, registers spilled for 0.1 KB 118, four threads to a row 137.
 //
@@ -686,8 +687,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
         for (int t = 0; t < 4; ++t) {
           const float2 dyv = __bfloat1622float2(dyb[t]);
           const float2 gf = __bfloat1622float2(gb[t]);
-          // (1 - sigmoid(g)) / 8 = (1 - tanh(g / 2)) / 16
-          wo[t] = pack_bf16x2(dyv.x * fmaf(tanh_fast(0.5f * gf.x), -0.0625f, 0.0625f), dyv.y * fmaf(tanh_fast(0.5f * gf.y), -0.0625f, 0.0625f));
+          // the sigmoid is rounded before it is taken from 1, as the forward pass has it
+          wo[t] = pack_bf16x2(dyv.x * fmaf(sigmoid_f(gf.x), -0.125f, 0.125f), dyv.y * fmaf(sigmoid_f(gf.y), -0.125f, 0.125f));
         }
         ab_piece(sP + TILE_BYTES + mine_at, j) = o;
       }
@@ -783,12 +784,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
                   make_smem_desc_sw128((sB3) + k * 2048, 0, 1024), idesc_o, k > 0);
       umma_commit(&bars[3]);
     }
-    // ---- element-wise stage 1: under the product dlocal = dy * g (in place in B2) and dlocal * (1 - g), behind it
-    // dGate = dy (local - memory) g (1 - g) and D = sum(dlocal * local)
-    float dl[AB_PIECES * 8], dg[AB_PIECES * 8];
+    // ---- element-wise stage 1: under the product dlocal = dy * g (in place in B2), behind it dGate = dy (local - memory) g (1 - g),
+    // in that order, and D = sum(dlocal * local)
+    uint4 dy_row[AB_PIECES];
+    float sig[AB_PIECES * 8];
 #pragma unroll
     for (int i = 0; i < AB_PIECES; ++i) {
       uint4 dyq = ab_piece(sB2 + mine_at, i);
+      dy_row[i] = dyq;
       const uint4 gq = gate_row[i];
       uint32_t* w = reinterpret_cast<uint32_t*>(&dyq);
       const __nv_bfloat162* gb = reinterpret_cast<const __nv_bfloat162*>(&gq);
@@ -796,13 +799,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
       for (int t = 0; t < 4; ++t) {
         const float2 dyv = __bfloat1622float2(*reinterpret_cast<__nv_bfloat162*>(&w[t]));
         const float2 gf = __bfloat1622float2(gb[t]);
-        const float g0 = sigmoid_f(gf.x), g1 = sigmoid_f(gf.y);
         const int e0 = i * 8 + 2 * t, e1 = e0 + 1;
-        dl[e0] = dyv.x * g0;
-        dl[e1] = dyv.y * g1;
-        dg[e0] = dl[e0] * (1.f - g0);
-        dg[e1] = dl[e1] * (1.f - g1);
-        w[t] = pack_bf16x2(dl[e0], dl[e1]);
+        sig[e0] = sigmoid_f(gf.x);
+        sig[e1] = sigmoid_f(gf.y);
+        w[t] = pack_bf16x2(dyv.x * sig[e0], dyv.y * sig[e1]);
       }
       ab_piece(sB2 + mine_at, i) = dyq;
     }
@@ -820,9 +820,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_const
 #pragma unroll
       for (int j = 0; j < 16; j += 2) {
         const float l0 = __uint_as_float(ro[j]), l1 = __uint_as_float(ro[j + 1]);
-        const int e0 = i * 8 + j, e1 = e0 + 1;
-        Drow += dl[e0] * l0 + dl[e1] * l1;
-        w[j >> 1] = pack_bf16x2(dg[e0] * fmaf(__uint_as_float(rm[j]), -0.125f, l0), dg[e1] * fmaf(__uint_as_float(rm[j + 1]), -0.125f, l1));
+        const float m0 = __uint_as_float(rm[j]) * 0.125f, m1 = __uint_as_float(rm[j + 1]) * 0.125f;
+        const uint4& dyq = dy_row[i + (j >> 3)];
+        const float2 dyv = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(&dyq)[(j & 7) >> 1]);
+        const float g0 = sig[i * 8 + j], g1 = sig[i * 8 + j + 1];
+        const float dl0 = dyv.x * g0, dl1 = dyv.y * g1;
+        Drow += dl0 * l0 + dl1 * l1;
+        w[j >> 1] = pack_bf16x2(dyv.x * (l0 - m0) * g0 * (1.f - g0), dyv.y * (l1 - m1) * g1 * (1.f - g1));
       }
       dgate_row[i] = make_uint4(w[0], w[1], w[2], w[3]);
       dgate_row[i + 1] = make_uint4(w[4], w[5], w[6], w[7]);
