@@ -114,3 +114,25 @@ def test_a_short_prompt_streams_its_weights(monkeypatch, batch, length, d, ffn):
         for name in ("fast", "slow", "mixed", "k", "v", "u"):
             a, b = getattr(mine, name).float(), getattr(theirs, name).float()
             assert float((a - b).norm()) <= 0.01 * float(b.norm()), name
+
+
+# fewer rows than the decode projections take, which read the norms ahead of the launches in front of them; few heads, so that a vector of
+# logits is shorter than 16 bytes
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,length,d", [(1, 5, 512), (2, 60, 640), (1, 128, 512), (1, 200, 128)])
+def test_vectors_that_are_not_fp32_are_copied_once_and_before_the_chain(batch, length, d):
+    """The chain refuses to copy one once it has begun.  Norms and logits of values that BF16 holds: the same bits as in FP32."""
+    torch.manual_seed(d)
+    with torch.device("cuda"):
+        model = WarpStateLM(config(d, 704, depth=6, cores=2)).eval().requires_grad_(False)
+    vectors = [(core.norm1, "weight") for core in model.cores] + [(core.norm2, "weight") for core in model.cores]
+    vectors += [(core, name) for core in model.cores for name in ("fast_decay_logit", "slow_decay_logit", "memory_mix_logit")]
+    for owner, name in vectors:
+        getattr(owner, name).data = (torch.randn_like(getattr(owner, name)) * 0.2 + 1).bfloat16().float()
+    ids = torch.randint(0, 512, (batch, length), device="cuda")
+    want = DecodeEngine(model).prefill(ids).clone()
+    for owner, name in vectors:
+        getattr(owner, name).data = getattr(owner, name).data.bfloat16()
+    got = DecodeEngine(model).prefill(ids)
+    gemm.check_device_errors()
+    assert torch.equal(got, want)

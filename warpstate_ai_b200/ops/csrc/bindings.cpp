@@ -593,12 +593,24 @@ class ForwardBlocks {
     part_ = reinterpret_cast<float*>(at);
   }
 
-  // FP32 [d] or [H], in place or as a copy that lives as long as this object
+  // FP32 [d] (aligned to 16 bytes) or [H], in place or as a copy, one per tensor, that lives as long as this object.  All of them
+  // before `begin`: launches of the chain read norms and modulations ahead of their turn, so no launch in it may write them.
   const float* vector(const at::Tensor& t, int64_t n) {
     TORCH_CHECK(t.is_cuda() && t.numel() == n, "blocks: norms and modulation must have d elements, logits one per head");
-    if (t.scalar_type() == at::kFloat && t.is_contiguous() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0) return t.data_ptr<float>();
-    copies_.push_back(t.detach().to(at::kFloat).contiguous().clone());
-    return copies_.back().data_ptr<float>();
+    const auto usable = [&](const at::Tensor& v) { return n == H_ || reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 == 0; };
+    if (t.scalar_type() == at::kFloat && t.is_contiguous() && usable(t)) return t.data_ptr<float>();
+    for (const auto& [source, copy] : copies_)
+      if (source == t.unsafeGetTensorImpl()) return copy.data_ptr<float>();
+    TORCH_INTERNAL_ASSERT(residual_ == nullptr, "blocks: a copy of a vector behind the start of the chain");
+    at::Tensor copy = t.detach().to(at::kFloat).contiguous();
+    if (copy.data_ptr() == t.data_ptr()) copy = copy.clone();
+    copies_.emplace_back(t.unsafeGetTensorImpl(), std::move(copy));
+    return copies_.back().second.data_ptr<float>();
+  }
+  // norms [d] and logits [H] of a block
+  struct Vectors { const float *n1, *n2, *fast, *slow, *mix; };
+  Vectors vectors(const at::Tensor& n1, const at::Tensor& n2, const at::Tensor& fast, const at::Tensor& slow, const at::Tensor& mix) {
+    return {vector(n1, d_), vector(n2, d_), vector(fast, H_), vector(slow, H_), vector(mix, H_)};
   }
 
   void check_weights(const Weights& w) {
@@ -627,18 +639,18 @@ class ForwardBlocks {
     run(g, 1, "in_proj");
   }
 
-  void attention(const float* fast, const float* slow, const float* mix) {
+  void attention(const Vectors& v) {
     const bool memory = T_ > 128;
     if (memory) {
       check_rc(ws_chunk_writes(qkvgu_, rope_, writes_, (int)B_, (int)T_, (int)H_, (int)d_, flag_, stream_), "chunk_writes");
-      check_rc(ws_memory_scan(writes_, fast, slow, mix, states_, nullptr, nullptr, nullptr, nullptr, (int)B_, (int)(T_ / 128), (int)H_, stream_),
+      check_rc(ws_memory_scan(writes_, v.fast, v.slow, v.mix, states_, nullptr, nullptr, nullptr, nullptr, (int)B_, (int)(T_ / 128), (int)H_, stream_),
                "memory_scan");
     }
     check_rc(ws_attn_fwd(qkvgu_, memory ? states_ : nullptr, rope_, y_, (int)B_, (int)T_, (int)H_, (int)d_, flag_, stream_), "attn_fwd");
   }
 
-  void attention_prompt(const float* fast_logit, const float* slow_logit, const float* mix_logit, const at::Tensor* state) {
-    check_rc(ws_attn_prefill(qkvgu_, rope_, fast_logit, slow_logit, mix_logit, writes_, states_, y_, state[0].data_ptr<float>(),
+  void attention_prompt(const Vectors& v, const at::Tensor* state) {
+    check_rc(ws_attn_prefill(qkvgu_, rope_, v.fast, v.slow, v.mix, writes_, states_, y_, state[0].data_ptr<float>(),
                              state[1].data_ptr<float>(), state[2].data_ptr(), state[3].data_ptr(), state[4].data_ptr(), state[5].data_ptr(),
                              (int)B_, (int)T_, (int)H_, (int)d_, flag_, stream_), "attn_prefill");
   }
@@ -731,7 +743,7 @@ class ForwardBlocks {
   cudaStream_t stream_;
   int64_t pieces_out_ = 1, pieces_down_ = 1;
   at::Tensor scratch_;
-  std::vector<at::Tensor> copies_;
+  std::vector<std::pair<const c10::TensorImpl*, at::Tensor>> copies_;   // of vectors that the caller holds meanwhile
   float *x_, *xmod_, *rstd_, *writes_, *x2_, *part_;
   const float* residual_ = nullptr;
   uint8_t *z_, *y_, *qkvgu_, *states_, *act_;
@@ -828,11 +840,11 @@ struct BlockFn : public torch::autograd::Function<BlockFn> {
       ForwardBlocks blocks(B, T, spec->H, w.ug->size(0) / 2, spec->rope, spec->eps, spec->flag, false, x_in.options());
       blocks.check_weights(w);
       at::Tensor out = at::empty({B, T, d}, x_in.options());
-      blocks.begin(x_in.data_ptr<float>(), sc.defined() ? blocks.vector(sc, d) : nullptr, bi.defined() ? blocks.vector(bi, d) : nullptr,
-                   blocks.vector(n1, d));
+      const ForwardBlocks::Vectors v = blocks.vectors(n1, n2, fast, slow, mix);
+      blocks.begin(x_in.data_ptr<float>(), sc.defined() ? blocks.vector(sc, d) : nullptr, bi.defined() ? blocks.vector(bi, d) : nullptr, v.n1);
       blocks.project_in(w);
-      blocks.attention(blocks.vector(fast, spec->H), blocks.vector(slow, spec->H), blocks.vector(mix, spec->H));
-      blocks.finish(w, blocks.vector(n2, d), out.data_ptr<float>());
+      blocks.attention(v);
+      blocks.finish(w, v.n2, out.data_ptr<float>());
       return out;
     }
     const at::Tensor logits[3] = {vector(fast), vector(slow), vector(mix)};
@@ -950,13 +962,16 @@ std::tuple<at::Tensor, at::Tensor> blocks_prefill(const at::Tensor& x, const at:
       TORCH_CHECK(st[j].device() == x.device() && st[j].is_contiguous() && st[j].scalar_type() == (j < 2 ? at::kFloat : at::kBFloat16) &&
                   st[j].numel() == B * H * (j < 3 ? 4096 : 8192), "blocks_prefill: FP32 memories, BF16 mix and caches");
   }
-  blocks.begin(x.data_ptr<float>(), scale, bias, blocks.vector(vectors[0], d));
+  std::vector<ForwardBlocks::Vectors> v;
   for (int64_t i = 0; i < n; ++i) {
-    const at::Tensor* v = &vectors[5 * i];
+    const at::Tensor* t = &vectors[5 * i];
+    v.push_back(blocks.vectors(t[0], t[1], t[2], t[3], t[4]));
+  }
+  blocks.begin(x.data_ptr<float>(), scale, bias, v[0].n1);
+  for (int64_t i = 0; i < n; ++i) {
     blocks.project_in(of(i));
-    blocks.attention_prompt(blocks.vector(v[2], H), blocks.vector(v[3], H), blocks.vector(v[4], H), &states[6 * i]);
-    if (i + 1 < n)
-      blocks.finish(of(i), blocks.vector(v[1], d), nullptr, scale + (i + 1) * d, bias + (i + 1) * d, blocks.vector(v[5], d));
+    blocks.attention_prompt(v[i], &states[6 * i]);
+    if (i + 1 < n) blocks.finish(of(i), v[i].n2, nullptr, scale + (i + 1) * d, bias + (i + 1) * d, v[i + 1].n1);
   }
   at::Tensor last = at::empty({B, d}, x.options()), y = at::empty({B, d}, x.options().dtype(at::kBFloat16));
   const auto rows = [&](at::Tensor& to, const void* from, size_t element) {
