@@ -628,6 +628,7 @@ def cores_prefill_state(cores, x: torch.Tensor, depth_scale, depth_bias, batch: 
                                  G.error_flag(x.device))
 
 
+@torch.no_grad()
 def core_prefill_state(core, x: torch.Tensor, depth_scale, depth_bias, batch: int, seq: int, state, last: bool):
     """Forward of one core over prompts of any length ``x [B*T, d]``; ``state`` receives what a decode continues from.
     Returns the rows ``[B*T, d]``, or with ``last`` (nothing reads the other positions of the last block) the block's
