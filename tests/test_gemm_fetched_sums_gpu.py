@@ -34,3 +34,22 @@ def test_fetched_sums_equal_the_single_cta_kernels(tokens, shapes, alpha):
     gemm.check_device_errors()
     for mine, theirs, old in zip(*results, before):
         assert torch.equal(mine, theirs) and not torch.equal(mine, old)
+
+
+# the same gradient twice; two halves of the columns of one; rows that two share
+@pytest.mark.gpu
+@pytest.mark.parametrize("places", [lambda g: (g[:, :2048], g[:, :2048]), lambda g: (g[:, :2048], g[:, 2048:]), lambda g: (g[:8192, :2048], g[2048:, :2048])])
+def test_gradients_of_a_group_that_share_memory(places):
+    """Products and sums of small whole numbers, so that their order does not matter."""
+    torch.manual_seed(2)
+    tokens = 1024
+    total = torch.randint(-50, 50, (10240, 4096), device="cuda").float()
+    grads = places(total)
+    dys = [torch.randint(-1, 2, (tokens, g.shape[0]), device="cuda").bfloat16() for g in grads]
+    xs = [torch.randint(-1, 2, (tokens, g.shape[1]), device="cuda").bfloat16() for g in grads]
+    want = total.clone()
+    for g, dy, x in zip(places(want), dys, xs):
+        g += dy.float().t() @ x.float()
+    torch.ops.ws_b200.grad_weight_group(dys, xs, list(grads), [1.0] * len(grads), gemm.error_flag(total.device))
+    gemm.check_device_errors()
+    assert torch.equal(total, want)

@@ -1114,11 +1114,17 @@ extern "C" int ws_gemm_pair_split_norm(const WsGemm* g, int splits, float* part,
 // rows 129 -> 112, 512 134 -> 119, 1024 165 -> 151, 2048 247 -> 243, 4096 424 -> 427; 1280 at 256 49 -> 52, 512 56 -> 54, 896 65 -> 60, 1280 74 ->
 // 73, 1792 91 -> 92; 256 at 1024 16 -> 17; a head of 32768 x 2048 at 512 125 -> 110, 1024 154 -> 134, 2304 249 -> 248, 8192 742 -> 765, of
 // 32768 x 1280 at 1024 111 -> 92, of 32768 x 256 26 -> 30.  So up to 24 k-blocks where the tiles are four rounds, and below eight
-// only where the sums lie outside L2.
+// only where the sums lie outside L2.  Reductions of two items into one place add up; a fetch and a store lose one of them: so only
+// where no two gradients of the group share addresses.
 static bool sums_are_fetched(const WsGemm* items, int count, int tiles, int sms) {
   long long sums = 0;
+  const auto begin = [&](int i) { return static_cast<const float*>(items[i].out); };
+  const auto end = [&](int i) { return begin(i) + static_cast<size_t>(items[i].m - 1) * items[i].ldo + items[i].n; };
   for (int i = 0; i < count; ++i) {
     if (items[i].beta != 1.f || items[i].k > 1536) return false;   // with selected rows k is the most there can be
+    if (items[i].ldo < items[i].n) return false;
+    for (int j = 0; j < i; ++j)
+      if (begin(i) < end(j) && begin(j) < end(i)) return false;
     sums += static_cast<long long>(items[i].m) * items[i].n;
   }
   return tiles >= 4 * (sms / 2) && (items[0].k >= 512 || sums > (32ll << 20));

@@ -80,7 +80,8 @@ int ws_gemm_split(const WsGemm* g, int splits, float* part, cudaStream_t stream)
 // Number of SMs the GEMM may use on this stream's device (0 = all).  Lets a communication
 // kernel keep a few SMs for itself while persistent GEMM CTAs fill the rest.
 // `count` problems in one persistent launch where possible (same operand majors and epilogue, each
-// with >= 256 rows, count <= 4); otherwise equivalent to calling ws_gemm on each item in order.
+// with >= 256 rows, count <= 4); otherwise equivalent to calling ws_gemm on each item in order.  Sums (beta 1) of one group may share
+// memory.  No other launch may add to them at the same time: whether a sum is reduced into or fetched and stored depends on sizes.
 int ws_gemm_group(const WsGemm* items, int count, cudaStream_t stream);
 void ws_gemm_set_sm_limit(int sms);
 // Fused all-gather + FP32->BF16 cast + GEMM for a row-sharded weight (ops/csrc/gemm2_tcgen05.cu):
