@@ -136,3 +136,15 @@ def test_vectors_that_are_not_fp32_are_copied_once_and_before_the_chain(batch, l
     got = DecodeEngine(model).prefill(ids)
     gemm.check_device_errors()
     assert torch.equal(got, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("train", [False, True])
+@pytest.mark.parametrize("which", [0, 1])
+def test_a_modulation_of_another_device_is_refused(train, which):
+    with torch.device("cuda"):
+        core = WarpStateCore(config(256, 192)).requires_grad_(train)
+        x, mod = torch.randn(1, 128, 256), [torch.zeros(256), torch.zeros(256)]
+    mod[which] = mod[which].cpu()
+    with pytest.raises(RuntimeError, match="device"), torch.autocast("cuda", dtype=torch.bfloat16):
+        core(x, *mod)

@@ -161,14 +161,14 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_fwd(const at::Tensor& x,
                                                            const at::Tensor& w, double eps, bool want_xmod) {
   TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.is_contiguous(), "rmsnorm_fwd: x must be contiguous [rows,d]");
   TORCH_CHECK(x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16, "rmsnorm_fwd: x dtype");
-  TORCH_CHECK(w.scalar_type() == at::kFloat && w.is_contiguous() && w.numel() == x.size(1), "rmsnorm_fwd: w");
+  TORCH_CHECK(w.device() == x.device() && w.scalar_type() == at::kFloat && w.is_contiguous() && w.numel() == x.size(1), "rmsnorm_fwd: w");
   c10::cuda::CUDAGuard guard(x.device());
   const int rows = (int)x.size(0), d = (int)x.size(1);
   const bool mod = col_scale.has_value() && col_scale->defined();
   if (mod) {
-    TORCH_CHECK(col_scale->scalar_type() == at::kFloat && col_scale->is_contiguous() && col_scale->numel() == d &&
-                col_bias.has_value() && col_bias->scalar_type() == at::kFloat && col_bias->is_contiguous() &&
-                col_bias->numel() == d, "rmsnorm_fwd: depth modulation vectors must be float32 [d]");
+    TORCH_CHECK(col_scale->device() == x.device() && col_scale->scalar_type() == at::kFloat && col_scale->is_contiguous() &&
+                col_scale->numel() == d && col_bias.has_value() && col_bias->device() == x.device() && col_bias->scalar_type() == at::kFloat &&
+                col_bias->is_contiguous() && col_bias->numel() == d, "rmsnorm_fwd: depth modulation vectors must be float32 [d] on the device of x");
   }
   at::Tensor z = at::empty({rows, d}, x.options().dtype(at::kBFloat16));
   at::Tensor rstd = at::empty({rows}, x.options().dtype(at::kFloat));
@@ -566,7 +566,8 @@ class ForwardBlocks {
                 const at::TensorOptions& f32)
       : B_(B), T_(T), H_(H), M_(B * T), d_(H * 64), h_(h), rope_(rope.data_ptr<float>()), eps_((float)eps),
         flag_(reinterpret_cast<int*>(const_cast<void*>(opt_ptr(flag)))), wide_(wide), stream_(cur_stream()) {
-    TORCH_CHECK(rope.scalar_type() == at::kFloat && rope.is_contiguous() && rope.numel() == 128 * 64, "blocks: rope table");
+    TORCH_CHECK(rope.device() == f32.device() && rope.scalar_type() == at::kFloat && rope.is_contiguous() && rope.numel() == 128 * 64,
+                "blocks: rope table");
     TORCH_CHECK(B >= 1 && T >= 1 && H >= 1 && d_ % 128 == 0 && h % 8 == 0 && h > 0, "blocks: d must be a multiple of 128, the FFN width of 8");
     const int64_t chunks = (T + 127) / 128, memories = B * chunks * H * 4096;
     // the second half of a block lies where the first one's packed projections and memories were
@@ -596,7 +597,8 @@ class ForwardBlocks {
   // FP32 [d] (aligned to 16 bytes) or [H], in place or as a copy, one per tensor, that lives as long as this object.  All of them
   // before `begin`: launches of the chain read norms and modulations ahead of their turn, so no launch in it may write them.
   const float* vector(const at::Tensor& t, int64_t n) {
-    TORCH_CHECK(t.is_cuda() && t.numel() == n, "blocks: norms and modulation must have d elements, logits one per head");
+    TORCH_CHECK(t.device() == scratch_.device() && t.numel() == n,
+                "blocks: norms and modulation must have d elements, logits one per head, on the device of x");
     const auto usable = [&](const at::Tensor& v) { return n == H_ || reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 == 0; };
     if (t.scalar_type() == at::kFloat && t.is_contiguous() && usable(t)) return t.data_ptr<float>();
     for (const auto& [source, copy] : copies_)
