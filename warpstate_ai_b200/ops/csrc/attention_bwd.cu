@@ -1061,11 +1061,10 @@ extern "C" int ws_memory_scan_bwd(const float* dstate, const float* writes, cons
   static int sms = 0;
   if (sms == 0) {
     int dev = 0, n = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(memory_scan_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SCAN_SMEM) != cudaSuccess)
-      return -20;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -20;
     sms = n;
   }
+  if (!allow_shared_memory<memory_scan_bwd_kernel>(SCAN_SMEM)) return -20;
   const int units = B * H * 16;
   launch_dependent(memory_scan_bwd_kernel, dim3(units < 3 * sms ? units : 3 * sms), dim3(SCAN_THREADS), SCAN_SMEM, stream, dstate, writes,
                    fast_logit, slow_logit, mix_logit, (__nv_bfloat16*)dwrites, partials, B, N, H);

@@ -415,12 +415,7 @@ static int launch_rmsnorm_bwd_step(const void* dz, const void* x, const float* r
                                    const float* out_scale, int rows, int d, void* dx_out, void* dx_bf16, float* dw_partial,
                                    const float* mod_bias, int grid, cudaStream_t stream) {
   using Cfg = NormBackward<T, MOD, STEP>;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(rmsnorm_bwd_kernel<T, MOD, STEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
-      return -20;
-    configured = true;
-  }
+  if (!allow_shared_memory<rmsnorm_bwd_kernel<T, MOD, STEP>>(Cfg::SMEM)) return -20;
   launch_dependent(rmsnorm_bwd_kernel<T, MOD, STEP>, dim3(grid), dim3(ROW_THREADS), Cfg::SMEM, stream, static_cast<const __nv_bfloat16*>(dz),
                    static_cast<const T*>(x), rstd, w, static_cast<const T*>(dres), out_scale, rows, d, static_cast<T*>(dx_out),
                    static_cast<__nv_bfloat16*>(dx_bf16), dw_partial, mod_bias);

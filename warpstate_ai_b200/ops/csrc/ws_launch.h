@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdlib>
 
 namespace ws {
@@ -46,6 +47,19 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                                     Args... args) {
   return launch_kernel(true, kern, grid, block, smem, stream, args...);
+}
+
+// Allows KERNEL more shared memory than a launch has by default, once on each device of the process.
+template <auto KERNEL>
+inline bool allow_shared_memory(int bytes) {
+  static std::atomic<unsigned long long> allowed{0};
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess || device >= 64) return false;
+  const unsigned long long bit = 1ull << device;
+  if (allowed.load(std::memory_order_relaxed) & bit) return true;
+  if (cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+  allowed.fetch_or(bit, std::memory_order_relaxed);
+  return true;
 }
 
 }  // namespace ws
