@@ -37,3 +37,24 @@ def test_a_warp_per_head_gives_what_a_cta_per_head_gives(batch, heads, pos):
         assert float((y[part].float() - want.float()).norm() / want.float().norm()) < 1e-3
         for mine, theirs in zip(many, few):
             assert torch.equal(mine[part].view(torch.int16), theirs.view(torch.int16))
+
+
+@pytest.mark.gpu
+def test_outputs_at_any_element():
+    """The kernel with a warp per head stores 16 bytes at a time; outputs that begin elsewhere are written by the other one."""
+    _ext.require()
+    torch.manual_seed(3)
+    batch, heads = 40, 32
+    ops, d = torch.ops.ws_b200, 64 * heads
+    rope, at = attention.rope_table(torch.device("cuda", 0)), torch.tensor(50, device="cuda")
+    qkvgu = torch.randn(batch, 5 * d, device="cuda").bfloat16()
+    caches = [torch.randn(batch, heads, 128, 64, device="cuda").bfloat16() for _ in range(3)]
+    mixed = torch.randn(batch, heads, 64, 64, device="cuda").bfloat16()
+    room = torch.zeros(2, batch * d + 8, device="cuda", dtype=torch.bfloat16)
+    results = []
+    for part, offset in zip(room, (0, 3)):
+        y = part[offset:offset + batch * d].view(batch, d)
+        ops.decode_attn(qkvgu, *[t.clone() for t in caches], mixed, rope, at, heads, y, False)
+        results.append(y.float())
+    assert float((results[0] - results[1]).norm() / results[1].norm()) < 1e-3
+    assert not room[1, :3].any() and not room[1, 3 + batch * d:].any()

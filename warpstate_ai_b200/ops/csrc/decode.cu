@@ -1391,7 +1391,8 @@ extern "C" int ws_decode_attn(const void* qkvgu, void* kc, void* vc, void* uc, c
   }();
   const int items = batch * H;
   cudaError_t err;
-  if (!rows_form && items > 2 * ATTN_ROUND)
+  // (the warp form stores eight outputs at a time)
+  if (!rows_form && items > 2 * ATTN_ROUND && reinterpret_cast<uintptr_t>(y) % 16 == 0)
     err = launch_chained(decode_attn_warp_kernel, dim3((items + ATTN_WARPS - 1) / ATTN_WARPS), dim3(32 * ATTN_WARPS), 0, stream,
                          static_cast<const __nv_bfloat16*>(qkvgu), static_cast<__nv_bfloat16*>(kc), static_cast<__nv_bfloat16*>(vc),
                          static_cast<__nv_bfloat16*>(uc), static_cast<const __nv_bfloat16*>(mixed), reinterpret_cast<const float2*>(rope), pos,
