@@ -2,7 +2,9 @@
 import pytest
 import torch
 
-from warpstate_ai_b200.ops import _ext, attention
+from warpstate_ai_b200 import WarpStateConfig, WarpStateLM
+from warpstate_ai_b200.ops import _ext, attention, gemm
+from warpstate_ai_b200.serve.engine import DecodeEngine
 
 
 # the first row, the edges of the 32 rows that come at a time, the last row; a count that leaves warps of the last CTA idle
@@ -58,3 +60,25 @@ def test_outputs_at_any_element():
         results.append(y.float())
     assert float((results[0] - results[1]).norm() / results[1].norm()) < 1e-3
     assert not room[1, :3].any() and not room[1, 3 + batch * d:].any()
+
+
+# captured, the step requests the position, the caches and half of the memories ahead of its turn; a count that leaves warps of the last CTA
+# idle, over the edges of the 32 rows that come at a time, the end of a chunk and the first rows of the next
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,heads", [(40, 32), (41, 29)])
+def test_captured_steps_give_what_steps_one_by_one_give(batch, heads):
+    torch.manual_seed(heads)
+    cfg = WarpStateConfig(vocab_size=512, d_model=64 * heads, n_heads=heads, n_cores=2, logical_depth=2, ffn_hidden=128, chunk_size=128,
+                          gradient_checkpointing=False, parallel_memory=True)
+    with torch.device("cuda"):
+        model = WarpStateLM(cfg).eval().requires_grad_(False)
+    assert batch * heads > 1184
+    ids = torch.randint(0, 512, (batch, 170), device="cuda")
+    captured, single = DecodeEngine(model), DecodeEngine(model, use_cuda_graph=False)
+    for position in range(ids.shape[1]):
+        got, want = captured.step(ids[:, position]), single.step(ids[:, position])
+        assert torch.equal(got, want), position
+    gemm.check_device_errors()
+    assert captured.graph_counters.replay_calls == ids.shape[1] and single.graph_counters.eager_steps == ids.shape[1]
+    for mine, theirs in zip(captured.states, single.states):
+        assert all(torch.equal(getattr(mine, name), getattr(theirs, name)) for name in ("fast", "slow", "mixed", "k", "v", "u"))

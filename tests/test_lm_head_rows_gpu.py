@@ -184,3 +184,31 @@ def test_a_model_that_checkpoints_its_blocks_keeps_no_logits(checkpointing, hold
         loss.backward()
         del loss
     assert (held > 2048 * 8192 * 2) is holds                 # 32 MiB of logits
+
+
+# at most 1536 rows and at least four rounds of tiles: the weight gradient fetches its old sums, adds to them and stores them, for as many
+# k-blocks as the selection has rows
+@pytest.mark.parametrize("rows,d,kind", [(1200, 1024, 0), (1200, 1024, 1), (1200, 1024, 64), (1536, 768, 65), (1200, 1024, "span"), (1531, 1024, "random"),
+                                         (1536, 768, 1536)])
+def test_fetched_sums_of_a_selection(rows, d, kind):
+    _ext.require()
+    torch.manual_seed(rows + d)
+    vocab = 32768
+    hidden = torch.randn(rows, d, device="cuda").bfloat16()
+    labels, keep = labels_with(kind, rows, vocab)
+    hidden[~keep] = float("nan")
+    hidden.requires_grad_(True)
+    weight = (torch.randn(vocab, d, device="cuda") * 0.05).requires_grad_(True)
+    coef = torch.randn(rows, device="cuda")
+    before = torch.randn(vocab, d, device="cuda") * 0.01
+    weight.main_grad = before.clone()
+    logp = lmhead.token_logps(hidden, weight, labels)
+    (logp * coef).sum().backward()
+    check_device_errors()
+    if not keep.any():
+        assert torch.equal(weight.main_grad, before)
+        return
+    w32 = weight.detach().bfloat16().float().requires_grad_(True)
+    (R.lm_head_token_logps(hidden.detach()[keep].float(), w32, labels[keep]) * coef[keep]).sum().backward()
+    # the product as above; the sum and the difference here round once each
+    assert rel(weight.main_grad.double() - before.double(), w32.grad) < 0.02 + 2.0 ** -23 * float(before.norm() / w32.grad.norm())
