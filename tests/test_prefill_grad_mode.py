@@ -19,7 +19,6 @@ def test_a_block_with_gradients_enabled(monkeypatch, last):
         modes.append(torch.is_grad_enabled())
         return t * core.norm1.weight
 
-    monkeypatch.setattr(fused, "_native", lambda core, weights: False)
     monkeypatch.setattr(fused, "_prefill_norm", lambda core, x, scale, bias: (rows(x), rows(x)))
     monkeypatch.setattr(fused, "bf16_weight", lambda p: p)
     monkeypatch.setattr(fused.G, "linear", lambda x, w: rows(x))

@@ -469,8 +469,8 @@ at::Tensor memory_logit_grads(const at::Tensor& partials, const at::Tensor& fast
 // Smoke model (d 256, 4 depths, 2 x 512 tokens), forward + backward: 2.53 -> 2.03 ms.
 at::Tensor project(const at::Tensor& x, const at::Tensor& w, bool b_mn, int64_t epilogue, int64_t n, at::Tensor out,
                    const c10::optional<at::Tensor>& out2, const c10::optional<at::Tensor>& aux,
-                   const c10::optional<at::Tensor>& flag, bool wide = false) {
-  gemm(x, w, false, b_mn, epilogue, x.size(0), n, x.size(1), out, out2, aux, c10::nullopt, 1.0, 0.0, flag, wide);
+                   const c10::optional<at::Tensor>& flag) {
+  gemm(x, w, false, b_mn, epilogue, x.size(0), n, x.size(1), out, out2, aux, c10::nullopt, 1.0, 0.0, flag, false);
   return out;
 }
 at::Tensor project_bf16(const at::Tensor& x, const at::Tensor& w, const c10::optional<at::Tensor>& flag) {
@@ -520,17 +520,17 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> project_residual_norm(const at::T
 }
 
 // x2 = xmod + out_proj(y), then x2 + down(swiglu(up_gate(norm2 x2))).  -> (x2, rstd2, z2, packed, act, x3); packed only
-// with `keep` (the backward pass reads it), x3 only with `want_output`.  `wide` (serving): (up, gate) are not rounded.
+// with `keep` (the backward pass reads it), x3 only with `want_output`.
 struct BlockTail { at::Tensor x2, rstd2, z2, packed, act, x3; };
 BlockTail block_tail(const at::Tensor& y, const at::Tensor& xmod, const at::Tensor& w_out, const at::Tensor& n2,
                      const at::Tensor& w_ug, const at::Tensor& w_down, double eps, bool keep, bool want_output,
-                     const c10::optional<at::Tensor>& flag, bool wide = false) {
+                     const c10::optional<at::Tensor>& flag) {
   BlockTail t;
   std::tie(t.x2, t.z2, t.rstd2) = project_residual_norm(y, w_out, xmod, n2, eps, flag);
   const int64_t h = w_ug.size(0) / 2;
   if (keep) t.packed = at::empty({y.size(0), 2 * h}, y.options());
   t.act = at::empty({y.size(0), h}, y.options());
-  project(t.z2, w_ug, false, WS_EPI_SWIGLU, h, t.packed, t.act, c10::nullopt, flag, wide);
+  project(t.z2, w_ug, false, WS_EPI_SWIGLU, h, t.packed, t.act, c10::nullopt, flag);
   if (want_output) t.x3 = project_residual(t.act, w_down, t.x2, flag);
   return t;
 }
@@ -919,27 +919,8 @@ at::Tensor block(const at::Tensor& x, const c10::optional<at::Tensor>& scale, co
                         weights[3], fast, slow, mix, static_cast<const BlockSpec*>(&spec));
 }
 
-// Forward over prompts of any length; the layer's decode state is written.  -> the block's output rows [B*T, d], or with
-// `last` (residual input, attention output) at the final position of every sequence, [B, d] each.
-std::vector<at::Tensor> block_prefill(const at::Tensor& x, const at::Tensor& scale, const at::Tensor& bias,
-                                      const at::Tensor& n1, const at::Tensor& w_in, const at::Tensor& w_out,
-                                      const at::Tensor& n2, const at::Tensor& w_ug, const at::Tensor& w_down,
-                                      const at::Tensor& fast_logit, const at::Tensor& slow_logit, const at::Tensor& mix_logit,
-                                      const at::Tensor& rope, double eps, int64_t B, int64_t T, int64_t H, at::Tensor fast,
-                                      at::Tensor slow, at::Tensor mixed, at::Tensor kc, at::Tensor vc, at::Tensor uc, bool last,
-                                      const c10::optional<at::Tensor>& flag) {
-  auto [z1, rstd1, xmod] = rmsnorm_fwd(x, scale, bias, n1, eps, true);
-  at::Tensor y = attn_prefill(project_bf16(z1, w_in, flag), rope, fast_logit, slow_logit, mix_logit, B, T, H, fast, slow,
-                              mixed, kc, vc, uc, flag);
-  if (last) {
-    const int64_t d = x.size(1);
-    return {xmod.view({B, T, d}).select(1, T - 1).contiguous(), y.view({B, T, d}).select(1, T - 1).contiguous()};
-  }
-  return {block_tail(y, xmod, w_out, n2, w_ug, w_down, eps, false, true, flag, true).x3};
-}
-
-// All blocks over prompts of any length x [B*T, d] FP32, as `block_prefill` one by one: per block weights in, out, up/gate, down (BF16),
-// vectors n1, n2 and the three logits, states fast, slow, mixed, k, v, u (written); depth_scale and depth_bias [blocks, d].
+// All blocks over prompts of any length x [B*T, d] FP32: per block weights in, out, up/gate, down (BF16), vectors n1, n2 and the three
+// logits, and what a decode continues from, fast, slow, mixed, k, v, u (written); depth_scale and depth_bias [blocks, d].
 // -> (residual input, attention output) of the last block at the final position of every sequence, [B, d] each.
 std::tuple<at::Tensor, at::Tensor> blocks_prefill(const at::Tensor& x, const at::Tensor& depth_scale, const at::Tensor& depth_bias,
                                                   at::TensorList weights, at::TensorList vectors, at::TensorList states, const at::Tensor& rope,
@@ -1754,10 +1735,6 @@ TORCH_LIBRARY(ws_b200, m) {
   m.def("core_finished(int core, bool notify, Tensor[] small) -> bool");
   m.def("blocks_prefill(Tensor x, Tensor depth_scale, Tensor depth_bias, Tensor[] weights, Tensor[] vectors, Tensor(a!)[] states, Tensor rope, "
         "float eps, int B, int T, int H, Tensor(b!)? flag) -> (Tensor, Tensor)");
-  m.def("block_prefill(Tensor x, Tensor scale, Tensor bias, Tensor n1, Tensor w_in, Tensor w_out, Tensor n2, Tensor w_ug, "
-        "Tensor w_down, Tensor fast_logit, Tensor slow_logit, Tensor mix_logit, Tensor rope, float eps, int B, int T, int H, "
-        "Tensor(a!) fast, Tensor(b!) slow, Tensor(c!) mixed, Tensor(d!) kc, Tensor(e!) vc, Tensor(f!) uc, bool last, "
-        "Tensor(g!)? flag) -> Tensor[]");
   m.def("grad_norm_clip(Tensor g, float max_norm, Tensor? extra_sumsq, Tensor? status=None) -> Tensor");
   m.def("clip_from_partials(Tensor partial, float max_norm, Tensor? extra_sumsq=None, Tensor? status=None) -> Tensor");
   m.def("grad_reduce_segments(int[] grad_ptrs, int[] flag_ptrs, int mc_grad, int rank, int world, int[] starts, "
@@ -1816,7 +1793,6 @@ TORCH_LIBRARY_IMPL(ws_b200, CUDA, m) {
   m.impl("memory_logit_grads", &memory_logit_grads);
   m.impl("block_fwd", &block_fwd);
   m.impl("block_bwd", &block_bwd);
-  m.impl("block_prefill", &block_prefill);
   m.impl("blocks_prefill", &blocks_prefill);
   m.impl("attn_fwd", &attn_fwd);
   m.impl("attn_prefill", &attn_prefill);

@@ -630,19 +630,10 @@ def cores_prefill_state(cores, x: torch.Tensor, depth_scale, depth_bias, batch: 
 
 @torch.no_grad()
 def core_prefill_state(core, x: torch.Tensor, depth_scale, depth_bias, batch: int, seq: int, state, last: bool):
-    """Forward of one core over prompts of any length ``x [B*T, d]``; ``state`` receives what a decode continues from.
+    """Forward of one core over prompts of any length ``x [B*T, d]``, launch by launch; ``state`` receives what a decode continues from.
     Returns the rows ``[B*T, d]``, or with ``last`` (nothing reads the other positions of the last block) the block's
     residual input and its attention output at the final position of every sequence, ``[B, d]`` each."""
     from . import attention
-    weights = LocalWeights(core.in_proj.weight, core.out_proj.weight, core.ffn.up_gate.weight, core.ffn.down.weight)
-    if _native(core, weights):
-        w_in, w_out, w_ug, w_down = weights.backward_weights()
-        out = _ops().block_prefill(x, depth_scale.detach().float().contiguous(), depth_bias.detach().float().contiguous(),
-                                   core.norm1.weight.detach().float(), w_in, w_out, core.norm2.weight.detach().float(),
-                                   w_ug, w_down, *_native_arguments(core, x.device), core.cfg.rms_eps, batch, seq, core.h,
-                                   state.fast, state.slow, state.mixed, state.k, state.v, state.u, last,
-                                   G.error_flag(x.device))
-        return tuple(out) if last else out[0]
     z1, xmod = _prefill_norm(core, x, depth_scale, depth_bias)
     y = attention.prefill(G.linear(z1, bf16_weight(core.in_proj.weight)), core, batch, seq, state)
     if last:
