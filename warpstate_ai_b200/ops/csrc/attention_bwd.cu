@@ -12,8 +12,8 @@
 //                         the region the reference handles with flash-attention backward plus
 //                         its "paired backward layout" kernels (ops/backward_layout.py:114-210).
 //
-// All ten matrix products of the tile run on tcgen05 with accumulators in TMEM; one thread owns
-// one token row in every element-wise stage.
+// All ten matrix products of the tile run on tcgen05 with accumulators in TMEM; two threads share
+// a token row in every element-wise stage.
 #include <type_traits>
 #include "ws_ptx.cuh"
 #include "ws_api.h"
@@ -587,7 +587,7 @@ __device__ __forceinline__ uint4 tanh_piece(uint4 v) {
 __global__ void __launch_bounds__(AB_THREADS, 2)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_qkvgu, const __grid_constant__ CUtensorMap tm_state,
                 const __grid_constant__ CUtensorMap tm_dy, const __grid_constant__ CUtensorMap tm_dw,
-                const __grid_constant__ CUtensorMap tm_dout, const float2* rope, int T, int H, int d,
+                const __grid_constant__ CUtensorMap tm_dout, const float2* rope, int H, int d,
                 int tiles, int* error_flag) {
   extern __shared__ __align__(1024) uint8_t smem_ab[];
   uint8_t* smem = smem_ab;
@@ -1100,7 +1100,7 @@ extern "C" int ws_attn_bwd(const void* qkvgu, const void* states, const void* dy
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -20;
   }
   launch_dependent(attn_bwd_kernel, dim3(tiles < 2 * sms ? tiles : 2 * sms), dim3(AB_THREADS), AB_SMEM, stream, tm, ts, td, tw, to,
-                   reinterpret_cast<const float2*>(rope), T, H, d, tiles, error_flag);
+                   reinterpret_cast<const float2*>(rope), H, d, tiles, error_flag);
   ws_count_launch();
   return cudaGetLastError() == cudaSuccess ? 0 : -21;
 }

@@ -181,8 +181,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_fwd(const at::Tensor& x,
   return {z, rstd, xmod.defined() ? xmod : x};
 }
 
-// returns (dx, dx_bf16, dw) ; dw is the finished column sum [d]
-// dx, its BF16 copy where asked for, and the partial rows of the weight's gradient
+// -> (dx, its BF16 copy where asked for, the partial rows [parts, d] of the weight's gradient)
 std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd_partial(const at::Tensor& dz, const at::Tensor& x,
                                                                    const at::Tensor& rstd, const at::Tensor& w,
                                                                    const c10::optional<at::Tensor>& dres,
@@ -207,6 +206,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd_partial(const at::Ten
   return {dx, dxb, partial};
 }
 
+// The same with dw [d], their sum, in the place of the partial rows.
 std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz, const at::Tensor& x,
                                                            const at::Tensor& rstd, const at::Tensor& w,
                                                            const c10::optional<at::Tensor>& dres,
@@ -221,10 +221,9 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_bwd(const at::Tensor& dz,
   return {dx, dxb, dw};
 }
 
-// The norm behind a depth modulation (FP32 stream): -> (dx, FP32 [3, d]: gradients of w, of the bias, of the scale).  From
-// the modulation's input x; a caller that has only its output xmod gets x back as (xmod - bias) / (1 + scale), 0 where
-// scale is -1, with an error of an ulp of xmod over 1 + scale.
-// The same with the gradients' sums (`summed`), or with the partial rows [3, parts, d] that they are made of.
+// The norm behind a depth modulation (FP32 stream): -> (dx, the gradients of w, of the bias, of the scale: FP32 [3, d] where they are
+// `summed`, otherwise the partial rows [3, parts, d] that they are made of).  From the modulation's input x; a caller that has only its
+// output xmod gets x back as (xmod - bias) / (1 + scale), 0 where scale is -1, with an error of an ulp of xmod over 1 + scale.
 std::tuple<at::Tensor, at::Tensor> rmsnorm_bwd_modulated(const at::Tensor& dz, const c10::optional<at::Tensor>& xmod,
                                                          const at::Tensor& rstd, const at::Tensor& w, const at::Tensor& dres,
                                                          const at::Tensor& scale, const at::Tensor& bias,
@@ -576,10 +575,11 @@ class ForwardBlocks {
     pieces_down_ = streamed() ? ws_decode_gemm_splits((int)d_, (int)h_) : pieces(residual(nullptr, nullptr, nullptr, nullptr, h_));
     const int64_t cut = std::max(pieces_out_, pieces_down_);
     const int64_t back = aligned(4 * M_ * d_) + aligned(2 * M_ * h_) + (cut > 1 || streamed() ? aligned(4 * cut * M_ * d_) : 0);
-    scratch_ = at::empty({aligned(4 * M_ * d_) * 2 + aligned(2 * M_ * d_) * 2 + aligned(4 * M_) + std::max(front, back)}, f32.dtype(at::kByte));
+    const int64_t stream = wide ? aligned(4 * M_ * d_) : 0;   // between blocks; scoring is one block
+    scratch_ = at::empty({stream + aligned(4 * M_ * d_) + aligned(2 * M_ * d_) * 2 + aligned(4 * M_) + std::max(front, back)}, f32.dtype(at::kByte));
     uint8_t* at = scratch_.data_ptr<uint8_t>();
     const auto take = [&](int64_t bytes) { uint8_t* p = at; at += aligned(bytes); return p; };
-    x_ = reinterpret_cast<float*>(take(4 * M_ * d_));
+    x_ = wide ? reinterpret_cast<float*>(take(4 * M_ * d_)) : nullptr;
     xmod_ = reinterpret_cast<float*>(take(4 * M_ * d_));
     z_ = take(2 * M_ * d_);
     y_ = take(2 * M_ * d_);
@@ -853,20 +853,19 @@ struct BlockFn : public torch::autograd::Function<BlockFn> {
     std::vector<at::Tensor> s = block_fwd(x_in, maybe(sc), maybe(bi), vector(n1), spec->bf16[0], spec->bf16[1], vector(n2),
                                           spec->bf16[2], spec->bf16[3], logits[0], logits[1], logits[2], spec->rope, spec->eps,
                                           B, T, spec->H, true, true, spec->flag);
-    {   // x3, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, writes, states
-      const at::Tensor none = s[2];
-      ctx->save_for_backward({x_in, sc.defined() ? sc : none, bi.defined() ? bi : none, n1, n2, s[2], s[3], s[4], s[5], s[6],
-                              s[7], s[8], s[9], s[10]});
-      auto& data = ctx->saved_data;
-      data["attention"] = std::vector<at::Tensor>{s[11], s[12]};
-      data["weights"] = std::vector<at::Tensor>(spec->bf16, spec->bf16 + 4);
-      data["gradients"] = std::vector<at::Tensor>(spec->main, spec->main + 4);
-      data["logits"] = std::vector<at::Tensor>(logits, logits + 3);
-      data["rope"] = spec->rope;
-      data["flag"] = spec->flag.has_value() ? *spec->flag : at::Tensor();
-      data["hooked"] = spec->hooked;
-      data["shape"] = std::vector<int64_t>{B, T, d, spec->H, sc.defined() ? 1 : 0, spec->core, spec->notify ? 1 : 0};
-    }
+    // x3, xmod, rstd1, z1, qkvgu, y, x2, rstd2, z2, packed, act, writes, states
+    const at::Tensor none = s[2];
+    ctx->save_for_backward({x_in, sc.defined() ? sc : none, bi.defined() ? bi : none, n1, n2, s[2], s[3], s[4], s[5], s[6],
+                            s[7], s[8], s[9], s[10]});
+    auto& data = ctx->saved_data;
+    data["attention"] = std::vector<at::Tensor>{s[11], s[12]};
+    data["weights"] = std::vector<at::Tensor>(spec->bf16, spec->bf16 + 4);
+    data["gradients"] = std::vector<at::Tensor>(spec->main, spec->main + 4);
+    data["logits"] = std::vector<at::Tensor>(logits, logits + 3);
+    data["rope"] = spec->rope;
+    data["flag"] = spec->flag.has_value() ? *spec->flag : at::Tensor();
+    data["hooked"] = spec->hooked;
+    data["shape"] = std::vector<int64_t>{B, T, d, spec->H, sc.defined() ? 1 : 0, spec->core, spec->notify ? 1 : 0};
     return s[0].view({B, T, d});
   }
 
