@@ -148,3 +148,20 @@ def test_a_modulation_of_another_device_is_refused(train, which):
     mod[which] = mod[which].cpu()
     with pytest.raises(RuntimeError, match="device"), torch.autocast("cuda", dtype=torch.bfloat16):
         core(x, *mod)
+
+
+# the first length past those that stream at every width, and the last that would; one sequence and several
+@pytest.mark.gpu
+@pytest.mark.parametrize("batch,length,d,ffn", [(1, 97, 640, 704), (1, 128, 1280, 4480), (8, 16, 512, 704), (1, 128, 1920, 1024)])
+def test_past_96_tokens_only_the_widest_stream(monkeypatch, batch, length, d, ffn):
+    """The products' own kernels: the same bits as launch by launch."""
+    torch.manual_seed(length + d)
+    with torch.device("cuda"):
+        model = WarpStateLM(config(d, ffn, depth=4, cores=2)).eval().requires_grad_(False)
+    ids = torch.randint(0, 512, (batch, length), device="cuda")
+    together, apart = DecodeEngine(model), DecodeEngine(model)
+    got = together.prefill(ids).clone()
+    monkeypatch.setattr(fused, "cores_prefill_state", lambda *a: None)
+    want = apart.prefill(ids)
+    gemm.check_device_errors()
+    assert torch.equal(got, want)

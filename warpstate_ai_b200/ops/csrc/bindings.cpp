@@ -677,13 +677,16 @@ class ForwardBlocks {
   const void* attention_rows() const { return y_; }
 
  private:
-  // A prompt of at most 128 tokens is the rows of a decode step as far as its projections go: their time is that of the weights, which
-  // the step's kernels stream (decode.cu), and the rounding of (up, gate) is the step's too.  28 blocks of width 2048, with the products'
-  // own kernels -> so: 5 tokens 3911 -> 1450 us, 32 3991 -> 1567, 64 4139 -> 1909, 65 3811 -> 1999, 96 2226 -> 2055, 128 2440 -> 2253; 16 of
-  // 1280 at 16, 64, 96, 128 tokens 1605 -> 691, 1756 -> 843, 1050 -> 977, 1121 -> 1096.  Narrower blocks have projections of a few k-blocks,
-  // which there is nothing to stream of.
+  // A prompt of few tokens is the rows of a decode step as far as its projections go: their time is that of the weights, which
+  // the step's kernels stream (decode.cu), and the rounding of (up, gate) is the step's too.  12 blocks, with the products' own kernels ->
+  // so, us at 64, 96, 97, 112 and 128 tokens: width 2048 1570 -> 800, 927 -> 859, 940 -> 966, 950 -> 908, 1065 -> 950; 1792 1448 -> 709,
+  // 866 -> 790, 875 -> 920, 880 -> 856, 956 -> 887; 1536 1331 -> 647, 782 -> 745, 793 -> 879, 794 -> 840, 862 -> 870; 1280 1160 -> 595,
+  // 713 -> 688, 723 -> 746, 728 -> 760, 790 -> 814.  16 blocks: 1024 1288 -> 728, 946 -> 870, 961 -> 935, 962 -> 898, 1029 -> 974; 768 1180 -> 711,
+  // 877 -> 830, 887 -> 922, 900 -> 902, 973 -> 916; 512 998 -> 657, 785 -> 792, 794 -> 862, 814 -> 889, 893 -> 949; at 5 tokens 855 -> 650 and, at
+  // 1280, 1405 -> 660.  So up to 96 tokens, and past them, where the products have whole tiles, only the widest.  Narrower blocks have
+  // projections of a few k-blocks, which there is nothing to stream of.
   // Weights are read as they lie, row behind row, and the chain starts behind everything before it, as those kernels demand.
-  bool streamed() const { return wide_ && M_ <= 128 && d_ >= 512 && h_ % 64 == 0; }
+  bool streamed() const { return wide_ && M_ <= (d_ >= 2048 ? 128 : 96) && d_ >= 512 && h_ % 64 == 0; }
 
   void stream(const at::Tensor& w, const void* x, int64_t n, int64_t k, int epilogue, void* out, const char* what) {
     check_rc(ws_decode_gemm(w.data_ptr(), x, (int)n, (int)k, (int)M_, epilogue, out, (int)n, flag_, 0, stream_), what);
