@@ -909,7 +909,10 @@ decode_attn_rows_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bflo
 // the 16-byte piece jg of the rows rg, rg + 4, ...: eight lanes hold a score, all of them its weight, and the sums over rows meet at the end.
 // The first 32 rows of K and V and half of M are requested ahead of the wait where that is allowed (`early`, as above).
 // us a layer with a CTA per pair -> so, at positions 20, 70 and 120: 64 sequences x 32 heads 13.5 -> 7.2, 16.4 -> 12.4, 20.3 -> 15.8; 32 sequences
-// 7.4 -> 5.4, 8.9 -> 9.7, 10.4 -> 11.9; one 2.6 -> 2.4, 2.6 -> 4.1, 2.6 -> 4.8.  So from more than two rounds of CTAs (four to an SM) on.
+// 7.4 -> 5.4, 8.9 -> 9.7, 10.4 -> 11.9; one 2.6 -> 2.4, 2.6 -> 4.1, 2.6 -> 4.8.  So from more than two rounds of CTAs (four to an SM) on, where
+// the third begins; at 20, 70, 100 and 127 there: 38 sequences x 32 heads 9.0 -> 6.1, 10.6 -> 10.6, 11.8 -> 12.7, 12.9 -> 13.0; 40 9.5 -> 6.2,
+// 11.5 -> 10.8, 12.8 -> 12.7, 14.0 -> 13.0; 48 10.4 -> 6.5, 12.6 -> 11.0, 13.9 -> 13.2, 15.1 -> 13.7; 60 x 20 heads as 38 x 32.  Over the positions
+// of a chunk that is a gain at every count; only at 38 and around position 100 is a step slower by 8 % of this kernel.
 constexpr int ATTN_WARPS = 4;
 constexpr int ATTN_ROUND = 148 * 4;   // CTAs of decode_attn_kernel that the chip holds at once
 
@@ -1229,9 +1232,10 @@ static int launch_decode_gemm_depth(const CUtensorMap& tw, const CUtensorMap& tx
   return err == cudaSuccess ? 0 : -21;
 }
 
-// WS_DECODE_STAGES=9 is the deepest ring that fits (217 KiB at batch 64).  WS_DECODE_STAGES=4 selects the shallow ring (two CTAs per SM); the default is 8 (one CTA per SM): measured at
-// batch 64, 2.14 ms per token with 8 stages against 2.42 with 4 (2.21 with twice the K splits) -- the bytes a CTA
-// keeps in flight matter more than letting the next launch become resident early.
+// WS_DECODE_STAGES=9 is the deepest ring that fits (217 KiB at batch 64).  WS_DECODE_STAGES=4 selects the shallow ring (two CTAs per SM); the default is 8
+// (one CTA per SM): measured at batch 64, 2.14 ms per token with 8 stages against 2.42 with 4 (2.21 with twice the K splits) -- the bytes a
+// CTA keeps in flight matter more than letting the next launch become resident early.  The switch is for batches that are padded to 16
+// and 64 rows; those padded to 32 and 48 have 8 stages, prompts past 64 tokens what fits.
 static int decode_ring_depth() {
   static const int depth = [] {
     const char* e = std::getenv("WS_DECODE_STAGES");
