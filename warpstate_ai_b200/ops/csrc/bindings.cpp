@@ -552,7 +552,7 @@ std::vector<at::Tensor> block_fwd(const at::Tensor& x, const c10::optional<at::T
 }
 
 // Blocks that nothing differentiates, one after another in one call: scoring (one block) and prompts (all of them).  What passes
-// between the kernels lies in one allocation instead of fifteen a block, and goes from kernel to kernel by address; the
+// between the kernels lies in one allocation (or six) instead of fifteen a block, and goes from kernel to kernel by address; the
 // launches are those of `block_fwd`, but that the kernel which adds the pieces of a cut down projection forms the next
 // block's modulation and norm as well, and that one-chunk sequences, whose memories are empty, have no launches for them.
 // Scoring 128 tokens by a block of width 2048 95 -> 75 us, a prompt of 300 tokens in 28 blocks 2.92 -> 2.84 ms.
@@ -575,29 +575,38 @@ class ForwardBlocks {
     pieces_down_ = streamed() ? ws_decode_gemm_splits((int)d_, (int)h_) : pieces(residual(nullptr, nullptr, nullptr, nullptr, h_));
     const int64_t cut = std::max(pieces_out_, pieces_down_);
     const int64_t back = aligned(4 * M_ * d_) + aligned(2 * M_ * h_) + (cut > 1 || streamed() ? aligned(4 * cut * M_ * d_) : 0);
-    const int64_t stream = wide ? aligned(4 * M_ * d_) : 0;   // between blocks; scoring is one block
-    scratch_ = at::empty({stream + aligned(4 * M_ * d_) + aligned(2 * M_ * d_) * 2 + aligned(4 * M_) + std::max(front, back)}, f32.dtype(at::kByte));
-    uint8_t* at = scratch_.data_ptr<uint8_t>();
-    const auto take = [&](int64_t bytes) { uint8_t* p = at; at += aligned(bytes); return p; };
-    x_ = wide ? reinterpret_cast<float*>(take(4 * M_ * d_)) : nullptr;
+    // One allocation for scoring, whose time is the host's.  A prompt's are hundreds of megabytes, and the pool gives them back when a
+    // new engine captures its step (a graph's capture empties the pool's cache): as one piece that cost the first pass of 64 x 128 tokens
+    // with 40 steps a millisecond more than in parts, 35.0 and 33.8 ms.
+    const int64_t shared = std::max(front, back);
+    if (!wide) scratch_.push_back(at::empty({aligned(4 * M_ * d_) + aligned(2 * M_ * d_) * 2 + aligned(4 * M_) + shared}, f32.dtype(at::kByte)));
+    uint8_t* at = wide ? nullptr : scratch_.back().data_ptr<uint8_t>();
+    const auto take = [&](int64_t bytes) {
+      if (wide) {
+        scratch_.push_back(at::empty({aligned(bytes)}, f32.dtype(at::kByte)));
+        return scratch_.back().data_ptr<uint8_t>();
+      }
+      uint8_t* p = at;
+      at += aligned(bytes);
+      return p;
+    };
+    x_ = wide ? reinterpret_cast<float*>(take(4 * M_ * d_)) : nullptr;   // between blocks; scoring is one block
     xmod_ = reinterpret_cast<float*>(take(4 * M_ * d_));
     z_ = take(2 * M_ * d_);
     y_ = take(2 * M_ * d_);
     rstd_ = reinterpret_cast<float*>(take(4 * M_));
-    uint8_t* shared = at;
-    qkvgu_ = take(10 * M_ * d_);
-    writes_ = reinterpret_cast<float*>(take(4 * memories));
-    states_ = take(2 * memories);
-    at = shared;
-    x2_ = reinterpret_cast<float*>(take(4 * M_ * d_));
-    act_ = take(2 * M_ * h_);
-    part_ = reinterpret_cast<float*>(at);
+    qkvgu_ = take(shared);
+    writes_ = reinterpret_cast<float*>(qkvgu_ + aligned(10 * M_ * d_));
+    states_ = qkvgu_ + aligned(10 * M_ * d_) + aligned(4 * memories);
+    x2_ = reinterpret_cast<float*>(qkvgu_);
+    act_ = qkvgu_ + aligned(4 * M_ * d_);
+    part_ = reinterpret_cast<float*>(act_ + aligned(2 * M_ * h_));
   }
 
   // FP32 [d] (aligned to 16 bytes) or [H], in place or as a copy, one per tensor, that lives as long as this object.  All of them
   // before `begin`: launches of the chain read norms and modulations ahead of their turn, so no launch in it may write them.
   const float* vector(const at::Tensor& t, int64_t n) {
-    TORCH_CHECK(t.device() == scratch_.device() && t.numel() == n,
+    TORCH_CHECK(t.device() == scratch_[0].device() && t.numel() == n,
                 "blocks: norms and modulation must have d elements, logits one per head, on the device of x");
     const auto usable = [&](const at::Tensor& v) { return n == H_ || reinterpret_cast<uintptr_t>(v.data_ptr()) % 16 == 0; };
     if (t.scalar_type() == at::kFloat && t.is_contiguous() && usable(t)) return t.data_ptr<float>();
@@ -619,7 +628,7 @@ class ForwardBlocks {
     const int64_t rows[4] = {5 * d_, d_, 2 * h_, d_}, cols[4] = {d_, d_, d_, h_};
     const at::Tensor* t[4] = {w.in, w.out, w.ug, w.down};
     for (int i = 0; i < 4; ++i)
-      TORCH_CHECK(t[i]->device() == scratch_.device() && t[i]->scalar_type() == at::kBFloat16 && t[i]->dim() == 2 && t[i]->size(0) == rows[i] &&
+      TORCH_CHECK(t[i]->device() == scratch_[0].device() && t[i]->scalar_type() == at::kBFloat16 && t[i]->dim() == 2 && t[i]->size(0) == rows[i] &&
                   t[i]->size(1) == cols[i] && t[i]->stride(1) == 1 && t[i]->stride(0) % 8 == 0 &&
                   reinterpret_cast<uintptr_t>(t[i]->data_ptr()) % 16 == 0 && (!streamed() || t[i]->is_contiguous()),
                   "blocks: BF16 CUDA weights [5d, d], [d, d], [2 ffn, d], [d, ffn]");
@@ -747,7 +756,7 @@ class ForwardBlocks {
   const bool wide_;
   cudaStream_t stream_;
   int64_t pieces_out_ = 1, pieces_down_ = 1;
-  at::Tensor scratch_;
+  std::vector<at::Tensor> scratch_;
   std::vector<std::pair<const c10::TensorImpl*, at::Tensor>> copies_;   // of vectors that the caller holds meanwhile
   float *x_, *xmod_, *rstd_, *writes_, *x2_, *part_;
   const float* residual_ = nullptr;
