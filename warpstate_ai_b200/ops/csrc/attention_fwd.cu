@@ -409,8 +409,8 @@ memory_scan_kernel(const float* writes, const float* fast_logit,
     float4 w[SCAN_AHEAD];
 #pragma unroll
     for (int j = 0; j < SCAN_AHEAD; ++j)
-      if (PROMPT ? n0 + j < complete : n0 + j < N) w[j] = *reinterpret_cast<const float4*>(writes + base + (n0 + j) * chunk_stride);
-      else w[j] = make_float4(0.f, 0.f, 0.f, 0.f);   // nothing reads the state behind it
+      if (n0 + j < (PROMPT ? complete : N)) w[j] = *reinterpret_cast<const float4*>(writes + base + (n0 + j) * chunk_stride);
+      else if constexpr (PROMPT) w[j] = make_float4(0.f, 0.f, 0.f, 0.f);   // of the open chunk: nothing reads the state behind it
 #pragma unroll
     for (int j = 0; j < SCAN_AHEAD; ++j) {
       if (n0 + j >= N) break;
