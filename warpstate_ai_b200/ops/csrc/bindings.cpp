@@ -567,7 +567,7 @@ class ForwardBlocks {
         flag_(reinterpret_cast<int*>(const_cast<void*>(opt_ptr(flag)))), wide_(wide), stream_(cur_stream()) {
     TORCH_CHECK(rope.device() == f32.device() && rope.scalar_type() == at::kFloat && rope.is_contiguous() && rope.numel() == 128 * 64,
                 "blocks: rope table");
-    TORCH_CHECK(B >= 1 && T >= 1 && H >= 1 && d_ % 128 == 0 && h % 8 == 0 && h > 0, "blocks: d must be a multiple of 128, the FFN width of 8");
+    TORCH_CHECK(B >= 1 && T >= 1 && H >= 1 && d_ % 128 == 0 && h % 8 == 0 && h > 0, "blocks: no rows, or d not a multiple of 128, or an FFN width that is not one of 8");
     const int64_t chunks = (T + 127) / 128, memories = B * chunks * H * 4096;
     // the second half of a block lies where the first one's packed projections and memories were
     const int64_t front = aligned(10 * M_ * d_) + aligned(4 * memories) + aligned(2 * memories);
