@@ -31,6 +31,7 @@
 // ~40 eager PyTorch ops per layer at batch 1.
 #include "ws_ptx.cuh"
 #include "ws_api.h"
+#include "ws_launch.h"
 #include "ws_tma_host.h"
 
 #include <cuda_bf16.h>
@@ -914,7 +915,7 @@ decode_attn_rows_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bflo
 // 11.5 -> 10.8, 12.8 -> 12.7, 14.0 -> 13.0; 48 10.4 -> 6.5, 12.6 -> 11.0, 13.9 -> 13.2, 15.1 -> 13.7; 60 x 20 heads as 38 x 32.  Over the positions
 // of a chunk that is a gain at every count; only at 38 and around position 100 is a step slower by 8 % of this kernel.
 constexpr int ATTN_WARPS = 4;
-constexpr int ATTN_ROUND = 148 * 4;   // CTAs of decode_attn_kernel that the chip holds at once
+constexpr int ATTN_ROUND = CHIP_SMS * 4;   // CTAs of decode_attn_kernel that the chip holds at once
 
 __global__ void __launch_bounds__(32 * ATTN_WARPS, 4)
 decode_attn_warp_kernel(const __nv_bfloat16* qkvgu, __nv_bfloat16* kc, __nv_bfloat16* vc, __nv_bfloat16* uc, const __nv_bfloat16* mixed,

@@ -431,7 +431,7 @@ static int launch_rmsnorm_bwd(const void* dz, const void* x, const float* rstd, 
                               int rows, int d, void* dx_out, void* dx_bf16, float* dw_partial, const float* mod_bias, int grid,
                               cudaStream_t stream) {
   if constexpr (!MOD) {
-    if (grid > 148 * 2)
+    if (grid > CHIP_SMS * 2)
       return launch_rmsnorm_bwd_step<T, MOD, 1>(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, dw_partial, mod_bias, grid, stream);
   }
   return launch_rmsnorm_bwd_step<T, MOD, 2>(dz, x, rstd, w, dres, out_scale, rows, d, dx_out, dx_bf16, dw_partial, mod_bias, grid, stream);
@@ -607,7 +607,7 @@ embed_bwd_kernel(const T* __restrict__ dx, const long long* __restrict__ sorted_
   }
 }
 
-constexpr int CHIP_BLOCKS = 148 * 8;   // blocks of ROW_THREADS that the chip holds at once
+constexpr int CHIP_BLOCKS = CHIP_SMS * 8;   // blocks of ROW_THREADS that the chip holds at once
 static int row_grid(int rows) {
   int blocks = (rows + ROW_WARPS - 1) / ROW_WARPS;
   return blocks < CHIP_BLOCKS ? (blocks > 0 ? blocks : 1) : CHIP_BLOCKS;
@@ -666,7 +666,7 @@ extern "C" int ws_rmsnorm_fwd(const void* x, int x_bf16, const float* col_scale,
 }
 
 // Number of partial rows ws_rmsnorm_bwd writes (the caller sizes dw_partial as parts*d floats).
-constexpr int kRmsBwdMaxParts = 148 * 3;  // three resident blocks per SM
+constexpr int kRmsBwdMaxParts = CHIP_SMS * 3;  // three resident blocks per SM
 extern "C" int ws_rmsnorm_bwd_parts(int rows) {
   int blocks = (rows + RB_ROWS - 1) / RB_ROWS;
   return blocks < kRmsBwdMaxParts ? (blocks > 0 ? blocks : 1) : kRmsBwdMaxParts;
@@ -685,7 +685,7 @@ extern "C" int ws_rmsnorm_bwd(const void* dz, const void* x, int x_bf16, const f
 // Two resident blocks per SM: the modulation's column sums take the registers of the third.
 extern "C" int ws_rmsnorm_bwd_mod_parts(int rows) {
   const int blocks = (rows + RB_ROWS - 1) / RB_ROWS;
-  return blocks < 148 * 2 ? (blocks > 0 ? blocks : 1) : 148 * 2;
+  return blocks < CHIP_SMS * 2 ? (blocks > 0 ? blocks : 1) : CHIP_SMS * 2;
 }
 
 extern "C" int ws_rmsnorm_bwd_mod(const void* dz, const float* x, const float* rstd, const float* w, const float* dres,

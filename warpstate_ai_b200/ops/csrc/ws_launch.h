@@ -19,6 +19,10 @@
 
 namespace ws {
 
+// SMs of the chip that these kernels are built for.  Where a grid or a rule counts on this number and not on the device's, it decides how sums are
+// divided (partial rows whose number callers compute), or a line was measured with it.
+constexpr int CHIP_SMS = 148;
+
 inline bool train_pdl_enabled() {
   static const bool enabled = [] {
     const char* e = std::getenv("WS_TRAIN_PDL");
